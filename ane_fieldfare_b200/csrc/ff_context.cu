@@ -82,7 +82,7 @@ void ff_destroy(FFContext *ctx) {
                     ctx->partials, ctx->xDev, ctx->yDev, ctx->xSorted, ctx->sortedPairs,
                     ctx->expertOffsets, ctx->blockCounts, ctx->units, ctx->unitCount,
                     ctx->errorFlag, ctx->gridBarrier, ctx->phaseStamps, ctx->mapScratch, ctx->taggedLogits, ctx->taggedActs,
-                    ctx->logitsRows, ctx->routeIds, ctx->routeWeights};
+                    ctx->logitsRows, ctx->routeIds, ctx->routeWeights, ctx->xSums, ctx->actSums};
     for (void *p : ptrs) cudaFree(p);
     if (ctx->hostStream) cudaStreamDestroy(ctx->hostStream);
     if (ctx->mailbox) cudaFreeHost(const_cast<unsigned long long *>(ctx->mailbox));
@@ -424,7 +424,7 @@ bool ff_load_shared_int8(FFContext *ctx, uint32_t layer, const FFProjection *gat
             return false;
         ctx->weightBytes += codes + 2 * aux;
     }
-    return true;
+    return alloc_int8_gemm(ctx, error);
 }
 
 bool ff_load_router_int8(FFContext *ctx, uint32_t layer, const uint8_t *codes, const uint16_t *scales,

@@ -786,6 +786,10 @@ bool launch_shared_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, 
     if (D % 64 || Fs % 64) return fail(error, "widths must be multiples of 64");
     if (xStride % 2 || ((uintptr_t)x & 3)) return fail(error, "input rows must be 4-byte aligned");
     if (tokens > ctx->cfg.maxTokens) return fail(error, "rows exceed the context's maxTokens");
+    // more rows than a block, 16-byte aligned (what the tile copies and stores need): the tensor cores
+    if (tokens > (uint32_t)kMaxGemvRows && !((uintptr_t)x & 15) && !((uintptr_t)y & 15) && xStride % 8 == 0 &&
+        int8_gemm_fits(D, Fs))
+        return launch_shared_int8_gemm(ctx, L, x, xStride, tokens, y, stream, error);
     uint16_t *acts = ctx->sharedActs;
     const unsigned tokenBlocks = (tokens + kInt8RouterTokens - 1) / kInt8RouterTokens;
     {

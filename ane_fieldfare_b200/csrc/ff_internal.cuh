@@ -168,6 +168,7 @@ struct FFContext {
     uint32_t *units = nullptr;              // GEMM work units
     uint32_t *unitCount = nullptr;          // [4]
     uint32_t maxUnits = 0;
+    uint16_t *xSums = nullptr, *actSums = nullptr;  // group sums of the INT8 shared FFN's GEMM
     uint32_t *errorFlag = nullptr;          // device: set by a kernel that gave up waiting
     unsigned long long *phaseStamps = nullptr;  // device: 8 phase + 288 per-warp timestamps of the fused decode kernel
     unsigned long long *taggedLogits = nullptr;  // device: [kMaxExperts] router logits of the fused decode kernel
@@ -282,6 +283,12 @@ bool launch_route_sort(FFContext *ctx, const uint32_t *groupIds, uint32_t tokens
 bool launch_router_prefill(FFContext *ctx, const LayerStore &L, const uint16_t *x,
                            uint32_t xStride, uint32_t tokens, uint32_t *ids, uint16_t *weights,
                            float *logits, cudaStream_t stream, const char **error);
+
+// ff_int8_gemm.cu
+bool int8_gemm_fits(uint32_t d, uint32_t f);  // contraction lengths within the kernel's shared memory
+bool launch_shared_int8_gemm(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens,
+                             uint16_t *y, cudaStream_t stream, const char **error);
+bool alloc_int8_gemm(FFContext *ctx, const char **error);
 
 // nine offsets for a blob holding gate/up [f][d] and down [d][f]
 FFExpertOffsets packed_offsets(uint32_t d, uint32_t f, uint64_t *payload);
