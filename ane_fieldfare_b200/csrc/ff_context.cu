@@ -57,6 +57,10 @@ static void free_layer(LayerStore &L) {
     cudaFree(L.routerQ);
     cudaFree(L.routerQScale);
     cudaFree(L.routerQBias);
+    cudaFree(L.routerFolded);
+    cudaFree(L.routerCoef);
+    cudaFree(L.routerLanes);
+    cudaFree(L.routerAux);
     cudaFree(L.routerW);
     cudaFree(L.routerScale);
     cudaFree(L.gain);
@@ -82,7 +86,7 @@ void ff_destroy(FFContext *ctx) {
                     ctx->partials, ctx->xDev, ctx->yDev, ctx->xSorted, ctx->sortedPairs,
                     ctx->expertOffsets, ctx->blockCounts, ctx->units, ctx->unitCount,
                     ctx->errorFlag, ctx->gridBarrier, ctx->phaseStamps, ctx->mapScratch, ctx->taggedLogits, ctx->taggedActs,
-                    ctx->logitsRows, ctx->routeIds, ctx->routeWeights, ctx->xSums, ctx->actSums};
+                    ctx->logitsRows, ctx->routeIds, ctx->routeWeights, ctx->xSums, ctx->actSums, ctx->routerParts};
     for (void *p : ptrs) cudaFree(p);
     if (ctx->hostStream) cudaStreamDestroy(ctx->hostStream);
     if (ctx->mailbox) cudaFreeHost(const_cast<unsigned long long *>(ctx->mailbox));
@@ -181,6 +185,7 @@ FFContext *ff_create(int32_t deviceOrdinal, const FFConfig *config, const char *
         ok = ok && dev_alloc(ctx, &ctx->expertOffsets, c.experts + 1, error);
         ok = ok && dev_alloc(ctx, &ctx->blockCounts, (permuteBlocks + 1) * c.experts, error);
         ok = ok && dev_alloc(ctx, &ctx->units, (size_t)ctx->maxUnits * 4, error);
+        ok = ok && dev_alloc(ctx, &ctx->routerParts, router_parts_rows(T) * c.experts, error);
         ok = ok && dev_alloc(ctx, &ctx->unitCount, 8, error);
         if (ok) ok = cudaMemset(ctx->unitCount, 0, 32) == cudaSuccess;
     }
@@ -378,6 +383,14 @@ static void free_router(ff::LayerStore &L) {
     cudaFree(L.routerQ);
     cudaFree(L.routerQScale);
     cudaFree(L.routerQBias);
+    cudaFree(L.routerFolded);
+    cudaFree(L.routerCoef);
+    cudaFree(L.routerLanes);
+    cudaFree(L.routerAux);
+    L.routerFolded = nullptr;
+    L.routerCoef = nullptr;
+    L.routerLanes = nullptr;
+    L.routerAux = nullptr;
     L.routerW = L.routerScale = L.gain = L.routerQScale = L.routerQBias = nullptr;
     L.routerQ = nullptr;
     L.logitBias = nullptr;
@@ -464,7 +477,7 @@ bool ff_load_router_int8(FFContext *ctx, uint32_t layer, const uint8_t *codes, c
         FF_CUDA_OK(cudaMalloc(reinterpret_cast<void **>(&ctx->routeIds), (size_t)ctx->cfg.topK * sizeof(uint32_t)), error);
         FF_CUDA_OK(cudaMalloc(reinterpret_cast<void **>(&ctx->routeWeights), (size_t)ctx->cfg.topK * sizeof(uint16_t)), error);
     }
-    return true;
+    return router_prepare(ctx, L, error);
 }
 
 bool ff_load_router(FFContext *ctx, uint32_t layer, const uint16_t *weights,
@@ -499,7 +512,7 @@ bool ff_load_router(FFContext *ctx, uint32_t layer, const uint16_t *weights,
     }
     L.routerExperts = experts;
     ctx->weightBytes += wBytes;
-    return true;
+    return router_prepare(ctx, L, error);
 }
 
 uint64_t ff_expert_address(const FFContext *ctx, uint32_t layer, uint32_t expert) {

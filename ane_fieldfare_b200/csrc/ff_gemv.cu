@@ -657,58 +657,7 @@ static bool launch_inline_job(FFContext *ctx, const GemvJob &job, cudaStream_t s
     return true;
 }
 
-// INT8 affine router (the shipped checkpoints' form), one warp per expert row and up to four
-// tokens.  The order of the reference's kernel (Metal/MoE/moe.metal:65-103) is kept and made
-// definite: lane l takes elements 64 g + 2 l and 64 g + 2 l + 1 of every group g in increasing g,
-// with x' = float(x) * float(effective scale): acc = fma(s_g, fma(q1, x1', q0 * x0'), acc), then
-// acc = fma(b_g, x0' + x1', acc); the lane sums are added by an xor butterfly (16, 8, 4, 2, 1) and the
-// per-expert logit bias comes last.
-constexpr int kInt8RouterTokens = 4;
-__global__ void __launch_bounds__(256)
-k_router_logits_int8(const uint8_t *W, const uint16_t *scales, const uint16_t *biases, const uint16_t *effScale,
-                     const float *bias, const uint16_t *x, uint32_t xStride, int T, int E, int D, float *logits) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int e = blockIdx.x * 8 + warp;
-    const int t0 = blockIdx.y * kInt8RouterTokens;
-    if (e >= E) return;
-    const int groups = D / 64;
-    const uint8_t *wr = W + (size_t)e * D;
-    const uint16_t *sr = scales + (size_t)e * groups, *br = biases + (size_t)e * groups;
-    float acc[kInt8RouterTokens];
-#pragma unroll
-    for (int r = 0; r < kInt8RouterTokens; ++r) acc[r] = 0.0f;
-    for (int g = 0; g < groups; ++g) {
-        const int idx = g * 64 + 2 * lane;
-        const uint32_t q = *reinterpret_cast<const uint16_t *>(wr + idx);
-        const float q0 = (float)(q & 0xFFu), q1 = (float)(q >> 8);
-        const float s = bf2f(sr[g]), b = bf2f(br[g]);
-        float e0 = 1.0f, e1 = 1.0f;
-        if (effScale) {
-            const uint32_t ev = *reinterpret_cast<const uint32_t *>(effScale + idx);
-            e0 = __uint_as_float(ev << 16);
-            e1 = __uint_as_float(ev & 0xFFFF0000u);
-        }
-#pragma unroll
-        for (int r = 0; r < kInt8RouterTokens; ++r) {
-            const int t = min(t0 + r, T - 1);
-            const uint32_t xv = *reinterpret_cast<const uint32_t *>(x + (size_t)t * xStride + idx);
-            float x0 = __uint_as_float(xv << 16), x1 = __uint_as_float(xv & 0xFFFF0000u);
-            if (effScale) {
-                x0 = x0 * e0;
-                x1 = x1 * e1;
-            }
-            acc[r] = fmaf(s, fmaf(q1, x1, q0 * x0), acc[r]);
-            acc[r] = fmaf(b, x0 + x1, acc[r]);
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < kInt8RouterTokens; ++r) {
-        float v = acc[r];
-#pragma unroll
-        for (int offset = 16; offset >= 1; offset >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, offset);
-        if (lane == 0 && t0 + r < T) logits[(size_t)(t0 + r) * E + e] = bias ? v + bias[e] : v;
-    }
-}
+constexpr int kInt8Rows = 4;  // input rows of a warp
 
 // INT8 affine shared FFN (Metal/Quant/dequant_int8.metal:41-138; Kernels/MoE/SharedExpertInt8.swift),
 // one warp per output row and up to four input rows, in the reference kernels' order made definite:
@@ -723,15 +672,15 @@ k_int8_rows(const uint8_t *W0, const uint16_t *S0, const uint16_t *B0, const uin
             uint32_t outStride) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = blockIdx.x * 8 + warp;
-    const int t0 = blockIdx.y * kInt8RouterTokens;
+    const int t0 = blockIdx.y * kInt8Rows;
     if (r >= rows) return;
     const int groups = cols / 64;
     const uint8_t *w0 = W0 + (size_t)r * cols, *w1 = DUAL ? W1 + (size_t)r * cols : nullptr;
     const uint16_t *s0 = S0 + (size_t)r * groups, *b0 = B0 + (size_t)r * groups;
     const uint16_t *s1 = DUAL ? S1 + (size_t)r * groups : nullptr, *b1 = DUAL ? B1 + (size_t)r * groups : nullptr;
-    float acc0[kInt8RouterTokens], acc1[kInt8RouterTokens];
+    float acc0[kInt8Rows], acc1[kInt8Rows];
 #pragma unroll
-    for (int i = 0; i < kInt8RouterTokens; ++i) acc0[i] = acc1[i] = 0.0f;
+    for (int i = 0; i < kInt8Rows; ++i) acc0[i] = acc1[i] = 0.0f;
     for (int g = 0; g < groups; ++g) {
         const int idx = g * 64 + 2 * lane;
         const uint32_t q = *reinterpret_cast<const uint16_t *>(w0 + idx);
@@ -746,7 +695,7 @@ k_int8_rows(const uint8_t *W0, const uint16_t *S0, const uint16_t *B0, const uin
             bb = bf2f(b1[g]);
         }
 #pragma unroll
-        for (int i = 0; i < kInt8RouterTokens; ++i) {
+        for (int i = 0; i < kInt8Rows; ++i) {
             const int t = min(t0 + i, T - 1);
             const uint32_t xv = *reinterpret_cast<const uint32_t *>(x + (size_t)t * xStride + idx);
             const float x0 = __uint_as_float(xv << 16), x1 = __uint_as_float(xv & 0xFFFF0000u);
@@ -760,7 +709,7 @@ k_int8_rows(const uint8_t *W0, const uint16_t *S0, const uint16_t *B0, const uin
         }
     }
 #pragma unroll
-    for (int i = 0; i < kInt8RouterTokens; ++i) {
+    for (int i = 0; i < kInt8Rows; ++i) {
         float a = acc0[i], b = acc1[i];
 #pragma unroll
         for (int offset = 16; offset >= 1; offset >>= 1) {
@@ -791,7 +740,7 @@ bool launch_shared_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, 
         int8_gemm_fits(D, Fs))
         return launch_shared_int8_gemm(ctx, L, x, xStride, tokens, y, stream, error);
     uint16_t *acts = ctx->sharedActs;
-    const unsigned tokenBlocks = (tokens + kInt8RouterTokens - 1) / kInt8RouterTokens;
+    const unsigned tokenBlocks = (tokens + kInt8Rows - 1) / kInt8Rows;
     {
         LaunchScope scope(ctx, stream, "shared_int8_gate_up_act");
         k_int8_rows<true><<<dim3((Fs + 7) / 8, tokenBlocks), 256, 0, stream>>>(
@@ -816,26 +765,15 @@ k_topk_rows(const float *logits, const uint16_t *gain, int T, int E, int K, uint
     warp_topk(logits + (size_t)t * E, E, K, gain, ids + (size_t)t * K, weights + (size_t)t * K);
 }
 
-bool launch_router_logits_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride,
-                               uint32_t tokens, float *logits, cudaStream_t stream, const char **error) {
-    const int E = (int)L.routerExperts, D = (int)ctx->cfg.d;
-    if (xStride % 2 || ((uintptr_t)x & 3)) return fail(error, "input rows must be 4-byte aligned");
-    dim3 grid((E + 7) / 8, (tokens + kInt8RouterTokens - 1) / kInt8RouterTokens);
-    {
-        LaunchScope scope(ctx, stream, "router_logits_int8");
-        k_router_logits_int8<<<grid, 256, 0, stream>>>(L.routerQ, L.routerQScale, L.routerQBias, L.routerScale,
-                                                       L.logitBias, x, xStride, (int)tokens, E, D, logits);
-    }
-    FF_CUDA_OK(cudaGetLastError(), error);
-    return true;
-}
-
 bool launch_router_topk(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride,
                         uint32_t tokens, uint32_t *ids, uint16_t *weights, float *logits,
                         cudaStream_t stream, const char **error) {
     if (tokens == 0) return true;
     if (!L.has_router()) return fail(error, "layer has no resident router");
     const int E = (int)L.routerExperts, D = (int)ctx->cfg.d;
+    // (16-byte aligned rows for the tile copies; a CTA's rows as fp32 in shared memory)
+    if (tokens > kMaxGemvRows && !logits && !((uintptr_t)x & 15) && xStride % 8 == 0 && D % 64 == 0 && D <= 12288)
+        return launch_router_select(ctx, L, x, xStride, tokens, ids, weights, stream, error);
     if (L.routerQ && tokens > kMaxGemvRows) {
         float *lg = logits ? logits : ctx->logitsRows;
         if (!launch_router_logits_int8(ctx, L, x, xStride, tokens, lg, stream, error)) return false;

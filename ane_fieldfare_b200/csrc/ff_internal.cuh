@@ -117,6 +117,12 @@ struct LayerStore {
     // bias per group of 64 inputs; set instead of routerW
     uint8_t *routerQ = nullptr;
     uint16_t *routerQScale = nullptr, *routerQBias = nullptr;
+    // for a prefill chunk's routes: the weights as the tensor cores multiply them (null: routerW), and a
+    // bound of each approximate logit's error per unit of the row's 2-norm
+    uint16_t *routerFolded = nullptr;
+    float *routerCoef = nullptr;
+    uint16_t *routerLanes = nullptr;  // INT8 router rows in lane order, and their scales | biases
+    uint32_t *routerAux = nullptr;
     bool has_router() const { return routerW != nullptr || routerQ != nullptr; }
     // INT8 affine shared FFN (the shipped checkpoints' form): gate, up [sharedF][d] and down
     // [d][sharedF] as codes with one bf16 scale and bias per group of 64; set instead of `shared`
@@ -168,6 +174,7 @@ struct FFContext {
     uint32_t *units = nullptr;              // GEMM work units
     uint32_t *unitCount = nullptr;          // [4]
     uint32_t maxUnits = 0;
+    float *routerParts = nullptr;           // approximate logits of a prefill chunk
     uint16_t *xSums = nullptr, *actSums = nullptr;  // group sums of the INT8 shared FFN's GEMM
     uint32_t *errorFlag = nullptr;          // device: set by a kernel that gave up waiting
     unsigned long long *phaseStamps = nullptr;  // device: 8 phase + 288 per-warp timestamps of the fused decode kernel
@@ -283,6 +290,15 @@ bool launch_route_sort(FFContext *ctx, const uint32_t *groupIds, uint32_t tokens
 bool launch_router_prefill(FFContext *ctx, const LayerStore &L, const uint16_t *x,
                            uint32_t xStride, uint32_t tokens, uint32_t *ids, uint16_t *weights,
                            float *logits, cudaStream_t stream, const char **error);
+
+// ff_router.cu
+size_t router_parts_rows(size_t maxTokens);
+bool router_prepare(FFContext *ctx, LayerStore &L, const char **error);
+bool launch_router_select(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens,
+                          uint32_t *ids, uint16_t *weights, cudaStream_t stream, const char **error);
+
+bool launch_router_logits_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens,
+                               float *logits, cudaStream_t stream, const char **error);
 
 // ff_int8_gemm.cu
 bool int8_gemm_fits(uint32_t d, uint32_t f);  // contraction lengths within the kernel's shared memory
