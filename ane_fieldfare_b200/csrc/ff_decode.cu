@@ -19,16 +19,16 @@
 // tile's rows lie at one stride (one request brings 8 or 16 row pieces), cp.async.bulk for scale
 // runs and for the routed down rows of the eight scattered experts.
 //
-// Row arithmetic runs on the tensor cores without dequantizing: a warp task is a tile of 16 weight
-// rows; per group of 64 codes the packed nibbles are turned into the bf16 values 16+q with two
-// integer instructions per pair (the code goes into the mantissa of 16.0) and multiplied with the
-// bf16 input by mma.sync m16n8k16 (fp32 accumulate; the product of a 5-bit integer and a bf16 is
-// exact).  The group's sum is then scaled:
-//     acc += scale * sum((16+q) x) + (bias - 16 scale) * sum(x).
-// The eight columns of the MMA are one input row for the gate/up and shared rows, and the eight
-// routed experts' activations for the routed down rows (a tile = two output rows of all eight
-// experts).  Long rows are split along K between the warps of a pair (or triple) of one CTA and
-// added in a fixed order, so results do not depend on scheduling.
+// Row arithmetic runs on the integer tensor cores straight on the codes (ff_int_device.cuh): a warp task
+// is a tile of 16 weight rows, two runs of eight — gate and up rows of the same features, sixteen rows
+// of the shared down projection, or the same eight output rows of two routed experts, whose
+// activations then fill the eight digit columns of the MMA.  Long rows are split along K between the
+// warps of a pair (quad, triple) of one CTA and added in a fixed order, the experts' down rows in rank
+// order, so results do not depend on scheduling.
+//
+// What bounds a step: the chain router row -> logits through L2 -> routes -> routed rows from HBM (3.8
+// us for 19.5 MB) -> activations through L2 -> down rows.  Turning nibbles into bf16 pairs used to add
+// 4.6 us behind the routed rows' arrival and 1.0 us of ranking stood in front of them (23.7 us a step).
 //
 // Grid-wide waits poll arrival counters in global memory; cooperative launch guarantees that all
 // CTAs are resident.  Every spin (grid barrier, copy completion) is bounded: on running
@@ -42,7 +42,7 @@
 #include <cstring>
 #include <string>
 
-#include "ff_mma_device.cuh"
+#include "ff_int_device.cuh"
 
 namespace ff {
 
@@ -50,6 +50,7 @@ constexpr int kFusedThreads = 512;
 constexpr int kFusedWarps = kFusedThreads / 32;
 constexpr int kBigWarps = 10;      // warps 0..9: gate/up pairs and the routed down tiles
 constexpr int kSharedGuWarps = 8;  // warps 0..7 take the shared gate/up tiles in phase A (K quarters)
+constexpr int kRouterWarps = 2;    // warps 8, 9 the router rows
 constexpr uint32_t kBarrierSpinLimit = 1u << 24;
 
 struct DecodeArgs {
@@ -64,7 +65,6 @@ struct DecodeArgs {
     const uint16_t *residual;
     const uint32_t *idsIn;  // non-null: routes are given, the router is skipped
     const uint16_t *weightsIn;
-    float *logits;
     // Values handed from CTA to CTA travel as 64-bit words (launch tag << 32 | payload) that the
     // readers poll: a word is valid when its tag is the running launch's, so nothing is cleared.
     unsigned long long *taggedLogits;  // [E] payload: the logit's bits
@@ -72,57 +72,33 @@ struct DecodeArgs {
     unsigned long long *taggedH1;      // [D / 2] payload: two rows of the shared FFN's output (bf16)
     uint32_t *ids;
     uint16_t *weights;
-    uint16_t *acts, *sharedActs, *h1, *y;
+    uint16_t *sharedActs, *y;
     unsigned long long *barrier;  // arrival counter of the grid barrier
     uint32_t *errorFlag;
     unsigned long long *stamps;  // null, or the phase / per-warp timestamp slots (ns)
     int E, D, F, Fs, K;          // K = 0: shared FFN only (y receives its output)
     int expertCount;             // resident experts of the layer: routes at or past it are refused
-    int prefetch;                // bit 0: L2 prefetch of the chosen experts' down projections (off by default)
     // host hand-off (null when unused): the last CTA to finish copies y to `hostY` (host memory the
     // device can write), then stores (error flag << 32 | epoch) to `mailbox`, which the host polls
     uint16_t *hostY;
     unsigned long long *mailbox;
     uint32_t epoch;
     // shared-memory carve-up (fused_layout)
-    uint32_t regionOffset, partialOffset, slotsOffset, bigBytes, smallBytes;
-    uint32_t strideGU, strideGUA, strideSD, strideRD, actStride, winBytes, winPitch;
+    uint32_t regionOffset, regionAux, partialOffset, downOffset, slotsOffset, rowsBytes, pairBytes, tripleBytes, downBytes;
+    uint32_t strideGU, strideGUA, strideSD, strideRD;
 };
 
 // Row-box tensor maps of the layer (kernel parameters): routed gate, routed up, shared gate, shared
-// up, shared down.  A tile's eight (sixteen) row pieces arrive as one tensor copy per matrix.
+// up, shared down, routed down.  A tile's eight (sixteen) row pieces arrive as one tensor copy per matrix.
 struct alignas(64) DecodeMaps {
-    CUtensorMap m[5];
+    CUtensorMap m[kDecodeMaps];
 };
-enum : int { kMapRoutedGate = 0, kMapRoutedUp = 1, kMapSharedGate = 2, kMapSharedUp = 3, kMapSharedDown = 4 };
+enum : int { kMapRoutedGate = 0, kMapRoutedUp = 1, kMapSharedGate = 2, kMapSharedUp = 3, kMapSharedDown = 4, kMapRoutedDown = 5 };
 
 // Fetches a tensor map's descriptor ahead of its first use (the first copy through a map otherwise
 // waits for it).
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
-}
-
-// Bulk L2 prefetch of [p, p + bytes); bytes a multiple of 16, p 16-byte aligned.
-__device__ __forceinline__ void prefetch_l2_bulk(const void *p, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
-// The grid prefetches [base, base+bytes) in 8 KiB pieces.  Piece i belongs to CTA (i + cursor) mod
-// gridDim and to one of its `nthreads` issuing threads (this one is number `tid`), so every SM
-// issues the same share: a bulk prefetch is executed by the issuing SM's copy engine, whose
-// throughput is a small fraction of HBM's.
-// `issue` false: only the cursor moves on (another warp takes this region).
-__device__ __forceinline__ void prefetch_region(const uint8_t *base, uint64_t bytes, uint32_t &cursor, uint32_t tid,
-                                                uint32_t nthreads, bool issue) {
-    constexpr uint32_t kPiece = 8192;
-    const uint32_t pieces = (uint32_t)((bytes + kPiece - 1) / kPiece);
-    const uint32_t first = (blockIdx.x + gridDim.x - cursor % gridDim.x) % gridDim.x;
-    for (uint32_t i = first + tid * gridDim.x; issue && i < pieces; i += gridDim.x * nthreads) {
-        const uint64_t offset = (uint64_t)i * kPiece;
-        const uint32_t len = (uint32_t)min((uint64_t)kPiece, bytes - offset) & ~15u;
-        if (len) prefetch_l2_bulk(base + offset, len);
-    }
-    cursor += pieces;
 }
 
 // Grid-wide synchronisation on 64-bit counters that only grow.  At its start every CTA draws a
@@ -189,45 +165,6 @@ __device__ __forceinline__ void warp_stamp(const DecodeArgs &a, int phase, int w
     }
 }
 
-// `n` consecutive groups of a 16-row tile: acc0 / acc1 = this thread's sums for tile rows g and
-// g+8.  s0/b0 and s1/b1: the two rows' scales and biases, xs: the input's group sums, all starting
-// at the first group.  `odd` picks MMA column 2t+1 instead of 2t.  Groups are taken in ascending
-// order whatever the batching, so the result does not depend on it.  Shared by every phase.
-__device__ __noinline__ void tile_rows(const uint8_t *lo, const uint8_t *hi, const uint8_t *xg, const uint16_t *s0,
-                                       const uint16_t *b0, const uint16_t *s1, const uint16_t *b1, const float *xs,
-                                       int n, bool odd, float &acc0, float &acc1) {
-    float v0 = 0.0f, v1 = 0.0f;
-    int i = 0;
-#pragma unroll 1
-    for (; i + 4 <= n; i += 4) {
-        float d[4][4];
-        groups_mma<4>(lo + 32 * i, hi + 32 * i, xg + 128 * i, d);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            v0 = group_scale(v0, s0[i + u], b0[i + u], odd ? d[u][1] : d[u][0], xs[i + u]);
-            v1 = group_scale(v1, s1[i + u], b1[i + u], odd ? d[u][3] : d[u][2], xs[i + u]);
-        }
-    }
-    if (i + 2 <= n) {
-        float d[2][4];
-        groups_mma<2>(lo + 32 * i, hi + 32 * i, xg + 128 * i, d);
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            v0 = group_scale(v0, s0[i + u], b0[i + u], odd ? d[u][1] : d[u][0], xs[i + u]);
-            v1 = group_scale(v1, s1[i + u], b1[i + u], odd ? d[u][3] : d[u][2], xs[i + u]);
-        }
-        i += 2;
-    }
-    if (i < n) {
-        float d[1][4];
-        groups_mma<1>(lo + 32 * i, hi + 32 * i, xg + 128 * i, d);
-        v0 = group_scale(v0, s0[i], b0[i], odd ? d[0][1] : d[0][0], xs[i]);
-        v1 = group_scale(v1, s1[i], b1[i], odd ? d[0][3] : d[0][2], xs[i]);
-    }
-    acc0 = v0;
-    acc1 = v1;
-}
-
 // Box of a row-box map at (64-bit word x, row y, expert z) into shared memory (128-byte aligned).
 // x * 8 bytes must be a multiple of 16.
 __device__ __forceinline__ void box_copy(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
@@ -238,33 +175,89 @@ __device__ __forceinline__ void box_copy(uint32_t dst, const CUtensorMap *map, i
         : "memory");
 }
 
-// stage_input for rows that other CTAs are still writing as tagged words (two bf16 values each):
-// every run of eight values is polled (bounded) until its four words carry `tag`.
-__device__ __forceinline__ void stage_tagged(const unsigned long long *src, uint32_t tag, int rows, int n, uint8_t *dst,
-                                             uint32_t dstStride, float *sums, uint32_t *errorFlag) {
-    const int runsPerRow = n >> 3, runs = rows * runsPerRow;
-    auto fetch = [&](int i, uint4 &v) {
-        unsigned long long w0, w1, w2, w3;
-        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w0), "=l"(w1) : "l"(src + 4 * (size_t)i) : "memory");
-        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w2), "=l"(w3) : "l"(src + 4 * (size_t)i + 2) : "memory");
-        v = make_uint4((uint32_t)w0, (uint32_t)w1, (uint32_t)w2, (uint32_t)w3);
-        return (uint32_t)(w0 >> 32) == tag && (uint32_t)(w1 >> 32) == tag && (uint32_t)(w2 >> 32) == tag &&
-               (uint32_t)(w3 >> 32) == tag;
-    };
-    for (int base = (threadIdx.x >> 5) << 5; base < runs; base += 2 * blockDim.x) {
-        const int i = base + (threadIdx.x & 31), j = i + blockDim.x;
-        const bool vi = i < runs, vj = j < runs;
-        uint4 v0 = make_uint4(0, 0, 0, 0), v1 = make_uint4(0, 0, 0, 0);
-        bool ok0 = !vi, ok1 = !vj;
-        for (uint32_t spins = 0; spins < kBarrierSpinLimit && !(ok0 && ok1); ++spins) {
-            if (!ok0) ok0 = fetch(i, v0);
-            if (!ok1) ok1 = fetch(j, v1);
-        }
-        if (!(ok0 && ok1)) atomicExch(errorFlag, 9u);
-        stage_put(i, vi, v0, runsPerRow, dst, dstStride, sums);
-        if (base + (int)blockDim.x < runs) stage_put(j, vj, v1, runsPerRow, dst, dstStride, sums);  // warp-uniform
+// Rows of bf16 values as digits (flat run index over all rows) by `threads` threads, this one number
+// `tid`; `fetch` returns the run's eight values.  No barrier at the end.
+template <typename Fetch>
+__device__ __forceinline__ void stage_digits(int runs, int tid, int threads, uint8_t *digits, GroupAux *aux, Fetch fetch) {
+    for (int base = tid & ~31; base < runs; base += threads) {
+        const int i = base + (tid & 31);
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (i < runs) v = fetch(i);
+        digits_put(i, i < runs, v, digits, aux);
     }
-    __syncthreads();
+}
+// A run of eight values that another CTA is still writing as four tagged words, polled (bounded).
+__device__ __forceinline__ uint4 fetch_tagged(const unsigned long long *src, uint32_t tag, uint32_t *errorFlag) {
+    unsigned long long w0 = 0, w1 = 0, w2 = 0, w3 = 0;
+    bool ok = false;
+    for (uint32_t spins = 0; spins < kBarrierSpinLimit && !ok; ++spins) {
+        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w0), "=l"(w1) : "l"(src) : "memory");
+        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w2), "=l"(w3) : "l"(src + 2) : "memory");
+        ok = (uint32_t)(w0 >> 32) == tag && (uint32_t)(w1 >> 32) == tag && (uint32_t)(w2 >> 32) == tag && (uint32_t)(w3 >> 32) == tag;
+    }
+    if (!ok) atomicExch(errorFlag, 9u);
+    return make_uint4((uint32_t)w0, (uint32_t)w1, (uint32_t)w2, (uint32_t)w3);
+}
+
+// A float as an unsigned number of the same order.
+__device__ __forceinline__ uint32_t ordered_key(float f) {
+    const uint32_t u = __float_as_uint(f);
+    return (u >> 31) ? ~u : (u | 0x80000000u);
+}
+
+// The K largest of E logits that arrive as tagged words, by one warp: higher score, then lower id;
+// -inf and NaN are never taken.  Lane r < K returns route r's id (0 when there is none) and score.
+// Each round is two warp-wide reductions over register keys (0.3 us for eight routes of 128; counting
+// every logit's rank by 256 threads through shared memory took 1.0 us).
+__device__ __forceinline__ void poll_and_rank(const DecodeArgs &a, uint32_t tag, int lane, uint32_t &myId, float &myScore) {
+    uint32_t key[8];
+#pragma unroll
+    for (int blk = 0; blk < 2; ++blk) {
+        const int e0 = 128 * blk + 4 * lane;
+        const unsigned long long filler = (unsigned long long)tag << 32;
+        unsigned long long w[4] = {filler, filler, filler, filler};
+        bool ready = 128 * blk >= a.E;
+        const bool here = !ready;
+        for (uint32_t spins = 0; spins < kBarrierSpinLimit && !ready; ++spins) {
+            if (e0 + 3 < a.E) {
+                asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w[0]), "=l"(w[1]) : "l"(a.taggedLogits + e0) : "memory");
+                asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w[2]), "=l"(w[3]) : "l"(a.taggedLogits + e0 + 2) : "memory");
+            } else {
+                for (int i = 0; i < 4; ++i)
+                    if (e0 + i < a.E) w[i] = ld_tagged(a.taggedLogits + e0 + i);
+            }
+            const bool mine = (uint32_t)(w[0] >> 32) == tag && (uint32_t)(w[1] >> 32) == tag && (uint32_t)(w[2] >> 32) == tag &&
+                              (uint32_t)(w[3] >> 32) == tag;
+            ready = __all_sync(0xFFFFFFFFu, mine);
+        }
+        if (!ready && lane == 0) atomicExch(a.errorFlag, 9u);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float v = __uint_as_float((uint32_t)w[i]);
+            key[4 * blk + i] = here && e0 + i < a.E && v > -INFINITY ? ordered_key(v) : 0u;
+        }
+    }
+    myId = 0u;
+    myScore = -INFINITY;
+    for (int r = 0; r < a.K; ++r) {
+        uint32_t best = key[0], at = 4u * (uint32_t)lane;
+#pragma unroll
+        for (int j = 1; j < 8; ++j)
+            if (key[j] > best) {
+                best = key[j];
+                at = (uint32_t)(128 * (j >> 2) + 4 * lane + (j & 3));
+            }
+        const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, best);
+        if (top == 0u) break;
+        const uint32_t id = __reduce_min_sync(0xFFFFFFFFu, best == top ? at : 0xFFFFFFFFu);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (id == (uint32_t)(128 * (j >> 2) + 4 * lane + (j & 3))) key[j] = 0u;
+        if (lane == r) {
+            myId = id;
+            myScore = __uint_as_float((top >> 31) ? (top & 0x7FFFFFFFu) : ~top);
+        }
+    }
 }
 
 // The input row travelling inside the kernel's parameters (no host-to-device copy before the
@@ -276,11 +269,9 @@ struct InlineRow {
 // xInline: null, or the input row in parameter space (read with plain loads).
 __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMaps &maps, const uint16_t *xInline) {
     extern __shared__ __align__(128) uint8_t smemRaw[];
-    __shared__ __align__(16) float sLogits[kMaxExperts + 8];  // padded with -inf up to two spans of the ranking
     __shared__ uint32_t sIds[8];
     __shared__ float sWeights[8];
-    __shared__ float sScore[8];
-    __shared__ __align__(8) uint64_t sCopyBar[kFusedWarps];
+    __shared__ __align__(8) uint64_t sCopyBar[kFusedWarps + kRouterWarps];
     __shared__ unsigned long long sTarget;  // (generation + 1) * gridDim
     __shared__ uint32_t sTag;               // the launch's tag for polled words, from the generation
 
@@ -290,24 +281,32 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     const int g = lane >> 2, t = lane & 3;
     const int groupsD = D >> 6, groupsF = F >> 6, groupsFs = Fs >> 6;
 
-    // shared memory: x (bf16, run-permuted) | its group sums | region for the shared / routed
-    // activations | K-split partial sums | kBigWarps big slots | small slots for the other warps
-    uint8_t *xPerm = smemRaw;
-    float *xSum = reinterpret_cast<float *>(smemRaw + D * 2);
+    // shared memory: x as digits | its group sums | region: x as it is (router), then the shared
+    // activations, then the routed activations | K-split partial sums | routed down rows per expert |
+    // slots: five pairs (two tile parts, the tile's scales), two triples of the other six warps
+    const uint32_t smem = sm_addr(smemRaw);
     uint8_t *region = smemRaw + a.regionOffset;
+    GroupAux *regionAux = reinterpret_cast<GroupAux *>(smemRaw + a.regionAux);
+    GroupAux *xAux = reinterpret_cast<GroupAux *>(smemRaw + D * 4);
     float *partial = reinterpret_cast<float *>(smemRaw + a.partialOffset);  // [warp][16]
-    uint8_t *slots = smemRaw + a.slotsOffset;
-    uint8_t *mySlot = warp < kBigWarps ? slots + (size_t)warp * a.bigBytes
-                                        : slots + (size_t)kBigWarps * a.bigBytes + (size_t)(warp - kBigWarps) * a.smallBytes;
-    const uint32_t slotAddr = sm_addr(mySlot);
-    const uint32_t myBar = sm_addr(&sCopyBar[warp]);
+    float *downRows = reinterpret_cast<float *>(smemRaw + a.downOffset);    // [row tile][expert][8]
+    const int pair = warp >> 1;
+    const int triple = warp >= kBigWarps ? (warp - kBigWarps) / 3 : 0;
+    const int part3 = warp >= kBigWarps ? (warp - kBigWarps) % 3 : 0;
+    const uint32_t tripleBase = smem + a.slotsOffset + (kBigWarps / 2) * a.pairBytes + (uint32_t)triple * a.tripleBytes;
+    const uint32_t slot = warp < kBigWarps ? smem + a.slotsOffset + (uint32_t)pair * a.pairBytes + (uint32_t)(warp & 1) * a.rowsBytes
+                                            : tripleBase + (uint32_t)part3 * 16u * a.strideSD;
+    const uint32_t downSlot = warp < kBigWarps ? slot : tripleBase + (uint32_t)part3 * a.downBytes;
+    auto scalesOfPair = [&](int p) { return smem + a.slotsOffset + (uint32_t)p * a.pairBytes + 2u * a.rowsBytes; };
+    auto barOf = [&](int w) { return sm_addr(&sCopyBar[w]); };
+    const uint32_t myBar = barOf(warp);
     uint32_t parity = 0;
 
     if (threadIdx.x == 0) {
-        for (int w = 0; w < kFusedWarps; ++w) bar_init(sm_addr(&sCopyBar[w]), 1);
+        for (int w = 0; w < kFusedWarps + kRouterWarps; ++w) bar_init(barOf(w), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp >= 11 && lane == 0) prefetch_tensormap(&maps.m[warp - 11]);  // warps 11..15: the five maps
+    if (warp >= 10 && lane == 0) prefetch_tensormap(&maps.m[warp - 10]);  // warps 10..15: the six maps
     // the ticket: drawn now by a thread with nothing to request (warp 9), published to the CTA
     // further down so that nobody waits for the atomic's round trip here
     unsigned long long ticket = 0;
@@ -315,86 +314,97 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     // this thread's share of the input row is requested before anything else
     const bool xPlain = xInline != nullptr;
     const uint16_t *xSrc = xPlain ? xInline : a.x;
+    auto fetchX = [&](int i) {  // plain loads for a row in the kernel's parameters
+        return xPlain ? reinterpret_cast<const uint4 *>(xSrc)[i] : __ldcg(reinterpret_cast<const uint4 *>(xSrc) + i);
+    };
     uint4 xMine = make_uint4(0, 0, 0, 0);
-    if ((int)threadIdx.x < (D >> 3))
-        xMine = xPlain ? reinterpret_cast<const uint4 *>(xSrc)[threadIdx.x]
-                       : __ldcg(reinterpret_cast<const uint4 *>(xSrc) + threadIdx.x);
+    if ((int)threadIdx.x < (D >> 3)) xMine = fetchX((int)threadIdx.x);
     __syncthreads();
-    uint32_t cursor = 0;
     stamp(a, 0);
 
     const uint8_t *sh = a.shared;
-    const int tilesSGU = sh ? Fs >> 3 : 0;  // 8 gate + 8 up rows per tile, two K halves
+    const int tilesSGU = sh ? Fs >> 3 : 0;  // 8 gate + 8 up rows per tile, four K quarters
     const int tilesSD = sh ? D >> 4 : 0;    // 16 down rows per tile, three K parts
 
     // Requests of part `part` of `parts` (along K) of a gate/up tile: one box of eight row pieces per
     // matrix (`pitch` bytes per row in the slot: the box is as wide as the pitch, what it reads past
-    // the part is not used), then the eight rows' scales and biases of both matrices over the full K
-    // (contiguous runs).
+    // the part is not used); with the first part the eight rows' scales and biases of both matrices
+    // over the full K (contiguous runs) to `scales`.
     auto issue_gate_up = [&](const CUtensorMap *gateMap, const CUtensorMap *upMap, int expert, const uint8_t *blob,
-                             const FFExpertOffsets &off, int tile, int part, int parts, uint32_t pitch) {
+                             const FFExpertOffsets &off, int tile, int part, int parts, uint32_t pitch, uint32_t scales) {
         int gb, ge;
         part_range(groupsD, parts, part, gb, ge);
         const uint32_t sb = (uint32_t)groupsD * 16u;
-        if (lane == 0) bar_expect(myBar, (ge > gb ? 16u * pitch : 0u) + 4u * sb);
+        if (lane == 0) bar_expect(myBar, (ge > gb ? 16u * pitch : 0u) + (part == 0 ? 4u * sb : 0u));
         __syncwarp();
         if (lane < 2) {
-            if (ge > gb) box_copy(slotAddr + (uint32_t)lane * 8u * pitch, lane ? upMap : gateMap, gb * 4, tile * 8, expert, myBar);
-        } else if (lane >= 16 && lane < 20) {
+            if (ge > gb) box_copy(slot + (uint32_t)lane * 8u * pitch, lane ? upMap : gateMap, gb * 4, tile * 8, expert, myBar);
+        } else if (part == 0 && lane >= 16 && lane < 20) {
             const uint32_t which = (uint32_t)lane - 16u;
             const uint32_t src = which == 0 ? off.gateSOff : which == 1 ? off.gateBOff : which == 2 ? off.upSOff : off.upBOff;
-            bulk_copy(slotAddr + 16u * pitch + which * sb, blob + src + (size_t)tile * sb, sb, myBar);
+            bulk_copy(scales + which * sb, blob + src + (size_t)tile * sb, sb, myBar);
         }
     };
-    // Gate/up tile part -> this thread's partial sums of gate row tile*8+g and up row tile*8+g.
-    auto compute_gate_up = [&](int part, int parts, uint32_t pitch, const uint8_t *xp, const float *xs, float &gate, float &up) {
-        int gb, ge;
-        part_range(groupsD, parts, part, gb, ge);
-        const uint8_t *lo = mySlot + (size_t)g * pitch + 8 * t;
-        const uint8_t *hi = mySlot + (size_t)(g + 8) * pitch + 8 * t;
-        const uint16_t *sc = reinterpret_cast<const uint16_t *>(mySlot + 16u * pitch);
-        const uint16_t *gS = sc + g * groupsD, *gB = gS + 8 * groupsD, *uS = gB + 8 * groupsD, *uB = uS + 8 * groupsD;
-        gate = 0.0f;
-        up = 0.0f;
-        tile_rows(lo, hi, xp + gb * 128 + t * 32, gS + gb, gB + gb, uS + gb, uB + gb, xs + gb, ge - gb, false, gate, up);
+    // Two runs of eight rows (lanes t < 2 account for the first, t >= 2 for the second), scales as
+    // [scales | biases | scales | biases] runs of eight rows: the product over groups [gb, ge) with
+    // the inputs at `dig` / `aux` (already those of this lane's column and row).
+    auto two_runs = [&](uint32_t rows, uint32_t pitch, uint32_t scales, int groups, int gb, int ge, uint32_t dig, uint32_t aux) {
+        const uint32_t run = (uint32_t)groups * 16u;
+        const uint32_t s = scales + (t < 2 ? 0u : 2u * run) + (uint32_t)(g * groups + gb) * 2u;
+        return tile_int4(rows + (uint32_t)g * pitch + 8u * t, rows + (uint32_t)(g + 8) * pitch + 8u * t,
+                         dig + (uint32_t)gb * kDigitGroupBytes + (uint32_t)(g & 3) * 64u + (uint32_t)t * 16u, s, s + run,
+                         aux + 8u * (uint32_t)gb, ge - gb);
     };
     auto issue_shared_down = [&](int tile, int part) {
         int gb, ge;
         part_range(groupsFs, 3, part, gb, ge);
         const uint32_t sb = (uint32_t)groupsFs * 32u;
-        if (lane == 0) bar_expect(myBar, (ge > gb ? 16u * a.strideSD : 0u) + 2u * sb);
+        if (lane == 0) bar_expect(myBar, (ge > gb ? 16u * a.strideSD : 0u) + (part == 0 ? 2u * sb : 0u));
         __syncwarp();
         if (lane == 0) {
-            if (ge > gb) box_copy(slotAddr, &maps.m[kMapSharedDown], gb * 4, tile * 16, 0, myBar);
-        } else if (lane >= 16 && lane < 18) {
+            if (ge > gb) box_copy(slot, &maps.m[kMapSharedDown], gb * 4, tile * 16, 0, myBar);
+        } else if (part == 0 && lane >= 16 && lane < 18) {
             const uint32_t which = (uint32_t)lane - 16u;
-            bulk_copy(slotAddr + 16u * a.strideSD + which * sb,
+            bulk_copy(tripleBase + 48u * a.strideSD + which * sb,
                       sh + (which ? a.sharedOff.downBOff : a.sharedOff.downSOff) + (size_t)tile * sb, sb, myBar);
         }
+    };
+    // A warp's copies and, for the scales, those of the first warp of its pair, quad or triple.  (All
+    // warps of a group take the same number of tiles, so one parity serves both barriers.)
+    auto wait_tile = [&](int first) {
+        if (warp != first) {
+            uint32_t p = parity;
+            slot_wait(barOf(first), p, a.errorFlag);
+        }
+        slot_wait(myBar, parity, a.errorFlag);
     };
 
     // ---------------- phase A: router logits, shared gate/up/GeGLU ----------------
     // The router rows are requested first, alone: top-8 heads the critical path, and the copy
     // engine serves an SM's requests in order.
-    int eA = (!a.idsIn && K > 0 && warp >= kSharedGuWarps && warp < kBigWarps) ? (warp - kSharedGuWarps) * G + cta
-                                                                             : 0x7FFFFFFF;
-    if (eA < E) {
+    const int rw = warp - kSharedGuWarps;  // router warps 8, 9
+    int eA = (!a.idsIn && K > 0 && rw >= 0 && rw < kRouterWarps) ? rw * G + cta : 0x7FFFFFFF;
+    const uint32_t routerBar = barOf(kFusedWarps + (rw >= 0 && rw < kRouterWarps ? rw : 0));
+    uint32_t routerParity = 0;
+    auto issue_router = [&](int e) {
         // the router's per-column scales (the same for every expert) come along behind the row
         if (lane == 0) {
-            bar_expect(myBar, (uint32_t)D * (a.routerScale ? 4u : 2u));
-            bulk_copy(slotAddr, a.routerW + (size_t)eA * D, (uint32_t)D * 2u, myBar);
-            if (a.routerScale) bulk_copy(slotAddr + (uint32_t)D * 2u, a.routerScale, (uint32_t)D * 2u, myBar);
+            bar_expect(routerBar, (uint32_t)D * (a.routerScale ? 4u : 2u));
+            bulk_copy(slot, a.routerW + (size_t)e * D, (uint32_t)D * 2u, routerBar);
+            if (a.routerScale) bulk_copy(slot + (uint32_t)D * 2u, a.routerScale, (uint32_t)D * 2u, routerBar);
         }
         __syncwarp();
-    }
+    };
+    if (eA < E) issue_router(eA);
     __syncthreads();
     // shared gate/up tiles: four warps per tile (K quarters), two tiles per CTA and round
     const int partA = warp & 3;
     int tA = warp < kSharedGuWarps ? (warp >> 2) * G + cta : 0x7FFFFFFF;
-    if (tA < tilesSGU)
-        issue_gate_up(&maps.m[kMapSharedGate], &maps.m[kMapSharedUp], 0, sh, a.sharedOff, tA, partA, 4, a.strideGUA);
-    const int triple = warp >= kBigWarps ? (warp - kBigWarps) / 3 : 0;
-    const int part3 = warp >= kBigWarps ? (warp - kBigWarps) % 3 : 0;
+    auto issue_shared_gate_up = [&](int tile) {
+        issue_gate_up(&maps.m[kMapSharedGate], &maps.m[kMapSharedUp], 0, sh, a.sharedOff, tile, partA, 4, a.strideGUA,
+                      scalesOfPair((warp & ~3) >> 1));
+    };
+    if (tA < tilesSGU) issue_shared_gate_up(tA);
     int tSD = warp >= kBigWarps ? triple * G + cta : 0x7FFFFFFF;
     if (tSD < tilesSD) issue_shared_down(tSD, part3);
     warp_stamp(a, 0, 0);
@@ -403,314 +413,203 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
         sTarget = gen1 * gridDim.x;
         sTag = (uint32_t)(gen1 % 0xFFFFFFFFull) + 1u;  // 1 .. 2^32-1: never 0, consecutive launches differ
     }
-    stage_input(xSrc, 1, D, xPerm, 0, xSum, xPlain, &xMine);  // ends with a CTA barrier: target and tag are published
+    // the input row, as digits and (for the router) as it is
+    stage_digits(D >> 3, (int)threadIdx.x, kFusedThreads, smemRaw, xAux, [&](int i) {
+        const uint4 v = i == (int)threadIdx.x ? xMine : fetchX(i);
+        reinterpret_cast<uint4 *>(region)[i] = v;
+        return v;
+    });
+    __syncthreads();  // target and tag are published, too
     const uint32_t tag = sTag;
     for (; tA < tilesSGU; tA += (kSharedGuWarps / 4) * G) {
-        slot_wait(myBar, parity, a.errorFlag);
+        wait_tile(warp & ~3);
         warp_stamp(a, 0, 1);
-        float gate, up;
-        compute_gate_up(partA, 4, a.strideGUA, xPerm, xSum, gate, up);
-        slot_release();
-        const int next = tA + (kSharedGuWarps / 4) * G;
-        if (next < tilesSGU)
-            issue_gate_up(&maps.m[kMapSharedGate], &maps.m[kMapSharedUp], 0, sh, a.sharedOff, next, partA, 4, a.strideGUA);
+        int gb, ge;
+        part_range(groupsD, 4, partA, gb, ge);
+        const float v = two_runs(slot, a.strideGUA, scalesOfPair((warp & ~3) >> 1), groupsD, gb, ge, smem, sm_addr(xAux));
         float *mine = partial + warp * 16;
-        if (partA && t == 0) {
-            mine[g] = gate;
-            mine[8 + g] = up;
-        }
-        named_barrier(1 + (warp >> 2), 128);
-        if (!partA && t == 0) {
-            gate = ((gate + mine[16 + g]) + mine[32 + g]) + mine[48 + g];
-            up = ((up + mine[16 + 8 + g]) + mine[32 + 8 + g]) + mine[48 + 8 + g];
-            a.sharedActs[tA * 8 + g] = f2bf(gelu_tanh(bf16_round(gate)) * bf16_round(up));
+        if (partA && !(t & 1)) mine[(t >> 1) * 8 + g] = v;
+        named_barrier(1 + (warp >> 2), 128);  // every part is read, too: the slots are free
+        const int next = tA + (kSharedGuWarps / 4) * G;
+        if (next < tilesSGU) issue_shared_gate_up(next);
+        if (!partA) {
+            const float *m = mine + (t >> 1) * 8 + g;
+            const float sum = ((v + m[16]) + m[32]) + m[48];
+            const float up = __shfl_down_sync(0xFFFFFFFFu, sum, 2);
+            if (t == 0) a.sharedActs[tA * 8 + g] = f2bf(gelu_tanh(bf16_round(sum)) * bf16_round(up));
         }
         named_barrier(1 + (warp >> 2), 128);
     }
-    // eight products of one run: the row's weights and, behind them in the slot, the router's
-    // per-column scales (if any); staged input at `base`
-    auto router_run = [&](const uint16_t *wr, int base, float acc) {
-        const uint4 wv = *reinterpret_cast<const uint4 *>(wr + base);
-        // the staged run holds elements 0,4,1,5,2,6,3,7: low halves are 0..3, high halves 4..7
-        const uint4 xv = *reinterpret_cast<const uint4 *>(xPerm + base * 2);
-        float xe[8] = {__uint_as_float(xv.x << 16),         __uint_as_float(xv.y << 16),
-                       __uint_as_float(xv.z << 16),         __uint_as_float(xv.w << 16),
-                       __uint_as_float(xv.x & 0xFFFF0000u), __uint_as_float(xv.y & 0xFFFF0000u),
-                       __uint_as_float(xv.z & 0xFFFF0000u), __uint_as_float(xv.w & 0xFFFF0000u)};
-        if (a.routerScale) {
-            const uint4 sv = *reinterpret_cast<const uint4 *>(wr + D + base);
+    for (; eA < E; eA += kRouterWarps * G) {
+        slot_wait(routerBar, routerParity, a.errorFlag);
+        warp_stamp(a, 0, 1);
+        // lane l chains fmaf over elements [256 i + 8 l, +8): the order of every router kernel
+        float acc = 0.0f;
+#pragma unroll 4
+        for (int c = lane; c < (D >> 3); c += 32) {
+            const uint4 wv = lds128(slot + 16u * (uint32_t)c), xv = lds128(sm_addr(region) + 16u * (uint32_t)c);
+            const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w}, xx[4] = {xv.x, xv.y, xv.z, xv.w};
+            uint4 sv = make_uint4(0, 0, 0, 0);
+            if (a.routerScale) sv = lds128(slot + (uint32_t)D * 2u + 16u * (uint32_t)c);
             const uint32_t ss[4] = {sv.x, sv.y, sv.z, sv.w};
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                xe[2 * k] = xe[2 * k] * __uint_as_float(ss[k] << 16);
-                xe[2 * k + 1] = xe[2 * k + 1] * __uint_as_float(ss[k] & 0xFFFF0000u);
+                float x0 = __uint_as_float(xx[k] << 16), x1 = __uint_as_float(xx[k] & 0xFFFF0000u);
+                if (a.routerScale) {
+                    x0 = x0 * __uint_as_float(ss[k] << 16);
+                    x1 = x1 * __uint_as_float(ss[k] & 0xFFFF0000u);
+                }
+                acc = fmaf(__uint_as_float(ww[k] << 16), x0, acc);
+                acc = fmaf(__uint_as_float(ww[k] & 0xFFFF0000u), x1, acc);
             }
         }
-        const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            acc = fmaf(__uint_as_float(ww[k] << 16), xe[2 * k], acc);
-            acc = fmaf(__uint_as_float(ww[k] & 0xFFFF0000u), xe[2 * k + 1], acc);
-        }
-        return acc;
-    };
-    for (; eA < E; eA += (kBigWarps - kSharedGuWarps) * G) {
-        slot_wait(myBar, parity, a.errorFlag);
-        warp_stamp(a, 0, 1);
-        const uint16_t *wr = reinterpret_cast<const uint16_t *>(mySlot);
-        float acc = 0.0f;
-        for (int base = 8 * lane; base < D; base += 256) acc = router_run(wr, base, acc);
 #pragma unroll
         for (int offset = 16; offset >= 1; offset >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, offset);
-        if (lane == 0) {
-            const float logit = a.logitBias ? acc + a.logitBias[eA] : acc;
-            a.logits[eA] = logit;
-            // value and validity in one 64-bit store: the readers poll these words
-            st_tagged(a.taggedLogits + eA, tag, __float_as_uint(logit));
-        }
+        // value and validity in one 64-bit store: the readers poll these words
+        if (lane == 0) st_tagged(a.taggedLogits + eA, tag, __float_as_uint(a.logitBias ? acc + a.logitBias[eA] : acc));
         slot_release();
-        const int next = eA + (kBigWarps - kSharedGuWarps) * G;
-        if (next < E && lane == 0) {
-            bar_expect(myBar, (uint32_t)D * (a.routerScale ? 4u : 2u));
-            bulk_copy(slotAddr, a.routerW + (size_t)next * D, (uint32_t)D * 2u, myBar);
-            if (a.routerScale) bulk_copy(slotAddr + (uint32_t)D * 2u, a.routerScale, (uint32_t)D * 2u, myBar);
-        }
-        __syncwarp();
+        const int next = eA + kRouterWarps * G;
+        if (next < E) issue_router(next);
     }
     warp_stamp(a, 0, 2);
     stamp(a, 1);
 
-    // ---------------- top-8 by warps 8..15 while warps 0..7 finish the shared gate/up rows ----------
-    // Each logit travels as one 64-bit word (validity | value) that the readers poll, so ranking
-    // waits neither for a counter round trip nor for the other CTAs' shared rows.
-    if (K > 0 && !a.idsIn && warp >= kSharedGuWarps) {
-        constexpr int kTopkThreads = (kFusedWarps - kSharedGuWarps) * 32;
-        const int tid2 = (int)threadIdx.x - kSharedGuWarps * 32;
-        // one warp fetches the logits, polling the tagged words (four per lane, coalesced) until
-        // every writer's store has shown up
-        if (warp == kSharedGuWarps) {
-            for (int base = 0; base < E; base += 128) {
-                const int e0 = base + 4 * lane;
-                const unsigned long long filler = (unsigned long long)tag << 32;
-                unsigned long long w[4] = {filler, filler, filler, filler};
-                bool ready = false;
-                for (uint32_t spins = 0; spins < kBarrierSpinLimit && !ready; ++spins) {
-                    if (e0 + 3 < E) {
-                        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w[0]), "=l"(w[1]) : "l"(a.taggedLogits + e0) : "memory");
-                        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w[2]), "=l"(w[3]) : "l"(a.taggedLogits + e0 + 2) : "memory");
-                    } else {
-                        for (int i = 0; i < 4; ++i)
-                            if (e0 + i < E)
-                                asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w[i]) : "l"(a.taggedLogits + e0 + i) : "memory");
-                    }
-                    const bool mine = (uint32_t)(w[0] >> 32) == tag && (uint32_t)(w[1] >> 32) == tag &&
-                                      (uint32_t)(w[2] >> 32) == tag && (uint32_t)(w[3] >> 32) == tag;
-                    ready = __all_sync(0xFFFFFFFFu, mine);
-                }
-                if (!ready && lane == 0) atomicExch(a.errorFlag, 9u);
-                for (int i = 0; i < 4; ++i)
-                    if (e0 + i < E) sLogits[e0 + i] = __uint_as_float((uint32_t)w[i]);
-            }
-        }
-        const int rankSpan = (((E + 1) >> 1) + 3) & ~3;
-        if (tid2 < 8) {
-            sIds[tid2] = 0u;
-            sScore[tid2] = -INFINITY;
-        } else if (tid2 >= 32 && tid2 < 40 && E + tid2 - 32 < 2 * rankSpan) {
-            sLogits[E + tid2 - 32] = -INFINITY;
-        }
-        named_barrier(8, kTopkThreads);
-        // rank of every logit under (higher score, then lower expert id); scores of -inf or NaN
-        // are never taken — the order of the serial top-8 (moe.metal:269-303).  Two threads per
-        // expert, each counting the competitors of one span (a multiple of four, read as float4).
-        {
-            for (int idx = tid2; idx < 2 * ((E + 127) & ~127); idx += kTopkThreads) {
-                const int e = idx >> 1, half = idx & 1;
-                const float v = e < E ? sLogits[e] : -INFINITY;
-                const int begin = half * rankSpan;
-                int rank = 0;
-#pragma unroll 4
-                for (int o = begin; o < begin + rankSpan; o += 4) {
-                    const float4 c = *reinterpret_cast<const float4 *>(sLogits + o);
-                    // a competitor wins with a higher score, or the same score and a lower id
-                    rank += (c.x > v || (c.x == v && o < e)) ? 1 : 0;
-                    rank += (c.y > v || (c.y == v && o + 1 < e)) ? 1 : 0;
-                    rank += (c.z > v || (c.z == v && o + 2 < e)) ? 1 : 0;
-                    rank += (c.w > v || (c.w == v && o + 3 < e)) ? 1 : 0;
-                }
-                rank += __shfl_xor_sync(0xFFFFFFFFu, rank, 1);
-                if (half == 0 && v > -INFINITY && rank < K) {
-                    sIds[rank] = (uint32_t)e;
-                    sScore[rank] = v;
-                }
-            }
-        }
-        named_barrier(8, kTopkThreads);
-        if (warp == kSharedGuWarps) {
-            // softmax over the chosen scores: exponentials in parallel, the sum in rank order
-            const float score = lane < K ? sScore[lane] : -INFINITY;
-            const float top = __shfl_sync(0xFFFFFFFFu, score, 0);
-            const float ex = lane < K ? expf(score - top) : 0.0f;
-            float sum = 0.0f;
-            for (int r = 0; r < K; ++r) sum += __shfl_sync(0xFFFFFFFFu, ex, r);
-            if (lane < K) {
-                float w = ex / sum;
-                if (a.gain) w = w * bf2f(a.gain[sIds[lane]]);
-                const uint16_t wb = f2bf(w);
-                sWeights[lane] = bf2f(wb);
-                if (blockIdx.x == 0) {
-                    a.ids[lane] = sIds[lane];
-                    a.weights[lane] = wb;
-                }
-            }
-        }
-    } else {
+    // ---------------- top-8 by warp 8 while warps 0..7 finish the shared gate/up rows ----------------
+    uint32_t myId = 0u;
+    float myScore = -INFINITY;
+    const bool ranking = K > 0 && !a.idsIn && warp == kSharedGuWarps;
+    if (ranking) {
+        poll_and_rank(a, tag, lane, myId, myScore);
+        if (lane < K) sIds[lane] = myId;
+    } else if (K > 0 && a.idsIn && (int)threadIdx.x < K) {
         // Given routes.  A route past the resident experts would address memory outside the layer:
         // it is replaced by expert 0 with weight 0 and reported through the error flag (the
         // reference refuses such a route with "route expert N is out of range").
-        if (K > 0 && a.idsIn && threadIdx.x < K) {
-            uint32_t id = a.idsIn[threadIdx.x];
-            float w = bf2f(a.weightsIn[threadIdx.x]);
-            if (id >= (uint32_t)a.expertCount) {
-                atomicExch(a.errorFlag, 12u);
-                id = 0u;
-                w = 0.0f;
-            }
-            sIds[threadIdx.x] = id;
-            sWeights[threadIdx.x] = w;
+        uint32_t id = a.idsIn[threadIdx.x];
+        float w = bf2f(a.weightsIn[threadIdx.x]);
+        if (id >= (uint32_t)a.expertCount) {
+            atomicExch(a.errorFlag, 12u);
+            id = 0u;
+            w = 0.0f;
         }
+        sIds[threadIdx.x] = id;
+        sWeights[threadIdx.x] = w;
     }
-    // barrier 1 covers the shared activations; the routed rows are requested between arriving
-    // and waiting (the CTA barrier also publishes the routes to all warps)
+    // the arrival covers the shared activations, the CTA barrier also publishes the routes
     __syncthreads();
     if (is_barrier_thread()) counter_arrive(a.barrier + kCountShared);
     stamp(a, 2);
     stamp(a, 3);
     const int tilesF = F >> 3;
     const int tilesRouted = K * tilesF;
-    int tB = warp < kBigWarps ? (warp >> 1) * G + cta : 0x7FFFFFFF;
-    if (tB < tilesRouted) {
-        const int slot = tB / tilesF;
-        issue_gate_up(&maps.m[kMapRoutedGate], &maps.m[kMapRoutedUp], (int)sIds[slot],
-                      a.experts + (size_t)sIds[slot] * a.stride, a.off, tB - slot * tilesF, warp & 1, 2, a.strideGU);
-    }
+    int tB = warp < kBigWarps ? pair * G + cta : 0x7FFFFFFF;
+    auto issue_routed_gate_up = [&](int tile) {
+        const int k = tile / tilesF;
+        issue_gate_up(&maps.m[kMapRoutedGate], &maps.m[kMapRoutedUp], (int)sIds[k], a.experts + (size_t)sIds[k] * a.stride, a.off,
+                      tile - k * tilesF, warp & 1, 2, a.strideGU, scalesOfPair(pair));
+    };
+    if (tB < tilesRouted) issue_routed_gate_up(tB);
     warp_stamp(a, 1, 0);
-    // Routed down tile: output rows 2*tile, 2*tile+1 of all eight experts.  Tile row rho*8 + e is
-    // row 2*tile+rho of expert e; lane l copies row piece l (l < 16), or the 16-byte aligned window
-    // around the two rows' scales (l even) or biases (l odd) of expert (l-16)/2.
-    // Tiles go to the warps in the order 10..15, 0..9: the warps of the shared down rows are done
-    // early in phase B and request their routed down tile then, into their own slot, so that it is
-    // in shared memory when the second grid barrier opens; warps 0..9 request theirs at the barrier.
-    const int tilesRD = D >> 1;
-    const int orderC = warp >= kBigWarps ? warp - kBigWarps : warp + (kFusedWarps - kBigWarps);
+    if (ranking) {
+        // softmax over the chosen scores: exponentials in parallel, the sum in rank order
+        const float top = __shfl_sync(0xFFFFFFFFu, myScore, 0);
+        const float ex = lane < K ? expf(myScore - top) : 0.0f;
+        float sum = 0.0f;
+        for (int r = 0; r < K; ++r) sum += __shfl_sync(0xFFFFFFFFu, ex, r);
+        if (lane < K) {
+            float w = ex / sum;
+            if (a.gain) w = w * bf2f(a.gain[myId]);
+            const uint16_t wb = f2bf(w);
+            sWeights[lane] = bf2f(wb);  // read in phase C
+            if (blockIdx.x == 0) {
+                a.ids[lane] = myId;
+                a.weights[lane] = wb;
+            }
+        }
+    }
+
+    // ---------------- phase B: routed gate/up/GeGLU (warps 0..9), shared down rows (10..15) ----------
+    // Routed down task j of a round (16 / pairsK row tiles of eight rows, pairsK expert pairs each), tasks
+    // in the order of warps 10..15, 0..9: the shared down warps are done first.  Lanes 0, 1 copy the two
+    // experts' rows (one box each), lanes 16..19 their scale and bias runs.
+    const int tilesRD = D >> 3, pairsK = (K + 1) >> 1, perRound = pairsK ? kFusedWarps / pairsK : 1;
+    const int task = warp >= kBigWarps ? warp - kBigWarps : warp + (kFusedWarps - kBigWarps);
+    const int myTile = pairsK ? task / pairsK : 0, myPair = pairsK ? task - myTile * pairsK : 0;
+    const int eLo = 2 * myPair, eHi = min(2 * myPair + 1, K - 1);
+    auto tileOf = [&](int round) { return cta + G * (round * perRound + myTile); };
+    auto has_task = [&](int round) { return K > 0 && myTile < perRound && tileOf(round) < tilesRD; };
     auto issue_routed_down = [&](int tile) {
-        const uint32_t piece = (uint32_t)groupsF * 32u;
-        if (lane == 0) bar_expect(myBar, 16u * piece + 16u * a.winBytes);
+        const uint32_t sb = (uint32_t)groupsF * 16u;
+        if (lane == 0) bar_expect(myBar, 16u * a.strideRD + 4u * sb);
         __syncwarp();
-        const int e = lane < 16 ? (lane & 7) : ((lane - 16) >> 1);
-        const uint8_t *blob = a.experts + (size_t)sIds[e < K ? e : 0] * a.stride;
-        if (lane < 16) {
-            const int row = tile * 2 + (lane >> 3);
-            bulk_copy(slotAddr + (uint32_t)lane * a.strideRD, blob + a.off.downWOff + (size_t)row * (F >> 1), piece, myBar);
-        } else {
-            const uint32_t srcOff = ((lane & 1) ? a.off.downBOff : a.off.downSOff) + (uint32_t)tile * 4u * (uint32_t)groupsF;
-            // windows: scales of expert e at e * winPitch, biases at (8 + e) * winPitch
-            bulk_copy(slotAddr + 16u * a.strideRD + (uint32_t)(((lane & 1) << 3) + e) * a.winPitch, blob + (srcOff & ~15u),
-                      a.winBytes, myBar);
+        if (lane < 2) {
+            box_copy(downSlot + (uint32_t)lane * 8u * a.strideRD, &maps.m[kMapRoutedDown], 0, tile * 8, (int)sIds[lane ? eHi : eLo], myBar);
+        } else if (lane >= 16 && lane < 20) {
+            const uint32_t which = (uint32_t)lane - 16u;
+            const uint8_t *blob = a.experts + (size_t)sIds[which < 2 ? eLo : eHi] * a.stride;
+            bulk_copy(downSlot + 16u * a.strideRD + which * sb, blob + ((which & 1) ? a.off.downBOff : a.off.downSOff) + (size_t)tile * sb,
+                      sb, myBar);
         }
     };
-    uint8_t *saPerm = region;
-    float *saSum = reinterpret_cast<float *>(region + Fs * 2);
-    if (sh) {
+    if (warp >= kBigWarps && sh) {
+        // the shared activations, staged by the six warps that use them
         if (is_barrier_thread()) counter_wait(a.barrier + kCountShared, sTarget, a.errorFlag);
-        __syncthreads();
-        stage_input(a.sharedActs, 1, Fs, saPerm, 0, saSum);
+        named_barrier(8, (kFusedWarps - kBigWarps) * 32);
+        stage_digits(Fs >> 3, (int)threadIdx.x - kBigWarps * 32, (kFusedWarps - kBigWarps) * 32, region, regionAux,
+                     [&](int i) { return __ldcg(reinterpret_cast<const uint4 *>(a.sharedActs) + i); });
+        named_barrier(8, (kFusedWarps - kBigWarps) * 32);
     }
-    bool downAsked = !(a.prefetch & 1) || warp >= K;
     for (; tB < tilesRouted; tB += (kBigWarps / 2) * G) {
-        slot_wait(myBar, parity, a.errorFlag);
+        wait_tile(warp & ~1);
         warp_stamp(a, 1, 1);
-        if (!downAsked) {
-            // The down projections of the chosen experts go to L2 for phase C: warp k asks for
-            // expert k's once its own rows are there.  Earlier, the prefetch shares HBM with the
-            // gate/up rows that the arithmetic is waiting for; from here on it runs under the
-            // arithmetic.
-            for (int k = 0; k < K; ++k) {
-                const uint8_t *blob = a.experts + (size_t)sIds[k] * a.stride;
-                prefetch_region(blob + a.off.downWOff,
-                                (uint64_t)a.off.downBOff - a.off.downWOff + (uint64_t)D * F / kGroup * 2, cursor, lane, 32,
-                                k == warp);
-            }
-            downAsked = true;
-        }
-        float gate, up;
-        compute_gate_up(warp & 1, 2, a.strideGU, xPerm, xSum, gate, up);
-        slot_release();
-        const int next = tB + (kBigWarps / 2) * G;
-        if (next < tilesRouted) {
-            const int slot = next / tilesF;
-            issue_gate_up(&maps.m[kMapRoutedGate], &maps.m[kMapRoutedUp], (int)sIds[slot],
-                          a.experts + (size_t)sIds[slot] * a.stride, a.off, next - slot * tilesF, warp & 1, 2, a.strideGU);
-        }
+        int gb, ge;
+        part_range(groupsD, 2, warp & 1, gb, ge);
+        const float v = two_runs(slot, a.strideGU, scalesOfPair(pair), groupsD, gb, ge, smem, sm_addr(xAux));
         float *mine = partial + warp * 16;
-        if ((warp & 1) && t == 0) {
-            mine[g] = gate;
-            mine[8 + g] = up;
-        }
-        named_barrier(1 + (warp >> 1), 64);
+        if ((warp & 1) && !(t & 1)) mine[(t >> 1) * 8 + g] = v;
+        named_barrier(1 + pair, 64);
+        const int next = tB + (kBigWarps / 2) * G;
+        if (next < tilesRouted) issue_routed_gate_up(next);
         if (!(warp & 1)) {
             // the tile's eight activations are one run of the staged row: four tagged words,
             // written by the lanes t == 0 of even g (the odd neighbour's value comes by shuffle)
-            gate += mine[16 + g];
-            up += mine[16 + 8 + g];
-            const uint32_t act = f2bf(gelu_tanh(gate) * up);
+            const float sum = v + mine[16 + (t >> 1) * 8 + g];
+            const float up = __shfl_down_sync(0xFFFFFFFFu, sum, 2);
+            const uint32_t act = f2bf(gelu_tanh(sum) * up);
             const uint32_t two = act | (__shfl_down_sync(0xFFFFFFFFu, act, 4) << 16);
             if (t == 0 && !(g & 1)) st_tagged(a.taggedActs + ((tB * 8 + g) >> 1), tag, two);
         }
-        named_barrier(1 + (warp >> 1), 64);
+        named_barrier(1 + pair, 64);
     }
     for (; tSD < tilesSD; tSD += 2 * G) {
-        slot_wait(myBar, parity, a.errorFlag);
+        wait_tile(kBigWarps + 3 * triple);
         warp_stamp(a, 1, 1);
         int gb, ge;
         part_range(groupsFs, 3, part3, gb, ge);
-        const uint8_t *lo = mySlot + (size_t)g * a.strideSD + 8 * t;
-        const uint8_t *hi = mySlot + (size_t)(g + 8) * a.strideSD + 8 * t;
-        const uint16_t *sS = reinterpret_cast<const uint16_t *>(mySlot + 16u * a.strideSD);
-        const uint16_t *sB = sS + 16 * groupsFs;
-        float v0, v1;
-        tile_rows(lo, hi, saPerm + gb * 128 + t * 32, sS + g * groupsFs + gb, sB + g * groupsFs + gb,
-                  sS + (g + 8) * groupsFs + gb, sB + (g + 8) * groupsFs + gb, saSum + gb, ge - gb, false, v0, v1);
-        slot_release();
+        const uint32_t s = tripleBase + 48u * a.strideSD + (uint32_t)((t < 2 ? g : g + 8) * groupsFs + gb) * 2u;
+        const float v = tile_int4(slot + (uint32_t)g * a.strideSD + 8u * t, slot + (uint32_t)(g + 8) * a.strideSD + 8u * t,
+                                  sm_addr(region) + (uint32_t)gb * kDigitGroupBytes + (uint32_t)(g & 3) * 64u + (uint32_t)t * 16u, s,
+                                  s + (uint32_t)groupsFs * 32u, sm_addr(regionAux) + 8u * (uint32_t)gb, ge - gb);
+        float *mine = partial + warp * 16;
+        if (part3 && !(t & 1)) mine[(t >> 1) * 8 + g] = v;
+        named_barrier(6 + triple, 96);
         const int next = tSD + 2 * G;
         if (next < tilesSD) issue_shared_down(next, part3);
-        float *mine = partial + warp * 16;
-        if (part3 && t == 0) {
-            mine[g] = v0;
-            mine[8 + g] = v1;
-        }
-        named_barrier(6 + triple, 96);
         if (!part3) {
-            v0 = (v0 + mine[16 + g]) + mine[32 + g];
-            v1 = (v1 + mine[16 + 8 + g]) + mine[32 + 8 + g];
-            const uint32_t r0 = f2bf(v0), r1 = f2bf(v1);
+            const float *m = mine + (t >> 1) * 8 + g;
+            const uint32_t r = f2bf((v + m[16]) + m[32]);  // row 8 (t / 2) + g, valid in even t
+            const int row = tSD * 16 + (t >> 1) * 8 + g;
             if (K > 0) {
                 // read as the residual of the routed rows in phase C: tagged words of two rows
-                const uint32_t two0 = r0 | (__shfl_down_sync(0xFFFFFFFFu, r0, 4) << 16);
-                const uint32_t two1 = r1 | (__shfl_down_sync(0xFFFFFFFFu, r1, 4) << 16);
-                if (t == 0 && !(g & 1)) {
-                    st_tagged(a.taggedH1 + ((tSD * 16 + g) >> 1), tag, two0);
-                    st_tagged(a.taggedH1 + ((tSD * 16 + 8 + g) >> 1), tag, two1);
-                }
-            } else if (t == 0) {
-                a.y[tSD * 16 + g] = (uint16_t)r0;
-                a.y[tSD * 16 + 8 + g] = (uint16_t)r1;
+                const uint32_t two = r | (__shfl_down_sync(0xFFFFFFFFu, r, 4) << 16);
+                if (!(t & 1) && !(g & 1)) st_tagged(a.taggedH1 + (row >> 1), tag, two);
+            } else if (!(t & 1)) {
+                a.y[row] = (uint16_t)r;
             }
         }
         named_barrier(6 + triple, 96);
     }
-    int tC = orderC * G + cta;
-    if (K > 0 && warp >= kBigWarps && tC < tilesRD) issue_routed_down(tC);
+    if (has_task(0)) issue_routed_down(tileOf(0));
     warp_stamp(a, 1, 2);
     stamp(a, 4);
     if (K == 0) {
@@ -721,71 +620,53 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
 
     // No grid barrier before phase C: the routed activations and the shared output rows are polled
     // as tagged words while they are staged.
-    if (warp < kBigWarps && tC < tilesRD) issue_routed_down(tC);
     warp_stamp(a, 2, 0);
     __syncthreads();  // the region still holds the shared activations that phase B's warps read
     stamp(a, 5);
 
     // ---------------- phase C: routed down rows and the combine ----------------
-    {
-        // activations of slot e: run-permuted bf16 at region + e * actStride, group sums behind them
-        float *actSum = reinterpret_cast<float *>(region + 8 * a.actStride);
-        if (K < 8) {
-            for (int e = K; e < 8; ++e) {
-                for (int i = threadIdx.x; i < (F >> 3); i += blockDim.x)
-                    reinterpret_cast<uint4 *>(region + (size_t)e * a.actStride)[i] = make_uint4(0, 0, 0, 0);
-                for (int i = threadIdx.x; i < groupsF; i += blockDim.x) actSum[e * groupsF + i] = 0.0f;
-            }
+    stage_digits(K * (F >> 3), (int)threadIdx.x, kFusedThreads, region, regionAux,
+                 [&](int i) { return fetch_tagged(a.taggedActs + 4 * (size_t)i, tag, a.errorFlag); });
+    __syncthreads();
+    for (int round = 0; cta + G * round * perRound < tilesRD; ++round) {
+        // warp w combines the round's row tile w, lane r its row r; its residual is asked for first
+        const int myRowTile = cta + G * (round * perRound + warp);
+        const bool combines = warp < perRound && myRowTile < tilesRD && lane < 8;
+        const int row = myRowTile * 8 + lane;
+        unsigned long long resWord = 0;
+        float acc = 0.0f;
+        if (combines) {
+            if (a.shared) resWord = ld_tagged(a.taggedH1 + (row >> 1));
+            else if (a.residual) acc = bf2f(__ldcg(a.residual + row));
         }
-        stage_tagged(a.taggedActs, tag, K, F, region, a.actStride, actSum, a.errorFlag);
-        for (; tC < tilesRD; tC += kFusedWarps * G) {
+        if (has_task(round)) {
             slot_wait(myBar, parity, a.errorFlag);
             warp_stamp(a, 2, 1);
-            // this thread: expert g, tile rows g (rho 0) and g+8 (rho 1); column g of the MMA is
-            // held by the lane with t == g/2 as d[g&1] (rho 0) and d[2 + (g&1)] (rho 1)
-            const uint8_t *lo = mySlot + (size_t)g * a.strideRD + 8 * t;
-            const uint8_t *hi = mySlot + (size_t)(g + 8) * a.strideRD + 8 * t;
-            const uint8_t *xe = region + (size_t)g * a.actStride + t * 32;
-            const uint32_t rowOff = (uint32_t)tC * 4u * (uint32_t)groupsF;
-            const uint8_t *win = mySlot + 16u * a.strideRD + (uint32_t)g * a.winPitch;
-            const uint16_t *sS = reinterpret_cast<const uint16_t *>(win + ((a.off.downSOff + rowOff) & 15u));
-            const uint16_t *sB = reinterpret_cast<const uint16_t *>(win + 8u * a.winPitch + ((a.off.downBOff + rowOff) & 15u));
-            const float *xs = actSum + g * groupsF;
-            const bool odd = g & 1;
-            const int row = tC * 2 + (lane & 1);
-            // the residual: rows 2*tile and 2*tile+1 of the shared output are one tagged word, asked
-            // for now and checked after the arithmetic; or the caller's residual row
-            unsigned long long resWord = 0;
-            if (a.shared && lane == 0) resWord = ld_tagged(a.taggedH1 + tC);
-            float acc = (!a.shared && a.residual && lane < 2) ? bf2f(__ldcg(a.residual + row)) : 0.0f;
-            float v0, v1;
-            tile_rows(lo, hi, xe, sS, sB, sS + groupsF, sB + groupsF, xs, groupsF, odd, v0, v1);
-            slot_release();
-            if (a.shared) {
-                if (lane == 0) {
-                    uint32_t spins = 0;
-                    while ((uint32_t)(resWord >> 32) != tag) {
-                        if (++spins > kBarrierSpinLimit) {
-                            atomicExch(a.errorFlag, 9u);
-                            break;
-                        }
-                        resWord = ld_tagged(a.taggedH1 + tC);
-                    }
-                }
-                const uint32_t two = __shfl_sync(0xFFFFFFFFu, (uint32_t)resWord, 0);
-                acc = bf2f((uint16_t)((lane & 1) ? two >> 16 : two & 0xFFFFu));
-            }
-            const int next = tC + kFusedWarps * G;
-            if (next < tilesRD) issue_routed_down(next);
-            // lane 0 combines row 2*tile, lane 1 row 2*tile+1, experts in rank order
-            for (int k = 0; k < K; ++k) {
-                const int src = 4 * k + (k >> 1);
-                const float e0 = __shfl_sync(0xFFFFFFFFu, v0, src);
-                const float e1 = __shfl_sync(0xFFFFFFFFu, v1, src);
-                acc = __fadd_rn(acc, __fmul_rn(sWeights[k], (lane & 1) ? e1 : e0));
-            }
-            if (lane < 2) a.y[row] = f2bf(acc);
+            // rows 0..7 of the tile: expert eLo, columns 0..3; rows 8..15: expert eHi, columns 4..7
+            const int mine = t < 2 ? eLo : eHi, column = g < 4 ? eLo : eHi;
+            const float v = two_runs(downSlot, a.strideRD, downSlot + 16u * a.strideRD, groupsF, 0, groupsF,
+                                     sm_addr(region) + (uint32_t)(column * groupsF) * kDigitGroupBytes,
+                                     sm_addr(regionAux) + 8u * (uint32_t)(mine * groupsF));
+            if (!(t & 1) && (t == 0 || eHi > eLo)) downRows[(myTile * 8 + mine) * 8 + g] = v;
         }
+        __syncthreads();
+        if (has_task(round + 1)) issue_routed_down(tileOf(round + 1));
+        if (combines) {
+            if (a.shared) {
+                uint32_t spins = 0;
+                while ((uint32_t)(resWord >> 32) != tag) {
+                    if (++spins > kBarrierSpinLimit) {
+                        atomicExch(a.errorFlag, 9u);
+                        break;
+                    }
+                    resWord = ld_tagged(a.taggedH1 + (row >> 1));
+                }
+                acc = bf2f((uint16_t)((lane & 1) ? (uint32_t)resWord >> 16 : (uint32_t)resWord & 0xFFFFu));
+            }
+            for (int k = 0; k < K; ++k) acc = __fadd_rn(acc, __fmul_rn(sWeights[k], downRows[(warp * 8 + k) * 8 + lane]));
+            a.y[row] = f2bf(acc);
+        }
+        __syncthreads();  // the rows are rewritten in the next round
     }
     warp_stamp(a, 2, 2);
     stamp(a, 6);
@@ -828,40 +709,32 @@ k_decode_fused_inline_x(const DecodeArgs a, const __grid_constant__ DecodeMaps m
 }
 
 struct FusedLayout {
-    uint32_t regionOffset, partialOffset, slotsOffset, bigBytes, smallBytes;
-    uint32_t strideGU, strideGUA, strideSD, strideRD, actStride, winBytes, winPitch;
+    uint32_t regionOffset, regionAux, partialOffset, downOffset, slotsOffset, rowsBytes, pairBytes, tripleBytes, downBytes;
+    uint32_t strideGU, strideGUA, strideSD, strideRD;
     size_t total;
 };
 
 static FusedLayout fused_layout(const FFConfig &c) {
-    const uint32_t D = c.d, F = c.f, Fs = c.sharedF;
+    const uint32_t D = c.d, F = c.f, Fs = c.sharedF, K = c.topK;
     const uint32_t groupsD = D / 64, groupsF = F / 64, groupsFs = Fs / 64;
+    auto up128 = [](uint32_t v) { return (v + 127u) & ~127u; };
     FusedLayout l{};
     l.strideGU = piece_stride(((groupsD + 1) / 2) * 32);   // routed tiles: K halves
     l.strideGUA = piece_stride(((groupsD + 3) / 4) * 32);  // shared tiles: K quarters
     l.strideSD = Fs ? piece_stride(((groupsFs + 2) / 3) * 32) : 32;
     l.strideRD = piece_stride(groupsF * 32);
-    l.winBytes = pad16u(4 * groupsF) + 16;
-    // window pitch: 80 modulo 128 puts the eight experts' windows on different banks
-    l.winPitch = l.winBytes;
-    while ((l.winPitch & 127u) != 80u) l.winPitch += 16u;
-    // per-expert activation stride: 16 modulo 128.  A quarter-warp's 128-bit load covers two
-    // experts, four lanes each reading 16 bytes at 32-byte steps; the second expert's chunks then
-    // fall into the gaps of the first.
-    l.actStride = F * 2;
-    while ((l.actStride & 127u) != 16u) l.actStride += 16u;
-    const uint32_t xPart = (D * 2 + groupsD * 4 + 127u) & ~127u;
-    const uint32_t sharedPart = Fs ? Fs * 2 + groupsFs * 4 : 0;
-    const uint32_t actsPart = 8 * l.actStride + 8 * groupsF * 4;
-    l.regionOffset = xPart;
-    l.partialOffset = (l.regionOffset + std::max(sharedPart, actsPart) + 127u) & ~127u;
-    l.slotsOffset = l.partialOffset + kFusedWarps * 16 * 4;
-    const uint32_t gateUp = 16 * l.strideGU + 4 * groupsD * 16;
-    const uint32_t down8 = 16 * l.strideRD + 16 * l.winPitch;
-    const uint32_t sharedDown = Fs ? 16 * l.strideSD + 2 * groupsFs * 32 : 0;
-    l.bigBytes = (std::max({gateUp, down8, D * 4}) + 127u) & ~127u;
-    l.smallBytes = (std::max({sharedDown, down8, 128u}) + 127u) & ~127u;
-    l.total = (size_t)l.slotsOffset + (size_t)kBigWarps * l.bigBytes + (size_t)(kFusedWarps - kBigWarps) * l.smallBytes;
+    l.regionOffset = up128(D * 4 + groupsD * (uint32_t)sizeof(GroupAux));
+    // the region holds x (bf16), then the shared activations' digits, then K (even) rows of routed ones
+    const uint32_t rows = (K + 1) / 2 * 2;
+    l.regionAux = l.regionOffset + std::max({D * 2, Fs * 4, rows * F * 4});
+    l.partialOffset = up128(l.regionAux + (uint32_t)sizeof(GroupAux) * std::max(groupsFs, rows * groupsF));
+    l.downOffset = l.partialOffset + kFusedWarps * 16 * 4;
+    l.slotsOffset = up128(l.downOffset + kFusedWarps * 8 * 8 * 4);
+    l.downBytes = up128(16 * l.strideRD + 4 * 16 * groupsF);
+    l.rowsBytes = up128(std::max({16 * l.strideGU, 16 * l.strideGUA, l.downBytes, D * 4}));
+    l.pairBytes = up128(2 * l.rowsBytes + 4 * 16 * groupsD);
+    l.tripleBytes = up128(std::max(Fs ? 48 * l.strideSD + 2 * 32 * groupsFs : 0u, 3 * l.downBytes));
+    l.total = (size_t)l.slotsOffset + (size_t)(kBigWarps / 2) * l.pairBytes + 2 * (size_t)l.tripleBytes;
     return l;
 }
 
@@ -902,24 +775,16 @@ bool launch_decode_fused(FFContext *ctx, const LayerStore &L, const uint16_t *x,
     a.residual = residual;
     a.idsIn = idsIn;
     a.weightsIn = weightsIn;
-    a.logits = ctx->logits;
     a.taggedLogits = ctx->taggedLogits;
     a.taggedActs = ctx->taggedActs;
     a.taggedH1 = ctx->taggedActs + (size_t)c.topK * c.f / 2;
     a.ids = ctx->ids;
     a.weights = ctx->weights;
-    a.acts = ctx->acts;
     a.sharedActs = ctx->sharedActs;
-    a.h1 = ctx->h1;
     a.y = y;
     a.barrier = reinterpret_cast<unsigned long long *>(ctx->gridBarrier);
     a.errorFlag = ctx->errorFlag;
     a.stamps = ctx->tracing ? ctx->phaseStamps : nullptr;
-    static const int prefetchMode = [] {
-        const char *env = getenv("FF_DECODE_PREFETCH");
-        return env ? atoi(env) : 0;  // off: measured slower than the early requests of phase C's tiles
-    }();
-    a.prefetch = prefetchMode;
     a.E = idsIn ? (int)L.expertCount : (int)L.routerExperts;
     a.expertCount = (int)L.expertCount;
     if (routed && !idsIn && L.routerExperts != L.expertCount)
@@ -950,6 +815,9 @@ bool launch_decode_fused(FFContext *ctx, const LayerStore &L, const uint16_t *x,
                 if (!make_row_box_map(&Lm.decodeMap[kMapRoutedGate + m], L.experts + o[3 * m], c.f, c.d / 2,
                                       L.expertCount, L.stride, lay.strideGU, 8, error))
                     return false;
+            if (!make_row_box_map(&Lm.decodeMap[kMapRoutedDown], L.experts + o[6], c.d, c.f / 2, L.expertCount, L.stride,
+                                  lay.strideRD, 8, error))
+                return false;
         }
         if (L.shared && c.sharedF) {
             const uint32_t *o = &L.sharedOff.gateWOff;
@@ -966,17 +834,18 @@ bool launch_decode_fused(FFContext *ctx, const LayerStore &L, const uint16_t *x,
     static thread_local DecodeMaps maps;
     memcpy(maps.m, L.decodeMap, sizeof(maps.m));
     a.regionOffset = lay.regionOffset;
+    a.regionAux = lay.regionAux;
     a.partialOffset = lay.partialOffset;
+    a.downOffset = lay.downOffset;
     a.slotsOffset = lay.slotsOffset;
-    a.bigBytes = lay.bigBytes;
-    a.smallBytes = lay.smallBytes;
+    a.rowsBytes = lay.rowsBytes;
+    a.pairBytes = lay.pairBytes;
+    a.tripleBytes = lay.tripleBytes;
+    a.downBytes = lay.downBytes;
     a.strideGU = lay.strideGU;
     a.strideGUA = lay.strideGUA;
     a.strideSD = lay.strideSD;
     a.strideRD = lay.strideRD;
-    a.actStride = lay.actStride;
-    a.winBytes = lay.winBytes;
-    a.winPitch = lay.winPitch;
     static KernelSmemMemo memo, memoInline;
     int perSm = 0;
     if (!memo.prepare(k_decode_fused, ctx->device, smem, kFusedThreads, &perSm, error)) return false;

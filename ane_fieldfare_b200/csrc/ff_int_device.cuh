@@ -1,0 +1,172 @@
+// Device helpers for packed INT4 (or INT8) rows against one input row on the integer tensor cores.
+//
+// mma.sync m16n8k32 u8 x s8 takes the codes as bytes, straight from memory: the low nibbles of a word
+// are one AND away, the high ones another (they stay in place and count 16 times, which the input
+// makes up for) — two integer instructions for eight codes, where bf16 operands cost eight.  The input
+// row enters as integers: per group of 64 values x = V 2^-E with |V| < 2^30, V written as four signed
+// base-256 digits, one digit per MMA column.  A bf16 value has eight significant bits, so a value down
+// to 2^-19 of its group's largest is exact, a smaller one is off by less than 2^-27 of it, below what a
+// 32-bit floating sum of the products would round; the integer sums themselves are exact.
+#pragma once
+
+#include "ff_mma_device.cuh"
+
+namespace ff {
+
+constexpr uint32_t kDigitGroupBytes = 256;  // four digits of 64 values
+
+__device__ __forceinline__ void mma_u8s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                         uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// What a group of an input row carries besides its digits.
+struct alignas(8) GroupAux {
+    float unit;  // 2^-E: the value of the digits' last place
+    float sum;   // sum of the group's values
+};
+
+// Eight consecutive bf16 values `v` (run `run` of a row, runs of a group in eight adjacent lanes; called
+// by whole warps, `valid` false for lanes past the row) as digits at `digits` and the group's `aux`.
+// Layout of a group: digit column c (0 = highest) at 64 c; inside, per 16 values [even 0..6 | even 8..14
+// | odd 1..7 | odd 9..15] — what lane (column, t) of the MMA loads as 16 bytes for the low and the high
+// nibbles of its eight packed bytes.
+template <bool INT8 = false>
+__device__ __forceinline__ void digits_put(int run, bool valid, const uint4 &v, uint8_t *digits, GroupAux *aux) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    float x[8];
+    uint32_t top = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        x[2 * i] = __uint_as_float(w[i] << 16);
+        x[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+        top = max(top, max(w[i] & 0x7FFFu, (w[i] >> 16) & 0x7FFFu));
+    }
+    float sum = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+#pragma unroll
+    for (int o = 1; o <= 4; o <<= 1) {
+        top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
+        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    }
+    // |x| < 2^(e - 126) for exponent field e: E = 156 - e, held to what a float can carry
+    const int e = (int)(top >> 7), E = min(156 - e, 126);
+    const float scale = __int_as_float((E + 127) << 23), scaleOdd = INT8 ? scale : scale * 0.0625f;
+    uint32_t U[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        // balanced digits: bytes of V + 0x808080, the lower three less 128
+        const uint32_t V = (uint32_t)__float2int_rn(x[i] * ((i & 1) ? scaleOdd : scale));
+        U[i] = (V + 0x00808080u) ^ 0x00808080u;
+    }
+    if (!valid) return;
+    uint8_t *dst = digits + (size_t)(run >> 3) * kDigitGroupBytes + (run & 7) / 2 * 16 + (run & 1) * 4;
+    if (INT8) {
+        // codes in their own order: values 16 t + 0..3 | 4..7 | 8..11 | 12..15 of a quarter
+        dst += (run & 1) * 4;  // (a run is eight bytes there)
+    }
+#pragma unroll
+    for (int odd = 0; odd < 2; ++odd) {
+        const uint32_t u0 = INT8 ? U[4 * odd] : U[odd], u1 = INT8 ? U[4 * odd + 1] : U[2 + odd],
+                       u2 = INT8 ? U[4 * odd + 2] : U[4 + odd], u3 = INT8 ? U[4 * odd + 3] : U[6 + odd];
+        const uint32_t l0 = __byte_perm(u0, u1, 0x5140), l1 = __byte_perm(u2, u3, 0x5140);
+        const uint32_t h0 = __byte_perm(u0, u1, 0x7362), h1 = __byte_perm(u2, u3, 0x7362);
+        uint8_t *at = dst + odd * (INT8 ? 4 : 8);
+        *reinterpret_cast<uint32_t *>(at + 192) = __byte_perm(l0, l1, 0x5410);
+        *reinterpret_cast<uint32_t *>(at + 128) = __byte_perm(l0, l1, 0x7632);
+        *reinterpret_cast<uint32_t *>(at + 64) = __byte_perm(h0, h1, 0x5410);
+        *reinterpret_cast<uint32_t *>(at) = __byte_perm(h0, h1, 0x7632);
+    }
+    if ((run & 7) == 0) aux[run >> 3] = GroupAux{e == 255 ? __int_as_float(0x7FFFFFFF) : __int_as_float((127 - E) << 23), sum};
+}
+
+// (shared-memory addresses: the tile function is not inlined, so a pointer would be a generic one)
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ float lds_bf16(uint32_t a) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+    return bf2f(v);
+}
+
+// N consecutive groups of a 16-row tile: lo / hi this lane's eight packed bytes of tile rows g and g + 8
+// (g = lane / 4, t = lane % 4: bytes [8 t, + 8) of the group's 32; next group 32 bytes on), dig this
+// lane's 16 digit bytes of MMA column g; all shared-memory addresses.  The lane accounts for row g
+// (t < 2) or g + 8 (t >= 2), two neighbouring columns' digits joined (t even: the two high digits):
+// acc += s unit (digit sums), accBias += b sum, with s, b this lane's row's scales and biases and aux
+// its input's groups.
+template <int N>
+__device__ __forceinline__ void groups_int4(uint32_t lo, uint32_t hi, uint32_t dig, uint32_t s, uint32_t b, uint32_t aux,
+                                            bool lower, float &acc, float &accBias) {
+    uint2 wl[N], wh[N], ax[N];
+    uint4 x[N];
+    float sc[N], bi[N];
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        wl[u] = lds64(lo + 32 * u);
+        wh[u] = lds64(hi + 32 * u);
+        x[u] = lds128(dig + kDigitGroupBytes * u);
+    }
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        ax[u] = lds64(aux + 8 * u);
+        sc[u] = lds_bf16(s + 2 * u);
+        bi[u] = lds_bf16(b + 2 * u);
+    }
+    int d[N][4];
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        d[u][0] = d[u][1] = d[u][2] = d[u][3] = 0;
+        mma_u8s8(d[u], wl[u].x & 0x0F0F0F0Fu, wh[u].x & 0x0F0F0F0Fu, wl[u].y & 0x0F0F0F0Fu, wh[u].y & 0x0F0F0F0Fu, x[u].x, x[u].y);
+    }
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+        mma_u8s8(d[u], wl[u].x & 0xF0F0F0F0u, wh[u].x & 0xF0F0F0F0u, wl[u].y & 0xF0F0F0F0u, wh[u].y & 0xF0F0F0F0u, x[u].z, x[u].w);
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        const int v = (lower ? d[u][0] : d[u][2]) * 256 + (lower ? d[u][1] : d[u][3]);
+        acc = fmaf(sc[u] * __uint_as_float(ax[u].x), (float)v, acc);
+        accBias = fmaf(bi[u], __uint_as_float(ax[u].y), accBias);
+    }
+}
+
+// `n` consecutive groups of a 16-row tile against one input per row half: the dot product of row g in
+// lane (g, t = 0) and of row g + 8 in lane (g, t = 2) (other lanes hold parts).  Groups are taken in
+// ascending order.
+static __device__ __noinline__ float tile_int4(uint32_t lo, uint32_t hi, uint32_t dig, uint32_t s, uint32_t b, uint32_t aux, int n) {
+    const bool lower = (threadIdx.x & 3) < 2;
+    float acc = 0.0f, accBias = 0.0f;
+#pragma unroll 1
+    for (; n >= 4; n -= 4) {
+        groups_int4<4>(lo, hi, dig, s, b, aux, lower, acc, accBias);
+        lo += 128;
+        hi += 128;
+        dig += 4 * kDigitGroupBytes;
+        s += 8;
+        b += 8;
+        aux += 32;
+    }
+#pragma unroll 1
+    for (; n > 0; --n) {
+        groups_int4<1>(lo, hi, dig, s, b, aux, lower, acc, accBias);
+        lo += 32;
+        hi += 32;
+        dig += kDigitGroupBytes;
+        s += 2;
+        b += 2;
+        aux += 8;
+    }
+    const float low = __shfl_xor_sync(0xFFFFFFFFu, acc, 1);
+    return fmaf(acc, 65536.0f, low) + accBias;
+}
+
+}  // namespace ff

@@ -15,6 +15,7 @@ namespace ff {
 
 constexpr int kGroup = 64;        // codes per scale/bias pair
 constexpr int kMaxGemvRows = 16;  // input rows one GEMV job can carry (a verify block)
+constexpr int kDecodeMaps = 6;
 constexpr int kMaxExperts = 256;  // router width limit, as in the reference's prefill router
 
 // ---- error plumbing ------------------------------------------------------------------------
@@ -134,9 +135,10 @@ struct LayerStore {
     bool mapsReady = false;
     CUtensorMap routedMap[3];
     CUtensorMap sharedMap[3];
-    // one-token kernel: row-box maps of routed gate, routed up, shared gate, shared up, shared down
+    // one-token kernel: row-box maps of routed gate, routed up, shared gate, shared up, shared down,
+    // routed down
     bool decodeMapsReady = false;
-    CUtensorMap decodeMap[5];
+    CUtensorMap decodeMap[kDecodeMaps];
 };
 
 }  // namespace ff
