@@ -157,13 +157,13 @@ FFContext *ff_create(int32_t deviceOrdinal, const FFConfig *config, const char *
     if (ok) ok = cudaMemset(ctx->errorFlag, 0, 16) == cudaSuccess;
     ok = ok && dev_alloc(ctx, &ctx->phaseStamps, kPhaseStampSlots, error);
     if (ok) ok = cudaMemset(ctx->phaseStamps, 0, kPhaseStampSlots * 8) == cudaSuccess;
-    ok = ok && dev_alloc(ctx, &ctx->taggedLogits, kMaxExperts, error);
-    if (ok) ok = cudaMemset(ctx->taggedLogits, 0, kMaxExperts * 8) == cudaSuccess;
-    const size_t taggedWords = (size_t)K * c.f / 2 + c.d / 2;
+    ok = ok && dev_alloc(ctx, &ctx->taggedLogits, (size_t)ctx->smCount * kMaxExperts, error);
+    if (ok) ok = cudaMemset(ctx->taggedLogits, 0, (size_t)ctx->smCount * kMaxExperts * 8) == cudaSuccess;
+    const size_t taggedWords = (size_t)K * c.f / 2 + c.d / 2 + c.sharedF / 2;
     ok = ok && dev_alloc(ctx, &ctx->taggedActs, taggedWords, error);
     if (ok) ok = cudaMemset(ctx->taggedActs, 0, taggedWords * 8) == cudaSuccess;
-    ok = ok && dev_alloc(ctx, &ctx->gridBarrier, 16, error);
-    if (ok) ok = cudaMemset(ctx->gridBarrier, 0, 64) == cudaSuccess;
+    ok = ok && dev_alloc(ctx, &ctx->gridBarrier, 24, error);
+    if (ok) ok = cudaMemset(ctx->gridBarrier, 0, 96) == cudaSuccess;
     if (ok) {
         void *box = nullptr;
         ok = cudaHostAlloc(&box, 64, cudaHostAllocMapped) == cudaSuccess;

@@ -41,6 +41,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 #include "ff_int_device.cuh"
 
@@ -51,7 +52,9 @@ constexpr int kFusedWarps = kFusedThreads / 32;
 constexpr int kBigWarps = 10;      // warps 0..9: gate/up pairs and the routed down tiles
 constexpr int kSharedGuWarps = 8;  // warps 0..7 take the shared gate/up tiles in phase A (K quarters)
 constexpr int kRouterWarps = 2;    // warps 8, 9 the router rows
+constexpr int kRankWarp = 10;      // polls the logits
 constexpr uint32_t kBarrierSpinLimit = 1u << 24;
+constexpr uint32_t kHintSpinLimit = 1u << 12;
 
 struct DecodeArgs {
     const uint16_t *routerW, *routerScale, *gain;
@@ -67,13 +70,15 @@ struct DecodeArgs {
     const uint16_t *weightsIn;
     // Values handed from CTA to CTA travel as 64-bit words (launch tag << 32 | payload) that the
     // readers poll: a word is valid when its tag is the running launch's, so nothing is cleared.
-    unsigned long long *taggedLogits;  // [E] payload: the logit's bits
+    unsigned long long *taggedLogits;  // [CTA][kMaxExperts] payload: the logit's bits
     unsigned long long *taggedActs;    // [K * F / 2] payload: two routed activations (bf16)
     unsigned long long *taggedH1;      // [D / 2] payload: two rows of the shared FFN's output (bf16)
+    unsigned long long *taggedShared;  // [Fs / 2] payload: two shared activations (bf16)
     uint32_t *ids;
     uint16_t *weights;
-    uint16_t *sharedActs, *y;
-    unsigned long long *barrier;  // arrival counter of the grid barrier
+    uint16_t *y;
+    unsigned long long *barrier;  // ticket and hand-off counters
+    uint32_t *hints;              // [kHintSets][2]: finished shared and routed gate/up tiles
     uint32_t *errorFlag;
     unsigned long long *stamps;  // null, or the phase / per-warp timestamp slots (ns)
     int E, D, F, Fs, K;          // K = 0: shared FFN only (y receives its output)
@@ -101,41 +106,28 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
-// Grid-wide synchronisation on 64-bit counters that only grow.  At its start every CTA draws a
-// ticket from counter [3]; ticket / gridDim is the launch's generation g (launches on a context
-// are serialised, so all CTAs of a launch get the same g).  Every launch adds exactly gridDim to
-// counter [0] (shared activations written) — also when a mode does not wait on it — so "everyone
-// has arrived" is counter >= (g + 1) * gridDim.  An arrival is a release reduction without a
-// return value; a wait polls the counter with acquire loads, bounded.  No reset, no host-side
-// state.  [2] counts finished CTAs for the host hand-off.  g also gives the launch's 32-bit tag
-// (never 0, different for consecutive launches) for the values that travel as polled words
-// (logits, routed activations, shared output rows).
-enum : int { kCountShared = 0, kCountDone = 2, kCountTicket = 3 };
+// Values cross CTAs as tagged words only.  Two 64-bit counters that only grow go with them: at its
+// start every CTA draws a ticket from counter [3]; ticket / gridDim is the launch's generation (launches
+// on a context are serialised, so all CTAs of a launch get the same one), and the generation gives the
+// launch's 32-bit tag (never 0, different for consecutive launches).  [2] counts finished CTAs for the
+// host hand-off.  No reset, no host-side state.
+// Polling all of a row's words from every CTA would fill L2's bandwidth and hold up the stores it
+// waits for, so tile counters say when it is worth looking: four sets used in turn, the one of the
+// launch after next cleared by CTA 0.  They are hints, not ordered with the words; the words' tags
+// decide.
+enum : int { kCountDone = 2, kCountTicket = 3, kHintSets = 4 };
+__device__ __forceinline__ void hint_add(uint32_t *hint) {
+    asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(hint) : "memory");
+}
+// By one thread, bounded (the words behind the hint are waited for in any case).
+__device__ __forceinline__ void hint_wait(const uint32_t *hint, uint32_t count) {
+    uint32_t v = 0;
+    for (uint32_t spins = 0; spins < kHintSpinLimit && v < count; ++spins)
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(hint) : "memory");
+}
 
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long *p) {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-// Called by ONE thread after a CTA-level barrier that covers the writes to publish.
-__device__ __forceinline__ void counter_arrive(unsigned long long *count) {
-    asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(count) : "memory");
-}
-// Called by ONE thread; a CTA-level barrier afterwards releases the other threads.
-__device__ __forceinline__ void counter_wait(const unsigned long long *count, unsigned long long target,
-                                             uint32_t *errorFlag) {
-    uint32_t spins = 0;
-    while (ld_acquire_u64(count) < target) {
-        if (++spins > kBarrierSpinLimit) {
-            atomicExch(errorFlag, 9u);
-            break;
-        }
-    }
-    __threadfence();
-}
-// The thread that arrives at and waits for the CTA-wide barriers: lane 0 of the last warp (a warp
-// with no requests to issue between arriving and waiting).
-__device__ __forceinline__ bool is_barrier_thread() { return threadIdx.x == blockDim.x - 32; }
+// The thread that waits for the CTA: lane 0 of the last warp.
+__device__ __forceinline__ bool is_waiting_thread() { return threadIdx.x == blockDim.x - 32; }
 
 __device__ __forceinline__ void st_tagged(unsigned long long *p, uint32_t tag, uint32_t payload) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(((unsigned long long)tag << 32) | payload) : "memory");
@@ -176,27 +168,37 @@ __device__ __forceinline__ void box_copy(uint32_t dst, const CUtensorMap *map, i
 }
 
 // Rows of bf16 values as digits (flat run index over all rows) by `threads` threads, this one number
-// `tid`; `fetch` returns the run's eight values.  No barrier at the end.
+// `tid`; fetch(i, j, v, w) reads runs i and j (negative: none).  No barrier at the end.
 template <typename Fetch>
 __device__ __forceinline__ void stage_digits(int runs, int tid, int threads, uint8_t *digits, GroupAux *aux, Fetch fetch) {
-    for (int base = tid & ~31; base < runs; base += threads) {
-        const int i = base + (tid & 31);
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (i < runs) v = fetch(i);
+    // two runs in flight
+    for (int base = tid & ~31; base < runs; base += 2 * threads) {
+        const int i = base + (tid & 31), j = i + threads;
+        uint4 v = make_uint4(0, 0, 0, 0), w = make_uint4(0, 0, 0, 0);
+        fetch(i < runs ? i : -1, j < runs ? j : -1, v, w);
         digits_put(i, i < runs, v, digits, aux);
+        if (base + threads < runs) digits_put(j, j < runs, w, digits, aux);  // the same for the whole warp
     }
 }
-// A run of eight values that another CTA is still writing as four tagged words, polled (bounded).
-__device__ __forceinline__ uint4 fetch_tagged(const unsigned long long *src, uint32_t tag, uint32_t *errorFlag) {
-    unsigned long long w0 = 0, w1 = 0, w2 = 0, w3 = 0;
-    bool ok = false;
-    for (uint32_t spins = 0; spins < kBarrierSpinLimit && !ok; ++spins) {
-        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w0), "=l"(w1) : "l"(src) : "memory");
-        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w2), "=l"(w3) : "l"(src + 2) : "memory");
-        ok = (uint32_t)(w0 >> 32) == tag && (uint32_t)(w1 >> 32) == tag && (uint32_t)(w2 >> 32) == tag && (uint32_t)(w3 >> 32) == tag;
+// Runs of eight values that other CTAs are still writing as four tagged words each, polled (bounded);
+// i, j < 0: none.
+__device__ __forceinline__ void fetch_tagged(const unsigned long long *src, uint32_t tag, int i, int j, uint4 &v, uint4 &w,
+                                             uint32_t *errorFlag) {
+    auto one = [&](int r, uint4 &out) {
+        const unsigned long long *p = src + 4 * (size_t)r;
+        unsigned long long w0, w1, w2, w3;
+        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w0), "=l"(w1) : "l"(p) : "memory");
+        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w2), "=l"(w3) : "l"(p + 2) : "memory");
+        out = make_uint4((uint32_t)w0, (uint32_t)w1, (uint32_t)w2, (uint32_t)w3);
+        return (uint32_t)(w0 >> 32) == tag && (uint32_t)(w1 >> 32) == tag && (uint32_t)(w2 >> 32) == tag && (uint32_t)(w3 >> 32) == tag;
+    };
+    bool okI = i < 0, okJ = j < 0;
+    for (uint32_t spins = 0; spins < kBarrierSpinLimit && !(okI && okJ); ++spins) {
+        const bool askI = !okI, askJ = !okJ;
+        if (askI) okI = one(i, v);
+        if (askJ) okJ = one(j, w);
     }
-    if (!ok) atomicExch(errorFlag, 9u);
-    return make_uint4((uint32_t)w0, (uint32_t)w1, (uint32_t)w2, (uint32_t)w3);
+    if (!(okI && okJ)) atomicExch(errorFlag, 9u);
 }
 
 // A float as an unsigned number of the same order.
@@ -205,59 +207,61 @@ __device__ __forceinline__ uint32_t ordered_key(float f) {
     return (u >> 31) ? ~u : (u | 0x80000000u);
 }
 
-// The K largest of E logits that arrive as tagged words, by one warp: higher score, then lower id;
-// -inf and NaN are never taken.  Lane r < K returns route r's id (0 when there is none) and score.
-// Each round is two warp-wide reductions over register keys (0.3 us for eight routes of 128; counting
-// every logit's rank by 256 threads through shared memory took 1.0 us).
-__device__ __forceinline__ void poll_and_rank(const DecodeArgs &a, uint32_t tag, int lane, uint32_t &myId, float &myScore) {
-    uint32_t key[8];
-#pragma unroll
-    for (int blk = 0; blk < 2; ++blk) {
-        const int e0 = 128 * blk + 4 * lane;
-        const unsigned long long filler = (unsigned long long)tag << 32;
-        unsigned long long w[4] = {filler, filler, filler, filler};
-        bool ready = 128 * blk >= a.E;
-        const bool here = !ready;
-        for (uint32_t spins = 0; spins < kBarrierSpinLimit && !ready; ++spins) {
-            if (e0 + 3 < a.E) {
-                asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w[0]), "=l"(w[1]) : "l"(a.taggedLogits + e0) : "memory");
-                asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w[2]), "=l"(w[3]) : "l"(a.taggedLogits + e0 + 2) : "memory");
-            } else {
-                for (int i = 0; i < 4; ++i)
-                    if (e0 + i < a.E) w[i] = ld_tagged(a.taggedLogits + e0 + i);
+// The K largest logits, by the whole CTA: one warp polls the CTA's copy of the tagged words and puts
+// their keys into shared memory (0: never taken — -inf or NaN); then four threads per expert count the
+// experts that come before it (higher score, then lower id), a quarter of the keys each.  The loop is
+// short and rolled: this code runs once per launch, where unrolled code is bound by instruction fetch
+// (one warp taking the maximum eight times 2 us, votes per expert unrolled 3 us, this 0.5 us).
+// sKey: four quarters of kKeyQuarter words.  Ends with a CTA barrier.
+constexpr int kKeyQuarter = kMaxExperts / 4 + 4;  // (+4: the quarters' 128-bit reads fall on different banks)
+__device__ __forceinline__ void poll_and_rank(const DecodeArgs &a, uint32_t tag, uint32_t *sKey, uint32_t *sIds, float *sScore) {
+    const int tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int quarter = ((a.E + 3) / 4 + 3) & ~3;  // keys of a quarter, a multiple of four
+    if (warp == kRankWarp) {
+        const unsigned long long *words = a.taggedLogits + (size_t)blockIdx.x * kMaxExperts;
+        for (int base = 0; base < 4 * quarter; base += 64) {
+            const int e = base + 2 * lane;  // (quarters are multiples of four: both words in one)
+            if (e >= 4 * quarter) break;
+            unsigned long long w[2] = {0, 0};
+            bool ok = false;
+            for (uint32_t spins = 0; spins < kBarrierSpinLimit && !ok; ++spins) {
+                asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w[0]), "=l"(w[1]) : "l"(words + e) : "memory");
+                ok = (e >= a.E || (uint32_t)(w[0] >> 32) == tag) && (e + 1 >= a.E || (uint32_t)(w[1] >> 32) == tag);
             }
-            const bool mine = (uint32_t)(w[0] >> 32) == tag && (uint32_t)(w[1] >> 32) == tag && (uint32_t)(w[2] >> 32) == tag &&
-                              (uint32_t)(w[3] >> 32) == tag;
-            ready = __all_sync(0xFFFFFFFFu, mine);
-        }
-        if (!ready && lane == 0) atomicExch(a.errorFlag, 9u);
+            if (!ok) atomicExch(a.errorFlag, 9u);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float v = __uint_as_float((uint32_t)w[i]);
-            key[4 * blk + i] = here && e0 + i < a.E && v > -INFINITY ? ordered_key(v) : 0u;
+            for (int i = 0; i < 2; ++i) {
+                const float v = __uint_as_float((uint32_t)w[i]);
+                sKey[e / quarter * kKeyQuarter + e % quarter + i] = e + i < a.E && v > -INFINITY ? ordered_key(v) : 0u;
+            }
         }
     }
-    myId = 0u;
-    myScore = -INFINITY;
-    for (int r = 0; r < a.K; ++r) {
-        uint32_t best = key[0], at = 4u * (uint32_t)lane;
-#pragma unroll
-        for (int j = 1; j < 8; ++j)
-            if (key[j] > best) {
-                best = key[j];
-                at = (uint32_t)(128 * (j >> 2) + 4 * lane + (j & 3));
-            }
-        const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, best);
-        if (top == 0u) break;
-        const uint32_t id = __reduce_min_sync(0xFFFFFFFFu, best == top ? at : 0xFFFFFFFFu);
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (id == (uint32_t)(128 * (j >> 2) + 4 * lane + (j & 3))) key[j] = 0u;
-        if (lane == r) {
-            myId = id;
-            myScore = __uint_as_float((top >> 31) ? (top & 0x7FFFFFFFu) : ~top);
+    if (tid < 8) {
+        sIds[tid] = 0u;
+        sScore[tid] = -INFINITY;
+    }
+    __syncthreads();
+    for (int base = 0; base < a.E; base += kFusedThreads / 4) {
+        const int e = base + (tid >> 2), q = tid & 3;
+        const uint32_t mine = e < a.E ? sKey[e / quarter * kKeyQuarter + e % quarter] : 0u;
+        const uint32_t *keys = sKey + q * kKeyQuarter;
+        int rank = 0, before = e - q * quarter;  // of the quarter, this many come before e by id
+#pragma unroll 1
+        for (int o = 0; o < quarter; o += 4, before -= 4) {
+            const uint4 k = *reinterpret_cast<const uint4 *>(keys + o);
+            rank += k.x >= mine + (before > 0 ? 0u : 1u) ? 1 : 0;
+            rank += k.y >= mine + (before > 1 ? 0u : 1u) ? 1 : 0;
+            rank += k.z >= mine + (before > 2 ? 0u : 1u) ? 1 : 0;
+            rank += k.w >= mine + (before > 3 ? 0u : 1u) ? 1 : 0;
+        }
+        rank += __shfl_xor_sync(0xFFFFFFFFu, rank, 1);
+        rank += __shfl_xor_sync(0xFFFFFFFFu, rank, 2);
+        if (q == 0 && mine && rank < a.K) {
+            sIds[rank] = (uint32_t)e;
+            sScore[rank] = __uint_as_float((mine >> 31) ? (mine & 0x7FFFFFFFu) : ~mine);
         }
     }
+    __syncthreads();
 }
 
 // The input row travelling inside the kernel's parameters (no host-to-device copy before the
@@ -270,9 +274,10 @@ struct InlineRow {
 __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMaps &maps, const uint16_t *xInline) {
     extern __shared__ __align__(128) uint8_t smemRaw[];
     __shared__ uint32_t sIds[8];
-    __shared__ float sWeights[8];
+    __shared__ __align__(16) uint32_t sKey[4 * kKeyQuarter];
+    __shared__ float sWeights[8], sScore[8];
     __shared__ __align__(8) uint64_t sCopyBar[kFusedWarps + kRouterWarps];
-    __shared__ unsigned long long sTarget;  // (generation + 1) * gridDim
+    __shared__ uint32_t *sHints;            // this launch's tile counters
     __shared__ uint32_t sTag;               // the launch's tag for polled words, from the generation
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -409,17 +414,17 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     if (tSD < tilesSD) issue_shared_down(tSD, part3);
     warp_stamp(a, 0, 0);
     if (threadIdx.x == 9 * 32) {
-        const unsigned long long gen1 = ticket / gridDim.x + 1ull;
-        sTarget = gen1 * gridDim.x;
-        sTag = (uint32_t)(gen1 % 0xFFFFFFFFull) + 1u;  // 1 .. 2^32-1: never 0, consecutive launches differ
+        const unsigned long long generation = ticket / gridDim.x;
+        sTag = (uint32_t)((generation + 1ull) % 0xFFFFFFFFull) + 1u;  // 1 .. 2^32-1: never 0, consecutive launches differ
+        sHints = a.hints + 2 * (generation % kHintSets);
+        if (cta == 0) *reinterpret_cast<uint2 *>(a.hints + 2 * ((generation + 2) % kHintSets)) = make_uint2(0u, 0u);
     }
     // the input row, as digits and (for the router) as it is
-    stage_digits(D >> 3, (int)threadIdx.x, kFusedThreads, smemRaw, xAux, [&](int i) {
-        const uint4 v = i == (int)threadIdx.x ? xMine : fetchX(i);
-        reinterpret_cast<uint4 *>(region)[i] = v;
-        return v;
+    stage_digits(D >> 3, (int)threadIdx.x, kFusedThreads, smemRaw, xAux, [&](int i, int j, uint4 &v, uint4 &w) {
+        if (i >= 0) reinterpret_cast<uint4 *>(region)[i] = v = i == (int)threadIdx.x ? xMine : fetchX(i);
+        if (j >= 0) reinterpret_cast<uint4 *>(region)[j] = w = fetchX(j);
     });
-    __syncthreads();  // target and tag are published, too
+    __syncthreads();  // the tag is published, too
     const uint32_t tag = sTag;
     for (; tA < tilesSGU; tA += (kSharedGuWarps / 4) * G) {
         wait_tile(warp & ~3);
@@ -436,37 +441,61 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
             const float *m = mine + (t >> 1) * 8 + g;
             const float sum = ((v + m[16]) + m[32]) + m[48];
             const float up = __shfl_down_sync(0xFFFFFFFFu, sum, 2);
-            if (t == 0) a.sharedActs[tA * 8 + g] = f2bf(gelu_tanh(bf16_round(sum)) * bf16_round(up));
+            // two activations of a tile per tagged word, the odd neighbour's by shuffle
+            const uint32_t act = f2bf(gelu_tanh(bf16_round(sum)) * bf16_round(up));
+            const uint32_t two = act | (__shfl_down_sync(0xFFFFFFFFu, act, 4) << 16);
+            if (t == 0 && !(g & 1)) st_tagged(a.taggedShared + ((tA * 8 + g) >> 1), tag, two);
+            if (lane == 0) hint_add(sHints);
         }
         named_barrier(1 + (warp >> 2), 128);
     }
     for (; eA < E; eA += kRouterWarps * G) {
+        const float biasE = a.logitBias ? __ldg(a.logitBias + eA) : 0.0f;
         slot_wait(routerBar, routerParity, a.errorFlag);
         warp_stamp(a, 0, 1);
         // lane l chains fmaf over elements [256 i + 8 l, +8): the order of every router kernel
-        float acc = 0.0f;
-#pragma unroll 4
-        for (int c = lane; c < (D >> 3); c += 32) {
-            const uint4 wv = lds128(slot + 16u * (uint32_t)c), xv = lds128(sm_addr(region) + 16u * (uint32_t)c);
-            const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w}, xx[4] = {xv.x, xv.y, xv.z, xv.w};
-            uint4 sv = make_uint4(0, 0, 0, 0);
-            if (a.routerScale) sv = lds128(slot + (uint32_t)D * 2u + 16u * (uint32_t)c);
-            const uint32_t ss[4] = {sv.x, sv.y, sv.z, sv.w};
+        const uint32_t xRow = sm_addr(region);
+        const int chunks = D >> 3;
+        auto chain = [&](auto scaled) {
+            float acc = 0.0f;
+            auto run = [&](const uint4 &wv, const uint4 &xv, const uint4 &sv) {
+                const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w}, xx[4] = {xv.x, xv.y, xv.z, xv.w}, ss[4] = {sv.x, sv.y, sv.z, sv.w};
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                float x0 = __uint_as_float(xx[k] << 16), x1 = __uint_as_float(xx[k] & 0xFFFF0000u);
-                if (a.routerScale) {
-                    x0 = x0 * __uint_as_float(ss[k] << 16);
-                    x1 = x1 * __uint_as_float(ss[k] & 0xFFFF0000u);
+                for (int k = 0; k < 4; ++k) {
+                    float x0 = __uint_as_float(xx[k] << 16), x1 = __uint_as_float(xx[k] & 0xFFFF0000u);
+                    if (decltype(scaled)::value) {
+                        x0 = x0 * __uint_as_float(ss[k] << 16);
+                        x1 = x1 * __uint_as_float(ss[k] & 0xFFFF0000u);
+                    }
+                    acc = fmaf(__uint_as_float(ww[k] << 16), x0, acc);
+                    acc = fmaf(__uint_as_float(ww[k] & 0xFFFF0000u), x1, acc);
                 }
-                acc = fmaf(__uint_as_float(ww[k] << 16), x0, acc);
-                acc = fmaf(__uint_as_float(ww[k] & 0xFFFF0000u), x1, acc);
+            };
+            // four steps' loads ahead of their multiply-adds; steps past the row add 0 * 0
+#pragma unroll 1
+            for (int c = lane; c < chunks + 31; c += 128) {
+                uint4 wv[4], xv[4], sv[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    wv[i] = xv[i] = sv[i] = make_uint4(0, 0, 0, 0);
+                    if (c + 32 * i < chunks) {
+                        wv[i] = lds128(slot + 16u * (uint32_t)(c + 32 * i));
+                        xv[i] = lds128(xRow + 16u * (uint32_t)(c + 32 * i));
+                        if (decltype(scaled)::value) sv[i] = lds128(slot + (uint32_t)D * 2u + 16u * (uint32_t)(c + 32 * i));
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) run(wv[i], xv[i], sv[i]);
             }
-        }
+            return acc;
+        };
+        float acc = a.routerScale ? chain(std::true_type{}) : chain(std::false_type{});
 #pragma unroll
         for (int offset = 16; offset >= 1; offset >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, offset);
-        // value and validity in one 64-bit store: the readers poll these words
-        if (lane == 0) st_tagged(a.taggedLogits + eA, tag, __float_as_uint(a.logitBias ? acc + a.logitBias[eA] : acc));
+        // Value and validity in one 64-bit store, one copy for every CTA: the readers poll their own
+        // copies (all CTAs' polls on eight lines held the stores up for microseconds).
+        const float logit = a.logitBias ? acc + biasE : acc;
+        for (int c = lane; c < G; c += 32) st_tagged(a.taggedLogits + (size_t)c * kMaxExperts + eA, tag, __float_as_uint(logit));
         slot_release();
         const int next = eA + kRouterWarps * G;
         if (next < E) issue_router(next);
@@ -474,49 +503,55 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     warp_stamp(a, 0, 2);
     stamp(a, 1);
 
-    // ---------------- top-8 by warp 8 while warps 0..7 finish the shared gate/up rows ----------------
-    uint32_t myId = 0u;
-    float myScore = -INFINITY;
-    const bool ranking = K > 0 && !a.idsIn && warp == kSharedGuWarps;
-    if (ranking) {
-        poll_and_rank(a, tag, lane, myId, myScore);
-        if (lane < K) sIds[lane] = myId;
-    } else if (K > 0 && a.idsIn && (int)threadIdx.x < K) {
-        // Given routes.  A route past the resident experts would address memory outside the layer:
-        // it is replaced by expert 0 with weight 0 and reported through the error flag (the
-        // reference refuses such a route with "route expert N is out of range").
-        uint32_t id = a.idsIn[threadIdx.x];
-        float w = bf2f(a.weightsIn[threadIdx.x]);
-        if (id >= (uint32_t)a.expertCount) {
-            atomicExch(a.errorFlag, 12u);
-            id = 0u;
-            w = 0.0f;
-        }
-        sIds[threadIdx.x] = id;
-        sWeights[threadIdx.x] = w;
-    }
-    // the arrival covers the shared activations, the CTA barrier also publishes the routes
-    __syncthreads();
-    if (is_barrier_thread()) counter_arrive(a.barrier + kCountShared);
-    stamp(a, 2);
-    stamp(a, 3);
+    // ---------------- top-8 ----------------
     const int tilesF = F >> 3;
     const int tilesRouted = K * tilesF;
     int tB = warp < kBigWarps ? pair * G + cta : 0x7FFFFFFF;
-    auto issue_routed_gate_up = [&](int tile) {
-        const int k = tile / tilesF;
-        issue_gate_up(&maps.m[kMapRoutedGate], &maps.m[kMapRoutedUp], (int)sIds[k], a.experts + (size_t)sIds[k] * a.stride, a.off,
-                      tile - k * tilesF, warp & 1, 2, a.strideGU, scalesOfPair(pair));
+    int kB = 0x7FFFFFFF;  // route and tile inside its expert, ready before the routes are
+    int tileB = 0;
+    auto place = [&](int tile) {
+        kB = tile / tilesF;
+        tileB = tile - kB * tilesF;
     };
-    if (tB < tilesRouted) issue_routed_gate_up(tB);
-    warp_stamp(a, 1, 0);
-    if (ranking) {
+    if (tB < tilesRouted) place(tB);
+    if (K > 0) {
+        if (!a.idsIn) {
+            poll_and_rank(a, tag, sKey, sIds, sScore);
+        } else {
+            // Given routes.  A route past the resident experts would address memory outside the layer:
+            // it is replaced by expert 0 with weight 0 and reported through the error flag (the
+            // reference refuses such a route with "route expert N is out of range").
+            if ((int)threadIdx.x < K) {
+                uint32_t id = a.idsIn[threadIdx.x];
+                float w = bf2f(a.weightsIn[threadIdx.x]);
+                if (id >= (uint32_t)a.expertCount) {
+                    atomicExch(a.errorFlag, 12u);
+                    id = 0u;
+                    w = 0.0f;
+                }
+                sIds[threadIdx.x] = id;
+                sWeights[threadIdx.x] = w;
+            }
+            __syncthreads();
+        }
+    }
+    stamp(a, 2);
+    stamp(a, 3);
+    auto issue_routed_gate_up = [&]() {
+        issue_gate_up(&maps.m[kMapRoutedGate], &maps.m[kMapRoutedUp], (int)sIds[kB], a.experts + (size_t)sIds[kB] * a.stride, a.off,
+                      tileB, warp & 1, 2, a.strideGU, scalesOfPair(pair));
+    };
+    if (tB < tilesRouted) issue_routed_gate_up();
+    if (warp < kBigWarps) warp_stamp(a, 1, 0);
+    if (K > 0 && !a.idsIn && warp == kSharedGuWarps) {
         // softmax over the chosen scores: exponentials in parallel, the sum in rank order
+        const float myScore = lane < K ? sScore[lane] : -INFINITY;
         const float top = __shfl_sync(0xFFFFFFFFu, myScore, 0);
         const float ex = lane < K ? expf(myScore - top) : 0.0f;
         float sum = 0.0f;
         for (int r = 0; r < K; ++r) sum += __shfl_sync(0xFFFFFFFFu, ex, r);
         if (lane < K) {
+            const uint32_t myId = sIds[lane];
             float w = ex / sum;
             if (a.gain) w = w * bf2f(a.gain[myId]);
             const uint16_t wb = f2bf(w);
@@ -553,10 +588,10 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     };
     if (warp >= kBigWarps && sh) {
         // the shared activations, staged by the six warps that use them
-        if (is_barrier_thread()) counter_wait(a.barrier + kCountShared, sTarget, a.errorFlag);
+        if (is_waiting_thread()) hint_wait(sHints, (uint32_t)tilesSGU);
         named_barrier(8, (kFusedWarps - kBigWarps) * 32);
         stage_digits(Fs >> 3, (int)threadIdx.x - kBigWarps * 32, (kFusedWarps - kBigWarps) * 32, region, regionAux,
-                     [&](int i) { return __ldcg(reinterpret_cast<const uint4 *>(a.sharedActs) + i); });
+                     [&](int i, int j, uint4 &v, uint4 &w) { fetch_tagged(a.taggedShared, tag, i, j, v, w, a.errorFlag); });
         named_barrier(8, (kFusedWarps - kBigWarps) * 32);
     }
     for (; tB < tilesRouted; tB += (kBigWarps / 2) * G) {
@@ -569,7 +604,10 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
         if ((warp & 1) && !(t & 1)) mine[(t >> 1) * 8 + g] = v;
         named_barrier(1 + pair, 64);
         const int next = tB + (kBigWarps / 2) * G;
-        if (next < tilesRouted) issue_routed_gate_up(next);
+        if (next < tilesRouted) {
+            place(next);
+            issue_routed_gate_up();
+        }
         if (!(warp & 1)) {
             // the tile's eight activations are one run of the staged row: four tagged words,
             // written by the lanes t == 0 of even g (the odd neighbour's value comes by shuffle)
@@ -578,6 +616,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
             const uint32_t act = f2bf(gelu_tanh(sum) * up);
             const uint32_t two = act | (__shfl_down_sync(0xFFFFFFFFu, act, 4) << 16);
             if (t == 0 && !(g & 1)) st_tagged(a.taggedActs + ((tB * 8 + g) >> 1), tag, two);
+            if (lane == 0) hint_add(sHints + 1);
         }
         named_barrier(1 + pair, 64);
     }
@@ -621,24 +660,28 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     // No grid barrier before phase C: the routed activations and the shared output rows are polled
     // as tagged words while they are staged.
     warp_stamp(a, 2, 0);
+    if (is_waiting_thread()) hint_wait(sHints + 1, (uint32_t)tilesRouted);
     __syncthreads();  // the region still holds the shared activations that phase B's warps read
     stamp(a, 5);
 
     // ---------------- phase C: routed down rows and the combine ----------------
+    // Warp w combines a round's row tile w, lane r its row r; the residual (two rows of the shared
+    // output in a tagged word, or the caller's row) is asked for ahead of the activations.
+    auto combine_tile = [&](int round) { return cta + G * (round * perRound + warp); };
+    auto combines = [&](int round) { return warp < perRound && combine_tile(round) < tilesRD && lane < 8; };
+    unsigned long long resWord = 0;
+    float residual = 0.0f;
+    auto ask_residual = [&](int round) {
+        if (!combines(round)) return;
+        const int row = combine_tile(round) * 8 + lane;
+        if (a.shared) resWord = ld_tagged(a.taggedH1 + (row >> 1));
+        else residual = a.residual ? bf2f(__ldcg(a.residual + row)) : 0.0f;
+    };
+    ask_residual(0);
     stage_digits(K * (F >> 3), (int)threadIdx.x, kFusedThreads, region, regionAux,
-                 [&](int i) { return fetch_tagged(a.taggedActs + 4 * (size_t)i, tag, a.errorFlag); });
+                 [&](int i, int j, uint4 &v, uint4 &w) { fetch_tagged(a.taggedActs, tag, i, j, v, w, a.errorFlag); });
     __syncthreads();
     for (int round = 0; cta + G * round * perRound < tilesRD; ++round) {
-        // warp w combines the round's row tile w, lane r its row r; its residual is asked for first
-        const int myRowTile = cta + G * (round * perRound + warp);
-        const bool combines = warp < perRound && myRowTile < tilesRD && lane < 8;
-        const int row = myRowTile * 8 + lane;
-        unsigned long long resWord = 0;
-        float acc = 0.0f;
-        if (combines) {
-            if (a.shared) resWord = ld_tagged(a.taggedH1 + (row >> 1));
-            else if (a.residual) acc = bf2f(__ldcg(a.residual + row));
-        }
         if (has_task(round)) {
             slot_wait(myBar, parity, a.errorFlag);
             warp_stamp(a, 2, 1);
@@ -651,7 +694,9 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
         }
         __syncthreads();
         if (has_task(round + 1)) issue_routed_down(tileOf(round + 1));
-        if (combines) {
+        if (combines(round)) {
+            const int row = combine_tile(round) * 8 + lane;
+            float acc = residual;
             if (a.shared) {
                 uint32_t spins = 0;
                 while ((uint32_t)(resWord >> 32) != tag) {
@@ -666,6 +711,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
             for (int k = 0; k < K; ++k) acc = __fadd_rn(acc, __fmul_rn(sWeights[k], downRows[(warp * 8 + k) * 8 + lane]));
             a.y[row] = f2bf(acc);
         }
+        ask_residual(round + 1);
         __syncthreads();  // the rows are rewritten in the next round
     }
     warp_stamp(a, 2, 2);
@@ -778,11 +824,12 @@ bool launch_decode_fused(FFContext *ctx, const LayerStore &L, const uint16_t *x,
     a.taggedLogits = ctx->taggedLogits;
     a.taggedActs = ctx->taggedActs;
     a.taggedH1 = ctx->taggedActs + (size_t)c.topK * c.f / 2;
+    a.taggedShared = a.taggedH1 + c.d / 2;
     a.ids = ctx->ids;
     a.weights = ctx->weights;
-    a.sharedActs = ctx->sharedActs;
     a.y = y;
     a.barrier = reinterpret_cast<unsigned long long *>(ctx->gridBarrier);
+    a.hints = ctx->gridBarrier + 16;
     a.errorFlag = ctx->errorFlag;
     a.stamps = ctx->tracing ? ctx->phaseStamps : nullptr;
     a.E = idsIn ? (int)L.expertCount : (int)L.routerExperts;

@@ -155,16 +155,10 @@ static __device__ __noinline__ float tile_int4(uint32_t lo, uint32_t hi, uint32_
         b += 8;
         aux += 32;
     }
-#pragma unroll 1
-    for (; n > 0; --n) {
-        groups_int4<1>(lo, hi, dig, s, b, aux, lower, acc, accBias);
-        lo += 32;
-        hi += 32;
-        dig += kDigitGroupBytes;
-        s += 2;
-        b += 2;
-        aux += 8;
-    }
+    // the rest in one batch, so that its latencies overlap
+    if (n == 3) groups_int4<3>(lo, hi, dig, s, b, aux, lower, acc, accBias);
+    else if (n == 2) groups_int4<2>(lo, hi, dig, s, b, aux, lower, acc, accBias);
+    else if (n == 1) groups_int4<1>(lo, hi, dig, s, b, aux, lower, acc, accBias);
     const float low = __shfl_xor_sync(0xFFFFFFFFu, acc, 1);
     return fmaf(acc, 65536.0f, low) + accBias;
 }
