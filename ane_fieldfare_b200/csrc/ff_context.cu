@@ -53,6 +53,8 @@ static void free_shared8(LayerStore &L) {
 static void free_layer(LayerStore &L) {
     cudaFree(L.experts);
     cudaFree(L.shared);
+    cudaFree(L.routedScales);
+    cudaFree(L.sharedScales);
     free_shared8(L);
     cudaFree(L.routerQ);
     cudaFree(L.routerQScale);
@@ -327,7 +329,7 @@ bool ff_load_layer(FFContext *ctx, uint32_t layer, const void *hostBytes, uint64
     L.mapsReady = false;
     L.decodeMapsReady = false;
     ctx->weightBytes += total;
-    return true;
+    return pack_scales(ctx, L.experts, L.stride, L.off, d, f, expertCount, &L.routedScales, error);
 }
 
 static bool check_projection(const FFProjection *p, uint32_t rows, uint32_t cols, const char *name,
@@ -372,7 +374,7 @@ bool ff_load_shared(FFContext *ctx, uint32_t layer, const FFProjection *gate,
     L.mapsReady = false;
     L.decodeMapsReady = false;
     ctx->weightBytes += payload;
-    return true;
+    return pack_scales(ctx, L.shared, 0, L.sharedOff, d, fs, 1, &L.sharedScales, error);
 }
 
 static void free_router(ff::LayerStore &L) {

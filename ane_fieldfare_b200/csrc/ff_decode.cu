@@ -52,18 +52,18 @@ constexpr int kFusedWarps = kFusedThreads / 32;
 constexpr int kBigWarps = 10;      // warps 0..9: gate/up pairs and the routed down tiles
 constexpr int kSharedGuWarps = 8;  // warps 0..7 take the shared gate/up tiles in phase A (K quarters)
 constexpr int kRouterWarps = 2;    // warps 8, 9 the router rows
-constexpr int kRankWarp = 10;      // polls the logits
+constexpr int kRankWarp = 9;       // polls the logits
+static_assert(kRankWarp < kBigWarps && 8 <= kBigWarps, "warps 0..9 rank");
 constexpr uint32_t kBarrierSpinLimit = 1u << 24;
 constexpr uint32_t kHintSpinLimit = 1u << 12;
 
 struct DecodeArgs {
     const uint16_t *routerW, *routerScale, *gain;
     const float *logitBias;
-    const uint8_t *experts;
-    uint64_t stride;
-    FFExpertOffsets off;
+    const uint32_t *scales;       // routed scale | bias words, scaleStride words per expert (see pack_scales)
+    uint64_t scaleStride;
+    const uint32_t *sharedScales;
     const uint8_t *shared;  // null: no shared FFN, `residual` is added instead
-    FFExpertOffsets sharedOff;
     const uint16_t *x;
     const uint16_t *residual;
     const uint32_t *idsIn;  // non-null: routes are given, the router is skipped
@@ -89,7 +89,7 @@ struct DecodeArgs {
     unsigned long long *mailbox;
     uint32_t epoch;
     // shared-memory carve-up (fused_layout)
-    uint32_t regionOffset, regionAux, partialOffset, downOffset, slotsOffset, rowsBytes, pairBytes, tripleBytes, downBytes;
+    uint32_t x32Offset, regionOffset, regionAux, partialOffset, downOffset, slotsOffset, rowsBytes, pairBytes, tripleBytes, downBytes;
     uint32_t strideGU, strideGUA, strideSD, strideRD;
 };
 
@@ -126,6 +126,9 @@ __device__ __forceinline__ void hint_wait(const uint32_t *hint, uint32_t count) 
         asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(hint) : "memory");
 }
 
+__device__ __forceinline__ void named_arrive(int id, int threads) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
 // The thread that waits for the CTA: lane 0 of the last warp.
 __device__ __forceinline__ bool is_waiting_thread() { return threadIdx.x == blockDim.x - 32; }
 
@@ -168,16 +171,21 @@ __device__ __forceinline__ void box_copy(uint32_t dst, const CUtensorMap *map, i
 }
 
 // Rows of bf16 values as digits (flat run index over all rows) by `threads` threads, this one number
-// `tid`; fetch(i, j, v, w) reads runs i and j (negative: none).  No barrier at the end.
+// `tid`; fetch(i, j, v, w) reads runs i and j (negative: none).  Rows of `groups` groups have their aux
+// entries `auxGroups` apart (0: one row).  No barrier at the end.
 template <typename Fetch>
-__device__ __forceinline__ void stage_digits(int runs, int tid, int threads, uint8_t *digits, GroupAux *aux, Fetch fetch) {
+__device__ __forceinline__ void stage_digits(int runs, int tid, int threads, uint8_t *digits, GroupAux *aux, int groups, int auxGroups, Fetch fetch) {
+    auto auxOf = [&](int run) {
+        const int group = run >> 3;
+        return aux + (auxGroups ? group / groups * auxGroups + group % groups : group);
+    };
     // two runs in flight
     for (int base = tid & ~31; base < runs; base += 2 * threads) {
         const int i = base + (tid & 31), j = i + threads;
         uint4 v = make_uint4(0, 0, 0, 0), w = make_uint4(0, 0, 0, 0);
         fetch(i < runs ? i : -1, j < runs ? j : -1, v, w);
-        digits_put(i, i < runs, v, digits, aux);
-        if (base + threads < runs) digits_put(j, j < runs, w, digits, aux);  // the same for the whole warp
+        digits_put(i, i < runs, v, digits, auxOf(i));
+        if (base + threads < runs) digits_put(j, j < runs, w, digits, auxOf(j));  // the same for the whole warp
     }
 }
 // Runs of eight values that other CTAs are still writing as four tagged words each, polled (bounded);
@@ -207,21 +215,22 @@ __device__ __forceinline__ uint32_t ordered_key(float f) {
     return (u >> 31) ? ~u : (u | 0x80000000u);
 }
 
-// The K largest logits, by the whole CTA: one warp polls the CTA's copy of the tagged words and puts
-// their keys into shared memory (0: never taken — -inf or NaN); then four threads per expert count the
-// experts that come before it (higher score, then lower id), a quarter of the keys each.  The loop is
-// short and rolled: this code runs once per launch, where unrolled code is bound by instruction fetch
-// (one warp taking the maximum eight times 2 us, votes per expert unrolled 3 us, this 0.5 us).
-// sKey: four quarters of kKeyQuarter words.  Ends with a CTA barrier.
-constexpr int kKeyQuarter = kMaxExperts / 4 + 4;  // (+4: the quarters' 128-bit reads fall on different banks)
+// The K largest logits, by warps 0..9: one of them polls the CTA's copy of the tagged words and puts
+// their keys into shared memory (0: never taken — -inf or NaN, or past the experts); then two threads
+// per expert count the larger keys, half of them each.  Equal keys leave a place empty; then the count
+// is repeated with the lower id first.  (Dependent instructions cost here, one warp waits 5 cycles for
+// each: taking the maximum eight times cost 2 us, a rolled count with the tie rule in it 1.3 us.)
+// sKey: two halves of kKeyHalf words.  Ends with a barrier of the ten warps.
+constexpr uint32_t kNoRoute = 0xFFFFFFFFu;
+constexpr int kKeyHalf = kMaxExperts / 2 + 4;  // (+4: the halves' 128-bit reads fall on different banks)
 __device__ __forceinline__ void poll_and_rank(const DecodeArgs &a, uint32_t tag, uint32_t *sKey, uint32_t *sIds, float *sScore) {
     const int tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int quarter = ((a.E + 3) / 4 + 3) & ~3;  // keys of a quarter, a multiple of four
+    const int half = ((a.E + 1) / 2 + 15) & ~15;  // keys of a half, a multiple of sixteen
     if (warp == kRankWarp) {
         const unsigned long long *words = a.taggedLogits + (size_t)blockIdx.x * kMaxExperts;
-        for (int base = 0; base < 4 * quarter; base += 64) {
-            const int e = base + 2 * lane;  // (quarters are multiples of four: both words in one)
-            if (e >= 4 * quarter) break;
+        for (int base = 0; base < 2 * half; base += 64) {
+            const int e = base + 2 * lane;  // (both words in one half)
+            if (e >= 2 * half) break;
             unsigned long long w[2] = {0, 0};
             bool ok = false;
             for (uint32_t spins = 0; spins < kBarrierSpinLimit && !ok; ++spins) {
@@ -232,36 +241,58 @@ __device__ __forceinline__ void poll_and_rank(const DecodeArgs &a, uint32_t tag,
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const float v = __uint_as_float((uint32_t)w[i]);
-                sKey[e / quarter * kKeyQuarter + e % quarter + i] = e + i < a.E && v > -INFINITY ? ordered_key(v) : 0u;
+                sKey[(e >= half ? kKeyHalf + e - half : e) + i] = e + i < a.E && v > -INFINITY ? ordered_key(v) : 0u;
             }
         }
     }
     if (tid < 8) {
-        sIds[tid] = 0u;
+        sIds[tid] = kNoRoute;
         sScore[tid] = -INFINITY;
     }
-    __syncthreads();
-    for (int base = 0; base < a.E; base += kFusedThreads / 4) {
-        const int e = base + (tid >> 2), q = tid & 3;
-        const uint32_t mine = e < a.E ? sKey[e / quarter * kKeyQuarter + e % quarter] : 0u;
-        const uint32_t *keys = sKey + q * kKeyQuarter;
-        int rank = 0, before = e - q * quarter;  // of the quarter, this many come before e by id
-#pragma unroll 1
-        for (int o = 0; o < quarter; o += 4, before -= 4) {
-            const uint4 k = *reinterpret_cast<const uint4 *>(keys + o);
-            rank += k.x >= mine + (before > 0 ? 0u : 1u) ? 1 : 0;
-            rank += k.y >= mine + (before > 1 ? 0u : 1u) ? 1 : 0;
-            rank += k.z >= mine + (before > 2 ? 0u : 1u) ? 1 : 0;
-            rank += k.w >= mine + (before > 3 ? 0u : 1u) ? 1 : 0;
-        }
-        rank += __shfl_xor_sync(0xFFFFFFFFu, rank, 1);
-        rank += __shfl_xor_sync(0xFFFFFFFFu, rank, 2);
-        if (q == 0 && mine && rank < a.K) {
+    named_barrier(9, kBigWarps * 32);
+    auto key_of = [&](int e) { return e < a.E ? sKey[e >= half ? kKeyHalf + e - half : e] : 0u; };
+    auto place = [&](int e, uint32_t key, int rank) {
+        if (key && rank < a.K) {
             sIds[rank] = (uint32_t)e;
-            sScore[rank] = __uint_as_float((mine >> 31) ? (mine & 0x7FFFFFFFu) : ~mine);
+            sScore[rank] = __uint_as_float((key >> 31) ? (key & 0x7FFFFFFFu) : ~key);
         }
+    };
+    for (int base = 0; base < a.E && tid < 256; base += 128) {
+        const int e = base + (tid >> 1), h = tid & 1;
+        const uint32_t mine = key_of(e);
+        int n[4] = {0, 0, 0, 0};
+#pragma unroll 1
+        for (int o = 0; o < half; o += 16) {
+            uint4 k[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) k[i] = *reinterpret_cast<const uint4 *>(sKey + h * kKeyHalf + o + 4 * i);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                n[0] += k[i].x > mine ? 1 : 0;
+                n[1] += k[i].y > mine ? 1 : 0;
+                n[2] += k[i].z > mine ? 1 : 0;
+                n[3] += k[i].w > mine ? 1 : 0;
+            }
+        }
+        int rank = (n[0] + n[1]) + (n[2] + n[3]);
+        rank += __shfl_xor_sync(0xFFFFFFFFu, rank, 1);
+        if (h == 0) place(e, mine, rank);
     }
-    __syncthreads();
+    named_barrier(9, kBigWarps * 32);
+    bool empty = false;
+    for (int r = 0; r < a.K; ++r) empty |= sIds[r] == kNoRoute;
+    if (empty) {  // the same for the ten warps
+        named_barrier(9, kBigWarps * 32);
+        if (tid < 8) sIds[tid] = 0u;  // what stays without a route: expert 0, weight 0
+        named_barrier(9, kBigWarps * 32);
+        for (int e = tid; e < a.E; e += kBigWarps * 32) {
+            const uint32_t mine = key_of(e);
+            int rank = 0;
+            for (int o = 0; o < a.E; ++o) rank += key_of(o) >= mine + (o < e ? 0u : 1u) ? 1 : 0;
+            place(e, mine, rank);
+        }
+        named_barrier(9, kBigWarps * 32);
+    }
 }
 
 // The input row travelling inside the kernel's parameters (no host-to-device copy before the
@@ -274,7 +305,7 @@ struct InlineRow {
 __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMaps &maps, const uint16_t *xInline) {
     extern __shared__ __align__(128) uint8_t smemRaw[];
     __shared__ uint32_t sIds[8];
-    __shared__ __align__(16) uint32_t sKey[4 * kKeyQuarter];
+    __shared__ __align__(16) uint32_t sKey[2 * kKeyHalf];
     __shared__ float sWeights[8], sScore[8];
     __shared__ __align__(8) uint64_t sCopyBar[kFusedWarps + kRouterWarps];
     __shared__ uint32_t *sHints;            // this launch's tile counters
@@ -285,9 +316,10 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     const int D = a.D, F = a.F, Fs = a.Fs, K = a.K, E = a.E;
     const int g = lane >> 2, t = lane & 3;
     const int groupsD = D >> 6, groupsF = F >> 6, groupsFs = Fs >> 6;
+    const int auxGroups = (groupsF + 1) & ~1;  // a routed row's aux groups, 16-byte aligned
 
-    // shared memory: x as digits | its group sums | region: x as it is (router), then the shared
-    // activations, then the routed activations | K-split partial sums | routed down rows per expert |
+    // shared memory: x as digits | its group sums | x as it is (router) | region: the shared activations,
+    // then the routed activations | K-split partial sums | routed down rows per expert |
     // slots: five pairs (two tile parts, the tile's scales), two triples of the other six warps
     const uint32_t smem = sm_addr(smemRaw);
     uint8_t *region = smemRaw + a.regionOffset;
@@ -333,46 +365,41 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
 
     // Requests of part `part` of `parts` (along K) of a gate/up tile: one box of eight row pieces per
     // matrix (`pitch` bytes per row in the slot: the box is as wide as the pitch, what it reads past
-    // the part is not used); with the first part the eight rows' scales and biases of both matrices
-    // over the full K (contiguous runs) to `scales`.
-    auto issue_gate_up = [&](const CUtensorMap *gateMap, const CUtensorMap *upMap, int expert, const uint8_t *blob,
-                             const FFExpertOffsets &off, int tile, int part, int parts, uint32_t pitch, uint32_t scales) {
+    // the part is not used); with the first part the tile's scale | bias words over the full K to `sb`.
+    const uint32_t wordsGU = 16u * padded_groups((uint32_t)groupsD), wordsSD = 16u * padded_groups((uint32_t)groupsFs),
+                   wordsRD = 8u * padded_groups((uint32_t)groupsF);
+    auto issue_gate_up = [&](const CUtensorMap *gateMap, const CUtensorMap *upMap, int expert, const uint32_t *words, int tile,
+                             int part, int parts, uint32_t pitch, uint32_t sb) {
         int gb, ge;
-        part_range(groupsD, parts, part, gb, ge);
-        const uint32_t sb = (uint32_t)groupsD * 16u;
-        if (lane == 0) bar_expect(myBar, (ge > gb ? 16u * pitch : 0u) + (part == 0 ? 4u * sb : 0u));
-        __syncwarp();
-        if (lane < 2) {
-            if (ge > gb) box_copy(slot + (uint32_t)lane * 8u * pitch, lane ? upMap : gateMap, gb * 4, tile * 8, expert, myBar);
-        } else if (part == 0 && lane >= 16 && lane < 20) {
-            const uint32_t which = (uint32_t)lane - 16u;
-            const uint32_t src = which == 0 ? off.gateSOff : which == 1 ? off.gateBOff : which == 2 ? off.upSOff : off.upBOff;
-            bulk_copy(scales + which * sb, blob + src + (size_t)tile * sb, sb, myBar);
+        even_range(groupsD, parts, part, gb, ge);
+        if (lane == 0) {
+            bar_expect(myBar, (ge > gb ? 16u * pitch : 0u) + (part == 0 ? 4u * wordsGU : 0u));
+            if (ge > gb) {
+                box_copy(slot, gateMap, gb * 4, tile * 8, expert, myBar);
+                box_copy(slot + 8u * pitch, upMap, gb * 4, tile * 8, expert, myBar);
+            }
+            if (part == 0) bulk_copy(sb, words + (size_t)tile * wordsGU, 4u * wordsGU, myBar);
         }
+        __syncwarp();
     };
-    // Two runs of eight rows (lanes t < 2 account for the first, t >= 2 for the second), scales as
-    // [scales | biases | scales | biases] runs of eight rows: the product over groups [gb, ge) with
-    // the inputs at `dig` / `aux` (already those of this lane's column and row).
-    auto two_runs = [&](uint32_t rows, uint32_t pitch, uint32_t scales, int groups, int gb, int ge, uint32_t dig, uint32_t aux) {
-        const uint32_t run = (uint32_t)groups * 16u;
-        const uint32_t s = scales + (t < 2 ? 0u : 2u * run) + (uint32_t)(g * groups + gb) * 2u;
-        return tile_int4(rows + (uint32_t)g * pitch + 8u * t, rows + (uint32_t)(g + 8) * pitch + 8u * t,
-                         dig + (uint32_t)gb * kDigitGroupBytes + (uint32_t)(g & 3) * 64u + (uint32_t)t * 16u, s, s + run,
-                         aux + 8u * (uint32_t)gb, ge - gb);
+    // A gate/up tile's part: lane (g, t = 0) gets gate row g and up row g.
+    auto gate_up = [&](int part, int parts, uint32_t pitch, uint32_t sb) {
+        int gb, ge;
+        even_range(groupsD, parts, part, gb, ge);
+        const uint32_t s = sb + 4u * ((uint32_t)g * padded_groups((uint32_t)groupsD) + (uint32_t)gb);
+        return tile_int4<false>(slot + (uint32_t)g * pitch + 8u * t, slot + (uint32_t)(g + 8) * pitch + 8u * t,
+                                smem + (uint32_t)gb * kDigitGroupBytes + (uint32_t)(g & 3) * 64u + (uint32_t)t * 16u, s, s + 2u * wordsGU,
+                                sm_addr(xAux) + 8u * (uint32_t)gb, ge - gb);
     };
     auto issue_shared_down = [&](int tile, int part) {
         int gb, ge;
-        part_range(groupsFs, 3, part, gb, ge);
-        const uint32_t sb = (uint32_t)groupsFs * 32u;
-        if (lane == 0) bar_expect(myBar, (ge > gb ? 16u * a.strideSD : 0u) + (part == 0 ? 2u * sb : 0u));
-        __syncwarp();
+        even_range(groupsFs, 3, part, gb, ge);
         if (lane == 0) {
+            bar_expect(myBar, (ge > gb ? 16u * a.strideSD : 0u) + (part == 0 ? 4u * wordsSD : 0u));
             if (ge > gb) box_copy(slot, &maps.m[kMapSharedDown], gb * 4, tile * 16, 0, myBar);
-        } else if (part == 0 && lane >= 16 && lane < 18) {
-            const uint32_t which = (uint32_t)lane - 16u;
-            bulk_copy(tripleBase + 48u * a.strideSD + which * sb,
-                      sh + (which ? a.sharedOff.downBOff : a.sharedOff.downSOff) + (size_t)tile * sb, sb, myBar);
+            if (part == 0) bulk_copy(tripleBase + 48u * a.strideSD, a.sharedScales + (Fs >> 3) * wordsGU + (size_t)tile * wordsSD, 4u * wordsSD, myBar);
         }
+        __syncwarp();
     };
     // A warp's copies and, for the scales, those of the first warp of its pair, quad or triple.  (All
     // warps of a group take the same number of tiles, so one parity serves both barriers.)
@@ -406,7 +433,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     const int partA = warp & 3;
     int tA = warp < kSharedGuWarps ? (warp >> 2) * G + cta : 0x7FFFFFFF;
     auto issue_shared_gate_up = [&](int tile) {
-        issue_gate_up(&maps.m[kMapSharedGate], &maps.m[kMapSharedUp], 0, sh, a.sharedOff, tile, partA, 4, a.strideGUA,
+        issue_gate_up(&maps.m[kMapSharedGate], &maps.m[kMapSharedUp], 0, a.sharedScales, tile, partA, 4, a.strideGUA,
                       scalesOfPair((warp & ~3) >> 1));
     };
     if (tA < tilesSGU) issue_shared_gate_up(tA);
@@ -420,29 +447,37 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
         if (cta == 0) *reinterpret_cast<uint2 *>(a.hints + 2 * ((generation + 2) % kHintSets)) = make_uint2(0u, 0u);
     }
     // the input row, as digits and (for the router) as it is
-    stage_digits(D >> 3, (int)threadIdx.x, kFusedThreads, smemRaw, xAux, [&](int i, int j, uint4 &v, uint4 &w) {
-        if (i >= 0) reinterpret_cast<uint4 *>(region)[i] = v = i == (int)threadIdx.x ? xMine : fetchX(i);
-        if (j >= 0) reinterpret_cast<uint4 *>(region)[j] = w = fetchX(j);
+    stage_digits(D >> 3, (int)threadIdx.x, kFusedThreads, smemRaw, xAux, groupsD, 0, [&](int i, int j, uint4 &v, uint4 &w) {
+        // as fp32 [step of 32 runs][half][lane] for the router's chains
+        float4 *x32 = reinterpret_cast<float4 *>(smemRaw + a.x32Offset);
+        auto keep = [&](int r, const uint4 &q) {
+            x32[2 * r - (r & 31)] = make_float4(__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xFFFF0000u),
+                                                __uint_as_float(q.y << 16), __uint_as_float(q.y & 0xFFFF0000u));
+            x32[2 * r - (r & 31) + 32] = make_float4(__uint_as_float(q.z << 16), __uint_as_float(q.z & 0xFFFF0000u),
+                                                     __uint_as_float(q.w << 16), __uint_as_float(q.w & 0xFFFF0000u));
+        };
+        if (i >= 0) keep(i, v = i == (int)threadIdx.x ? xMine : fetchX(i));
+        if (j >= 0) keep(j, w = fetchX(j));
     });
     __syncthreads();  // the tag is published, too
     const uint32_t tag = sTag;
     for (; tA < tilesSGU; tA += (kSharedGuWarps / 4) * G) {
         wait_tile(warp & ~3);
         warp_stamp(a, 0, 1);
-        int gb, ge;
-        part_range(groupsD, 4, partA, gb, ge);
-        const float v = two_runs(slot, a.strideGUA, scalesOfPair((warp & ~3) >> 1), groupsD, gb, ge, smem, sm_addr(xAux));
+        const float2 v = gate_up(partA, 4, a.strideGUA, scalesOfPair((warp & ~3) >> 1));
         float *mine = partial + warp * 16;
-        if (partA && !(t & 1)) mine[(t >> 1) * 8 + g] = v;
+        if (partA && t == 0) {
+            mine[g] = v.x;
+            mine[8 + g] = v.y;
+        }
         named_barrier(1 + (warp >> 2), 128);  // every part is read, too: the slots are free
         const int next = tA + (kSharedGuWarps / 4) * G;
         if (next < tilesSGU) issue_shared_gate_up(next);
         if (!partA) {
-            const float *m = mine + (t >> 1) * 8 + g;
-            const float sum = ((v + m[16]) + m[32]) + m[48];
-            const float up = __shfl_down_sync(0xFFFFFFFFu, sum, 2);
+            const float *m = mine + g;
+            const float gate = ((v.x + m[16]) + m[32]) + m[48], up = ((v.y + m[24]) + m[40]) + m[56];
             // two activations of a tile per tagged word, the odd neighbour's by shuffle
-            const uint32_t act = f2bf(gelu_tanh(bf16_round(sum)) * bf16_round(up));
+            const uint32_t act = f2bf(gelu_tanh(bf16_round(gate)) * bf16_round(up));
             const uint32_t two = act | (__shfl_down_sync(0xFFFFFFFFu, act, 4) << 16);
             if (t == 0 && !(g & 1)) st_tagged(a.taggedShared + ((tA * 8 + g) >> 1), tag, two);
             if (lane == 0) hint_add(sHints);
@@ -454,15 +489,16 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
         slot_wait(routerBar, routerParity, a.errorFlag);
         warp_stamp(a, 0, 1);
         // lane l chains fmaf over elements [256 i + 8 l, +8): the order of every router kernel
-        const uint32_t xRow = sm_addr(region);
+        const uint32_t xRow = smem + a.x32Offset;
         const int chunks = D >> 3;
         auto chain = [&](auto scaled) {
             float acc = 0.0f;
-            auto run = [&](const uint4 &wv, const uint4 &xv, const uint4 &sv) {
-                const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w}, xx[4] = {xv.x, xv.y, xv.z, xv.w}, ss[4] = {sv.x, sv.y, sv.z, sv.w};
+            auto run = [&](const uint4 &wv, const uint4 &lo, const uint4 &hi, const uint4 &sv) {
+                const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w}, ss[4] = {sv.x, sv.y, sv.z, sv.w};
+                const uint32_t xx[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    float x0 = __uint_as_float(xx[k] << 16), x1 = __uint_as_float(xx[k] & 0xFFFF0000u);
+                    float x0 = __uint_as_float(xx[2 * k]), x1 = __uint_as_float(xx[2 * k + 1]);
                     if (decltype(scaled)::value) {
                         x0 = x0 * __uint_as_float(ss[k] << 16);
                         x1 = x1 * __uint_as_float(ss[k] & 0xFFFF0000u);
@@ -471,21 +507,24 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
                     acc = fmaf(__uint_as_float(ww[k] & 0xFFFF0000u), x1, acc);
                 }
             };
-            // four steps' loads ahead of their multiply-adds; steps past the row add 0 * 0
+            // a short loop, the next step's loads ahead of this step's chain
+            auto load = [&](int c, uint4 &wv, uint4 &lo, uint4 &hi, uint4 &sv) {
+                wv = lds128(slot + 16u * (uint32_t)c);
+                lo = lds128(xRow + 16u * (uint32_t)(2 * c - (c & 31)));
+                hi = lds128(xRow + 16u * (uint32_t)(2 * c - (c & 31) + 32));
+                sv = decltype(scaled)::value ? lds128(slot + (uint32_t)D * 2u + 16u * (uint32_t)c) : make_uint4(0, 0, 0, 0);
+            };
+            uint4 wv, lo, hi, sv;
+            load(min(lane, chunks - 1), wv, lo, hi, sv);
 #pragma unroll 1
-            for (int c = lane; c < chunks + 31; c += 128) {
-                uint4 wv[4], xv[4], sv[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    wv[i] = xv[i] = sv[i] = make_uint4(0, 0, 0, 0);
-                    if (c + 32 * i < chunks) {
-                        wv[i] = lds128(slot + 16u * (uint32_t)(c + 32 * i));
-                        xv[i] = lds128(xRow + 16u * (uint32_t)(c + 32 * i));
-                        if (decltype(scaled)::value) sv[i] = lds128(slot + (uint32_t)D * 2u + 16u * (uint32_t)(c + 32 * i));
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) run(wv[i], xv[i], sv[i]);
+            for (int c = lane; c < chunks; c += 32) {
+                uint4 wn, ln, hn, sn;
+                load(min(c + 32, chunks - 1), wn, ln, hn, sn);
+                run(wv, lo, hi, sv);
+                wv = wn;
+                lo = ln;
+                hi = hn;
+                sv = sn;
             }
             return acc;
         };
@@ -514,7 +553,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
         tileB = tile - kB * tilesF;
     };
     if (tB < tilesRouted) place(tB);
-    if (K > 0) {
+    if (K > 0 && warp < kBigWarps) {
         if (!a.idsIn) {
             poll_and_rank(a, tag, sKey, sIds, sScore);
         } else {
@@ -532,14 +571,15 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
                 sIds[threadIdx.x] = id;
                 sWeights[threadIdx.x] = w;
             }
-            __syncthreads();
+            named_barrier(9, kBigWarps * 32);
         }
+        named_arrive(10, kFusedThreads);  // for the warps of the shared down rows
     }
     stamp(a, 2);
     stamp(a, 3);
     auto issue_routed_gate_up = [&]() {
-        issue_gate_up(&maps.m[kMapRoutedGate], &maps.m[kMapRoutedUp], (int)sIds[kB], a.experts + (size_t)sIds[kB] * a.stride, a.off,
-                      tileB, warp & 1, 2, a.strideGU, scalesOfPair(pair));
+        issue_gate_up(&maps.m[kMapRoutedGate], &maps.m[kMapRoutedUp], (int)sIds[kB], a.scales + (size_t)sIds[kB] * a.scaleStride, tileB,
+                      warp & 1, 2, a.strideGU, scalesOfPair(pair));
     };
     if (tB < tilesRouted) issue_routed_gate_up();
     if (warp < kBigWarps) warp_stamp(a, 1, 0);
@@ -565,8 +605,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
 
     // ---------------- phase B: routed gate/up/GeGLU (warps 0..9), shared down rows (10..15) ----------
     // Routed down task j of a round (16 / pairsK row tiles of eight rows, pairsK expert pairs each), tasks
-    // in the order of warps 10..15, 0..9: the shared down warps are done first.  Lanes 0, 1 copy the two
-    // experts' rows (one box each), lanes 16..19 their scale and bias runs.
+    // in the order of warps 10..15, 0..9: the shared down warps are done first.
     const int tilesRD = D >> 3, pairsK = (K + 1) >> 1, perRound = pairsK ? kFusedWarps / pairsK : 1;
     const int task = warp >= kBigWarps ? warp - kBigWarps : warp + (kFusedWarps - kBigWarps);
     const int myTile = pairsK ? task / pairsK : 0, myPair = pairsK ? task - myTile * pairsK : 0;
@@ -574,34 +613,36 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     auto tileOf = [&](int round) { return cta + G * (round * perRound + myTile); };
     auto has_task = [&](int round) { return K > 0 && myTile < perRound && tileOf(round) < tilesRD; };
     auto issue_routed_down = [&](int tile) {
-        const uint32_t sb = (uint32_t)groupsF * 16u;
-        if (lane == 0) bar_expect(myBar, 16u * a.strideRD + 4u * sb);
-        __syncwarp();
-        if (lane < 2) {
-            box_copy(downSlot + (uint32_t)lane * 8u * a.strideRD, &maps.m[kMapRoutedDown], 0, tile * 8, (int)sIds[lane ? eHi : eLo], myBar);
-        } else if (lane >= 16 && lane < 20) {
-            const uint32_t which = (uint32_t)lane - 16u;
-            const uint8_t *blob = a.experts + (size_t)sIds[which < 2 ? eLo : eHi] * a.stride;
-            bulk_copy(downSlot + 16u * a.strideRD + which * sb, blob + ((which & 1) ? a.off.downBOff : a.off.downSOff) + (size_t)tile * sb,
-                      sb, myBar);
+        // the two experts' rows (one box each) and scale words
+        if (lane == 0) {
+            bar_expect(myBar, 16u * a.strideRD + 8u * wordsRD);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const uint32_t id = sIds[i ? eHi : eLo];
+                box_copy(downSlot + (uint32_t)i * 8u * a.strideRD, &maps.m[kMapRoutedDown], 0, tile * 8, (int)id, myBar);
+                bulk_copy(downSlot + 16u * a.strideRD + (uint32_t)i * 4u * wordsRD,
+                          a.scales + (size_t)id * a.scaleStride + (F >> 3) * wordsGU + (size_t)tile * wordsRD, 4u * wordsRD, myBar);
+            }
         }
+        __syncwarp();
     };
     if (warp >= kBigWarps && sh) {
         // the shared activations, staged by the six warps that use them
         if (is_waiting_thread()) hint_wait(sHints, (uint32_t)tilesSGU);
         named_barrier(8, (kFusedWarps - kBigWarps) * 32);
-        stage_digits(Fs >> 3, (int)threadIdx.x - kBigWarps * 32, (kFusedWarps - kBigWarps) * 32, region, regionAux,
+        stage_digits(Fs >> 3, (int)threadIdx.x - kBigWarps * 32, (kFusedWarps - kBigWarps) * 32, region, regionAux, groupsFs, 0,
                      [&](int i, int j, uint4 &v, uint4 &w) { fetch_tagged(a.taggedShared, tag, i, j, v, w, a.errorFlag); });
         named_barrier(8, (kFusedWarps - kBigWarps) * 32);
     }
     for (; tB < tilesRouted; tB += (kBigWarps / 2) * G) {
         wait_tile(warp & ~1);
         warp_stamp(a, 1, 1);
-        int gb, ge;
-        part_range(groupsD, 2, warp & 1, gb, ge);
-        const float v = two_runs(slot, a.strideGU, scalesOfPair(pair), groupsD, gb, ge, smem, sm_addr(xAux));
+        const float2 v = gate_up(warp & 1, 2, a.strideGU, scalesOfPair(pair));
         float *mine = partial + warp * 16;
-        if ((warp & 1) && !(t & 1)) mine[(t >> 1) * 8 + g] = v;
+        if ((warp & 1) && t == 0) {
+            mine[g] = v.x;
+            mine[8 + g] = v.y;
+        }
         named_barrier(1 + pair, 64);
         const int next = tB + (kBigWarps / 2) * G;
         if (next < tilesRouted) {
@@ -611,9 +652,8 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
         if (!(warp & 1)) {
             // the tile's eight activations are one run of the staged row: four tagged words,
             // written by the lanes t == 0 of even g (the odd neighbour's value comes by shuffle)
-            const float sum = v + mine[16 + (t >> 1) * 8 + g];
-            const float up = __shfl_down_sync(0xFFFFFFFFu, sum, 2);
-            const uint32_t act = f2bf(gelu_tanh(sum) * up);
+            const float gate = v.x + mine[16 + g], up = v.y + mine[24 + g];
+            const uint32_t act = f2bf(gelu_tanh(gate) * up);
             const uint32_t two = act | (__shfl_down_sync(0xFFFFFFFFu, act, 4) << 16);
             if (t == 0 && !(g & 1)) st_tagged(a.taggedActs + ((tB * 8 + g) >> 1), tag, two);
             if (lane == 0) hint_add(sHints + 1);
@@ -624,30 +664,40 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
         wait_tile(kBigWarps + 3 * triple);
         warp_stamp(a, 1, 1);
         int gb, ge;
-        part_range(groupsFs, 3, part3, gb, ge);
-        const uint32_t s = tripleBase + 48u * a.strideSD + (uint32_t)((t < 2 ? g : g + 8) * groupsFs + gb) * 2u;
-        const float v = tile_int4(slot + (uint32_t)g * a.strideSD + 8u * t, slot + (uint32_t)(g + 8) * a.strideSD + 8u * t,
-                                  sm_addr(region) + (uint32_t)gb * kDigitGroupBytes + (uint32_t)(g & 3) * 64u + (uint32_t)t * 16u, s,
-                                  s + (uint32_t)groupsFs * 32u, sm_addr(regionAux) + 8u * (uint32_t)gb, ge - gb);
+        even_range(groupsFs, 3, part3, gb, ge);
+        const uint32_t padded = padded_groups((uint32_t)groupsFs), s = tripleBase + 48u * a.strideSD + 4u * ((uint32_t)g * padded + (uint32_t)gb);
+        const float2 v = tile_int4<false>(slot + (uint32_t)g * a.strideSD + 8u * t, slot + (uint32_t)(g + 8) * a.strideSD + 8u * t,
+                                          sm_addr(region) + (uint32_t)gb * kDigitGroupBytes + (uint32_t)(g & 3) * 64u + (uint32_t)t * 16u, s,
+                                          s + 32u * padded, sm_addr(regionAux) + 8u * (uint32_t)gb, ge - gb);
         float *mine = partial + warp * 16;
-        if (part3 && !(t & 1)) mine[(t >> 1) * 8 + g] = v;
+        if (part3 && t == 0) {
+            mine[g] = v.x;
+            mine[8 + g] = v.y;
+        }
         named_barrier(6 + triple, 96);
         const int next = tSD + 2 * G;
         if (next < tilesSD) issue_shared_down(next, part3);
         if (!part3) {
-            const float *m = mine + (t >> 1) * 8 + g;
-            const uint32_t r = f2bf((v + m[16]) + m[32]);  // row 8 (t / 2) + g, valid in even t
-            const int row = tSD * 16 + (t >> 1) * 8 + g;
+            const float *m = mine + g;
+            const uint32_t r0 = f2bf((v.x + m[16]) + m[32]), r1 = f2bf((v.y + m[24]) + m[40]);
+            const int row = tSD * 16 + g;  // and row + 8
             if (K > 0) {
                 // read as the residual of the routed rows in phase C: tagged words of two rows
-                const uint32_t two = r | (__shfl_down_sync(0xFFFFFFFFu, r, 4) << 16);
-                if (!(t & 1) && !(g & 1)) st_tagged(a.taggedH1 + (row >> 1), tag, two);
-            } else if (!(t & 1)) {
-                a.y[row] = (uint16_t)r;
+                const uint32_t two0 = r0 | (__shfl_down_sync(0xFFFFFFFFu, r0, 4) << 16);
+                const uint32_t two1 = r1 | (__shfl_down_sync(0xFFFFFFFFu, r1, 4) << 16);
+                if (t == 0 && !(g & 1)) {
+                    st_tagged(a.taggedH1 + (row >> 1), tag, two0);
+                    st_tagged(a.taggedH1 + ((row + 8) >> 1), tag, two1);
+                }
+            } else if (t == 0) {
+                a.y[row] = (uint16_t)r0;
+                a.y[row + 8] = (uint16_t)r1;
             }
         }
         named_barrier(6 + triple, 96);
     }
+    // warps 10..15 meet the routes only here: the shared down rows need none
+    if (K > 0 && warp >= kBigWarps) named_barrier(10, kFusedThreads);
     if (has_task(0)) issue_routed_down(tileOf(0));
     warp_stamp(a, 1, 2);
     stamp(a, 4);
@@ -678,7 +728,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
         else residual = a.residual ? bf2f(__ldcg(a.residual + row)) : 0.0f;
     };
     ask_residual(0);
-    stage_digits(K * (F >> 3), (int)threadIdx.x, kFusedThreads, region, regionAux,
+    stage_digits(K * (F >> 3), (int)threadIdx.x, kFusedThreads, region, regionAux, groupsF, auxGroups,
                  [&](int i, int j, uint4 &v, uint4 &w) { fetch_tagged(a.taggedActs, tag, i, j, v, w, a.errorFlag); });
     __syncthreads();
     for (int round = 0; cta + G * round * perRound < tilesRD; ++round) {
@@ -687,9 +737,11 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
             warp_stamp(a, 2, 1);
             // rows 0..7 of the tile: expert eLo, columns 0..3; rows 8..15: expert eHi, columns 4..7
             const int mine = t < 2 ? eLo : eHi, column = g < 4 ? eLo : eHi;
-            const float v = two_runs(downSlot, a.strideRD, downSlot + 16u * a.strideRD, groupsF, 0, groupsF,
-                                     sm_addr(region) + (uint32_t)(column * groupsF) * kDigitGroupBytes,
-                                     sm_addr(regionAux) + 8u * (uint32_t)(mine * groupsF));
+            const uint32_t s = downSlot + 16u * a.strideRD + 4u * ((t < 2 ? 0u : wordsRD) + (uint32_t)g * padded_groups((uint32_t)groupsF));
+            const float v = tile_int4<true>(downSlot + (uint32_t)g * a.strideRD + 8u * t, downSlot + (uint32_t)(g + 8) * a.strideRD + 8u * t,
+                                            sm_addr(region) + (uint32_t)(column * groupsF) * kDigitGroupBytes + (uint32_t)(g & 3) * 64u + (uint32_t)t * 16u,
+                                            s, s, sm_addr(regionAux) + 8u * (uint32_t)(mine * auxGroups), groupsF)
+                                .x;
             if (!(t & 1) && (t == 0 || eHi > eLo)) downRows[(myTile * 8 + mine) * 8 + g] = v;
         }
         __syncthreads();
@@ -754,8 +806,57 @@ k_decode_fused_inline_x(const DecodeArgs a, const __grid_constant__ DecodeMaps m
     decode_body(a, maps, reinterpret_cast<const uint16_t *>(&row));
 }
 
+// Scale | bias words of `count` blobs, tile by tile: [F/8 gate/up tiles][8 gate rows, 8 up rows] of
+// padded_groups(D/64) words, then [D down rows] of padded_groups(F/64).
+static uint64_t scale_words(uint32_t D, uint32_t F) {
+    return (uint64_t)(F / 8) * 16 * padded_groups(D / 64) + (uint64_t)D * padded_groups(F / 64);
+}
+__global__ void __launch_bounds__(256)
+k_pack_scales(const uint8_t *blobs, uint64_t stride, FFExpertOffsets off, uint32_t D, uint32_t F, uint32_t *out, uint64_t words) {
+    const uint8_t *blob = blobs + blockIdx.y * stride;
+    const uint32_t gD = D / 64, gF = F / 64, pD = padded_groups(gD), pF = padded_groups(gF);
+    const uint64_t gateUp = (uint64_t)(F / 8) * 16 * pD;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += (uint64_t)gridDim.x * blockDim.x) {
+        uint32_t g, row, groups, sOff, bOff;
+        if (i < gateUp) {
+            const uint32_t r = (uint32_t)(i / pD), in = r & 15u;  // rows of a tile: 8 gate, 8 up
+            g = (uint32_t)(i % pD);
+            row = (r >> 4) * 8u + (in & 7u);
+            groups = gD;
+            sOff = in < 8u ? off.gateSOff : off.upSOff;
+            bOff = in < 8u ? off.gateBOff : off.upBOff;
+        } else {
+            g = (uint32_t)((i - gateUp) % pF);
+            row = (uint32_t)((i - gateUp) / pF);  // down rows stay in order: tiles of any height are contiguous
+            groups = gF;
+            sOff = off.downSOff;
+            bOff = off.downBOff;
+        }
+        uint32_t word = 0u;
+        if (g < groups) {
+            const size_t at = ((size_t)row * groups + g) * 2;
+            word = (uint32_t)*reinterpret_cast<const uint16_t *>(blob + sOff + at) |
+                   ((uint32_t)*reinterpret_cast<const uint16_t *>(blob + bOff + at) << 16);
+        }
+        out[blockIdx.y * words + i] = word;
+    }
+}
+// Lays out `count` blobs' scales; *out is allocated when null (its size depends on the shape alone).
+bool pack_scales(FFContext *ctx, const uint8_t *blobs, uint64_t stride, const FFExpertOffsets &off, uint32_t D, uint32_t F,
+                 uint32_t count, uint32_t **out, const char **error) {
+    const uint64_t words = scale_words(D, F);
+    if (!*out) {
+        FF_CUDA_OK(cudaMalloc(reinterpret_cast<void **>(out), words * count * 4), error);
+        ctx->scratchBytes += words * count * 4;
+    }
+    k_pack_scales<<<dim3((unsigned)((words + 1023) / 1024), count), 256>>>(blobs, stride, off, D, F, *out, words);
+    FF_CUDA_OK(cudaGetLastError(), error);
+    FF_CUDA_OK(cudaStreamSynchronize(nullptr), error);
+    return true;
+}
+
 struct FusedLayout {
-    uint32_t regionOffset, regionAux, partialOffset, downOffset, slotsOffset, rowsBytes, pairBytes, tripleBytes, downBytes;
+    uint32_t x32Offset, regionOffset, regionAux, partialOffset, downOffset, slotsOffset, rowsBytes, pairBytes, tripleBytes, downBytes;
     uint32_t strideGU, strideGUA, strideSD, strideRD;
     size_t total;
 };
@@ -764,22 +865,28 @@ static FusedLayout fused_layout(const FFConfig &c) {
     const uint32_t D = c.d, F = c.f, Fs = c.sharedF, K = c.topK;
     const uint32_t groupsD = D / 64, groupsF = F / 64, groupsFs = Fs / 64;
     auto up128 = [](uint32_t v) { return (v + 127u) & ~127u; };
+    auto longest = [](uint32_t groups, int parts) {  // groups of the first (longest) part
+        int begin, end;
+        even_range((int)groups, parts, 0, begin, end);
+        return (uint32_t)(end - begin);
+    };
     FusedLayout l{};
-    l.strideGU = piece_stride(((groupsD + 1) / 2) * 32);   // routed tiles: K halves
-    l.strideGUA = piece_stride(((groupsD + 3) / 4) * 32);  // shared tiles: K quarters
-    l.strideSD = Fs ? piece_stride(((groupsFs + 2) / 3) * 32) : 32;
+    l.strideGU = piece_stride(longest(groupsD, 2) * 32);   // routed tiles: K halves
+    l.strideGUA = piece_stride(longest(groupsD, 4) * 32);  // shared tiles: K quarters
+    l.strideSD = Fs ? piece_stride(longest(groupsFs, 3) * 32) : 32;
     l.strideRD = piece_stride(groupsF * 32);
-    l.regionOffset = up128(D * 4 + groupsD * (uint32_t)sizeof(GroupAux));
-    // the region holds x (bf16), then the shared activations' digits, then K (even) rows of routed ones
+    l.x32Offset = up128(D * 4 + groupsD * (uint32_t)sizeof(GroupAux));
+    l.regionOffset = up128(l.x32Offset + (D + 255) / 256 * 1024);
+    // the region holds the shared activations' digits, then K (even) rows of routed ones
     const uint32_t rows = (K + 1) / 2 * 2;
-    l.regionAux = l.regionOffset + std::max({D * 2, Fs * 4, rows * F * 4});
-    l.partialOffset = up128(l.regionAux + (uint32_t)sizeof(GroupAux) * std::max(groupsFs, rows * groupsF));
+    l.regionAux = l.regionOffset + std::max(Fs * 4, rows * F * 4);
+    l.partialOffset = up128(l.regionAux + (uint32_t)sizeof(GroupAux) * (std::max(groupsFs, rows * ((groupsF + 1) & ~1u)) + 2));
     l.downOffset = l.partialOffset + kFusedWarps * 16 * 4;
     l.slotsOffset = up128(l.downOffset + kFusedWarps * 8 * 8 * 4);
-    l.downBytes = up128(16 * l.strideRD + 4 * 16 * groupsF);
+    l.downBytes = up128(16 * l.strideRD + 64 * padded_groups(groupsF));
     l.rowsBytes = up128(std::max({16 * l.strideGU, 16 * l.strideGUA, l.downBytes, D * 4}));
-    l.pairBytes = up128(2 * l.rowsBytes + 4 * 16 * groupsD);
-    l.tripleBytes = up128(std::max(Fs ? 48 * l.strideSD + 2 * 32 * groupsFs : 0u, 3 * l.downBytes));
+    l.pairBytes = up128(2 * l.rowsBytes + 64 * padded_groups(groupsD));
+    l.tripleBytes = up128(std::max(Fs ? 48 * l.strideSD + 64 * padded_groups(groupsFs) : 0u, 3 * l.downBytes));
     l.total = (size_t)l.slotsOffset + (size_t)(kBigWarps / 2) * l.pairBytes + 2 * (size_t)l.tripleBytes;
     return l;
 }
@@ -812,11 +919,10 @@ bool launch_decode_fused(FFContext *ctx, const LayerStore &L, const uint16_t *x,
     a.routerScale = L.routerScale;
     a.gain = L.gain;
     a.logitBias = L.logitBias;
-    a.experts = L.experts;
-    a.stride = L.stride;
-    a.off = L.off;
+    a.scales = L.routedScales;
+    a.scaleStride = scale_words(c.d, c.f);
+    a.sharedScales = L.sharedScales;
     a.shared = withShared ? L.shared : nullptr;
-    a.sharedOff = L.sharedOff;
     a.x = x;
     a.residual = residual;
     a.idsIn = idsIn;
@@ -880,6 +986,7 @@ bool launch_decode_fused(FFContext *ctx, const LayerStore &L, const uint16_t *x,
     }
     static thread_local DecodeMaps maps;
     memcpy(maps.m, L.decodeMap, sizeof(maps.m));
+    a.x32Offset = lay.x32Offset;
     a.regionOffset = lay.regionOffset;
     a.regionAux = lay.regionAux;
     a.partialOffset = lay.partialOffset;

@@ -35,6 +35,7 @@ struct alignas(8) GroupAux {
 // nibbles of its eight packed bytes.
 template <bool INT8 = false>
 __device__ __forceinline__ void digits_put(int run, bool valid, const uint4 &v, uint8_t *digits, GroupAux *aux) {
+    // (aux: the run's group's entry)
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     float x[8];
     uint32_t top = 0;
@@ -78,7 +79,7 @@ __device__ __forceinline__ void digits_put(int run, bool valid, const uint4 &v, 
         *reinterpret_cast<uint32_t *>(at + 64) = __byte_perm(h0, h1, 0x5410);
         *reinterpret_cast<uint32_t *>(at) = __byte_perm(h0, h1, 0x7632);
     }
-    if ((run & 7) == 0) aux[run >> 3] = GroupAux{e == 255 ? __int_as_float(0x7FFFFFFF) : __int_as_float((127 - E) << 23), sum};
+    if ((run & 7) == 0) *aux = GroupAux{e == 255 ? __int_as_float(0x7FFFFFFF) : __int_as_float((127 - E) << 23), sum};
 }
 
 // (shared-memory addresses: the tile function is not inlined, so a pointer would be a generic one)
@@ -92,35 +93,45 @@ __device__ __forceinline__ uint4 lds128(uint32_t a) {
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
     return v;
 }
-__device__ __forceinline__ float lds_bf16(uint32_t a) {
-    uint16_t v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
-    return bf2f(v);
+// Scales and biases as the kernels read them: u32 scale | bias << 16 per (row, group), the groups of a
+// row padded to a multiple of four (ff_load_layer lays them out once, tile by tile).
+__host__ __device__ inline uint32_t padded_groups(uint32_t groups) { return (groups + 3u) & ~3u; }
+// Groups [begin, end) of part p when `groups` are split into `parts` runs of even length (64-bit reads of
+// two groups' scales).
+__host__ __device__ inline void even_range(int groups, int parts, int p, int &begin, int &end) {
+    const int per = ((groups + parts - 1) / parts + 1) & ~1;
+    begin = min(groups, p * per);
+    end = min(groups, begin + per);
 }
 
-// N consecutive groups of a 16-row tile: lo / hi this lane's eight packed bytes of tile rows g and g + 8
-// (g = lane / 4, t = lane % 4: bytes [8 t, + 8) of the group's 32; next group 32 bytes on), dig this
-// lane's 16 digit bytes of MMA column g; all shared-memory addresses.  The lane accounts for row g
-// (t < 2) or g + 8 (t >= 2), two neighbouring columns' digits joined (t even: the two high digits):
-// acc += s unit (digit sums), accBias += b sum, with s, b this lane's row's scales and biases and aux
-// its input's groups.
-template <int N>
-__device__ __forceinline__ void groups_int4(uint32_t lo, uint32_t hi, uint32_t dig, uint32_t s, uint32_t b, uint32_t aux,
-                                            bool lower, float &acc, float &accBias) {
-    uint2 wl[N], wh[N], ax[N];
-    uint4 x[N];
-    float sc[N], bi[N];
+// N consecutive groups of a 16-row tile (N even, or the last ones): lo / hi this lane's eight packed
+// bytes of tile rows g and g + 8 (g = lane / 4, t = lane % 4: bytes [8 t, + 8) of the group's 32; next
+// group 32 bytes on), dig this lane's 16 digit bytes of MMA column g, sb0 / sb1 the scale | bias words of
+// its row(s), aux its input's groups; all shared-memory addresses.
+//   PAIR = false: one input, its digits in columns 0..3 (lanes g < 4 load them): lane t = 0 (high digits)
+//     and 1 (low) account for both rows, acc[0] and acc[1].
+//   PAIR = true: two inputs, columns 0..3 and 4..7: lanes t < 2 account for row g with the first, t >= 2
+//     for row g + 8 with the second, acc[0]; aux and sb0 are that row's.
+// Shared-memory bandwidth bounds this (512 bytes of codes and 256 or 512 of digits per group), so the
+// small operands come two groups at a time.
+template <int N, bool PAIR>
+__device__ __forceinline__ void groups_int4(uint32_t lo, uint32_t hi, uint32_t dig, uint32_t sb0, uint32_t sb1, uint32_t aux,
+                                            bool useDigits, bool lower, float (&acc)[2], float (&accBias)[2]) {
+    constexpr int N2 = (N + 1) / 2;
+    uint2 wl[N], wh[N], s0[N2], s1[N2];
+    uint4 x[N], ax[N2];
 #pragma unroll
     for (int u = 0; u < N; ++u) {
         wl[u] = lds64(lo + 32 * u);
         wh[u] = lds64(hi + 32 * u);
-        x[u] = lds128(dig + kDigitGroupBytes * u);
+        x[u] = make_uint4(0, 0, 0, 0);
+        if (PAIR || useDigits) x[u] = lds128(dig + kDigitGroupBytes * u);
     }
 #pragma unroll
-    for (int u = 0; u < N; ++u) {
-        ax[u] = lds64(aux + 8 * u);
-        sc[u] = lds_bf16(s + 2 * u);
-        bi[u] = lds_bf16(b + 2 * u);
+    for (int u = 0; u < N2; ++u) {
+        ax[u] = lds128(aux + 16 * u);
+        s0[u] = lds64(sb0 + 8 * u);
+        if (!PAIR) s1[u] = lds64(sb1 + 8 * u);
     }
     int d[N][4];
 #pragma unroll
@@ -133,34 +144,42 @@ __device__ __forceinline__ void groups_int4(uint32_t lo, uint32_t hi, uint32_t d
         mma_u8s8(d[u], wl[u].x & 0xF0F0F0F0u, wh[u].x & 0xF0F0F0F0u, wl[u].y & 0xF0F0F0F0u, wh[u].y & 0xF0F0F0F0u, x[u].z, x[u].w);
 #pragma unroll
     for (int u = 0; u < N; ++u) {
-        const int v = (lower ? d[u][0] : d[u][2]) * 256 + (lower ? d[u][1] : d[u][3]);
-        acc = fmaf(sc[u] * __uint_as_float(ax[u].x), (float)v, acc);
-        accBias = fmaf(bi[u], __uint_as_float(ax[u].y), accBias);
+        const float unit = __uint_as_float((u & 1) ? ax[u >> 1].z : ax[u >> 1].x), sum = __uint_as_float((u & 1) ? ax[u >> 1].w : ax[u >> 1].y);
+        const uint32_t w0 = (u & 1) ? s0[u >> 1].y : s0[u >> 1].x;
+        const int v0 = PAIR ? (lower ? d[u][0] : d[u][2]) * 256 + (lower ? d[u][1] : d[u][3]) : d[u][0] * 256 + d[u][1];
+        acc[0] = fmaf(__uint_as_float(w0 << 16) * unit, (float)v0, acc[0]);
+        accBias[0] = fmaf(__uint_as_float(w0 & 0xFFFF0000u), sum, accBias[0]);
+        if (!PAIR) {
+            const uint32_t w1 = (u & 1) ? s1[u >> 1].y : s1[u >> 1].x;
+            acc[1] = fmaf(__uint_as_float(w1 << 16) * unit, (float)(d[u][2] * 256 + d[u][3]), acc[1]);
+            accBias[1] = fmaf(__uint_as_float(w1 & 0xFFFF0000u), sum, accBias[1]);
+        }
     }
 }
 
-// `n` consecutive groups of a 16-row tile against one input per row half: the dot product of row g in
-// lane (g, t = 0) and of row g + 8 in lane (g, t = 2) (other lanes hold parts).  Groups are taken in
-// ascending order.
-static __device__ __noinline__ float tile_int4(uint32_t lo, uint32_t hi, uint32_t dig, uint32_t s, uint32_t b, uint32_t aux, int n) {
-    const bool lower = (threadIdx.x & 3) < 2;
-    float acc = 0.0f, accBias = 0.0f;
+// `n` consecutive groups of a 16-row tile, in ascending order.  PAIR = false: x = row g, y = row g + 8 in
+// lanes t = 0; PAIR = true: x = row g in lanes t = 0, row g + 8 in lanes t = 2 (other lanes hold parts).
+template <bool PAIR>
+static __device__ __noinline__ float2 tile_int4(uint32_t lo, uint32_t hi, uint32_t dig, uint32_t sb0, uint32_t sb1, uint32_t aux, int n) {
+    const bool lower = (threadIdx.x & 3) < 2, useDigits = (threadIdx.x & 31) < 16;
+    float acc[2] = {0.0f, 0.0f}, accBias[2] = {0.0f, 0.0f};
 #pragma unroll 1
     for (; n >= 4; n -= 4) {
-        groups_int4<4>(lo, hi, dig, s, b, aux, lower, acc, accBias);
+        groups_int4<4, PAIR>(lo, hi, dig, sb0, sb1, aux, useDigits, lower, acc, accBias);
         lo += 128;
         hi += 128;
         dig += 4 * kDigitGroupBytes;
-        s += 8;
-        b += 8;
+        sb0 += 16;
+        sb1 += 16;
         aux += 32;
     }
     // the rest in one batch, so that its latencies overlap
-    if (n == 3) groups_int4<3>(lo, hi, dig, s, b, aux, lower, acc, accBias);
-    else if (n == 2) groups_int4<2>(lo, hi, dig, s, b, aux, lower, acc, accBias);
-    else if (n == 1) groups_int4<1>(lo, hi, dig, s, b, aux, lower, acc, accBias);
-    const float low = __shfl_xor_sync(0xFFFFFFFFu, acc, 1);
-    return fmaf(acc, 65536.0f, low) + accBias;
+    if (n == 3) groups_int4<3, PAIR>(lo, hi, dig, sb0, sb1, aux, useDigits, lower, acc, accBias);
+    else if (n == 2) groups_int4<2, PAIR>(lo, hi, dig, sb0, sb1, aux, useDigits, lower, acc, accBias);
+    else if (n == 1) groups_int4<1, PAIR>(lo, hi, dig, sb0, sb1, aux, useDigits, lower, acc, accBias);
+    const float x = fmaf(acc[0], 65536.0f, __shfl_xor_sync(0xFFFFFFFFu, acc[0], 1)) + accBias[0];
+    const float y = PAIR ? 0.0f : fmaf(acc[1], 65536.0f, __shfl_xor_sync(0xFFFFFFFFu, acc[1], 1)) + accBias[1];
+    return make_float2(x, y);
 }
 
 }  // namespace ff

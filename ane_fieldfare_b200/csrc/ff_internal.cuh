@@ -109,6 +109,7 @@ struct LayerStore {
     FFExpertOffsets off{};
     uint8_t *shared = nullptr;  // gate, up, down of the shared FFN in the same nine-part order
     FFExpertOffsets sharedOff{};
+    uint32_t *routedScales = nullptr, *sharedScales = nullptr;  // scale | bias words, tile by tile (pack_scales)
     uint16_t *routerW = nullptr;
     uint16_t *routerScale = nullptr;
     uint16_t *gain = nullptr;
@@ -250,6 +251,8 @@ bool launch_dequant_probe(FFContext *ctx, const uint8_t *w, const uint16_t *s, c
                           cudaStream_t stream, const char **error);
 
 // ff_decode.cu
+bool pack_scales(FFContext *ctx, const uint8_t *blobs, uint64_t stride, const FFExpertOffsets &off, uint32_t D, uint32_t F,
+                 uint32_t count, uint32_t **out, const char **error);
 bool make_row_box_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t rowBytes, uint64_t experts,
                       uint64_t expertStride, uint32_t boxBytes, uint32_t boxRows, const char **error);
 
