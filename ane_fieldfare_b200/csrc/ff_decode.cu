@@ -41,7 +41,6 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
-#include <type_traits>
 
 #include "ff_int_device.cuh"
 
@@ -52,6 +51,7 @@ constexpr int kFusedWarps = kFusedThreads / 32;
 constexpr int kBigWarps = 10;      // warps 0..9: gate/up pairs and the routed down tiles
 constexpr int kSharedGuWarps = 8;  // warps 0..7 take the shared gate/up tiles in phase A (K quarters)
 constexpr int kRouterWarps = 2;    // warps 8, 9 the router rows
+constexpr int kRouterChunks = 12;  // 16-byte pieces of a router row a lane holds: 3072 inputs
 constexpr int kRankWarp = 9;       // polls the logits
 static_assert(kRankWarp < kBigWarps && 8 <= kBigWarps, "warps 0..9 rank");
 constexpr uint32_t kBarrierSpinLimit = 1u << 24;
@@ -70,7 +70,7 @@ struct DecodeArgs {
     const uint16_t *weightsIn;
     // Values handed from CTA to CTA travel as 64-bit words (launch tag << 32 | payload) that the
     // readers poll: a word is valid when its tag is the running launch's, so nothing is cleared.
-    unsigned long long *taggedLogits;  // [CTA][kMaxExperts] payload: the logit's bits
+    unsigned long long *taggedLogits;  // [CTA / 4][kMaxExperts] payload: the logit's bits
     unsigned long long *taggedActs;    // [K * F / 2] payload: two routed activations (bf16)
     unsigned long long *taggedH1;      // [D / 2] payload: two rows of the shared FFN's output (bf16)
     unsigned long long *taggedShared;  // [Fs / 2] payload: two shared activations (bf16)
@@ -227,7 +227,7 @@ __device__ __forceinline__ void poll_and_rank(const DecodeArgs &a, uint32_t tag,
     const int tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int half = ((a.E + 1) / 2 + 15) & ~15;  // keys of a half, a multiple of sixteen
     if (warp == kRankWarp) {
-        const unsigned long long *words = a.taggedLogits + (size_t)blockIdx.x * kMaxExperts;
+        const unsigned long long *words = a.taggedLogits + (size_t)(blockIdx.x >> 2) * kMaxExperts;
         for (int base = 0; base < 2 * half; base += 64) {
             const int e = base + 2 * lane;  // (both words in one half)
             if (e >= 2 * half) break;
@@ -307,7 +307,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     __shared__ uint32_t sIds[8];
     __shared__ __align__(16) uint32_t sKey[2 * kKeyHalf];
     __shared__ float sWeights[8], sScore[8];
-    __shared__ __align__(8) uint64_t sCopyBar[kFusedWarps + kRouterWarps];
+    __shared__ __align__(8) uint64_t sCopyBar[kFusedWarps];
     __shared__ uint32_t *sHints;            // this launch's tile counters
     __shared__ uint32_t sTag;               // the launch's tag for polled words, from the generation
 
@@ -340,7 +340,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     uint32_t parity = 0;
 
     if (threadIdx.x == 0) {
-        for (int w = 0; w < kFusedWarps + kRouterWarps; ++w) bar_init(barOf(w), 1);
+        for (int w = 0; w < kFusedWarps; ++w) bar_init(barOf(w), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp >= 10 && lane == 0) prefetch_tensormap(&maps.m[warp - 10]);  // warps 10..15: the six maps
@@ -354,6 +354,20 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     auto fetchX = [&](int i) {  // plain loads for a row in the kernel's parameters
         return xPlain ? reinterpret_cast<const uint4 *>(xSrc)[i] : __ldcg(reinterpret_cast<const uint4 *>(xSrc) + i);
     };
+    // Router rows: warps 8, 9 take one expert each and hold its row in registers, 3072 inputs at a time
+    // (through shared memory the row's loads waited for the barriers' set-up, and the chain for the loads).
+    const int rw = warp - kSharedGuWarps, chunksD = D >> 3;
+    int eA = (!a.idsIn && K > 0 && rw >= 0 && rw < kRouterWarps) ? rw * G + cta : 0x7FFFFFFF;
+    uint4 wr[kRouterChunks];
+    auto load_router = [&](int first) {
+        const uint4 *row = reinterpret_cast<const uint4 *>(a.routerW + (size_t)eA * D);
+#pragma unroll
+        for (int i = 0; i < kRouterChunks; ++i) {
+            const int c = first + 32 * i + lane;
+            wr[i] = c < chunksD ? __ldcs(row + c) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    if (eA < E) load_router(0);
     uint4 xMine = make_uint4(0, 0, 0, 0);
     if ((int)threadIdx.x < (D >> 3)) xMine = fetchX((int)threadIdx.x);
     __syncthreads();
@@ -412,23 +426,6 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     };
 
     // ---------------- phase A: router logits, shared gate/up/GeGLU ----------------
-    // The router rows are requested first, alone: top-8 heads the critical path, and the copy
-    // engine serves an SM's requests in order.
-    const int rw = warp - kSharedGuWarps;  // router warps 8, 9
-    int eA = (!a.idsIn && K > 0 && rw >= 0 && rw < kRouterWarps) ? rw * G + cta : 0x7FFFFFFF;
-    const uint32_t routerBar = barOf(kFusedWarps + (rw >= 0 && rw < kRouterWarps ? rw : 0));
-    uint32_t routerParity = 0;
-    auto issue_router = [&](int e) {
-        // the router's per-column scales (the same for every expert) come along behind the row
-        if (lane == 0) {
-            bar_expect(routerBar, (uint32_t)D * (a.routerScale ? 4u : 2u));
-            bulk_copy(slot, a.routerW + (size_t)e * D, (uint32_t)D * 2u, routerBar);
-            if (a.routerScale) bulk_copy(slot + (uint32_t)D * 2u, a.routerScale, (uint32_t)D * 2u, routerBar);
-        }
-        __syncwarp();
-    };
-    if (eA < E) issue_router(eA);
-    __syncthreads();
     // shared gate/up tiles: four warps per tile (K quarters), two tiles per CTA and round
     const int partA = warp & 3;
     int tA = warp < kSharedGuWarps ? (warp >> 2) * G + cta : 0x7FFFFFFF;
@@ -451,10 +448,24 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
         // as fp32 [step of 32 runs][half][lane] for the router's chains
         float4 *x32 = reinterpret_cast<float4 *>(smemRaw + a.x32Offset);
         auto keep = [&](int r, const uint4 &q) {
-            x32[2 * r - (r & 31)] = make_float4(__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xFFFF0000u),
-                                                __uint_as_float(q.y << 16), __uint_as_float(q.y & 0xFFFF0000u));
-            x32[2 * r - (r & 31) + 32] = make_float4(__uint_as_float(q.z << 16), __uint_as_float(q.z & 0xFFFF0000u),
-                                                     __uint_as_float(q.w << 16), __uint_as_float(q.w & 0xFFFF0000u));
+            const uint32_t qq[4] = {q.x, q.y, q.z, q.w};
+            float f[8];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                f[2 * k] = __uint_as_float(qq[k] << 16);
+                f[2 * k + 1] = __uint_as_float(qq[k] & 0xFFFF0000u);
+            }
+            if (a.routerScale) {  // times the router's per-input scales
+                const uint4 sv = __ldg(reinterpret_cast<const uint4 *>(a.routerScale) + r);
+                const uint32_t ss[4] = {sv.x, sv.y, sv.z, sv.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    f[2 * k] = f[2 * k] * __uint_as_float(ss[k] << 16);
+                    f[2 * k + 1] = f[2 * k + 1] * __uint_as_float(ss[k] & 0xFFFF0000u);
+                }
+            }
+            x32[2 * r - (r & 31)] = make_float4(f[0], f[1], f[2], f[3]);
+            x32[2 * r - (r & 31) + 32] = make_float4(f[4], f[5], f[6], f[7]);
         };
         if (i >= 0) keep(i, v = i == (int)threadIdx.x ? xMine : fetchX(i));
         if (j >= 0) keep(j, w = fetchX(j));
@@ -484,60 +495,37 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
         }
         named_barrier(1 + (warp >> 2), 128);
     }
-    for (; eA < E; eA += kRouterWarps * G) {
+    while (eA < E) {
         const float biasE = a.logitBias ? __ldg(a.logitBias + eA) : 0.0f;
-        slot_wait(routerBar, routerParity, a.errorFlag);
-        warp_stamp(a, 0, 1);
-        // lane l chains fmaf over elements [256 i + 8 l, +8): the order of every router kernel
-        const uint32_t xRow = smem + a.x32Offset;
-        const int chunks = D >> 3;
-        auto chain = [&](auto scaled) {
-            float acc = 0.0f;
-            auto run = [&](const uint4 &wv, const uint4 &lo, const uint4 &hi, const uint4 &sv) {
-                const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w}, ss[4] = {sv.x, sv.y, sv.z, sv.w};
-                const uint32_t xx[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        // lane l chains fmaf over elements [256 i + 8 l, +8): the order of every router kernel.  (Chunks
+        // past the row are skipped: a lane's last step may not exist.)
+        float acc = 0.0f;
+        for (int first = 0; first < chunksD; first += 32 * kRouterChunks) {
+            if (first) load_router(first);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    float x0 = __uint_as_float(xx[2 * k]), x1 = __uint_as_float(xx[2 * k + 1]);
-                    if (decltype(scaled)::value) {
-                        x0 = x0 * __uint_as_float(ss[k] << 16);
-                        x1 = x1 * __uint_as_float(ss[k] & 0xFFFF0000u);
+            for (int i = 0; i < kRouterChunks; ++i) {
+                const int c = first + 32 * i + lane;
+                if (c < chunksD) {
+                    const uint32_t at = smem + a.x32Offset + 16u * (uint32_t)(2 * c - lane);
+                    const uint4 lo = lds128(at), hi = lds128(at + 512u);
+                    const uint32_t xx[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+                    const uint32_t ww[4] = {wr[i].x, wr[i].y, wr[i].z, wr[i].w};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        acc = fmaf(__uint_as_float(ww[k] << 16), __uint_as_float(xx[2 * k]), acc);
+                        acc = fmaf(__uint_as_float(ww[k] & 0xFFFF0000u), __uint_as_float(xx[2 * k + 1]), acc);
                     }
-                    acc = fmaf(__uint_as_float(ww[k] << 16), x0, acc);
-                    acc = fmaf(__uint_as_float(ww[k] & 0xFFFF0000u), x1, acc);
                 }
-            };
-            // a short loop, the next step's loads ahead of this step's chain
-            auto load = [&](int c, uint4 &wv, uint4 &lo, uint4 &hi, uint4 &sv) {
-                wv = lds128(slot + 16u * (uint32_t)c);
-                lo = lds128(xRow + 16u * (uint32_t)(2 * c - (c & 31)));
-                hi = lds128(xRow + 16u * (uint32_t)(2 * c - (c & 31) + 32));
-                sv = decltype(scaled)::value ? lds128(slot + (uint32_t)D * 2u + 16u * (uint32_t)c) : make_uint4(0, 0, 0, 0);
-            };
-            uint4 wv, lo, hi, sv;
-            load(min(lane, chunks - 1), wv, lo, hi, sv);
-#pragma unroll 1
-            for (int c = lane; c < chunks; c += 32) {
-                uint4 wn, ln, hn, sn;
-                load(min(c + 32, chunks - 1), wn, ln, hn, sn);
-                run(wv, lo, hi, sv);
-                wv = wn;
-                lo = ln;
-                hi = hn;
-                sv = sn;
             }
-            return acc;
-        };
-        float acc = a.routerScale ? chain(std::true_type{}) : chain(std::false_type{});
+        }
 #pragma unroll
         for (int offset = 16; offset >= 1; offset >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, offset);
-        // Value and validity in one 64-bit store, one copy for every CTA: the readers poll their own
+        // Value and validity in one 64-bit store, a copy for every four CTAs: the readers poll their own
         // copies (all CTAs' polls on eight lines held the stores up for microseconds).
         const float logit = a.logitBias ? acc + biasE : acc;
-        for (int c = lane; c < G; c += 32) st_tagged(a.taggedLogits + (size_t)c * kMaxExperts + eA, tag, __float_as_uint(logit));
-        slot_release();
-        const int next = eA + kRouterWarps * G;
-        if (next < E) issue_router(next);
+        for (int c = lane; c < (G + 3) / 4; c += 32) st_tagged(a.taggedLogits + (size_t)c * kMaxExperts + eA, tag, __float_as_uint(logit));
+        eA += kRouterWarps * G;
+        if (eA < E) load_router(0);
     }
     warp_stamp(a, 0, 2);
     stamp(a, 1);
@@ -710,7 +698,8 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     // No grid barrier before phase C: the routed activations and the shared output rows are polled
     // as tagged words while they are staged.
     warp_stamp(a, 2, 0);
-    if (is_waiting_thread()) hint_wait(sHints + 1, (uint32_t)tilesRouted);
+    // (seven eighths: the last tiles' words are polled for, by the few threads that stage them)
+    if (is_waiting_thread()) hint_wait(sHints + 1, (uint32_t)(tilesRouted - tilesRouted / 8));
     __syncthreads();  // the region still holds the shared activations that phase B's warps read
     stamp(a, 5);
 
@@ -884,7 +873,7 @@ static FusedLayout fused_layout(const FFConfig &c) {
     l.downOffset = l.partialOffset + kFusedWarps * 16 * 4;
     l.slotsOffset = up128(l.downOffset + kFusedWarps * 8 * 8 * 4);
     l.downBytes = up128(16 * l.strideRD + 64 * padded_groups(groupsF));
-    l.rowsBytes = up128(std::max({16 * l.strideGU, 16 * l.strideGUA, l.downBytes, D * 4}));
+    l.rowsBytes = up128(std::max({16 * l.strideGU, 16 * l.strideGUA, l.downBytes}));
     l.pairBytes = up128(2 * l.rowsBytes + 64 * padded_groups(groupsD));
     l.tripleBytes = up128(std::max(Fs ? 48 * l.strideSD + 64 * padded_groups(groupsFs) : 0u, 3 * l.downBytes));
     l.total = (size_t)l.slotsOffset + (size_t)(kBigWarps / 2) * l.pairBytes + 2 * (size_t)l.tripleBytes;
