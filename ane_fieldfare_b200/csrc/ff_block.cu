@@ -1,304 +1,528 @@
-// INT4 matrices against 2..16 input rows (a verify block): gate/up + GeGLU jobs and down jobs of
-// the routed experts a block touches and of the shared FFN, on the tensor cores without
-// dequantizing (see ff_mma_device.cuh), replacing the per-row GEMV kernels for these sizes.
+// Packed matrices against 1..16 input rows (a verify block): gate/up + GeGLU and down of the routed
+// experts a block touches and of the shared FFN (INT4 or INT8), on the integer tensor cores straight
+// on the codes (see ff_int_device.cuh).
 //
-// A job (GemvJob, built on the device by the route plan) is one matrix (or a gate/up pair) and the
-// 1..16 input rows that use it.  A warp task is one tile of the job's weight rows (8 gate + 8 up
-// rows, or 16 down rows) against up to eight of the job's input rows — the eight columns of
-// mma.sync m16n8k16; a job with more than eight rows yields two tasks per tile.  A task walks its
-// K range in parts: the part's packed rows (and, once, the tile's scales and biases) come in as
-// bulk asynchronous copies into the warp's shared-memory slot, then every group of 64 codes is
-// multiplied as bf16(16+q) and scaled (acc += s * sum((16+q) x) + (b - 16 s) * sum(x)).  All parts
-// of a task accumulate in the same registers, so no partial sums cross warps and results do not
-// depend on scheduling.  Persistent CTAs of 16 (gate/up) or 10 (down) warps deal tasks round robin;
-// the slots of an SM keep 100 KB and more of weights in flight.
+// Work is cut into tasks: a tile of 16 weight rows (8 gate + 8 up, or 16 down rows) of one job — the
+// shared FFN or an expert — against up to four of the job's input rows, which fill two MMAs' digit
+// columns.  Every CTA makes the same plan from the route ids in shared memory (which routes chose each
+// expert, in order; prefix sums of tasks) and takes one contiguous run of tasks, so it meets one or two
+// experts, whose few input rows it stages as digits: a job's rows are staged where they are used, not
+// all sixteen rows everywhere.  The CTA's warps deal the run's tiles round robin; a tile's rows come in
+// parts along K as tensor copies into the warp's two slots, so one part is in flight while the other is
+// multiplied, across tasks and experts.  All parts of a tile accumulate in the same registers, so no
+// partial sums cross warps and results do not depend on scheduling.
 //
-// Gate/up jobs read the block's input rows, staged once per CTA as bf16 with every aligned run of
-// eight in the order 0,4,1,5,2,6,3,7 (the order the MMA operands use), with their per-group sums.
-// Their GeGLU outputs are written in the same run order, so a down task can copy its input pieces
-// straight into its slot; the group sums of those inputs come from one extra MMA per K slice
-// against all-ones rows.
+// What bounds it: HBM for a block of many experts (16 rows, 48 experts: 170 MB), the staging of a job's
+// rows and the last tasks of a run for few.  With codes turned into bf16 pairs, the integer pipe
+// bounded it: gate/up 56 us and down 39 us for 16 rows.
 //
 // Reference kernels replaced (paths inside the reference project):
 //   Sources/ANEFieldfareHotpath/Metal/Prefill/prefill.metal:1246-1529 (verify grouped GEMV)
 //   Sources/ANEFieldfareHotpath/Metal/Quant/dequant_int4.metal:230-459 (multi-row INT4 GEMV)
+//   Sources/ANEFieldfareHotpath/Metal/Quant/dequant_int8.metal:41-138 (INT8 rows)
 #include <algorithm>
+#include <cstring>
 
-#include "ff_mma_device.cuh"
+#include <type_traits>
+
+#include "ff_int_device.cuh"
+#include "ff_tc_device.cuh"
 
 namespace ff {
+namespace {
 
-// warps (= slots) per CTA: the gate/up kernel shares its shared memory with the staged input rows
-// and takes short K parts in many slots; the down kernel's slots also hold the input pieces
-constexpr int kGateUpWarps = 16;
-constexpr int kDownWarps = 10;
-constexpr int kMaxBlockJobs = kMaxExperts + 1;
+constexpr int kMaxWarps = 12;
+constexpr int kTaskRows = 4;          // input rows of a task
+constexpr uint32_t kPartGroups = 12;  // groups of a part along K (INT8: 8), a multiple of four
+constexpr uint32_t kPartGroups8 = 8;
+
+enum Mode : int { kGateUp = 0, kDown = 1 };
+
+// One kind of job: where its weight rows and scale words are (maps) and how its rows are laid out.
+struct BlockKind {
+    uint32_t tiles;       // tiles of 16 weight rows
+    uint32_t groups;      // groups along K
+    uint32_t pitch;       // bytes between a slot's rows (= the weight box's width)
+    uint32_t sbWords;     // scale words of a row in a slot (= the scale box's width)
+    const uint16_t *in;   // input rows (bf16)
+    uint32_t inStride;
+    uint16_t *out;        // output rows
+    uint32_t outStride;
+};
 
 struct BlockArgs {
-    const GemvJob *jobs;
-    const uint32_t *jobCountPtr;
-    const uint16_t *allIn;  // gate/up: the block's input rows
-    uint32_t allStride, allRows, cols;
-    uint32_t maxPartGroups;  // groups of 64 per K part
-    uint32_t xPitch;         // gate/up: bytes between staged input rows in shared memory
-    uint32_t pieceStride;    // bytes between the 16 row pieces of a slot
-    uint32_t scaleArea;      // bytes of one scale (or bias) run in a slot
-    uint32_t inputPitch;     // down: bytes between a slot's input pieces
-    uint32_t slotBytes, slotsOffset;
+    BlockKind kind[2];    // [0] shared FFN, [1] routed experts
+    const uint32_t *ids;  // [T][K] (routed), null: shared FFN only
+    int T, K, E, withShared;
+    uint32_t *activeExperts;  // gate/up: receives the count (may be null)
     uint32_t *errorFlag;
+    uint32_t listOffset, digitsOffset, rowBytes, auxOffset, auxRow, slotsOffset, slotBytes, sbOffset;
 };
 
-// N consecutive groups: as groups_mma, plus (ONES) the sums of the inputs themselves from MMAs
-// against rows of ones: ones[u][0], ones[u][1] = sum over group u of input columns 2t, 2t+1.
-template <int N, bool ONES>
-__device__ __forceinline__ void groups_mma_cols(const uint8_t *lo, const uint8_t *hi, const uint8_t *xg,
-                                                float (&d)[N][4], float (&ones)[N][4]) {
-    groups_mma<N>(lo, hi, xg, d);
-    if (ONES) {
-        constexpr uint32_t kOne2 = 0x3F803F80u;  // bf16 (1.0, 1.0)
+struct alignas(64) BlockMaps {
+    CUtensorMap w[2][2];  // [kind][gate, up] or [kind][down]
+    CUtensorMap sb[2];
+};
+
+__device__ __forceinline__ void box3(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar)
+        : "memory");
+}
+
+// Four groups of a tile against NT pairs of input rows.  lo / hi: this lane's packed bytes of tile rows g
+// and g + 8 (INT4 8 bytes, INT8 16 per group), dig[j] its digits of pair j (columns 0..3 one row, 4..7
+// the other), sb0 / sb1 the rows' scale words, aux[j] the groups of the row this lane accounts for (t < 2
+// the pair's first, else its second).  acc[j][r]: r = 0 row g, 1 row g + 8, in units of 2^16 for the high
+// digits (t even), whose lanes also take the bias part (biasUnit = 2^-16, else 0).  A group's scale and
+// bias parts, which cancel in part, are joined before they are added up, and four groups before they
+// join the running sum.
+template <int NT, bool INT8>
+__device__ __forceinline__ void four_groups(uint32_t lo, uint32_t hi, const uint32_t (&dig)[NT], uint32_t sb0, uint32_t sb1,
+                                            const uint32_t (&aux)[NT], float biasUnit, float (&acc)[NT][2]) {
+    constexpr uint32_t kStep = INT8 ? 64 : 32;
+    uint4 a[4], b[4], x[NT][4], ax[NT][2];
 #pragma unroll
-        for (int u = 0; u < N; ++u) {
-            const uint4 x0 = *reinterpret_cast<const uint4 *>(xg + 128 * u);
-            const uint4 x1 = *reinterpret_cast<const uint4 *>(xg + 128 * u + 16);
-            ones[u][0] = ones[u][1] = ones[u][2] = ones[u][3] = 0.0f;
-            mma_16816(ones[u], kOne2, kOne2, kOne2, kOne2, x0.x, x0.y);
-            mma_16816(ones[u], kOne2, kOne2, kOne2, kOne2, x0.z, x0.w);
-            mma_16816(ones[u], kOne2, kOne2, kOne2, kOne2, x1.x, x1.y);
-            mma_16816(ones[u], kOne2, kOne2, kOne2, kOne2, x1.z, x1.w);
+    for (int u = 0; u < 4; ++u) {
+        if (INT8) {
+            a[u] = lds128(lo + kStep * u);
+            b[u] = lds128(hi + kStep * u);
+        } else {
+            const uint2 p = lds64(lo + kStep * u), q = lds64(hi + kStep * u);
+            a[u] = make_uint4(p.x & 0x0F0F0F0Fu, p.y & 0x0F0F0F0Fu, p.x & 0xF0F0F0F0u, p.y & 0xF0F0F0F0u);
+            b[u] = make_uint4(q.x & 0x0F0F0F0Fu, q.y & 0x0F0F0F0Fu, q.x & 0xF0F0F0F0u, q.y & 0xF0F0F0F0u);
         }
+#pragma unroll
+        for (int j = 0; j < NT; ++j) x[j][u] = lds128(dig[j] + kDigitGroupBytes * u);
+    }
+    const uint4 s0 = lds128(sb0), s1 = lds128(sb1);
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+        ax[j][0] = lds128(aux[j]);
+        ax[j][1] = lds128(aux[j] + 16u);
+    }
+    const uint32_t w0[4] = {s0.x, s0.y, s0.z, s0.w}, w1[4] = {s1.x, s1.y, s1.z, s1.w};
+    int d[NT][4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+            d[j][u][0] = d[j][u][1] = d[j][u][2] = d[j][u][3] = 0;
+            mma_u8s8(d[j][u], a[u].x, b[u].x, a[u].y, b[u].y, x[j][u].x, x[j][u].y);
+        }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) mma_u8s8(d[j][u], a[u].z, b[u].z, a[u].w, b[u].w, x[j][u].z, x[j][u].w);
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+        float sum0 = 0.0f, sum1 = 0.0f;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint4 &q = ax[j][u >> 1];
+            const float unit = __uint_as_float((u & 1) ? q.z : q.x), xs = __uint_as_float((u & 1) ? q.w : q.y) * biasUnit;
+            sum0 += fmaf(__uint_as_float(w0[u] << 16) * unit, (float)(d[j][u][0] * 256 + d[j][u][1]), __uint_as_float(w0[u] & 0xFFFF0000u) * xs);
+            sum1 += fmaf(__uint_as_float(w1[u] << 16) * unit, (float)(d[j][u][2] * 256 + d[j][u][3]), __uint_as_float(w1[u] & 0xFFFF0000u) * xs);
+        }
+        acc[j][0] += sum0;
+        acc[j][1] += sum1;
     }
 }
 
-// `n` consecutive groups of a 16-row tile against two input columns per thread: acc[0], acc[1] =
-// tile row g, columns 2t and 2t+1; acc[2], acc[3] = tile row g+8.  s0/b0, s1/b1: the two rows'
-// scales and biases; xs0/xs1: the two columns' group sums (ignored with ONES).  Groups are taken
-// in ascending order whatever the batching.
-template <bool ONES>
-__device__ __noinline__ void tile_rows_cols(const uint8_t *lo, const uint8_t *hi, const uint8_t *xg,
-                                            const uint16_t *s0, const uint16_t *b0, const uint16_t *s1,
-                                            const uint16_t *b1, const float *xs0, const float *xs1, int n,
-                                            float (&acc)[4]) {
-    float v[4] = {acc[0], acc[1], acc[2], acc[3]};
-    auto apply = [&](const float (&d)[4], const float (&o)[4], int i) {
-        const float x0 = ONES ? o[0] : xs0[i], x1 = ONES ? o[1] : xs1[i];
-        v[0] = group_scale(v[0], s0[i], b0[i], d[0], x0);
-        v[1] = group_scale(v[1], s0[i], b0[i], d[1], x1);
-        v[2] = group_scale(v[2], s1[i], b1[i], d[2], x0);
-        v[3] = group_scale(v[3], s1[i], b1[i], d[3], x1);
-    };
-    int i = 0;
-#pragma unroll 1
-    for (; i + 2 <= n; i += 2) {
-        float d[2][4], o[2][4];
-        groups_mma_cols<2, ONES>(lo + 32 * i, hi + 32 * i, xg + 128 * i, d, o);
-        apply(d[0], o[0], i);
-        apply(d[1], o[1], i + 1);
-    }
-    if (i < n) {
-        float d[1][4], o[1][4];
-        groups_mma_cols<1, ONES>(lo + 32 * i, hi + 32 * i, xg + 128 * i, d, o);
-        apply(d[0], o[0], i);
-    }
-    acc[0] = v[0];
-    acc[1] = v[1];
-    acc[2] = v[2];
-    acc[3] = v[3];
-}
-
-template <bool DUAL>
-__global__ void __launch_bounds__((DUAL ? kGateUpWarps : kDownWarps) * 32, 1) k_block_mma(const BlockArgs a) {
-    constexpr int kBlockWarps = DUAL ? kGateUpWarps : kDownWarps;
+template <int MODE, bool INT8>
+__global__ void __launch_bounds__(kMaxWarps * 32, 1)
+k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
     extern __shared__ __align__(128) uint8_t smemRaw[];
-    __shared__ uint32_t sPrefix[kMaxBlockJobs + 1];
-    __shared__ __align__(8) uint64_t sCopyBar[kBlockWarps];
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ uint32_t sFirst[kMaxExperts + 2];  // first task of job j: 0 shared, 1 + e expert e
+    __shared__ uint32_t sCount[kMaxExperts], sWarpSum[2][kMaxWarps];
+    __shared__ __align__(8) uint64_t sBar[2 * kMaxWarps];
+    uint8_t *sList = smemRaw + a.listOffset;  // [expert][16] route numbers (< 128)
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = (int)(blockDim.x >> 5);
     const int g = lane >> 2, t = lane & 3;
-    const uint32_t nJobs = min(*a.jobCountPtr, (uint32_t)kMaxBlockJobs);
-    uint8_t *mySlot = smemRaw + a.slotsOffset + (size_t)warp * a.slotBytes;
-    const uint32_t slotAddr = sm_addr(mySlot);
-    const uint32_t myBar = sm_addr(&sCopyBar[warp]);
-    uint32_t parity = 0;
-
+    const uint32_t smem = sm_addr(smemRaw);
+    constexpr uint32_t kPart = INT8 ? kPartGroups8 : kPartGroups, kGroupBytes = INT8 ? 64 : 32;
     if (threadIdx.x == 0) {
-        for (int w = 0; w < kBlockWarps; ++w) bar_init(sm_addr(&sCopyBar[w]), 1);
+        for (int i = 0; i < 2 * kMaxWarps; ++i) bar_init(sm_addr(&sBar[i]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // tasks per job: tiles x column halves; prefix sums by one thread (at most 257 jobs)
-    for (uint32_t j = threadIdx.x; j < nJobs; j += blockDim.x) {
-        const uint32_t tiles = DUAL ? a.jobs[j].rows >> 3 : a.jobs[j].rows >> 4;
-        sPrefix[j + 1] = tiles * ((a.jobs[j].n + 7u) >> 3);
-    }
+    // ---- the plan: routes of every expert in (token, rank) order, tasks per job ----
+    const int routes = a.ids ? a.T * a.K : 0;
+    for (int e = threadIdx.x; e < kMaxExperts; e += blockDim.x) sCount[e] = 0u;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        sPrefix[0] = 0;
-        for (uint32_t j = 0; j < nJobs; ++j) sPrefix[j + 1] += sPrefix[j];
-    }
-    __syncthreads();
-    uint8_t *xAll = smemRaw;
-    float *xSumAll = reinterpret_cast<float *>(smemRaw + (size_t)a.allRows * a.xPitch);
-    const int groupsIn = (int)(a.cols >> 6);
-    if (DUAL) stage_input(a.allIn, (int)a.allRows, (int)a.cols, xAll, a.xPitch, xSumAll, false, nullptr, a.allStride);
-    const uint32_t total = sPrefix[nJobs];
-
-    for (uint32_t task = (uint32_t)warp * gridDim.x + blockIdx.x; task < total; task += kBlockWarps * gridDim.x) {
-        // job of the task: last j with prefix[j] <= task
-        uint32_t loJ = 0, hiJ = nJobs;
-        while (hiJ - loJ > 1) {
-            const uint32_t mid = (loJ + hiJ) >> 1;
-            if (sPrefix[mid] <= task) loJ = mid;
-            else hiJ = mid;
-        }
-        const GemvJob &job = a.jobs[loJ];
-        const uint32_t local = task - sPrefix[loJ];
-        const uint32_t halves = (job.n + 7u) >> 3;
-        const uint32_t tile = local / halves, colBase = (local - tile * halves) * 8u;
-        const int nc = min(8, (int)job.n - (int)colBase);
-        const int groups = (int)(job.cols >> 6);
-        const int parts = (groups + (int)a.maxPartGroups - 1) / (int)a.maxPartGroups;
-        const uint32_t sb = DUAL ? (uint32_t)groups * 16u : (uint32_t)groups * 32u;  // one scale run of the tile
-        // this thread's input columns: g supplies the MMA's column g, results are columns 2t, 2t+1
-        const uint32_t colRowG = job.inRow[colBase + (uint32_t)(g < nc ? g : 0)];
-        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        for (int p = 0; p < parts; ++p) {
-            int gb, ge;
-            part_range(groups, parts, p, gb, ge);
-            const uint32_t piece = (uint32_t)(ge - gb) * 32u;
-            const uint32_t inPiece = (uint32_t)(ge - gb) * 128u;
-            if (lane == 0)
-                bar_expect(myBar, 16u * piece + (p == 0 ? (DUAL ? 4u : 2u) * sb : 0u) + (DUAL ? 0u : (uint32_t)nc * inPiece));
+    if (warp < 4) {
+        const int r = warp * 32 + lane;
+        const uint32_t id = r < routes ? a.ids[r] : 0xFFFFFFFFu;
+        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, id), before = __popc(peers & ((1u << lane) - 1u));
+        const bool known = id < (uint32_t)a.E;
+        // A token's routes are distinct experts, so an expert is chosen by at most T routes; repeats
+        // beyond that and routes past the resident experts keep their rows unwritten and raise the flag
+        // (the reference refuses such a route with "route expert N is out of range").
+        for (int w = 0; w < 4; ++w) {  // warps in turn: a route's place counts all earlier ones
+            if (warp == w && r < routes) {
+                const uint32_t place = known ? sCount[id] + before : 0u;
+                if (known && place < (uint32_t)a.T) sList[id * kMaxGemvRows + place] = (uint8_t)r;
+                else atomicExch(a.errorFlag, 12u);
+            }
             __syncwarp();
-            if (lane < 16) {
-                const uint32_t row = DUAL ? tile * 8u + ((uint32_t)lane & 7u) : tile * 16u + (uint32_t)lane;
-                const uint8_t *w = ((DUAL && lane >= 8) ? job.w1 : job.w0) + (size_t)row * (job.cols >> 1) + gb * 32;
-                bulk_copy(slotAddr + (uint32_t)lane * a.pieceStride, w, piece, myBar);
-            } else if (p == 0 && lane < (DUAL ? 20 : 18)) {
-                const uint32_t which = (uint32_t)lane - 16u;
-                const uint16_t *src = which == 0 ? job.s0 : which == 1 ? job.b0 : which == 2 ? job.s1 : job.b1;
-                bulk_copy(slotAddr + 16u * a.pieceStride + which * a.scaleArea,
-                          reinterpret_cast<const uint8_t *>(src) + (size_t)tile * sb, sb, myBar);
-            } else if (!DUAL && lane >= 20 && lane < 20 + nc) {
-                const uint32_t c = (uint32_t)lane - 20u;
-                const uint16_t *src = job.in + (size_t)job.inRow[colBase + c] * job.inStride + (size_t)gb * 64;
-                bulk_copy(slotAddr + 16u * a.pieceStride + 2u * a.scaleArea + c * a.inputPitch, src, inPiece, myBar);
-            }
-            slot_wait(myBar, parity, a.errorFlag);
-            const uint8_t *lo = mySlot + (size_t)g * a.pieceStride + 8 * t;
-            const uint8_t *hi = mySlot + (size_t)(g + 8) * a.pieceStride + 8 * t;
-            const uint16_t *sc = reinterpret_cast<const uint16_t *>(mySlot + 16u * a.pieceStride);
-            const uint32_t run = a.scaleArea >> 1;  // elements per scale run
-            if (DUAL) {
-                // rows g: gate row, g+8: up row of the same index; runs: gate s, gate b, up s, up b
-                const uint16_t *gS = sc + g * groups + gb, *gB = gS + run, *uS = gB + run, *uB = uS + run;
-                const uint8_t *xq = xAll + (size_t)colRowG * a.xPitch + (size_t)gb * 128 + t * 32;
-                const uint32_t r0 = job.inRow[colBase + (uint32_t)min(2 * t, nc - 1)];
-                const uint32_t r1 = job.inRow[colBase + (uint32_t)min(2 * t + 1, nc - 1)];
-                tile_rows_cols<false>(lo, hi, xq, gS, gB, uS, uB, xSumAll + (size_t)r0 * groupsIn + gb,
-                                      xSumAll + (size_t)r1 * groupsIn + gb, ge - gb, acc);
-            } else {
-                const uint16_t *s0 = sc + g * groups + gb, *b0 = s0 + run;
-                const uint16_t *s1 = sc + (g + 8) * groups + gb, *b1 = s1 + run;
-                const uint8_t *xq = mySlot + 16u * a.pieceStride + 2u * a.scaleArea + (size_t)(g < nc ? g : 0) * a.inputPitch + t * 32;
-                tile_rows_cols<true>(lo, hi, xq, s0, b0, s1, b1, nullptr, nullptr, ge - gb, acc);
-            }
-            slot_release();
+            if (warp == w && r < routes && known && before == 0) sCount[id] = min(sCount[id] + (uint32_t)__popc(peers), (uint32_t)a.T);
+            named_barrier(1, 128);
         }
-        // epilogue: this thread holds columns 2t, 2t+1 of tile rows g and g+8
+    }
+    __syncthreads();
+    {
+        // tasks of expert e = threadIdx.x (two passes cover 256 experts whatever the block size)
+        uint32_t base = a.withShared ? a.kind[0].tiles * ((uint32_t)(a.T + kTaskRows - 1) / kTaskRows) : 0u, active = 0;
+        if (threadIdx.x == 0) sFirst[0] = 0u;
+        for (int e0 = 0; e0 < a.E; e0 += (int)blockDim.x) {
+            const int e = e0 + (int)threadIdx.x;
+            const uint32_t n = e < a.E ? sCount[e] : 0u;
+            uint32_t tasks = a.kind[1].tiles * ((n + kTaskRows - 1) / kTaskRows), incl = tasks;
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const int c = 2 * t + k;
-            if (c >= nc) continue;
-            uint16_t *dst = job.out + (size_t)job.outRow[colBase + (uint32_t)c] * job.outStride;
-            if (DUAL) {
-                float gate = acc[k], up = acc[2 + k];
-                if (job.flags & kJobRoundGateUp) {
-                    gate = bf16_round(gate);
-                    up = bf16_round(up);
-                }
-                // run order 0,4,1,5,2,6,3,7: the order the down tasks' operands use
-                dst[tile * 8u + (uint32_t)((g & 3) * 2 + (g >> 2))] = f2bf(gelu_tanh(gate) * up);
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            const uint32_t act = __popc(__ballot_sync(0xFFFFFFFFu, n > 0u));
+            if (lane == 31) {
+                sWarpSum[0][warp] = incl;
+                sWarpSum[1][warp] = act;
+            }
+            __syncthreads();
+            uint32_t earlier = base;
+            for (int w = 0; w < warps; ++w) {
+                if (w < warp) earlier += sWarpSum[0][w];
+                base += sWarpSum[0][w];
+                active += sWarpSum[1][w];
+            }
+            if (e < a.E) sFirst[1 + e] = earlier + incl - tasks;
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) sFirst[1 + a.E] = base;
+        if (MODE == kGateUp && threadIdx.x == 0 && blockIdx.x == 0 && a.activeExperts) *a.activeExperts = active;
+    }
+    __syncthreads();
+    const uint32_t total = sFirst[1 + a.E];
+    const uint32_t first = (uint32_t)((uint64_t)blockIdx.x * total / gridDim.x),
+                   last = (uint32_t)((uint64_t)(blockIdx.x + 1) * total / gridDim.x);
+    if (first >= last) return;
+
+    // A run of tasks that share their input rows: rows [4 * rowGroup, +4) of job `job`.
+    struct Segment {
+        uint32_t job, rowGroup, begin, end;
+    };
+    auto segment_of = [&](uint32_t task) {  // last job whose first task is not behind `task`
+        uint32_t lo = 0, hi = (uint32_t)a.E + 1u;
+        while (hi - lo > 1u) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (sFirst[mid] <= task) lo = mid;
+            else hi = mid;
+        }
+        const uint32_t tiles = a.kind[lo ? 1 : 0].tiles, rg = (task - sFirst[lo]) / tiles;
+        return Segment{lo, rg, sFirst[lo] + rg * tiles, sFirst[lo] + (rg + 1u) * tiles};
+    };
+    auto rows_of = [&](const Segment &s) { return min(kTaskRows, (s.job ? (int)sCount[s.job - 1] : a.T) - (int)s.rowGroup * kTaskRows); };
+
+    // ---- copies: this warp's steps (task, part) in order, two slots in turn ----
+    const uint32_t slots = smem + a.slotsOffset + (uint32_t)warp * 2u * a.slotBytes;
+    const uint32_t bars = sm_addr(&sBar[2 * warp]);
+    uint32_t askTask = first + (uint32_t)warp, askPart = 0, asked = 0;
+    Segment askSeg{0, 0, 0, 0};
+    auto ask = [&]() {
+        if (askTask >= last) return;
+        if (askTask >= askSeg.end || askTask < askSeg.begin) askSeg = segment_of(askTask);
+        const int kind = askSeg.job ? 1 : 0;
+        const BlockKind &k = a.kind[kind];
+        if (lane == 0) {
+            const uint32_t slot = slots + (asked & 1u) * a.slotBytes, bar = bars + 8u * (asked & 1u);
+            const int tile = (int)(askTask - askSeg.begin), z = askSeg.job ? (int)askSeg.job - 1 : 0;
+            const int x = (int)(askPart * kPart * kGroupBytes / 8u);
+            bar_expect(bar, 16u * k.pitch + 64u * k.sbWords);
+            if (MODE == kGateUp) {
+                box3(slot, &maps.w[kind][0], x, tile * 8, z, bar);
+                box3(slot + 8u * k.pitch, &maps.w[kind][1], x, tile * 8, z, bar);
             } else {
-                dst[tile * 16u + (uint32_t)g] = f2bf(acc[k]);
-                dst[tile * 16u + 8u + (uint32_t)g] = f2bf(acc[2 + k]);
+                box3(slot, &maps.w[kind][0], x, tile * 16, z, bar);
+            }
+            box3(slot + a.sbOffset, &maps.sb[kind], (int)(askPart * kPart), tile * 16, z, bar);
+        }
+        ++asked;
+        if (++askPart * kPart >= k.groups) {
+            askPart = 0;
+            askTask += (uint32_t)warps;
+        }
+    };
+    ask();
+    ask();
+
+    const float biasUnit = (t & 1) ? 0.0f : 1.52587890625e-5f;  // 2^-16
+    uint32_t used = 0;
+    for (uint32_t at = first; at < last;) {
+        const Segment seg = segment_of(at);
+        const int kind = seg.job ? 1 : 0, n = rows_of(seg);
+        const BlockKind &k = a.kind[kind];
+        const uint32_t segEnd = min(seg.end, last);
+        auto row_of = [&](int i) {  // row i of the segment: its route (routed) or token (shared)
+            const int r = (int)seg.rowGroup * kTaskRows + i;
+            return kind ? (int)sList[(seg.job - 1u) * kMaxGemvRows + (uint32_t)r] : r;
+        };
+        __syncthreads();  // the previous segment's digits are no longer read
+        // ---- stage the rows as digits, two runs in flight per thread ----
+        {
+            const int runsPerRow = (int)k.groups * 8, runs = n * runsPerRow;
+            auto fetch = [&](int i, bool ok) {
+                if (!ok) return make_uint4(0, 0, 0, 0);
+                const int r = i / runsPerRow;
+                int row = row_of(r);
+                if (MODE == kGateUp && kind) row /= a.K;  // a route's token
+                return __ldcg(reinterpret_cast<const uint4 *>(k.in + (size_t)row * k.inStride) + (i - r * runsPerRow));
+            };
+            auto put = [&](int i, bool ok, const uint4 &v) {
+                const int r = ok ? i / runsPerRow : 0, in = ok ? i - r * runsPerRow : 0;
+                digits_put<INT8>(in, ok, v, smemRaw + a.digitsOffset + (size_t)r * a.rowBytes,
+                                 reinterpret_cast<GroupAux *>(smemRaw + a.auxOffset + (size_t)r * a.auxRow) + (in >> 3));
+            };
+            for (int base = warp * 32; base < runs; base += 2 * (int)blockDim.x) {
+                const int i = base + lane, j = i + (int)blockDim.x;
+                const uint4 v = fetch(i, i < runs), w = fetch(j, j < runs);
+                put(i, i < runs, v);
+                if (base + (int)blockDim.x < runs) put(j, j < runs, w);  // the same for the whole warp
+            }
+            // groups past the row, up to a batch of four: nothing is added for them
+            const int padded = ((int)k.groups + 3) & ~3;
+            for (int i = threadIdx.x; i < n * 4; i += blockDim.x) {
+                const int group = padded - 4 + (i & 3);
+                if (group >= (int)k.groups)
+                    *(reinterpret_cast<GroupAux *>(smemRaw + a.auxOffset + (size_t)(i >> 2) * a.auxRow) + group) = GroupAux{0.0f, 0.0f};
             }
         }
+        __syncthreads();
+        // ---- this warp's tiles of the segment ----
+        const uint32_t phase = (at - first) % (uint32_t)warps;
+        uint32_t task = at + ((uint32_t)warp + (uint32_t)warps - phase) % (uint32_t)warps;
+        auto run_tiles = [&](auto pairs) {
+            constexpr int NT = decltype(pairs)::value;
+            for (; task < segEnd; task += (uint32_t)warps) {
+                float acc[NT][2];
+                uint32_t dig[NT], aux[NT];
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    acc[j][0] = acc[j][1] = 0.0f;
+                    const int column = min(2 * j + (g >> 2), n - 1), mine = min(2 * j + (t >> 1), n - 1);
+                    dig[j] = smem + a.digitsOffset + (uint32_t)column * a.rowBytes + (uint32_t)(g & 3) * 64u + (uint32_t)t * 16u;
+                    aux[j] = smem + a.auxOffset + (uint32_t)mine * a.auxRow;
+                }
+                for (uint32_t p0 = 0; p0 < k.groups; p0 += kPart) {
+                    const uint32_t slot = slots + (used & 1u) * a.slotBytes;
+                    uint32_t parity = (used >> 1) & 1u;
+                    slot_wait(bars + 8u * (used & 1u), parity, a.errorFlag);
+                    uint32_t lo = slot + (uint32_t)g * k.pitch + (INT8 ? 16u : 8u) * t, hi = lo + 8u * k.pitch;
+                    uint32_t sb0 = slot + a.sbOffset + (uint32_t)g * k.sbWords * 4u, sb1 = sb0 + 32u * k.sbWords;
+                    const int batches = ((int)min(kPart, k.groups - p0) + 3) >> 2;
+#pragma unroll 1
+                    for (int b = 0; b < batches; ++b) {
+                        four_groups<NT, INT8>(lo, hi, dig, sb0, sb1, aux, biasUnit, acc);
+                        lo += 4u * kGroupBytes;
+                        hi += 4u * kGroupBytes;
+                        sb0 += 16u;
+                        sb1 += 16u;
+#pragma unroll
+                        for (int j = 0; j < NT; ++j) {
+                            dig[j] += 4u * kDigitGroupBytes;
+                            aux[j] += 32u;
+                        }
+                    }
+                    slot_release();
+                    ++used;
+                    ask();
+                }
+                const uint32_t tile = task - seg.begin;
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    // lane (g, t = 0): the pair's first row, t = 2: its second
+                    const float r0 = fmaf(acc[j][0], 65536.0f, __shfl_xor_sync(0xFFFFFFFFu, acc[j][0], 1));
+                    const float r1 = fmaf(acc[j][1], 65536.0f, __shfl_xor_sync(0xFFFFFFFFu, acc[j][1], 1));
+                    const int mine = 2 * j + (t >> 1);
+                    if ((t & 1) || mine >= n) continue;
+                    uint16_t *dst = k.out + (size_t)row_of(mine) * k.outStride;
+                    if (MODE == kGateUp) {
+                        // the shared FFN rounds gate and up before the activation
+                        const float gate = kind ? r0 : bf16_round(r0), up = kind ? r1 : bf16_round(r1);
+                        dst[tile * 8u + (uint32_t)g] = f2bf(gelu_tanh(gate) * up);
+                    } else {
+                        dst[tile * 16u + (uint32_t)g] = f2bf(r0);
+                        dst[tile * 16u + 8u + (uint32_t)g] = f2bf(r1);
+                    }
+                }
+            }
+        };
+        if (n > 2) run_tiles(std::integral_constant<int, 2>{});
+        else run_tiles(std::integral_constant<int, 1>{});
+        at = segEnd;
     }
 }
 
-struct BlockLayout {
-    uint32_t maxPartGroups, xPitch, pieceStride, scaleArea, inputPitch, slotBytes, slotsOffset;
-    size_t total;
-};
+// ---- host ------------------------------------------------------------------------------------------
 
-// dual: gate/up jobs over `cols` input columns and `rows` staged input rows; otherwise down jobs
-// whose widest matrix has `cols` columns.  Picks the largest K part that fits 227 KB.
-static bool block_layout(bool dual, uint32_t cols, uint32_t rows, BlockLayout *out) {
-    const uint32_t groups = cols / 64;
-    const uint32_t kBlockWarps = dual ? kGateUpWarps : kDownWarps;
-    for (uint32_t mpg = std::min(groups, 22u); mpg >= 1; --mpg) {
-        BlockLayout l{};
-        l.maxPartGroups = mpg;
-        l.pieceStride = piece_stride(mpg * 32);
-        l.scaleArea = dual ? groups * 16 : groups * 32;
-        l.inputPitch = mpg * 128 + 16;
-        l.xPitch = cols * 2 + 16;
-        uint32_t slot = 16 * l.pieceStride + (dual ? 4u : 2u) * l.scaleArea + (dual ? 0u : 8u * l.inputPitch);
-        l.slotBytes = (slot + 127u) & ~127u;
-        l.slotsOffset = dual ? ((rows * l.xPitch + rows * groups * 4 + 127u) & ~127u) : 0u;
-        l.total = (size_t)l.slotsOffset + (size_t)kBlockWarps * l.slotBytes;
-        if (l.total + 2048 <= 227 * 1024) {  // 2 KB kept for the static arrays
-            *out = l;
-            return true;
-        }
-    }
-    return false;
+bool encode3(CUtensorMap *map, CUtensorMapDataType type, const void *base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1,
+             uint64_t s2, uint32_t b0, uint32_t b1, const char **error) {
+    EncodeTiledFn fn = encode_tiled(error);
+    if (!fn) return false;
+    const cuuint64_t dims[3] = {d0, d1, d2}, strides[2] = {s1, s2};
+    const cuuint32_t box[3] = {b0, b1, 1}, elem[3] = {1, 1, 1};
+    const CUresult rc = fn(map, type, 3, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (rc != CUDA_SUCCESS) return fail(error, "cuTensorMapEncodeTiled(block) failed: " + std::to_string((int)rc));
+    return true;
 }
 
-template <bool DUAL>
-static bool launch_block_class(FFContext *ctx, const GemvJob *jobs, const uint32_t *jobCountPtr,
-                               const uint16_t *allIn, uint32_t allStride, uint32_t allRows, uint32_t cols,
-                               const char *name, cudaStream_t stream, const char **error) {
-    BlockLayout lay{};
-    if (!block_layout(DUAL, cols, allRows, &lay))
-        return fail(error, "model shape too large for the block kernels' shared memory");
-    BlockArgs a{};
-    a.jobs = jobs;
-    a.jobCountPtr = jobCountPtr;
-    a.allIn = allIn;
-    a.allStride = allStride;
-    a.allRows = allRows;
-    a.cols = cols;
-    a.maxPartGroups = lay.maxPartGroups;
-    a.xPitch = lay.xPitch;
-    a.pieceStride = lay.pieceStride;
-    a.scaleArea = lay.scaleArea;
-    a.inputPitch = lay.inputPitch;
-    a.slotBytes = lay.slotBytes;
-    a.slotsOffset = lay.slotsOffset;
-    a.errorFlag = ctx->errorFlag;
+// Slot row pitch of a kind: a part's bytes, padded so that a half-warp's reads fall on different banks
+// (INT4 64-bit reads of four rows: 32 or 96 modulo 128; INT8 128-bit reads of two rows: 64).
+uint32_t row_pitch(uint32_t groups, bool int8) {
+    if (!int8) return piece_stride(std::min(groups, kPartGroups) * 32);
+    uint32_t p = std::min(groups, kPartGroups8) * 64;
+    while ((p & 127u) != 64u) p += 16;
+    return p;
+}
+
+// Fills a kind and its maps.  mode kGateUp: w0, w1 [rows][cols], tiles of 8 + 8 rows; kDown: w0, 16 rows.
+bool setup_kind(int mode, bool int8, BlockKind &k, CUtensorMap (&w)[2], CUtensorMap &sb, const uint8_t *w0, const uint8_t *w1,
+                uint32_t rows, uint32_t cols, uint32_t experts, uint64_t stride, const uint32_t *scales, uint64_t scaleStride,
+                const char **error) {
+    const uint32_t groups = cols / 64, padded = padded_groups(groups), part = int8 ? kPartGroups8 : kPartGroups;
+    const uint64_t rowBytes = int8 ? cols : cols / 2;
+    k.tiles = mode == kGateUp ? rows / 8 : rows / 16;
+    k.groups = groups;
+    k.pitch = row_pitch(groups, int8);
+    k.sbWords = std::min(padded, part);
+    const uint8_t *ws[2] = {w0, w1};
+    for (int m = 0; m < (mode == kGateUp ? 2 : 1); ++m)
+        if (!encode3(&w[m], CU_TENSOR_MAP_DATA_TYPE_UINT64, ws[m], rowBytes / 8, rows, experts, rowBytes, stride, k.pitch / 8,
+                     mode == kGateUp ? 8 : 16, error))
+            return false;
+    const uint64_t scaleRows = mode == kGateUp ? (uint64_t)rows * 2 : rows;
+    return encode3(&sb, CU_TENSOR_MAP_DATA_TYPE_UINT32, scales, padded, scaleRows, experts, (uint64_t)padded * 4,
+                   experts > 1 ? scaleStride * 4 : scaleRows * padded * 4, k.sbWords, 16, error);
+}
+
+template <int MODE, bool INT8>
+bool launch_kernel(FFContext *ctx, BlockArgs a, const BlockMaps &maps, const char *name, cudaStream_t stream, const char **error) {
+    uint32_t groups = 0, slot = 0, sb = 0;
+    for (int i = 0; i < 2; ++i) {
+        if (!a.kind[i].tiles) continue;
+        groups = std::max(groups, a.kind[i].groups);
+        slot = std::max(slot, 16 * a.kind[i].pitch);
+        sb = std::max(sb, 64 * a.kind[i].sbWords);
+    }
+    auto up128 = [](uint32_t v) { return (v + 127u) & ~127u; };
+    const uint32_t rows = (uint32_t)std::min(a.T, kTaskRows), padded = padded_groups(groups);
+    a.listOffset = 0;
+    a.digitsOffset = a.ids ? up128((uint32_t)a.E * kMaxGemvRows) : 0;
+    a.rowBytes = padded * kDigitGroupBytes;
+    a.auxOffset = a.digitsOffset + rows * a.rowBytes;
+    a.auxRow = padded * (uint32_t)sizeof(GroupAux);
+    a.slotsOffset = up128(a.auxOffset + rows * a.auxRow);
+    a.sbOffset = up128(slot);
+    a.slotBytes = a.sbOffset + up128(sb);
+    const uint32_t limit = 227 * 1024 - 4096;  // less the static arrays
+    // (a batch of four groups may read up to three groups past a slot's last row: within the scale area
+    // or the next slot; behind the last slot a group's worth is kept)
+    const uint32_t slack = 3 * 64 * 2;
+    if (a.slotsOffset + 4 * 2 * a.slotBytes + slack > limit) return fail(error, "model shape too large for the block kernels' shared memory");
+    const uint32_t warps = std::min<uint32_t>(kMaxWarps, (limit - slack - a.slotsOffset) / (2 * a.slotBytes));
+    const size_t smem = a.slotsOffset + (size_t)warps * 2 * a.slotBytes + slack;
     static KernelSmemMemo memo;
-    if (!memo.prepare(k_block_mma<DUAL>, ctx->device, lay.total, (DUAL ? kGateUpWarps : kDownWarps) * 32, nullptr, error))
-        return false;
-    LaunchScope scope(ctx, stream, name);
-    k_block_mma<DUAL><<<ctx->smCount, (DUAL ? kGateUpWarps : kDownWarps) * 32, lay.total, stream>>>(a);
+    if (!memo.prepare(k_block_int<MODE, INT8>, ctx->device, 227 * 1024 - 4096, kMaxWarps * 32, nullptr, error)) return false;
+    {
+        LaunchScope scope(ctx, stream, name);
+        k_block_int<MODE, INT8><<<ctx->smCount, warps * 32, smem, stream>>>(a, maps);
+    }
     FF_CUDA_OK(cudaGetLastError(), error);
     return true;
 }
 
-// The gate/up + GeGLU jobs and then the down jobs of a planned block (jobs[0], jobs[1] of the
-// context, counts in its route plan).  x: the block's `tokens` input rows.
-bool launch_block_mma(FFContext *ctx, const uint16_t *x, uint32_t xStride, uint32_t tokens, bool withShared,
-                      bool haveDownJobs, cudaStream_t stream, const char **error) {
+}  // namespace
+
+// Routed experts (ids [tokens][K], partial rows to `partials`) and / or the INT4 shared FFN (rows to
+// `sharedOut`) of up to 16 rows.
+bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens,
+                       const uint32_t *ids, bool withShared, uint16_t *partials, uint16_t *sharedOut, cudaStream_t stream,
+                       const char **error) {
     const FFConfig &c = ctx->cfg;
     if (c.d % 64 || c.f % 64 || c.sharedF % 64) return fail(error, "widths must be multiples of 64");
     if (((uintptr_t)x & 15) || (xStride % 8)) return fail(error, "input rows must be 16-byte aligned");
-    if (!launch_block_class<true>(ctx, ctx->jobs[0], &ctx->plan->jobCount[0], x, xStride, tokens, c.d,
-                                  "int4_block_gate_up_act", stream, error))
-        return false;
-    if (!haveDownJobs) return true;
-    const uint32_t maxCols = withShared ? std::max(c.f, c.sharedF) : c.f;
-    return launch_block_class<false>(ctx, ctx->jobs[1], &ctx->plan->jobCount[1], nullptr, 0, 0, maxCols,
-                                     "int4_block_down", stream, error);
+    const uint64_t words = scale_words(c.d, c.f);
+    for (int mode = 0; mode < 2; ++mode) {
+        BlockArgs a{};
+        BlockMaps maps;
+        memset(&maps, 0, sizeof(maps));
+        a.ids = ids;
+        a.T = (int)tokens;
+        a.K = (int)c.topK;
+        a.E = ids ? (int)L.expertCount : 0;
+        a.withShared = withShared;
+        a.activeExperts = &ctx->plan->activeExperts;
+        a.errorFlag = ctx->errorFlag;
+        const bool down = mode == kDown;
+        if (ids) {
+            const uint32_t *o = &L.off.gateWOff;
+            BlockKind &k = a.kind[1];
+            if (!setup_kind(mode, false, k, maps.w[1], maps.sb[1], L.experts + (down ? o[6] : o[0]), L.experts + o[3], down ? c.d : c.f,
+                            down ? c.f : c.d, L.expertCount, L.stride,
+                            L.routedScales + (down ? (uint64_t)(c.f / 8) * 16 * padded_groups(c.d / 64) : 0), words, error))
+                return false;
+            k.in = down ? ctx->acts : x;
+            k.inStride = down ? c.f : xStride;
+            k.out = down ? partials : ctx->acts;
+            k.outStride = down ? c.d : c.f;
+        }
+        if (withShared) {
+            const uint32_t *o = &L.sharedOff.gateWOff;
+            BlockKind &k = a.kind[0];
+            if (!setup_kind(mode, false, k, maps.w[0], maps.sb[0], L.shared + (down ? o[6] : o[0]), L.shared + o[3], down ? c.d : c.sharedF,
+                            down ? c.sharedF : c.d, 1, (uint64_t)c.d * c.sharedF / 2,
+                            L.sharedScales + (down ? (uint64_t)(c.sharedF / 8) * 16 * padded_groups(c.d / 64) : 0), 0, error))
+                return false;
+            k.in = down ? ctx->sharedActs : x;
+            k.inStride = down ? c.sharedF : xStride;
+            k.out = down ? sharedOut : ctx->sharedActs;
+            k.outStride = down ? c.d : c.sharedF;
+        }
+        const bool ok = down ? launch_kernel<kDown, false>(ctx, a, maps, "int4_block_down", stream, error)
+                             : launch_kernel<kGateUp, false>(ctx, a, maps, "int4_block_gate_up_act", stream, error);
+        if (!ok) return false;
+    }
+    return true;
+}
+
+// The INT8 shared FFN of up to 16 rows.
+bool launch_block_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens, uint16_t *y,
+                       cudaStream_t stream, const char **error) {
+    const FFConfig &c = ctx->cfg;
+    for (int mode = 0; mode < 2; ++mode) {
+        BlockArgs a{};
+        BlockMaps maps;
+        memset(&maps, 0, sizeof(maps));
+        a.T = (int)tokens;
+        a.K = 1;
+        a.withShared = 1;
+        a.errorFlag = ctx->errorFlag;
+        const bool down = mode == kDown;
+        BlockKind &k = a.kind[0];
+        if (!setup_kind(mode, true, k, maps.w[0], maps.sb[0], L.shared8W[down ? 2 : 0], L.shared8W[1], down ? c.d : c.sharedF,
+                        down ? c.sharedF : c.d, 1, (uint64_t)c.d * c.sharedF,
+                        L.sharedScales + (down ? (uint64_t)(c.sharedF / 8) * 16 * padded_groups(c.d / 64) : 0), 0, error))
+            return false;
+        k.in = down ? ctx->sharedActs : x;
+        k.inStride = down ? c.sharedF : xStride;
+        k.out = down ? y : ctx->sharedActs;
+        k.outStride = down ? c.d : c.sharedF;
+        const bool ok = down ? launch_kernel<kDown, true>(ctx, a, maps, "shared_int8_down", stream, error)
+                             : launch_kernel<kGateUp, true>(ctx, a, maps, "shared_int8_gate_up_act", stream, error);
+        if (!ok) return false;
+    }
+    return true;
 }
 
 }  // namespace ff

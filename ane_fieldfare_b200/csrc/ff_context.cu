@@ -83,8 +83,7 @@ void ff_destroy(FFContext *ctx) {
     cudaSetDevice(ctx->device);
     cudaDeviceSynchronize();
     for (auto &L : ctx->layers) free_layer(L);
-    void *ptrs[] = {ctx->logits, ctx->ids, ctx->weights, ctx->plan, ctx->jobs[0], ctx->jobs[1],
-                    ctx->acts, ctx->sharedActs, ctx->h1,
+    void *ptrs[] = {ctx->logits, ctx->ids, ctx->weights, ctx->plan, ctx->acts, ctx->sharedActs, ctx->h1,
                     ctx->partials, ctx->xDev, ctx->yDev, ctx->xSorted, ctx->sortedPairs,
                     ctx->expertOffsets, ctx->blockCounts, ctx->units, ctx->unitCount,
                     ctx->errorFlag, ctx->gridBarrier, ctx->phaseStamps, ctx->mapScratch, ctx->taggedLogits, ctx->taggedActs,
@@ -141,14 +140,11 @@ FFContext *ff_create(int32_t deviceOrdinal, const FFConfig *config, const char *
     ctx->layers.resize(c.layers);
     const size_t T = c.maxTokens, K = c.topK;
     const size_t smallT = std::min<size_t>(T, kMaxGemvRows);
-    const size_t planExperts = std::min<size_t>(c.experts, kMaxGemvRows * K);
     bool ok = cudaStreamCreateWithFlags(&ctx->hostStream, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && dev_alloc(ctx, &ctx->logits, smallT * kMaxExperts, error);
     ok = ok && dev_alloc(ctx, &ctx->ids, T * K, error);
     ok = ok && dev_alloc(ctx, &ctx->weights, T * K, error);
     ok = ok && dev_alloc(ctx, &ctx->plan, 1, error);
-    ok = ok && dev_alloc(ctx, &ctx->jobs[0], 1 + planExperts, error);
-    ok = ok && dev_alloc(ctx, &ctx->jobs[1], 1 + planExperts, error);
     ok = ok && dev_alloc(ctx, &ctx->acts, (T * K + 256) * c.f, error);  // +256: a GEMM row tile may overhang
     ok = ok && dev_alloc(ctx, &ctx->sharedActs, (T + 256) * c.sharedF, error);
     ok = ok && dev_alloc(ctx, &ctx->h1, T * c.d, error);
@@ -329,7 +325,9 @@ bool ff_load_layer(FFContext *ctx, uint32_t layer, const void *hostBytes, uint64
     L.mapsReady = false;
     L.decodeMapsReady = false;
     ctx->weightBytes += total;
-    return pack_scales(ctx, L.experts, L.stride, L.off, d, f, expertCount, &L.routedScales, error);
+    const uint8_t *e = L.experts;
+    return pack_scales(ctx, ScaleSource{{e + o[1], e + o[4], e + o[7]}, {e + o[2], e + o[5], e + o[8]}, L.stride}, d, f, expertCount,
+                       &L.routedScales, error);
 }
 
 static bool check_projection(const FFProjection *p, uint32_t rows, uint32_t cols, const char *name,
@@ -374,7 +372,9 @@ bool ff_load_shared(FFContext *ctx, uint32_t layer, const FFProjection *gate,
     L.mapsReady = false;
     L.decodeMapsReady = false;
     ctx->weightBytes += payload;
-    return pack_scales(ctx, L.shared, 0, L.sharedOff, d, fs, 1, &L.sharedScales, error);
+    const uint8_t *b = L.shared;
+    return pack_scales(ctx, ScaleSource{{b + o[1], b + o[4], b + o[7]}, {b + o[2], b + o[5], b + o[8]}, 0}, d, fs, 1, &L.sharedScales,
+                       error);
 }
 
 static void free_router(ff::LayerStore &L) {
@@ -439,7 +439,12 @@ bool ff_load_shared_int8(FFContext *ctx, uint32_t layer, const FFProjection *gat
             return false;
         ctx->weightBytes += codes + 2 * aux;
     }
-    return alloc_int8_gemm(ctx, error);
+    ScaleSource src{};
+    for (int m = 0; m < 3; ++m) {
+        src.scales[m] = reinterpret_cast<const uint8_t *>(L.shared8S[m]);
+        src.biases[m] = reinterpret_cast<const uint8_t *>(L.shared8B[m]);
+    }
+    return pack_scales(ctx, src, d, fs, 1, &L.sharedScales, error) && alloc_int8_gemm(ctx, error);
 }
 
 bool ff_load_router_int8(FFContext *ctx, uint32_t layer, const uint8_t *codes, const uint16_t *scales,

@@ -797,48 +797,45 @@ k_decode_fused_inline_x(const DecodeArgs a, const __grid_constant__ DecodeMaps m
 
 // Scale | bias words of `count` blobs, tile by tile: [F/8 gate/up tiles][8 gate rows, 8 up rows] of
 // padded_groups(D/64) words, then [D down rows] of padded_groups(F/64).
-static uint64_t scale_words(uint32_t D, uint32_t F) {
+uint64_t scale_words(uint32_t D, uint32_t F) {
     return (uint64_t)(F / 8) * 16 * padded_groups(D / 64) + (uint64_t)D * padded_groups(F / 64);
 }
 __global__ void __launch_bounds__(256)
-k_pack_scales(const uint8_t *blobs, uint64_t stride, FFExpertOffsets off, uint32_t D, uint32_t F, uint32_t *out, uint64_t words) {
-    const uint8_t *blob = blobs + blockIdx.y * stride;
+k_pack_scales(ScaleSource src, uint32_t D, uint32_t F, uint32_t *out, uint64_t words) {
     const uint32_t gD = D / 64, gF = F / 64, pD = padded_groups(gD), pF = padded_groups(gF);
     const uint64_t gateUp = (uint64_t)(F / 8) * 16 * pD;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t g, row, groups, sOff, bOff;
+        uint32_t g, row, groups, matrix;
         if (i < gateUp) {
             const uint32_t r = (uint32_t)(i / pD), in = r & 15u;  // rows of a tile: 8 gate, 8 up
             g = (uint32_t)(i % pD);
             row = (r >> 4) * 8u + (in & 7u);
             groups = gD;
-            sOff = in < 8u ? off.gateSOff : off.upSOff;
-            bOff = in < 8u ? off.gateBOff : off.upBOff;
+            matrix = in < 8u ? 0u : 1u;
         } else {
             g = (uint32_t)((i - gateUp) % pF);
             row = (uint32_t)((i - gateUp) / pF);  // down rows stay in order: tiles of any height are contiguous
             groups = gF;
-            sOff = off.downSOff;
-            bOff = off.downBOff;
+            matrix = 2u;
         }
         uint32_t word = 0u;
         if (g < groups) {
-            const size_t at = ((size_t)row * groups + g) * 2;
-            word = (uint32_t)*reinterpret_cast<const uint16_t *>(blob + sOff + at) |
-                   ((uint32_t)*reinterpret_cast<const uint16_t *>(blob + bOff + at) << 16);
+            const size_t at = ((size_t)row * groups + g) * 2 + blockIdx.y * src.stride;
+            word = (uint32_t)*reinterpret_cast<const uint16_t *>(src.scales[matrix] + at) |
+                   ((uint32_t)*reinterpret_cast<const uint16_t *>(src.biases[matrix] + at) << 16);
         }
         out[blockIdx.y * words + i] = word;
     }
 }
 // Lays out `count` blobs' scales; *out is allocated when null (its size depends on the shape alone).
-bool pack_scales(FFContext *ctx, const uint8_t *blobs, uint64_t stride, const FFExpertOffsets &off, uint32_t D, uint32_t F,
-                 uint32_t count, uint32_t **out, const char **error) {
+bool pack_scales(FFContext *ctx, const ScaleSource &src, uint32_t D, uint32_t F, uint32_t count,
+                 uint32_t **out, const char **error) {
     const uint64_t words = scale_words(D, F);
     if (!*out) {
         FF_CUDA_OK(cudaMalloc(reinterpret_cast<void **>(out), words * count * 4), error);
         ctx->scratchBytes += words * count * 4;
     }
-    k_pack_scales<<<dim3((unsigned)((words + 1023) / 1024), count), 256>>>(blobs, stride, off, D, F, *out, words);
+    k_pack_scales<<<dim3((unsigned)((words + 1023) / 1024), count), 256>>>(src, D, F, *out, words);
     FF_CUDA_OK(cudaGetLastError(), error);
     FF_CUDA_OK(cudaStreamSynchronize(nullptr), error);
     return true;

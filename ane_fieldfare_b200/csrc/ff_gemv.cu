@@ -158,178 +158,11 @@ k_router_logits(const uint16_t *W, const uint16_t *scale, const float *bias, con
     if (lane == 0) logits[(size_t)t * E + e] = bias ? acc + bias[e] : acc;
 }
 
-struct PlanArgs {
-    const float *logits;      // [T][E] or null (ids given)
-    const uint16_t *gain;
-    const uint32_t *idsIn;    // used when logits is null
-    uint32_t *idsOut;         // written when logits is given
-    uint16_t *weightsOut;
-    int T, E, K, D, F, Fs;
-    const uint8_t *experts;
-    uint64_t stride;
-    FFExpertOffsets off;
-    const uint8_t *shared;    // null: no shared job
-    FFExpertOffsets sharedOff;
-    const uint16_t *x;
-    uint32_t xStride;
-    uint16_t *acts;
-    uint16_t *sharedActs;
-    uint16_t *partials;       // null in decode mode: no routed down jobs
-    uint16_t *sharedOut;
-    GemvJob *jobs0, *jobs1;
-    RoutePlan *plan;
-    int buildPlan;            // 0: top-K only
-    uint32_t *errorFlag;      // raised when a route names an expert that is not resident
-};
-
-// One CTA: top-K per token (when logits are given), then the route plan — the role of the
-// reference's verify_bound_plan (Metal/Prefill/prefill.metal:1458-1493): per active expert the
-// routes that chose it, in (token, rank) order, as one gate/up job and one down job, experts
-// ascending; the shared FFN is job 0 of each phase.
-__global__ void __launch_bounds__(512) k_topk_plan(PlanArgs a) {
-    __shared__ uint32_t sIds[kMaxGemvRows * 8];
-    __shared__ uint32_t sPos[kMaxExperts];
-    __shared__ uint32_t sCount[kMaxExperts];
-    __shared__ __align__(16) uint8_t sList[kMaxExperts * kMaxGemvRows];  // route numbers (< 128)
-    const int warp = threadIdx.x >> 5;
-    const int routes = a.T * a.K;
-    if (a.logits) {
-        if (warp < a.T) {
-            warp_topk(a.logits + (size_t)warp * a.E, a.E, a.K, a.gain, a.idsOut + warp * a.K,
-                      a.weightsOut + warp * a.K, sIds + warp * a.K);
-        }
-    } else {
-        for (int i = threadIdx.x; i < routes; i += blockDim.x) sIds[i] = a.idsIn[i];
-    }
-    if (!a.buildPlan) return;
-    __syncthreads();
-    // Lists of routes per expert, built from the routes' side: route r's place in its expert's list
-    // is the number of earlier routes with the same expert, so every list is in (token, rank) order.
-    // A token's routes are distinct experts, so an expert is chosen by at most T routes; repeats
-    // beyond that are dropped rather than overrunning the row class.
-    for (int i = threadIdx.x; i < kMaxExperts; i += blockDim.x) sCount[i] = 0u;
-    __syncthreads();
-    if ((int)threadIdx.x < routes) {
-        const int r = threadIdx.x;
-        const uint32_t mine = sIds[r];
-        int place = 0;
-        for (int q = 0; q < r; ++q) place += sIds[q] == mine ? 1 : 0;
-        if (mine < (uint32_t)a.E && place < a.T) {
-            sList[mine * kMaxGemvRows + place] = (uint8_t)r;
-            atomicAdd(&sCount[mine], 1u);
-        } else {
-            // the reference refuses such a route ("route expert N is out of range"); here its
-            // partial row stays unwritten and the context's error flag says so
-            atomicExch(a.errorFlag, 12u);
-        }
-    }
-    __syncthreads();
-    const int e = threadIdx.x;
-    uint32_t list[kMaxGemvRows];
-    const int n = e < a.E ? (int)sCount[e] : 0;
-    {
-        const uint4 packed = e < a.E ? *reinterpret_cast<const uint4 *>(&sList[e * kMaxGemvRows]) : make_uint4(0, 0, 0, 0);
-        const uint32_t words[4] = {packed.x, packed.y, packed.z, packed.w};
-#pragma unroll
-        for (int i = 0; i < kMaxGemvRows; ++i) list[i] = i < n ? (words[i >> 2] >> (8 * (i & 3))) & 0xFFu : 0u;
-    }
-    // position of expert e among the active experts: ballots inside a warp, warp totals through
-    // shared memory
-    const bool isActive = e < a.E && n > 0;
-    const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, isActive);
-    const int lane = threadIdx.x & 31;
-    if (lane == 0) sPos[warp] = __popc(ballot);
-    __syncthreads();
-    uint32_t before = 0, active = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-        const uint32_t c = sPos[w];
-        if (w < warp) before += c;
-        active += c;
-    }
-    const uint32_t myPos = before + __popc(ballot & ((1u << lane) - 1u));
-    const uint32_t sharedJobs = a.shared ? 1u : 0u;
-    if (e < a.E && n > 0) {
-        const uint8_t *blob = a.experts + (size_t)e * a.stride;
-        GemvJob j0{};
-        j0.w0 = blob + a.off.gateWOff;
-        j0.s0 = reinterpret_cast<const uint16_t *>(blob + a.off.gateSOff);
-        j0.b0 = reinterpret_cast<const uint16_t *>(blob + a.off.gateBOff);
-        j0.w1 = blob + a.off.upWOff;
-        j0.s1 = reinterpret_cast<const uint16_t *>(blob + a.off.upSOff);
-        j0.b1 = reinterpret_cast<const uint16_t *>(blob + a.off.upBOff);
-        j0.in = a.x;
-        j0.out = a.acts;
-        j0.rows = (uint32_t)a.F;
-        j0.cols = (uint32_t)a.D;
-        j0.inStride = a.xStride;
-        j0.outStride = (uint32_t)a.F;
-        j0.n = (uint32_t)n;
-        j0.flags = 0;
-        for (int i = 0; i < kMaxGemvRows; ++i) {
-            j0.inRow[i] = i < n ? list[i] / (uint32_t)a.K : 0u;
-            j0.outRow[i] = i < n ? list[i] : 0u;
-        }
-        a.jobs0[sharedJobs + myPos] = j0;
-        if (a.partials) {
-            GemvJob j1{};
-            j1.w0 = blob + a.off.downWOff;
-            j1.s0 = reinterpret_cast<const uint16_t *>(blob + a.off.downSOff);
-            j1.b0 = reinterpret_cast<const uint16_t *>(blob + a.off.downBOff);
-            j1.in = a.acts;
-            j1.out = a.partials;
-            j1.rows = (uint32_t)a.D;
-            j1.cols = (uint32_t)a.F;
-            j1.inStride = (uint32_t)a.F;
-            j1.outStride = (uint32_t)a.D;
-            j1.n = (uint32_t)n;
-            for (int i = 0; i < kMaxGemvRows; ++i) {
-                j1.inRow[i] = i < n ? list[i] : 0u;
-                j1.outRow[i] = i < n ? list[i] : 0u;
-            }
-            a.jobs1[sharedJobs + myPos] = j1;
-        }
-    }
-    if (threadIdx.x == 0 && a.shared) {
-        GemvJob j0{};
-        j0.w0 = a.shared + a.sharedOff.gateWOff;
-        j0.s0 = reinterpret_cast<const uint16_t *>(a.shared + a.sharedOff.gateSOff);
-        j0.b0 = reinterpret_cast<const uint16_t *>(a.shared + a.sharedOff.gateBOff);
-        j0.w1 = a.shared + a.sharedOff.upWOff;
-        j0.s1 = reinterpret_cast<const uint16_t *>(a.shared + a.sharedOff.upSOff);
-        j0.b1 = reinterpret_cast<const uint16_t *>(a.shared + a.sharedOff.upBOff);
-        j0.in = a.x;
-        j0.out = a.sharedActs;
-        j0.rows = (uint32_t)a.Fs;
-        j0.cols = (uint32_t)a.D;
-        j0.inStride = a.xStride;
-        j0.outStride = (uint32_t)a.Fs;
-        j0.n = (uint32_t)a.T;
-        j0.flags = kJobRoundGateUp;
-        GemvJob j1{};
-        j1.w0 = a.shared + a.sharedOff.downWOff;
-        j1.s0 = reinterpret_cast<const uint16_t *>(a.shared + a.sharedOff.downSOff);
-        j1.b0 = reinterpret_cast<const uint16_t *>(a.shared + a.sharedOff.downBOff);
-        j1.in = a.sharedActs;
-        j1.out = a.sharedOut;
-        j1.rows = (uint32_t)a.D;
-        j1.cols = (uint32_t)a.Fs;
-        j1.inStride = (uint32_t)a.Fs;
-        j1.outStride = (uint32_t)a.D;
-        j1.n = (uint32_t)a.T;
-        for (int i = 0; i < kMaxGemvRows; ++i) {
-            j0.inRow[i] = j0.outRow[i] = j1.inRow[i] = j1.outRow[i] = i < a.T ? (uint32_t)i : 0u;
-        }
-        a.jobs0[0] = j0;
-        a.jobs1[0] = j1;
-    }
-    const uint32_t routedJobs1 = a.partials ? active : 0u;
-    if (threadIdx.x == 0) {
-        a.plan->jobCount[0] = sharedJobs + active;
-        a.plan->jobCount[1] = sharedJobs + routedJobs1;
-        a.plan->itemCount[0] = 0;
-        a.plan->itemCount[1] = 0;
-        a.plan->activeExperts = active;
-    }
+// Top-K of 1..16 rows' logits, one warp per row.
+__global__ void __launch_bounds__(512) k_topk_small(const float *logits, const uint16_t *gain, int T, int E, int K, uint32_t *ids,
+                                                    uint16_t *weights) {
+    const int t = threadIdx.x >> 5;
+    if (t < T) warp_topk(logits + (size_t)t * E, E, K, gain, ids + t * K, weights + t * K);
 }
 
 // Metal/Prefill/prefill.metal:544-565 plus an optional residual row added after the ranks.
@@ -659,8 +492,9 @@ static bool launch_inline_job(FFContext *ctx, const GemvJob &job, cudaStream_t s
 
 constexpr int kInt8Rows = 4;  // input rows of a warp
 
-// INT8 affine shared FFN (Metal/Quant/dequant_int8.metal:41-138; Kernels/MoE/SharedExpertInt8.swift),
-// one warp per output row and up to four input rows, in the reference kernels' order made definite:
+// INT8 affine shared FFN (Metal/Quant/dequant_int8.metal:41-138; Kernels/MoE/SharedExpertInt8.swift) for the
+// shapes and alignments the tensor-core kernels do not take: one warp per output row and up to four
+// input rows, in the reference kernels' order made definite:
 // lane l takes elements 64 g + 2 l and + 1 of every group g in increasing g,
 //   acc = fma(s_g, fma(q1, x1, q0 * x0), acc);  acc = fma(b_g, x0 + x1, acc);
 // lane sums by an xor butterfly (16..1).  DUAL: gate and up rows of the same index, both rounded to
@@ -739,6 +573,8 @@ bool launch_shared_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, 
     if (tokens > (uint32_t)kMaxGemvRows && !((uintptr_t)x & 15) && !((uintptr_t)y & 15) && xStride % 8 == 0 &&
         int8_gemm_fits(D, Fs))
         return launch_shared_int8_gemm(ctx, L, x, xStride, tokens, y, stream, error);
+    if (tokens <= (uint32_t)kMaxGemvRows && !((uintptr_t)x & 15) && xStride % 8 == 0 && D <= 8192 && Fs <= 8192)
+        return launch_block_int8(ctx, L, x, xStride, tokens, y, stream, error);
     uint16_t *acts = ctx->sharedActs;
     const unsigned tokenBlocks = (tokens + kInt8Rows - 1) / kInt8Rows;
     {
@@ -796,19 +632,9 @@ bool launch_router_topk(FFContext *ctx, const LayerStore &L, const uint16_t *x, 
         k_router_logits<<<grid, 256, 0, stream>>>(L.routerW, L.routerScale, L.logitBias, x, xStride,
                                                   E, D, lg);
     }
-    PlanArgs a{};
-    a.logits = lg;
-    a.gain = L.gain;
-    a.idsOut = ids;
-    a.weightsOut = weights;
-    a.T = (int)tokens;
-    a.E = E;
-    a.K = (int)ctx->cfg.topK;
-    a.buildPlan = 0;
-    a.errorFlag = ctx->errorFlag;
     {
-        LaunchScope scope(ctx, stream, "topk_plan");
-        k_topk_plan<<<1, 512, 0, stream>>>(a);
+        LaunchScope scope(ctx, stream, "topk");
+        k_topk_small<<<1, 512, 0, stream>>>(lg, L.gain, (int)tokens, E, (int)ctx->cfg.topK, ids, weights);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
     return true;
@@ -823,7 +649,6 @@ bool launch_block_small(FFContext *ctx, const LayerStore &L, const uint16_t *x, 
                         bool withShared, bool decodeCombine, const uint16_t *residual,
                         uint16_t *partials, uint16_t *sharedOut, uint16_t *y,
                         cudaStream_t stream, const char **error) {
-    const FFConfig &c = ctx->cfg;
     if (tokens == 0) return true;
     if (tokens > kMaxGemvRows) return fail(error, "more than 16 rows in a decode/verify block");
     if (decodeCombine && tokens != 1) return fail(error, "decode combine takes exactly one row");
@@ -831,61 +656,12 @@ bool launch_block_small(FFContext *ctx, const LayerStore &L, const uint16_t *x, 
     if (withShared && !L.shared) return fail(error, "layer has no resident shared FFN");
     if (decodeCombine)
         return launch_decode_fused(ctx, L, x, ids, weights, withShared, true, residual, y, stream, error);
-    const int E = (int)L.expertCount;
-    PlanArgs a{};
-    uint32_t *idsDev = ctx->ids;
-    uint16_t *weightsDev = ctx->weights;
     if (!ids) {
-        if (!L.has_router()) return fail(error, "layer has no resident router");
         if (L.routerExperts != L.expertCount) return fail(error, "router and layer disagree on the expert count");
-        if (L.routerQ) {
-            if (!launch_router_logits_int8(ctx, L, x, xStride, tokens, ctx->logits, stream, error)) return false;
-        } else {
-            dim3 grid((L.routerExperts + 7) / 8, tokens);
-            LaunchScope scope(ctx, stream, "router_logits");
-            k_router_logits<<<grid, 256, 0, stream>>>(L.routerW, L.routerScale, L.logitBias, x,
-                                                      xStride, (int)L.routerExperts, (int)c.d,
-                                                      ctx->logits);
-        }
-        a.logits = ctx->logits;
-        a.gain = L.gain;
-        a.idsOut = idsDev;
-        a.weightsOut = weightsDev;
-    } else {
-        a.idsIn = ids;
-        idsDev = const_cast<uint32_t *>(ids);
-        weightsDev = const_cast<uint16_t *>(weights);
+        if (!launch_router_topk(ctx, L, x, xStride, tokens, ctx->ids, ctx->weights, nullptr, stream, error)) return false;
+        ids = ctx->ids;
     }
-    a.T = (int)tokens;
-    a.E = E;
-    a.K = (int)c.topK;
-    a.D = (int)c.d;
-    a.F = (int)c.f;
-    a.Fs = (int)c.sharedF;
-    a.experts = L.experts;
-    a.stride = L.stride;
-    a.off = L.off;
-    a.shared = withShared ? L.shared : nullptr;
-    a.sharedOff = L.sharedOff;
-    a.x = x;
-    a.xStride = xStride;
-    a.acts = ctx->acts;
-    a.sharedActs = ctx->sharedActs;
-    a.partials = decodeCombine ? nullptr : partials;
-    a.sharedOut = sharedOut;
-    a.jobs0 = ctx->jobs[0];
-    a.jobs1 = ctx->jobs[1];
-    a.plan = ctx->plan;
-    a.buildPlan = 1;
-    a.errorFlag = ctx->errorFlag;
-    {
-        LaunchScope scope(ctx, stream, "topk_plan");
-        k_topk_plan<<<1, 512, 0, stream>>>(a);
-    }
-    FF_CUDA_OK(cudaGetLastError(), error);
-
-    // the planned jobs run on the tensor-core block kernels
-    return launch_block_mma(ctx, x, xStride, tokens, withShared, withShared || !decodeCombine, stream, error);
+    return launch_block_int4(ctx, L, x, xStride, tokens, ids, withShared, partials, sharedOut, stream, error);
 }
 
 bool launch_reduce(FFContext *ctx, const uint16_t *partials, const uint16_t *weights,

@@ -94,10 +94,8 @@ struct GemvJob {
 };
 constexpr uint32_t kJobRoundGateUp = 1u;  // round gate and up to bf16 before the activation
 
-// Output of the device-side route plan for a decode/verify block.
+// What a decode/verify block reports.
 struct RoutePlan {
-    uint32_t jobCount[2];    // [0] gate/up jobs, [1] down jobs
-    uint32_t itemCount[2];   // (job, row block) work items per phase
     uint32_t activeExperts;  // distinct routed experts in the block
     uint32_t pad[3];
 };
@@ -161,7 +159,6 @@ struct FFContext {
     uint32_t *ids = nullptr;        // [maxTokens][topK]
     uint16_t *weights = nullptr;    // [maxTokens][topK]
     ff::RoutePlan *plan = nullptr;
-    ff::GemvJob *jobs[2] = {nullptr, nullptr};
     uint16_t *acts = nullptr;       // [maxTokens*topK][f]
     uint16_t *sharedActs = nullptr; // [maxTokens][sharedF]
     uint16_t *h1 = nullptr;         // [maxTokens][d]
@@ -251,14 +248,22 @@ bool launch_dequant_probe(FFContext *ctx, const uint8_t *w, const uint16_t *s, c
                           cudaStream_t stream, const char **error);
 
 // ff_decode.cu
-bool pack_scales(FFContext *ctx, const uint8_t *blobs, uint64_t stride, const FFExpertOffsets &off, uint32_t D, uint32_t F,
-                 uint32_t count, uint32_t **out, const char **error);
+uint64_t scale_words(uint32_t D, uint32_t F);  // words of one blob
+// Scales and biases of gate, up and down (bytes, blobs `stride` apart).
+struct ScaleSource {
+    const uint8_t *scales[3], *biases[3];
+    uint64_t stride;
+};
+bool pack_scales(FFContext *ctx, const ScaleSource &src, uint32_t D, uint32_t F, uint32_t count, uint32_t **out, const char **error);
 bool make_row_box_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t rowBytes, uint64_t experts,
                       uint64_t expertStride, uint32_t boxBytes, uint32_t boxRows, const char **error);
 
-// Gate/up + GeGLU jobs, then down jobs, of a planned 2..16-row block on the tensor-core block kernels.
-bool launch_block_mma(FFContext *ctx, const uint16_t *x, uint32_t xStride, uint32_t tokens, bool withShared,
-                      bool haveDownJobs, cudaStream_t stream, const char **error);
+// ff_block.cu
+bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens,
+                       const uint32_t *ids, bool withShared, uint16_t *partials, uint16_t *sharedOut, cudaStream_t stream,
+                       const char **error);
+bool launch_block_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens, uint16_t *y,
+                       cudaStream_t stream, const char **error);
 
 // Host hand-off of the one-token kernel: `inlineX` (host memory) travels in the kernel parameters
 // instead of `x`; the last CTA copies the output to `hostY` (host memory mapped for the device) and
