@@ -16,6 +16,7 @@
 //   Sources/ANEFieldfareHotpath/Metal/Prefill/prefill.metal:544-565,1246-1529
 //   Sources/ANEFieldfareHotpath/Metal/Quant/dequant_int4.metal:78-347
 #include <algorithm>
+#include <initializer_list>
 
 #include "ff_gemv_device.cuh"
 #include "ff_internal.cuh"
@@ -232,113 +233,243 @@ k_reduce_token_major_x8(const uint16_t *partials, const uint32_t *rowIndex, cons
     *reinterpret_cast<uint4 *>(y + (size_t)t * D + d) = o;
 }
 
-// y = x * w * rsqrt(mean(x^2) + eps) per row; one CTA per row, fp32 throughout.
-__global__ void __launch_bounds__(256)
-k_rmsnorm(const uint16_t *x, const uint16_t *w, float eps, int D, uint16_t *y) {
-    __shared__ float warpSums[8];
-    __shared__ float inv;
-    const uint16_t *xr = x + (size_t)blockIdx.x * D;
-    float sum = 0.0f;
-    for (int i = threadIdx.x; i < D; i += blockDim.x) {
-        const float v = bf2f(xr[i]);
-        sum = fmaf(v, v, sum);
-    }
+// ---- row kernels: RMSNorm and the fused steps either side of the block ----------------------------
+//
+// One CTA of 256 threads per row.  A row moves as 16-byte pieces (thread t takes pieces t, t + 256, ...;
+// every operand is asked for before the first sum is formed), and goes through shared memory for the
+// sum of squares, whose order is fixed: thread t chains fmaf over elements t, t + 256, ..., butterfly
+// inside a warp, warps in order.  Bound by HBM for many rows (32768 rows of 2816: RMSNorm 213 us with
+// 2-byte accesses) and by one load latency and the two sums for one row (the step in front of the block
+// 21 us, the one behind it 15 us, when every pass read its row again).
+
+constexpr int kRowThreads = 256;
+
+// Piece c of a row; WIDE: 16-byte aligned rows.
+template <bool WIDE>
+__device__ __forceinline__ uint4 load_piece(const uint16_t *row, int c) {
+    uint4 v;
+    if (WIDE) {
+        v = *(reinterpret_cast<const uint4 *>(row) + c);
+    } else {
+        uint16_t h[8];
 #pragma unroll
-    for (int offset = 16; offset >= 1; offset >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, offset);
-    if ((threadIdx.x & 31) == 0) warpSums[threadIdx.x >> 5] = sum;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float total = 0.0f;
-        for (int i = 0; i < 8; ++i) total += warpSums[i];
-        inv = 1.0f / sqrtf(total / (float)D + eps);
+        for (int i = 0; i < 8; ++i) h[i] = row[8 * c + i];
+        v = make_uint4(h[0] | ((uint32_t)h[1] << 16), h[2] | ((uint32_t)h[3] << 16), h[4] | ((uint32_t)h[5] << 16), h[6] | ((uint32_t)h[7] << 16));
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < D; i += blockDim.x) {
-        const float wv = w ? bf2f(w[i]) : 1.0f;
-        y[(size_t)blockIdx.x * D + i] = f2bf(bf2f(xr[i]) * wv * inv);
+    return v;
+}
+template <bool WIDE>
+__device__ __forceinline__ void store_piece(uint16_t *row, int c, const uint4 &v) {
+    if (WIDE) {
+        *(reinterpret_cast<uint4 *>(row) + c) = v;
+        return;
+    }
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        row[8 * c + 2 * i] = (uint16_t)w[i];
+        row[8 * c + 2 * i + 1] = (uint16_t)(w[i] >> 16);
     }
 }
-
-// ---- the fused steps either side of the block ----------------------------------------------------
-
-// Sum over the CTA (256 threads) of one float per thread; every thread gets the total.
-__device__ __forceinline__ float cta_sum_256(float v, float *warpSums) {
+// out[i] = f(a[i], b[i], c[i]) over the eight elements of pieces, f giving bf16 bits.
+template <typename F>
+__device__ __forceinline__ uint4 map_pieces(const uint4 &a, const uint4 &b, const uint4 &c, F f) {
+    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w}, cw[4] = {c.x, c.y, c.z, c.w};
+    uint32_t o[4];
 #pragma unroll
-    for (int offset = 16; offset >= 1; offset >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, offset);
-    __syncthreads();  // warpSums may still be read from the previous use
-    if ((threadIdx.x & 31) == 0) warpSums[threadIdx.x >> 5] = v;
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t lo = f(__uint_as_float(aw[i] << 16), __uint_as_float(bw[i] << 16), __uint_as_float(cw[i] << 16));
+        const uint32_t hi = f(__uint_as_float(aw[i] & 0xFFFF0000u), __uint_as_float(bw[i] & 0xFFFF0000u),
+                              __uint_as_float(cw[i] & 0xFFFF0000u));
+        o[i] = lo | (hi << 16);
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// 1 / rms of `row` (in shared memory, written by the caller's threads just before).
+__device__ __forceinline__ float row_rms_inv(const uint16_t *row, int D, float eps, float *warpSums) {
+    __syncthreads();  // the row is there, and warpSums no longer read
+    float sq = 0.0f;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < D; i += kRowThreads) {
+        const float v = bf2f(row[i]);
+        sq = fmaf(v, v, sq);
+    }
+#pragma unroll
+    for (int offset = 16; offset >= 1; offset >>= 1) sq += __shfl_xor_sync(0xFFFFFFFFu, sq, offset);
+    if ((threadIdx.x & 31) == 0) warpSums[threadIdx.x >> 5] = sq;
     __syncthreads();
     float total = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) total += warpSums[i];
-    return total;
+    for (int i = 0; i < kRowThreads / 32; ++i) total += warpSums[i];
+    return 1.0f / sqrtf(total / (float)D + eps);
 }
 
-// prefill_post_attn_setup_block (Metal/Prefill/prefill.metal:244-318), one CTA per row:
+// y = x * w * rsqrt(mean(x^2) + eps).  C: pieces per thread.
+template <int C, bool WIDE>
+__global__ void __launch_bounds__(kRowThreads)
+k_rmsnorm(const uint16_t *x, const uint16_t *w, float eps, int D, uint16_t *y) {
+    extern __shared__ __align__(16) uint16_t glueRow[];
+    __shared__ float warpSums[kRowThreads / 32];
+    const size_t row = (size_t)blockIdx.x * D;
+    const uint4 ones = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
+    uint4 xv[C], wv[C];
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+        const int c = threadIdx.x + kRowThreads * i;
+        if (8 * c < D) {
+            xv[i] = load_piece<WIDE>(x + row, c);
+            wv[i] = w ? load_piece<WIDE>(w, c) : ones;
+            reinterpret_cast<uint4 *>(glueRow)[c] = xv[i];
+        }
+    }
+    const float inv = row_rms_inv(glueRow, D, eps, warpSums);
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+        const int c = threadIdx.x + kRowThreads * i;
+        if (8 * c < D)
+            store_piece<WIDE>(y + row, c, map_pieces(xv[i], wv[i], wv[i], [&](float a, float b, float) { return (uint32_t)f2bf(a * b * inv); }));
+    }
+}
+
+// The same for rows too wide for the row buffer.
+__global__ void __launch_bounds__(kRowThreads)
+k_rmsnorm_long(const uint16_t *x, const uint16_t *w, float eps, int D, uint16_t *y) {
+    __shared__ float warpSums[kRowThreads / 32];
+    const size_t row = (size_t)blockIdx.x * D;
+    const float inv = row_rms_inv(x + row, D, eps, warpSums);
+    for (int i = threadIdx.x; i < D; i += kRowThreads) y[row + i] = f2bf(bf2f(x[row + i]) * (w ? bf2f(w[i]) : 1.0f) * inv);
+}
+
+// prefill_post_attn_setup_block (Metal/Prefill/prefill.metal:244-318):
 //   a = r16(attn * rms_inv(attn) * w_post_attn);  hidden = r16(hidden + a);
 //   n = hidden * rms_inv(hidden);  dense_x = r16(n * w_pre_ffn);  routed_x = r16(n * w_pre_ffn2);
-//   router_x = r16(n).  The new hidden row is kept in shared memory between the two passes.
-__global__ void __launch_bounds__(256)
+//   router_x = r16(n).
+template <int C, bool WIDE>
+__global__ void __launch_bounds__(kRowThreads)
 k_post_attn_setup(uint16_t *hidden, const uint16_t *attn, const uint16_t *wPostAttn, const uint16_t *wPreFfn,
                   const uint16_t *wPreFfn2, float eps, int D, uint16_t *denseX, uint16_t *routedX,
                   uint16_t *routerX) {
-    extern __shared__ uint16_t glueRow[];
-    __shared__ float warpSums[8];
+    extern __shared__ __align__(16) uint16_t glueRow[];
+    __shared__ float warpSums[kRowThreads / 32];
     const size_t row = (size_t)blockIdx.x * D;
-    float sq = 0.0f;
-    for (int i = threadIdx.x; i < D; i += blockDim.x) {
-        const float v = bf2f(attn[row + i]);
-        sq = fmaf(v, v, sq);
+    uint4 av[C], hv[C], wA[C], w1[C], w2[C];
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+        const int c = threadIdx.x + kRowThreads * i;
+        if (8 * c < D) {
+            av[i] = load_piece<WIDE>(attn + row, c);
+            hv[i] = load_piece<WIDE>(hidden + row, c);
+            wA[i] = load_piece<WIDE>(wPostAttn, c);
+            w1[i] = load_piece<WIDE>(wPreFfn, c);
+            w2[i] = load_piece<WIDE>(wPreFfn2, c);
+            reinterpret_cast<uint4 *>(glueRow)[c] = av[i];
+        }
     }
-    const float attnInv = 1.0f / sqrtf(cta_sum_256(sq, warpSums) / (float)D + eps);
-    sq = 0.0f;
-    for (int i = threadIdx.x; i < D; i += blockDim.x) {
-        const uint16_t an = f2bf(bf2f(attn[row + i]) * attnInv * bf2f(wPostAttn[i]));
-        const uint16_t h = f2bf(bf2f(hidden[row + i]) + bf2f(an));
-        glueRow[i] = h;
-        hidden[row + i] = h;
-        const float hf = bf2f(h);
-        sq = fmaf(hf, hf, sq);
+    const float attnInv = row_rms_inv(glueRow, D, eps, warpSums);  // (every read of the row is behind its barrier)
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+        const int c = threadIdx.x + kRowThreads * i;
+        if (8 * c < D) {
+            hv[i] = map_pieces(av[i], hv[i], wA[i],
+                               [&](float a, float h, float w) { return (uint32_t)f2bf(h + bf16_round(a * attnInv * w)); });
+            reinterpret_cast<uint4 *>(glueRow)[c] = hv[i];
+            store_piece<WIDE>(hidden + row, c, hv[i]);
+        }
     }
-    const float hiddenInv = 1.0f / sqrtf(cta_sum_256(sq, warpSums) / (float)D + eps);
-    for (int i = threadIdx.x; i < D; i += blockDim.x) {
-        const float n = bf2f(glueRow[i]) * hiddenInv;
-        denseX[row + i] = f2bf(n * bf2f(wPreFfn[i]));
-        routedX[row + i] = f2bf(n * bf2f(wPreFfn2[i]));
-        routerX[row + i] = f2bf(n);
+    const float inv = row_rms_inv(glueRow, D, eps, warpSums);
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+        const int c = threadIdx.x + kRowThreads * i;
+        if (8 * c < D) {
+            store_piece<WIDE>(denseX + row, c, map_pieces(hv[i], w1[i], w1[i], [&](float h, float w, float) { return (uint32_t)f2bf(h * inv * w); }));
+            store_piece<WIDE>(routedX + row, c, map_pieces(hv[i], w2[i], w2[i], [&](float h, float w, float) { return (uint32_t)f2bf(h * inv * w); }));
+            store_piece<WIDE>(routerX + row, c, map_pieces(hv[i], hv[i], hv[i], [&](float h, float, float) { return (uint32_t)f2bf(h * inv); }));
+        }
     }
 }
 
 // prefill_layer_tail_block (Metal/Prefill/prefill.metal:321-399; one row: Metal/Fusions/fused.metal:470-474):
 //   t = r16(h2 * rms_inv(h2) * w_postffn2);  h12 = r16(h1 + t);
 //   u = r16(h12 * rms_inv(h12) * w_postffn);  hidden = r16(r16(hidden + u) * r16(layer_scalar)).
-__global__ void __launch_bounds__(256)
+template <int C, bool WIDE>
+__global__ void __launch_bounds__(kRowThreads)
 k_layer_tail(const uint16_t *h2, const uint16_t *h1, uint16_t *hidden, const uint16_t *wPostFfn2,
              const uint16_t *wPostFfn, float eps, float layerScalar, int D) {
-    extern __shared__ uint16_t glueRow[];
-    __shared__ float warpSums[8];
+    extern __shared__ __align__(16) uint16_t glueRow[];
+    __shared__ float warpSums[kRowThreads / 32];
     const size_t row = (size_t)blockIdx.x * D;
-    float sq = 0.0f;
-    for (int i = threadIdx.x; i < D; i += blockDim.x) {
-        const float v = bf2f(h2[row + i]);
-        sq = fmaf(v, v, sq);
+    uint4 bv[C], av[C], hv[C], w2[C], w1[C];
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+        const int c = threadIdx.x + kRowThreads * i;
+        if (8 * c < D) {
+            bv[i] = load_piece<WIDE>(h2 + row, c);
+            av[i] = load_piece<WIDE>(h1 + row, c);
+            hv[i] = load_piece<WIDE>(hidden + row, c);
+            w2[i] = load_piece<WIDE>(wPostFfn2, c);
+            w1[i] = load_piece<WIDE>(wPostFfn, c);
+            reinterpret_cast<uint4 *>(glueRow)[c] = bv[i];
+        }
     }
-    const float inv2 = 1.0f / sqrtf(cta_sum_256(sq, warpSums) / (float)D + eps);
-    sq = 0.0f;
-    for (int i = threadIdx.x; i < D; i += blockDim.x) {
-        const uint16_t tmp = f2bf(bf2f(h2[row + i]) * inv2 * bf2f(wPostFfn2[i]));
-        const uint16_t h12 = f2bf(bf2f(h1[row + i]) + bf2f(tmp));
-        glueRow[i] = h12;
-        const float v = bf2f(h12);
-        sq = fmaf(v, v, sq);
+    const float inv2 = row_rms_inv(glueRow, D, eps, warpSums);
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+        const int c = threadIdx.x + kRowThreads * i;
+        if (8 * c < D) {
+            av[i] = map_pieces(bv[i], av[i], w2[i],
+                               [&](float b, float a, float w) { return (uint32_t)f2bf(a + bf16_round(b * inv2 * w)); });
+            reinterpret_cast<uint4 *>(glueRow)[c] = av[i];
+        }
     }
-    const float inv12 = 1.0f / sqrtf(cta_sum_256(sq, warpSums) / (float)D + eps);
-    const float scale = bf2f(f2bf(layerScalar));
-    for (int i = threadIdx.x; i < D; i += blockDim.x) {
-        const uint16_t u = f2bf(bf2f(glueRow[i]) * inv12 * bf2f(wPostFfn[i]));
-        const uint16_t sum = f2bf(bf2f(hidden[row + i]) + bf2f(u));
-        hidden[row + i] = f2bf(bf2f(sum) * scale);
+    const float inv12 = row_rms_inv(glueRow, D, eps, warpSums);
+    const float scale = bf16_round(layerScalar);
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+        const int c = threadIdx.x + kRowThreads * i;
+        if (8 * c < D)
+            store_piece<WIDE>(hidden + row, c, map_pieces(av[i], hv[i], w1[i], [&](float a, float h, float w) {
+                                  return (uint32_t)f2bf(bf16_round(h + bf16_round(a * inv12 * w)) * scale);
+                              }));
     }
+}
+
+// A row kernel by the pieces a thread holds (rows of 4096 values and less: two) and the rows' alignment.
+#define FF_ROW_KERNEL(NAME, D, WIDE, ...)                                                                              \
+    do {                                                                                                               \
+        const size_t smem_ = (size_t)(D) * 2;                                                                          \
+        static KernelSmemMemo memo_[6];                                                                                \
+        auto go_ = [&](auto kernel, KernelSmemMemo &memo) {                                                            \
+            if (!memo.prepare(kernel, ctx->device, smem_, kRowThreads, nullptr, error)) return false;                  \
+            LaunchScope scope(ctx, stream, #NAME);                                                                     \
+            kernel<<<tokens, kRowThreads, smem_, stream>>>(__VA_ARGS__);                                               \
+            return true;                                                                                               \
+        };                                                                                                             \
+        const bool ok_ = (D) <= 4096    ? ((WIDE) ? go_(k_##NAME<2, true>, memo_[0]) : go_(k_##NAME<2, false>, memo_[1]))  \
+                         : (D) <= 16384 ? ((WIDE) ? go_(k_##NAME<8, true>, memo_[2]) : go_(k_##NAME<8, false>, memo_[3]))  \
+                                        : ((WIDE) ? go_(k_##NAME<24, true>, memo_[4]) : go_(k_##NAME<24, false>, memo_[5])); \
+        if (!ok_) return false;                                                                                        \
+    } while (0)
+
+static bool aligned16(std::initializer_list<const void *> pointers) {
+    uintptr_t all = 0;
+    for (const void *p : pointers) all |= reinterpret_cast<uintptr_t>(p);
+    return (all & 15u) == 0;
+}
+
+bool launch_rmsnorm(FFContext *ctx, const uint16_t *x, const uint16_t *w, float eps, uint32_t tokens, uint16_t *y,
+                    cudaStream_t stream, const char **error) {
+    if (tokens == 0) return true;
+    const int D = (int)ctx->cfg.d;
+    if ((size_t)D * 2 > 96 * 1024) {
+        LaunchScope scope(ctx, stream, "rmsnorm");
+        k_rmsnorm_long<<<tokens, kRowThreads, 0, stream>>>(x, w, eps, D, y);
+        FF_CUDA_OK(cudaGetLastError(), error);
+        return true;
+    }
+    FF_ROW_KERNEL(rmsnorm, D, aligned16({x, w, y}), x, w, eps, D, y);
+    FF_CUDA_OK(cudaGetLastError(), error);
+    return true;
 }
 
 bool launch_post_attn_setup(FFContext *ctx, uint16_t *hidden, const uint16_t *attn, const uint16_t *wPostAttn,
@@ -348,11 +479,8 @@ bool launch_post_attn_setup(FFContext *ctx, uint16_t *hidden, const uint16_t *at
     if (tokens == 0) return true;
     const int D = (int)ctx->cfg.d;
     if ((size_t)D * 2 > 96 * 1024) return fail(error, "model width too large for the row buffer");
-    {
-        LaunchScope scope(ctx, stream, "post_attn_setup");
-        k_post_attn_setup<<<tokens, 256, (size_t)D * 2, stream>>>(hidden, attn, wPostAttn, wPreFfn, wPreFfn2, eps, D,
-                                                                  denseX, routedX, routerX);
-    }
+    FF_ROW_KERNEL(post_attn_setup, D, aligned16({hidden, attn, wPostAttn, wPreFfn, wPreFfn2, denseX, routedX, routerX}), hidden, attn,
+                  wPostAttn, wPreFfn, wPreFfn2, eps, D, denseX, routedX, routerX);
     FF_CUDA_OK(cudaGetLastError(), error);
     return true;
 }
@@ -363,10 +491,7 @@ bool launch_layer_tail(FFContext *ctx, const uint16_t *h2, const uint16_t *h1, u
     if (tokens == 0) return true;
     const int D = (int)ctx->cfg.d;
     if ((size_t)D * 2 > 96 * 1024) return fail(error, "model width too large for the row buffer");
-    {
-        LaunchScope scope(ctx, stream, "layer_tail");
-        k_layer_tail<<<tokens, 256, (size_t)D * 2, stream>>>(h2, h1, hidden, wPostFfn2, wPostFfn, eps, layerScalar, D);
-    }
+    FF_ROW_KERNEL(layer_tail, D, aligned16({h2, h1, hidden, wPostFfn2, wPostFfn}), h2, h1, hidden, wPostFfn2, wPostFfn, eps, layerScalar, D);
     FF_CUDA_OK(cudaGetLastError(), error);
     return true;
 }
@@ -746,17 +871,6 @@ bool launch_shared_small(FFContext *ctx, const LayerStore &L, const uint16_t *x,
         j0.inRow[i] = j0.outRow[i] = j1.inRow[i] = j1.outRow[i] = i < tokens ? i : 0u;
     if (!launch_inline_job<true>(ctx, j0, stream, error)) return false;
     return launch_inline_job<false>(ctx, j1, stream, error);
-}
-
-bool launch_rmsnorm(FFContext *ctx, const uint16_t *x, const uint16_t *w, float eps,
-                    uint32_t tokens, uint16_t *y, cudaStream_t stream, const char **error) {
-    if (tokens == 0) return true;
-    {
-        LaunchScope scope(ctx, stream, "rmsnorm");
-        k_rmsnorm<<<tokens, 256, 0, stream>>>(x, w, eps, (int)ctx->cfg.d, y);
-    }
-    FF_CUDA_OK(cudaGetLastError(), error);
-    return true;
 }
 
 bool launch_dequant_probe(FFContext *ctx, const uint8_t *w, const uint16_t *s, const uint16_t *b,
