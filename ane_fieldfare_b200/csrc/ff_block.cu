@@ -5,16 +5,17 @@
 // Work is cut into tasks: a tile of 16 weight rows (8 gate + 8 up, or 16 down rows) of one job — the
 // shared FFN or an expert — against up to four of the job's input rows, which fill two MMAs' digit
 // columns.  Every CTA makes the same plan from the route ids in shared memory (which routes chose each
-// expert, in order; prefix sums of tasks) and takes one contiguous run of tasks, so it meets one or two
-// experts, whose few input rows it stages as digits: a job's rows are staged where they are used, not
-// all sixteen rows everywhere.  The CTA's warps deal the run's tiles round robin; a tile's rows come in
-// parts along K as tensor copies into the warp's two slots, so one part is in flight while the other is
-// multiplied, across tasks and experts.  All parts of a tile accumulate in the same registers, so no
-// partial sums cross warps and results do not depend on scheduling.
+// expert, in order; the jobs' costs) and takes a contiguous run of tasks, the same cost for every CTA,
+// so it meets one or two experts, whose few input rows it stages as digits: a job's rows are staged
+// where they are used, not all sixteen rows everywhere.  The CTA's warps deal the run's tiles round
+// robin; a tile's rows come in parts along K as tensor copies into the warp's two slots, so one part is
+// in flight while the other is multiplied, across tasks and experts.  All parts of a tile accumulate in
+// the same registers, so no partial sums cross warps and results do not depend on scheduling.
 //
-// What bounds it: HBM for a block of many experts (16 rows, 48 experts: 170 MB), the staging of a job's
-// rows and the last tasks of a run for few.  With codes turned into bf16 pairs, the integer pipe
-// bounded it: gate/up 56 us and down 39 us for 16 rows.
+// INT4: an input row has one scale for its digits, a group's sums are scaled once by the weights' scale,
+// and the bias part is a few small bf16 MMAs on the group sums: 13 instructions per group for the
+// weights and 9 for a pair of rows, per warp.  INT8: the two parts cancel in part, so they are joined
+// group by group.
 //
 // Reference kernels replaced (paths inside the reference project):
 //   Sources/ANEFieldfareHotpath/Metal/Prefill/prefill.metal:1246-1529 (verify grouped GEMV)
@@ -31,10 +32,10 @@
 namespace ff {
 namespace {
 
-constexpr int kMaxWarps = 12;
+constexpr int kMaxWarps = 16;
 constexpr int kTaskRows = 4;          // input rows of a task
-constexpr uint32_t kPartGroups = 12;  // groups of a part along K (INT8: 8), a multiple of four
-constexpr uint32_t kPartGroups8 = 8;
+constexpr uint32_t kPartGroups = 8;   // groups of a part along K, a multiple of four
+constexpr int kMaxJobs = kMaxGemvRows * 8 + 1;
 
 enum Mode : int { kGateUp = 0, kDown = 1 };
 
@@ -42,6 +43,7 @@ enum Mode : int { kGateUp = 0, kDown = 1 };
 struct BlockKind {
     uint32_t tiles;       // tiles of 16 weight rows
     uint32_t groups;      // groups along K
+    uint32_t part;        // groups of a part (all of them when that is little more than kPartGroups)
     uint32_t pitch;       // bytes between a slot's rows (= the weight box's width)
     uint32_t sbWords;     // scale words of a row in a slot (= the scale box's width)
     const uint16_t *in;   // input rows (bf16)
@@ -72,28 +74,22 @@ __device__ __forceinline__ void box3(uint32_t dst, const CUtensorMap *map, int x
         : "memory");
 }
 
-// Four groups of a tile against NT pairs of input rows.  lo / hi: this lane's packed bytes of tile rows g
-// and g + 8 (INT4 8 bytes, INT8 16 per group), dig[j] its digits of pair j (columns 0..3 one row, 4..7
+// ---- INT8: four groups of a tile against NT pairs of input rows ------------------------------------
+//
+// lo / hi: this lane's 16 codes of tile rows g and g + 8 per group, dig[j] its digits of pair j (columns 0..3 one row, 4..7
 // the other), sb0 / sb1 the rows' scale words, aux[j] the groups of the row this lane accounts for (t < 2
 // the pair's first, else its second).  acc[j][r]: r = 0 row g, 1 row g + 8, in units of 2^16 for the high
 // digits (t even), whose lanes also take the bias part (biasUnit = 2^-16, else 0).  A group's scale and
 // bias parts, which cancel in part, are joined before they are added up, and four groups before they
 // join the running sum.
-template <int NT, bool INT8>
-__device__ __forceinline__ void four_groups(uint32_t lo, uint32_t hi, const uint32_t (&dig)[NT], uint32_t sb0, uint32_t sb1,
+template <int NT>
+__device__ __forceinline__ void four_groups8(uint32_t lo, uint32_t hi, const uint32_t (&dig)[NT], uint32_t sb0, uint32_t sb1,
                                             const uint32_t (&aux)[NT], float biasUnit, float (&acc)[NT][2]) {
-    constexpr uint32_t kStep = INT8 ? 64 : 32;
     uint4 a[4], b[4], x[NT][4], ax[NT][2];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-        if (INT8) {
-            a[u] = lds128(lo + kStep * u);
-            b[u] = lds128(hi + kStep * u);
-        } else {
-            const uint2 p = lds64(lo + kStep * u), q = lds64(hi + kStep * u);
-            a[u] = make_uint4(p.x & 0x0F0F0F0Fu, p.y & 0x0F0F0F0Fu, p.x & 0xF0F0F0F0u, p.y & 0xF0F0F0F0u);
-            b[u] = make_uint4(q.x & 0x0F0F0F0Fu, q.y & 0x0F0F0F0Fu, q.x & 0xF0F0F0F0u, q.y & 0xF0F0F0F0u);
-        }
+        a[u] = lds128(lo + 64 * u);
+        b[u] = lds128(hi + 64 * u);
 #pragma unroll
         for (int j = 0; j < NT; ++j) x[j][u] = lds128(dig[j] + kDigitGroupBytes * u);
     }
@@ -131,25 +127,76 @@ __device__ __forceinline__ void four_groups(uint32_t lo, uint32_t hi, const uint
     }
 }
 
+// ---- INT4: four groups of a tile against NT pairs of input rows ------------------------------------
+//
+// lo / hi: this lane's eight packed bytes of tile rows g and g + 8 per group, dig[j] its digits of pair j
+// (columns 0..3 one row, 4..7 the other), sb0 / sb1 the rows' scale words.  acc[j][r] += scale * digits
+// (r = 0 row g, 1 row g + 8) in the input row's unit; t even holds the high digits, in units of 2^16.
+template <int NT>
+__device__ __forceinline__ void four_groups4(uint32_t lo, uint32_t hi, const uint32_t (&dig)[NT], uint32_t sb0, uint32_t sb1,
+                                             float (&acc)[NT][2]) {
+    uint2 p[4], q[4];
+    uint4 x[NT][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        p[u] = lds64(lo + 32 * u);
+        q[u] = lds64(hi + 32 * u);
+#pragma unroll
+        for (int j = 0; j < NT; ++j) x[j][u] = lds128(dig[j] + kDigitGroupBytes * u);
+    }
+    const uint4 s0 = lds128(sb0), s1 = lds128(sb1);
+    int d[NT][4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+            d[j][u][0] = d[j][u][1] = d[j][u][2] = d[j][u][3] = 0;
+            mma_u8s8(d[j][u], p[u].x & 0x0F0F0F0Fu, q[u].x & 0x0F0F0F0Fu, p[u].y & 0x0F0F0F0Fu, q[u].y & 0x0F0F0F0Fu, x[j][u].x, x[j][u].y);
+        }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+            mma_u8s8(d[j][u], p[u].x & 0xF0F0F0F0u, q[u].x & 0xF0F0F0F0u, p[u].y & 0xF0F0F0F0u, q[u].y & 0xF0F0F0F0u, x[j][u].z, x[j][u].w);
+    const uint32_t w0[4] = {s0.x, s0.y, s0.z, s0.w}, w1[4] = {s1.x, s1.y, s1.z, s1.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+            acc[j][0] = fmaf(__uint_as_float(w0[u] << 16), (float)(d[j][u][0] * 256 + d[j][u][1]), acc[j][0]);
+            acc[j][1] = fmaf(__uint_as_float(w1[u] << 16), (float)(d[j][u][2] * 256 + d[j][u][3]), acc[j][1]);
+        }
+}
+// Bias part of eight groups: the biases (high halves of the scale words) against the group sums, which lie
+// as bf16 pieces in MMA columns 0..3 (a pair's first row) and 4..7 (its second).
+__device__ __forceinline__ void mma_1688(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(b0));
+}
+constexpr uint32_t kSumBlockBytes = 128;  // [column][8 groups] bf16
+
 template <int MODE, bool INT8>
 __global__ void __launch_bounds__(kMaxWarps * 32, 1)
 k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
     extern __shared__ __align__(128) uint8_t smemRaw[];
-    __shared__ uint32_t sFirst[kMaxExperts + 2];  // first task of job j: 0 shared, 1 + e expert e
-    __shared__ uint32_t sCount[kMaxExperts], sWarpSum[2][kMaxWarps];
+    __shared__ uint32_t sFirst[kMaxJobs + 1];   // cost of the jobs before job k (active jobs, the shared FFN first)
+    __shared__ uint16_t sJob[kMaxJobs];         // 0 the shared FFN, 1 + e expert e
+    __shared__ uint32_t sCount[kMaxExperts], sWarpSum[2][kMaxWarps], sTop[kMaxWarps];
+    __shared__ float sUnit[kTaskRows];
     __shared__ __align__(8) uint64_t sBar[2 * kMaxWarps];
     uint8_t *sList = smemRaw + a.listOffset;  // [expert][16] route numbers (< 128)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = (int)(blockDim.x >> 5);
     const int g = lane >> 2, t = lane & 3;
     const uint32_t smem = sm_addr(smemRaw);
-    constexpr uint32_t kPart = INT8 ? kPartGroups8 : kPartGroups, kGroupBytes = INT8 ? 64 : 32;
+    constexpr uint32_t kGroupBytes = INT8 ? 64 : 32;
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2 * kMaxWarps; ++i) bar_init(sm_addr(&sBar[i]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // ---- the plan: routes of every expert in (token, rank) order, tasks per job ----
+    // ---- the plan: routes of every expert in (token, rank) order, cost of every job ----
     const int routes = a.ids ? a.T * a.K : 0;
-    for (int e = threadIdx.x; e < kMaxExperts; e += blockDim.x) sCount[e] = 0u;
+    for (int e = threadIdx.x; e < a.E; e += blockDim.x) sCount[e] = 0u;
     __syncthreads();
     if (warp < 4) {
         const int r = warp * 32 + lane;
@@ -171,73 +218,114 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
         }
     }
     __syncthreads();
+    // instructions of a tile: per group what the weights cost and what a pair of rows costs, and its set-up
+    auto tile_cost = [&](int kind, int rows) { return a.kind[kind].groups * (rows > 2 ? 31u : 22u) + 100u; };
+    auto job_cost = [&](int kind, int rows) {
+        const uint32_t full = (uint32_t)rows / kTaskRows, rest = (uint32_t)rows % kTaskRows;
+        return a.kind[kind].tiles * (full * tile_cost(kind, kTaskRows) + (rest ? tile_cost(kind, (int)rest) : 0u));
+    };
+    uint32_t nJobs = a.withShared ? 1u : 0u;
     {
-        // tasks of expert e = threadIdx.x (two passes cover 256 experts whatever the block size)
-        uint32_t base = a.withShared ? a.kind[0].tiles * ((uint32_t)(a.T + kTaskRows - 1) / kTaskRows) : 0u, active = 0;
-        if (threadIdx.x == 0) sFirst[0] = 0u;
+        uint32_t base = a.withShared ? job_cost(0, a.T) : 0u;
+        if (threadIdx.x == 0) {
+            sFirst[0] = 0u;
+            sJob[0] = 0;
+        }
+        __syncthreads();
         for (int e0 = 0; e0 < a.E; e0 += (int)blockDim.x) {
             const int e = e0 + (int)threadIdx.x;
-            const uint32_t n = e < a.E ? sCount[e] : 0u;
-            uint32_t tasks = a.kind[1].tiles * ((n + kTaskRows - 1) / kTaskRows), incl = tasks;
+            const uint32_t n = e < a.E ? sCount[e] : 0u, cost = n ? job_cost(1, (int)n) : 0u;
+            uint32_t incl = cost;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
                 if (lane >= o) incl += v;
             }
-            const uint32_t act = __popc(__ballot_sync(0xFFFFFFFFu, n > 0u));
+            const uint32_t active = __ballot_sync(0xFFFFFFFFu, n > 0u);
             if (lane == 31) {
                 sWarpSum[0][warp] = incl;
-                sWarpSum[1][warp] = act;
+                sWarpSum[1][warp] = __popc(active);
             }
             __syncthreads();
-            uint32_t earlier = base;
+            uint32_t costBefore = base, jobsBefore = nJobs;
             for (int w = 0; w < warps; ++w) {
-                if (w < warp) earlier += sWarpSum[0][w];
+                if (w < warp) {
+                    costBefore += sWarpSum[0][w];
+                    jobsBefore += sWarpSum[1][w];
+                }
                 base += sWarpSum[0][w];
-                active += sWarpSum[1][w];
+                nJobs += sWarpSum[1][w];
             }
-            if (e < a.E) sFirst[1 + e] = earlier + incl - tasks;
+            if (n) {
+                const uint32_t k = jobsBefore + __popc(active & ((1u << lane) - 1u));
+                sJob[k] = (uint16_t)(1 + e);
+                sFirst[k] = costBefore + incl - cost;
+            }
             __syncthreads();
         }
-        if (threadIdx.x == 0) sFirst[1 + a.E] = base;
-        if (MODE == kGateUp && threadIdx.x == 0 && blockIdx.x == 0 && a.activeExperts) *a.activeExperts = active;
+        if (threadIdx.x == 0) sFirst[nJobs] = base;
+        if (MODE == kGateUp && threadIdx.x == 0 && blockIdx.x == 0 && a.activeExperts) *a.activeExperts = nJobs - (a.withShared ? 1u : 0u);
     }
     __syncthreads();
-    const uint32_t total = sFirst[1 + a.E];
-    const uint32_t first = (uint32_t)((uint64_t)blockIdx.x * total / gridDim.x),
-                   last = (uint32_t)((uint64_t)(blockIdx.x + 1) * total / gridDim.x);
-    if (first >= last) return;
+    if (nJobs == 0) return;
 
-    // A run of tasks that share their input rows: rows [4 * rowGroup, +4) of job `job`.
-    struct Segment {
-        uint32_t job, rowGroup, begin, end;
+    // A tile of four input rows (`rowGroup`) of a job; tiles in order are a CTA's run.
+    struct Place {
+        uint32_t job, rowGroup, tile;
     };
-    auto segment_of = [&](uint32_t task) {  // last job whose first task is not behind `task`
-        uint32_t lo = 0, hi = (uint32_t)a.E + 1u;
+    auto kind_of = [&](uint32_t job) { return sJob[job] ? 1 : 0; };
+    auto rows_of = [&](uint32_t job) { return sJob[job] ? (int)sCount[sJob[job] - 1] : a.T; };
+    auto place_of = [&](uint32_t cta) {  // the first tile whose cost position is not before the CTA's share
+        if (cta == gridDim.x) return Place{nJobs, 0u, 0u};
+        const uint32_t target = (uint32_t)((uint64_t)sFirst[nJobs] * cta / gridDim.x);
+        uint32_t lo = 0, hi = nJobs;
         while (hi - lo > 1u) {
             const uint32_t mid = (lo + hi) >> 1;
-            if (sFirst[mid] <= task) lo = mid;
+            if (sFirst[mid] <= target) lo = mid;
             else hi = mid;
         }
-        const uint32_t tiles = a.kind[lo ? 1 : 0].tiles, rg = (task - sFirst[lo]) / tiles;
-        return Segment{lo, rg, sFirst[lo] + rg * tiles, sFirst[lo] + (rg + 1u) * tiles};
+        const int kind = kind_of(lo), rows = rows_of(lo);
+        const uint32_t tiles = a.kind[kind].tiles, full = (uint32_t)rows / kTaskRows;
+        uint32_t cost = tile_cost(kind, kTaskRows), rest = target - sFirst[lo];
+        const uint32_t rg = min(full, rest / (tiles * cost));
+        rest -= rg * tiles * cost;
+        if (rg == full) cost = tile_cost(kind, rows % kTaskRows);
+        return Place{lo, rg, (rest + cost - 1u) / cost};  // (may be one past the row group's last tile)
     };
-    auto rows_of = [&](const Segment &s) { return min(kTaskRows, (s.job ? (int)sCount[s.job - 1] : a.T) - (int)s.rowGroup * kTaskRows); };
+    auto before = [](const Place &p, const Place &q) {
+        return p.job != q.job ? p.job < q.job : p.rowGroup != q.rowGroup ? p.rowGroup < q.rowGroup : p.tile < q.tile;
+    };
+    auto settle = [&](Place &p) {  // tiles past a row group belong to the next
+        while (p.job < nJobs) {
+            const uint32_t tiles = a.kind[kind_of(p.job)].tiles;
+            if (p.tile < tiles) break;
+            p.tile -= tiles;
+            if ((int)(++p.rowGroup * kTaskRows) >= rows_of(p.job)) {
+                p.rowGroup = 0;
+                ++p.job;
+            }
+        }
+        if (p.job >= nJobs) p = Place{nJobs, 0u, 0u};
+    };
+    Place at = place_of(blockIdx.x), end = place_of(blockIdx.x + 1u);
+    settle(at);
+    settle(end);
 
-    // ---- copies: this warp's steps (task, part) in order, two slots in turn ----
+    // ---- copies: this warp's steps (tile, part) in order, two slots in turn ----
     const uint32_t slots = smem + a.slotsOffset + (uint32_t)warp * 2u * a.slotBytes;
     const uint32_t bars = sm_addr(&sBar[2 * warp]);
-    uint32_t askTask = first + (uint32_t)warp, askPart = 0, asked = 0;
-    Segment askSeg{0, 0, 0, 0};
+    Place askAt = at;
+    askAt.tile += (uint32_t)warp;
+    settle(askAt);
+    uint32_t askPart = 0, asked = 0;
     auto ask = [&]() {
-        if (askTask >= last) return;
-        if (askTask >= askSeg.end || askTask < askSeg.begin) askSeg = segment_of(askTask);
-        const int kind = askSeg.job ? 1 : 0;
+        if (!before(askAt, end)) return;
+        const int kind = kind_of(askAt.job);
         const BlockKind &k = a.kind[kind];
         if (lane == 0) {
             const uint32_t slot = slots + (asked & 1u) * a.slotBytes, bar = bars + 8u * (asked & 1u);
-            const int tile = (int)(askTask - askSeg.begin), z = askSeg.job ? (int)askSeg.job - 1 : 0;
-            const int x = (int)(askPart * kPart * kGroupBytes / 8u);
+            const int tile = (int)askAt.tile, z = kind ? (int)sJob[askAt.job] - 1 : 0;
+            const int x = (int)(askPart * kGroupBytes / 8u);
             bar_expect(bar, 16u * k.pitch + 64u * k.sbWords);
             if (MODE == kGateUp) {
                 box3(slot, &maps.w[kind][0], x, tile * 8, z, bar);
@@ -245,105 +333,173 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
             } else {
                 box3(slot, &maps.w[kind][0], x, tile * 16, z, bar);
             }
-            box3(slot + a.sbOffset, &maps.sb[kind], (int)(askPart * kPart), tile * 16, z, bar);
+            box3(slot + a.sbOffset, &maps.sb[kind], (int)askPart, tile * 16, z, bar);
         }
         ++asked;
-        if (++askPart * kPart >= k.groups) {
+        askPart += k.part;
+        if (askPart >= k.groups) {
             askPart = 0;
-            askTask += (uint32_t)warps;
+            askAt.tile += (uint32_t)warps;
+            settle(askAt);
         }
     };
     ask();
     ask();
 
-    const float biasUnit = (t & 1) ? 0.0f : 1.52587890625e-5f;  // 2^-16
-    uint32_t used = 0;
-    for (uint32_t at = first; at < last;) {
-        const Segment seg = segment_of(at);
-        const int kind = seg.job ? 1 : 0, n = rows_of(seg);
-        const BlockKind &k = a.kind[kind];
-        const uint32_t segEnd = min(seg.end, last);
-        auto row_of = [&](int i) {  // row i of the segment: its route (routed) or token (shared)
-            const int r = (int)seg.rowGroup * kTaskRows + i;
-            return kind ? (int)sList[(seg.job - 1u) * kMaxGemvRows + (uint32_t)r] : r;
-        };
-        __syncthreads();  // the previous segment's digits are no longer read
-        // ---- stage the rows as digits, two runs in flight per thread ----
-        {
-            const int runsPerRow = (int)k.groups * 8, runs = n * runsPerRow;
-            auto fetch = [&](int i, bool ok) {
-                if (!ok) return make_uint4(0, 0, 0, 0);
-                const int r = i / runsPerRow;
-                int row = row_of(r);
-                if (MODE == kGateUp && kind) row /= a.K;  // a route's token
-                return __ldcg(reinterpret_cast<const uint4 *>(k.in + (size_t)row * k.inStride) + (i - r * runsPerRow));
+    // ---- input rows as digits: row r by warps [r per, (r + 1) per) ----
+    const float biasUnit = (t & 1) ? 0.0f : 1.52587890625e-5f;  // 2^-16 (INT8, see four_groups8)
+    auto stage = [&](const BlockKind &k, int kind, int n, auto row_of) {
+        const int per = warps / n, r = warp / per, threads = per * 32, tid = (int)threadIdx.x - r * threads;
+        const int runs = (int)k.groups * 8;
+        if (r >= n) return;
+        int row = row_of(r);
+        if (MODE == kGateUp && kind) row /= a.K;  // a route's token
+        const uint4 *src = reinterpret_cast<const uint4 *>(k.in + (size_t)row * k.inStride);
+        uint8_t *digits = smemRaw + a.digitsOffset + (size_t)r * a.rowBytes;
+        constexpr int kHeld = 3;  // runs a thread keeps between the two passes
+        uint4 held[kHeld];
+#pragma unroll
+        for (int i = 0; i < kHeld; ++i) {
+            held[i] = make_uint4(0, 0, 0, 0);
+            if (tid + i * threads < runs) held[i] = __ldcg(src + tid + i * threads);
+        }
+        if constexpr (INT8) {
+            GroupAux *rowAux = reinterpret_cast<GroupAux *>(smemRaw + a.auxOffset + (size_t)r * a.auxRow);
+            auto put = [&](int i, const uint4 &v) { digits_put<true>(i, i < runs, v, digits, rowAux + (i >> 3)); };
+#pragma unroll
+            for (int i = 0; i < kHeld; ++i)
+                if ((tid & ~31) + i * threads < runs) put(tid + i * threads, held[i]);  // the same for the whole warp
+            for (int i = tid + kHeld * threads; (i & ~31) < runs; i += threads) put(i, i < runs ? __ldcg(src + i) : make_uint4(0, 0, 0, 0));
+            const int padded = ((int)k.groups + 3) & ~3;  // groups past the row add nothing
+            if (tid < padded - (int)k.groups) rowAux[(int)k.groups + tid] = GroupAux{0.0f, 0.0f};
+        } else {
+            uint32_t top = 0;
+#pragma unroll
+            for (int i = 0; i < kHeld; ++i) top = max(top, top_exponent(held[i]));
+            for (int i = tid + kHeld * threads; i < runs; i += threads) top = max(top, top_exponent(__ldcg(src + i)));
+            top = __reduce_max_sync(0xFFFFFFFFu, top);
+            if (lane == 0) sTop[warp] = top;
+            named_barrier(2 + r, threads);
+            for (int w = 0; w < per; ++w) top = max(top, sTop[r * per + w]);
+            const RowScale scale = row_scale(top);
+            if (tid == 0) sUnit[r] = scale.unit;
+            // pair r / 2, columns 4 (r & 1).. of the sums
+            uint8_t *sums = smemRaw + a.auxOffset + (size_t)(r >> 1) * a.auxRow + (uint32_t)(r & 1) * 64u;
+            auto put = [&](int i, const uint4 &v) {
+                float sum = sum_of_run(v);
+#pragma unroll
+                for (int o = 1; o <= 4; o <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+                if (i >= runs) return;
+                digits_store<false>(i, v, scale.toInt, digits);
+                if ((i & 7) == 0) {
+                    const int group = i >> 3;
+                    uint16_t *dst = reinterpret_cast<uint16_t *>(sums + (uint32_t)(group >> 3) * kSumBlockBytes) + (group & 7);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {  // (a fourth piece: what is left, mostly zero)
+                        const uint16_t piece = f2bf(sum);
+                        dst[8 * c] = piece;
+                        sum -= bf2f(piece);
+                    }
+                }
             };
-            auto put = [&](int i, bool ok, const uint4 &v) {
-                const int r = ok ? i / runsPerRow : 0, in = ok ? i - r * runsPerRow : 0;
-                digits_put<INT8>(in, ok, v, smemRaw + a.digitsOffset + (size_t)r * a.rowBytes,
-                                 reinterpret_cast<GroupAux *>(smemRaw + a.auxOffset + (size_t)r * a.auxRow) + (in >> 3));
-            };
-            for (int base = warp * 32; base < runs; base += 2 * (int)blockDim.x) {
-                const int i = base + lane, j = i + (int)blockDim.x;
-                const uint4 v = fetch(i, i < runs), w = fetch(j, j < runs);
-                put(i, i < runs, v);
-                if (base + (int)blockDim.x < runs) put(j, j < runs, w);  // the same for the whole warp
-            }
-            // groups past the row, up to a batch of four: nothing is added for them
-            const int padded = ((int)k.groups + 3) & ~3;
-            for (int i = threadIdx.x; i < n * 4; i += blockDim.x) {
-                const int group = padded - 4 + (i & 3);
-                if (group >= (int)k.groups)
-                    *(reinterpret_cast<GroupAux *>(smemRaw + a.auxOffset + (size_t)(i >> 2) * a.auxRow) + group) = GroupAux{0.0f, 0.0f};
+#pragma unroll
+            for (int i = 0; i < kHeld; ++i)
+                if ((tid & ~31) + i * threads < runs) put(tid + i * threads, held[i]);  // the same for the whole warp
+            for (int i = tid + kHeld * threads; (i & ~31) < runs; i += threads) put(i, i < runs ? __ldcg(src + i) : make_uint4(0, 0, 0, 0));
+            // groups past the row up to a block of eight: their biases are zero, the sums have to be finite
+            const int past = (((int)k.groups + 7) & ~7) - (int)k.groups;
+            for (int i = tid; i < 4 * past; i += threads) {
+                const int group = (int)k.groups + (i >> 2);
+                *(reinterpret_cast<uint16_t *>(sums + (uint32_t)(group >> 3) * kSumBlockBytes) + (group & 7) + 8 * (i & 3)) = 0;
             }
         }
+    };
+
+    uint32_t used = 0, done = 0;  // done: tiles of this CTA's earlier segments, modulo the warps
+    while (before(at, end)) {
+        // a segment: the run's tiles of one row group
+        const int kind = kind_of(at.job), n = min(kTaskRows, rows_of(at.job) - (int)at.rowGroup * kTaskRows);
+        const BlockKind &k = a.kind[kind];
+        const bool same = at.job == end.job && at.rowGroup == end.rowGroup;
+        const uint32_t tileEnd = same ? end.tile : k.tiles;
+        const uint32_t listAt = kind ? (sJob[at.job] - 1u) * kMaxGemvRows + at.rowGroup * kTaskRows : at.rowGroup * kTaskRows;
+        auto row_of = [&](int i) { return kind ? (int)sList[listAt + (uint32_t)i] : (int)listAt + i; };  // row i: its route or token
+        __syncthreads();  // the previous segment's digits are no longer read
+        stage(k, kind, n, row_of);
         __syncthreads();
         // ---- this warp's tiles of the segment ----
-        const uint32_t phase = (at - first) % (uint32_t)warps;
-        uint32_t task = at + ((uint32_t)warp + (uint32_t)warps - phase) % (uint32_t)warps;
+        uint32_t tile = at.tile + ((uint32_t)warp + (uint32_t)warps - done) % (uint32_t)warps;
         auto run_tiles = [&](auto pairs) {
             constexpr int NT = decltype(pairs)::value;
-            for (; task < segEnd; task += (uint32_t)warps) {
-                float acc[NT][2];
+            for (; tile < tileEnd; tile += (uint32_t)warps) {
+                float acc[NT][2], accBias[NT][4];
                 uint32_t dig[NT], aux[NT];
 #pragma unroll
                 for (int j = 0; j < NT; ++j) {
                     acc[j][0] = acc[j][1] = 0.0f;
+                    accBias[j][0] = accBias[j][1] = accBias[j][2] = accBias[j][3] = 0.0f;
                     const int column = min(2 * j + (g >> 2), n - 1), mine = min(2 * j + (t >> 1), n - 1);
                     dig[j] = smem + a.digitsOffset + (uint32_t)column * a.rowBytes + (uint32_t)(g & 3) * 64u + (uint32_t)t * 16u;
-                    aux[j] = smem + a.auxOffset + (uint32_t)mine * a.auxRow;
+                    // INT8: the groups of the row this lane accounts for; INT4: its column's sums of the pair
+                    aux[j] = smem + a.auxOffset + (INT8 ? (uint32_t)mine * a.auxRow : (uint32_t)j * a.auxRow + (uint32_t)g * 16u + (uint32_t)t * 4u);
                 }
-                for (uint32_t p0 = 0; p0 < k.groups; p0 += kPart) {
+                for (uint32_t p0 = 0; p0 < k.groups; p0 += k.part) {
                     const uint32_t slot = slots + (used & 1u) * a.slotBytes;
                     uint32_t parity = (used >> 1) & 1u;
                     slot_wait(bars + 8u * (used & 1u), parity, a.errorFlag);
                     uint32_t lo = slot + (uint32_t)g * k.pitch + (INT8 ? 16u : 8u) * t, hi = lo + 8u * k.pitch;
                     uint32_t sb0 = slot + a.sbOffset + (uint32_t)g * k.sbWords * 4u, sb1 = sb0 + 32u * k.sbWords;
-                    const int batches = ((int)min(kPart, k.groups - p0) + 3) >> 2;
+                    const uint32_t inPart = min(k.part, k.groups - p0);
+                    if (!INT8) {
+                        uint32_t w0 = sb0 + 8u * (uint32_t)t, w1 = sb1 + 8u * (uint32_t)t;
 #pragma unroll 1
-                    for (int b = 0; b < batches; ++b) {
-                        four_groups<NT, INT8>(lo, hi, dig, sb0, sb1, aux, biasUnit, acc);
+                        for (uint32_t b = 0; b < inPart; b += 8) {
+                            const uint2 v0 = lds64(w0), v1 = lds64(w1);
+                            const uint32_t a0 = __byte_perm(v0.x, v0.y, 0x7632), a1 = __byte_perm(v1.x, v1.y, 0x7632);
+#pragma unroll
+                            for (int j = 0; j < NT; ++j) {
+                                uint32_t sum;
+                                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sum) : "r"(aux[j] + ((p0 + b) >> 3) * kSumBlockBytes));
+                                mma_1688(accBias[j], a0, a1, sum);
+                            }
+                            w0 += 32u;
+                            w1 += 32u;
+                        }
+                    }
+#pragma unroll 1
+                    for (uint32_t b = 0; b < inPart; b += 4) {
+                        if constexpr (INT8) {
+                            four_groups8<NT>(lo, hi, dig, sb0, sb1, aux, biasUnit, acc);
+#pragma unroll
+                            for (int j = 0; j < NT; ++j) aux[j] += 32u;
+                        } else {
+                            four_groups4<NT>(lo, hi, dig, sb0, sb1, acc);
+                        }
                         lo += 4u * kGroupBytes;
                         hi += 4u * kGroupBytes;
                         sb0 += 16u;
                         sb1 += 16u;
 #pragma unroll
-                        for (int j = 0; j < NT; ++j) {
-                            dig[j] += 4u * kDigitGroupBytes;
-                            aux[j] += 32u;
-                        }
+                        for (int j = 0; j < NT; ++j) dig[j] += 4u * kDigitGroupBytes;
                     }
                     slot_release();
                     ++used;
                     ask();
                 }
-                const uint32_t tile = task - seg.begin;
 #pragma unroll
                 for (int j = 0; j < NT; ++j) {
                     // lane (g, t = 0): the pair's first row, t = 2: its second
-                    const float r0 = fmaf(acc[j][0], 65536.0f, __shfl_xor_sync(0xFFFFFFFFu, acc[j][0], 1));
-                    const float r1 = fmaf(acc[j][1], 65536.0f, __shfl_xor_sync(0xFFFFFFFFu, acc[j][1], 1));
                     const int mine = 2 * j + (t >> 1);
+                    float r0 = fmaf(acc[j][0], 65536.0f, __shfl_xor_sync(0xFFFFFFFFu, acc[j][0], 1));
+                    float r1 = fmaf(acc[j][1], 65536.0f, __shfl_xor_sync(0xFFFFFFFFu, acc[j][1], 1));
+                    if (!INT8) {
+                        float b0 = accBias[j][0] + accBias[j][1], b1 = accBias[j][2] + accBias[j][3];
+                        b0 += __shfl_xor_sync(0xFFFFFFFFu, b0, 1);
+                        b1 += __shfl_xor_sync(0xFFFFFFFFu, b1, 1);
+                        const float unit = sUnit[min(mine, n - 1)];
+                        r0 = fmaf(r0, unit, b0);
+                        r1 = fmaf(r1, unit, b1);
+                    }
                     if ((t & 1) || mine >= n) continue;
                     uint16_t *dst = k.out + (size_t)row_of(mine) * k.outStride;
                     if (MODE == kGateUp) {
@@ -359,7 +515,10 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
         };
         if (n > 2) run_tiles(std::integral_constant<int, 2>{});
         else run_tiles(std::integral_constant<int, 1>{});
-        at = segEnd;
+        done = (done + tileEnd - at.tile) % (uint32_t)warps;
+        if (same) break;
+        at.tile = k.tiles;
+        settle(at);
     }
 }
 
@@ -379,9 +538,9 @@ bool encode3(CUtensorMap *map, CUtensorMapDataType type, const void *base, uint6
 
 // Slot row pitch of a kind: a part's bytes, padded so that a half-warp's reads fall on different banks
 // (INT4 64-bit reads of four rows: 32 or 96 modulo 128; INT8 128-bit reads of two rows: 64).
-uint32_t row_pitch(uint32_t groups, bool int8) {
-    if (!int8) return piece_stride(std::min(groups, kPartGroups) * 32);
-    uint32_t p = std::min(groups, kPartGroups8) * 64;
+uint32_t row_pitch(uint32_t part, bool int8) {
+    if (!int8) return piece_stride(part * 32);
+    uint32_t p = part * 64;
     while ((p & 127u) != 64u) p += 16;
     return p;
 }
@@ -390,12 +549,13 @@ uint32_t row_pitch(uint32_t groups, bool int8) {
 bool setup_kind(int mode, bool int8, BlockKind &k, CUtensorMap (&w)[2], CUtensorMap &sb, const uint8_t *w0, const uint8_t *w1,
                 uint32_t rows, uint32_t cols, uint32_t experts, uint64_t stride, const uint32_t *scales, uint64_t scaleStride,
                 const char **error) {
-    const uint32_t groups = cols / 64, padded = padded_groups(groups), part = int8 ? kPartGroups8 : kPartGroups;
+    const uint32_t groups = cols / 64, padded = padded_groups(groups);
     const uint64_t rowBytes = int8 ? cols : cols / 2;
     k.tiles = mode == kGateUp ? rows / 8 : rows / 16;
     k.groups = groups;
-    k.pitch = row_pitch(groups, int8);
-    k.sbWords = std::min(padded, part);
+    k.part = padded <= kPartGroups + 4 ? padded : kPartGroups;
+    k.pitch = row_pitch(k.part, int8);
+    k.sbWords = (k.part + 7u) & ~7u;  // (words past the row read as zero)
     const uint8_t *ws[2] = {w0, w1};
     for (int m = 0; m < (mode == kGateUp ? 2 : 1); ++m)
         if (!encode3(&w[m], CU_TENSOR_MAP_DATA_TYPE_UINT64, ws[m], rowBytes / 8, rows, experts, rowBytes, stride, k.pitch / 8,
@@ -421,19 +581,18 @@ bool launch_kernel(FFContext *ctx, BlockArgs a, const BlockMaps &maps, const cha
     a.digitsOffset = a.ids ? up128((uint32_t)a.E * kMaxGemvRows) : 0;
     a.rowBytes = padded * kDigitGroupBytes;
     a.auxOffset = a.digitsOffset + rows * a.rowBytes;
-    a.auxRow = padded * (uint32_t)sizeof(GroupAux);
-    a.slotsOffset = up128(a.auxOffset + rows * a.auxRow);
+    // INT8: a row's group entries; INT4: a pair's group sums
+    a.auxRow = INT8 ? padded * (uint32_t)sizeof(GroupAux) : (groups + 7u) / 8u * kSumBlockBytes;
+    a.slotsOffset = up128(a.auxOffset + (INT8 ? rows : (rows + 1u) / 2u) * a.auxRow);
     a.sbOffset = up128(slot);
     a.slotBytes = a.sbOffset + up128(sb);
-    const uint32_t limit = 227 * 1024 - 4096;  // less the static arrays
-    // (a batch of four groups may read up to three groups past a slot's last row: within the scale area
-    // or the next slot; behind the last slot a group's worth is kept)
-    const uint32_t slack = 3 * 64 * 2;
-    if (a.slotsOffset + 4 * 2 * a.slotBytes + slack > limit) return fail(error, "model shape too large for the block kernels' shared memory");
-    const uint32_t warps = std::min<uint32_t>(kMaxWarps, (limit - slack - a.slotsOffset) / (2 * a.slotBytes));
-    const size_t smem = a.slotsOffset + (size_t)warps * 2 * a.slotBytes + slack;
+    // (a batch of four groups may read up to three groups past a slot's last row, within the scale area)
+    constexpr uint32_t kLimit = 227 * 1024 - 6144;  // less the static arrays
+    if (a.slotsOffset + 4 * 2 * a.slotBytes > kLimit) return fail(error, "model shape too large for the block kernels' shared memory");
+    const uint32_t warps = std::min<uint32_t>(kMaxWarps, (kLimit - a.slotsOffset) / (2 * a.slotBytes));
+    const size_t smem = a.slotsOffset + (size_t)warps * 2 * a.slotBytes;
     static KernelSmemMemo memo;
-    if (!memo.prepare(k_block_int<MODE, INT8>, ctx->device, 227 * 1024 - 4096, kMaxWarps * 32, nullptr, error)) return false;
+    if (!memo.prepare(k_block_int<MODE, INT8>, ctx->device, kLimit, kMaxWarps * 32, nullptr, error)) return false;
     {
         LaunchScope scope(ctx, stream, name);
         k_block_int<MODE, INT8><<<ctx->smCount, warps * 32, smem, stream>>>(a, maps);

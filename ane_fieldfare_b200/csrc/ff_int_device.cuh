@@ -3,10 +3,11 @@
 // mma.sync m16n8k32 u8 x s8 takes the codes as bytes, straight from memory: the low nibbles of a word
 // are one AND away, the high ones another (they stay in place and count 16 times, which the input
 // makes up for) — two integer instructions for eight codes, where bf16 operands cost eight.  The input
-// row enters as integers: per group of 64 values x = V 2^-E with |V| < 2^30, V written as four signed
-// base-256 digits, one digit per MMA column.  A bf16 value has eight significant bits, so a value down
-// to 2^-19 of its group's largest is exact, a smaller one is off by less than 2^-27 of it, below what a
-// 32-bit floating sum of the products would round; the integer sums themselves are exact.
+// row enters as integers: per group of 64 values (or per row) x = V 2^-E with |V| < 2^30, V written as four
+// signed base-256 digits, one digit per MMA column.  A bf16 value has eight significant bits, so a value
+// down to 2^-19 of the largest is exact, a smaller one is off by less than 2^-27 of the largest (odd codes;
+// even ones 2^-31), below what a 32-bit floating sum of the products would round; the integer sums
+// themselves are exact.
 #pragma once
 
 #include "ff_mma_device.cuh"
@@ -28,45 +29,49 @@ struct alignas(8) GroupAux {
     float sum;   // sum of the group's values
 };
 
-// Eight consecutive bf16 values `v` (run `run` of a row, runs of a group in eight adjacent lanes; called
-// by whole warps, `valid` false for lanes past the row) as digits at `digits` and the group's `aux`.
-// Layout of a group: digit column c (0 = highest) at 64 c; inside, per 16 values [even 0..6 | even 8..14
-// | odd 1..7 | odd 9..15] — what lane (column, t) of the MMA loads as 16 bytes for the low and the high
-// nibbles of its eight packed bytes.
-template <bool INT8 = false>
-__device__ __forceinline__ void digits_put(int run, bool valid, const uint4 &v, uint8_t *digits, GroupAux *aux) {
-    // (aux: the run's group's entry)
+// The largest magnitude's bf16 bits among eight values.
+__device__ __forceinline__ uint32_t top_exponent(const uint4 &v) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-    float x[8];
     uint32_t top = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        x[2 * i] = __uint_as_float(w[i] << 16);
-        x[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-        top = max(top, max(w[i] & 0x7FFFu, (w[i] >> 16) & 0x7FFFu));
-    }
-    float sum = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+    for (int i = 0; i < 4; ++i) top = max(top, max(w[i] & 0x7FFFu, (w[i] >> 16) & 0x7FFFu));
+    return top;
+}
+__device__ __forceinline__ float sum_of_run(const uint4 &v) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    float p[4];
 #pragma unroll
-    for (int o = 1; o <= 4; o <<= 1) {
-        top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
-        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-    }
-    // |x| < 2^(e - 126) for exponent field e: E = 156 - e, held to what a float can carry
+    for (int i = 0; i < 4; ++i) p[i] = __uint_as_float(w[i] << 16) + __uint_as_float(w[i] & 0xFFFF0000u);
+    return (p[0] + p[1]) + (p[2] + p[3]);
+}
+// 2^E for values up to `top` (bf16 bits): |x| < 2^(e - 126) for exponent field e, E = 156 - e held to what a
+// float can carry; `unit` = 2^-E, NaN when there is an infinity or a NaN among them.
+struct RowScale {
+    float toInt, unit;
+};
+__device__ __forceinline__ RowScale row_scale(uint32_t top) {
     const int e = (int)(top >> 7), E = min(156 - e, 126);
-    const float scale = __int_as_float((E + 127) << 23), scaleOdd = INT8 ? scale : scale * 0.0625f;
+    return RowScale{__int_as_float((E + 127) << 23), e == 255 ? __int_as_float(0x7FFFFFFF) : __int_as_float((127 - E) << 23)};
+}
+
+// Eight consecutive bf16 values `v` (run `run` of a row) as digits.  Layout of a group: digit column c (0 =
+// highest) at 64 c; inside, per 16 values [even 0..6 | even 8..14 | odd 1..7 | odd 9..15] — what lane
+// (column, t) of the MMA loads as 16 bytes for the low and the high nibbles of its eight packed bytes.
+// INT8: values in their own order.
+template <bool INT8>
+__device__ __forceinline__ void digits_store(int run, const uint4 &v, float scale, uint8_t *digits) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    const float scaleOdd = INT8 ? scale : scale * 0.0625f;
     uint32_t U[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         // balanced digits: bytes of V + 0x808080, the lower three less 128
-        const uint32_t V = (uint32_t)__float2int_rn(x[i] * ((i & 1) ? scaleOdd : scale));
+        const float x = __uint_as_float((i & 1) ? w[i >> 1] & 0xFFFF0000u : w[i >> 1] << 16);
+        const uint32_t V = (uint32_t)__float2int_rn(x * ((i & 1) ? scaleOdd : scale));
         U[i] = (V + 0x00808080u) ^ 0x00808080u;
     }
-    if (!valid) return;
-    uint8_t *dst = digits + (size_t)(run >> 3) * kDigitGroupBytes + (run & 7) / 2 * 16 + (run & 1) * 4;
-    if (INT8) {
-        // codes in their own order: values 16 t + 0..3 | 4..7 | 8..11 | 12..15 of a quarter
-        dst += (run & 1) * 4;  // (a run is eight bytes there)
-    }
+    // (INT8: a run is eight bytes, 16 t + 0..3 | 4..7 | 8..11 | 12..15 of a quarter)
+    uint8_t *dst = digits + (size_t)(run >> 3) * kDigitGroupBytes + (run & 7) / 2 * 16 + (run & 1) * (INT8 ? 8 : 4);
 #pragma unroll
     for (int odd = 0; odd < 2; ++odd) {
         const uint32_t u0 = INT8 ? U[4 * odd] : U[odd], u1 = INT8 ? U[4 * odd + 1] : U[2 + odd],
@@ -79,7 +84,23 @@ __device__ __forceinline__ void digits_put(int run, bool valid, const uint4 &v, 
         *reinterpret_cast<uint32_t *>(at + 64) = __byte_perm(h0, h1, 0x5410);
         *reinterpret_cast<uint32_t *>(at) = __byte_perm(h0, h1, 0x7632);
     }
-    if ((run & 7) == 0) *aux = GroupAux{e == 255 ? __int_as_float(0x7FFFFFFF) : __int_as_float((127 - E) << 23), sum};
+}
+
+// A run with its group's own scale, and the group's `aux` (runs of a group in eight adjacent lanes; called by
+// whole warps, `valid` false for lanes past the row).
+template <bool INT8 = false>
+__device__ __forceinline__ void digits_put(int run, bool valid, const uint4 &v, uint8_t *digits, GroupAux *aux) {
+    uint32_t top = top_exponent(v);
+    float sum = sum_of_run(v);
+#pragma unroll
+    for (int o = 1; o <= 4; o <<= 1) {
+        top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
+        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    }
+    if (!valid) return;
+    const RowScale scale = row_scale(top);
+    digits_store<INT8>(run, v, scale.toInt, digits);
+    if ((run & 7) == 0) *aux = GroupAux{scale.unit, sum};
 }
 
 // (shared-memory addresses: the tile function is not inlined, so a pointer would be a generic one)
