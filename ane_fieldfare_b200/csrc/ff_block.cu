@@ -62,8 +62,9 @@ struct BlockArgs {
 };
 
 struct alignas(64) BlockMaps {
-    CUtensorMap w[2][2];  // [kind][gate, up] or [kind][down]
-    CUtensorMap sb[2];
+    struct {
+        CUtensorMap w[3];  // gate, up | down, -; scale words
+    } kind[2];
 };
 
 __device__ __forceinline__ void box3(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
@@ -190,6 +191,8 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
     const int g = lane >> 2, t = lane & 3;
     const uint32_t smem = sm_addr(smemRaw);
     constexpr uint32_t kGroupBytes = INT8 ? 64 : 32;
+    if (!(MODE == kDown)) pdl_wait();  // (the down kernel's plan and first weights need only what was there before its predecessor)
+    if (MODE == kGateUp) pdl_trigger();
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2 * kMaxWarps; ++i) bar_init(sm_addr(&sBar[i]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -267,7 +270,10 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
         if (MODE == kGateUp && threadIdx.x == 0 && blockIdx.x == 0 && a.activeExperts) *a.activeExperts = nJobs - (a.withShared ? 1u : 0u);
     }
     __syncthreads();
-    if (nJobs == 0) return;
+    if (nJobs == 0) {
+        pdl_wait();
+        return;
+    }
 
     // A tile of four input rows (`rowGroup`) of a job; tiles in order are a CTA's run.
     struct Place {
@@ -316,31 +322,41 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
     const uint32_t bars = sm_addr(&sBar[2 * warp]);
     Place askAt = at;
     askAt.tile += (uint32_t)warp;
-    settle(askAt);
-    uint32_t askPart = 0, asked = 0;
-    auto ask = [&]() {
+    uint32_t askLimit = 0, askX = 0, askGroups = 0, askPart = 0, askBytes = 0, askHalf = 0, asked = 0;
+    int askZ = 0;
+    const CUtensorMap *askMap = nullptr;
+    // the next row group the warp has a tile in, or none (askLimit 0)
+    auto seek = [&]() {
+        settle(askAt);
+        askLimit = 0;
         if (!before(askAt, end)) return;
         const int kind = kind_of(askAt.job);
         const BlockKind &k = a.kind[kind];
+        askLimit = askAt.job == end.job && askAt.rowGroup == end.rowGroup ? end.tile : k.tiles;
+        askGroups = k.groups;
+        askPart = k.part;
+        askBytes = 16u * k.pitch + 64u * k.sbWords;
+        askHalf = 8u * k.pitch;
+        askZ = kind ? (int)sJob[askAt.job] - 1 : 0;
+        askMap = &maps.kind[kind].w[0];
+    };
+    seek();
+    auto ask = [&]() {
+        if (askLimit == 0) return;
         if (lane == 0) {
             const uint32_t slot = slots + (asked & 1u) * a.slotBytes, bar = bars + 8u * (asked & 1u);
-            const int tile = (int)askAt.tile, z = kind ? (int)sJob[askAt.job] - 1 : 0;
-            const int x = (int)(askPart * kGroupBytes / 8u);
-            bar_expect(bar, 16u * k.pitch + 64u * k.sbWords);
-            if (MODE == kGateUp) {
-                box3(slot, &maps.w[kind][0], x, tile * 8, z, bar);
-                box3(slot + 8u * k.pitch, &maps.w[kind][1], x, tile * 8, z, bar);
-            } else {
-                box3(slot, &maps.w[kind][0], x, tile * 16, z, bar);
-            }
-            box3(slot + a.sbOffset, &maps.sb[kind], (int)askPart, tile * 16, z, bar);
+            const int row = (int)askAt.tile * (MODE == kGateUp ? 8 : 16), x = (int)(askX * (kGroupBytes / 8u));
+            bar_expect(bar, askBytes);
+            box3(slot, askMap, x, row, askZ, bar);
+            if (MODE == kGateUp) box3(slot + askHalf, askMap + 1, x, row, askZ, bar);
+            box3(slot + a.sbOffset, askMap + 2, (int)askX, (int)askAt.tile * 16, askZ, bar);
         }
         ++asked;
-        askPart += k.part;
-        if (askPart >= k.groups) {
-            askPart = 0;
+        askX += askPart;
+        if (askX >= askGroups) {
+            askX = 0;
             askAt.tile += (uint32_t)warps;
-            settle(askAt);
+            if (askAt.tile >= askLimit) seek();
         }
     };
     ask();
@@ -415,6 +431,10 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
         }
     };
 
+    if (MODE == kDown) {
+        pdl_wait();  // from here on: the activations
+        pdl_trigger();
+    }
     uint32_t used = 0, done = 0;  // done: tiles of this CTA's earlier segments, modulo the warps
     while (before(at, end)) {
         // a segment: the run's tiles of one row group
@@ -429,6 +449,8 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
         __syncthreads();
         // ---- this warp's tiles of the segment ----
         uint32_t tile = at.tile + ((uint32_t)warp + (uint32_t)warps - done) % (uint32_t)warps;
+        const uint32_t groups = k.groups, part = k.part, half = 8u * k.pitch, sbHalf = 32u * k.sbWords;
+        const uint32_t rowAt = (uint32_t)g * k.pitch + (INT8 ? 16u : 8u) * (uint32_t)t, sbAt = a.sbOffset + (uint32_t)g * k.sbWords * 4u;
         auto run_tiles = [&](auto pairs) {
             constexpr int NT = decltype(pairs)::value;
             for (; tile < tileEnd; tile += (uint32_t)warps) {
@@ -443,13 +465,13 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
                     // INT8: the groups of the row this lane accounts for; INT4: its column's sums of the pair
                     aux[j] = smem + a.auxOffset + (INT8 ? (uint32_t)mine * a.auxRow : (uint32_t)j * a.auxRow + (uint32_t)g * 16u + (uint32_t)t * 4u);
                 }
-                for (uint32_t p0 = 0; p0 < k.groups; p0 += k.part) {
+                for (uint32_t p0 = 0; p0 < groups; p0 += part) {
                     const uint32_t slot = slots + (used & 1u) * a.slotBytes;
                     uint32_t parity = (used >> 1) & 1u;
                     slot_wait(bars + 8u * (used & 1u), parity, a.errorFlag);
-                    uint32_t lo = slot + (uint32_t)g * k.pitch + (INT8 ? 16u : 8u) * t, hi = lo + 8u * k.pitch;
-                    uint32_t sb0 = slot + a.sbOffset + (uint32_t)g * k.sbWords * 4u, sb1 = sb0 + 32u * k.sbWords;
-                    const uint32_t inPart = min(k.part, k.groups - p0);
+                    uint32_t lo = slot + rowAt, hi = lo + half;
+                    uint32_t sb0 = slot + sbAt, sb1 = sb0 + sbHalf;
+                    const uint32_t inPart = min(part, groups - p0);
                     if (!INT8) {
                         uint32_t w0 = sb0 + 8u * (uint32_t)t, w1 = sb1 + 8u * (uint32_t)t;
 #pragma unroll 1
@@ -546,7 +568,7 @@ uint32_t row_pitch(uint32_t part, bool int8) {
 }
 
 // Fills a kind and its maps.  mode kGateUp: w0, w1 [rows][cols], tiles of 8 + 8 rows; kDown: w0, 16 rows.
-bool setup_kind(int mode, bool int8, BlockKind &k, CUtensorMap (&w)[2], CUtensorMap &sb, const uint8_t *w0, const uint8_t *w1,
+bool setup_kind(int mode, bool int8, BlockKind &k, CUtensorMap (&w)[3], const uint8_t *w0, const uint8_t *w1,
                 uint32_t rows, uint32_t cols, uint32_t experts, uint64_t stride, const uint32_t *scales, uint64_t scaleStride,
                 const char **error) {
     const uint32_t groups = cols / 64, padded = padded_groups(groups);
@@ -562,7 +584,7 @@ bool setup_kind(int mode, bool int8, BlockKind &k, CUtensorMap (&w)[2], CUtensor
                      mode == kGateUp ? 8 : 16, error))
             return false;
     const uint64_t scaleRows = mode == kGateUp ? (uint64_t)rows * 2 : rows;
-    return encode3(&sb, CU_TENSOR_MAP_DATA_TYPE_UINT32, scales, padded, scaleRows, experts, (uint64_t)padded * 4,
+    return encode3(&w[2], CU_TENSOR_MAP_DATA_TYPE_UINT32, scales, padded, scaleRows, experts, (uint64_t)padded * 4,
                    experts > 1 ? scaleStride * 4 : scaleRows * padded * 4, k.sbWords, 16, error);
 }
 
@@ -595,9 +617,8 @@ bool launch_kernel(FFContext *ctx, BlockArgs a, const BlockMaps &maps, const cha
     if (!memo.prepare(k_block_int<MODE, INT8>, ctx->device, kLimit, kMaxWarps * 32, nullptr, error)) return false;
     {
         LaunchScope scope(ctx, stream, name);
-        k_block_int<MODE, INT8><<<ctx->smCount, warps * 32, smem, stream>>>(a, maps);
+        FF_CUDA_OK(launch_pdl(k_block_int<MODE, INT8>, ctx->smCount, warps * 32, smem, stream, a, maps), error);
     }
-    FF_CUDA_OK(cudaGetLastError(), error);
     return true;
 }
 
@@ -627,7 +648,7 @@ bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
         if (ids) {
             const uint32_t *o = &L.off.gateWOff;
             BlockKind &k = a.kind[1];
-            if (!setup_kind(mode, false, k, maps.w[1], maps.sb[1], L.experts + (down ? o[6] : o[0]), L.experts + o[3], down ? c.d : c.f,
+            if (!setup_kind(mode, false, k, maps.kind[1].w, L.experts + (down ? o[6] : o[0]), L.experts + o[3], down ? c.d : c.f,
                             down ? c.f : c.d, L.expertCount, L.stride,
                             L.routedScales + (down ? (uint64_t)(c.f / 8) * 16 * padded_groups(c.d / 64) : 0), words, error))
                 return false;
@@ -639,7 +660,7 @@ bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
         if (withShared) {
             const uint32_t *o = &L.sharedOff.gateWOff;
             BlockKind &k = a.kind[0];
-            if (!setup_kind(mode, false, k, maps.w[0], maps.sb[0], L.shared + (down ? o[6] : o[0]), L.shared + o[3], down ? c.d : c.sharedF,
+            if (!setup_kind(mode, false, k, maps.kind[0].w, L.shared + (down ? o[6] : o[0]), L.shared + o[3], down ? c.d : c.sharedF,
                             down ? c.sharedF : c.d, 1, (uint64_t)c.d * c.sharedF / 2,
                             L.sharedScales + (down ? (uint64_t)(c.sharedF / 8) * 16 * padded_groups(c.d / 64) : 0), 0, error))
                 return false;
@@ -669,7 +690,7 @@ bool launch_block_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
         a.errorFlag = ctx->errorFlag;
         const bool down = mode == kDown;
         BlockKind &k = a.kind[0];
-        if (!setup_kind(mode, true, k, maps.w[0], maps.sb[0], L.shared8W[down ? 2 : 0], L.shared8W[1], down ? c.d : c.sharedF,
+        if (!setup_kind(mode, true, k, maps.kind[0].w, L.shared8W[down ? 2 : 0], L.shared8W[1], down ? c.d : c.sharedF,
                         down ? c.sharedF : c.d, 1, (uint64_t)c.d * c.sharedF,
                         L.sharedScales + (down ? (uint64_t)(c.sharedF / 8) * 16 * padded_groups(c.d / 64) : 0), 0, error))
             return false;

@@ -128,6 +128,7 @@ k_int4_gemv(const GemvJob *jobs, const uint32_t *items, const uint32_t *itemCoun
 __global__ void __launch_bounds__(256)
 k_router_logits(const uint16_t *W, const uint16_t *scale, const float *bias, const uint16_t *x,
                 uint32_t xStride, int E, int D, float *logits) {
+    pdl_enter();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e = blockIdx.x * 8 + warp;
     const int t = blockIdx.y;
@@ -162,6 +163,7 @@ k_router_logits(const uint16_t *W, const uint16_t *scale, const float *bias, con
 // Top-K of 1..16 rows' logits, one warp per row.
 __global__ void __launch_bounds__(512) k_topk_small(const float *logits, const uint16_t *gain, int T, int E, int K, uint32_t *ids,
                                                     uint16_t *weights) {
+    pdl_enter();
     const int t = threadIdx.x >> 5;
     if (t < T) warp_topk(logits + (size_t)t * E, E, K, gain, ids + t * K, weights + t * K);
 }
@@ -198,6 +200,7 @@ k_reduce_token_major(const uint16_t *partials, const uint32_t *rowIndex, const u
 __global__ void __launch_bounds__(256)
 k_reduce_token_major_x8(const uint16_t *partials, const uint32_t *rowIndex, const uint16_t *weights,
                         const uint16_t *residual, uint16_t *y, int T, int K, int D) {
+    pdl_enter();
     const int perRow = D >> 3;
     const size_t item = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (item >= (size_t)T * perRow) return;
@@ -309,6 +312,7 @@ __device__ __forceinline__ float row_rms_inv(const uint16_t *row, int D, float e
 template <int C, bool WIDE>
 __global__ void __launch_bounds__(kRowThreads)
 k_rmsnorm(const uint16_t *x, const uint16_t *w, float eps, int D, uint16_t *y) {
+    pdl_enter();
     extern __shared__ __align__(16) uint16_t glueRow[];
     __shared__ float warpSums[kRowThreads / 32];
     const size_t row = (size_t)blockIdx.x * D;
@@ -335,6 +339,7 @@ k_rmsnorm(const uint16_t *x, const uint16_t *w, float eps, int D, uint16_t *y) {
 // The same for rows too wide for the row buffer.
 __global__ void __launch_bounds__(kRowThreads)
 k_rmsnorm_long(const uint16_t *x, const uint16_t *w, float eps, int D, uint16_t *y) {
+    pdl_enter();
     __shared__ float warpSums[kRowThreads / 32];
     const size_t row = (size_t)blockIdx.x * D;
     const float inv = row_rms_inv(x + row, D, eps, warpSums);
@@ -350,6 +355,7 @@ __global__ void __launch_bounds__(kRowThreads)
 k_post_attn_setup(uint16_t *hidden, const uint16_t *attn, const uint16_t *wPostAttn, const uint16_t *wPreFfn,
                   const uint16_t *wPreFfn2, float eps, int D, uint16_t *denseX, uint16_t *routedX,
                   uint16_t *routerX) {
+    pdl_enter();
     extern __shared__ __align__(16) uint16_t glueRow[];
     __shared__ float warpSums[kRowThreads / 32];
     const size_t row = (size_t)blockIdx.x * D;
@@ -396,6 +402,7 @@ template <int C, bool WIDE>
 __global__ void __launch_bounds__(kRowThreads)
 k_layer_tail(const uint16_t *h2, const uint16_t *h1, uint16_t *hidden, const uint16_t *wPostFfn2,
              const uint16_t *wPostFfn, float eps, float layerScalar, int D) {
+    pdl_enter();
     extern __shared__ __align__(16) uint16_t glueRow[];
     __shared__ float warpSums[kRowThreads / 32];
     const size_t row = (size_t)blockIdx.x * D;
@@ -442,7 +449,7 @@ k_layer_tail(const uint16_t *h2, const uint16_t *h1, uint16_t *hidden, const uin
         auto go_ = [&](auto kernel, KernelSmemMemo &memo) {                                                            \
             if (!memo.prepare(kernel, ctx->device, smem_, kRowThreads, nullptr, error)) return false;                  \
             LaunchScope scope(ctx, stream, #NAME);                                                                     \
-            kernel<<<tokens, kRowThreads, smem_, stream>>>(__VA_ARGS__);                                               \
+            FF_CUDA_OK(launch_pdl(kernel, tokens, kRowThreads, smem_, stream, __VA_ARGS__), error);                      \
             return true;                                                                                               \
         };                                                                                                             \
         const bool ok_ = (D) <= 4096    ? ((WIDE) ? go_(k_##NAME<2, true>, memo_[0]) : go_(k_##NAME<2, false>, memo_[1]))  \
@@ -754,12 +761,16 @@ bool launch_router_topk(FFContext *ctx, const LayerStore &L, const uint16_t *x, 
     } else {
         dim3 grid((E + 7) / 8, tokens);
         LaunchScope scope(ctx, stream, "router_logits");
-        k_router_logits<<<grid, 256, 0, stream>>>(L.routerW, L.routerScale, L.logitBias, x, xStride,
-                                                  E, D, lg);
+        FF_CUDA_OK(launch_pdl(k_router_logits, grid, 256, 0, stream,
+                              L.routerW, L.routerScale, L.logitBias, x, xStride,
+                                                  E, D, lg),
+                   error);
     }
     {
         LaunchScope scope(ctx, stream, "topk");
-        k_topk_small<<<1, 512, 0, stream>>>(lg, L.gain, (int)tokens, E, (int)ctx->cfg.topK, ids, weights);
+        FF_CUDA_OK(launch_pdl(k_topk_small, 1, 512, 0, stream,
+                              lg, L.gain, (int)tokens, E, (int)ctx->cfg.topK, ids, weights),
+                   error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
     return true;
@@ -800,8 +811,9 @@ bool launch_reduce(FFContext *ctx, const uint16_t *partials, const uint16_t *wei
         LaunchScope scope(ctx, stream, "reduce_token_major");
         if (wide) {
             const size_t items = (size_t)tokens * (D / 8);
-            k_reduce_token_major_x8<<<(unsigned)((items + 255) / 256), 256, 0, stream>>>(
-                partials, rowIndex, weights, residual, y, (int)tokens, (int)ctx->cfg.topK, D);
+            FF_CUDA_OK(launch_pdl(k_reduce_token_major_x8, (unsigned)((items + 255) / 256), 256, 0, stream,
+                              partials, rowIndex, weights, residual, y, (int)tokens, (int)ctx->cfg.topK, D),
+                   error);
         } else {
             dim3 grid((D / 2 + 255) / 256, tokens);
             k_reduce_token_major<<<grid, 256, 0, stream>>>(partials, rowIndex, weights, residual, y, (int)tokens,

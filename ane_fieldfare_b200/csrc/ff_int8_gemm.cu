@@ -87,6 +87,7 @@ __device__ __forceinline__ float sum8(const uint4 &v) {
 // Group sums of x's rows; eight neighbouring threads hold one group.  Memory bound (x once).
 __global__ void __launch_bounds__(256)
 k_group_sums(const uint16_t *x, uint32_t xStride, uint32_t rows, uint32_t D, uint16_t *sums) {
+    pdl_enter();
     const uint32_t chunks = D / 8, pitch = sums_pitch(D);
     const size_t total = (size_t)rows * chunks;
     // (total, the block and the grid stride are multiples of eight: a group's threads stay together)
@@ -167,6 +168,7 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
     cluster_sync_all();
     tc_fence_after();
     const uint32_t tmemBase = tmemBaseSlot;
+    pdl_enter();
 
     // A pair's unit: one token tile, two neighbouring weight-row tiles (this CTA takes 2 np + rank).
     const uint32_t nPairs = (args.nTiles + 1u) >> 1, units = args.rowTiles * nPairs;
@@ -516,7 +518,9 @@ bool launch_one(FFContext *ctx, const CUtensorMap &tok, const CUtensorMap &sums,
     const uint32_t grid = 2u * std::max(1u, std::min(clusters, args.rowTiles * nPairs));
     {
         LaunchScope scope(ctx, stream, MODE == kGateUp ? "int8_gemm_gate_up_act" : "int8_gemm_down");
-        k_int8_gemm<MODE><<<grid, kThreads, smem, stream>>>(tok, sums, w0, w1, args);
+        FF_CUDA_OK(launch_pdl(k_int8_gemm<MODE>, grid, kThreads, smem, stream,
+                              tok, sums, w0, w1, args),
+                   error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
     return true;
@@ -537,7 +541,9 @@ bool launch_shared_int8_gemm(FFContext *ctx, const LayerStore &L, const uint16_t
         LaunchScope scope(ctx, stream, "group_sums");
         const size_t threads = (size_t)tokens * (c.d / 8);
         const unsigned blocks = (unsigned)std::min<size_t>((threads + 255) / 256, (size_t)ctx->smCount * 8);
-        k_group_sums<<<blocks, 256, 0, stream>>>(x, xStride, tokens, c.d, ctx->xSums);
+        FF_CUDA_OK(launch_pdl(k_group_sums, blocks, 256, 0, stream,
+                              x, xStride, tokens, c.d, ctx->xSums),
+                   error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
     CUtensorMap tok, sums, w[2];

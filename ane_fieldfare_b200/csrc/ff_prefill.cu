@@ -310,6 +310,7 @@ __device__ __forceinline__ void segment_histogram(const uint32_t *routes, int n,
 // Pass 1: per block of 256 tokens, how many routes name each expert.
 __global__ void __launch_bounds__(256)
 k_route_count(const uint32_t *ids, int T, int K, int E, uint32_t *blockCounts) {
+    pdl_enter();
     extern __shared__ uint32_t sRoutes[];
     __shared__ uint32_t segCount[8 * kMaxExperts];
     const int t0 = blockIdx.x * kSortTokens;
@@ -333,6 +334,7 @@ k_route_count(const uint32_t *ids, int T, int K, int E, uint32_t *blockCounts) {
 __global__ void __launch_bounds__(256)
 k_route_scan(uint32_t *blockCounts, int blocks, int E, uint32_t *expertOffsets, RowTile *tiles,
              uint32_t maxTiles, uint32_t *counts) {
+    pdl_enter();
     __shared__ uint32_t total[kMaxExperts];
     __shared__ uint32_t offset[kMaxExperts + 1];
     __shared__ uint32_t tileBase[kMaxExperts + 1];
@@ -387,6 +389,7 @@ __global__ void __launch_bounds__(256)
 k_route_scatter(const uint32_t *ids, const uint16_t *weights, int T, int K, int E,
                 const uint32_t *blockCounts, const uint32_t *expertOffsets,
                 FFTokenExpertPair *sorted) {
+    pdl_enter();
     extern __shared__ uint32_t sRoutes[];
     __shared__ uint32_t segCount[8 * kMaxExperts];
     const int t0 = blockIdx.x * kSortTokens;
@@ -431,6 +434,7 @@ k_route_scatter(const uint32_t *ids, const uint16_t *weights, int T, int K, int 
 
 // Row tiles of a dense problem: T rows of one "expert" (the shared FFN).
 __global__ void k_dense_tiles(int T, RowTile *tiles, uint32_t *counts) {
+    pdl_enter();
     const int n = (T + (int)kRowTile - 1) / (int)kRowTile;
     for (int i = threadIdx.x; i < n; i += blockDim.x)
         tiles[i] = RowTile{(uint32_t)i * kRowTile, (uint32_t)min((int)kRowTile, T - i * (int)kRowTile), 0u, 0u};
@@ -448,6 +452,7 @@ __global__ void k_dense_tiles(int T, RowTile *tiles, uint32_t *counts) {
 __global__ void __launch_bounds__(256)
 k_gather_rows(const uint16_t *x, uint32_t xStride, const FFTokenExpertPair *pairs,
               const uint32_t *rowCountPtr, uint32_t rowCount, int D, uint16_t *out) {
+    pdl_enter();
     const uint32_t rows = rowCountPtr ? rowCountPtr[1] : rowCount;
     const int chunksPerRow = D / 8;
     const size_t total = (size_t)rows * chunksPerRow;
@@ -603,6 +608,7 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
     cluster_sync_all();  // the other CTA's barriers are initialised before anything arrives on them
     tc_fence_after();
     const uint32_t tmemBase = tmemBaseSlot;
+    pdl_enter();
 
     // A pair's unit: one row tile, two neighbouring weight-row tiles (this CTA takes 2 np + rank).
     const uint32_t rowTiles = args.counts[0];
@@ -1065,7 +1071,9 @@ static bool launch_gemm(FFContext *ctx, const CUtensorMap &mapA, const CUtensorM
     const uint32_t grid = 2u * std::max(1u, std::min<uint32_t>((uint32_t)ctx->smCount / 2u, pairUnits));
     {
         LaunchScope scope(ctx, stream, MODE == kModeGateUp ? "int4_gemm_gate_up_act" : "int4_gemm_down");
-        kernel<<<grid, kGemmThreads, smem, stream>>>(mapA, mapW0, mapW1, args);
+        FF_CUDA_OK(launch_pdl(kernel, grid, kGemmThreads, smem, stream,
+                              mapA, mapW0, mapW1, args),
+                   error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
     return true;
@@ -1091,23 +1099,31 @@ bool launch_prefill_routed(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     const uint32_t maxTiles = ctx->maxUnits / 2;  // first half of the tile buffer
     {
         LaunchScope scope(ctx, stream, "route_count");
-        k_route_count<<<blocks, 256, sortSmem, stream>>>(ids, T, K, E, ctx->blockCounts);
+        FF_CUDA_OK(launch_pdl(k_route_count, blocks, 256, sortSmem, stream,
+                              ids, T, K, E, ctx->blockCounts),
+                   error);
     }
     {
         LaunchScope scope(ctx, stream, "route_scan");
-        k_route_scan<<<1, 256, 0, stream>>>(ctx->blockCounts, (int)blocks, E, ctx->expertOffsets, tiles,
-                                            maxTiles, ctx->unitCount);
+        FF_CUDA_OK(launch_pdl(k_route_scan, 1, 256, 0, stream,
+                              ctx->blockCounts, (int)blocks, E, ctx->expertOffsets, tiles,
+                                            maxTiles, ctx->unitCount),
+                   error);
     }
     {
         LaunchScope scope(ctx, stream, "route_scatter");
-        k_route_scatter<<<blocks, 256, sortSmem, stream>>>(ids, nullptr, T, K, E, ctx->blockCounts,
-                                                           ctx->expertOffsets, ctx->sortedPairs);
+        FF_CUDA_OK(launch_pdl(k_route_scatter, blocks, 256, sortSmem, stream,
+                              ids, nullptr, T, K, E, ctx->blockCounts,
+                                                           ctx->expertOffsets, ctx->sortedPairs),
+                   error);
     }
     const uint32_t pairs = tokens * c.topK;
     {
         LaunchScope scope(ctx, stream, "gather_rows");
-        k_gather_rows<<<ctx->smCount * 8, 256, 0, stream>>>(x, xStride, ctx->sortedPairs, nullptr, pairs,
-                                                            (int)c.d, ctx->xSorted);
+        FF_CUDA_OK(launch_pdl(k_gather_rows, ctx->smCount * 8, 256, 0, stream,
+                              x, xStride, ctx->sortedPairs, nullptr, pairs,
+                                                            (int)c.d, ctx->xSorted),
+                   error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
 
@@ -1166,17 +1182,23 @@ bool launch_route_sort(FFContext *ctx, const uint32_t *groupIds, uint32_t tokens
     RowTile *tiles = reinterpret_cast<RowTile *>(ctx->units);
     {
         LaunchScope scope(ctx, stream, "route_count");
-        k_route_count<<<blocks, 256, sortSmem, stream>>>(groupIds, T, K, E, ctx->blockCounts);
+        FF_CUDA_OK(launch_pdl(k_route_count, blocks, 256, sortSmem, stream,
+                              groupIds, T, K, E, ctx->blockCounts),
+                   error);
     }
     {
         LaunchScope scope(ctx, stream, "route_scan");
-        k_route_scan<<<1, 256, 0, stream>>>(ctx->blockCounts, (int)blocks, E, offsets, tiles, ctx->maxUnits / 2,
-                                            ctx->unitCount);
+        FF_CUDA_OK(launch_pdl(k_route_scan, 1, 256, 0, stream,
+                              ctx->blockCounts, (int)blocks, E, offsets, tiles, ctx->maxUnits / 2,
+                                            ctx->unitCount),
+                   error);
     }
     {
         LaunchScope scope(ctx, stream, "route_scatter");
-        k_route_scatter<<<blocks, 256, sortSmem, stream>>>(groupIds, nullptr, T, K, E, ctx->blockCounts, offsets,
-                                                           sortedPairs);
+        FF_CUDA_OK(launch_pdl(k_route_scatter, blocks, 256, sortSmem, stream,
+                              groupIds, nullptr, T, K, E, ctx->blockCounts, offsets,
+                                                           sortedPairs),
+                   error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
     return true;
@@ -1194,12 +1216,16 @@ bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     uint32_t *counts = ctx->unitCount + 4;
     {
         LaunchScope scope(ctx, stream, "dense_tiles");
-        k_dense_tiles<<<1, 256, 0, stream>>>((int)tokens, tiles, counts);
+        FF_CUDA_OK(launch_pdl(k_dense_tiles, 1, 256, 0, stream,
+                              (int)tokens, tiles, counts),
+                   error);
     }
     {
         LaunchScope scope(ctx, stream, "gather_rows");
-        k_gather_rows<<<ctx->smCount * 8, 256, 0, stream>>>(x, xStride, nullptr, nullptr, tokens,
-                                                            (int)c.d, ctx->xSorted);
+        FF_CUDA_OK(launch_pdl(k_gather_rows, ctx->smCount * 8, 256, 0, stream,
+                              x, xStride, nullptr, nullptr, tokens,
+                                                            (int)c.d, ctx->xSorted),
+                   error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
     const uint32_t rowTiles = (tokens + kRowTile - 1) / kRowTile;

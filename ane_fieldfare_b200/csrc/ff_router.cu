@@ -88,6 +88,7 @@ k_router_approx(const __grid_constant__ CUtensorMap mapW, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmemBase = tmemBaseSlot;
+    pdl_enter();
     if (warp == 0) {
         if (lane == 0) {
             uint32_t st = 0, phase = 0;
@@ -288,6 +289,7 @@ __device__ __forceinline__ void exact_pair_int8(const SelectArgs &a, const float
 template <bool INT8>
 __global__ void __launch_bounds__(kSelectWarps * 32, INT8 ? 4 : 3)
 k_router_select(const SelectArgs a) {
+    pdl_enter();
     extern __shared__ __align__(16) uint8_t selectSmem[];
     constexpr int kMaxRows = INT8 ? kSelectWarps / 2 : kSelectWarps;
     __shared__ uint16_t sExpert[kMaxRows][kMaxExperts + 8];
@@ -462,6 +464,7 @@ template <int NT>
 __global__ void __launch_bounds__(128)
 k_router_logits_int8(const uint4 *Q, const uint32_t *aux, const uint16_t *effScale, const float *bias, const uint16_t *x,
                      uint32_t xStride, int T, int E, int D, float *logits) {
+    pdl_enter();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e = blockIdx.x * 4 + warp, t0 = blockIdx.y * NT;
     if (e >= E) return;
@@ -632,8 +635,10 @@ bool launch_router_select(FFContext *ctx, const LayerStore &L, const uint16_t *x
         return false;
     {
         LaunchScope scope(ctx, stream, "router_approx");
-        k_router_approx<<<dim3(tiles, expertTiles, splits), kApproxThreads, smem, stream>>>(mapW, mapX, tileTokens, tokens, E, steps,
-                                                                                         splits, ctx->routerParts, ctx->errorFlag);
+        FF_CUDA_OK(launch_pdl(k_router_approx, dim3(tiles, expertTiles, splits), kApproxThreads, smem, stream,
+                              mapW, mapX, tileTokens, tokens, E, steps,
+                                                                                         splits, ctx->routerParts, ctx->errorFlag),
+                   error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
     SelectArgs a{};
@@ -663,7 +668,9 @@ bool launch_router_select(FFContext *ctx, const LayerStore &L, const uint16_t *x
         return false;
     {
         LaunchScope scope(ctx, stream, "router_select");
-        kernel<<<(tokens + perCta - 1) / perCta, kSelectWarps * 32, perCta * rowBytes, stream>>>(a);
+        FF_CUDA_OK(launch_pdl(kernel, (tokens + perCta - 1) / perCta, kSelectWarps * 32, perCta * rowBytes, stream,
+                              a),
+                   error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
     return true;
@@ -677,11 +684,14 @@ bool launch_router_logits_int8(FFContext *ctx, const LayerStore &L, const uint16
     {
         LaunchScope scope(ctx, stream, "router_logits_int8");
         if (tokens == 1)
-            k_router_logits_int8<1><<<dim3((E + 3) / 4, 1), 128, 0, stream>>>(lanes, L.routerAux, L.routerScale, L.logitBias, x, xStride,
-                                                                           1, E, D, logits);
+            FF_CUDA_OK(launch_pdl(k_router_logits_int8<1>, dim3((E + 3) / 4, 1), 128, 0, stream,
+                              lanes, L.routerAux, L.routerScale, L.logitBias, x, xStride,
+                                                                           1, E, D, logits),
+                   error);
         else
-            k_router_logits_int8<2><<<dim3((E + 3) / 4, (tokens + 1) / 2), 128, 0, stream>>>(
-                lanes, L.routerAux, L.routerScale, L.logitBias, x, xStride, (int)tokens, E, D, logits);
+            FF_CUDA_OK(launch_pdl(k_router_logits_int8<2>, dim3((E + 3) / 4, (tokens + 1) / 2), 128, 0, stream,
+                              lanes, L.routerAux, L.routerScale, L.logitBias, x, xStride, (int)tokens, E, D, logits),
+                   error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
     return true;
