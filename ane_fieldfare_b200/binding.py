@@ -7,7 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import os
-from ctypes import (POINTER, c_bool, c_char_p, c_float, c_int32, c_uint16, c_uint32, c_uint64,
+from ctypes import (POINTER, byref, c_bool, c_char_p, c_float, c_int32, c_uint16, c_uint32, c_uint64,
                     c_void_p)
 
 from .gturbo import MoEExpertOffsets
@@ -143,12 +143,16 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+_entry = {}
+
+
 def call(name: str, *args):
     """Calls a bool-returning entry point; raises FieldfareError with the library's message."""
-    lib = load()
+    fn = _entry.get(name)
+    if fn is None:
+        fn = _entry.setdefault(name, getattr(load(), name))
     err = c_char_p()
-    ok = getattr(lib, name)(*args, ctypes.byref(err))
-    if not ok:
+    if not fn(*args, byref(err)):
         message = err.value.decode("utf-8", "replace") if err.value else "unknown error"
         raise FieldfareError(message)
     return True

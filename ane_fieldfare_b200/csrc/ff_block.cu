@@ -66,6 +66,7 @@ struct alignas(64) BlockMaps {
         CUtensorMap w[3];  // gate, up | down, -; scale words
     } kind[2];
 };
+static_assert(sizeof(BlockMaps) == sizeof(LayerStore::blockMap[0]), "copied as one");
 
 __device__ __forceinline__ void box3(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
     asm volatile(
@@ -567,8 +568,8 @@ uint32_t row_pitch(uint32_t part, bool int8) {
     return p;
 }
 
-// Fills a kind and its maps.  mode kGateUp: w0, w1 [rows][cols], tiles of 8 + 8 rows; kDown: w0, 16 rows.
-bool setup_kind(int mode, bool int8, BlockKind &k, CUtensorMap (&w)[3], const uint8_t *w0, const uint8_t *w1,
+// Fills a kind and, unless they are there already, its maps.  mode kGateUp: w0, w1 [rows][cols], tiles of 8 + 8 rows; kDown: w0, 16 rows.
+bool setup_kind(int mode, bool int8, uint32_t &ready, uint32_t bit, BlockKind &k, CUtensorMap (&w)[3], const uint8_t *w0, const uint8_t *w1,
                 uint32_t rows, uint32_t cols, uint32_t experts, uint64_t stride, const uint32_t *scales, uint64_t scaleStride,
                 const char **error) {
     const uint32_t groups = cols / 64, padded = padded_groups(groups);
@@ -578,6 +579,8 @@ bool setup_kind(int mode, bool int8, BlockKind &k, CUtensorMap (&w)[3], const ui
     k.part = padded <= kPartGroups + 4 ? padded : kPartGroups;
     k.pitch = row_pitch(k.part, int8);
     k.sbWords = (k.part + 7u) & ~7u;  // (words past the row read as zero)
+    if (ready & bit) return true;
+    ready |= bit;
     const uint8_t *ws[2] = {w0, w1};
     for (int m = 0; m < (mode == kGateUp ? 2 : 1); ++m)
         if (!encode3(&w[m], CU_TENSOR_MAP_DATA_TYPE_UINT64, ws[m], rowBytes / 8, rows, experts, rowBytes, stride, k.pitch / 8,
@@ -633,10 +636,9 @@ bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
     if (c.d % 64 || c.f % 64 || c.sharedF % 64) return fail(error, "widths must be multiples of 64");
     if (((uintptr_t)x & 15) || (xStride % 8)) return fail(error, "input rows must be 16-byte aligned");
     const uint64_t words = scale_words(c.d, c.f);
+    LayerStore &Lm = const_cast<LayerStore &>(L);  // (its maps are encoded once per load)
     for (int mode = 0; mode < 2; ++mode) {
         BlockArgs a{};
-        BlockMaps maps;
-        memset(&maps, 0, sizeof(maps));
         a.ids = ids;
         a.T = (int)tokens;
         a.K = (int)c.topK;
@@ -648,7 +650,7 @@ bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
         if (ids) {
             const uint32_t *o = &L.off.gateWOff;
             BlockKind &k = a.kind[1];
-            if (!setup_kind(mode, false, k, maps.kind[1].w, L.experts + (down ? o[6] : o[0]), L.experts + o[3], down ? c.d : c.f,
+            if (!setup_kind(mode, false, Lm.blockMapsReady, 1u << (2 * mode + 1), k, Lm.blockMap[mode][1], L.experts + (down ? o[6] : o[0]), L.experts + o[3], down ? c.d : c.f,
                             down ? c.f : c.d, L.expertCount, L.stride,
                             L.routedScales + (down ? (uint64_t)(c.f / 8) * 16 * padded_groups(c.d / 64) : 0), words, error))
                 return false;
@@ -660,7 +662,7 @@ bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
         if (withShared) {
             const uint32_t *o = &L.sharedOff.gateWOff;
             BlockKind &k = a.kind[0];
-            if (!setup_kind(mode, false, k, maps.kind[0].w, L.shared + (down ? o[6] : o[0]), L.shared + o[3], down ? c.d : c.sharedF,
+            if (!setup_kind(mode, false, Lm.blockMapsReady, 1u << (2 * mode + 0), k, Lm.blockMap[mode][0], L.shared + (down ? o[6] : o[0]), L.shared + o[3], down ? c.d : c.sharedF,
                             down ? c.sharedF : c.d, 1, (uint64_t)c.d * c.sharedF / 2,
                             L.sharedScales + (down ? (uint64_t)(c.sharedF / 8) * 16 * padded_groups(c.d / 64) : 0), 0, error))
                 return false;
@@ -669,6 +671,8 @@ bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
             k.out = down ? sharedOut : ctx->sharedActs;
             k.outStride = down ? c.d : c.sharedF;
         }
+        BlockMaps maps;
+        memcpy(&maps, Lm.blockMap[mode], sizeof(maps));
         const bool ok = down ? launch_kernel<kDown, false>(ctx, a, maps, "int4_block_down", stream, error)
                              : launch_kernel<kGateUp, false>(ctx, a, maps, "int4_block_gate_up_act", stream, error);
         if (!ok) return false;
@@ -680,17 +684,16 @@ bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
 bool launch_block_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens, uint16_t *y,
                        cudaStream_t stream, const char **error) {
     const FFConfig &c = ctx->cfg;
+    LayerStore &Lm = const_cast<LayerStore &>(L);  // (its maps are encoded once per load)
     for (int mode = 0; mode < 2; ++mode) {
         BlockArgs a{};
-        BlockMaps maps;
-        memset(&maps, 0, sizeof(maps));
         a.T = (int)tokens;
         a.K = 1;
         a.withShared = 1;
         a.errorFlag = ctx->errorFlag;
         const bool down = mode == kDown;
         BlockKind &k = a.kind[0];
-        if (!setup_kind(mode, true, k, maps.kind[0].w, L.shared8W[down ? 2 : 0], L.shared8W[1], down ? c.d : c.sharedF,
+        if (!setup_kind(mode, true, Lm.blockMapsReady, 1u << (2 * mode + 0), k, Lm.blockMap[mode][0], L.shared8W[down ? 2 : 0], L.shared8W[1], down ? c.d : c.sharedF,
                         down ? c.sharedF : c.d, 1, (uint64_t)c.d * c.sharedF,
                         L.sharedScales + (down ? (uint64_t)(c.sharedF / 8) * 16 * padded_groups(c.d / 64) : 0), 0, error))
             return false;
@@ -698,6 +701,8 @@ bool launch_block_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
         k.inStride = down ? c.sharedF : xStride;
         k.out = down ? y : ctx->sharedActs;
         k.outStride = down ? c.d : c.sharedF;
+        BlockMaps maps;
+        memcpy(&maps, Lm.blockMap[mode], sizeof(maps));
         const bool ok = down ? launch_kernel<kDown, true>(ctx, a, maps, "shared_int8_down", stream, error)
                              : launch_kernel<kGateUp, true>(ctx, a, maps, "shared_int8_gate_up_act", stream, error);
         if (!ok) return false;

@@ -83,7 +83,7 @@ void ff_destroy(FFContext *ctx) {
     cudaSetDevice(ctx->device);
     cudaDeviceSynchronize();
     for (auto &L : ctx->layers) free_layer(L);
-    void *ptrs[] = {ctx->logits, ctx->ids, ctx->weights, ctx->plan, ctx->acts, ctx->sharedActs, ctx->h1,
+    void *ptrs[] = {ctx->logits, ctx->ids, ctx->weights, ctx->plan, ctx->routerCounts, ctx->acts, ctx->sharedActs, ctx->h1,
                     ctx->partials, ctx->xDev, ctx->yDev, ctx->xSorted, ctx->sortedPairs,
                     ctx->expertOffsets, ctx->blockCounts, ctx->units, ctx->unitCount,
                     ctx->errorFlag, ctx->gridBarrier, ctx->phaseStamps, ctx->mapScratch, ctx->taggedLogits, ctx->taggedActs,
@@ -145,6 +145,9 @@ FFContext *ff_create(int32_t deviceOrdinal, const FFConfig *config, const char *
     ok = ok && dev_alloc(ctx, &ctx->ids, T * K, error);
     ok = ok && dev_alloc(ctx, &ctx->weights, T * K, error);
     ok = ok && dev_alloc(ctx, &ctx->plan, 1, error);
+    if (ok) ok = cudaMemset(ctx->plan, 0, sizeof(RoutePlan)) == cudaSuccess;
+    ok = ok && dev_alloc(ctx, &ctx->routerCounts, kMaxGemvRows, error);
+    if (ok) ok = cudaMemset(ctx->routerCounts, 0, kMaxGemvRows * 4) == cudaSuccess;
     ok = ok && dev_alloc(ctx, &ctx->acts, (T * K + 256) * c.f, error);  // +256: a GEMM row tile may overhang
     ok = ok && dev_alloc(ctx, &ctx->sharedActs, (T + 256) * c.sharedF, error);
     ok = ok && dev_alloc(ctx, &ctx->h1, T * c.d, error);
@@ -324,6 +327,7 @@ bool ff_load_layer(FFContext *ctx, uint32_t layer, const void *hostBytes, uint64
     L.off = *offsets;
     L.mapsReady = false;
     L.decodeMapsReady = false;
+    L.blockMapsReady = 0;
     ctx->weightBytes += total;
     const uint8_t *e = L.experts;
     return pack_scales(ctx, ScaleSource{{e + o[1], e + o[4], e + o[7]}, {e + o[2], e + o[5], e + o[8]}, L.stride}, d, f, expertCount,
@@ -371,6 +375,7 @@ bool ff_load_shared(FFContext *ctx, uint32_t layer, const FFProjection *gate,
     }
     L.mapsReady = false;
     L.decodeMapsReady = false;
+    L.blockMapsReady = 0;
     ctx->weightBytes += payload;
     const uint8_t *b = L.shared;
     return pack_scales(ctx, ScaleSource{{b + o[1], b + o[4], b + o[7]}, {b + o[2], b + o[5], b + o[8]}, 0}, d, fs, 1, &L.sharedScales,
@@ -429,6 +434,7 @@ bool ff_load_shared_int8(FFContext *ctx, uint32_t layer, const FFProjection *gat
         L.shared = nullptr;
         L.mapsReady = false;
         L.decodeMapsReady = false;
+    L.blockMapsReady = 0;
     }
     free_shared8(L);
     for (int m = 0; m < 3; ++m) {
@@ -439,6 +445,7 @@ bool ff_load_shared_int8(FFContext *ctx, uint32_t layer, const FFProjection *gat
             return false;
         ctx->weightBytes += codes + 2 * aux;
     }
+    L.blockMapsReady = 0;
     ScaleSource src{};
     for (int m = 0; m < 3; ++m) {
         src.scales[m] = reinterpret_cast<const uint8_t *>(L.shared8S[m]);

@@ -209,12 +209,6 @@ __device__ __forceinline__ void fetch_tagged(const unsigned long long *src, uint
     if (!(okI && okJ)) atomicExch(errorFlag, 9u);
 }
 
-// A float as an unsigned number of the same order.
-__device__ __forceinline__ uint32_t ordered_key(float f) {
-    const uint32_t u = __float_as_uint(f);
-    return (u >> 31) ? ~u : (u | 0x80000000u);
-}
-
 // The K largest logits, by warps 0..9: one of them polls the CTA's copy of the tagged words and puts
 // their keys into shared memory (0: never taken — -inf or NaN, or past the experts); then two threads
 // per expert count the larger keys, half of them each.  Equal keys leave a place empty; then the count

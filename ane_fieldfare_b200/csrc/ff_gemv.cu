@@ -127,12 +127,11 @@ k_int4_gemv(const GemvJob *jobs, const uint32_t *items, const uint32_t *itemCoun
 // butterfly (16, 8, 4, 2, 1), then the per-expert logit bias is added.
 __global__ void __launch_bounds__(256)
 k_router_logits(const uint16_t *W, const uint16_t *scale, const float *bias, const uint16_t *x,
-                uint32_t xStride, int E, int D, float *logits) {
+                uint32_t xStride, int E, int D, float *logits, RouterTail tail) {
     pdl_enter();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int e = blockIdx.x * 8 + warp;
+    const int e = min((int)blockIdx.x * 8 + warp, E - 1);  // (a warp past the experts repeats the last)
     const int t = blockIdx.y;
-    if (e >= E) return;
     const uint16_t *wr = W + (size_t)e * D;
     const uint16_t *xr = x + (size_t)t * xStride;
     float acc = 0.0f;
@@ -158,14 +157,9 @@ k_router_logits(const uint16_t *W, const uint16_t *scale, const float *bias, con
 #pragma unroll
     for (int offset = 16; offset >= 1; offset >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, offset);
     if (lane == 0) logits[(size_t)t * E + e] = bias ? acc + bias[e] : acc;
-}
-
-// Top-K of 1..16 rows' logits, one warp per row.
-__global__ void __launch_bounds__(512) k_topk_small(const float *logits, const uint16_t *gain, int T, int E, int K, uint32_t *ids,
-                                                    uint16_t *weights) {
-    pdl_enter();
-    const int t = threadIdx.x >> 5;
-    if (t < T) warp_topk(logits + (size_t)t * E, E, K, gain, ids + t * K, weights + t * K);
+    if (tail.ids)
+        topk_by_last_cta(logits + (size_t)t * E, E, tail.K, tail.gain, tail.ids + t * tail.K, tail.weights + t * tail.K, tail.counts + t,
+                         gridDim.x);
 }
 
 // Metal/Prefill/prefill.metal:544-565 plus an optional residual row added after the ranks.
@@ -744,7 +738,7 @@ bool launch_router_topk(FFContext *ctx, const LayerStore &L, const uint16_t *x, 
         return launch_router_select(ctx, L, x, xStride, tokens, ids, weights, stream, error);
     if (L.routerQ && tokens > kMaxGemvRows) {
         float *lg = logits ? logits : ctx->logitsRows;
-        if (!launch_router_logits_int8(ctx, L, x, xStride, tokens, lg, stream, error)) return false;
+        if (!launch_router_logits_int8(ctx, L, x, xStride, tokens, lg, RouterTail{}, stream, error)) return false;
         {
             LaunchScope scope(ctx, stream, "topk_rows");
             k_topk_rows<<<(tokens + 7) / 8, 256, 0, stream>>>(lg, L.gain, (int)tokens, E, (int)ctx->cfg.topK, ids,
@@ -756,23 +750,14 @@ bool launch_router_topk(FFContext *ctx, const LayerStore &L, const uint16_t *x, 
     if (tokens > kMaxGemvRows)
         return launch_router_prefill(ctx, L, x, xStride, tokens, ids, weights, logits, stream, error);
     float *lg = logits ? logits : ctx->logits;
-    if (L.routerQ) {
-        if (!launch_router_logits_int8(ctx, L, x, xStride, tokens, lg, stream, error)) return false;
-    } else {
-        dim3 grid((E + 7) / 8, tokens);
-        LaunchScope scope(ctx, stream, "router_logits");
-        FF_CUDA_OK(launch_pdl(k_router_logits, grid, 256, 0, stream,
-                              L.routerW, L.routerScale, L.logitBias, x, xStride,
-                                                  E, D, lg),
-                   error);
-    }
+    const RouterTail tail{ids, weights, L.gain, ctx->routerCounts, (int)ctx->cfg.topK};
+    if (L.routerQ) return launch_router_logits_int8(ctx, L, x, xStride, tokens, lg, tail, stream, error);
     {
-        LaunchScope scope(ctx, stream, "topk");
-        FF_CUDA_OK(launch_pdl(k_topk_small, 1, 512, 0, stream,
-                              lg, L.gain, (int)tokens, E, (int)ctx->cfg.topK, ids, weights),
+        LaunchScope scope(ctx, stream, "router_logits");
+        FF_CUDA_OK(launch_pdl(k_router_logits, dim3((E + 7) / 8, tokens), 256, 0, stream, L.routerW, L.routerScale, L.logitBias, x, xStride,
+                              E, D, lg, tail),
                    error);
     }
-    FF_CUDA_OK(cudaGetLastError(), error);
     return true;
 }
 

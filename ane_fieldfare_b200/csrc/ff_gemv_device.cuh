@@ -282,68 +282,74 @@ __device__ __forceinline__ void row_dot(const uint8_t *w0, const uint16_t *s0, c
     }
 }
 
-// Warp-wide top-K over E <= 256 logits held four-plus per lane: K rounds of argmax (higher score,
-// then lower expert id), softmax over the selected scores, times the per-expert gain.  Selection
-// rule and softmax: Metal/MoE/moe.metal:186-237,269-319.
-// sharedIds: optional copy of the ids in shared memory.
-__device__ inline void warp_topk(const float *logits, int E, int K, const uint16_t *gain, uint32_t *ids,
-                          uint16_t *weights, uint32_t *sharedIds = nullptr) {
+// A float as an unsigned number of the same order (the two zeros are one).
+__device__ __forceinline__ uint32_t ordered_key(float f) {
+    const uint32_t u = __float_as_uint(f + 0.0f);
+    return (u >> 31) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float from_ordered_key(uint32_t k) { return __uint_as_float((k >> 31) ? (k & 0x7FFFFFFFu) : ~k); }
+
+// Warp-wide top-K over E <= 256 logits held eight per lane: K rounds of argmax (higher score, then lower
+// expert id; -inf and NaN are never taken), softmax over the selected scores, times the per-expert gain.
+// Selection rule and softmax: Metal/MoE/moe.metal:186-237,269-319.  A round is two warp-wide reductions
+// over register keys.  `logits` may be in shared or global memory (volatile: other SMs may have written it).
+__device__ inline void warp_topk(const float *logits, int E, int K, const uint16_t *gain, uint32_t *ids, uint16_t *weights) {
     const int lane = threadIdx.x & 31;
-    float v[8];
-    uint32_t live = 0;  // bit j: candidate j of this lane is still in the race (a register, not an indexed array)
+    uint32_t key[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const int e = j * 32 + lane;
-        v[j] = e < E ? logits[e] : -INFINITY;
-        if (e < E && v[j] > -INFINITY) live |= 1u << j;
+        const float v = e < E ? *static_cast<const volatile float *>(logits + e) : -INFINITY;
+        key[j] = v > -INFINITY ? ordered_key(v) : 0u;
     }
-    float topScore[8];
-    uint32_t topIdx[8];
-    for (int r = 0; r < 8; ++r) {
-        float best = -INFINITY;
-        uint32_t bestE = 0xFFFFFFFFu;
-        if (r < K) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint32_t e = (uint32_t)(j * 32 + lane);
-                if (((live >> j) & 1u) && (v[j] > best || (v[j] == best && e < bestE))) {
-                    best = v[j];
-                    bestE = e;
-                }
-            }
-        }
-#pragma unroll
-        for (int offset = 16; offset >= 1; offset >>= 1) {
-            const float ob = __shfl_xor_sync(0xFFFFFFFFu, best, offset);
-            const uint32_t oe = __shfl_xor_sync(0xFFFFFFFFu, bestE, offset);
-            if (oe != 0xFFFFFFFFu && (bestE == 0xFFFFFFFFu || ob > best || (ob == best && oe < bestE))) {
-                best = ob;
-                bestE = oe;
-            }
-        }
-        if (bestE != 0xFFFFFFFFu && (bestE & 31u) == (uint32_t)lane) live &= ~(1u << (bestE >> 5));
-        topIdx[r] = bestE == 0xFFFFFFFFu ? 0u : bestE;
-        topScore[r] = bestE == 0xFFFFFFFFu ? -INFINITY : best;
-    }
-    // softmax over the chosen scores: lane r holds route r; exponentials in parallel, the sum in
-    // rank order (the same additions as a serial loop)
+    uint32_t myId = 0u;
     float myScore = -INFINITY;
-    uint32_t myIdx = 0;
+    for (int r = 0; r < K; ++r) {
+        uint32_t best = key[0], at = (uint32_t)lane;
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
+        for (int j = 1; j < 8; ++j)
+            if (key[j] > best) {
+                best = key[j];
+                at = (uint32_t)(32 * j + lane);
+            }
+        const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, best);
+        if (top == 0u) break;
+        const uint32_t id = __reduce_min_sync(0xFFFFFFFFu, best == top ? at : 0xFFFFFFFFu);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (id == (uint32_t)(32 * j + lane)) key[j] = 0u;
         if (lane == r) {
-            myScore = topScore[r];
-            myIdx = topIdx[r];
+            myId = id;
+            myScore = from_ordered_key(top);
         }
-    const float ex = lane < K ? expf(myScore - topScore[0]) : 0.0f;
+    }
+    // softmax over the chosen scores: exponentials in parallel, the sum in rank order
+    const float best = __shfl_sync(0xFFFFFFFFu, myScore, 0);
+    const float ex = lane < K ? expf(myScore - best) : 0.0f;
     float sum = 0.0f;
     for (int r = 0; r < K; ++r) sum += __shfl_sync(0xFFFFFFFFu, ex, r);
     if (lane < K) {
         float w = ex / sum;
-        if (gain) w = w * bf2f(gain[myIdx]);
-        ids[lane] = myIdx;
+        if (gain) w = w * bf2f(gain[myId]);
+        ids[lane] = myId;
         weights[lane] = f2bf(w);
-        if (sharedIds) sharedIds[lane] = myIdx;
+    }
+}
+
+// The top-K of a row by the last of the `blocks` CTAs that form its logits (a launch of its own cost 5 us
+// behind them).  `count` returns to 0 by itself.  All threads of the CTA call this.
+__device__ __forceinline__ void topk_by_last_cta(const float *logits, int E, int K, const uint16_t *gain, uint32_t *ids,
+                                                 uint16_t *weights, uint32_t *count, uint32_t blocks) {
+    __shared__ uint32_t sLastCta;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        sLastCta = atomicInc(count, blocks - 1u) == blocks - 1u ? 1u : 0u;
+    }
+    __syncthreads();
+    if (sLastCta && threadIdx.x < 32) {
+        __threadfence();
+        warp_topk(logits, E, K, gain, ids, weights);
     }
 }
 

@@ -138,6 +138,9 @@ struct LayerStore {
     // routed down
     bool decodeMapsReady = false;
     CUtensorMap decodeMap[kDecodeMaps];
+    // verify block: [gate/up, down][shared, routed] maps of the weights and scale words
+    uint32_t blockMapsReady = 0;  // bit 2 * mode + kind
+    CUtensorMap blockMap[2][2][3];
 };
 
 }  // namespace ff
@@ -159,6 +162,7 @@ struct FFContext {
     uint32_t *ids = nullptr;        // [maxTokens][topK]
     uint16_t *weights = nullptr;    // [maxTokens][topK]
     ff::RoutePlan *plan = nullptr;
+    uint32_t *routerCounts = nullptr;  // [kMaxGemvRows] CTAs that have formed a row's logits
     uint16_t *acts = nullptr;       // [maxTokens*topK][f]
     uint16_t *sharedActs = nullptr; // [maxTokens][sharedF]
     uint16_t *h1 = nullptr;         // [maxTokens][d]
@@ -333,8 +337,17 @@ bool router_prepare(FFContext *ctx, LayerStore &L, const char **error);
 bool launch_router_select(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens,
                           uint32_t *ids, uint16_t *weights, cudaStream_t stream, const char **error);
 
+// Where a logits kernel's last CTA per row puts the row's top-K (ids null: logits only; at most
+// kMaxGemvRows rows).
+struct RouterTail {
+    uint32_t *ids;
+    uint16_t *weights;
+    const uint16_t *gain;
+    uint32_t *counts;  // [kMaxGemvRows], zero between launches
+    int K;
+};
 bool launch_router_logits_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens,
-                               float *logits, cudaStream_t stream, const char **error);
+                               float *logits, const RouterTail &tail, cudaStream_t stream, const char **error);
 
 // ff_int8_gemm.cu
 bool int8_gemm_fits(uint32_t d, uint32_t f);  // contraction lengths within the kernel's shared memory

@@ -155,15 +155,6 @@ k_router_approx(const __grid_constant__ CUtensorMap mapW, const __grid_constant_
 // Warps of a CTA; `warpsPerRow` (1, 2, 4 or 8) of them share a row.
 constexpr int kSelectWarps = 8;
 
-// a float as an unsigned number of the same order
-__device__ __forceinline__ uint32_t ordered(float f) {
-    const uint32_t u = __float_as_uint(f);
-    return (u >> 31) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float from_ordered(uint32_t k) {
-    return __uint_as_float((k >> 31) ? (k & 0x7FFFFFFFu) : ~k);
-}
-
 // Butterfly 16, 8, 4, 2, 1 over N values per lane at once: every level halves the values a lane carries
 // (a lane keeps the ones of its side), the additions are those of N separate butterflies.  Returns the
 // sum of value index `which` (the same for all lanes that differ only in the low bits).
@@ -368,7 +359,7 @@ k_router_select(const SelectArgs a) {
                 const float eps = fmaf(a.coef[e], norm, fabsf(l) * 2.5e-7f);
                 const float lo = l - eps, hi = l + eps;
                 const bool bounded = lo > -INFINITY && hi < INFINITY;  // false for NaN, too
-                low[j] = bounded ? ordered(lo) : 0u;
+                low[j] = bounded ? ordered_key(lo) : 0u;
                 high[j] = bounded || l == -INFINITY ? hi : INFINITY;
             }
         }
@@ -387,7 +378,7 @@ k_router_select(const SelectArgs a) {
             const uint32_t holders = __ballot_sync(0xFFFFFFFFu, best == threshold);
             if (lane == __ffs(holders) - 1) gone |= 1u << at;
         }
-        const float cut = threshold ? from_ordered(threshold) : -INFINITY;
+        const float cut = threshold ? from_ordered_key(threshold) : -INFINITY;
         int kept = 0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -463,11 +454,10 @@ k_router_select(const SelectArgs a) {
 template <int NT>
 __global__ void __launch_bounds__(128)
 k_router_logits_int8(const uint4 *Q, const uint32_t *aux, const uint16_t *effScale, const float *bias, const uint16_t *x,
-                     uint32_t xStride, int T, int E, int D, float *logits) {
+                     uint32_t xStride, int T, int E, int D, float *logits, RouterTail tail) {
     pdl_enter();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int e = blockIdx.x * 4 + warp, t0 = blockIdx.y * NT;
-    if (e >= E) return;
+    const int e = min((int)blockIdx.x * 4 + warp, E - 1), t0 = blockIdx.y * NT;  // (a warp past the experts repeats the last)
     const int groups = D >> 6, runs = (groups + 7) >> 3;
     const uint4 *q = Q + (size_t)e * runs * 32 + lane;
     const uint4 *sb = reinterpret_cast<const uint4 *>(aux + (size_t)e * runs * 8);
@@ -513,6 +503,10 @@ k_router_logits_int8(const uint4 *Q, const uint32_t *aux, const uint16_t *effSca
         for (int offset = 16; offset >= 1; offset >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, offset);
         if (lane == 0 && t0 + k < T) logits[(size_t)(t0 + k) * E + e] = bias ? v + bias[e] : v;
     }
+    if (tail.ids)
+        for (int k = 0; k < NT && t0 + k < T; ++k)
+            topk_by_last_cta(logits + (size_t)(t0 + k) * E, E, tail.K, tail.gain, tail.ids + (t0 + k) * tail.K,
+                             tail.weights + (t0 + k) * tail.K, tail.counts + t0 + k, gridDim.x);
 }
 
 // ---- at load: folded bf16 weights and the bound's coefficients --------------------------------------
@@ -677,7 +671,7 @@ bool launch_router_select(FFContext *ctx, const LayerStore &L, const uint16_t *x
 }
 
 bool launch_router_logits_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens,
-                               float *logits, cudaStream_t stream, const char **error) {
+                               float *logits, const RouterTail &tail, cudaStream_t stream, const char **error) {
     const int E = (int)L.routerExperts, D = (int)ctx->cfg.d;
     if (xStride % 2 || ((uintptr_t)x & 3)) return fail(error, "input rows must be 4-byte aligned");
     const uint4 *lanes = reinterpret_cast<const uint4 *>(L.routerLanes);
@@ -686,11 +680,11 @@ bool launch_router_logits_int8(FFContext *ctx, const LayerStore &L, const uint16
         if (tokens == 1)
             FF_CUDA_OK(launch_pdl(k_router_logits_int8<1>, dim3((E + 3) / 4, 1), 128, 0, stream,
                               lanes, L.routerAux, L.routerScale, L.logitBias, x, xStride,
-                                                                           1, E, D, logits),
+                                                                           1, E, D, logits, tail),
                    error);
         else
             FF_CUDA_OK(launch_pdl(k_router_logits_int8<2>, dim3((E + 3) / 4, (tokens + 1) / 2), 128, 0, stream,
-                              lanes, L.routerAux, L.routerScale, L.logitBias, x, xStride, (int)tokens, E, D, logits),
+                              lanes, L.routerAux, L.routerScale, L.logitBias, x, xStride, (int)tokens, E, D, logits, tail),
                    error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);

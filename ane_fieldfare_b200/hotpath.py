@@ -45,8 +45,11 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _stream(stream: Optional[torch.cuda.Stream]) -> Optional[int]:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream or None
+    if stream is not None:
+        return stream.cuda_stream or None
+    # torch.cuda.current_stream() without the stream object it makes (several microseconds a call,
+    # more than a decode operator's own launch)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()) or None
 
 
 def validateGTurboLayout(path: str, d: int, f: int) -> binding.FFGTurboLayoutInfo:
