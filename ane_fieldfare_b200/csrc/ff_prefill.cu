@@ -759,16 +759,7 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
         uint32_t ps = grp % kPackStages, pPhase = 0, ownSteps = 0;
         while (u < units) {
             const uint32_t sb = myScales[((g - gFirst) >> 2) * (uint32_t)(kDequantWarps * 32)];
-            // The weight stage `grp` was last read by the MMAs of this group's previous step, four
-            // steps back: its completion is that step's signal on the token ring (stage ps - 4,
-            // which in a ring of eight is ps + 4; the group's n-th step, n >= 1, meets that
-            // barrier's completion number (n - 1) / 2).
-            static_assert(kTokStages == 2 * kWStages, "the weight stages are released through the token ring");
-            if (!mbar_wait(barPackFull(ps), pPhase, &abortFlag) ||
-                (ownSteps && !mbar_wait(barTokEmpty((ps + kWStages) % kTokStages), ((ownSteps - 1u) >> 1) & 1u, &abortFlag)))
-                break;
-            tc_fence_after();
-
+            if (!mbar_wait(barPackFull(ps), pPhase, &abortFlag)) break;
             uint32_t s2, b2;
             asm("prmt.b32 %0, %1, %1, 0x1010;" : "=r"(s2) : "r"(sb));
             asm("prmt.b32 %0, %1, %1, 0x3232;" : "=r"(b2) : "r"(sb));
@@ -793,6 +784,17 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
                     o[j * 4 + i] = v2;
                 }
             }
+            // the codes are in registers: their tile may be copied over
+            __syncwarp();
+            if (lane == 0) mbar_arrive(barPackEmpty(ps));
+            // The weight stage `grp` was last read by the MMAs of this group's previous step, four
+            // steps back: its completion is that step's signal on the token ring (stage ps - 4,
+            // which in a ring of eight is ps + 4; the group's n-th step, n >= 1, meets that
+            // barrier's completion number (n - 1) / 2).  Waited for only here: the conversion above
+            // runs under those MMAs.
+            static_assert(kTokStages == 2 * kWStages, "the weight stages are released through the token ring");
+            if (ownSteps && !mbar_wait(barTokEmpty((ps + kWStages) % kTokStages), ((ownSteps - 1u) >> 1) & 1u, &abortFlag)) break;
+            tc_fence_after();
             tc_store_32cols(tmemW, o);
             // this CTA's half of the step's token tile must have landed before the MMA is told to go
             const bool landed = mbar_wait(barTokFull(ps), pPhase, &abortFlag);
@@ -800,10 +802,7 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
             if (!landed) break;
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive_cluster(leaderWFull);
-                mbar_arrive(barPackEmpty(ps));
-            }
+            if (lane == 0) mbar_arrive_cluster(leaderWFull);
             ps += kWStages;
             if (ps >= kPackStages) {
                 ps -= kPackStages;
