@@ -791,9 +791,8 @@ k_decode_fused_inline_x(const DecodeArgs a, const __grid_constant__ DecodeMaps m
 
 // Scale | bias words of `count` blobs, tile by tile: [F/8 gate/up tiles][8 gate rows, 8 up rows] of
 // padded_groups(D/64) words, then [D down rows] of padded_groups(F/64).
-uint64_t scale_words(uint32_t D, uint32_t F) {
-    return (uint64_t)(F / 8) * 16 * padded_groups(D / 64) + (uint64_t)D * padded_groups(F / 64);
-}
+uint64_t scale_words_gate_up(uint32_t D, uint32_t F) { return (uint64_t)(F / 8) * 16 * padded_groups(D / 64); }
+uint64_t scale_words(uint32_t D, uint32_t F) { return scale_words_gate_up(D, F) + (uint64_t)D * padded_groups(F / 64); }
 __global__ void __launch_bounds__(256)
 k_pack_scales(ScaleSource src, uint32_t D, uint32_t F, uint32_t *out, uint64_t words) {
     const uint32_t gD = D / 64, gF = F / 64, pD = padded_groups(gD), pF = padded_groups(gF);

@@ -278,7 +278,8 @@ bool launch_dequant_probe(FFContext *ctx, const uint8_t *w, const uint16_t *s, c
                           cudaStream_t stream, const char **error);
 
 // ff_decode.cu
-uint64_t scale_words(uint32_t D, uint32_t F);  // words of one blob
+uint64_t scale_words(uint32_t D, uint32_t F);          // words of one blob
+uint64_t scale_words_gate_up(uint32_t D, uint32_t F);  // of those, in front of the down rows
 // Scales and biases of gate, up and down (bytes, blobs `stride` apart).
 struct ScaleSource {
     const uint8_t *scales[3], *biases[3];

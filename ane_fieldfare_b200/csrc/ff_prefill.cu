@@ -477,37 +477,44 @@ k_gather_rows(const uint16_t *x, uint32_t xStride, const FFTokenExpertPair *pair
 constexpr int kWeightRows = 128;  // weight rows of a unit = TMEM lanes of its accumulator
 constexpr int kTileK = 64;        // one quantization group per step
 constexpr int kTokStages = 8;     // token half tiles (TMA destinations)
-constexpr int kPackStages = 8;    // packed-code tiles (TMA destinations)
-constexpr int kGroups = 4;        // dequantizing groups
+constexpr int kQuad = 4;          // steps whose packed codes come as one copy (128 bytes of a weight row)
+constexpr int kPackStages = 3;    // quads of packed codes in flight
+constexpr int kGroups = 4;        // dequantizing groups: one for each step of a quad
 constexpr int kWStages = kGroups; // dequantized weight tiles in TMEM, one per dequantizing group
 constexpr int kDequantWarps = 16; // four groups of four warps; a group covers the 128 TMEM lanes
-// warp 0 TMA, warp 1 MMA, warps 2-17 dequantize, warps 18-21 epilogue (TMEM lane quarter = warp & 3)
-constexpr int kGemmThreads = (2 + kDequantWarps + 4) * 32;
+constexpr int kEpilogueSets = 2;  // of four warps each, taking turns at 32-token chunks
+// warp 0 token copies, warp 1 MMA, warps 2-17 dequantize, warps 18-25 epilogue (TMEM lane quarter =
+// warp & 3), warp 26 code copies
+constexpr int kFirstEpilogueWarp = 2 + kDequantWarps;
+constexpr int kCodeWarp = kFirstEpilogueWarp + 4 * kEpilogueSets;
+constexpr int kGemmThreads = (kCodeWarp + 1) * 32;
+constexpr int kEpilogueThreads = 128 * kEpilogueSets;
 constexpr uint32_t kTokHalfRows = kRowTile / 2;                   // rows of a token tile held by either CTA of a pair
 constexpr uint32_t kTokTileBytes = kTokHalfRows * kTileK * 2;     // 12288 (a multiple of the 1024-byte swizzle atom)
-constexpr uint32_t kPackTileBytes = kWeightRows * kTileK / 2;     // 4096: two [64 rows x 32 bytes] boxes
+constexpr uint32_t kPackTileBytes = kWeightRows * kTileK / 2 * kQuad;  // 16384: two [64 rows x 128 bytes] boxes
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kAccCols = kRowTile;                           // accumulators at columns 0 and 192
 constexpr uint32_t kWCol0 = 2 * kAccCols;                         // weight stages: 32 columns each from 384
 constexpr int kXchgPitch = 17;                                    // floats per exchanged row (16 + 1 pad)
-constexpr uint32_t kXchgBytes = 2u * 128u * kXchgPitch * 4u;      // two buffers x 128 rows
+constexpr uint32_t kXchgBytes = 128u * kXchgPitch * 4u;           // one set's exchange buffer
 constexpr uint32_t kStagePitchGateUp = 64 * 2 + 16;               // bytes per token row of the output tile
 constexpr uint32_t kStagePitchDown = 128 * 2 + 16;
 constexpr uint32_t kStageBytesGateUp = 32u * kStagePitchGateUp;   // one 32-token output tile
 constexpr uint32_t kStageBytesDown = 32u * kStagePitchDown;
-// gate/up: exchange buffers + two output tiles; down: two output tiles + two row tables
-constexpr uint32_t kEpilogueBytesGateUp = kXchgBytes + 2u * kStageBytesGateUp;
-constexpr uint32_t kEpilogueBytesDown = 2u * kStageBytesDown + 2u * kRowTile * 4u;
+// gate/up: per set an exchange buffer and an output tile; down: per set two output tiles, two row tables
+constexpr uint32_t kEpilogueBytesGateUp = kEpilogueSets * (kXchgBytes + kStageBytesGateUp);
+constexpr uint32_t kEpilogueBytesDown = kEpilogueSets * 2u * kStageBytesDown + 2u * kRowTile * 4u;
+constexpr uint32_t kScaleSlotBytes = kDequantWarps * 32 * 4;      // a scale word of every dequantizing thread
 static_assert(kWCol0 + kWStages * 32 <= kTmemCols, "tensor memory layout");
-static_assert(kRowTile % 32 == 0 && kRowTile <= 256, "row tile");
+static_assert(kRowTile % 32 == 0 && kRowTile <= 256 && (int)kRowTile <= kEpilogueThreads, "row tile");
+static_assert(kQuad == kGroups, "a group takes one step of every quad");
 
 enum GemmMode : int { kModeGateUp = 0, kModeDown = 1 };
 
 struct GemmArgs {
-    const uint8_t *blobBase;   // expert 0's blob
-    uint64_t expertStride;
-    uint32_t scaleOff[2];      // byte offsets of the scales of matrix 0 / 1 inside a blob
-    uint32_t biasOff[2];
+    const uint32_t *scaleWords;  // scale | bias words of expert 0 (see pack_scales), of its down rows for the down GEMM
+    uint64_t scaleStride;        // words between experts
+    uint32_t scaleBuffers;       // units whose scale words are held in shared memory: 2, 1 or 0 (read per step)
     uint32_t K;                // contraction length (multiple of 64)
     uint32_t N;                // outputs per row: F (gate/up) or D (down)
     uint32_t nTiles;           // weight-row tiles: ceil(N/64) for gate/up, ceil(N/128) for down
@@ -524,34 +531,36 @@ struct GemmArgs {
 __device__ __forceinline__ uint32_t interleaved_position(uint32_t i) {
     return (i & ~7u) | (((i & 3u) << 1) | ((i >> 2) & 1u));
 }
+// two floats as bf16, the first in the low half
+__device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
 
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ CUtensorMap mapW0,
                     const __grid_constant__ CUtensorMap mapW1, const GemmArgs args) {
     extern __shared__ uint8_t gemmSmemRaw[];
-    __shared__ uint64_t barriers[2 * kTokStages + 2 * kPackStages + 2 * kWStages + 4 + 5];
+    __shared__ uint64_t barriers[2 * kTokStages + 2 * kPackStages + kWStages + 4 + 3 * kEpilogueSets + 1];
     __shared__ uint32_t tmemBaseSlot;
     __shared__ volatile uint32_t abortFlag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rawBase = smem_u32(gemmSmemRaw);
     const uint32_t base = (rawBase + 1023u) & ~1023u;
-    const uint32_t groupsK = args.K / kTileK;
+    const uint32_t groupsK = args.K / kTileK, quadsK = (groupsK + kQuad - 1) / kQuad;
 
-    // carve-up: token stages (1024-aligned), packed stages, the epilogue's exchange buffers
+    // carve-up: token stages (1024-aligned), packed stages, the epilogue's buffers, scale words
     // (stage addresses are computed, not tabulated: an array indexed by the running stage would
     // live in local memory)
     const uint32_t tokBase = base, packBase = tokBase + kTokStages * kTokTileBytes;
     auto tokAddrOf = [&](uint32_t s) { return tokBase + s * kTokTileBytes; };
     auto packAddrOf = [&](uint32_t s) { return packBase + s * kPackTileBytes; };
-    uint8_t *epilogueSmem = gemmSmemRaw + (packBase + kPackStages * kPackTileBytes - rawBase);
-    constexpr uint32_t kStageBytes = MODE == kModeGateUp ? kStageBytesGateUp : kStageBytesDown;
-    float *xchg = reinterpret_cast<float *>(epilogueSmem);                                 // gate/up only
-    uint8_t *stageBuf = epilogueSmem + (MODE == kModeGateUp ? kXchgBytes : 0u);
-    uint32_t *rowTable = reinterpret_cast<uint32_t *>(stageBuf + 2u * kStageBytes);        // down only
-    uint32_t *scaleSlots = reinterpret_cast<uint32_t *>(
-        epilogueSmem + (MODE == kModeGateUp ? kEpilogueBytesGateUp : kEpilogueBytesDown));  // [ceil(groupsK/4)][512]
+    const uint32_t epilogueOffset = packBase + kPackStages * kPackTileBytes - rawBase;
+    uint8_t *epilogueSmem = gemmSmemRaw + epilogueOffset;
+    const uint32_t scaleBase = rawBase + epilogueOffset + (MODE == kModeGateUp ? kEpilogueBytesGateUp : kEpilogueBytesDown);
 
     const uint32_t barBase = smem_u32(barriers);
     auto barAt = [&](int i) { return barBase + 8u * (uint32_t)i; };
@@ -559,13 +568,13 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
     auto barTokEmpty = [&](int s) { return barAt(kTokStages + s); };
     auto barPackFull = [&](int s) { return barAt(2 * kTokStages + s); };
     auto barPackEmpty = [&](int s) { return barAt(2 * kTokStages + kPackStages + s); };
-    auto barWFull = [&](int s) { return barAt(2 * kTokStages + 2 * kPackStages + s); };
-    auto barWEmpty = [&](int s) { return barAt(2 * kTokStages + 2 * kPackStages + kWStages + s); };
-    auto barAccFull = [&](int s) { return barAt(2 * kTokStages + 2 * kPackStages + 2 * kWStages + s); };
-    auto barAccEmpty = [&](int s) { return barAt(2 * kTokStages + 2 * kPackStages + 2 * kWStages + 2 + s); };
-    auto barXchg = [&](int s) { return barAt(2 * kTokStages + 2 * kPackStages + 2 * kWStages + 4 + s); };
-    auto barStage = [&](int s) { return barAt(2 * kTokStages + 2 * kPackStages + 2 * kWStages + 6 + s); };
-    const uint32_t barRows = barAt(2 * kTokStages + 2 * kPackStages + 2 * kWStages + 8);
+    constexpr int kBarW = 2 * kTokStages + 2 * kPackStages;
+    auto barWFull = [&](int s) { return barAt(kBarW + s); };
+    auto barAccFull = [&](int s) { return barAt(kBarW + kWStages + s); };
+    auto barAccEmpty = [&](int s) { return barAt(kBarW + kWStages + 2 + s); };
+    auto barXchg = [&](int set) { return barAt(kBarW + kWStages + 4 + set); };
+    auto barStage = [&](int set, int buffer) { return barAt(kBarW + kWStages + 4 + kEpilogueSets + 2 * set + buffer); };
+    const uint32_t barRows = barAt(kBarW + kWStages + 4 + 3 * kEpilogueSets);
 
     // The two CTAs of a cluster work as one unit of the tensor core: the leader (rank 0) issues
     // the MMAs for both.  Barriers that say "full" to the MMA issuer live in the leader and count
@@ -581,19 +590,19 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
         }
         for (int s = 0; s < kPackStages; ++s) {
             mbar_init(barPackFull(s), 1);
-            mbar_init(barPackEmpty(s), 4);  // the four warps of the group that read it
+            mbar_init(barPackEmpty(s), kDequantWarps);  // every dequantizing warp
         }
-        for (int s = 0; s < kWStages; ++s) {
-            mbar_init(barWFull(s), 8);   // (leader's is used) the four warps of the group in either CTA
-            mbar_init(barWEmpty(s), 1);  // (unused: the weight stages are released through the token ring)
-        }
+        for (int s = 0; s < kWStages; ++s) mbar_init(barWFull(s), 8);  // (leader's is used) the group's four warps in either CTA
         for (int s = 0; s < 2; ++s) {
-            mbar_init(barAccFull(s), 1);   // one tcgen05.commit
-            mbar_init(barAccEmpty(s), 8);  // (leader's is used) four epilogue warps in either CTA
-            mbar_init(barXchg(s), 128);    // every epilogue thread
-            mbar_init(barStage(s), 128);
+            mbar_init(barAccFull(s), 1);                     // one tcgen05.commit
+            mbar_init(barAccEmpty(s), 8 * kEpilogueSets);    // (leader's is used) the epilogue warps of either CTA
         }
-        mbar_init(barRows, 128);
+        for (int s = 0; s < kEpilogueSets; ++s) {
+            mbar_init(barXchg(s), 128);  // every thread of the set
+            mbar_init(barStage(s, 0), 128);
+            mbar_init(barStage(s, 1), 128);
+        }
+        mbar_init(barRows, kEpilogueThreads);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -607,15 +616,19 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
     __syncthreads();
     cluster_sync_all();  // the other CTA's barriers are initialised before anything arrives on them
     tc_fence_after();
-    const uint32_t tmemBase = tmemBaseSlot;
+    const uint32_t tmemBase = __shfl_sync(0xFFFFFFFFu, tmemBaseSlot, 0);
     pdl_enter();
 
     // A pair's unit: one row tile, two neighbouring weight-row tiles (this CTA takes 2 np + rank).
+    // Every role reads a unit's tile one unit ahead, so that the load's latency is not in its loop.
     const uint32_t rowTiles = args.counts[0];
     const uint32_t nPairs = (args.nTiles + 1u) >> 1;
     const uint32_t units = rowTiles * nPairs;
     const uint32_t firstUnit = blockIdx.x >> 1, unitStride = gridDim.x >> 1;
-    auto tileOf = [&](uint32_t u) { return args.tiles[u / nPairs]; };
+    auto tileOf = [&](uint32_t u) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(args.tiles + (u < units ? u : firstUnit) / nPairs));
+        return RowTile{v.x, v.y, v.z, v.w};
+    };
     auto ntOf = [&](uint32_t u) { return 2u * (u % nPairs) + ctaRank; };
     // accumulator columns of a tile: its rows to the next multiple of 32, half of them in either CTA
     auto columnsOf = [&](const RowTile &tile) { return max(32u, (tile.rows + 31u) & ~31u); };
@@ -623,33 +636,18 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
     // GEMM, matrix rows [128 nt, +128) for the down GEMM; loaded as two boxes of 64 rows
 
     if (warp == 0) {
-        // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            uint32_t ts = 0, tPhase = 0, ps = 0, pPhase = 0;
+        // ---------------- token copies ----------------
+        if (lane == 0 && firstUnit < units) {
+            uint32_t ts = 0, phase = 0;
             bool ok = true;
+            RowTile next = tileOf(firstUnit);
             for (uint32_t u = firstUnit; u < units && ok; u += unitStride) {
-                const RowTile tile = tileOf(u);
-                const uint32_t nt = ntOf(u);
+                const RowTile tile = next;
+                next = tileOf(u + unitStride);
                 // this CTA's half of the tile's rows
                 const int row0 = (int)(tile.rowStart + ctaRank * (columnsOf(tile) >> 1));
                 for (uint32_t g = 0; g < groupsK; ++g) {
-                    if (!mbar_wait_idle(barPackEmpty(ps), pPhase ^ 1u, &abortFlag)) {
-                        ok = false;
-                        break;
-                    }
-                    mbar_expect_tx(barPackFull(ps), kPackTileBytes);
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        const CUtensorMap *map = (MODE == kModeGateUp && q == 1) ? &mapW1 : &mapW0;
-                        const int wRow = MODE == kModeGateUp ? (int)nt * 64 : (int)nt * 128 + q * 64;
-                        tma_load_3d(packAddrOf(ps) + (uint32_t)q * (kPackTileBytes / 2), map,
-                                    (int)(g * (kTileK / 2)), wRow, (int)tile.expert, barPackFull(ps));
-                    }
-                    if (++ps == kPackStages) {
-                        ps = 0;
-                        pPhase ^= 1u;
-                    }
-                    if (!mbar_wait_idle(barTokEmpty(ts), tPhase ^ 1u, &abortFlag)) {
+                    if (!mbar_wait_idle(barTokEmpty(ts), phase ^ 1u, &abortFlag)) {
                         ok = false;
                         break;
                     }
@@ -657,231 +655,306 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
                     tma_load_2d(tokAddrOf(ts), &mapTok, (int)(g * kTileK), row0, barTokFull(ts));
                     if (++ts == kTokStages) {
                         ts = 0;
-                        tPhase ^= 1u;
+                        phase ^= 1u;
+                    }
+                }
+            }
+        }
+    } else if (warp == kCodeWarp) {
+        // ---------------- code copies: a quad of steps at a time ----------------
+        if (lane == 0 && firstUnit < units) {
+            uint32_t ps = 0, phase = 0;
+            bool ok = true;
+            RowTile next = tileOf(firstUnit);
+            for (uint32_t u = firstUnit; u < units && ok; u += unitStride) {
+                const RowTile tile = next;
+                next = tileOf(u + unitStride);
+                const uint32_t nt = ntOf(u);
+                for (uint32_t q = 0; q < quadsK; ++q) {
+                    if (!mbar_wait_idle(barPackEmpty(ps), phase ^ 1u, &abortFlag)) {
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(barPackFull(ps), kPackTileBytes);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const CUtensorMap *map = (MODE == kModeGateUp && h == 1) ? &mapW1 : &mapW0;
+                        const int wRow = MODE == kModeGateUp ? (int)nt * 64 : (int)nt * 128 + h * 64;
+                        tma_load_3d(packAddrOf(ps) + (uint32_t)h * (kPackTileBytes / 2), map,
+                                    (int)(q * (kQuad * kTileK / 2)), wRow, (int)tile.expert, barPackFull(ps));
+                    }
+                    if (++ps == kPackStages) {
+                        ps = 0;
+                        phase ^= 1u;
                     }
                 }
             }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (leader CTA only) ----------------
-        if (lane == 0 && leader) {
-            uint32_t ts = 0, ws = 0, wPhase = 0, acc = 0, accPhase = 0;
+        // The whole warp runs the loop and one elected lane issues: with the loop inside a `lane == 0`
+        // branch every operand goes to the uniform registers by a loop over the active lanes, and a step
+        // cost this thread 820 cycles for 384 of the tensor core.
+        if (leader && firstUnit < units) {
+            uint32_t ts = 0, wPhases = 0, acc = 0, accPhase = 0;  // wPhases: bit s = parity of weight stage s
             bool ok = true;
+            RowTile next = tileOf(firstUnit);
             for (uint32_t u = firstUnit; u < units && ok; u += unitStride) {
-                const RowTile tile = tileOf(u);
+                const RowTile tile = next;
+                next = tileOf(u + unitStride);
                 const uint32_t idesc = umma_idesc_bf16_m256(columnsOf(tile));
-                if (!mbar_wait_cluster<true>(barAccEmpty(acc), accPhase ^ 1u, &abortFlag)) break;
+                if (!mbar_wait_warp<true>(barAccEmpty(acc), accPhase ^ 1u, &abortFlag)) break;
                 tc_fence_after();
                 const uint32_t tmemD = tmemBase + acc * kAccCols;
                 for (uint32_t g = 0; g < groupsK; ++g) {
+                    const uint32_t ws = g % kWStages;
                     // (the group that arrives here has also seen both token halves land)
-                    if (!mbar_wait_cluster<false>(barWFull(ws), wPhase, &abortFlag)) {
+                    if (!mbar_wait_warp<false>(barWFull(ws), (wPhases >> ws) & 1u, &abortFlag)) {
                         ok = false;
                         break;
                     }
+                    wPhases ^= 1u << ws;
                     tc_fence_after();
                     const uint64_t descTok = umma_desc_sw128(tokAddrOf(ts));
                     const uint32_t tmemW = tmemBase + kWCol0 + ws * 32u;
+                    if (elect_one()) {
 #pragma unroll
-                    for (uint32_t kk = 0; kk < kTileK / 16; ++kk) {
-                        // per 16-element slice: eight columns further in TMEM, 32 bytes (>> 4 = 2)
-                        // further in the token tile
-                        tc_mma_bf16_a_tmem(tmemD, tmemW + 8u * kk, descTok + 2u * kk, idesc,
-                                           (g | kk) != 0u ? 1u : 0u);
+                        for (uint32_t kk = 0; kk < kTileK / 16; ++kk) {
+                            // per 16-element slice: eight columns further in TMEM, 32 bytes (>> 4 = 2)
+                            // further in the token tile
+                            tc_mma_bf16_a_tmem(tmemD, tmemW + 8u * kk, descTok + 2u * kk, idesc,
+                                               (g | kk) != 0u ? 1u : 0u);
+                        }
+                        // one signal per step: the token stage is free, and so is the weight stage that
+                        // the same step used (the dequantizers wait on the token ring's barrier, too)
+                        tc_commit_pair(barTokEmpty(ts));
                     }
-                    // one signal per step: the token stage is free, and so is the weight stage that
-                    // the same step used (the dequantizers wait on the token ring's barrier, too)
-                    tc_commit_pair(barTokEmpty(ts));
                     if (++ts == kTokStages) ts = 0;
-                    if (++ws == kWStages) {
-                        ws = 0;
-                        wPhase ^= 1u;
-                    }
                 }
                 if (!ok) break;
-                tc_commit_pair(barAccFull(acc));
+                if (elect_one()) tc_commit_pair(barAccFull(acc));
                 if (++acc == 2) {
                     acc = 0;
                     accPhase ^= 1u;
                 }
             }
         }
-    } else if (warp < 2 + kDequantWarps) {
+    } else if (warp < kFirstEpilogueWarp) {
         // ---------------- dequantizers ----------------
-        // Group `grp` (four warps, one per TMEM lane quarter) takes every fourth step of the CTA's
-        // sequence of steps and owns weight stage `grp`; a thread turns one weight row's 64 codes
-        // of the step into 32 bf16 pairs and stores them to its TMEM lane.  Four steps are in
-        // work at once, which hides a step's latencies behind the other groups' arithmetic.
+        // Group `grp` (four warps, one per TMEM lane quarter) takes step `grp` of every quad and owns
+        // weight stage `grp`; a thread turns one weight row's 64 codes of the step into 32 bf16 pairs
+        // and stores them to its TMEM lane.  Four steps are in work at once, which hides a step's
+        // latencies behind the other groups' arithmetic.
         const uint32_t grp = (uint32_t)(warp - 2) >> 2;
         const uint32_t m = (uint32_t)(warp & 3) * 32u + (uint32_t)lane;  // weight row of the unit = TMEM lane
         const uint32_t tmemW = tmemBase + kWCol0 + grp * 32u + (((uint32_t)(warp & 3) * 32u) << 16);
-        const uint32_t matrix = MODE == kModeGateUp ? (m >> 6) : 0u;
+        const uint32_t paddedK = (groupsK + 3u) & ~3u;
 
-        // The thread's scale/bias pairs of a unit (one per step it takes there) are fetched in one
-        // batch when it enters the unit and kept in a private column of shared memory, so that no
-        // global load is in flight in the steady loop (a load in flight would hold up the
-        // releasing arrive below for the load's whole latency).
-        uint32_t *myScales = scaleSlots + (uint32_t)(threadIdx.x - 64);  // [slot][512 threads]
-        uint32_t u = firstUnit, g = grp;   // the thread's current step: unit and step inside it
-        uint32_t gFirst = 0;               // its first step inside the current unit
-        auto enter_unit = [&]() {          // after u or g changed so that g < groupsK again, or at the start
-            while (g >= groupsK && u < units) {
-                g -= groupsK;
-                u += unitStride;
-            }
-            gFirst = g;
-            if (u >= units) return;
-            const RowTile tile = tileOf(u);
+        // The thread's scale words of a unit (one per quad) come as asynchronous copies into a private
+        // column of shared memory, one unit ahead: no global load is in flight in the steady loop (one
+        // in flight would hold up the releasing arrive below for its whole latency), and none is
+        // waited for at a unit's start.
+        const uint32_t myScales = scaleBase + 4u * (uint32_t)(threadIdx.x - 64);  // [buffer][quad][512 threads]
+        auto scale_row = [&](uint32_t u, const RowTile &tile, bool &live) {
             const uint32_t nt = ntOf(u);
             const uint32_t wRow = MODE == kModeGateUp ? nt * 64u + (m & 63u) : nt * 128u + m;
-            const bool liveRow = wRow < args.N;
-            const uint8_t *blob = args.blobBase + (size_t)tile.expert * args.expertStride;
-            // (selected, not indexed: a run-time index into the parameters would copy them to local memory)
-            const uint32_t scaleOff = matrix ? args.scaleOff[1] : args.scaleOff[0];
-            const uint32_t biasOff = matrix ? args.biasOff[1] : args.biasOff[0];
-            const uint16_t *sg = reinterpret_cast<const uint16_t *>(blob + scaleOff) + (size_t)wRow * groupsK;
-            const uint16_t *bg = reinterpret_cast<const uint16_t *>(blob + biasOff) + (size_t)wRow * groupsK;
-            for (uint32_t i0 = 0; g + 4u * i0 < groupsK; i0 += 4) {
-                uint32_t v[4];
-#pragma unroll
-                for (uint32_t i = 0; i < 4; ++i) {
-                    const uint32_t gi = min(g + 4u * (i0 + i), groupsK - 1u);
-                    v[i] = liveRow ? ((uint32_t)__ldg(sg + gi) | ((uint32_t)__ldg(bg + gi) << 16)) : 0u;
-                }
-#pragma unroll
-                for (uint32_t i = 0; i < 4; ++i)
-                    if (g + 4u * (i0 + i) < groupsK) myScales[(i0 + i) * (uint32_t)(kDequantWarps * 32)] = v[i];
-            }
+            live = wRow < args.N;
+            const uint32_t row = MODE == kModeGateUp ? (wRow >> 3) * 16u + (wRow & 7u) + (m >> 6) * 8u : wRow;
+            return args.scaleWords + (size_t)tile.expert * args.scaleStride + (size_t)(live ? row : 0u) * paddedK + grp;
         };
-        enter_unit();
+        auto fetch_scales = [&](uint32_t u, const RowTile &tile, uint32_t buffer) {
+            bool live;
+            const uint32_t *src = scale_row(u, tile, live);
+            uint32_t dst = myScales + buffer * quadsK * kScaleSlotBytes;
+            for (uint32_t q = 0; q < quadsK; ++q, dst += kScaleSlotBytes, src += kQuad)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(live ? 4u : 0u) : "memory");
+        };
+        auto scales_arrived = [] { asm volatile("cp.async.wait_all;" ::: "memory"); };
         const uint32_t leaderWFull = map_to_cta(barWFull(grp), 0u);
-        static_assert(kTokStages == kPackStages, "the dequantizers use one ring index for both");
-        uint32_t ps = grp % kPackStages, pPhase = 0, ownSteps = 0;
-        while (u < units) {
-            const uint32_t sb = myScales[((g - gFirst) >> 2) * (uint32_t)(kDequantWarps * 32)];
-            if (!mbar_wait(barPackFull(ps), pPhase, &abortFlag)) break;
-            uint32_t s2, b2;
-            asm("prmt.b32 %0, %1, %1, 0x1010;" : "=r"(s2) : "r"(sb));
-            asm("prmt.b32 %0, %1, %1, 0x3232;" : "=r"(b2) : "r"(sb));
-            uint32_t w[8];
-            const uint32_t src = packAddrOf(ps) + m * 32u;
-            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
-                         : "r"(src));
-            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
-                         : "r"(src + 16u));
-            uint32_t o[32];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    // codes i and i+4 of the word as the bf16 pair (128+q_i, 128+q_{i+4})
-                    uint32_t pair = ((w[j] >> (4 * i)) & 0x000F000Fu) | 0x43004300u;
-                    uint32_t q2, v2;
-                    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(q2) : "r"(pair), "r"(0x43004300u));
-                    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(v2) : "r"(q2), "r"(s2), "r"(b2));
-                    o[j * 4 + i] = v2;
-                }
-            }
-            // the codes are in registers: their tile may be copied over
-            __syncwarp();
-            if (lane == 0) mbar_arrive(barPackEmpty(ps));
-            // The weight stage `grp` was last read by the MMAs of this group's previous step, four
-            // steps back: its completion is that step's signal on the token ring (stage ps - 4,
-            // which in a ring of eight is ps + 4; the group's n-th step, n >= 1, meets that
-            // barrier's completion number (n - 1) / 2).  Waited for only here: the conversion above
-            // runs under those MMAs.
-            static_assert(kTokStages == 2 * kWStages, "the weight stages are released through the token ring");
-            if (ownSteps && !mbar_wait(barTokEmpty((ps + kWStages) % kTokStages), ((ownSteps - 1u) >> 1) & 1u, &abortFlag)) break;
-            tc_fence_after();
-            tc_store_32cols(tmemW, o);
-            // this CTA's half of the step's token tile must have landed before the MMA is told to go
-            const bool landed = mbar_wait(barTokFull(ps), pPhase, &abortFlag);
-            tc_wait_st();
-            if (!landed) break;
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(leaderWFull);
-            ps += kWStages;
-            if (ps >= kPackStages) {
-                ps -= kPackStages;
-                pPhase ^= 1u;
-            }
-            ++ownSteps;
-            g += kWStages;
-            if (g >= groupsK) enter_unit();
+        uint32_t ps = 0, pPhase = 0;
+        uint32_t step0 = 0;                 // steps of the CTA's earlier units
+        uint32_t lastStep = 0xFFFFFFFFu;    // this group's previous step
+        bool ok = firstUnit < units;
+        RowTile tile{}, next{};
+        if (ok) {
+            next = tileOf(firstUnit);
+            if (args.scaleBuffers) fetch_scales(firstUnit, next, 0);
         }
+        uint32_t unitNo = 0;
+        for (uint32_t u = firstUnit; u < units && ok; u += unitStride, ++unitNo, step0 += groupsK) {
+            tile = next;
+            next = tileOf(u + unitStride);
+            const uint32_t buffer = args.scaleBuffers == 2 ? unitNo & 1u : 0u;
+            if (args.scaleBuffers == 2) {
+                scales_arrived();
+                if (u + unitStride < units) fetch_scales(u + unitStride, next, buffer ^ 1u);
+            } else if (args.scaleBuffers == 1) {
+                if (unitNo) fetch_scales(u, tile, 0);
+                scales_arrived();
+            }
+            for (uint32_t q = 0; q < quadsK; ++q) {
+                if (!mbar_wait(barPackFull(ps), pPhase, &abortFlag)) {
+                    ok = false;
+                    break;
+                }
+                const uint32_t g = q * kQuad + grp;
+                uint32_t o[32];
+                if (g < groupsK) {
+                    uint32_t sb;
+                    if (args.scaleBuffers) {
+                        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sb) : "r"(myScales + (buffer * quadsK + q) * kScaleSlotBytes));
+                    } else {
+                        bool live;
+                        const uint32_t *src = scale_row(u, tile, live);
+                        sb = live ? __ldg(src + q * kQuad) : 0u;
+                    }
+                    uint32_t s2, b2;
+                    asm("prmt.b32 %0, %1, %1, 0x1010;" : "=r"(s2) : "r"(sb));
+                    asm("prmt.b32 %0, %1, %1, 0x3232;" : "=r"(b2) : "r"(sb));
+                    // the row's 128 bytes lie as eight 16-byte chunks with the 128-byte swizzle
+                    const uint32_t src = packAddrOf(ps) + m * 128u, flip = m & 7u;
+                    uint32_t w[8];
+#pragma unroll
+                    for (uint32_t c = 0; c < 2; ++c)
+                        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                     : "=r"(w[4 * c]), "=r"(w[4 * c + 1]), "=r"(w[4 * c + 2]), "=r"(w[4 * c + 3])
+                                     : "r"(src + (((2u * grp + c) ^ flip) << 4)));
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            // codes i and i+4 of the word as the bf16 pair (128+q_i, 128+q_{i+4})
+                            uint32_t pair = ((w[j] >> (4 * i)) & 0x000F000Fu) | 0x43004300u;
+                            uint32_t q2, v2;
+                            asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(q2) : "r"(pair), "r"(0x43004300u));
+                            asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(v2) : "r"(q2), "r"(s2), "r"(b2));
+                            o[j * 4 + i] = v2;
+                        }
+                    }
+                }
+                // the codes are in registers: their tile may be copied over
+                __syncwarp();
+                if (lane == 0) mbar_arrive(barPackEmpty(ps));
+                if (++ps == kPackStages) {
+                    ps = 0;
+                    pPhase ^= 1u;
+                }
+                if (g >= groupsK) continue;
+                // The weight stage was last read by the MMAs of this group's previous step: their completion
+                // is that step's signal on the token ring.  Waited for only here: the conversion above runs
+                // under those MMAs.
+                const uint32_t step = step0 + g, ts = step % kTokStages;
+                if (lastStep != 0xFFFFFFFFu &&
+                    !mbar_wait(barTokEmpty(lastStep % kTokStages), (lastStep / kTokStages) & 1u, &abortFlag)) {
+                    ok = false;
+                    break;
+                }
+                lastStep = step;
+                tc_fence_after();
+                tc_store_32cols(tmemW, o);
+                // this CTA's half of the step's token tile must have landed before the MMA is told to go
+                const bool landed = mbar_wait(barTokFull(ts), (step / kTokStages) & 1u, &abortFlag);
+                tc_wait_st();
+                if (!landed) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(leaderWFull);
+            }
+        }
+        scales_arrived();  // nothing of this thread's is in flight when shared memory is released
     } else {
         // ---------------- epilogue: TMEM -> registers -> shared -> global ----------------
         // A thread holds one weight row's results for the unit's tokens (one token per accumulator
-        // column).  Per 32 tokens the four warps put their bf16 results into a [token][output]
-        // tile in shared memory and then write it out a token row at a time, 16 bytes per thread.
-        // All buffers alternate between two copies: a copy is rewritten two chunks (or units)
-        // later, after every thread has passed a barrier in between, hence after it was read.
+        // column).  Two sets of four warps take 32-token chunks in turn; a set puts its bf16 results
+        // into a [token][output] tile in shared memory and then writes it out a token row at a time,
+        // 16 bytes per thread.
+        const uint32_t set = (uint32_t)(warp - kFirstEpilogueWarp) >> 2;
         const uint32_t quarter = (uint32_t)(warp & 3);
         const uint32_t m = quarter * 32u + (uint32_t)lane;
-        const uint32_t t = (uint32_t)threadIdx.x - (2u + kDequantWarps) * 32u;  // 0..127
+        const uint32_t te = (uint32_t)threadIdx.x - kFirstEpilogueWarp * 32u;  // 0..255
+        const uint32_t t = te & 127u;                                          // within the set
+        float *xchg = reinterpret_cast<float *>(epilogueSmem + set * kXchgBytes);  // gate/up only
+        uint8_t *stageBuf = epilogueSmem + (MODE == kModeGateUp ? kEpilogueSets * kXchgBytes + set * kStageBytesGateUp
+                                                                : set * 2u * kStageBytesDown);
+        uint32_t *rowTable = reinterpret_cast<uint32_t *>(epilogueSmem + kEpilogueSets * 2u * kStageBytesDown);  // down only
         uint32_t acc = 0, accPhase = 0, chunk = 0, unitNo = 0;
         bool ok = true;
+        // where a row of a unit goes (down), looked up one unit ahead
+        auto row_target = [&](const RowTile &tile, uint32_t r) {
+            uint32_t outRow = tile.rowStart + min(r, tile.rows - 1u);
+            if (args.pairs) {
+                const uint4 p = __ldg(reinterpret_cast<const uint4 *>(args.pairs + outRow));
+                outRow = p.x * args.topK + p.z;  // token, expert, rank, -
+            }
+            return outRow;
+        };
+        RowTile tile{}, next{};
+        uint32_t nextTarget = 0;
+        if (firstUnit < units) {
+            next = tileOf(firstUnit);
+            if (MODE == kModeDown) nextTarget = row_target(next, te);
+        }
         for (uint32_t u = firstUnit; u < units && ok; u += unitStride, ++unitNo) {
-            const RowTile tile = tileOf(u);
+            tile = next;
+            next = tileOf(u + unitStride);
             const uint32_t nt = ntOf(u);
             uint32_t *rowOf = rowTable + (unitNo & 1u) * kRowTile;
             if (MODE == kModeDown) {
-                // where each of the unit's rows goes
-                for (uint32_t r = t; r < tile.rows; r += 128u) {
-                    uint32_t outRow = tile.rowStart + r;
-                    if (args.pairs) {
-                        const FFTokenExpertPair p = args.pairs[outRow];
-                        outRow = p.token * args.topK + p.rank;
-                    }
-                    rowOf[r] = outRow;
-                }
+                if (te < kRowTile) rowOf[te] = nextTarget;
                 mbar_arrive(barRows);
+                nextTarget = row_target(next, te);
             }
             if (!mbar_wait_idle(barAccFull(acc), accPhase, &abortFlag)) break;
             if (MODE == kModeDown && !mbar_wait(barRows, unitNo & 1u, &abortFlag)) break;
             tc_fence_after();
             const uint32_t taddr = tmemBase + acc * kAccCols + ((quarter * 32u) << 16);
 #pragma unroll 1
-            for (uint32_t c0 = 0; c0 < tile.rows; c0 += 32, ++chunk) {
+            for (uint32_t c0 = 32u * set; c0 < tile.rows; c0 += 32u * kEpilogueSets, ++chunk) {
                 uint32_t v[32];
                 tc_load_32cols(taddr + c0, v);
                 tc_wait_ld();
-                const uint32_t which = chunk & 1u, parity = (chunk >> 1) & 1u;
-                uint8_t *stage = stageBuf + which * kStageBytes;
                 if (MODE == kModeGateUp) {
                     // lanes 0..63 hold gate, lanes 64..127 up of features [64 nt, +64).  The gate
                     // warps hand the second 16 tokens' gates to the up warps and take the first 16
                     // tokens' ups from them; either side then finishes 16 tokens of its feature.
+                    // (One buffer each: the exchange rows are rewritten behind barStage, the output
+                    // tile behind the next barXchg, which every thread reaches after its last read.)
                     const bool isUp = m >= 64u;
-                    float *buf = xchg + which * (128u * kXchgPitch);
-                    float *mine = buf + m * kXchgPitch;
+                    float *mine = xchg + m * kXchgPitch;
 #pragma unroll
                     for (int j = 0; j < 16; ++j) mine[j] = __uint_as_float(isUp ? v[j] : v[16 + j]);
-                    mbar_arrive(barXchg(which));
-                    if (!mbar_wait(barXchg(which), parity, &abortFlag)) {
+                    mbar_arrive(barXchg(set));
+                    if (!mbar_wait(barXchg(set), chunk & 1u, &abortFlag)) {
                         ok = false;
                         break;
                     }
-                    const float *theirs = buf + (m ^ 64u) * kXchgPitch;
+                    const float *theirs = xchg + (m ^ 64u) * kXchgPitch;
                     // tile [32 tokens][64 features in the interleaved order], 144-byte pitch
-                    uint16_t *col = reinterpret_cast<uint16_t *>(stage) + (isUp ? 16u : 0u) * (kStagePitchGateUp / 2) +
+                    uint16_t *col = reinterpret_cast<uint16_t *>(stageBuf) + (isUp ? 16u : 0u) * (kStagePitchGateUp / 2) +
                                     interleaved_position(m & 63u);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const float own = __uint_as_float(isUp ? v[16 + j] : v[j]);
-                        const float other = theirs[j];
-                        float g = isUp ? other : own, uu = isUp ? own : other;
-                        if (args.roundGateUp) {
-                            g = bf2f(f2bf(g));
-                            uu = bf2f(f2bf(uu));
+                    for (int j = 0; j < 16; j += 2) {
+                        float act[2];
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const float own = __uint_as_float(isUp ? v[16 + j + i] : v[j + i]);
+                            const float other = theirs[j + i];
+                            float g = isUp ? other : own, uu = isUp ? own : other;
+                            if (args.roundGateUp) {
+                                g = bf16_round(g);
+                                uu = bf16_round(uu);
+                            }
+                            act[i] = gelu_tanh_fast(g) * uu;
                         }
-                        col[(uint32_t)j * (kStagePitchGateUp / 2)] = f2bf(gelu_tanh_fast(g) * uu);
+                        const uint32_t two = bf16_pair(act[0], act[1]);
+                        col[(uint32_t)j * (kStagePitchGateUp / 2)] = (uint16_t)two;
+                        col[(uint32_t)(j + 1) * (kStagePitchGateUp / 2)] = (uint16_t)(two >> 16);
                     }
-                    mbar_arrive(barStage(which));
-                    if (!mbar_wait(barStage(which), parity, &abortFlag)) {
+                    mbar_arrive(barStage(set, 0));
+                    if (!mbar_wait(barStage(set, 0), chunk & 1u, &abortFlag)) {
                         ok = false;
                         break;
                     }
@@ -892,18 +965,24 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
                     for (uint32_t pass = 0; pass < 2; ++pass) {
                         const uint32_t tok = pass * 16u + (t >> 3);
                         if (c0 + tok < tile.rows && col0 < args.N) {
-                            const uint4 val = *reinterpret_cast<const uint4 *>(stage + tok * kStagePitchGateUp + piece * 16u);
+                            const uint4 val = *reinterpret_cast<const uint4 *>(stageBuf + tok * kStagePitchGateUp + piece * 16u);
                             *reinterpret_cast<uint4 *>(args.out + (size_t)(tile.rowStart + c0 + tok) * args.N + col0) = val;
                         }
                     }
                 } else {
-                    // tile [32 tokens][128 outputs], 272-byte pitch
+                    // tile [32 tokens][128 outputs], 272-byte pitch; two tiles in turn (one is rewritten
+                    // two chunks later, after every thread has passed the barrier in between)
+                    const uint32_t buffer = chunk & 1u;
+                    uint8_t *stage = stageBuf + buffer * kStageBytesDown;
                     uint16_t *col = reinterpret_cast<uint16_t *>(stage) + m;
 #pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        col[(uint32_t)j * (kStagePitchDown / 2)] = f2bf(__uint_as_float(v[j]));
-                    mbar_arrive(barStage(which));
-                    if (!mbar_wait(barStage(which), parity, &abortFlag)) {
+                    for (int j = 0; j < 32; j += 2) {
+                        const uint32_t two = bf16_pair(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
+                        col[(uint32_t)j * (kStagePitchDown / 2)] = (uint16_t)two;
+                        col[(uint32_t)(j + 1) * (kStagePitchDown / 2)] = (uint16_t)(two >> 16);
+                    }
+                    mbar_arrive(barStage(set, buffer));
+                    if (!mbar_wait(barStage(set, buffer), (chunk >> 1) & 1u, &abortFlag)) {
                         ok = false;
                         break;
                     }
@@ -987,7 +1066,6 @@ static bool make_router_map(CUtensorMap *map, const void *base, uint64_t experts
     return true;
 }
 
-// packed codes of one matrix across all experts: bytes [experts][rows][cols/2], box 32 x 64 x 1.
 // Packed codes of one matrix across all experts seen as 64-bit words [experts][rows][rowBytes/8],
 // box `boxBytes` x `boxRows` x 1 without swizzle: a tile of whole row pieces in one copy, rows
 // `boxBytes` apart in shared memory.  Out-of-range parts of a box read as zero.
@@ -1008,16 +1086,19 @@ bool make_row_box_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_
     return true;
 }
 
+// Packed codes of one matrix across all experts: bytes [experts][rows][cols/2], box 64 rows x 128 bytes (four
+// steps; parts past a row read as zero), 128-byte swizzle so that a warp's 128-bit reads of 32 rows meet no
+// bank twice.  (Boxes of one step's 32 bytes kept the copying thread busy for 600 cycles a step.)
 static bool make_weight_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols,
                             uint64_t experts, uint64_t expertStride, const char **error) {
     EncodeTiledFn fn = encode_tiled(error);
     if (!fn) return false;
     cuuint64_t dims[3] = {cols / 2, rows, experts};
     cuuint64_t strides[2] = {cols / 2, expertStride};
-    cuuint32_t box[3] = {(cuuint32_t)(kTileK / 2), 64, 1};
+    cuuint32_t box[3] = {(cuuint32_t)(kQuad * kTileK / 2), 64, 1};
     cuuint32_t elem[3] = {1, 1, 1};
     CUresult rc = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void *>(base), dims, strides,
-                     box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                     box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (rc != CUDA_SUCCESS) return fail(error, "cuTensorMapEncodeTiled(weights) failed: " + std::to_string((int)rc));
     return true;
@@ -1050,19 +1131,22 @@ bool prefill_prepare_layer(FFContext *ctx, LayerStore &L, const char **error) {
     return true;
 }
 
-static size_t gemm_smem_bytes(int mode, uint32_t K) {
-    const size_t scaleSlots = (size_t)((K / kTileK + kGroups - 1) / kGroups) * kDequantWarps * 32 * sizeof(uint32_t);
+// Shared memory of a GEMM over K with `buffers` units' scale words.
+static size_t gemm_smem_bytes(int mode, uint32_t K, uint32_t buffers) {
+    const size_t quads = (K / kTileK + kQuad - 1) / kQuad;
     return 1024 + (size_t)kTokStages * kTokTileBytes + (size_t)kPackStages * kPackTileBytes +
-           (mode == kModeGateUp ? kEpilogueBytesGateUp : kEpilogueBytesDown) + scaleSlots;
+           (mode == kModeGateUp ? kEpilogueBytesGateUp : kEpilogueBytesDown) + buffers * quads * kScaleSlotBytes;
 }
 
 template <int MODE>
 static bool launch_gemm(FFContext *ctx, const CUtensorMap &mapA, const CUtensorMap &mapW0,
-                        const CUtensorMap &mapW1, const GemmArgs &args, uint32_t maxUnits,
+                        const CUtensorMap &mapW1, GemmArgs args, uint32_t maxUnits,
                         cudaStream_t stream, const char **error) {
     auto kernel = k_grouped_int4_gemm<MODE>;
-    const size_t smem = gemm_smem_bytes(MODE, args.K);
-    if (smem > 226 * 1024) return fail(error, "contraction length too large for the GEMM's shared memory");
+    // scale words one unit ahead where they fit, else the unit's own, else none (read step by step)
+    args.scaleBuffers = 2;
+    while (args.scaleBuffers && gemm_smem_bytes(MODE, args.K, args.scaleBuffers) > 226 * 1024) --args.scaleBuffers;
+    const size_t smem = gemm_smem_bytes(MODE, args.K, args.scaleBuffers);
     static KernelSmemMemo memo;
     if (!memo.prepare(kernel, ctx->device, smem, kGemmThreads, nullptr, error)) return false;
     // clusters of two CTAs; a cluster takes (row tile, pair of weight-row tiles) units
@@ -1132,12 +1216,8 @@ bool launch_prefill_routed(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     if (!make_activation_map(&mapActs, ctx->acts, (uint64_t)pairs + 256, c.f, c.f, error)) return false;
 
     GemmArgs a{};
-    a.blobBase = L.experts;
-    a.expertStride = L.stride;
-    a.scaleOff[0] = L.off.gateSOff;
-    a.biasOff[0] = L.off.gateBOff;
-    a.scaleOff[1] = L.off.upSOff;
-    a.biasOff[1] = L.off.upBOff;
+    a.scaleWords = L.routedScales;
+    a.scaleStride = scale_words(c.d, c.f);
     a.K = c.d;
     a.N = c.f;
     a.nTiles = (c.f + 63) / 64;
@@ -1153,8 +1233,7 @@ bool launch_prefill_routed(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
         return false;
 
     GemmArgs b = a;
-    b.scaleOff[0] = b.scaleOff[1] = L.off.downSOff;
-    b.biasOff[0] = b.biasOff[1] = L.off.downBOff;
+    b.scaleWords = L.routedScales + scale_words_gate_up(c.d, c.f);
     b.K = c.f;
     b.N = c.d;
     b.nTiles = (c.d + 127) / 128;
@@ -1232,15 +1311,8 @@ bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     if (!make_activation_map(&mapX, ctx->xSorted, (uint64_t)tokens + 256, c.d, c.d, error)) return false;
     if (!make_activation_map(&mapActs, ctx->sharedActs, (uint64_t)tokens + 256, c.sharedF, c.sharedF, error))
         return false;
-    uint64_t payload = 0;
-    packed_offsets(c.d, c.sharedF, &payload);
     GemmArgs a{};
-    a.blobBase = L.shared;
-    a.expertStride = (payload + 15) & ~15ull;
-    a.scaleOff[0] = L.sharedOff.gateSOff;
-    a.biasOff[0] = L.sharedOff.gateBOff;
-    a.scaleOff[1] = L.sharedOff.upSOff;
-    a.biasOff[1] = L.sharedOff.upBOff;
+    a.scaleWords = L.sharedScales;
     a.K = c.d;
     a.N = c.sharedF;
     a.nTiles = (c.sharedF + 63) / 64;
@@ -1254,8 +1326,7 @@ bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
                                   error))
         return false;
     GemmArgs b = a;
-    b.scaleOff[0] = b.scaleOff[1] = L.sharedOff.downSOff;
-    b.biasOff[0] = b.biasOff[1] = L.sharedOff.downBOff;
+    b.scaleWords = L.sharedScales + scale_words_gate_up(c.d, c.sharedF);
     b.K = c.sharedF;
     b.N = c.d;
     b.nTiles = (c.d + 127) / 128;

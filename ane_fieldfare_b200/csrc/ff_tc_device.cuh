@@ -212,6 +212,28 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
     if (mbar_try_wait_cluster(bar, parity)) return true;
     return mbar_wait_cluster_slow<kSleep>(bar, parity, abortFlag);
 }
+// A wait of a whole converged warp whose lanes then act as one: either all of them go on or none.  Acquires
+// at CTA scope also where the other CTA arrives: what that CTA wrote for the MMA is ordered by the
+// tcgen05 fences, and a cluster-scope acquire costs over a hundred cycles.
+template <bool kSleep>
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t *abortFlag) {
+    if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+    return __all_sync(0xFFFFFFFFu, mbar_wait_slow<kSleep>(bar, parity, abortFlag));
+}
+// one lane of the converged warp (the form in which the compiler knows that a single lane is active)
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "elect.sync _|p, 0xFFFFFFFF;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(one));
+    return one != 0;
+}
+// the warp's index, known to be the same in all its lanes
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n"
                  "barrier.cluster.wait.acquire.aligned;" ::: "memory");
