@@ -697,7 +697,7 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
         // cost this thread 820 cycles for 384 of the tensor core.
         if (leader && firstUnit < units) {
             uint32_t ts = 0, wPhases = 0, acc = 0, accPhase = 0;  // wPhases: bit s = parity of weight stage s
-            bool ok = true;
+            bool ok = true, ready = false;                        // ready: seen that the next step's weights are there
             RowTile next = tileOf(firstUnit);
             for (uint32_t u = firstUnit; u < units && ok; u += unitStride) {
                 const RowTile tile = next;
@@ -706,37 +706,43 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
                 if (!mbar_wait_warp<true>(barAccEmpty(acc), accPhase ^ 1u, &abortFlag)) break;
                 tc_fence_after();
                 const uint32_t tmemD = tmemBase + acc * kAccCols;
-                for (uint32_t g = 0; g < groupsK; ++g) {
-                    const uint32_t ws = g % kWStages;
-                    // (the group that arrives here has also seen both token halves land)
-                    if (!mbar_wait_warp<false>(barWFull(ws), (wPhases >> ws) & 1u, &abortFlag)) {
-                        ok = false;
-                        break;
-                    }
-                    wPhases ^= 1u << ws;
-                    tc_fence_after();
-                    const uint64_t descTok = umma_desc_sw128(tokAddrOf(ts));
-                    const uint32_t tmemW = tmemBase + kWCol0 + ws * 32u;
-                    if (elect_one()) {
+                for (uint32_t g0 = 0; g0 < groupsK && ok; g0 += kWStages) {
 #pragma unroll
-                        for (uint32_t kk = 0; kk < kTileK / 16; ++kk) {
-                            // per 16-element slice: eight columns further in TMEM, 32 bytes (>> 4 = 2)
-                            // further in the token tile
-                            tc_mma_bf16_a_tmem(tmemD, tmemW + 8u * kk, descTok + 2u * kk, idesc,
-                                               (g | kk) != 0u ? 1u : 0u);
+                    for (uint32_t ws = 0; ws < kWStages; ++ws) {
+                        const uint32_t g = g0 + ws;
+                        if (g >= groupsK) break;
+                        // (the group that arrives here has also seen both token halves land)
+                        if (!__all_sync(0xFFFFFFFFu, ready) &&
+                            !mbar_wait_warp<false>(barWFull(ws), (wPhases >> ws) & 1u, &abortFlag)) {
+                            ok = false;
+                            break;
                         }
-                        // one signal per step: the token stage is free, and so is the weight stage that
-                        // the same step used (the dequantizers wait on the token ring's barrier, too)
-                        tc_commit_pair(barTokEmpty(ts));
+                        wPhases ^= 1u << ws;
+                        tc_fence_after();
+                        // the next step's barrier is looked at now and the answer used after this step's MMAs
+                        const uint32_t wn = g + 1u < groupsK ? (ws + 1u) % kWStages : 0u;
+                        ready = mbar_test_wait(barWFull(wn), (wPhases >> wn) & 1u);
+                        const uint64_t descTok = umma_desc_sw128(tokAddrOf(ts));
+                        const uint32_t tmemW = tmemBase + kWCol0 + ws * 32u;
+                        if (elect_one()) {
+#pragma unroll
+                            for (uint32_t kk = 0; kk < kTileK / 16; ++kk) {
+                                // per 16-element slice: eight columns further in TMEM, 32 bytes (>> 4 = 2)
+                                // further in the token tile
+                                tc_mma_bf16_a_tmem(tmemD, tmemW + 8u * kk, descTok + 2u * kk, idesc,
+                                                   (g | kk) != 0u ? 1u : 0u);
+                            }
+                            // one signal per step: the token stage is free, and so is the weight stage that
+                            // the same step used (the dequantizers wait on the token ring's barrier, too)
+                            tc_commit_pair(barTokEmpty(ts));
+                        }
+                        ts = (ts + 1u) % kTokStages;
                     }
-                    if (++ts == kTokStages) ts = 0;
                 }
                 if (!ok) break;
                 if (elect_one()) tc_commit_pair(barAccFull(acc));
-                if (++acc == 2) {
-                    acc = 0;
-                    accPhase ^= 1u;
-                }
+                acc ^= 1u;
+                accPhase ^= acc == 0u ? 1u : 0u;
             }
         }
     } else if (warp < kFirstEpilogueWarp) {

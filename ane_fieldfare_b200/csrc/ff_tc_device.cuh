@@ -38,6 +38,20 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+// one look, without the suspension that a try_wait may take
+__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 // Bounded wait.  Returns false when the limit ran out or another thread of the CTA gave up; the
 // caller leaves its loop.  `abortFlag` lives in shared memory.  kSleep: pause between polls, for
 // the warps whose polling would otherwise take issue slots from the dequantizing warps.
