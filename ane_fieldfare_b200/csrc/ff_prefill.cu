@@ -495,14 +495,12 @@ constexpr uint32_t kPackTileBytes = kWeightRows * kTileK / 2 * kQuad;  // 16384:
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kAccCols = kRowTile;                           // accumulators at columns 0 and 192
 constexpr uint32_t kWCol0 = 2 * kAccCols;                         // weight stages: 32 columns each from 384
-constexpr int kXchgPitch = 17;                                    // floats per exchanged row (16 + 1 pad)
-constexpr uint32_t kXchgBytes = 128u * kXchgPitch * 4u;           // one set's exchange buffer
 constexpr uint32_t kStagePitchGateUp = 64 * 2 + 16;               // bytes per token row of the output tile
 constexpr uint32_t kStagePitchDown = 128 * 2 + 16;
 constexpr uint32_t kStageBytesGateUp = 32u * kStagePitchGateUp;   // one 32-token output tile
 constexpr uint32_t kStageBytesDown = 32u * kStagePitchDown;
-// gate/up: per set an exchange buffer and an output tile; down: per set two output tiles, two row tables
-constexpr uint32_t kEpilogueBytesGateUp = kEpilogueSets * (kXchgBytes + kStageBytesGateUp);
+// per set two output tiles; down: two row tables, too
+constexpr uint32_t kEpilogueBytesGateUp = kEpilogueSets * 2u * kStageBytesGateUp;
 constexpr uint32_t kEpilogueBytesDown = kEpilogueSets * 2u * kStageBytesDown + 2u * kRowTile * 4u;
 constexpr uint32_t kScaleSlotBytes = kDequantWarps * 32 * 4;      // a scale word of every dequantizing thread
 static_assert(kWCol0 + kWStages * 32 <= kTmemCols, "tensor memory layout");
@@ -527,9 +525,13 @@ struct GemmArgs {
     uint32_t *errorFlag;
 };
 
-// position of element i of an aligned run of eight in the order 0,4,1,5,2,6,3,7
-__device__ __forceinline__ uint32_t interleaved_position(uint32_t i) {
-    return (i & ~7u) | (((i & 3u) << 1) | ((i >> 2) & 1u));
+// element at position p of a run of eight in the order 0,4,1,5,2,6,3,7
+__device__ __forceinline__ uint32_t interleaved_element(uint32_t p) { return (p >> 1) | ((p & 1u) << 2); }
+// eight columns each of four 8 x 8 bf16 blocks, transposed: lane l gives the address of row l & 7 of block l >> 3
+__device__ __forceinline__ void store_blocks_transposed(uint32_t addr, const uint32_t (&p)[4]) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(p[0]), "r"(p[1]), "r"(p[2]),
+                 "r"(p[3])
+                 : "memory");
 }
 // two floats as bf16, the first in the low half
 __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
@@ -538,12 +540,49 @@ __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
     return r;
 }
 
+// bf16 fma(q, scale, bias) of the 64 codes of eight words, as pairs (code i, code i + 4).  A nibble masked in
+// place, at bits 0-3 or 4-7 of a half word, IS a bf16: the subnormal q * 2^-133 or (exponent field 0 or 1) the
+// number q * 2^-129.  The FMA takes it as it stands, with the scale times 2^133 or 2^129: the same product, the
+// same single rounding, 9 instructions for a word where taking the nibble to q itself needs 15.  Scales whose
+// product with 2^133 is no normal bf16 (from 2^-5 on, and subnormal ones) take the longer way, a warp at a time.
+__device__ __forceinline__ void dequantize_words(const uint32_t (&w)[8], uint32_t scaleBias, uint32_t (&o)[32]) {
+    uint32_t s2, b2;
+    asm("prmt.b32 %0, %1, %1, 0x1010;" : "=r"(s2) : "r"(scaleBias));
+    asm("prmt.b32 %0, %1, %1, 0x3232;" : "=r"(b2) : "r"(scaleBias));
+    const uint32_t magnitude = s2 & 0x7FFFu;
+    constexpr uint32_t kMinNormal = 0x0080u, kLimit = 0x3D00u;  // 2^-126, 2^-5
+    if (__all_sync(0xFFFFFFFFu, magnitude == 0u || magnitude - kMinNormal < kLimit - kMinNormal)) {
+        const uint32_t sLow = magnitude ? s2 + 0x42804280u : 0u;   // exponent + 133
+        const uint32_t sHigh = magnitude ? s2 + 0x40804080u : 0u;  // exponent + 129
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t upper = w[j] >> 8;
+            asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(o[4 * j]) : "r"(w[j] & 0x000F000Fu), "r"(sLow), "r"(b2));
+            asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(o[4 * j + 1]) : "r"(w[j] & 0x00F000F0u), "r"(sHigh), "r"(b2));
+            asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(o[4 * j + 2]) : "r"(upper & 0x000F000Fu), "r"(sLow), "r"(b2));
+            asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(o[4 * j + 3]) : "r"(upper & 0x00F000F0u), "r"(sHigh), "r"(b2));
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                // codes i and i+4 of the word as the bf16 pair (128+q_i, 128+q_{i+4})
+                const uint32_t pair = ((w[j] >> (4 * i)) & 0x000F000Fu) | 0x43004300u;
+                uint32_t q2;
+                asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(q2) : "r"(pair), "r"(0x43004300u));
+                asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(o[4 * j + i]) : "r"(q2), "r"(s2), "r"(b2));
+            }
+        }
+    }
+}
+
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ CUtensorMap mapW0,
                     const __grid_constant__ CUtensorMap mapW1, const GemmArgs args) {
     extern __shared__ uint8_t gemmSmemRaw[];
-    __shared__ uint64_t barriers[2 * kTokStages + 2 * kPackStages + kWStages + 4 + 3 * kEpilogueSets + 1];
+    __shared__ uint64_t barriers[2 * kTokStages + 2 * kPackStages + kWStages + 4 + 2 * kEpilogueSets + 1];
     __shared__ uint32_t tmemBaseSlot;
     __shared__ volatile uint32_t abortFlag;
 
@@ -572,9 +611,8 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
     auto barWFull = [&](int s) { return barAt(kBarW + s); };
     auto barAccFull = [&](int s) { return barAt(kBarW + kWStages + s); };
     auto barAccEmpty = [&](int s) { return barAt(kBarW + kWStages + 2 + s); };
-    auto barXchg = [&](int set) { return barAt(kBarW + kWStages + 4 + set); };
-    auto barStage = [&](int set, int buffer) { return barAt(kBarW + kWStages + 4 + kEpilogueSets + 2 * set + buffer); };
-    const uint32_t barRows = barAt(kBarW + kWStages + 4 + 3 * kEpilogueSets);
+    auto barStage = [&](int set, int buffer) { return barAt(kBarW + kWStages + 4 + 2 * set + buffer); };
+    const uint32_t barRows = barAt(kBarW + kWStages + 4 + 2 * kEpilogueSets);
 
     // The two CTAs of a cluster work as one unit of the tensor core: the leader (rank 0) issues
     // the MMAs for both.  Barriers that say "full" to the MMA issuer live in the leader and count
@@ -598,8 +636,7 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
             mbar_init(barAccEmpty(s), 8 * kEpilogueSets);    // (leader's is used) the epilogue warps of either CTA
         }
         for (int s = 0; s < kEpilogueSets; ++s) {
-            mbar_init(barXchg(s), 128);  // every thread of the set
-            mbar_init(barStage(s, 0), 128);
+            mbar_init(barStage(s, 0), 128);  // every thread of the set
             mbar_init(barStage(s, 1), 128);
         }
         mbar_init(barRows, kEpilogueThreads);
@@ -632,8 +669,11 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
     auto ntOf = [&](uint32_t u) { return 2u * (u % nPairs) + ctaRank; };
     // accumulator columns of a tile: its rows to the next multiple of 32, half of them in either CTA
     auto columnsOf = [&](const RowTile &tile) { return max(32u, (tile.rows + 31u) & ~31u); };
-    // weight rows 0..127 of a unit: gate rows [64 nt, +64) | up rows [64 nt, +64) for the gate/up
-    // GEMM, matrix rows [128 nt, +128) for the down GEMM; loaded as two boxes of 64 rows
+    // weight rows of a unit: gate rows [64 nt, +64) | up rows [64 nt, +64) for the gate/up
+    // GEMM, matrix rows [128 nt, +128) for the down GEMM; loaded as two boxes of 64 rows.  In tensor
+    // memory gate and up stand in turn, eight lanes each, so that the epilogue's threads find both
+    // values of a feature in their own registers, and a run of eight features stands in the
+    // interleaved order that the down GEMM reads.
 
     if (warp == 0) {
         // ---------------- token copies ----------------
@@ -752,7 +792,10 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
         // and stores them to its TMEM lane.  Four steps are in work at once, which hides a step's
         // latencies behind the other groups' arithmetic.
         const uint32_t grp = (uint32_t)(warp - 2) >> 2;
-        const uint32_t m = (uint32_t)(warp & 3) * 32u + (uint32_t)lane;  // weight row of the unit = TMEM lane
+        const uint32_t m = (uint32_t)(warp & 3) * 32u + (uint32_t)lane;  // TMEM lane
+        // its feature within the unit (gate/up), its row in the loaded boxes
+        const uint32_t feature = (m >> 4) * 8u + interleaved_element(m & 7u);
+        const uint32_t boxRow = MODE == kModeGateUp ? ((m >> 3) & 1u) * 64u + feature : m;
         const uint32_t tmemW = tmemBase + kWCol0 + grp * 32u + (((uint32_t)(warp & 3) * 32u) << 16);
         const uint32_t paddedK = (groupsK + 3u) & ~3u;
 
@@ -763,9 +806,9 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
         const uint32_t myScales = scaleBase + 4u * (uint32_t)(threadIdx.x - 64);  // [buffer][quad][512 threads]
         auto scale_row = [&](uint32_t u, const RowTile &tile, bool &live) {
             const uint32_t nt = ntOf(u);
-            const uint32_t wRow = MODE == kModeGateUp ? nt * 64u + (m & 63u) : nt * 128u + m;
+            const uint32_t wRow = MODE == kModeGateUp ? nt * 64u + feature : nt * 128u + m;
             live = wRow < args.N;
-            const uint32_t row = MODE == kModeGateUp ? (wRow >> 3) * 16u + (wRow & 7u) + (m >> 6) * 8u : wRow;
+            const uint32_t row = MODE == kModeGateUp ? (wRow >> 3) * 16u + (wRow & 7u) + (m & 8u) : wRow;
             return args.scaleWords + (size_t)tile.expert * args.scaleStride + (size_t)(live ? row : 0u) * paddedK + grp;
         };
         auto fetch_scales = [&](uint32_t u, const RowTile &tile, uint32_t buffer) {
@@ -814,29 +857,15 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
                         const uint32_t *src = scale_row(u, tile, live);
                         sb = live ? __ldg(src + q * kQuad) : 0u;
                     }
-                    uint32_t s2, b2;
-                    asm("prmt.b32 %0, %1, %1, 0x1010;" : "=r"(s2) : "r"(sb));
-                    asm("prmt.b32 %0, %1, %1, 0x3232;" : "=r"(b2) : "r"(sb));
                     // the row's 128 bytes lie as eight 16-byte chunks with the 128-byte swizzle
-                    const uint32_t src = packAddrOf(ps) + m * 128u, flip = m & 7u;
+                    const uint32_t src = packAddrOf(ps) + boxRow * 128u, flip = boxRow & 7u;
                     uint32_t w[8];
 #pragma unroll
                     for (uint32_t c = 0; c < 2; ++c)
                         asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                                      : "=r"(w[4 * c]), "=r"(w[4 * c + 1]), "=r"(w[4 * c + 2]), "=r"(w[4 * c + 3])
                                      : "r"(src + (((2u * grp + c) ^ flip) << 4)));
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            // codes i and i+4 of the word as the bf16 pair (128+q_i, 128+q_{i+4})
-                            uint32_t pair = ((w[j] >> (4 * i)) & 0x000F000Fu) | 0x43004300u;
-                            uint32_t q2, v2;
-                            asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(q2) : "r"(pair), "r"(0x43004300u));
-                            asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(v2) : "r"(q2), "r"(s2), "r"(b2));
-                            o[j * 4 + i] = v2;
-                        }
-                    }
+                    dequantize_words(w, sb, o);
                 }
                 // the codes are in registers: their tile may be copied over
                 __syncwarp();
@@ -873,18 +902,19 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
         scales_arrived();  // nothing of this thread's is in flight when shared memory is released
     } else {
         // ---------------- epilogue: TMEM -> registers -> shared -> global ----------------
-        // A thread holds one weight row's results for the unit's tokens (one token per accumulator
-        // column).  Two sets of four warps take 32-token chunks in turn; a set puts its bf16 results
-        // into a [token][output] tile in shared memory and then writes it out a token row at a time,
-        // 16 bytes per thread.
+        // Two sets of four warps take 32-token chunks (accumulator columns) in turn.  A warp reads its
+        // quarter's lanes as 16 x 8 blocks: a thread holds rows r and r + 8 (gate and up of one feature,
+        // or two outputs), r = lane / 4, of two neighbouring tokens.  Transposing 8 x 8 stores put the
+        // bf16 results into a [token][output] tile in shared memory, which the set then writes out a
+        // token row at a time, 16 bytes per thread.  (Two tiles in turn: one is rewritten two chunks
+        // later, after every thread has passed the barrier in between.)
         const uint32_t set = (uint32_t)(warp - kFirstEpilogueWarp) >> 2;
         const uint32_t quarter = (uint32_t)(warp & 3);
-        const uint32_t m = quarter * 32u + (uint32_t)lane;
         const uint32_t te = (uint32_t)threadIdx.x - kFirstEpilogueWarp * 32u;  // 0..255
         const uint32_t t = te & 127u;                                          // within the set
-        float *xchg = reinterpret_cast<float *>(epilogueSmem + set * kXchgBytes);  // gate/up only
-        uint8_t *stageBuf = epilogueSmem + (MODE == kModeGateUp ? kEpilogueSets * kXchgBytes + set * kStageBytesGateUp
-                                                                : set * 2u * kStageBytesDown);
+        constexpr uint32_t kPitch = MODE == kModeGateUp ? kStagePitchGateUp : kStagePitchDown;
+        constexpr uint32_t kStageBytes = 32u * kPitch;
+        uint8_t *stageBuf = epilogueSmem + set * 2u * kStageBytes;
         uint32_t *rowTable = reinterpret_cast<uint32_t *>(epilogueSmem + kEpilogueSets * 2u * kStageBytesDown);  // down only
         uint32_t acc = 0, accPhase = 0, chunk = 0, unitNo = 0;
         bool ok = true;
@@ -919,89 +949,56 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
             const uint32_t taddr = tmemBase + acc * kAccCols + ((quarter * 32u) << 16);
 #pragma unroll 1
             for (uint32_t c0 = 32u * set; c0 < tile.rows; c0 += 32u * kEpilogueSets, ++chunk) {
-                uint32_t v[32];
-                tc_load_32cols(taddr + c0, v);
-                tc_wait_ld();
-                if (MODE == kModeGateUp) {
-                    // lanes 0..63 hold gate, lanes 64..127 up of features [64 nt, +64).  The gate
-                    // warps hand the second 16 tokens' gates to the up warps and take the first 16
-                    // tokens' ups from them; either side then finishes 16 tokens of its feature.
-                    // (One buffer each: the exchange rows are rewritten behind barStage, the output
-                    // tile behind the next barXchg, which every thread reaches after its last read.)
-                    const bool isUp = m >= 64u;
-                    float *mine = xchg + m * kXchgPitch;
+                const uint32_t buffer = chunk & 1u;
+                uint8_t *stage = stageBuf + buffer * kStageBytes;
+                const uint32_t tokenRow = smem_u32(stage) + (uint32_t)lane * kPitch;  // of token `lane`
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) mine[j] = __uint_as_float(isUp ? v[j] : v[16 + j]);
-                    mbar_arrive(barXchg(set));
-                    if (!mbar_wait(barXchg(set), chunk & 1u, &abortFlag)) {
-                        ok = false;
-                        break;
-                    }
-                    const float *theirs = xchg + (m ^ 64u) * kXchgPitch;
-                    // tile [32 tokens][64 features in the interleaved order], 144-byte pitch
-                    uint16_t *col = reinterpret_cast<uint16_t *>(stageBuf) + (isUp ? 16u : 0u) * (kStagePitchGateUp / 2) +
-                                    interleaved_position(m & 63u);
+                for (uint32_t h = 0; h < 2; ++h) {
+                    uint32_t v[16];
+                    tc_load_16x32(taddr + ((16u * h) << 16) + c0, v);
+                    tc_wait_ld();
+                    uint32_t p[4];
+                    if (MODE == kModeGateUp) {
 #pragma unroll
-                    for (int j = 0; j < 16; j += 2) {
-                        float act[2];
+                        for (int j = 0; j < 4; ++j) {
+                            float act[2];
 #pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            const float own = __uint_as_float(isUp ? v[16 + j + i] : v[j + i]);
-                            const float other = theirs[j + i];
-                            float g = isUp ? other : own, uu = isUp ? own : other;
-                            if (args.roundGateUp) {
-                                g = bf16_round(g);
-                                uu = bf16_round(uu);
+                            for (int i = 0; i < 2; ++i) {
+                                float g = __uint_as_float(v[4 * j + i]), up = __uint_as_float(v[4 * j + 2 + i]);
+                                if (args.roundGateUp) {
+                                    g = bf16_round(g);
+                                    up = bf16_round(up);
+                                }
+                                act[i] = gelu_tanh_fast(g) * up;
                             }
-                            act[i] = gelu_tanh_fast(g) * uu;
+                            p[j] = bf16_pair(act[0], act[1]);
                         }
-                        const uint32_t two = bf16_pair(act[0], act[1]);
-                        col[(uint32_t)j * (kStagePitchGateUp / 2)] = (uint16_t)two;
-                        col[(uint32_t)(j + 1) * (kStagePitchGateUp / 2)] = (uint16_t)(two >> 16);
-                    }
-                    mbar_arrive(barStage(set, 0));
-                    if (!mbar_wait(barStage(set, 0), chunk & 1u, &abortFlag)) {
-                        ok = false;
-                        break;
-                    }
-                    // a token row of the tile is 128 bytes: eight threads, 16 tokens per pass
-                    const uint32_t piece = t & 7u;
-                    const uint32_t col0 = nt * 64u + piece * 8u;
+                        store_blocks_transposed(tokenRow + (2u * quarter + h) * 16u, p);
+                    } else {
 #pragma unroll
-                    for (uint32_t pass = 0; pass < 2; ++pass) {
-                        const uint32_t tok = pass * 16u + (t >> 3);
-                        if (c0 + tok < tile.rows && col0 < args.N) {
-                            const uint4 val = *reinterpret_cast<const uint4 *>(stageBuf + tok * kStagePitchGateUp + piece * 16u);
-                            *reinterpret_cast<uint4 *>(args.out + (size_t)(tile.rowStart + c0 + tok) * args.N + col0) = val;
+                        for (int r = 0; r < 2; ++r) {
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                p[j] = bf16_pair(__uint_as_float(v[4 * j + 2 * r]), __uint_as_float(v[4 * j + 2 * r + 1]));
+                            store_blocks_transposed(tokenRow + (4u * quarter + 2u * h + r) * 16u, p);
                         }
                     }
-                } else {
-                    // tile [32 tokens][128 outputs], 272-byte pitch; two tiles in turn (one is rewritten
-                    // two chunks later, after every thread has passed the barrier in between)
-                    const uint32_t buffer = chunk & 1u;
-                    uint8_t *stage = stageBuf + buffer * kStageBytesDown;
-                    uint16_t *col = reinterpret_cast<uint16_t *>(stage) + m;
+                }
+                mbar_arrive(barStage(set, buffer));
+                if (!mbar_wait(barStage(set, buffer), (chunk >> 1) & 1u, &abortFlag)) {
+                    ok = false;
+                    break;
+                }
+                // a token row of the tile is 128 (gate/up) or 256 bytes: eight or sixteen threads
+                constexpr uint32_t kPieces = MODE == kModeGateUp ? 8 : 16, kTokensPerPass = 128 / kPieces;
+                const uint32_t piece = t % kPieces, tok0 = t / kPieces;
+                const uint32_t col0 = nt * (8u * kPieces) + piece * 8u;
 #pragma unroll
-                    for (int j = 0; j < 32; j += 2) {
-                        const uint32_t two = bf16_pair(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
-                        col[(uint32_t)j * (kStagePitchDown / 2)] = (uint16_t)two;
-                        col[(uint32_t)(j + 1) * (kStagePitchDown / 2)] = (uint16_t)(two >> 16);
-                    }
-                    mbar_arrive(barStage(set, buffer));
-                    if (!mbar_wait(barStage(set, buffer), (chunk >> 1) & 1u, &abortFlag)) {
-                        ok = false;
-                        break;
-                    }
-                    // a token row of the tile is 256 bytes: sixteen threads, 8 tokens per pass
-                    const uint32_t piece = t & 15u;
-                    const uint32_t col0 = nt * 128u + piece * 8u;
-#pragma unroll
-                    for (uint32_t pass = 0; pass < 4; ++pass) {
-                        const uint32_t tok = pass * 8u + (t >> 4);
-                        if (c0 + tok < tile.rows && col0 < args.N) {
-                            const uint4 val = *reinterpret_cast<const uint4 *>(stage + tok * kStagePitchDown + piece * 16u);
-                            *reinterpret_cast<uint4 *>(args.out + (size_t)rowOf[c0 + tok] * args.N + col0) = val;
-                        }
+                for (uint32_t tok = tok0; tok < 32u + tok0; tok += kTokensPerPass) {
+                    if (c0 + tok < tile.rows && col0 < args.N) {
+                        const uint4 val = *reinterpret_cast<const uint4 *>(stage + tok * kPitch + piece * 16u);
+                        const uint32_t row = MODE == kModeGateUp ? tile.rowStart + c0 + tok : rowOf[c0 + tok];
+                        *reinterpret_cast<uint4 *>(args.out + (size_t)row * args.N + col0) = val;
                     }
                 }
             }
