@@ -112,7 +112,7 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
     __shared__ uint32_t tmemBaseSlot;
     __shared__ volatile uint32_t abortFlag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rawBase = smem_u32(smemRaw), base = (rawBase + 1023u) & ~1023u;
     const uint32_t groupsK = args.K / kStepK, steps = groupsK + 3u * sum_blocks(args.K);
 
@@ -167,7 +167,7 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
     __syncthreads();
     cluster_sync_all();
     tc_fence_after();
-    const uint32_t tmemBase = tmemBaseSlot;
+    const uint32_t tmemBase = __shfl_sync(0xFFFFFFFFu, tmemBaseSlot, 0);
     pdl_enter();
 
     // A pair's unit: one token tile, two neighbouring weight-row tiles (this CTA takes 2 np + rank).
@@ -180,31 +180,33 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
+        {
             uint32_t st = 0, phase = 0;
             bool ok = true;
             for (uint32_t u = firstUnit; u < units && ok; u += unitStride) {
                 const uint32_t nt = ntOf(u);
                 const int row0 = (int)(tokenOf(u) + ctaRank * (columnsOf(u) >> 1));
                 for (uint32_t g = 0; g < steps; ++g) {
-                    if (!mbar_wait_idle(barCodeEmpty(st), phase ^ 1u, &abortFlag) ||
-                        !mbar_wait_idle(barTokEmpty(st), phase ^ 1u, &abortFlag)) {
+                    if (!mbar_wait_warp<true>(barCodeEmpty(st), phase ^ 1u, &abortFlag) ||
+                        !mbar_wait_warp<true>(barTokEmpty(st), phase ^ 1u, &abortFlag)) {
                         ok = false;
                         break;
                     }
-                    if (g < groupsK) {
-                        mbar_expect_tx(barCodeFull(st), kCodeBytes);
+                    if (elect_one()) {
+                        if (g < groupsK) {
+                            mbar_expect_tx(barCodeFull(st), kCodeBytes);
 #pragma unroll
-                        for (int q = 0; q < 2; ++q)
-                            tma_load_3d(codeAddr(st) + (uint32_t)q * (kCodeBytes / 2), MODE == kGateUp && q == 1 ? &mapW1 : &mapW0,
-                                        (int)(g * kStepK), (int)(MODE == kGateUp ? nt * 64u : nt * 128u + (uint32_t)q * 64u), 0,
-                                        barCodeFull(st));
-                    } else {
-                        mbar_arrive(barCodeFull(st));  // a bias step reads no codes
+                            for (int q = 0; q < 2; ++q)
+                                tma_load_3d(codeAddr(st) + (uint32_t)q * (kCodeBytes / 2), MODE == kGateUp && q == 1 ? &mapW1 : &mapW0,
+                                            (int)(g * kStepK), (int)(MODE == kGateUp ? nt * 64u : nt * 128u + (uint32_t)q * 64u), 0,
+                                            barCodeFull(st));
+                        } else {
+                            mbar_arrive(barCodeFull(st));  // a bias step reads no codes
+                        }
+                        mbar_expect_tx(barTokFull(st), kTokBytes);
+                        if (g < groupsK) tma_load_2d(tokAddr(st), &mapTok, (int)(g * kStepK), row0, barTokFull(st));
+                        else tma_load_2d(tokAddr(st), &mapSums, (int)((g - groupsK) * kStepK), row0, barTokFull(st));
                     }
-                    mbar_expect_tx(barTokFull(st), kTokBytes);
-                    if (g < groupsK) tma_load_2d(tokAddr(st), &mapTok, (int)(g * kStepK), row0, barTokFull(st));
-                    else tma_load_2d(tokAddr(st), &mapSums, (int)((g - groupsK) * kStepK), row0, barTokFull(st));
                     if (++st == kStages) {
                         st = 0;
                         phase ^= 1u;
@@ -214,26 +216,30 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (leader CTA only) ----------------
-        if (lane == 0 && leader) {
+        // (the whole warp runs the loop and one elected lane issues: inside a `lane == 0` branch every
+        // operand would go to the uniform registers by a loop over the active lanes)
+        if (leader) {
             uint32_t st = 0, op = 0, opPhase = 0, acc = 0, accPhase = 0;
             bool ok = true;
             for (uint32_t u = firstUnit; u < units && ok; u += unitStride) {
                 const uint32_t idesc = umma_idesc_bf16_m256(columnsOf(u));
                 for (uint32_t g = 0; g < steps; ++g) {
                     // (the warps that arrive on the operand have also seen both token halves land)
-                    if (!mbar_wait_cluster<false>(barOperand(op), opPhase, &abortFlag) ||
-                        !mbar_wait_cluster<false>(barAccEmpty(acc), accPhase ^ 1u, &abortFlag)) {
+                    if (!mbar_wait_warp<false>(barOperand(op), opPhase, &abortFlag) ||
+                        !mbar_wait_warp<false>(barAccEmpty(acc), accPhase ^ 1u, &abortFlag)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
                     const uint64_t descTok = umma_desc_sw128(tokAddr(st));
                     const uint32_t tmemW = tmemBase + kOperandCol + op * 32u, tmemD = tmemBase + acc * kMaxRows;
+                    if (elect_one()) {
 #pragma unroll
-                    for (uint32_t kk = 0; kk < kStepK / 16; ++kk)
-                        tc_mma_bf16_a_tmem(tmemD, tmemW + 8u * kk, descTok + 2u * kk, idesc, kk ? 1u : 0u);
-                    tc_commit_pair(barTokEmpty(st));  // the token stage and the operand stage are free
-                    tc_commit_pair(barAccFull(acc));
+                        for (uint32_t kk = 0; kk < kStepK / 16; ++kk)
+                            tc_mma_bf16_a_tmem(tmemD, tmemW + 8u * kk, descTok + 2u * kk, idesc, kk ? 1u : 0u);
+                        tc_commit_pair(barTokEmpty(st));  // the token stage and the operand stage are free
+                        tc_commit_pair(barAccFull(acc));
+                    }
                     if (++st == kStages) st = 0;
                     if (++op == kOperandStages) {
                         op = 0;
