@@ -286,12 +286,11 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
                                  : "r"(src + ((c ^ flip) << 4)));
 #pragma unroll
                     for (uint32_t i = 0; i < 8; ++i) {
-                        // codes 2j, 2j+1 as floats (2^23 + q, minus 2^23); a bf16 holds them exactly
-                        uint32_t n0, n1;
-                        asm("prmt.b32 %0, %1, %2, %3;" : "=r"(n0) : "r"(w[i >> 1]), "r"(0x4B000000u), "r"(0x7440u | ((2u * i) & 3u)));
-                        asm("prmt.b32 %0, %1, %2, %3;" : "=r"(n1) : "r"(w[i >> 1]), "r"(0x4B000000u), "r"(0x7440u | ((2u * i + 1u) & 3u)));
-                        o[8 * c + i] = __byte_perm(__float_as_uint(__uint_as_float(n0) - 8388608.0f),
-                                                   __float_as_uint(__uint_as_float(n1) - 8388608.0f), 0x7632);
+                        // Two codes as 16-bit numbers ARE a pair of bf16: q * 2^-133, subnormal up to 127.
+                        // Times 2^126 they are the operand q / 128, exactly (the drain's scale makes up for
+                        // the 128): two instructions for two codes, five by way of floats.
+                        const uint32_t pair = __byte_perm(w[i >> 1], 0u, (i & 1u) ? 0x4342u : 0x4140u);
+                        asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(o[8 * c + i]) : "r"(pair), "r"(0x7E807E80u));
                     }
                 }
             } else {
@@ -366,7 +365,7 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
 #pragma unroll
             for (int j = 0; j < 64; ++j) sum[j] = 0.0f;
             for (uint32_t g = 0; g < steps; ++g) {
-                const float s = g < groupsK ? bf2f(myScale[g]) : 1.0f;
+                const float s = g < groupsK ? 128.0f * bf2f(myScale[g]) : 1.0f;  // (the codes come as q / 128)
                 if (!mbar_wait(barAccFull(accNo), accPhase, &abortFlag)) {
                     ok = false;
                     break;
