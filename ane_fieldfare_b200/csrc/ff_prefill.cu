@@ -579,7 +579,7 @@ __device__ __forceinline__ void dequantize_words(const uint32_t (&w)[8], uint32_
 
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
-k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ CUtensorMap mapW0,
+k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ CUtensorMap mapTok16, const __grid_constant__ CUtensorMap mapW0,
                     const __grid_constant__ CUtensorMap mapW1, const GemmArgs args) {
     extern __shared__ uint8_t gemmSmemRaw[];
     __shared__ uint64_t barriers[2 * kTokStages + 2 * kPackStages + kWStages + 4 + 2 * kEpilogueSets + 1];
@@ -677,26 +677,35 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
 
     if (warp == 0) {
         // ---------------- token copies ----------------
-        if (lane == 0 && firstUnit < units) {
+        // A full tile's half is one copy; of a smaller one only the rows that its columns need come, 16
+        // at a time (whole halves of 96 rows were three quarters of all that the SMs read where an
+        // expert has a handful of rows).
+        if (firstUnit < units) {
             uint32_t ts = 0, phase = 0;
             bool ok = true;
             RowTile next = tileOf(firstUnit);
             for (uint32_t u = firstUnit; u < units && ok; u += unitStride) {
                 const RowTile tile = next;
                 next = tileOf(u + unitStride);
-                // this CTA's half of the tile's rows
-                const int row0 = (int)(tile.rowStart + ctaRank * (columnsOf(tile) >> 1));
+                const uint32_t half = columnsOf(tile) >> 1;  // this CTA's half of the tile's rows
+                const int row0 = (int)(tile.rowStart + ctaRank * half);
                 for (uint32_t g = 0; g < groupsK; ++g) {
-                    if (!mbar_wait_idle(barTokEmpty(ts), phase ^ 1u, &abortFlag)) {
+                    if (!mbar_wait_warp<true>(barTokEmpty(ts), phase ^ 1u, &abortFlag)) {
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(barTokFull(ts), kTokTileBytes);
-                    tma_load_2d(tokAddrOf(ts), &mapTok, (int)(g * kTileK), row0, barTokFull(ts));
-                    if (++ts == kTokStages) {
-                        ts = 0;
-                        phase ^= 1u;
+                    if (elect_one()) {
+                        mbar_expect_tx(barTokFull(ts), half * (kTileK * 2));
+                        if (half == kTokHalfRows) {
+                            tma_load_2d(tokAddrOf(ts), &mapTok, (int)(g * kTileK), row0, barTokFull(ts));
+                        } else {
+#pragma unroll 1
+                            for (uint32_t r = 0; r < half; r += 16)
+                                tma_load_2d(tokAddrOf(ts) + r * (kTileK * 2), &mapTok16, (int)(g * kTileK), row0 + (int)r, barTokFull(ts));
+                        }
                     }
+                    ts = (ts + 1u) % kTokStages;
+                    if (ts == 0) phase ^= 1u;
                 }
             }
         }
@@ -1038,12 +1047,12 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
 // bf16 activations [rows][k] (row pitch `strideElems`), box 64 x kTokHalfRows (the half of a row
 // tile that one CTA of a pair holds), 128-byte swizzle.
 static bool make_activation_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t k,
-                                uint64_t strideElems, const char **error) {
+                                uint64_t strideElems, uint32_t boxRows, const char **error) {
     EncodeTiledFn fn = encode_tiled(error);
     if (!fn) return false;
     cuuint64_t dims[2] = {k, rows};
     cuuint64_t strides[1] = {strideElems * 2};
-    cuuint32_t box[2] = {(cuuint32_t)kTileK, (cuuint32_t)kTokHalfRows};
+    cuuint32_t box[2] = {(cuuint32_t)kTileK, boxRows};
     cuuint32_t elem[2] = {1, 1};
     CUresult rc = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides,
                      box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -1141,10 +1150,15 @@ static size_t gemm_smem_bytes(int mode, uint32_t K, uint32_t buffers) {
            (mode == kModeGateUp ? kEpilogueBytesGateUp : kEpilogueBytesDown) + buffers * quads * kScaleSlotBytes;
 }
 
+// `rows` activation rows of args.K elements at `x`
 template <int MODE>
-static bool launch_gemm(FFContext *ctx, const CUtensorMap &mapA, const CUtensorMap &mapW0,
+static bool launch_gemm(FFContext *ctx, const uint16_t *x, uint64_t rows, const CUtensorMap &mapW0,
                         const CUtensorMap &mapW1, GemmArgs args, uint32_t maxUnits,
                         cudaStream_t stream, const char **error) {
+    CUtensorMap mapA, mapA16;
+    if (!make_activation_map(&mapA, x, rows, args.K, args.K, kTokHalfRows, error) ||
+        !make_activation_map(&mapA16, x, rows, args.K, args.K, 16, error))
+        return false;
     auto kernel = k_grouped_int4_gemm<MODE>;
     // scale words one unit ahead where they fit, else the unit's own, else none (read step by step)
     args.scaleBuffers = 2;
@@ -1158,7 +1172,7 @@ static bool launch_gemm(FFContext *ctx, const CUtensorMap &mapA, const CUtensorM
     {
         LaunchScope scope(ctx, stream, MODE == kModeGateUp ? "int4_gemm_gate_up_act" : "int4_gemm_down");
         FF_CUDA_OK(launch_pdl(kernel, grid, kGemmThreads, smem, stream,
-                              mapA, mapW0, mapW1, args),
+                              mapA, mapA16, mapW0, mapW1, args),
                    error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
@@ -1214,10 +1228,7 @@ bool launch_prefill_routed(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     FF_CUDA_OK(cudaGetLastError(), error);
 
     const uint32_t tileBound = pairs / kRowTile + (uint32_t)E;
-    CUtensorMap mapX, mapActs;
-    if (!make_activation_map(&mapX, ctx->xSorted, (uint64_t)pairs + 256, c.d, c.d, error)) return false;
-    if (!make_activation_map(&mapActs, ctx->acts, (uint64_t)pairs + 256, c.f, c.f, error)) return false;
-
+    const uint64_t rows = (uint64_t)pairs + 256;
     GemmArgs a{};
     a.scaleWords = L.routedScales;
     a.scaleStride = scale_words(c.d, c.f);
@@ -1231,7 +1242,7 @@ bool launch_prefill_routed(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     a.topK = c.topK;
     a.roundGateUp = 0;
     a.errorFlag = ctx->errorFlag;
-    if (!launch_gemm<kModeGateUp>(ctx, mapX, L.routedMap[0], L.routedMap[1], a, tileBound * a.nTiles,
+    if (!launch_gemm<kModeGateUp>(ctx, ctx->xSorted, rows, L.routedMap[0], L.routedMap[1], a, tileBound * a.nTiles,
                                   stream, error))
         return false;
 
@@ -1242,7 +1253,7 @@ bool launch_prefill_routed(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     b.nTiles = (c.d + 127) / 128;
     b.out = partials;
     b.pairs = ctx->sortedPairs;
-    return launch_gemm<kModeDown>(ctx, mapActs, L.routedMap[2], L.routedMap[2], b, tileBound * b.nTiles,
+    return launch_gemm<kModeDown>(ctx, ctx->acts, rows, L.routedMap[2], L.routedMap[2], b, tileBound * b.nTiles,
                                   stream, error);
 }
 
@@ -1310,10 +1321,7 @@ bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     }
     FF_CUDA_OK(cudaGetLastError(), error);
     const uint32_t rowTiles = (tokens + kRowTile - 1) / kRowTile;
-    CUtensorMap mapX, mapActs;
-    if (!make_activation_map(&mapX, ctx->xSorted, (uint64_t)tokens + 256, c.d, c.d, error)) return false;
-    if (!make_activation_map(&mapActs, ctx->sharedActs, (uint64_t)tokens + 256, c.sharedF, c.sharedF, error))
-        return false;
+    const uint64_t rows = (uint64_t)tokens + 256;
     GemmArgs a{};
     a.scaleWords = L.sharedScales;
     a.K = c.d;
@@ -1325,7 +1333,7 @@ bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     a.topK = c.topK;
     a.roundGateUp = 1;
     a.errorFlag = ctx->errorFlag;
-    if (!launch_gemm<kModeGateUp>(ctx, mapX, L.sharedMap[0], L.sharedMap[1], a, rowTiles * a.nTiles, stream,
+    if (!launch_gemm<kModeGateUp>(ctx, ctx->xSorted, rows, L.sharedMap[0], L.sharedMap[1], a, rowTiles * a.nTiles, stream,
                                   error))
         return false;
     GemmArgs b = a;
@@ -1335,7 +1343,7 @@ bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     b.nTiles = (c.d + 127) / 128;
     b.out = y;
     b.pairs = nullptr;
-    return launch_gemm<kModeDown>(ctx, mapActs, L.sharedMap[2], L.sharedMap[2], b, rowTiles * b.nTiles,
+    return launch_gemm<kModeDown>(ctx, ctx->sharedActs, rows, L.sharedMap[2], L.sharedMap[2], b, rowTiles * b.nTiles,
                                   stream, error);
 }
 
