@@ -84,12 +84,15 @@ void ff_destroy(FFContext *ctx) {
     cudaDeviceSynchronize();
     for (auto &L : ctx->layers) free_layer(L);
     void *ptrs[] = {ctx->logits, ctx->ids, ctx->weights, ctx->plan, ctx->routerCounts, ctx->acts, ctx->sharedActs, ctx->h1,
-                    ctx->partials, ctx->xDev, ctx->yDev, ctx->xSorted, ctx->sortedPairs,
+                    ctx->partials, ctx->xDev, ctx->yDev, ctx->xSorted, ctx->xShared, ctx->sortedPairs,
                     ctx->expertOffsets, ctx->blockCounts, ctx->units, ctx->unitCount,
                     ctx->errorFlag, ctx->gridBarrier, ctx->phaseStamps, ctx->mapScratch, ctx->taggedLogits, ctx->taggedActs,
                     ctx->logitsRows, ctx->routeIds, ctx->routeWeights, ctx->xSums, ctx->actSums, ctx->routerParts};
     for (void *p : ptrs) cudaFree(p);
     if (ctx->hostStream) cudaStreamDestroy(ctx->hostStream);
+    if (ctx->sideStream) cudaStreamDestroy(ctx->sideStream);
+    if (ctx->forked) cudaEventDestroy(ctx->forked);
+    if (ctx->joined) cudaEventDestroy(ctx->joined);
     if (ctx->mailbox) cudaFreeHost(const_cast<unsigned long long *>(ctx->mailbox));
     delete ctx;
 }
@@ -182,6 +185,15 @@ FFContext *ff_create(int32_t deviceOrdinal, const FFConfig *config, const char *
         ctx->maxUnits = (uint32_t)(2 * (pairs / 128 + c.experts + 2));  // row tiles: routed half, dense half
         ok = ok && dev_alloc(ctx, &ctx->xSorted, (pairs + 256) * c.d, error);
         if (ok) ok = cudaMemset(ctx->xSorted, 0, (pairs + 256) * c.d * 2) == cudaSuccess;
+        if (c.sharedF) {
+            ok = ok && dev_alloc(ctx, &ctx->xShared, (T + 256) * c.d, error);
+            if (ok) ok = cudaMemset(ctx->xShared, 0, (T + 256) * c.d * 2) == cudaSuccess;
+            int least = 0, greatest = 0;
+            if (ok) ok = cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess;
+            if (ok) ok = cudaStreamCreateWithPriority(&ctx->sideStream, cudaStreamNonBlocking, least) == cudaSuccess;
+            if (ok) ok = cudaEventCreateWithFlags(&ctx->forked, cudaEventDisableTiming) == cudaSuccess;
+            if (ok) ok = cudaEventCreateWithFlags(&ctx->joined, cudaEventDisableTiming) == cudaSuccess;
+        }
         ok = ok && dev_alloc(ctx, &ctx->sortedPairs, pairs, error);
         ok = ok && dev_alloc(ctx, &ctx->expertOffsets, c.experts + 1, error);
         ok = ok && dev_alloc(ctx, &ctx->blockCounts, (permuteBlocks + 1) * c.experts, error);

@@ -172,6 +172,11 @@ struct FFContext {
 
     // prefill scratch (allocated when maxTokens > 16)
     uint16_t *xSorted = nullptr;            // [maxTokens*topK][d] rows in expert order
+    uint16_t *xShared = nullptr;            // [maxTokens][d] rows for the shared FFN's GEMM
+    // The shared FFN of a prefill block runs on a stream of its own beside the router and the sort, whose
+    // kernels leave most SMs idle: forked off and joined within the call.
+    cudaStream_t sideStream = nullptr;
+    cudaEvent_t forked = nullptr, joined = nullptr;
     FFTokenExpertPair *sortedPairs = nullptr;
     uint32_t *expertOffsets = nullptr;      // [experts+1]
     uint32_t *blockCounts = nullptr;        // permute: [blocks][experts]

@@ -490,6 +490,7 @@ constexpr int kCodeWarp = kFirstEpilogueWarp + 4 * kEpilogueSets;
 constexpr int kGemmThreads = (kCodeWarp + 1) * 32;
 constexpr int kEpilogueThreads = 128 * kEpilogueSets;
 constexpr uint32_t kTokHalfRows = kRowTile / 2;                   // rows of a token tile held by either CTA of a pair
+constexpr uint32_t kTokSmallRows = 32;                            // of those, copied for a small tile
 constexpr uint32_t kTokTileBytes = kTokHalfRows * kTileK * 2;     // 12288 (a multiple of the 1024-byte swizzle atom)
 constexpr uint32_t kPackTileBytes = kWeightRows * kTileK / 2 * kQuad;  // 16384: two [64 rows x 128 bytes] boxes
 constexpr uint32_t kTmemCols = 512;
@@ -579,7 +580,7 @@ __device__ __forceinline__ void dequantize_words(const uint32_t (&w)[8], uint32_
 
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
-k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ CUtensorMap mapTok16, const __grid_constant__ CUtensorMap mapW0,
+k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ CUtensorMap mapTokSmall, const __grid_constant__ CUtensorMap mapW0,
                     const __grid_constant__ CUtensorMap mapW1, const GemmArgs args) {
     extern __shared__ uint8_t gemmSmemRaw[];
     __shared__ uint64_t barriers[2 * kTokStages + 2 * kPackStages + kWStages + 4 + 2 * kEpilogueSets + 1];
@@ -677,9 +678,9 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
 
     if (warp == 0) {
         // ---------------- token copies ----------------
-        // A full tile's half is one copy; of a smaller one only the rows that its columns need come, 16
-        // at a time (whole halves of 96 rows were three quarters of all that the SMs read where an
-        // expert has a handful of rows).
+        // A step is one copy, of 32 rows where the tile's half needs no more and of 96 otherwise.  (16 rows
+        // at a time, as many as needed, were slower than 96 always: 353 us against 339 with 77 tokens.
+        // It is the copies, not their bytes, that cost.)
         if (firstUnit < units) {
             uint32_t ts = 0, phase = 0;
             bool ok = true;
@@ -689,20 +690,16 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
                 next = tileOf(u + unitStride);
                 const uint32_t half = columnsOf(tile) >> 1;  // this CTA's half of the tile's rows
                 const int row0 = (int)(tile.rowStart + ctaRank * half);
+                const CUtensorMap *map = half <= kTokSmallRows ? &mapTokSmall : &mapTok;
+                const uint32_t bytes = (half <= kTokSmallRows ? kTokSmallRows : kTokHalfRows) * kTileK * 2;
                 for (uint32_t g = 0; g < groupsK; ++g) {
                     if (!mbar_wait_warp<true>(barTokEmpty(ts), phase ^ 1u, &abortFlag)) {
                         ok = false;
                         break;
                     }
                     if (elect_one()) {
-                        mbar_expect_tx(barTokFull(ts), half * (kTileK * 2));
-                        if (half == kTokHalfRows) {
-                            tma_load_2d(tokAddrOf(ts), &mapTok, (int)(g * kTileK), row0, barTokFull(ts));
-                        } else {
-#pragma unroll 1
-                            for (uint32_t r = 0; r < half; r += 16)
-                                tma_load_2d(tokAddrOf(ts) + r * (kTileK * 2), &mapTok16, (int)(g * kTileK), row0 + (int)r, barTokFull(ts));
-                        }
+                        mbar_expect_tx(barTokFull(ts), bytes);
+                        tma_load_2d(tokAddrOf(ts), map, (int)(g * kTileK), row0, barTokFull(ts));
                     }
                     ts = (ts + 1u) % kTokStages;
                     if (ts == 0) phase ^= 1u;
@@ -1155,9 +1152,9 @@ template <int MODE>
 static bool launch_gemm(FFContext *ctx, const uint16_t *x, uint64_t rows, const CUtensorMap &mapW0,
                         const CUtensorMap &mapW1, GemmArgs args, uint32_t maxUnits,
                         cudaStream_t stream, const char **error) {
-    CUtensorMap mapA, mapA16;
+    CUtensorMap mapA, mapASmall;
     if (!make_activation_map(&mapA, x, rows, args.K, args.K, kTokHalfRows, error) ||
-        !make_activation_map(&mapA16, x, rows, args.K, args.K, 16, error))
+        !make_activation_map(&mapASmall, x, rows, args.K, args.K, kTokSmallRows, error))
         return false;
     auto kernel = k_grouped_int4_gemm<MODE>;
     // scale words one unit ahead where they fit, else the unit's own, else none (read step by step)
@@ -1172,7 +1169,7 @@ static bool launch_gemm(FFContext *ctx, const uint16_t *x, uint64_t rows, const 
     {
         LaunchScope scope(ctx, stream, MODE == kModeGateUp ? "int4_gemm_gate_up_act" : "int4_gemm_down");
         FF_CUDA_OK(launch_pdl(kernel, grid, kGemmThreads, smem, stream,
-                              mapA, mapA16, mapW0, mapW1, args),
+                              mapA, mapASmall, mapW0, mapW1, args),
                    error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
@@ -1300,7 +1297,7 @@ bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
                            uint32_t tokens, uint16_t *y, cudaStream_t stream, const char **error) {
     const FFConfig &c = ctx->cfg;
     if (tokens == 0) return true;
-    if (!ctx->xSorted) return fail(error, "context was created with maxTokens <= 16: no prefill scratch");
+    if (!ctx->xShared) return fail(error, "context was created with maxTokens <= 16: no prefill scratch");
     if (!L.shared) return fail(error, "layer has no resident shared FFN");
     if (!check_gemm_shapes(c, c.sharedF, error) || !prefill_prepare_layer(ctx, L, error)) return false;
     // dense problem: its row tiles live behind the routed ones in the units buffer
@@ -1316,7 +1313,7 @@ bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
         LaunchScope scope(ctx, stream, "gather_rows");
         FF_CUDA_OK(launch_pdl(k_gather_rows, ctx->smCount * 8, 256, 0, stream,
                               x, xStride, nullptr, nullptr, tokens,
-                                                            (int)c.d, ctx->xSorted),
+                                                            (int)c.d, ctx->xShared),
                    error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
@@ -1333,7 +1330,7 @@ bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     a.topK = c.topK;
     a.roundGateUp = 1;
     a.errorFlag = ctx->errorFlag;
-    if (!launch_gemm<kModeGateUp>(ctx, ctx->xSorted, rows, L.sharedMap[0], L.sharedMap[1], a, rowTiles * a.nTiles, stream,
+    if (!launch_gemm<kModeGateUp>(ctx, ctx->xShared, rows, L.sharedMap[0], L.sharedMap[1], a, rowTiles * a.nTiles, stream,
                                   error))
         return false;
     GemmArgs b = a;
