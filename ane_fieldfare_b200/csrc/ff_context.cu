@@ -84,7 +84,7 @@ void ff_destroy(FFContext *ctx) {
     cudaDeviceSynchronize();
     for (auto &L : ctx->layers) free_layer(L);
     void *ptrs[] = {ctx->logits, ctx->ids, ctx->weights, ctx->plan, ctx->routerCounts, ctx->acts, ctx->sharedActs, ctx->h1,
-                    ctx->partials, ctx->xDev, ctx->yDev, ctx->xSorted, ctx->xShared, ctx->sortedPairs,
+                    ctx->partials, ctx->xDev, ctx->yDev, ctx->xSorted, ctx->xShared, ctx->rowOfRoute, ctx->sortedPairs,
                     ctx->expertOffsets, ctx->blockCounts, ctx->units, ctx->unitCount,
                     ctx->errorFlag, ctx->gridBarrier, ctx->phaseStamps, ctx->mapScratch, ctx->taggedLogits, ctx->taggedActs,
                     ctx->logitsRows, ctx->routeIds, ctx->routeWeights, ctx->xSums, ctx->actSums, ctx->routerParts};
@@ -195,6 +195,7 @@ FFContext *ff_create(int32_t deviceOrdinal, const FFConfig *config, const char *
             if (ok) ok = cudaEventCreateWithFlags(&ctx->joined, cudaEventDisableTiming) == cudaSuccess;
         }
         ok = ok && dev_alloc(ctx, &ctx->sortedPairs, pairs, error);
+        ok = ok && dev_alloc(ctx, &ctx->rowOfRoute, pairs, error);
         ok = ok && dev_alloc(ctx, &ctx->expertOffsets, c.experts + 1, error);
         ok = ok && dev_alloc(ctx, &ctx->blockCounts, (permuteBlocks + 1) * c.experts, error);
         ok = ok && dev_alloc(ctx, &ctx->units, (size_t)ctx->maxUnits * 4, error);

@@ -172,6 +172,7 @@ struct FFContext {
 
     // prefill scratch (allocated when maxTokens > 16)
     uint16_t *xSorted = nullptr;            // [maxTokens*topK][d] rows in expert order
+    uint32_t *rowOfRoute = nullptr;         // [maxTokens*topK] row of a token's route in that order
     uint16_t *xShared = nullptr;            // [maxTokens][d] rows for the shared FFN's GEMM
     // The shared FFN of a prefill block runs on a stream of its own beside the router and the sort, whose
     // kernels leave most SMs idle: forked off and joined within the call.

@@ -385,10 +385,11 @@ k_route_scan(uint32_t *blockCounts, int blocks, int E, uint32_t *expertOffsets, 
 // Pass 3: every route's position in (expert, token, rank) order; writes the sorted pair list.
 // Position = expert offset + routes to the expert in earlier blocks + in earlier warp segments of
 // this block + earlier in this warp's segment (earlier 32-route batches, then lower lanes).
+constexpr uint32_t kNoRow = 0xFFFFFFFFu;  // of a route to no expert
 __global__ void __launch_bounds__(256)
 k_route_scatter(const uint32_t *ids, const uint16_t *weights, int T, int K, int E,
                 const uint32_t *blockCounts, const uint32_t *expertOffsets,
-                FFTokenExpertPair *sorted) {
+                FFTokenExpertPair *sorted, uint32_t *rowOfRoute) {
     pdl_enter();
     extern __shared__ uint32_t sRoutes[];
     __shared__ uint32_t segCount[8 * kMaxExperts];
@@ -429,6 +430,7 @@ k_route_scatter(const uint32_t *ids, const uint16_t *weights, int T, int K, int 
             const uint32_t wbits = weights ? (uint32_t)weights[(size_t)token * K + rank] : 0u;
             sorted[pos] = FFTokenExpertPair{token, ex, rank, wbits};
         }
+        if (rowOfRoute && valid) rowOfRoute[(size_t)t0 * K + i] = live ? pos : kNoRow;
     }
 }
 
@@ -447,28 +449,35 @@ __global__ void k_dense_tiles(int T, RowTile *tiles, uint32_t *counts) {
 }
 
 // Copies rows of x into the GEMM's activation buffer, reordering every aligned run of eight
-// elements to 0,4,1,5,2,6,3,7.  pairs == null: row r of the output is row r of x; otherwise row r
-// is the token of sorted pair r.  One thread per 16 bytes.
+// elements to 0,4,1,5,2,6,3,7: row t to row t (K = 0), or to the rows of its K routes.  One thread per
+// 16 bytes read; bound by the writes.  (Going through the sorted rows instead reads every token K times, from
+// memory where the rows exceed the L2: the block of 32768 tokens and eight routes took 160 us more.)
 __global__ void __launch_bounds__(256)
-k_gather_rows(const uint16_t *x, uint32_t xStride, const FFTokenExpertPair *pairs,
-              const uint32_t *rowCountPtr, uint32_t rowCount, int D, uint16_t *out) {
+k_gather_rows(const uint16_t *x, uint32_t xStride, uint32_t rows, const uint32_t *rowOfRoute, int K, int D, uint16_t *out) {
     pdl_enter();
-    const uint32_t rows = rowCountPtr ? rowCountPtr[1] : rowCount;
     const int chunksPerRow = D / 8;
     const size_t total = (size_t)rows * chunksPerRow;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (size_t)gridDim.x * blockDim.x) {
         const uint32_t r = (uint32_t)(i / chunksPerRow);
         const int c = (int)(i - (size_t)r * chunksPerRow);
-        const uint32_t src = pairs ? pairs[r].token : r;
-        const uint4 v = *reinterpret_cast<const uint4 *>(x + (size_t)src * xStride + c * 8);
+        const uint4 v = *reinterpret_cast<const uint4 *>(x + (size_t)r * xStride + c * 8);
         // halves h0..h7 -> h0,h4,h1,h5,h2,h6,h3,h7
         uint4 o;
         o.x = __byte_perm(v.x, v.z, 0x5410);
         o.y = __byte_perm(v.x, v.z, 0x7632);
         o.z = __byte_perm(v.y, v.w, 0x5410);
         o.w = __byte_perm(v.y, v.w, 0x7632);
-        *reinterpret_cast<uint4 *>(out + (size_t)r * D + c * 8) = o;
+        if (K == 0) {
+            *reinterpret_cast<uint4 *>(out + (size_t)r * D + c * 8) = o;
+        } else {
+            const uint32_t *routes = rowOfRoute + (size_t)r * K;
+#pragma unroll 8
+            for (int k = 0; k < K; ++k) {
+                const uint32_t row = __ldg(routes + k);
+                if (row != kNoRow) *reinterpret_cast<uint4 *>(out + (size_t)row * D + c * 8) = o;
+            }
+        }
     }
 }
 
@@ -1211,15 +1220,14 @@ bool launch_prefill_routed(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
         LaunchScope scope(ctx, stream, "route_scatter");
         FF_CUDA_OK(launch_pdl(k_route_scatter, blocks, 256, sortSmem, stream,
                               ids, nullptr, T, K, E, ctx->blockCounts,
-                                                           ctx->expertOffsets, ctx->sortedPairs),
+                              ctx->expertOffsets, ctx->sortedPairs, ctx->rowOfRoute),
                    error);
     }
     const uint32_t pairs = tokens * c.topK;
     {
         LaunchScope scope(ctx, stream, "gather_rows");
         FF_CUDA_OK(launch_pdl(k_gather_rows, ctx->smCount * 8, 256, 0, stream,
-                              x, xStride, ctx->sortedPairs, nullptr, pairs,
-                                                            (int)c.d, ctx->xSorted),
+                              x, xStride, tokens, ctx->rowOfRoute, K, (int)c.d, ctx->xSorted),
                    error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
@@ -1286,7 +1294,7 @@ bool launch_route_sort(FFContext *ctx, const uint32_t *groupIds, uint32_t tokens
         LaunchScope scope(ctx, stream, "route_scatter");
         FF_CUDA_OK(launch_pdl(k_route_scatter, blocks, 256, sortSmem, stream,
                               groupIds, nullptr, T, K, E, ctx->blockCounts, offsets,
-                                                           sortedPairs),
+                              sortedPairs, nullptr),
                    error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
@@ -1312,8 +1320,7 @@ bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     {
         LaunchScope scope(ctx, stream, "gather_rows");
         FF_CUDA_OK(launch_pdl(k_gather_rows, ctx->smCount * 8, 256, 0, stream,
-                              x, xStride, nullptr, nullptr, tokens,
-                                                            (int)c.d, ctx->xShared),
+                              x, xStride, tokens, nullptr, 0, (int)c.d, ctx->xShared),
                    error);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
