@@ -1,6 +1,6 @@
-// Bandwidth kernels of the INT4 MoE block for 1..16 token rows: router, top-K + route plan,
-// grouped INT4 GEMV (gate/up/GeGLU and down), decode combine, token-major reduce, RMSNorm and
-// the dequantization probe.
+// Bandwidth kernels of the INT4 MoE block: router rows, INT4 GEMV of one matrix or a gate/up pair for
+// 1..16 token rows, decode combine, token-major reduce, RMSNorm and the fused steps either side of the
+// block, and the dequantization probe.
 //
 // GEMV scheme (every matrix, every row count): a weight row of `cols` 4-bit codes is cut into
 // 16-byte chunks of 32 codes.  Eight lanes share a row; lane j takes chunks j, j+8, j+16, ...
@@ -23,20 +23,15 @@
 
 namespace ff {
 
-template <int NT, bool DUAL, bool STAGE_ALL>
+template <int NT, bool DUAL>
 __device__ __forceinline__ void run_item(const GemvJob &job, int row0, const float *xs,
                                          const float *xsum) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row = row0 + warp * 4 + (lane >> 3);
     const bool live = row < (int)job.rows;
-    // staged row each input reads: with all rows of the block staged once, the job's own row
-    // numbers; otherwise the job's rows were staged compactly in order
-    int sel[NT];
+    int sel[NT];  // staged row each input reads
 #pragma unroll
-    for (int t = 0; t < NT; ++t) {
-        const int tt = t < (int)job.n ? t : 0;
-        sel[t] = STAGE_ALL ? (int)job.inRow[tt] : tt;
-    }
+    for (int t = 0; t < NT; ++t) sel[t] = t < (int)job.n ? t : 0;
     float a0[NT], a1[NT];
     row_dot<NT, DUAL>(job.w0, job.s0, job.b0, job.w1, job.s1, job.b1, row, (int)job.cols, live, xs,
                       xsum, sel, a0, a1);
@@ -59,62 +54,31 @@ __device__ __forceinline__ void run_item(const GemvJob &job, int row0, const flo
     }
 }
 
-// Persistent grouped GEMV over (job, row block) items.  With `jobs` null the single `inlineJob`
-// is used.  STAGE_ALL: every job reads rows of one input block (`allRows` x `allCols`), which is
-// staged once per CTA and items are dealt round robin; otherwise a job's input rows are staged
-// when a CTA meets the job, and items are dealt in chunks of two so that a staging is shared.
-template <int MAXNT, bool DUAL, bool STAGE_ALL>
-__global__ void __launch_bounds__(kGemvThreads)
-k_int4_gemv(const GemvJob *jobs, const uint32_t *items, const uint32_t *itemCountPtr,
-            GemvJob inlineJob, uint32_t inlineItems, uint32_t maxCols, const uint16_t *allIn,
-            uint32_t allStride, uint32_t allRows) {
+// Persistent GEMV over a job's row blocks: its input rows are staged once per CTA.
+template <int MAXNT, bool DUAL>
+__global__ void __launch_bounds__(kGemvThreads) k_int4_gemv(const __grid_constant__ GemvJob job, uint32_t blocks) {
     extern __shared__ float smem[];
     __shared__ GemvJob sjob;
-    __shared__ uint32_t sAllRows[kMaxGemvRows];
     float *xs = smem;
-    const int stagedRows = STAGE_ALL ? (int)allRows : MAXNT;
-    float *xsum = smem + stagedRows * staged_stride((int)maxCols);
-    const uint32_t nItems = jobs ? *itemCountPtr : inlineItems;
-    if (STAGE_ALL) {
-        if (threadIdx.x < kMaxGemvRows) sAllRows[threadIdx.x] = threadIdx.x;
-        __syncthreads();
-        stage_rows(allIn, allStride, sAllRows, (int)allRows, (int)maxCols, xs, xsum);
-    }
-    constexpr uint32_t kItemChunk = STAGE_ALL ? 1 : 2;
-    const uint32_t nChunks = (nItems + kItemChunk - 1) / kItemChunk;
-    int current = -1;
-    for (uint32_t chunk = blockIdx.x; chunk < nChunks; chunk += gridDim.x)
-    for (uint32_t it = chunk * kItemChunk; it < min(nItems, (chunk + 1) * kItemChunk); ++it) {
-        uint32_t jobIdx = 0, block = it;
-        if (jobs) {
-            const uint32_t packed = items[it];
-            jobIdx = packed >> 16;
-            block = packed & 0xFFFFu;
-        }
-        if ((int)jobIdx != current) {
-            __syncthreads();
-            const uint32_t *src =
-                reinterpret_cast<const uint32_t *>(jobs ? jobs + jobIdx : &inlineJob);
-            uint32_t *dst = reinterpret_cast<uint32_t *>(&sjob);
-            for (int i = threadIdx.x; i < (int)(sizeof(GemvJob) / 4); i += blockDim.x) dst[i] = src[i];
-            __syncthreads();
-            if (!STAGE_ALL)
-                stage_rows(sjob.in, sjob.inStride, sjob.inRow, min((int)sjob.n, MAXNT), (int)sjob.cols,
-                           xs, xsum);
-            current = (int)jobIdx;
-        }
+    float *xsum = smem + MAXNT * staged_stride((int)job.cols);
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(&job);
+    uint32_t *dst = reinterpret_cast<uint32_t *>(&sjob);
+    for (int i = threadIdx.x; i < (int)(sizeof(GemvJob) / 4); i += blockDim.x) dst[i] = src[i];
+    __syncthreads();
+    const int n = (int)sjob.n;
+    stage_rows(sjob.in, sjob.inStride, sjob.inRow, min(n, MAXNT), (int)sjob.cols, xs, xsum);
+    for (uint32_t block = blockIdx.x; block < blocks; block += gridDim.x) {
         const int row0 = (int)block * kRowsPerItem;
-        const int n = (int)sjob.n;
         if (n <= 1) {
-            run_item<1, DUAL, STAGE_ALL>(sjob, row0, xs, xsum);
+            run_item<1, DUAL>(sjob, row0, xs, xsum);
         } else if (MAXNT >= 2 && n <= 2) {
-            run_item<(MAXNT >= 2 ? 2 : 1), DUAL, STAGE_ALL>(sjob, row0, xs, xsum);
+            run_item<(MAXNT >= 2 ? 2 : 1), DUAL>(sjob, row0, xs, xsum);
         } else if (MAXNT >= 4 && n <= 4) {
-            run_item<(MAXNT >= 4 ? 4 : 1), DUAL, STAGE_ALL>(sjob, row0, xs, xsum);
+            run_item<(MAXNT >= 4 ? 4 : 1), DUAL>(sjob, row0, xs, xsum);
         } else if (MAXNT >= 8 && n <= 8) {
-            run_item<(MAXNT >= 8 ? 8 : 1), DUAL, STAGE_ALL>(sjob, row0, xs, xsum);
+            run_item<(MAXNT >= 8 ? 8 : 1), DUAL>(sjob, row0, xs, xsum);
         } else if (MAXNT >= 16) {
-            run_item<(MAXNT >= 16 ? 16 : 1), DUAL, STAGE_ALL>(sjob, row0, xs, xsum);
+            run_item<(MAXNT >= 16 ? 16 : 1), DUAL>(sjob, row0, xs, xsum);
         }
     }
 }
@@ -540,58 +504,40 @@ static uint32_t gemv_pass_rows(uint32_t n, uint32_t cols) {
     return 0;
 }
 
-// The input block all jobs of a launch read (staged once per CTA), or null.
-struct StageAll {
-    const uint16_t *in = nullptr;
-    uint32_t stride = 0, rows = 0;
-};
+static uint32_t blocks_of(uint32_t rows) { return (rows + kRowsPerItem - 1) / kRowsPerItem; }
 
-template <int MAXNT, bool DUAL, bool STAGE_ALL>
-static bool launch_gemv_kernel(FFContext *ctx, const GemvJob *jobs, const uint32_t *items,
-                               const uint32_t *itemCountPtr, const GemvJob &inlineJob,
-                               uint32_t inlineItems, uint32_t maxCols, uint32_t itemBound,
-                               const StageAll &all, cudaStream_t stream, const char **error) {
-    auto kernel = k_int4_gemv<MAXNT, DUAL, STAGE_ALL>;
-    const size_t smem = gemv_smem_bytes(STAGE_ALL ? (int)all.rows : MAXNT, maxCols);
+template <int MAXNT, bool DUAL>
+static bool launch_gemv_kernel(FFContext *ctx, const GemvJob &job, cudaStream_t stream, const char **error) {
+    auto kernel = k_int4_gemv<MAXNT, DUAL>;
+    const size_t smem = gemv_smem_bytes(MAXNT, job.cols);
     if (smem > kGemvSmemLimit)
         return fail(error, "input rows do not fit in shared memory: " + std::to_string(MAXNT) +
-                               " rows x " + std::to_string(maxCols) + " columns");
+                               " rows x " + std::to_string(job.cols) + " columns");
     // attribute + occupancy are looked up once per (kernel, device, shared-memory size): nothing but
     // the launch itself happens on later calls, which keeps the call legal under stream capture
     static KernelSmemMemo memo;
     int perSm = 0;
     if (!memo.prepare(kernel, ctx->device, smem, kGemvThreads, &perSm, error)) return false;
     if (perSm < 1) return fail(error, "GEMV kernel does not fit on an SM");
-    uint32_t grid = (uint32_t)(ctx->smCount * perSm);
-    if (itemBound < grid) grid = itemBound;
+    const uint32_t blocks = blocks_of(job.rows);
+    const uint32_t grid = std::min(blocks, (uint32_t)(ctx->smCount * perSm));
     if (grid == 0) return true;
     {
         LaunchScope scope(ctx, stream, DUAL ? "int4_gemv_gate_up_act" : "int4_gemv_down");
-        kernel<<<grid, kGemvThreads, smem, stream>>>(jobs, items, itemCountPtr, inlineJob,
-                                                     inlineItems, maxCols, all.in, all.stride, all.rows);
+        kernel<<<grid, kGemvThreads, smem, stream>>>(job, blocks);
     }
     FF_CUDA_OK(cudaGetLastError(), error);
     return true;
 }
 
 template <bool DUAL>
-static bool launch_gemv_class(FFContext *ctx, uint32_t rowsClass, const GemvJob *jobs,
-                              const uint32_t *items, const uint32_t *itemCountPtr,
-                              const GemvJob &inlineJob, uint32_t inlineItems, uint32_t maxCols,
-                              uint32_t itemBound, cudaStream_t stream, const char **error,
-                              const StageAll &all = StageAll()) {
-#define FF_GEMV_DISPATCH(NTV)                                                                   \
-    return launch_gemv_kernel<NTV, DUAL, false>(ctx, jobs, items, itemCountPtr, inlineJob, inlineItems, \
-                                                maxCols, itemBound, all, stream, error)
-    if (rowsClass <= 1) FF_GEMV_DISPATCH(1);
-    if (rowsClass <= 2) FF_GEMV_DISPATCH(2);
-    if (rowsClass <= 4) FF_GEMV_DISPATCH(4);
-    if (rowsClass <= 8) FF_GEMV_DISPATCH(8);
-    FF_GEMV_DISPATCH(16);
-#undef FF_GEMV_DISPATCH
+static bool launch_gemv_class(FFContext *ctx, const GemvJob &job, cudaStream_t stream, const char **error) {
+    if (job.n <= 1) return launch_gemv_kernel<1, DUAL>(ctx, job, stream, error);
+    if (job.n <= 2) return launch_gemv_kernel<2, DUAL>(ctx, job, stream, error);
+    if (job.n <= 4) return launch_gemv_kernel<4, DUAL>(ctx, job, stream, error);
+    if (job.n <= 8) return launch_gemv_kernel<8, DUAL>(ctx, job, stream, error);
+    return launch_gemv_kernel<16, DUAL>(ctx, job, stream, error);
 }
-
-static uint32_t blocks_of(uint32_t rows) { return (rows + kRowsPerItem - 1) / kRowsPerItem; }
 
 // One job given by value (a matrix, or a gate/up pair, against job.n <= 16 input rows).  When the
 // rows of the job's class do not fit in shared memory together (wide matrices), the job runs as
@@ -609,9 +555,7 @@ static bool launch_inline_job(FFContext *ctx, const GemvJob &job, cudaStream_t s
             part.inRow[i] = i < part.n ? job.inRow[first + i] : 0u;
             part.outRow[i] = i < part.n ? job.outRow[first + i] : 0u;
         }
-        if (!launch_gemv_class<DUAL>(ctx, part.n, nullptr, nullptr, nullptr, part, blocks_of(part.rows), part.cols,
-                                     blocks_of(part.rows), stream, error))
-            return false;
+        if (!launch_gemv_class<DUAL>(ctx, part, stream, error)) return false;
     }
     return true;
 }

@@ -103,9 +103,6 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-__device__ __forceinline__ void fence_generic_to_async() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
 // 32 consecutive fp32 columns of this thread's TMEM lane.
 __device__ __forceinline__ void tc_load_32cols(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(
@@ -178,14 +175,6 @@ __device__ __forceinline__ void tc_store_32cols(uint32_t taddr, const uint32_t (
         "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
 }
-__device__ __forceinline__ void tc_store_16cols(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
 __device__ __forceinline__ void tc_wait_st() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
@@ -207,35 +196,6 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t clusterAddr) {
     // has in flight is acknowledged, over a thousand cycles here; what the other CTA's MMA reads
     // from this CTA is ordered by the tcgen05 fences and the TMA's own barrier, not by this arrive)
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(clusterAddr) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// bounded wait on a barrier that the other CTA of the pair arrives on
-template <bool kSleep>
-__device__ __noinline__ bool mbar_wait_cluster_slow(uint32_t bar, uint32_t parity, volatile uint32_t *abortFlag) {
-    for (uint32_t i = 0; i < kSpinLimit; ++i) {
-        if (mbar_try_wait_cluster(bar, parity)) return true;
-        if (kSleep) __nanosleep(40);
-        if ((i & 255u) == 255u && *abortFlag) return false;
-    }
-    *abortFlag = 1u;
-    return false;
-}
-template <bool kSleep>
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile uint32_t *abortFlag) {
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-    return mbar_wait_cluster_slow<kSleep>(bar, parity, abortFlag);
 }
 // A wait of a whole converged warp whose lanes then act as one: either all of them go on or none.  Acquires
 // at CTA scope also where the other CTA arrives: what that CTA wrote for the MMA is ordered by the
@@ -262,15 +222,6 @@ __device__ __forceinline__ int warp_index() { return __shfl_sync(0xFFFFFFFFu, (i
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n"
                  "barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// This CTA's part of a tile that the pair's MMA reads from both CTAs; completes on the leader's barrier.
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, int x, int y,
-                                                 uint32_t leaderBar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(leaderBar)
-        : "memory");
 }
 // arrives once on the barrier at this shared-memory offset in both CTAs when the MMAs issued so far are done
 __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {

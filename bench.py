@@ -52,7 +52,7 @@ def profiled_decode_traffic():
         return None, "no profile"
     text = open(path).read()
     h = hashlib.sha256()
-    for name in ("ff_decode.cu", "ff_mma_device.cuh"):
+    for name in ("ff_decode.cu", "ff_int_device.cuh", "ff_mma_device.cuh"):
         with open(os.path.join(ROOT, "ane_fieldfare_b200", "csrc", name), "rb") as fh:
             h.update(fh.read())
     digest = re.search(r"kernel sources sha256: ([0-9a-f]{64})", text)
