@@ -307,6 +307,55 @@ __device__ __forceinline__ void segment_histogram(const uint32_t *routes, int n,
     }
 }
 
+// The experts' offsets and row tiles (up to kRowTile rows of one expert each, experts ascending) from thread
+// e's number of routes to expert e (0 from E on); a CTA of 256 threads.  Returns the expert's offset.
+// counts[0] = row tiles, counts[1] = pairs, counts[2] = experts with at least one pair.
+__device__ __forceinline__ uint32_t plan_row_tiles(uint32_t total, int E, uint32_t *expertOffsets, RowTile *tiles, uint32_t maxTiles,
+                                                   uint32_t *counts) {
+    __shared__ uint32_t warpSums[3][8];
+    const int e = threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t myTiles = (total + kRowTile - 1u) / kRowTile;
+    uint32_t rows = total, tileEnd = myTiles;  // inclusive sums
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, rows, o), b = __shfl_up_sync(0xFFFFFFFFu, tileEnd, o);
+        if (lane >= o) {
+            rows += a;
+            tileEnd += b;
+        }
+    }
+    const uint32_t active = __popc(__ballot_sync(0xFFFFFFFFu, total != 0u));
+    if (lane == 31) {
+        warpSums[0][warp] = rows;
+        warpSums[1][warp] = tileEnd;
+        warpSums[2][warp] = active;
+    }
+    __syncthreads();
+    uint32_t activeAll = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        if (w < warp) {
+            rows += warpSums[0][w];
+            tileEnd += warpSums[1][w];
+        }
+        activeAll += warpSums[2][w];
+    }
+    const uint32_t start = rows - total;
+    if (e < E) {
+        expertOffsets[e] = start;
+        for (uint32_t i = 0, tix = tileEnd - myTiles; i < total; i += kRowTile, ++tix)
+            if (tix < maxTiles) tiles[tix] = RowTile{start + i, min(kRowTile, total - i), (uint32_t)e, 0u};
+    }
+    if (e == 255) {
+        expertOffsets[E] = rows;
+        counts[0] = min(tileEnd, maxTiles);
+        counts[1] = rows;
+        counts[2] = activeAll;
+        counts[3] = 0;
+    }
+    return start;
+}
+
 // Pass 1: per block of 256 tokens, how many routes name each expert.
 __global__ void __launch_bounds__(256)
 k_route_count(const uint32_t *ids, int T, int K, int E, uint32_t *blockCounts) {
@@ -328,16 +377,12 @@ k_route_count(const uint32_t *ids, int T, int K, int E, uint32_t *blockCounts) {
     }
 }
 
-// Pass 2 (one block): exclusive prefix of every expert's counts over the blocks, expert offsets,
-// and the list of row tiles (up to kRowTile rows of one expert each), experts ascending.
-// counts[0] = row tiles, counts[1] = pairs, counts[2] = experts with at least one pair.
+// Pass 2 (one block): exclusive prefix of every expert's counts over the blocks, then the plan.
 __global__ void __launch_bounds__(256)
 k_route_scan(uint32_t *blockCounts, int blocks, int E, uint32_t *expertOffsets, RowTile *tiles,
              uint32_t maxTiles, uint32_t *counts) {
     pdl_enter();
-    __shared__ uint32_t total[kMaxExperts];
-    __shared__ uint32_t offset[kMaxExperts + 1];
-    __shared__ uint32_t tileBase[kMaxExperts + 1];
+    uint32_t total = 0;
     const int e = threadIdx.x;
     if (e < E) {
         // eight blocks' counts are fetched together (independent loads), then turned into prefixes
@@ -353,58 +398,24 @@ k_route_scan(uint32_t *blockCounts, int blocks, int E, uint32_t *expertOffsets, 
                     run += c[i];
                 }
         }
-        total[e] = run;
+        total = run;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t run = 0, tilesRun = 0, active = 0;
-        for (int i = 0; i < E; ++i) {
-            offset[i] = run;
-            tileBase[i] = tilesRun;
-            run += total[i];
-            tilesRun += (total[i] + kRowTile - 1u) / kRowTile;
-            active += total[i] ? 1u : 0u;
-        }
-        offset[E] = run;
-        tileBase[E] = tilesRun;
-        counts[0] = min(tilesRun, maxTiles);
-        counts[1] = run;
-        counts[2] = active;
-        counts[3] = 0;
-    }
-    __syncthreads();
-    if (e < E) expertOffsets[e] = offset[e];
-    if (e == 0) expertOffsets[E] = offset[E];
-    if (e < E) {
-        const uint32_t n = total[e];
-        for (uint32_t i = 0, tix = tileBase[e]; i < n; i += kRowTile, ++tix)
-            if (tix < maxTiles) tiles[tix] = RowTile{offset[e] + i, min(kRowTile, n - i), (uint32_t)e, 0u};
-    }
+    plan_row_tiles(total, E, expertOffsets, tiles, maxTiles, counts);
 }
 
-// Pass 3: every route's position in (expert, token, rank) order; writes the sorted pair list.
+constexpr uint32_t kNoRow = 0xFFFFFFFFu;  // of a route to no expert
+
+// Every route's position in (expert, token, rank) order; writes the sorted pair list.
 // Position = expert offset + routes to the expert in earlier blocks + in earlier warp segments of
 // this block + earlier in this warp's segment (earlier 32-route batches, then lower lanes).
-constexpr uint32_t kNoRow = 0xFFFFFFFFu;  // of a route to no expert
-__global__ void __launch_bounds__(256)
-k_route_scatter(const uint32_t *ids, const uint16_t *weights, int T, int K, int E,
-                const uint32_t *blockCounts, const uint32_t *expertOffsets,
-                FFTokenExpertPair *sorted, uint32_t *rowOfRoute) {
-    pdl_enter();
-    extern __shared__ uint32_t sRoutes[];
-    __shared__ uint32_t segCount[8 * kMaxExperts];
-    const int t0 = blockIdx.x * kSortTokens;
-    const int n = min(kSortTokens, T - t0) * K;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) sRoutes[i] = ids[(size_t)t0 * K + i];
-    for (int i = threadIdx.x; i < 8 * E; i += blockDim.x) segCount[i] = 0;
-    __syncthreads();
-    const int seg = (n + 7) / 8;
-    segment_histogram(sRoutes, n, seg, E, segCount);
-    __syncthreads();
+// `base`: of expert threadIdx.x, the first two terms.
+__device__ __forceinline__ void place_routes(const uint32_t *sRoutes, uint32_t *segCount, int n, int seg, uint32_t base,
+                                             const uint16_t *weights, int t0, int K, int E, FFTokenExpertPair *sorted,
+                                             uint32_t *rowOfRoute) {
     const int e = threadIdx.x;
     if (e < E) {
         // turn the segment counts into each segment's first position for this expert
-        uint32_t run = expertOffsets[e] + blockCounts[(size_t)blockIdx.x * E + e];
+        uint32_t run = base;
         for (int w = 0; w < 8; ++w) {
             const uint32_t c = segCount[w * E + e];
             segCount[w * E + e] = run;
@@ -434,6 +445,49 @@ k_route_scatter(const uint32_t *ids, const uint16_t *weights, int T, int K, int 
     }
 }
 
+// Pass 3.
+__global__ void __launch_bounds__(256)
+k_route_scatter(const uint32_t *ids, const uint16_t *weights, int T, int K, int E,
+                const uint32_t *blockCounts, const uint32_t *expertOffsets,
+                FFTokenExpertPair *sorted, uint32_t *rowOfRoute) {
+    pdl_enter();
+    extern __shared__ uint32_t sRoutes[];
+    __shared__ uint32_t segCount[8 * kMaxExperts];
+    const int t0 = blockIdx.x * kSortTokens;
+    const int n = min(kSortTokens, T - t0) * K;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) sRoutes[i] = ids[(size_t)t0 * K + i];
+    for (int i = threadIdx.x; i < 8 * E; i += blockDim.x) segCount[i] = 0;
+    __syncthreads();
+    const int seg = (n + 7) / 8;
+    segment_histogram(sRoutes, n, seg, E, segCount);
+    __syncthreads();
+    const int e = threadIdx.x;
+    place_routes(sRoutes, segCount, n, seg, e < E ? expertOffsets[e] + blockCounts[(size_t)blockIdx.x * E + e] : 0u, weights, t0, K, E,
+                 sorted, rowOfRoute);
+}
+
+// All three passes for one block's worth of tokens: a chunk of up to 256 has one launch in front of its
+// gather instead of three (77 tokens: 14 us of a layer's 130 between the routes and the sorted list).
+__global__ void __launch_bounds__(256)
+k_route_sort(const uint32_t *ids, int T, int K, int E, uint32_t *expertOffsets, RowTile *tiles, uint32_t maxTiles, uint32_t *counts,
+             FFTokenExpertPair *sorted, uint32_t *rowOfRoute) {
+    pdl_enter();
+    extern __shared__ uint32_t sRoutes[];
+    __shared__ uint32_t segCount[8 * kMaxExperts];
+    const int n = T * K, seg = (n + 7) / 8;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) sRoutes[i] = ids[i];
+    for (int i = threadIdx.x; i < 8 * E; i += blockDim.x) segCount[i] = 0;
+    __syncthreads();
+    segment_histogram(sRoutes, n, seg, E, segCount);
+    __syncthreads();
+    const int e = threadIdx.x;
+    uint32_t total = 0;
+    if (e < E)
+        for (int w = 0; w < 8; ++w) total += segCount[w * E + e];
+    const uint32_t start = plan_row_tiles(total, E, expertOffsets, tiles, maxTiles, counts);
+    place_routes(sRoutes, segCount, n, seg, start, nullptr, 0, K, E, sorted, rowOfRoute);
+}
+
 // Row tiles of a dense problem: T rows of one "expert" (the shared FFN).
 __global__ void k_dense_tiles(int T, RowTile *tiles, uint32_t *counts) {
     pdl_enter();
@@ -457,10 +511,16 @@ k_gather_rows(const uint16_t *x, uint32_t xStride, uint32_t rows, const uint32_t
     pdl_enter();
     const int chunksPerRow = D / 8;
     const size_t total = (size_t)rows * chunksPerRow;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t r = (uint32_t)(i / chunksPerRow);
-        const int c = (int)(i - (size_t)r * chunksPerRow);
+    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t step = gridDim.x * blockDim.x, stepRows = step / chunksPerRow;
+    const int stepChunks = (int)(step - stepRows * chunksPerRow);
+    uint32_t r = (uint32_t)(first / chunksPerRow);
+    int c = (int)(first - (size_t)r * chunksPerRow);
+    for (size_t i = first; i < total; i += step, r += stepRows, c += stepChunks) {
+        if (c >= chunksPerRow) {
+            c -= chunksPerRow;
+            ++r;
+        }
         const uint4 v = *reinterpret_cast<const uint4 *>(x + (size_t)r * xStride + c * 8);
         // halves h0..h7 -> h0,h4,h1,h5,h2,h6,h3,h7
         uint4 o;
@@ -1190,6 +1250,36 @@ static bool check_gemm_shapes(const FFConfig &c, uint32_t f, const char **error)
     return true;
 }
 
+// Sorts the routes (stable, by expert) and plans the row tiles.
+static bool sort_routes(FFContext *ctx, const uint32_t *ids, uint32_t tokens, int E, uint32_t *offsets, RowTile *tiles,
+                              FFTokenExpertPair *sorted, uint32_t *rowOfRoute, cudaStream_t stream, const char **error) {
+    const int T = (int)tokens, K = (int)ctx->cfg.topK;
+    const uint32_t blocks = (tokens + kSortTokens - 1) / kSortTokens;
+    const size_t sortSmem = (size_t)kSortTokens * K * sizeof(uint32_t);
+    const uint32_t maxTiles = ctx->maxUnits / 2;  // first half of the tile buffer
+    if (blocks == 1) {
+        LaunchScope scope(ctx, stream, "route_sort");
+        FF_CUDA_OK(launch_pdl(k_route_sort, 1, 256, sortSmem, stream, ids, T, K, E, offsets, tiles, maxTiles, ctx->unitCount, sorted,
+                              rowOfRoute),
+                   error);
+        return true;
+    }
+    {
+        LaunchScope scope(ctx, stream, "route_count");
+        FF_CUDA_OK(launch_pdl(k_route_count, blocks, 256, sortSmem, stream, ids, T, K, E, ctx->blockCounts), error);
+    }
+    {
+        LaunchScope scope(ctx, stream, "route_scan");
+        FF_CUDA_OK(launch_pdl(k_route_scan, 1, 256, 0, stream, ctx->blockCounts, (int)blocks, E, offsets, tiles, maxTiles, ctx->unitCount),
+                   error);
+    }
+    LaunchScope scope(ctx, stream, "route_scatter");
+    FF_CUDA_OK(launch_pdl(k_route_scatter, blocks, 256, sortSmem, stream, ids, nullptr, T, K, E, ctx->blockCounts, offsets, sorted,
+                          rowOfRoute),
+               error);
+    return true;
+}
+
 bool launch_prefill_routed(FFContext *ctx, LayerStore &L, const uint16_t *x, uint32_t xStride,
                            uint32_t tokens, const uint32_t *ids, uint16_t *partials,
                            cudaStream_t stream, const char **error) {
@@ -1198,31 +1288,9 @@ bool launch_prefill_routed(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     if (!ctx->xSorted) return fail(error, "context was created with maxTokens <= 16: no prefill scratch");
     if (!L.experts) return fail(error, "layer has no resident experts");
     if (!check_gemm_shapes(c, c.f, error) || !prefill_prepare_layer(ctx, L, error)) return false;
-    const int T = (int)tokens, K = (int)c.topK, E = (int)L.expertCount;
-    const uint32_t blocks = (tokens + kSortTokens - 1) / kSortTokens;
-    const size_t sortSmem = (size_t)kSortTokens * K * sizeof(uint32_t);
+    const int K = (int)c.topK, E = (int)L.expertCount;
     RowTile *tiles = reinterpret_cast<RowTile *>(ctx->units);
-    const uint32_t maxTiles = ctx->maxUnits / 2;  // first half of the tile buffer
-    {
-        LaunchScope scope(ctx, stream, "route_count");
-        FF_CUDA_OK(launch_pdl(k_route_count, blocks, 256, sortSmem, stream,
-                              ids, T, K, E, ctx->blockCounts),
-                   error);
-    }
-    {
-        LaunchScope scope(ctx, stream, "route_scan");
-        FF_CUDA_OK(launch_pdl(k_route_scan, 1, 256, 0, stream,
-                              ctx->blockCounts, (int)blocks, E, ctx->expertOffsets, tiles,
-                                            maxTiles, ctx->unitCount),
-                   error);
-    }
-    {
-        LaunchScope scope(ctx, stream, "route_scatter");
-        FF_CUDA_OK(launch_pdl(k_route_scatter, blocks, 256, sortSmem, stream,
-                              ids, nullptr, T, K, E, ctx->blockCounts,
-                              ctx->expertOffsets, ctx->sortedPairs, ctx->rowOfRoute),
-                   error);
-    }
+    if (!sort_routes(ctx, ids, tokens, E, ctx->expertOffsets, tiles, ctx->sortedPairs, ctx->rowOfRoute, stream, error)) return false;
     const uint32_t pairs = tokens * c.topK;
     {
         LaunchScope scope(ctx, stream, "gather_rows");
@@ -1273,32 +1341,8 @@ bool launch_route_sort(FFContext *ctx, const uint32_t *groupIds, uint32_t tokens
     if (!ctx->xSorted) return fail(error, "context was created with maxTokens <= 16: no prefill scratch");
     if (groups == 0 || groups > c.experts) return fail(error, "group count must be 1..experts of the context");
     if (tokens > c.maxTokens) return fail(error, "rows exceed the context's maxTokens");
-    const int T = (int)tokens, K = (int)c.topK, E = (int)groups;
-    const uint32_t blocks = (tokens + kSortTokens - 1) / kSortTokens;
-    const size_t sortSmem = (size_t)kSortTokens * K * sizeof(uint32_t);
-    RowTile *tiles = reinterpret_cast<RowTile *>(ctx->units);
-    {
-        LaunchScope scope(ctx, stream, "route_count");
-        FF_CUDA_OK(launch_pdl(k_route_count, blocks, 256, sortSmem, stream,
-                              groupIds, T, K, E, ctx->blockCounts),
-                   error);
-    }
-    {
-        LaunchScope scope(ctx, stream, "route_scan");
-        FF_CUDA_OK(launch_pdl(k_route_scan, 1, 256, 0, stream,
-                              ctx->blockCounts, (int)blocks, E, offsets, tiles, ctx->maxUnits / 2,
-                                            ctx->unitCount),
-                   error);
-    }
-    {
-        LaunchScope scope(ctx, stream, "route_scatter");
-        FF_CUDA_OK(launch_pdl(k_route_scatter, blocks, 256, sortSmem, stream,
-                              groupIds, nullptr, T, K, E, ctx->blockCounts, offsets,
-                              sortedPairs, nullptr),
-                   error);
-    }
-    FF_CUDA_OK(cudaGetLastError(), error);
-    return true;
+    return sort_routes(ctx, groupIds, tokens, (int)groups, offsets, reinterpret_cast<RowTile *>(ctx->units), sortedPairs, nullptr, stream,
+                       error);
 }
 
 bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uint32_t xStride,
