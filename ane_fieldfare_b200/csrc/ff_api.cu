@@ -314,7 +314,7 @@ static bool moe_layer_host_one_token(FFContext *ctx, uint32_t layer, const uint1
                                      bool *handled, const char **error) {
     *handled = false;
     const FFConfig &cfg = ctx->cfg;
-    if (layer >= cfg.layers || cfg.d > 4096 || !ctx->mailbox) return true;
+    if (layer >= cfg.layers || cfg.d > 4096 || !ctx->mailbox || !decode_fused_fits(cfg)) return true;
     LayerStore &L = ctx->layers[layer];
     if (!L.experts || !L.routerW || L.has_shared8()) return true;
     cudaPointerAttributes attr{};

@@ -59,6 +59,8 @@ struct BlockArgs {
     uint32_t *activeExperts;  // gate/up: receives the count (may be null)
     uint32_t *errorFlag;
     uint32_t listOffset, digitsOffset, rowBytes, auxOffset, auxRow, slotsOffset, slotBytes, sbOffset;
+    int perExpert;            // routes of one expert at most
+    float *values;            // F32OUT: the routed rows
 };
 
 struct alignas(64) BlockMaps {
@@ -178,7 +180,8 @@ __device__ __forceinline__ void mma_1688(float (&d)[4], uint32_t a0, uint32_t a1
 }
 constexpr uint32_t kSumBlockBytes = 128;  // [column][8 groups] bf16
 
-template <int MODE, bool INT8>
+// F32OUT (down): the routed rows go to `values` unrounded.
+template <int MODE, bool INT8, bool F32OUT>
 __global__ void __launch_bounds__(kMaxWarps * 32, 1)
 k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
     extern __shared__ __align__(128) uint8_t smemRaw[];
@@ -207,17 +210,17 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
         const uint32_t id = r < routes ? a.ids[r] : 0xFFFFFFFFu;
         const uint32_t peers = __match_any_sync(0xFFFFFFFFu, id), before = __popc(peers & ((1u << lane) - 1u));
         const bool known = id < (uint32_t)a.E;
-        // A token's routes are distinct experts, so an expert is chosen by at most T routes; repeats
-        // beyond that and routes past the resident experts keep their rows unwritten and raise the flag
+        // A block's tokens choose distinct experts, so an expert has at most T routes (a single row may name
+        // one several times); repeats beyond that and routes past the resident experts keep their rows unwritten and raise the flag
         // (the reference refuses such a route with "route expert N is out of range").
         for (int w = 0; w < 4; ++w) {  // warps in turn: a route's place counts all earlier ones
             if (warp == w && r < routes) {
                 const uint32_t place = known ? sCount[id] + before : 0u;
-                if (known && place < (uint32_t)a.T) sList[id * kMaxGemvRows + place] = (uint8_t)r;
+                if (known && place < (uint32_t)a.perExpert) sList[id * kMaxGemvRows + place] = (uint8_t)r;
                 else atomicExch(a.errorFlag, 12u);
             }
             __syncwarp();
-            if (warp == w && r < routes && known && before == 0) sCount[id] = min(sCount[id] + (uint32_t)__popc(peers), (uint32_t)a.T);
+            if (warp == w && r < routes && known && before == 0) sCount[id] = min(sCount[id] + (uint32_t)__popc(peers), (uint32_t)a.perExpert);
             named_barrier(1, 128);
         }
     }
@@ -524,11 +527,15 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
                         r1 = fmaf(r1, unit, b1);
                     }
                     if ((t & 1) || mine >= n) continue;
-                    uint16_t *dst = k.out + (size_t)row_of(mine) * k.outStride;
+                    const size_t to = (size_t)row_of(mine) * k.outStride;
+                    uint16_t *dst = k.out + to;
                     if (MODE == kGateUp) {
                         // the shared FFN rounds gate and up before the activation
                         const float gate = kind ? r0 : bf16_round(r0), up = kind ? r1 : bf16_round(r1);
                         dst[tile * 8u + (uint32_t)g] = f2bf(gelu_tanh(gate) * up);
+                    } else if (F32OUT && kind) {
+                        a.values[to + tile * 16u + (uint32_t)g] = r0;
+                        a.values[to + tile * 16u + 8u + (uint32_t)g] = r1;
                     } else {
                         dst[tile * 16u + (uint32_t)g] = f2bf(r0);
                         dst[tile * 16u + 8u + (uint32_t)g] = f2bf(r1);
@@ -591,7 +598,7 @@ bool setup_kind(int mode, bool int8, uint32_t &ready, uint32_t bit, BlockKind &k
                    experts > 1 ? scaleStride * 4 : scaleRows * padded * 4, k.sbWords, 16, error);
 }
 
-template <int MODE, bool INT8>
+template <int MODE, bool INT8, bool F32OUT = false>
 bool launch_kernel(FFContext *ctx, BlockArgs a, const BlockMaps &maps, const char *name, cudaStream_t stream, const char **error) {
     uint32_t groups = 0, slot = 0, sb = 0;
     for (int i = 0; i < 2; ++i) {
@@ -601,7 +608,7 @@ bool launch_kernel(FFContext *ctx, BlockArgs a, const BlockMaps &maps, const cha
         sb = std::max(sb, 64 * a.kind[i].sbWords);
     }
     auto up128 = [](uint32_t v) { return (v + 127u) & ~127u; };
-    const uint32_t rows = (uint32_t)std::min(a.T, kTaskRows), padded = padded_groups(groups);
+    const uint32_t rows = (uint32_t)std::min(std::max(a.T, a.perExpert), kTaskRows), padded = padded_groups(groups);
     a.listOffset = 0;
     a.digitsOffset = a.ids ? up128((uint32_t)a.E * kMaxGemvRows) : 0;
     a.rowBytes = padded * kDigitGroupBytes;
@@ -617,10 +624,10 @@ bool launch_kernel(FFContext *ctx, BlockArgs a, const BlockMaps &maps, const cha
     const uint32_t warps = std::min<uint32_t>(kMaxWarps, (kLimit - a.slotsOffset) / (2 * a.slotBytes));
     const size_t smem = a.slotsOffset + (size_t)warps * 2 * a.slotBytes;
     static KernelSmemMemo memo;
-    if (!memo.prepare(k_block_int<MODE, INT8>, ctx->device, kLimit, kMaxWarps * 32, nullptr, error)) return false;
+    if (!memo.prepare(k_block_int<MODE, INT8, F32OUT>, ctx->device, kLimit, kMaxWarps * 32, nullptr, error)) return false;
     {
         LaunchScope scope(ctx, stream, name);
-        FF_CUDA_OK(launch_pdl(k_block_int<MODE, INT8>, ctx->smCount, warps * 32, smem, stream, a, maps), error);
+        FF_CUDA_OK(launch_pdl(k_block_int<MODE, INT8, F32OUT>, ctx->smCount, warps * 32, smem, stream, a, maps), error);
     }
     return true;
 }
@@ -628,10 +635,11 @@ bool launch_kernel(FFContext *ctx, BlockArgs a, const BlockMaps &maps, const cha
 }  // namespace
 
 // Routed experts (ids [tokens][K], partial rows to `partials`) and / or the INT4 shared FFN (rows to
-// `sharedOut`) of up to 16 rows.
+// `sharedOut`) of up to 16 rows.  `values` not null: the routed rows go there as fp32 instead, and one row's
+// routes may repeat an expert.
 bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens,
                        const uint32_t *ids, bool withShared, uint16_t *partials, uint16_t *sharedOut, cudaStream_t stream,
-                       const char **error) {
+                       const char **error, float *values) {
     const FFConfig &c = ctx->cfg;
     if (c.d % 64 || c.f % 64 || c.sharedF % 64) return fail(error, "widths must be multiples of 64");
     if (((uintptr_t)x & 15) || (xStride % 8)) return fail(error, "input rows must be 16-byte aligned");
@@ -643,6 +651,8 @@ bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
         a.T = (int)tokens;
         a.K = (int)c.topK;
         a.E = ids ? (int)L.expertCount : 0;
+        a.perExpert = values ? (int)c.topK : (int)tokens;
+        a.values = values;
         a.withShared = withShared;
         a.activeExperts = &ctx->plan->activeExperts;
         a.errorFlag = ctx->errorFlag;
@@ -673,7 +683,8 @@ bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
         }
         BlockMaps maps;
         memcpy(&maps, Lm.blockMap[mode], sizeof(maps));
-        const bool ok = down ? launch_kernel<kDown, false>(ctx, a, maps, "int4_block_down", stream, error)
+        const bool ok = values && down ? launch_kernel<kDown, false, true>(ctx, a, maps, "int4_block_down", stream, error)
+                        : down ? launch_kernel<kDown, false>(ctx, a, maps, "int4_block_down", stream, error)
                              : launch_kernel<kGateUp, false>(ctx, a, maps, "int4_block_gate_up_act", stream, error);
         if (!ok) return false;
     }
@@ -689,6 +700,7 @@ bool launch_block_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
         BlockArgs a{};
         a.T = (int)tokens;
         a.K = 1;
+        a.perExpert = (int)tokens;
         a.withShared = 1;
         a.errorFlag = ctx->errorFlag;
         const bool down = mode == kDown;

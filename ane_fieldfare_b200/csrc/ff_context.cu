@@ -87,7 +87,7 @@ void ff_destroy(FFContext *ctx) {
                     ctx->partials, ctx->xDev, ctx->yDev, ctx->xSorted, ctx->xShared, ctx->rowOfRoute, ctx->sortedPairs,
                     ctx->expertOffsets, ctx->blockCounts, ctx->units, ctx->unitCount,
                     ctx->errorFlag, ctx->gridBarrier, ctx->phaseStamps, ctx->mapScratch, ctx->taggedLogits, ctx->taggedActs,
-                    ctx->logitsRows, ctx->routeIds, ctx->routeWeights, ctx->xSums, ctx->actSums, ctx->routerParts};
+                    ctx->logitsRows, ctx->routeIds, ctx->routeWeights, ctx->xSums, ctx->actSums, ctx->routerParts, ctx->decodeValues};
     for (void *p : ptrs) cudaFree(p);
     if (ctx->hostStream) cudaStreamDestroy(ctx->hostStream);
     if (ctx->sideStream) cudaStreamDestroy(ctx->sideStream);
@@ -155,6 +155,7 @@ FFContext *ff_create(int32_t deviceOrdinal, const FFConfig *config, const char *
     ok = ok && dev_alloc(ctx, &ctx->sharedActs, (T + 256) * c.sharedF, error);
     ok = ok && dev_alloc(ctx, &ctx->h1, T * c.d, error);
     ok = ok && dev_alloc(ctx, &ctx->partials, T * K * c.d, error);
+    if (!decode_fused_fits(c)) ok = ok && dev_alloc(ctx, &ctx->decodeValues, K * c.d, error);
     ok = ok && dev_alloc(ctx, &ctx->xDev, T * c.d, error);
     ok = ok && dev_alloc(ctx, &ctx->yDev, T * c.d, error);
     ok = ok && dev_alloc(ctx, &ctx->errorFlag, 4, error);

@@ -89,7 +89,7 @@ struct DecodeArgs {
     unsigned long long *mailbox;
     uint32_t epoch;
     // shared-memory carve-up (fused_layout)
-    uint32_t x32Offset, regionOffset, regionAux, partialOffset, downOffset, slotsOffset, rowsBytes, pairBytes, tripleBytes, downBytes;
+    uint32_t regionOffset, regionAux, actsAux, partialOffset, downOffset, slotsOffset, rowsBytes, pairBytes, tripleBytes, downBytes;
     uint32_t strideGU, strideGUA, strideSD, strideRD;
 };
 
@@ -312,12 +312,16 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     const int groupsD = D >> 6, groupsF = F >> 6, groupsFs = Fs >> 6;
     const int auxGroups = (groupsF + 1) & ~1;  // a routed row's aux groups, 16-byte aligned
 
-    // shared memory: x as digits | its group sums | x as it is (router) | region: the shared activations,
-    // then the routed activations | K-split partial sums | routed down rows per expert |
-    // slots: five pairs (two tile parts, the tile's scales), two triples of the other six warps
+    // shared memory: x as digits | its group sums | the shared activations as digits | their group sums; over
+    // these, once phase B is done, the routed activations as digits | their group sums || K-split partial sums |
+    // routed down rows per expert | slots: five pairs (two tile parts, the tile's scales), two triples of the
+    // other six warps.  The fifth pair has no tile in phase A: its slot holds x as fp32 for the router until then.
     const uint32_t smem = sm_addr(smemRaw);
     uint8_t *region = smemRaw + a.regionOffset;
     GroupAux *regionAux = reinterpret_cast<GroupAux *>(smemRaw + a.regionAux);
+    GroupAux *actsAux = reinterpret_cast<GroupAux *>(smemRaw + a.actsAux);
+    const uint32_t x32Offset = a.slotsOffset + (kSharedGuWarps / 2) * a.pairBytes;
+    const bool routing = !a.idsIn && K > 0;
     GroupAux *xAux = reinterpret_cast<GroupAux *>(smemRaw + D * 4);
     float *partial = reinterpret_cast<float *>(smemRaw + a.partialOffset);  // [warp][16]
     float *downRows = reinterpret_cast<float *>(smemRaw + a.downOffset);    // [row tile][expert][8]
@@ -351,7 +355,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     // Router rows: warps 8, 9 take one expert each and hold its row in registers, 3072 inputs at a time
     // (through shared memory the row's loads waited for the barriers' set-up, and the chain for the loads).
     const int rw = warp - kSharedGuWarps, chunksD = D >> 3;
-    int eA = (!a.idsIn && K > 0 && rw >= 0 && rw < kRouterWarps) ? rw * G + cta : 0x7FFFFFFF;
+    int eA = (routing && rw >= 0 && rw < kRouterWarps) ? rw * G + cta : 0x7FFFFFFF;
     uint4 wr[kRouterChunks];
     auto load_router = [&](int first) {
         const uint4 *row = reinterpret_cast<const uint4 *>(a.routerW + (size_t)eA * D);
@@ -440,8 +444,9 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     // the input row, as digits and (for the router) as it is
     stage_digits(D >> 3, (int)threadIdx.x, kFusedThreads, smemRaw, xAux, groupsD, 0, [&](int i, int j, uint4 &v, uint4 &w) {
         // as fp32 [step of 32 runs][half][lane] for the router's chains
-        float4 *x32 = reinterpret_cast<float4 *>(smemRaw + a.x32Offset);
+        float4 *x32 = reinterpret_cast<float4 *>(smemRaw + x32Offset);
         auto keep = [&](int r, const uint4 &q) {
+            if (!routing) return;
             const uint32_t qq[4] = {q.x, q.y, q.z, q.w};
             float f[8];
 #pragma unroll
@@ -500,7 +505,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
             for (int i = 0; i < kRouterChunks; ++i) {
                 const int c = first + 32 * i + lane;
                 if (c < chunksD) {
-                    const uint32_t at = smem + a.x32Offset + 16u * (uint32_t)(2 * c - lane);
+                    const uint32_t at = smem + x32Offset + 16u * (uint32_t)(2 * c - lane);
                     const uint4 lo = lds128(at), hi = lds128(at + 512u);
                     const uint32_t xx[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
                     const uint32_t ww[4] = {wr[i].x, wr[i].y, wr[i].z, wr[i].w};
@@ -521,6 +526,9 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
         eA += kRouterWarps * G;
         if (eA < E) load_router(0);
     }
+    // The fifth pair's first copies, behind the ranking's barriers, overwrite x as fp32.  (By the warp that mostly has
+    // no router row, hence no stores in flight that the fence would wait for.)
+    if (routing && warp == kRankWarp) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     warp_stamp(a, 0, 2);
     stamp(a, 1);
 
@@ -565,7 +573,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     };
     if (tB < tilesRouted) issue_routed_gate_up();
     if (warp < kBigWarps) warp_stamp(a, 1, 0);
-    if (K > 0 && !a.idsIn && warp == kSharedGuWarps) {
+    if (routing && warp == kSharedGuWarps) {
         // softmax over the chosen scores: exponentials in parallel, the sum in rank order
         const float myScore = lane < K ? sScore[lane] : -INFINITY;
         const float top = __shfl_sync(0xFFFFFFFFu, myScore, 0);
@@ -694,7 +702,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
     warp_stamp(a, 2, 0);
     // (seven eighths: the last tiles' words are polled for, by the few threads that stage them)
     if (is_waiting_thread()) hint_wait(sHints + 1, (uint32_t)(tilesRouted - tilesRouted / 8));
-    __syncthreads();  // the region still holds the shared activations that phase B's warps read
+    __syncthreads();  // the routed activations take the place of the rows that phase B's warps read
     stamp(a, 5);
 
     // ---------------- phase C: routed down rows and the combine ----------------
@@ -711,7 +719,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
         else residual = a.residual ? bf2f(__ldcg(a.residual + row)) : 0.0f;
     };
     ask_residual(0);
-    stage_digits(K * (F >> 3), (int)threadIdx.x, kFusedThreads, region, regionAux, groupsF, auxGroups,
+    stage_digits(K * (F >> 3), (int)threadIdx.x, kFusedThreads, smemRaw, actsAux, groupsF, auxGroups,
                  [&](int i, int j, uint4 &v, uint4 &w) { fetch_tagged(a.taggedActs, tag, i, j, v, w, a.errorFlag); });
     __syncthreads();
     for (int round = 0; cta + G * round * perRound < tilesRD; ++round) {
@@ -722,8 +730,8 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
             const int mine = t < 2 ? eLo : eHi, column = g < 4 ? eLo : eHi;
             const uint32_t s = downSlot + 16u * a.strideRD + 4u * ((t < 2 ? 0u : wordsRD) + (uint32_t)g * padded_groups((uint32_t)groupsF));
             const float v = tile_int4<true>(downSlot + (uint32_t)g * a.strideRD + 8u * t, downSlot + (uint32_t)(g + 8) * a.strideRD + 8u * t,
-                                            sm_addr(region) + (uint32_t)(column * groupsF) * kDigitGroupBytes + (uint32_t)(g & 3) * 64u + (uint32_t)t * 16u,
-                                            s, s, sm_addr(regionAux) + 8u * (uint32_t)(mine * auxGroups), groupsF)
+                                            smem + (uint32_t)(column * groupsF) * kDigitGroupBytes + (uint32_t)(g & 3) * 64u + (uint32_t)t * 16u,
+                                            s, s, sm_addr(actsAux) + 8u * (uint32_t)(mine * auxGroups), groupsF)
                                 .x;
             if (!(t & 1) && (t == 0 || eHi > eLo)) downRows[(myTile * 8 + mine) * 8 + g] = v;
         }
@@ -835,7 +843,7 @@ bool pack_scales(FFContext *ctx, const ScaleSource &src, uint32_t D, uint32_t F,
 }
 
 struct FusedLayout {
-    uint32_t x32Offset, regionOffset, regionAux, partialOffset, downOffset, slotsOffset, rowsBytes, pairBytes, tripleBytes, downBytes;
+    uint32_t regionOffset, regionAux, actsAux, partialOffset, downOffset, slotsOffset, rowsBytes, pairBytes, tripleBytes, downBytes;
     uint32_t strideGU, strideGUA, strideSD, strideRD;
     size_t total;
 };
@@ -854,24 +862,71 @@ static FusedLayout fused_layout(const FFConfig &c) {
     l.strideGUA = piece_stride(longest(groupsD, 4) * 32);  // shared tiles: K quarters
     l.strideSD = Fs ? piece_stride(longest(groupsFs, 3) * 32) : 32;
     l.strideRD = piece_stride(groupsF * 32);
-    l.x32Offset = up128(D * 4 + groupsD * (uint32_t)sizeof(GroupAux));
-    l.regionOffset = up128(l.x32Offset + (D + 255) / 256 * 1024);
-    // the region holds the shared activations' digits, then K (even) rows of routed ones
+    // x and the shared activations, with their aux; in their place, later, K (even) rows of routed ones
+    l.regionOffset = up128(D * 4 + groupsD * (uint32_t)sizeof(GroupAux));
+    l.regionAux = l.regionOffset + Fs * 4;
     const uint32_t rows = (K + 1) / 2 * 2;
-    l.regionAux = l.regionOffset + std::max(Fs * 4, rows * F * 4);
-    l.partialOffset = up128(l.regionAux + (uint32_t)sizeof(GroupAux) * (std::max(groupsFs, rows * ((groupsF + 1) & ~1u)) + 2));
+    l.actsAux = rows * F * 4;
+    l.partialOffset = up128(std::max(l.regionAux + (uint32_t)sizeof(GroupAux) * (groupsFs + 2),
+                                     l.actsAux + (uint32_t)sizeof(GroupAux) * (rows * ((groupsF + 1) & ~1u) + 2)));
     l.downOffset = l.partialOffset + kFusedWarps * 16 * 4;
     l.slotsOffset = up128(l.downOffset + kFusedWarps * 8 * 8 * 4);
     l.downBytes = up128(16 * l.strideRD + 64 * padded_groups(groupsF));
     l.rowsBytes = up128(std::max({16 * l.strideGU, 16 * l.strideGUA, l.downBytes}));
-    l.pairBytes = up128(2 * l.rowsBytes + 64 * padded_groups(groupsD));
+    l.pairBytes = up128(std::max(2 * l.rowsBytes + 64 * padded_groups(groupsD), (D + 255) / 256 * 1024));  // x as fp32, too
     l.tripleBytes = up128(std::max(Fs ? 48 * l.strideSD + 64 * padded_groups(groupsFs) : 0u, 3 * l.downBytes));
     l.total = (size_t)l.slotsOffset + (size_t)(kBigWarps / 2) * l.pairBytes + 2 * (size_t)l.tripleBytes;
     return l;
 }
 
+// Whether the fused kernel's shared memory (its static arrays included) and its row boxes hold the shape.
+bool decode_fused_fits(const FFConfig &c) {
+    static const size_t staticBytes = [] {
+        size_t most = 0;
+        cudaFuncAttributes f{};
+        for (const void *k : {reinterpret_cast<const void *>(k_decode_fused), reinterpret_cast<const void *>(k_decode_fused_inline_x)})
+            most = std::max(most, cudaFuncGetAttributes(&f, k) == cudaSuccess ? f.sharedSizeBytes : (size_t)4096);
+        return most;
+    }();
+    const FusedLayout l = fused_layout(c);
+    return l.total + staticBytes <= 227 * 1024 && std::max({l.strideGU, l.strideGUA, l.strideSD, l.strideRD}) <= 2048;
+}
+
+// y = bf16(residual + sum_k w_k v_k) of one row, in rank order as the fused kernel adds.
+__global__ void __launch_bounds__(256)
+k_combine_values(const float *values, const uint32_t *ids, const uint16_t *weights, const uint16_t *residual, int D, int K,
+                 int expertCount, uint16_t *y) {
+    pdl_enter();
+    const int row = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (row >= D) return;
+    float acc = residual ? bf2f(residual[row]) : 0.0f;
+    for (int k = 0; k < K; ++k)  // (a route past the experts has no values: weight 0, as in the fused kernel)
+        if (ids[k] < (uint32_t)expertCount) acc = __fadd_rn(acc, __fmul_rn(bf2f(weights[k]), values[(size_t)k * D + row]));
+    y[row] = f2bf(acc);
+}
+
+// The same step as separate launches (router, block kernels with fp32 output rows, combine), for the shapes whose
+// rows and slots are too large for one CTA's shared memory: 2880 x 1024 with a shared width of 2112, for instance.
+static bool launch_decode_general(FFContext *ctx, const LayerStore &L, const uint16_t *x, const uint32_t *idsIn,
+                                  const uint16_t *weightsIn, bool withShared, bool routed, const uint16_t *residual,
+                                  uint16_t *y, cudaStream_t stream, const char **error) {
+    const FFConfig &c = ctx->cfg;
+    if (!routed) return launch_block_int4(ctx, L, x, c.d, 1, nullptr, true, nullptr, y, stream, error);
+    if (!idsIn) {
+        if (!launch_router_topk(ctx, L, x, c.d, 1, ctx->ids, ctx->weights, nullptr, stream, error)) return false;
+        idsIn = ctx->ids;
+        weightsIn = ctx->weights;
+    }
+    if (!launch_block_int4(ctx, L, x, c.d, 1, idsIn, withShared, nullptr, ctx->h1, stream, error, ctx->decodeValues)) return false;
+    LaunchScope scope(ctx, stream, "combine_values");
+    FF_CUDA_OK(launch_pdl(k_combine_values, (c.d + 255) / 256, 256, 0, stream, ctx->decodeValues, idsIn, weightsIn,
+                          withShared ? ctx->h1 : residual, (int)c.d, (int)c.topK, (int)L.expertCount, y),
+               error);
+    return true;
+}
+
 // One decode row through router (unless ids are given), routed experts and the shared FFN (or
-// the caller's residual), as one cooperative launch.  routed = false: the shared FFN alone, y
+// the caller's residual), as one cooperative launch where the shape fits.  routed = false: the shared FFN alone, y
 // receives its output.
 bool launch_decode_fused(FFContext *ctx, const LayerStore &L, const uint16_t *x, const uint32_t *idsIn,
                          const uint16_t *weightsIn, bool withShared, bool routed, const uint16_t *residual,
@@ -929,14 +984,16 @@ bool launch_decode_fused(FFContext *ctx, const LayerStore &L, const uint16_t *x,
     if (a.E > kMaxExperts) return fail(error, "too many experts for the decode kernel");
     const FusedLayout lay = fused_layout(c);
     const size_t smem = lay.total;
-    if (smem > 227 * 1024)
-        return fail(error, "model shape too large for the fused decode kernel's shared memory");
     // bulk copies need 16-byte aligned sources: every sub-tensor offset and the blob stride
     const uint32_t *ro = &L.off.gateWOff, *so = &L.sharedOff.gateWOff;
     for (int i = 0; i < 9; ++i)
         if ((routed && (ro[i] % 16 || L.stride % 16)) || (withShared && so[i] % 16))
             return fail(error, "sub-tensor offsets must be multiples of 16 bytes for the decode kernel");
     if (!(host && host->inlineX) && ((uintptr_t)x & 15) != 0) return fail(error, "input row must be 16-byte aligned");
+    if (!decode_fused_fits(c)) {
+        if (host) return fail(error, "the host hand-off needs the fused decode kernel");
+        return launch_decode_general(ctx, L, x, idsIn, weightsIn, withShared, routed, residual, y, stream, error);
+    }
     // row-box tensor maps of the layer, built once per loaded layer
     LayerStore &Lm = const_cast<LayerStore &>(L);
     if (!Lm.decodeMapsReady) {
@@ -965,9 +1022,9 @@ bool launch_decode_fused(FFContext *ctx, const LayerStore &L, const uint16_t *x,
     }
     static thread_local DecodeMaps maps;
     memcpy(maps.m, L.decodeMap, sizeof(maps.m));
-    a.x32Offset = lay.x32Offset;
     a.regionOffset = lay.regionOffset;
     a.regionAux = lay.regionAux;
+    a.actsAux = lay.actsAux;
     a.partialOffset = lay.partialOffset;
     a.downOffset = lay.downOffset;
     a.slotsOffset = lay.slotsOffset;

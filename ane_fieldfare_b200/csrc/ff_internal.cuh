@@ -167,6 +167,7 @@ struct FFContext {
     uint16_t *sharedActs = nullptr; // [maxTokens][sharedF]
     uint16_t *h1 = nullptr;         // [maxTokens][d]
     uint16_t *partials = nullptr;   // [maxTokens*topK][d]
+    float *decodeValues = nullptr;  // [topK][d] one row's routed outputs, where the shape does not fit the fused decode kernel
     uint16_t *xDev = nullptr;       // [maxTokens][d] staging for *_host
     uint16_t *yDev = nullptr;
 
@@ -298,7 +299,7 @@ bool make_row_box_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_
 // ff_block.cu
 bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens,
                        const uint32_t *ids, bool withShared, uint16_t *partials, uint16_t *sharedOut, cudaStream_t stream,
-                       const char **error);
+                       const char **error, float *values = nullptr);
 bool launch_block_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens, uint16_t *y,
                        cudaStream_t stream, const char **error);
 
@@ -311,6 +312,7 @@ struct DecodeHostHandoff {
     unsigned long long *mailbox;
     uint32_t epoch;
 };
+bool decode_fused_fits(const FFConfig &c);  // else launch_decode_fused takes the general kernels (no host hand-off)
 bool launch_decode_fused(FFContext *ctx, const LayerStore &L, const uint16_t *x, const uint32_t *idsIn,
                          const uint16_t *weightsIn, bool withShared, bool routed, const uint16_t *residual,
                          uint16_t *y, cudaStream_t stream, const char **error,
