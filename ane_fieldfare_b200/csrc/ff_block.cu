@@ -33,7 +33,7 @@ namespace ff {
 namespace {
 
 constexpr int kMaxWarps = 16;
-constexpr int kTaskRows = 4;          // input rows of a task
+constexpr int kTaskRows = 4;          // input rows of a task (2 where the rows are too wide for four as digits)
 constexpr uint32_t kPartGroups = 8;   // groups of a part along K, a multiple of four
 constexpr int kMaxJobs = kMaxGemvRows * 8 + 1;
 
@@ -60,6 +60,7 @@ struct BlockArgs {
     uint32_t *errorFlag;
     uint32_t listOffset, digitsOffset, rowBytes, auxOffset, auxRow, slotsOffset, slotBytes, sbOffset;
     int perExpert;            // routes of one expert at most
+    int taskShift;            // log2 of a task's input rows
     float *values;            // F32OUT: the routed rows
 };
 
@@ -226,10 +227,11 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
     }
     __syncthreads();
     // instructions of a tile: per group what the weights cost and what a pair of rows costs, and its set-up
+    const uint32_t taskRows = 1u << a.taskShift;
     auto tile_cost = [&](int kind, int rows) { return a.kind[kind].groups * (rows > 2 ? 31u : 22u) + 100u; };
     auto job_cost = [&](int kind, int rows) {
-        const uint32_t full = (uint32_t)rows / kTaskRows, rest = (uint32_t)rows % kTaskRows;
-        return a.kind[kind].tiles * (full * tile_cost(kind, kTaskRows) + (rest ? tile_cost(kind, (int)rest) : 0u));
+        const uint32_t full = (uint32_t)rows >> a.taskShift, rest = (uint32_t)rows & (taskRows - 1u);
+        return a.kind[kind].tiles * (full * tile_cost(kind, (int)taskRows) + (rest ? tile_cost(kind, (int)rest) : 0u));
     };
     uint32_t nJobs = a.withShared ? 1u : 0u;
     {
@@ -295,11 +297,11 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
             else hi = mid;
         }
         const int kind = kind_of(lo), rows = rows_of(lo);
-        const uint32_t tiles = a.kind[kind].tiles, full = (uint32_t)rows / kTaskRows;
-        uint32_t cost = tile_cost(kind, kTaskRows), rest = target - sFirst[lo];
+        const uint32_t tiles = a.kind[kind].tiles, full = (uint32_t)rows >> a.taskShift;
+        uint32_t cost = tile_cost(kind, (int)taskRows), rest = target - sFirst[lo];
         const uint32_t rg = min(full, rest / (tiles * cost));
         rest -= rg * tiles * cost;
-        if (rg == full) cost = tile_cost(kind, rows % kTaskRows);
+        if (rg == full) cost = tile_cost(kind, (int)((uint32_t)rows & (taskRows - 1u)));
         return Place{lo, rg, (rest + cost - 1u) / cost};  // (may be one past the row group's last tile)
     };
     auto before = [](const Place &p, const Place &q) {
@@ -310,7 +312,7 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
             const uint32_t tiles = a.kind[kind_of(p.job)].tiles;
             if (p.tile < tiles) break;
             p.tile -= tiles;
-            if ((int)(++p.rowGroup * kTaskRows) >= rows_of(p.job)) {
+            if ((int)(++p.rowGroup << a.taskShift) >= rows_of(p.job)) {
                 p.rowGroup = 0;
                 ++p.job;
             }
@@ -442,11 +444,11 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
     uint32_t used = 0, done = 0;  // done: tiles of this CTA's earlier segments, modulo the warps
     while (before(at, end)) {
         // a segment: the run's tiles of one row group
-        const int kind = kind_of(at.job), n = min(kTaskRows, rows_of(at.job) - (int)at.rowGroup * kTaskRows);
+        const int kind = kind_of(at.job), n = min((int)taskRows, rows_of(at.job) - (int)(at.rowGroup << a.taskShift));
         const BlockKind &k = a.kind[kind];
         const bool same = at.job == end.job && at.rowGroup == end.rowGroup;
         const uint32_t tileEnd = same ? end.tile : k.tiles;
-        const uint32_t listAt = kind ? (sJob[at.job] - 1u) * kMaxGemvRows + at.rowGroup * kTaskRows : at.rowGroup * kTaskRows;
+        const uint32_t listAt = kind ? (sJob[at.job] - 1u) * kMaxGemvRows + (at.rowGroup << a.taskShift) : at.rowGroup << a.taskShift;
         auto row_of = [&](int i) { return kind ? (int)sList[listAt + (uint32_t)i] : (int)listAt + i; };  // row i: its route or token
         __syncthreads();  // the previous segment's digits are no longer read
         stage(k, kind, n, row_of);
@@ -608,19 +610,24 @@ bool launch_kernel(FFContext *ctx, BlockArgs a, const BlockMaps &maps, const cha
         sb = std::max(sb, 64 * a.kind[i].sbWords);
     }
     auto up128 = [](uint32_t v) { return (v + 127u) & ~127u; };
-    const uint32_t rows = (uint32_t)std::min(std::max(a.T, a.perExpert), kTaskRows), padded = padded_groups(groups);
-    a.listOffset = 0;
-    a.digitsOffset = a.ids ? up128((uint32_t)a.E * kMaxGemvRows) : 0;
-    a.rowBytes = padded * kDigitGroupBytes;
-    a.auxOffset = a.digitsOffset + rows * a.rowBytes;
-    // INT8: a row's group entries; INT4: a pair's group sums
-    a.auxRow = INT8 ? padded * (uint32_t)sizeof(GroupAux) : (groups + 7u) / 8u * kSumBlockBytes;
-    a.slotsOffset = up128(a.auxOffset + (INT8 ? rows : (rows + 1u) / 2u) * a.auxRow);
+    const uint32_t padded = padded_groups(groups);
     a.sbOffset = up128(slot);
     a.slotBytes = a.sbOffset + up128(sb);
     // (a batch of four groups may read up to three groups past a slot's last row, within the scale area)
     constexpr uint32_t kLimit = 227 * 1024 - 6144;  // less the static arrays
-    if (a.slotsOffset + 4 * 2 * a.slotBytes > kLimit) return fail(error, "model shape too large for the block kernels' shared memory");
+    a.listOffset = 0;
+    a.digitsOffset = a.ids ? up128((uint32_t)a.E * kMaxGemvRows) : 0;
+    a.rowBytes = padded * kDigitGroupBytes;
+    // INT8: a row's group entries; INT4: a pair's group sums
+    a.auxRow = INT8 ? padded * (uint32_t)sizeof(GroupAux) : (groups + 7u) / 8u * kSumBlockBytes;
+    // four input rows a task; two where four leave no room for four warps' slots (widths from 11072 on)
+    for (a.taskShift = 2; a.taskShift >= 1; --a.taskShift) {
+        const uint32_t rows = (uint32_t)std::min(std::max(a.T, a.perExpert), 1 << a.taskShift);
+        a.auxOffset = a.digitsOffset + rows * a.rowBytes;
+        a.slotsOffset = up128(a.auxOffset + (INT8 ? rows : (rows + 1u) / 2u) * a.auxRow);
+        if (a.slotsOffset + 4 * 2 * a.slotBytes <= kLimit) break;
+    }
+    if (a.taskShift == 0) return fail(error, "model shape too large for the block kernels' shared memory");
     const uint32_t warps = std::min<uint32_t>(kMaxWarps, (kLimit - a.slotsOffset) / (2 * a.slotBytes));
     const size_t smem = a.slotsOffset + (size_t)warps * 2 * a.slotBytes;
     static KernelSmemMemo memo;

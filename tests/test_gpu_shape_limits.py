@@ -73,3 +73,20 @@ def test_one_row(oracle, d, f, fs, k, launches):
         assert np.linalg.norm(got - only) <= 1e-2 * np.linalg.norm(only)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("d,f,fs,k", [(64, 11072, 0, 2), (64, 64, 21376, 2), (128, 16384, 11136, 3)])
+@pytest.mark.parametrize("rows", [2, 3, 5, 16])
+def test_wide_blocks(oracle, d, f, fs, k, rows):
+    """Widths whose rows fit as digits two at a time, not four."""
+    L = workload.make_layer(0x83, 0, experts=6, d=d, f=f, sharedF=fs, topK=k)
+    hp, ctx = context(L, 16)
+    try:
+        x = workload.make_tokens(0x84, f"wide{rows}", rows, d)
+        y = ctx.moeLayer(0, hp.bf16_tensor(x, ctx.device))
+        torch.cuda.synchronize()
+        assert ctx.info().deviceErrorFlag == 0
+        want, *_ = oracle.moe_layer(oracle_layer(oracle, L), x, oracle.MODE_PARTIALS)
+        assert_layer_close(hp.bf16_numpy(y), want, oracle, f"wide block {d}x{f}+{fs} rows={rows}")
+    finally:
+        ctx.close()
