@@ -87,7 +87,7 @@ void ff_destroy(FFContext *ctx) {
                     ctx->partials, ctx->xDev, ctx->yDev, ctx->xSorted, ctx->xShared, ctx->rowOfRoute, ctx->sortedPairs,
                     ctx->expertOffsets, ctx->blockCounts, ctx->units, ctx->unitCount,
                     ctx->errorFlag, ctx->gridBarrier, ctx->phaseStamps, ctx->mapScratch, ctx->taggedLogits, ctx->taggedActs,
-                    ctx->logitsRows, ctx->routeIds, ctx->routeWeights, ctx->xSums, ctx->actSums, ctx->routerParts, ctx->decodeValues};
+                    ctx->logitsRows, ctx->xSums, ctx->actSums, ctx->routerParts, ctx->decodeValues};
     for (void *p : ptrs) cudaFree(p);
     if (ctx->hostStream) cudaStreamDestroy(ctx->hostStream);
     if (ctx->sideStream) cudaStreamDestroy(ctx->sideStream);
@@ -498,13 +498,10 @@ bool ff_load_router_int8(FFContext *ctx, uint32_t layer, const uint8_t *codes, c
         return false;
     L.routerExperts = experts;
     ctx->weightBytes += (size_t)experts * d + groups * 4;
-    // scratch of the INT8 router: logits of every row, and the one-token path's routes
-    if (!ctx->logitsRows) {
+    // scratch of the INT8 router: logits of every row
+    if (!ctx->logitsRows)
         FF_CUDA_OK(cudaMalloc(reinterpret_cast<void **>(&ctx->logitsRows),
                               (size_t)ctx->cfg.maxTokens * kMaxExperts * sizeof(float)), error);
-        FF_CUDA_OK(cudaMalloc(reinterpret_cast<void **>(&ctx->routeIds), (size_t)ctx->cfg.topK * sizeof(uint32_t)), error);
-        FF_CUDA_OK(cudaMalloc(reinterpret_cast<void **>(&ctx->routeWeights), (size_t)ctx->cfg.topK * sizeof(uint16_t)), error);
-    }
     return router_prepare(ctx, L, error);
 }
 

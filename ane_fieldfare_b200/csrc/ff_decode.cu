@@ -939,10 +939,10 @@ bool launch_decode_fused(FFContext *ctx, const LayerStore &L, const uint16_t *x,
         // front (logits, top-K), and the kernel takes the routes as given.
         if (host) return fail(error, "the host hand-off needs a bf16 router");
         if (L.routerExperts != L.expertCount) return fail(error, "router and layer disagree on the expert count");
-        if (!launch_router_topk(ctx, L, x, ctx->cfg.d, 1, ctx->routeIds, ctx->routeWeights, nullptr, stream, error))
+        if (!launch_router_topk(ctx, L, x, ctx->cfg.d, 1, ctx->ids, ctx->weights, nullptr, stream, error))
             return false;
-        idsIn = ctx->routeIds;
-        weightsIn = ctx->routeWeights;
+        idsIn = ctx->ids;
+        weightsIn = ctx->weights;
     }
     if (withShared && !L.shared) return fail(error, "layer has no resident shared FFN");
     if (!routed && !withShared) return fail(error, "nothing to compute");

@@ -157,8 +157,6 @@ struct FFContext {
     // decode / verify scratch
     float *logits = nullptr;        // [min(maxTokens,16)][experts]
     float *logitsRows = nullptr;    // [maxTokens][experts], allocated with the first INT8 router
-    uint32_t *routeIds = nullptr;   // [topK] routes of the one-token path when the router runs as its own launch
-    uint16_t *routeWeights = nullptr;
     uint32_t *ids = nullptr;        // [maxTokens][topK]
     uint16_t *weights = nullptr;    // [maxTokens][topK]
     ff::RoutePlan *plan = nullptr;

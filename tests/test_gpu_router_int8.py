@@ -117,6 +117,32 @@ def test_operators_take_the_int8_router(oracle, rows):
         ctx.close()
 
 
+@pytest.mark.parametrize("rows", [1, 5, 40])
+def test_layer_reports_the_int8_routers_routes(oracle, rows):
+    hp = _hp()
+    shape = SHAPES[0]
+    E, D, K = shape["experts"], shape["d"], shape["topK"]
+    L = workload.make_layer(0x1A, 0, **shape)
+    codes, scales, biases = int8_router(0x1A, E, D)
+    ctx = hp.HotpathContext(layers=1, maxTokens=64, **shape)
+    try:
+        ctx.loadLayer(0, L.blobs, L.layout.stride, L.layout.offsets)
+        ctx.loadShared(0, *L.shared_projections())
+        ctx.loadRouterInt8(0, codes, scales, biases)
+        for i in range(2):  # not those of an earlier call
+            x = workload.make_tokens(0x1A, f"int8.routes{rows}.{i}", rows, D)
+            ids = torch.full((rows, K), -1, dtype=torch.int32, device=ctx.device)
+            w = torch.zeros((rows, K), dtype=torch.bfloat16, device=ctx.device)
+            ctx.moeLayer(0, dev(x, ctx), ids=ids, weights=w)
+            torch.cuda.synchronize()
+            ref_ids, ref_w, _ = oracle.router_topk_int8(codes, scales, biases, x, K)
+            assert np.array_equal(ids.cpu().numpy().astype(np.uint32), ref_ids)
+            dw = np.abs(oracle.bf16_to_float(hp.bf16_numpy(w)) - oracle.bf16_to_float(ref_w))
+            assert dw.max() < 5e-3  # (another exp: the bound of the routers' other tests)
+    finally:
+        ctx.close()
+
+
 def test_int8_router_refusals():
     hp = _hp()
     shape = SHAPES[0]
