@@ -60,7 +60,7 @@ static void free_layer(LayerStore &L) {
     cudaFree(L.routerQScale);
     cudaFree(L.routerQBias);
     cudaFree(L.routerFolded);
-    cudaFree(L.routerCoef);
+    cudaFree(L.routerBounds);
     cudaFree(L.routerLanes);
     cudaFree(L.routerAux);
     cudaFree(L.routerW);
@@ -405,11 +405,11 @@ static void free_router(ff::LayerStore &L) {
     cudaFree(L.routerQScale);
     cudaFree(L.routerQBias);
     cudaFree(L.routerFolded);
-    cudaFree(L.routerCoef);
+    cudaFree(L.routerBounds);
     cudaFree(L.routerLanes);
     cudaFree(L.routerAux);
     L.routerFolded = nullptr;
-    L.routerCoef = nullptr;
+    L.routerBounds = nullptr;
     L.routerLanes = nullptr;
     L.routerAux = nullptr;
     L.routerW = L.routerScale = L.gain = L.routerQScale = L.routerQBias = nullptr;

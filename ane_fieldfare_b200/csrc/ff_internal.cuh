@@ -100,6 +100,12 @@ struct RoutePlan {
     uint32_t pad[3];
 };
 
+// How far an exact logit (without its bias) can be from its approximation on the tensor cores: perNorm |x| + floor,
+// for rows of |x| < limit (see ff_router.cu).
+struct RouterBound {
+    float perNorm, floor, limit;
+};
+
 struct LayerStore {
     uint8_t *experts = nullptr;  // expertCount blobs, stride apart (a layer file, verbatim)
     uint64_t stride = 0;
@@ -118,9 +124,9 @@ struct LayerStore {
     uint8_t *routerQ = nullptr;
     uint16_t *routerQScale = nullptr, *routerQBias = nullptr;
     // for a prefill chunk's routes: the weights as the tensor cores multiply them (null: routerW), and a
-    // bound of each approximate logit's error per unit of the row's 2-norm
+    // bound of each approximate logit's error
     uint16_t *routerFolded = nullptr;
-    float *routerCoef = nullptr;
+    RouterBound *routerBounds = nullptr;
     uint16_t *routerLanes = nullptr;  // INT8 router rows in lane order, and their scales | biases
     uint32_t *routerAux = nullptr;
     bool has_router() const { return routerW != nullptr || routerQ != nullptr; }

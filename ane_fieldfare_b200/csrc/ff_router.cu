@@ -11,9 +11,11 @@
 //      and ranks them.
 // The bound holds for any data: with unspecified rounding at single precision or better, a sum of n
 // products is within n 2^-23 sum|w x| of its value (the fixed-order sum likewise, with its own n), a
-// folded weight bf16(w * scale) within 2^-9 |w scale|, and sum|w x| <= |w| |x| in 2-norms.  Experts
-// whose bound is not finite (NaN or infinity in the row) are always kept, so at worst every logit is
-// formed exactly, as before.
+// folded weight bf16(w * scale) within 2^-9 |w scale|, and sum|w x| <= |w| |x| in 2-norms.  The norms are
+// formed where squares neither vanish nor overflow.  What underflows, flushed to zero or not, adds at most
+// 2^-126 per operation and operand (RouterBound::floor, and a part of perNorm); rows so large that a term
+// or a partial sum could overflow in some order (RouterBound::limit), or that hold a NaN or an infinity, keep
+// every expert, so at worst every logit is formed exactly.
 //
 // Rows of 2816 inputs, 128 experts: 4096 rows 160 -> 60 us (15 + 37 between launches), 32768 rows 1158 ->
 // 280 us; INT8, 2000 rows: 264 -> 65 us.  Bound by the latency and the L2 traffic of the exact logits
@@ -196,7 +198,8 @@ struct SelectArgs {
     const uint4 *Q;                  // INT8 router in lane order (see k_router_int8_lanes)
     const uint32_t *qAux;
     const uint16_t *scale, *gain;    // per input, per expert; or null
-    const float *bias, *coef;        // logit bias or null; error bound of a logit per unit of |x|
+    const float *bias;               // logit bias or null
+    const RouterBound *bounds;       // [E]
     const uint16_t *x;
     uint32_t xStride, splits, warpsPerRow;
     int T, E, D, K;
@@ -331,20 +334,26 @@ k_router_select(const SelectArgs a) {
         }
     }
     if (live && sub == 0) {
-        float sq = 0.0f;
-        for (int i = lane; i < (a.D >> 3); i += 32) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(xr) + i);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        auto square_sum = [&](float scale) {
+            float sq = 0.0f;
+            for (int i = lane; i < (a.D >> 3); i += 32) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4 *>(xr) + i);
+                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float lo = __uint_as_float(w[k] << 16), hi = __uint_as_float(w[k] & 0xFFFF0000u);
-                sq = fmaf(lo, lo, sq);
-                sq = fmaf(hi, hi, sq);
+                for (int k = 0; k < 4; ++k) {
+                    const float lo = __uint_as_float(w[k] << 16) * scale, hi = __uint_as_float(w[k] & 0xFFFF0000u) * scale;
+                    sq = fmaf(lo, lo, sq);
+                    sq = fmaf(hi, hi, sq);
+                }
             }
-        }
 #pragma unroll
-        for (int offset = 16; offset >= 1; offset >>= 1) sq += __shfl_xor_sync(0xFFFFFFFFu, sq, offset);
-        const float norm = sqrtf(sq) * 1.01f + 1e-30f;
+            for (int offset = 16; offset >= 1; offset >>= 1) sq += __shfl_xor_sync(0xFFFFFFFFu, sq, offset);
+            return sq;
+        };
+        // (below 2^-100 the squares lose digits or vanish: every |x| is below 2^-50 then, so 2^100 times the row has
+        // squares from 2^-66 to 2^100)
+        const float sq = square_sum(1.0f);
+        const float norm = sq < 0x1p-100f ? sqrtf(square_sum(0x1p100f)) * 1.01f * 0x1p-100f : sqrtf(sq) * 1.01f;
 
         // the K-th largest lower bound; an expert whose upper bound reaches it can be among the K largest
         uint32_t low[8];
@@ -356,11 +365,13 @@ k_router_select(const SelectArgs a) {
             high[j] = -INFINITY;
             if (e < E) {
                 const float l = a.bias ? approx[j] + a.bias[e] : approx[j];
-                const float eps = fmaf(a.coef[e], norm, fabsf(l) * 2.5e-7f);
+                const RouterBound bound = a.bounds[e];
+                const float eps = fmaf(bound.perNorm, norm, fmaf(fabsf(l), 2.5e-7f, bound.floor));
                 const float lo = l - eps, hi = l + eps;
-                const bool bounded = lo > -INFINITY && hi < INFINITY;  // false for NaN, too
+                const bool bounded = norm < bound.limit && lo > -INFINITY && hi < INFINITY;  // false for NaN, too
                 low[j] = bounded ? ordered_key(lo) : 0u;
-                high[j] = bounded || l == -INFINITY ? hi : INFINITY;
+                // (a bias of -inf makes a logit that is never taken, whatever the sum)
+                high[j] = bounded ? hi : a.bias && a.bias[e] == -INFINITY ? -INFINITY : INFINITY;
             }
         }
         uint32_t threshold = 0u, gone = 0u;
@@ -511,48 +522,66 @@ k_router_logits_int8(const uint4 *Q, const uint32_t *aux, const uint16_t *effSca
 
 // ---- at load: folded bf16 weights and the bound's coefficients --------------------------------------
 
-// One CTA per expert.  folded = bf16(w * scale) (null: the router's own bf16 rows are multiplied).
+// One CTA per expert.  folded = bf16(w * scale) (null: the router's own bf16 rows are multiplied).  Norms in
+// double: the squares of any product of two bf16 values are normal numbers there.
 __global__ void __launch_bounds__(256)
 k_router_prepare(const uint16_t *W, const uint8_t *Q, const uint16_t *qScale, const uint16_t *qBias, const uint16_t *scale,
-                 int D, uint16_t *folded, float *coef) {
-    __shared__ float sums[2][8];
+                 int D, uint16_t *folded, RouterBound *bounds) {
+    __shared__ double sums[4][8];
     const int e = blockIdx.x;
-    float sq = 0.0f, sqTerms = 0.0f;  // |w scale|^2, and of the terms the fixed order adds
+    // |w scale|^2, |the terms the fixed order adds|^2, sum |w|, and the largest factor of an input in either order
+    double sq = 0.0, sqTerms = 0.0, sumW = 0.0, factor = Q ? 255.0 : 1.0;
     for (int i = threadIdx.x; i < D; i += blockDim.x) {
-        const float f = scale ? bf2f(scale[i]) : 1.0f;
-        float w, terms;
+        const double f = scale ? (double)bf2f(scale[i]) : 1.0;
+        double w, terms, plain;
         if (Q) {
-            const float q = (float)Q[(size_t)e * D + i], s = bf2f(qScale[(size_t)e * (D / 64) + i / 64]),
-                        b = bf2f(qBias[(size_t)e * (D / 64) + i / 64]);
-            w = fmaf(q, s, b) * f;
-            terms = (q * fabsf(s) + fabsf(b)) * fabsf(f);
+            const double q = (double)Q[(size_t)e * D + i], s = (double)bf2f(qScale[(size_t)e * (D / 64) + i / 64]),
+                         b = (double)bf2f(qBias[(size_t)e * (D / 64) + i / 64]);
+            w = fma(q, s, b) * f;
+            plain = q * fabs(s) + fabs(b);
+            terms = plain * fabs(f);
+            factor = fmax(factor, 255.0 * fabs(f));
         } else {
-            w = bf2f(W[(size_t)e * D + i]) * f;
-            terms = fabsf(w);
+            plain = fabs((double)bf2f(W[(size_t)e * D + i]));
+            w = (double)bf2f(W[(size_t)e * D + i]) * f;
+            terms = fabs(w);
+            factor = fmax(factor, fabs(f));
         }
-        if (folded) folded[(size_t)e * D + i] = f2bf(w);
-        sq = fmaf(w, w, sq);
-        sqTerms = fmaf(terms, terms, sqTerms);
+        if (folded) folded[(size_t)e * D + i] = f2bf((float)w);
+        sq = fma(w, w, sq);
+        sqTerms = fma(terms, terms, sqTerms);
+        sumW += plain + fabs(w);
     }
 #pragma unroll
     for (int offset = 16; offset >= 1; offset >>= 1) {
         sq += __shfl_xor_sync(0xFFFFFFFFu, sq, offset);
         sqTerms += __shfl_xor_sync(0xFFFFFFFFu, sqTerms, offset);
+        sumW += __shfl_xor_sync(0xFFFFFFFFu, sumW, offset);
+        factor = fmax(factor, __shfl_xor_sync(0xFFFFFFFFu, factor, offset));
     }
     if ((threadIdx.x & 31) == 0) {
         sums[0][threadIdx.x >> 5] = sq;
         sums[1][threadIdx.x >> 5] = sqTerms;
+        sums[2][threadIdx.x >> 5] = sumW;
+        sums[3][threadIdx.x >> 5] = factor;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        float total = 0.0f, totalTerms = 0.0f;
-        for (int i = 0; i < 8; ++i) {
-            total += sums[0][i];
-            totalTerms += sums[1][i];
+        for (int i = 1; i < 8; ++i) {
+            sq += sums[0][i];
+            sqTerms += sums[1][i];
+            sumW += sums[2][i];
+            factor = fmax(factor, sums[3][i]);
         }
-        const float u = 1.1920929e-7f;  // 2^-23
-        const float chain = (float)(Q ? 4 * (D / 64) + 16 : 8 * ((D + 255) / 256) + 16);
-        coef[e] = 1.02f * (sqrtf(total) * ((float)(D + 16) * u + (folded ? 2.1e-3f : 0.0f)) + sqrtf(totalTerms) * chain * u);
+        const double u = 0x1p-23, tiny = 0x1p-126;
+        const double chain = (double)(Q ? 4 * (D / 64) + 16 : 8 * ((D + 255) / 256) + 16);
+        RouterBound b;
+        // (an input of a flushed weight: tiny |x| summed over the row, at most tiny sqrt(D) |x| in the 2-norm)
+        b.perNorm = (float)(1.02 * (sqrt(sq) * ((D + 16) * u + (folded ? 2.1e-3 : 0.0)) + sqrt(sqTerms) * chain * u) +
+                            2.0 * tiny * sqrt((double)D));
+        b.floor = (float)(tiny * (4.0 * D + 2.0 * sumW));  // products and sums; inputs and scaled inputs, times their weights
+        b.limit = (float)(0x1p120 / fmax(factor, sqrt(sqTerms)));
+        bounds[e] = b;
     }
 }
 
@@ -596,14 +625,15 @@ bool router_prepare(FFContext *ctx, LayerStore &L, const char **error) {
     const int E = (int)L.routerExperts, D = (int)ctx->cfg.d;
     if (L.routerQ || L.routerScale)
         FF_CUDA_OK(cudaMalloc(reinterpret_cast<void **>(&L.routerFolded), (size_t)E * D * 2), error);
-    FF_CUDA_OK(cudaMalloc(reinterpret_cast<void **>(&L.routerCoef), (size_t)E * 4), error);
+    FF_CUDA_OK(cudaMalloc(reinterpret_cast<void **>(&L.routerBounds), (size_t)E * sizeof(RouterBound)), error);
     if (L.routerQ) {
         const size_t padded = ((size_t)(D / 64) + 7) / 8 * 8;
         FF_CUDA_OK(cudaMalloc(reinterpret_cast<void **>(&L.routerLanes), (size_t)E * padded * 64), error);
         FF_CUDA_OK(cudaMalloc(reinterpret_cast<void **>(&L.routerAux), (size_t)E * padded * 4), error);
         k_router_int8_lanes<<<E, 256>>>(L.routerQ, L.routerQScale, L.routerQBias, D, L.routerLanes, L.routerAux);
     }
-    k_router_prepare<<<E, 256>>>(L.routerW, L.routerQ, L.routerQScale, L.routerQBias, L.routerScale, D, L.routerFolded, L.routerCoef);
+    k_router_prepare<<<E, 256>>>(L.routerW, L.routerQ, L.routerQScale, L.routerQBias, L.routerScale, D, L.routerFolded,
+                                  L.routerBounds);
     FF_CUDA_OK(cudaGetLastError(), error);
     FF_CUDA_OK(cudaStreamSynchronize(nullptr), error);
     return true;
@@ -642,7 +672,7 @@ bool launch_router_select(FFContext *ctx, const LayerStore &L, const uint16_t *x
     a.scale = L.routerScale;
     a.gain = L.gain;
     a.bias = L.logitBias;
-    a.coef = L.routerCoef;
+    a.bounds = L.routerBounds;
     a.x = x;
     a.xStride = xStride;
     a.splits = splits;

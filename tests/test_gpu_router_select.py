@@ -56,3 +56,45 @@ def test_selected_routes_equal_the_exact_ones(form, experts, d, k, rows):
         assert torch.equal(weights[0].view(torch.int16), weights[1].view(torch.int16))
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("form", ["bf16", "bf16_scaled", "int8"])
+@pytest.mark.parametrize("weights_times", [1.0, 2.0 ** -80, 2.0 ** 60])
+def test_selected_routes_of_tiny_and_huge_rows(form, weights_times):
+    """Without a bias, which would decide the ranks of such rows: rows whose squares vanish or overflow in fp32, whose
+    products underflow, subnormal ones, and rows that mix the scales."""
+    from ane_fieldfare_b200 import hotpath as hp
+    experts, d, k, per = 128, 2816, 8, 12
+    scales = [2.0 ** e for e in (-130, -126, -110, -90, -78, -75, -60, -50, -49, 0, 60, 64, 100, 118)]
+    rows = per * (len(scales) + 1)
+    ctx = hp.HotpathContext(layers=1, experts=experts, d=d, f=64, sharedF=0, topK=k, maxTokens=rows)
+
+    def times(bits):  # by a power of two
+        return synth.bf16_bits(synth.bf16_to_float(bits) * np.float32(weights_times)).reshape(bits.shape)
+
+    try:
+        eff = None if form == "bf16" else synth.bf16_bits(synth.uniform(7, d, 0.5, 1.5))
+        if form == "int8":
+            codes, s, b = int8_router(0x35, experts, d)
+            ctx.loadRouterInt8(0, codes, times(s), times(b), effectiveScale=eff)
+        else:
+            ctx.loadRouter(0, times(synth.normal_bf16(0x36, "tiny.router", (experts, d), 0.02)), effectiveScale=eff)
+        x = synth.bf16_to_float(workload.make_tokens(0x37, "tiny", rows, d)).reshape(rows, d)
+        for i, v in enumerate(scales):
+            x[i * per:(i + 1) * per] *= np.float32(v)
+        mixed = x[len(scales) * per:]
+        mixed *= np.exp2(np.rint(synth.uniform(9, mixed.size, -120, 20))).astype(np.float32).reshape(mixed.shape)
+        xd = hp.bf16_tensor(synth.bf16_bits(x), ctx.device)
+        got = [torch.full((rows, k), -1, dtype=torch.int32, device=ctx.device) for _ in range(2)]
+        weights = [torch.zeros((rows, k), dtype=torch.bfloat16, device=ctx.device) for _ in range(2)]
+        logits = torch.zeros((rows, experts), dtype=torch.float32, device=ctx.device)
+        router = hp.PrefillRouter(ctx)
+        router.encodeGemma4Block(None, 0, xd, got[0], weights[0], rows, outLogits=logits)
+        router.encodeGemma4Block(None, 0, xd, got[1], weights[1], rows)
+        torch.cuda.synchronize()
+        assert ctx.info().deviceErrorFlag == 0
+        wrong = (got[0] != got[1]).any(dim=1).nonzero().flatten().tolist()
+        assert not wrong, wrong
+        assert torch.equal(weights[0].view(torch.int16), weights[1].view(torch.int16))
+    finally:
+        ctx.close()
