@@ -44,7 +44,7 @@ constexpr uint32_t kCodeBytes = 128 * kStepK;
 constexpr uint32_t kOperandCol = kAccs * kMaxRows;
 constexpr int kDrainThreads = 256;
 constexpr int kThreads = (2 + 4 * kDequantGroups) * 32 + kDrainThreads;
-constexpr int kBarriers = 4 * kStages + kOperandStages + 2 * kAccs + 3;
+constexpr int kBarriers = 4 * kStages + 2 * kAccs + 3;
 constexpr uint32_t kXchgPitch = 17;                       // floats per exchanged row (16 + 1)
 constexpr uint32_t kXchgBytes = 128u * kXchgPitch * 4u;   // one half of the tokens
 constexpr uint32_t kTilePitchGateUp = 64 * 2 + 16, kTilePitchDown = 128 * 2 + 16;
@@ -125,29 +125,28 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
 
     const uint32_t barBase = smem_u32(barriers);
     auto barAt = [&](uint32_t i) { return barBase + 8u * i; };
-    auto barTokFull = [&](uint32_t s) { return barAt(s); };
+    auto barStep = [&](uint32_t s) { return barAt(s); };
     auto barTokEmpty = [&](uint32_t s) { return barAt(kStages + s); };
     auto barCodeFull = [&](uint32_t s) { return barAt(2 * kStages + s); };
     auto barCodeEmpty = [&](uint32_t s) { return barAt(3 * kStages + s); };
-    auto barOperand = [&](uint32_t s) { return barAt(4 * kStages + s); };
-    auto barAccFull = [&](uint32_t s) { return barAt(4 * kStages + kOperandStages + s); };
-    auto barAccEmpty = [&](uint32_t s) { return barAt(4 * kStages + kOperandStages + kAccs + s); };
-    auto barHalf = [&](uint32_t h) { return barAt(4 * kStages + kOperandStages + 2 * kAccs + h); };
-    const uint32_t barScales = barAt(4 * kStages + kOperandStages + 2 * kAccs + 2);
+    auto barAccFull = [&](uint32_t s) { return barAt(4 * kStages + s); };
+    auto barAccEmpty = [&](uint32_t s) { return barAt(4 * kStages + kAccs + s); };
+    auto barHalf = [&](uint32_t h) { return barAt(4 * kStages + 2 * kAccs + h); };
+    const uint32_t barScales = barAt(4 * kStages + 2 * kAccs + 2);
 
-    // Barriers that say "ready" to the MMA issuer live in the leader and count both CTAs' arrivals;
-    // barriers that the MMAs' completion frees exist in either CTA (one multicast commit).
+    // What the MMA issuer waits for lives in the leader: a step's barrier counts the arrivals of both CTAs'
+    // dequantizers and the bytes of both CTAs' token copies.  Barriers that the MMAs' completion frees exist
+    // in either CTA (one multicast commit).
     const uint32_t ctaRank = cluster_cta_rank();
     const bool leader = ctaRank == 0u;
     if (threadIdx.x == 0) {
         abortFlag = 0;
         for (uint32_t s = 0; s < kStages; ++s) {
-            mbar_init(barTokFull(s), 1);
+            mbar_init(barStep(s), 9);  // (leader's is used) a group's four warps in either CTA, the expected bytes
             mbar_init(barTokEmpty(s), 1);
             mbar_init(barCodeFull(s), 1);
             mbar_init(barCodeEmpty(s), 4);
         }
-        for (uint32_t s = 0; s < kOperandStages; ++s) mbar_init(barOperand(s), 8);  // four warps of either CTA
         for (uint32_t s = 0; s < kAccs; ++s) {
             mbar_init(barAccFull(s), 1);
             mbar_init(barAccEmpty(s), 2 * kDrainThreads / 32);
@@ -183,12 +182,13 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
         {
             uint32_t st = 0, phase = 0;
             bool ok = true;
+            const uint32_t leaderStep = map_to_cta(barStep(0), 0u);
             for (uint32_t u = firstUnit; u < units && ok; u += unitStride) {
                 const uint32_t nt = ntOf(u);
                 const int row0 = (int)(tokenOf(u) + ctaRank * (columnsOf(u) >> 1));
                 for (uint32_t g = 0; g < steps; ++g) {
-                    if (!mbar_wait_warp<true>(barCodeEmpty(st), phase ^ 1u, &abortFlag) ||
-                        !mbar_wait_warp<true>(barTokEmpty(st), phase ^ 1u, &abortFlag)) {
+                    if (!mbar_wait_warp<true, Order::kLocal>(barCodeEmpty(st), phase ^ 1u, &abortFlag) ||
+                        !mbar_wait_warp<true, Order::kPair>(barTokEmpty(st), phase ^ 1u, &abortFlag)) {
                         ok = false;
                         break;
                     }
@@ -203,9 +203,10 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
                         } else {
                             mbar_arrive(barCodeFull(st));  // a bias step reads no codes
                         }
-                        mbar_expect_tx(barTokFull(st), kTokBytes);
-                        if (g < groupsK) tma_load_2d(tokAddr(st), &mapTok, (int)(g * kStepK), row0, barTokFull(st));
-                        else tma_load_2d(tokAddr(st), &mapSums, (int)((g - groupsK) * kStepK), row0, barTokFull(st));
+                        if (leader) mbar_expect_tx(barStep(st), 2u * kTokBytes);
+                        const uint32_t bar = leaderStep + 8u * st;
+                        if (g < groupsK) tma_load_2d_pair(tokAddr(st), &mapTok, (int)(g * kStepK), row0, bar);
+                        else tma_load_2d_pair(tokAddr(st), &mapSums, (int)((g - groupsK) * kStepK), row0, bar);
                     }
                     if (++st == kStages) {
                         st = 0;
@@ -219,14 +220,13 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
         // (the whole warp runs the loop and one elected lane issues: inside a `lane == 0` branch every
         // operand would go to the uniform registers by a loop over the active lanes)
         if (leader) {
-            uint32_t st = 0, op = 0, opPhase = 0, acc = 0, accPhase = 0;
+            uint32_t st = 0, phase = 0, op = 0, acc = 0, accPhase = 0;
             bool ok = true;
             for (uint32_t u = firstUnit; u < units && ok; u += unitStride) {
                 const uint32_t idesc = umma_idesc_bf16_m256(columnsOf(u));
                 for (uint32_t g = 0; g < steps; ++g) {
-                    // (the warps that arrive on the operand have also seen both token halves land)
-                    if (!mbar_wait_warp<false>(barOperand(op), opPhase, &abortFlag) ||
-                        !mbar_wait_warp<false>(barAccEmpty(acc), accPhase ^ 1u, &abortFlag)) {
+                    if (!mbar_wait_warp<false, Order::kPair>(barStep(st), phase, &abortFlag) ||
+                        !mbar_wait_warp<false, Order::kPair>(barAccEmpty(acc), accPhase ^ 1u, &abortFlag)) {
                         ok = false;
                         break;
                     }
@@ -234,17 +234,20 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
                     const uint64_t descTok = umma_desc_sw128(tokAddr(st));
                     const uint32_t tmemW = tmemBase + kOperandCol + op * 32u, tmemD = tmemBase + acc * kMaxRows;
                     if (elect_one()) {
+                        // (the wait was for both CTAs' operands; this look acquires the token halves, whose copies
+                        // complete on this CTA's barrier)
+                        (void)mbar_test_wait(barStep(st), phase);
 #pragma unroll
                         for (uint32_t kk = 0; kk < kStepK / 16; ++kk)
                             tc_mma_bf16_a_tmem(tmemD, tmemW + 8u * kk, descTok + 2u * kk, idesc, kk ? 1u : 0u);
                         tc_commit_pair(barTokEmpty(st));  // the token stage and the operand stage are free
                         tc_commit_pair(barAccFull(acc));
                     }
-                    if (++st == kStages) st = 0;
-                    if (++op == kOperandStages) {
-                        op = 0;
-                        opPhase ^= 1u;
+                    if (++st == kStages) {
+                        st = 0;
+                        phase ^= 1u;
                     }
+                    op = (op + 1u) % kOperandStages;
                     if (++acc == kAccs) {
                         acc = 0;
                         accPhase ^= 1u;
@@ -271,7 +274,7 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
             const uint32_t back = (st + kStages - kOperandStages) % kStages;
             if (!mbar_wait(barCodeFull(st), phase, &abortFlag) ||
                 (stepNo >= kOperandStages &&
-                 !mbar_wait(barTokEmpty(back), ((stepNo - kOperandStages) / kStages) & 1u, &abortFlag)))
+                 !mbar_wait<Order::kPair>(barTokEmpty(back), ((stepNo - kOperandStages) / kStages) & 1u, &abortFlag)))
                 break;
             tc_fence_after();
             uint32_t o[32];
@@ -307,14 +310,11 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
                 }
             }
             tc_store_32cols(tmemLane + op * 32u, o);
-            // this CTA's half of the step's token tile must have landed before the MMA is told to go
-            const bool landed = mbar_wait(barTokFull(st), phase, &abortFlag);
             tc_wait_st();
-            if (!landed) break;
             tc_fence_before();
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive_cluster(map_to_cta(barOperand(op), 0u));
+                mbar_arrive_pair(map_to_cta(barStep(st), 0u));
                 mbar_arrive(barCodeEmpty(st));
             }
             st += kDequantGroups;
@@ -366,7 +366,7 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
             for (int j = 0; j < 64; ++j) sum[j] = 0.0f;
             for (uint32_t g = 0; g < steps; ++g) {
                 const float s = g < groupsK ? 128.0f * bf2f(myScale[g]) : 1.0f;  // (the codes come as q / 128)
-                if (!mbar_wait(barAccFull(accNo), accPhase, &abortFlag)) {
+                if (!mbar_wait<Order::kPair>(barAccFull(accNo), accPhase, &abortFlag)) {
                     ok = false;
                     break;
                 }
@@ -383,7 +383,7 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(map_to_cta(barAccEmpty(accNo), 0u));
+                if (lane == 0) mbar_arrive_pair(map_to_cta(barAccEmpty(accNo), 0u));
                 if (++accNo == kAccs) {
                     accNo = 0;
                     accPhase ^= 1u;

@@ -652,7 +652,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ CUtensorMap mapTokSmall, const __grid_constant__ CUtensorMap mapW0,
                     const __grid_constant__ CUtensorMap mapW1, const GemmArgs args) {
     extern __shared__ uint8_t gemmSmemRaw[];
-    __shared__ uint64_t barriers[2 * kTokStages + 2 * kPackStages + kWStages + 4 + 2 * kEpilogueSets + 1];
+    __shared__ uint64_t barriers[2 * kTokStages + 2 * kPackStages + 4 + 2 * kEpilogueSets + 1];
     __shared__ uint32_t tmemBaseSlot;
     __shared__ volatile uint32_t abortFlag;
 
@@ -673,34 +673,32 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
 
     const uint32_t barBase = smem_u32(barriers);
     auto barAt = [&](int i) { return barBase + 8u * (uint32_t)i; };
-    auto barTokFull = [&](int s) { return barAt(s); };
+    auto barStep = [&](int s) { return barAt(s); };
     auto barTokEmpty = [&](int s) { return barAt(kTokStages + s); };
     auto barPackFull = [&](int s) { return barAt(2 * kTokStages + s); };
     auto barPackEmpty = [&](int s) { return barAt(2 * kTokStages + kPackStages + s); };
-    constexpr int kBarW = 2 * kTokStages + 2 * kPackStages;
-    auto barWFull = [&](int s) { return barAt(kBarW + s); };
-    auto barAccFull = [&](int s) { return barAt(kBarW + kWStages + s); };
-    auto barAccEmpty = [&](int s) { return barAt(kBarW + kWStages + 2 + s); };
-    auto barStage = [&](int set, int buffer) { return barAt(kBarW + kWStages + 4 + 2 * set + buffer); };
-    const uint32_t barRows = barAt(kBarW + kWStages + 4 + 2 * kEpilogueSets);
+    constexpr int kBarAcc = 2 * kTokStages + 2 * kPackStages;
+    auto barAccFull = [&](int s) { return barAt(kBarAcc + s); };
+    auto barAccEmpty = [&](int s) { return barAt(kBarAcc + 2 + s); };
+    auto barStage = [&](int set, int buffer) { return barAt(kBarAcc + 4 + 2 * set + buffer); };
+    const uint32_t barRows = barAt(kBarAcc + 4 + 2 * kEpilogueSets);
 
     // The two CTAs of a cluster work as one unit of the tensor core: the leader (rank 0) issues
-    // the MMAs for both.  Barriers that say "full" to the MMA issuer live in the leader and count
-    // both CTAs' arrivals; barriers that the MMAs' completion frees exist in either CTA and are
-    // signalled in both by one multicast commit.
+    // the MMAs for both.  What the MMA issuer waits for lives in the leader: a step's barrier counts the
+    // arrivals of both CTAs' dequantizers and the bytes of both CTAs' token copies.  Barriers that the MMAs'
+    // completion frees exist in either CTA and are signalled in both by one multicast commit.
     const uint32_t ctaRank = cluster_cta_rank();
     const bool leader = ctaRank == 0u;
     if (threadIdx.x == 0) {
         abortFlag = 0;
         for (int s = 0; s < kTokStages; ++s) {
-            mbar_init(barTokFull(s), 1);
+            mbar_init(barStep(s), 9);      // (leader's is used) a group's four warps in either CTA, the expected bytes
             mbar_init(barTokEmpty(s), 1);  // one tcgen05.commit
         }
         for (int s = 0; s < kPackStages; ++s) {
             mbar_init(barPackFull(s), 1);
             mbar_init(barPackEmpty(s), kDequantWarps);  // every dequantizing warp
         }
-        for (int s = 0; s < kWStages; ++s) mbar_init(barWFull(s), 8);  // (leader's is used) the group's four warps in either CTA
         for (int s = 0; s < 2; ++s) {
             mbar_init(barAccFull(s), 1);                     // one tcgen05.commit
             mbar_init(barAccEmpty(s), 8 * kEpilogueSets);    // (leader's is used) the epilogue warps of either CTA
@@ -754,6 +752,7 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
             uint32_t ts = 0, phase = 0;
             bool ok = true;
             RowTile next = tileOf(firstUnit);
+            const uint32_t leaderStep = map_to_cta(barStep(0), 0u);
             for (uint32_t u = firstUnit; u < units && ok; u += unitStride) {
                 const RowTile tile = next;
                 next = tileOf(u + unitStride);
@@ -762,13 +761,13 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
                 const CUtensorMap *map = half <= kTokSmallRows ? &mapTokSmall : &mapTok;
                 const uint32_t bytes = (half <= kTokSmallRows ? kTokSmallRows : kTokHalfRows) * kTileK * 2;
                 for (uint32_t g = 0; g < groupsK; ++g) {
-                    if (!mbar_wait_warp<true>(barTokEmpty(ts), phase ^ 1u, &abortFlag)) {
+                    if (!mbar_wait_warp<true, Order::kPair>(barTokEmpty(ts), phase ^ 1u, &abortFlag)) {
                         ok = false;
                         break;
                     }
                     if (elect_one()) {
-                        mbar_expect_tx(barTokFull(ts), bytes);
-                        tma_load_2d(tokAddrOf(ts), map, (int)(g * kTileK), row0, barTokFull(ts));
+                        if (leader) mbar_expect_tx(barStep(ts), 2u * bytes);
+                        tma_load_2d_pair(tokAddrOf(ts), map, (int)(g * kTileK), row0, leaderStep + 8u * ts);
                     }
                     ts = (ts + 1u) % kTokStages;
                     if (ts == 0) phase ^= 1u;
@@ -811,14 +810,14 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
         // branch every operand goes to the uniform registers by a loop over the active lanes, and a step
         // cost this thread 820 cycles for 384 of the tensor core.
         if (leader && firstUnit < units) {
-            uint32_t ts = 0, wPhases = 0, acc = 0, accPhase = 0;  // wPhases: bit s = parity of weight stage s
-            bool ok = true, ready = false;                        // ready: seen that the next step's weights are there
+            uint32_t ts = 0, phase = 0, acc = 0, accPhase = 0;
+            bool ok = true, ready = false;  // ready: seen that the next step's weights and tokens are there
             RowTile next = tileOf(firstUnit);
             for (uint32_t u = firstUnit; u < units && ok; u += unitStride) {
                 const RowTile tile = next;
                 next = tileOf(u + unitStride);
                 const uint32_t idesc = umma_idesc_bf16_m256(columnsOf(tile));
-                if (!mbar_wait_warp<true>(barAccEmpty(acc), accPhase ^ 1u, &abortFlag)) break;
+                if (!mbar_wait_warp<true, Order::kPair>(barAccEmpty(acc), accPhase ^ 1u, &abortFlag)) break;
                 tc_fence_after();
                 const uint32_t tmemD = tmemBase + acc * kAccCols;
                 for (uint32_t g0 = 0; g0 < groupsK && ok; g0 += kWStages) {
@@ -826,20 +825,22 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
                     for (uint32_t ws = 0; ws < kWStages; ++ws) {
                         const uint32_t g = g0 + ws;
                         if (g >= groupsK) break;
-                        // (the group that arrives here has also seen both token halves land)
                         if (!__all_sync(0xFFFFFFFFu, ready) &&
-                            !mbar_wait_warp<false>(barWFull(ws), (wPhases >> ws) & 1u, &abortFlag)) {
+                            !mbar_wait_warp<false, Order::kPair>(barStep(ts), phase, &abortFlag)) {
                             ok = false;
                             break;
                         }
-                        wPhases ^= 1u << ws;
                         tc_fence_after();
                         // the next step's barrier is looked at now and the answer used after this step's MMAs
-                        const uint32_t wn = g + 1u < groupsK ? (ws + 1u) % kWStages : 0u;
-                        ready = mbar_test_wait(barWFull(wn), (wPhases >> wn) & 1u);
+                        const uint32_t tn = (ts + 1u) % kTokStages;
+                        if (tn == 0u) phase ^= 1u;
+                        ready = mbar_test_wait<Order::kPair>(barStep(tn), phase);
                         const uint64_t descTok = umma_desc_sw128(tokAddrOf(ts));
                         const uint32_t tmemW = tmemBase + kWCol0 + ws * 32u;
                         if (elect_one()) {
+                            // (the wait was for both CTAs' operands; this look acquires the token halves, whose copies
+                            // complete on this CTA's barrier)
+                            (void)mbar_test_wait(barStep(ts), tn == 0u ? phase ^ 1u : phase);
 #pragma unroll
                             for (uint32_t kk = 0; kk < kTileK / 16; ++kk) {
                                 // per 16-element slice: eight columns further in TMEM, 32 bytes (>> 4 = 2)
@@ -851,7 +852,7 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
                             // the same step used (the dequantizers wait on the token ring's barrier, too)
                             tc_commit_pair(barTokEmpty(ts));
                         }
-                        ts = (ts + 1u) % kTokStages;
+                        ts = tn;
                     }
                 }
                 if (!ok) break;
@@ -894,7 +895,7 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(live ? 4u : 0u) : "memory");
         };
         auto scales_arrived = [] { asm volatile("cp.async.wait_all;" ::: "memory"); };
-        const uint32_t leaderWFull = map_to_cta(barWFull(grp), 0u);
+        const uint32_t leaderStep = map_to_cta(barStep(0), 0u);
         uint32_t ps = 0, pPhase = 0;
         uint32_t step0 = 0;                 // steps of the CTA's earlier units
         uint32_t lastStep = 0xFFFFFFFFu;    // this group's previous step
@@ -953,25 +954,19 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
                 // The weight stage was last read by the MMAs of this group's previous step: their completion
                 // is that step's signal on the token ring.  Waited for only here: the conversion above runs
                 // under those MMAs.
-                const uint32_t step = step0 + g, ts = step % kTokStages;
+                const uint32_t step = step0 + g;
                 if (lastStep != 0xFFFFFFFFu &&
-                    !mbar_wait(barTokEmpty(lastStep % kTokStages), (lastStep / kTokStages) & 1u, &abortFlag)) {
+                    !mbar_wait<Order::kPair>(barTokEmpty(lastStep % kTokStages), (lastStep / kTokStages) & 1u, &abortFlag)) {
                     ok = false;
                     break;
                 }
                 lastStep = step;
                 tc_fence_after();
                 tc_store_32cols(tmemW, o);
-                // this CTA's half of the step's token tile must have landed before the MMA is told to go
-                const bool landed = mbar_wait(barTokFull(ts), (step / kTokStages) & 1u, &abortFlag);
                 tc_wait_st();
-                if (!landed) {
-                    ok = false;
-                    break;
-                }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(leaderWFull);
+                if (lane == 0) mbar_arrive_pair(leaderStep + 8u * (step % kTokStages));
             }
         }
         scales_arrived();  // nothing of this thread's is in flight when shared memory is released
@@ -1018,7 +1013,7 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
                 mbar_arrive(barRows);
                 nextTarget = row_target(next, te);
             }
-            if (!mbar_wait_idle(barAccFull(acc), accPhase, &abortFlag)) break;
+            if (!mbar_wait_idle<Order::kPair>(barAccFull(acc), accPhase, &abortFlag)) break;
             if (MODE == kModeDown && !mbar_wait(barRows, unitNo & 1u, &abortFlag)) break;
             tc_fence_after();
             const uint32_t taddr = tmemBase + acc * kAccCols + ((quarter * 32u) << 16);
@@ -1080,7 +1075,7 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
             if (!ok) break;
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_cta(barAccEmpty(acc), 0u));
+            if (lane == 0) mbar_arrive_pair(map_to_cta(barAccEmpty(acc), 0u));
             if (++acc == 2) {
                 acc = 0;
                 accPhase ^= 1u;

@@ -25,59 +25,59 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// How a wait orders what follows it: kLocal, acquire at CTA scope, where threads or copies of this CTA signal the
+// barrier; kPair, relaxed at cluster scope, where the other CTA of a pair or the MMAs of both do: what they hand over
+// is tensor memory, which the tcgen05 fences on either side order, or stages that completed MMAs have read.  (An
+// acquire at cluster scope in one warp's loop costs the whole CTA 4 to 10 % of a GEMM.)
+enum class Order { kLocal, kPair };
+#define FF_MBAR_POLL(instruction)                             \
+    asm volatile(                                             \
+        "{\n"                                                 \
+        ".reg .pred p;\n" instruction " p, [%1], %2;\n"       \
+        "selp.u32 %0, 1, 0, p;\n"                             \
+        "}\n"                                                 \
+        : "=r"(ok)                                            \
+        : "r"(bar), "r"(parity)                               \
+        : "memory")
+template <Order kOrder = Order::kLocal>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
+    if (kOrder == Order::kLocal) FF_MBAR_POLL("mbarrier.try_wait.parity.shared::cta.b64");
+    else FF_MBAR_POLL("mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64");
     return ok != 0;
 }
 // one look, without the suspension that a try_wait may take
+template <Order kOrder = Order::kLocal>
 __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
+    if (kOrder == Order::kLocal) FF_MBAR_POLL("mbarrier.test_wait.parity.shared::cta.b64");
+    else FF_MBAR_POLL("mbarrier.test_wait.parity.relaxed.cluster.shared::cta.b64");
     return ok != 0;
 }
+#undef FF_MBAR_POLL
 // Bounded wait.  Returns false when the limit ran out or another thread of the CTA gave up; the
 // caller leaves its loop.  `abortFlag` lives in shared memory.  kSleep: pause between polls, for
 // the warps whose polling would otherwise take issue slots from the dequantizing warps.
 // The first poll stands alone in front of the loop: measured on the device, a wait that finds its
 // barrier already complete costs 7 cycles this way and about 200 when the poll sits inside the
 // bounded loop.
-template <bool kSleep>
+template <bool kSleep, Order kOrder>
 __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile uint32_t *abortFlag) {
     for (uint32_t i = 0; i < kSpinLimit; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
+        if (mbar_try_wait<kOrder>(bar, parity)) return true;
         if (kSleep) __nanosleep(40);
         if ((i & 255u) == 255u && *abortFlag) return false;
     }
     *abortFlag = 1u;
     return false;
 }
-template <bool kSleep>
-__device__ __forceinline__ bool mbar_wait_impl(uint32_t bar, uint32_t parity, volatile uint32_t *abortFlag) {
-    if (mbar_try_wait(bar, parity)) return true;
-    return mbar_wait_slow<kSleep>(bar, parity, abortFlag);
-}
+template <Order kOrder = Order::kLocal>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abortFlag) {
-    return mbar_wait_impl<false>(bar, parity, abortFlag);
+    return mbar_try_wait<kOrder>(bar, parity) || mbar_wait_slow<false, kOrder>(bar, parity, abortFlag);
 }
+template <Order kOrder = Order::kLocal>
 __device__ __forceinline__ bool mbar_wait_idle(uint32_t bar, uint32_t parity, volatile uint32_t *abortFlag) {
-    return mbar_wait_impl<true>(bar, parity, abortFlag);
+    return mbar_try_wait<kOrder>(bar, parity) || mbar_wait_slow<true, kOrder>(bar, parity, abortFlag);
 }
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y,
@@ -190,20 +190,25 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(addr), "r"(rank));
     return out;
 }
-// arrive on a barrier that may live in the other CTA of the pair (`clusterAddr` from map_to_cta)
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t clusterAddr) {
-    // (default semantics, release at CTA scope: a cluster-scope release holds the warp until everything it
-    // has in flight is acknowledged, over a thousand cycles here; what the other CTA's MMA reads
-    // from this CTA is ordered by the tcgen05 fences and the TMA's own barrier, not by this arrive)
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(clusterAddr) : "memory");
+// Arrives on a barrier that may live in the other CTA of the pair (`clusterAddr` from map_to_cta), for a hand-over of
+// tensor memory: relaxed, since the tcgen05 fences in front of it and behind the wait order the accesses.  (A
+// cluster-scope release holds the warp until everything it has in flight is acknowledged, over a thousand cycles here.)
+__device__ __forceinline__ void mbar_arrive_pair(uint32_t clusterAddr) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(clusterAddr) : "memory");
 }
-// A wait of a whole converged warp whose lanes then act as one: either all of them go on or none.  Acquires
-// at CTA scope also where the other CTA arrives: what that CTA wrote for the MMA is ordered by the
-// tcgen05 fences, and a cluster-scope acquire costs over a hundred cycles.
-template <bool kSleep>
+// A copy into this CTA's shared memory whose completion is counted on a barrier of either CTA of the pair (`clusterBar`).
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t clusterBar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(clusterBar)
+        : "memory");
+}
+// A wait of a whole converged warp whose lanes then act as one: either all of them go on or none.
+template <bool kSleep, Order kOrder>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t *abortFlag) {
-    if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
-    return __all_sync(0xFFFFFFFFu, mbar_wait_slow<kSleep>(bar, parity, abortFlag));
+    if (__all_sync(0xFFFFFFFFu, mbar_try_wait<kOrder>(bar, parity))) return true;
+    return __all_sync(0xFFFFFFFFu, mbar_wait_slow<kSleep, kOrder>(bar, parity, abortFlag));
 }
 // one lane of the converged warp (the form in which the compiler knows that a single lane is active)
 __device__ __forceinline__ bool elect_one() {

@@ -107,3 +107,34 @@ def test_row_kernels(oracle, d, shift):
             assert np.mean(g != r) < 1e-2
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("rows", [40, 700])
+def test_gemms_repeat_bit_for_bit(rows):
+    """The CTA pairs' hand-overs: the same rows again and again beside other traffic on the chip give the same bits."""
+    from test_gpu_router_int8 import int8_projection
+    L = workload.make_layer(0x75, 0, experts=32, d=1088, f=320, sharedF=704, topK=8)
+    hp, ctx = context(L, rows)
+    int8 = hp.HotpathContext(layers=1, experts=8, d=1088, f=64, sharedF=704, topK=8, maxTokens=rows)
+    try:
+        int8.loadSharedInt8(0, int8_projection(1, 704, 1088, 0.02), int8_projection(2, 704, 1088, 0.02),
+                            int8_projection(3, 1088, 704, 0.02))
+        x = hp.bf16_tensor(workload.make_tokens(0x76, f"repeat{rows}", rows, 1088), ctx.device)
+        other = torch.cuda.Stream()
+        src = torch.ones(1 << 26, dtype=torch.uint8, device=ctx.device)
+        dst = torch.empty_like(src)
+        first = None
+        for i in range(12):
+            with torch.cuda.stream(other):
+                for _ in range(i % 4):
+                    dst.copy_(src)
+            y8 = torch.empty_like(x)
+            hp.PrefillSharedExpert(int8).encodeBlock(None, 0, x, y8, rows)
+            out = (ctx.moeLayer(0, x), y8)
+            torch.cuda.synchronize()
+            first = first or out
+            assert torch.equal(out[0], first[0]) and torch.equal(out[1], first[1])
+        assert ctx.info().deviceErrorFlag == 0 and int8.info().deviceErrorFlag == 0
+    finally:
+        int8.close()
+        ctx.close()
