@@ -14,8 +14,12 @@
 //
 // INT4: an input row has one scale for its digits, a group's sums are scaled once by the weights' scale,
 // and the bias part is a few small bf16 MMAs on the group sums: 13 instructions per group for the
-// weights and 9 for a pair of rows, per warp.  INT8: the two parts cancel in part, so they are joined
-// group by group.
+// weights and 9 for a pair of rows, per warp.  A row that has groups far below its largest value loses their
+// digits, which shows where the weights of that value are zero (one value of 2^20 times the rest: 2 % error
+// of the outputs), so a CTA forms its outputs of such rows once more in fp32 (redo_uneven_rows; the look at
+// the groups and the code behind the loop cost 2 to 4 %: four layers of 5 rows 218.1 -> 221.5 us, of 16 rows
+// 304.6 -> 315.8).  INT8: the two parts cancel in part, so they are joined group by group, and every group has
+// its own scale.
 //
 // Reference kernels replaced (paths inside the reference project):
 //   Sources/ANEFieldfareHotpath/Metal/Prefill/prefill.metal:1246-1529 (verify grouped GEMV)
@@ -35,6 +39,7 @@ namespace {
 constexpr int kMaxWarps = 16;
 constexpr int kTaskRows = 4;          // input rows of a task (2 where the rows are too wide for four as digits)
 constexpr uint32_t kPartGroups = 8;   // groups of a part along K, a multiple of four
+constexpr uint32_t kUneven = 10;      // INT4: a row is formed in fp32 if a group is this many powers of two below its largest value
 constexpr int kMaxJobs = kMaxGemvRows * 8 + 1;
 
 enum Mode : int { kGateUp = 0, kDown = 1 };
@@ -59,6 +64,7 @@ struct BlockArgs {
     uint32_t *activeExperts;  // gate/up: receives the count (may be null)
     uint32_t *errorFlag;
     uint32_t listOffset, digitsOffset, rowBytes, auxOffset, auxRow, slotsOffset, slotBytes, sbOffset;
+    uint32_t planOffset;      // INT4: this CTA's run and the jobs, for redo_run
     int perExpert;            // routes of one expert at most
     int taskShift;            // log2 of a task's input rows
     float *values;            // F32OUT: the routed rows
@@ -181,15 +187,120 @@ __device__ __forceinline__ void mma_1688(float (&d)[4], uint32_t a0, uint32_t a1
 }
 constexpr uint32_t kSumBlockBytes = 128;  // [column][8 groups] bf16
 
+// What redo_uneven_rows reads: the arguments once more (these are passed on by address), and per kind the weight rows and scale words behind the maps and what lies between experts.
+struct RedoArgs {
+    BlockArgs a;
+    struct {
+        const uint8_t *w[2];
+        const uint32_t *scales;
+        uint64_t stride, scaleStride;
+    } kind[2];
+};
+// A weight row against an input row in fp32, by one thread.
+__device__ __forceinline__ float fp32_row(const uint4 *w, const uint32_t *words, const uint4 *x, uint32_t groups) {
+    float acc = 0.0f;
+#pragma unroll 1
+    for (uint32_t g = 0; g < groups; ++g) {
+        float dot = 0.0f, sum = 0.0f;
+#pragma unroll
+        for (uint32_t half = 0; half < 2; ++half) {
+            const uint4 q = __ldg(w + 2u * g + half);
+            const uint32_t codes[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint4 v = __ldcg(x + 8u * g + 4u * half + (uint32_t)i);
+                const uint32_t xs[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float even = __uint_as_float(xs[j] << 16), odd = __uint_as_float(xs[j] & 0xFFFF0000u);
+                    dot = fmaf((float)((codes[i] >> (8 * j)) & 15u), even, dot);
+                    dot = fmaf((float)((codes[i] >> (8 * j + 4)) & 15u), odd, dot);
+                    sum += even + odd;
+                }
+            }
+        }
+        const uint32_t word = __ldg(words + g);
+        acc = fmaf(__uint_as_float(word << 16), dot, acc);
+        acc = fmaf(__uint_as_float(word & 0xFFFF0000u), sum, acc);
+    }
+    return acc;
+}
+// The outputs of one of a CTA's segments (tiles [tile0, tileEnd) of job `job`'s input rows [first, last)) for the rows that
+// have a group kUneven powers of two below their largest value (not all zero), once more, over what the digits gave.
+// A thread a weight row.
+template <int MODE, bool F32OUT>
+__device__ __forceinline__ void redo_uneven_rows(const RedoArgs &r, uint32_t job, const uint8_t *list, int first, int last, uint32_t tile0,
+                                                 uint32_t tileEnd) {
+    constexpr uint32_t kRows = MODE == kGateUp ? 8 : 16;
+    const int kind = job ? 1 : 0;
+    const uint64_t expert = kind ? job - 1u : 0u;
+    const BlockKind &k = r.a.kind[kind];
+    const uint32_t groups = k.groups;
+    for (int i = first; i < last; ++i) {
+        const int outRow = kind ? (int)list[expert * kMaxGemvRows + (uint32_t)i] : i, inRow = MODE == kGateUp && kind ? outRow / r.a.K : outRow;
+        const uint4 *x = reinterpret_cast<const uint4 *>(k.in + (size_t)inRow * k.inStride);
+        uint32_t top = 0, least = 0xFFFFu;  // the row's largest value, the smallest of its groups' largest ones
+#pragma unroll 1
+        for (uint32_t g = 0; g < groups; ++g) {
+            uint32_t group = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) group = max(group, top_exponent(__ldcg(x + 8u * g + j)));
+            top = max(top, group);
+            if (group) least = min(least, group);
+        }
+        if (least + (kUneven << 7) >= top) continue;
+        for (uint32_t row = tile0 * kRows + threadIdx.x; row < tileEnd * kRows; row += blockDim.x) {
+            const uint32_t scaleRow = row / kRows * 16u + row % kRows;
+            auto dot = [&](int matrix) {
+                return fp32_row(reinterpret_cast<const uint4 *>(r.kind[kind].w[matrix] + expert * r.kind[kind].stride) + (size_t)row * groups * 2u,
+                                r.kind[kind].scales + expert * r.kind[kind].scaleStride + (size_t)(scaleRow + 8u * matrix) * padded_groups(groups), x,
+                                groups);
+            };
+            const float v = dot(0);
+            const size_t to = (size_t)outRow * k.outStride + row;
+            if (MODE == kGateUp) {
+                const float u = dot(1);
+                const float gate = kind ? v : bf16_round(v), up = kind ? u : bf16_round(u);
+                k.out[to] = f2bf(gelu_tanh(gate) * up);
+            } else if (F32OUT && kind) {
+                r.a.values[to] = v;
+            } else {
+                k.out[to] = f2bf(v);
+            }
+        }
+    }
+}
+
+// redo_uneven_rows for every segment of a CTA's run, from a copy of the plan in dynamic shared memory.  (With the static
+// arrays' addresses passed on, the main loop reads them again after every store.)
+template <int MODE, bool F32OUT>
+__device__ __noinline__ void redo_run(const RedoArgs &r, const uint8_t *smemRaw) {
+    const uint32_t *plan = reinterpret_cast<const uint32_t *>(smemRaw + r.a.planOffset);
+    const uint32_t endJob = plan[3], endGroup = plan[4], endTile = plan[5], nJobs = plan[6];
+    uint32_t j = plan[0], rg = plan[1], tile = plan[2];
+    for (; j < nJobs && j <= endJob; ++j, rg = 0, tile = 0) {
+        const uint32_t job = plan[7u + j] & 0xFFFFu;
+        const int rows = (int)(plan[7u + j] >> 16);
+        for (; (int)(rg << r.a.taskShift) < rows; ++rg, tile = 0) {
+            const bool last = j == endJob && rg == endGroup;
+            const int first = (int)(rg << r.a.taskShift);
+            redo_uneven_rows<MODE, F32OUT>(r, job, smemRaw + r.a.listOffset, first, min(rows, first + (1 << r.a.taskShift)), tile,
+                                           last ? endTile : r.a.kind[job ? 1 : 0].tiles);
+            if (last) return;
+        }
+    }
+}
+
 // F32OUT (down): the routed rows go to `values` unrounded.
 template <int MODE, bool INT8, bool F32OUT>
 __global__ void __launch_bounds__(kMaxWarps * 32, 1)
-k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
+k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps, const __grid_constant__ RedoArgs redo) {
     extern __shared__ __align__(128) uint8_t smemRaw[];
     __shared__ uint32_t sFirst[kMaxJobs + 1];   // cost of the jobs before job k (active jobs, the shared FFN first)
     __shared__ uint16_t sJob[kMaxJobs];         // 0 the shared FFN, 1 + e expert e
     __shared__ uint32_t sCount[kMaxExperts], sWarpSum[2][kMaxWarps], sTop[kMaxWarps];
     __shared__ float sUnit[kTaskRows];
+    __shared__ uint32_t sUneven;  // a row of this CTA's run may be one for redo_uneven_rows
     __shared__ __align__(8) uint64_t sBar[2 * kMaxWarps];
     uint8_t *sList = smemRaw + a.listOffset;  // [expert][16] route numbers (< 128)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = (int)(blockDim.x >> 5);
@@ -199,6 +310,7 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
     if (!(MODE == kDown)) pdl_wait();  // (the down kernel's plan and first weights need only what was there before its predecessor)
     if (MODE == kGateUp) pdl_trigger();
     if (threadIdx.x == 0) {
+        sUneven = 0u;
         for (int i = 0; i < 2 * kMaxWarps; ++i) bar_init(sm_addr(&sBar[i]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -322,6 +434,17 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
     Place at = place_of(blockIdx.x), end = place_of(blockIdx.x + 1u);
     settle(at);
     settle(end);
+    if (!INT8) {
+        uint32_t *plan = reinterpret_cast<uint32_t *>(smemRaw + a.planOffset);
+        const uint32_t run[7] = {at.job, at.rowGroup, at.tile, end.job, end.rowGroup, end.tile, nJobs};
+        if (threadIdx.x < 7) {
+            uint32_t v = run[0];
+#pragma unroll
+            for (int i = 1; i < 7; ++i) v = threadIdx.x == i ? run[i] : v;
+            plan[threadIdx.x] = v;
+        }
+        for (uint32_t j = threadIdx.x; j < nJobs; j += blockDim.x) plan[7u + j] = sJob[j] | (uint32_t)rows_of(j) << 16;
+    }
 
     // ---- copies: this warp's steps (tile, part) in order, two slots in turn ----
     const uint32_t slots = smem + a.slotsOffset + (uint32_t)warp * 2u * a.slotBytes;
@@ -395,14 +518,33 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
             const int padded = ((int)k.groups + 3) & ~3;  // groups past the row add nothing
             if (tid < padded - (int)k.groups) rowAux[(int)k.groups + tid] = GroupAux{0.0f, 0.0f};
         } else {
-            uint32_t top = 0;
+            uint32_t top = 0, low = 0xFFFFu;  // the largest and the smallest of the runs' largest values
+            auto look = [&](int i, const uint4 &v) {
+                const uint32_t t = top_exponent(v);
+                top = max(top, t);
+                if (i < runs) low = min(low, t);
+            };
 #pragma unroll
-            for (int i = 0; i < kHeld; ++i) top = max(top, top_exponent(held[i]));
-            for (int i = tid + kHeld * threads; i < runs; i += threads) top = max(top, top_exponent(__ldcg(src + i)));
+            for (int i = 0; i < kHeld; ++i) look(tid + i * threads, held[i]);
+            for (int i = tid + kHeld * threads; i < runs; i += threads) look(i, __ldcg(src + i));
             top = __reduce_max_sync(0xFFFFFFFFu, top);
             if (lane == 0) sTop[warp] = top;
             named_barrier(2 + r, threads);
             for (int w = 0; w < per; ++w) top = max(top, sTop[r * per + w]);
+            if (!__all_sync(0xFFFFFFFFu, low + (kUneven << 7) >= top)) {  // a run of eight is that small: a whole group?
+                auto check = [&](int i, const uint4 &v) {  // a group's eight lanes are a byte of the ballots
+                    const uint32_t t = top_exponent(v);
+                    uint32_t large = __ballot_sync(0xFFFFFFFFu, t + (kUneven << 7) >= top), some = __ballot_sync(0xFFFFFFFFu, i < runs && t != 0u);
+                    large |= large >> 4 & 0x0F0F0F0Fu, some |= some >> 4 & 0x0F0F0F0Fu;
+                    large |= large >> 2, some |= some >> 2;
+                    large |= large >> 1, some |= some >> 1;
+                    if (some & ~large & 0x01010101u) sUneven = 1u;
+                };
+#pragma unroll
+                for (int i = 0; i < kHeld; ++i)
+                    if ((tid & ~31) + i * threads < runs) check(tid + i * threads, held[i]);  // the same for the whole warp
+                for (int i = tid + kHeld * threads; (i & ~31) < runs; i += threads) check(i, i < runs ? __ldcg(src + i) : make_uint4(0, 0, 0, 0));
+            }
             const RowScale scale = row_scale(top);
             if (tid == 0) sUnit[r] = scale.unit;
             // pair r / 2, columns 4 (r & 1).. of the sums
@@ -552,6 +694,10 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps) {
         at.tile = k.tiles;
         settle(at);
     }
+    if (!INT8) {
+        __syncthreads();
+        if (sUneven) redo_run<MODE, F32OUT>(redo, smemRaw);
+    }
 }
 
 // ---- host ------------------------------------------------------------------------------------------
@@ -578,18 +724,20 @@ uint32_t row_pitch(uint32_t part, bool int8) {
 }
 
 // Fills a kind and, unless they are there already, its maps.  mode kGateUp: w0, w1 [rows][cols], tiles of 8 + 8 rows; kDown: w0, 16 rows.
-bool setup_kind(int mode, bool int8, uint32_t &ready, uint32_t bit, BlockKind &k, CUtensorMap (&w)[3], const uint8_t *w0, const uint8_t *w1,
-                uint32_t rows, uint32_t cols, uint32_t experts, uint64_t stride, const uint32_t *scales, uint64_t scaleStride,
-                const char **error) {
-    const uint32_t groups = cols / 64, padded = padded_groups(groups);
+bool setup_kind(int mode, bool int8, int kind, RedoArgs &redo, LayerStore &L, const uint8_t *w0, const uint8_t *w1, uint32_t rows, uint32_t cols,
+                uint32_t experts, uint64_t stride, const uint32_t *scales, uint64_t scaleStride, const char **error) {
+    BlockKind &k = redo.a.kind[kind];
+    CUtensorMap(&w)[3] = L.blockMap[mode][kind];
+    const uint32_t groups = cols / 64, padded = padded_groups(groups), bit = 1u << (2 * mode + kind);
     const uint64_t rowBytes = int8 ? cols : cols / 2;
     k.tiles = mode == kGateUp ? rows / 8 : rows / 16;
     k.groups = groups;
     k.part = padded <= kPartGroups + 4 ? padded : kPartGroups;
     k.pitch = row_pitch(k.part, int8);
     k.sbWords = (k.part + 7u) & ~7u;  // (words past the row read as zero)
-    if (ready & bit) return true;
-    ready |= bit;
+    redo.kind[kind] = {{w0, w1}, scales, stride, scaleStride};
+    if (L.blockMapsReady & bit) return true;
+    L.blockMapsReady |= bit;
     const uint8_t *ws[2] = {w0, w1};
     for (int m = 0; m < (mode == kGateUp ? 2 : 1); ++m)
         if (!encode3(&w[m], CU_TENSOR_MAP_DATA_TYPE_UINT64, ws[m], rowBytes / 8, rows, experts, rowBytes, stride, k.pitch / 8,
@@ -601,7 +749,8 @@ bool setup_kind(int mode, bool int8, uint32_t &ready, uint32_t bit, BlockKind &k
 }
 
 template <int MODE, bool INT8, bool F32OUT = false>
-bool launch_kernel(FFContext *ctx, BlockArgs a, const BlockMaps &maps, const char *name, cudaStream_t stream, const char **error) {
+bool launch_kernel(FFContext *ctx, RedoArgs redo, const BlockMaps &maps, const char *name, cudaStream_t stream, const char **error) {
+    BlockArgs &a = redo.a;
     uint32_t groups = 0, slot = 0, sb = 0;
     for (int i = 0; i < 2; ++i) {
         if (!a.kind[i].tiles) continue;
@@ -616,7 +765,8 @@ bool launch_kernel(FFContext *ctx, BlockArgs a, const BlockMaps &maps, const cha
     // (a batch of four groups may read up to three groups past a slot's last row, within the scale area)
     constexpr uint32_t kLimit = 227 * 1024 - 6144;  // less the static arrays
     a.listOffset = 0;
-    a.digitsOffset = a.ids ? up128((uint32_t)a.E * kMaxGemvRows) : 0;
+    a.planOffset = a.ids ? (uint32_t)a.E * kMaxGemvRows : 0;
+    a.digitsOffset = up128(a.planOffset + (INT8 ? 0u : 4u * (7u + kMaxJobs)));
     a.rowBytes = padded * kDigitGroupBytes;
     // INT8: a row's group entries; INT4: a pair's group sums
     a.auxRow = INT8 ? padded * (uint32_t)sizeof(GroupAux) : (groups + 7u) / 8u * kSumBlockBytes;
@@ -634,7 +784,7 @@ bool launch_kernel(FFContext *ctx, BlockArgs a, const BlockMaps &maps, const cha
     if (!memo.prepare(k_block_int<MODE, INT8, F32OUT>, ctx->device, kLimit, kMaxWarps * 32, nullptr, error)) return false;
     {
         LaunchScope scope(ctx, stream, name);
-        FF_CUDA_OK(launch_pdl(k_block_int<MODE, INT8, F32OUT>, ctx->smCount, warps * 32, smem, stream, a, maps), error);
+        FF_CUDA_OK(launch_pdl(k_block_int<MODE, INT8, F32OUT>, ctx->smCount, warps * 32, smem, stream, a, maps, redo), error);
     }
     return true;
 }
@@ -653,7 +803,8 @@ bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
     const uint64_t words = scale_words(c.d, c.f);
     LayerStore &Lm = const_cast<LayerStore &>(L);  // (its maps are encoded once per load)
     for (int mode = 0; mode < 2; ++mode) {
-        BlockArgs a{};
+        RedoArgs redo{};
+        BlockArgs &a = redo.a;
         a.ids = ids;
         a.T = (int)tokens;
         a.K = (int)c.topK;
@@ -667,7 +818,7 @@ bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
         if (ids) {
             const uint32_t *o = &L.off.gateWOff;
             BlockKind &k = a.kind[1];
-            if (!setup_kind(mode, false, Lm.blockMapsReady, 1u << (2 * mode + 1), k, Lm.blockMap[mode][1], L.experts + (down ? o[6] : o[0]), L.experts + o[3], down ? c.d : c.f,
+            if (!setup_kind(mode, false, 1, redo, Lm, L.experts + (down ? o[6] : o[0]), L.experts + o[3], down ? c.d : c.f,
                             down ? c.f : c.d, L.expertCount, L.stride,
                             L.routedScales + (down ? (uint64_t)(c.f / 8) * 16 * padded_groups(c.d / 64) : 0), words, error))
                 return false;
@@ -679,7 +830,7 @@ bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
         if (withShared) {
             const uint32_t *o = &L.sharedOff.gateWOff;
             BlockKind &k = a.kind[0];
-            if (!setup_kind(mode, false, Lm.blockMapsReady, 1u << (2 * mode + 0), k, Lm.blockMap[mode][0], L.shared + (down ? o[6] : o[0]), L.shared + o[3], down ? c.d : c.sharedF,
+            if (!setup_kind(mode, false, 0, redo, Lm, L.shared + (down ? o[6] : o[0]), L.shared + o[3], down ? c.d : c.sharedF,
                             down ? c.sharedF : c.d, 1, (uint64_t)c.d * c.sharedF / 2,
                             L.sharedScales + (down ? (uint64_t)(c.sharedF / 8) * 16 * padded_groups(c.d / 64) : 0), 0, error))
                 return false;
@@ -690,9 +841,9 @@ bool launch_block_int4(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
         }
         BlockMaps maps;
         memcpy(&maps, Lm.blockMap[mode], sizeof(maps));
-        const bool ok = values && down ? launch_kernel<kDown, false, true>(ctx, a, maps, "int4_block_down", stream, error)
-                        : down ? launch_kernel<kDown, false>(ctx, a, maps, "int4_block_down", stream, error)
-                             : launch_kernel<kGateUp, false>(ctx, a, maps, "int4_block_gate_up_act", stream, error);
+        const bool ok = values && down ? launch_kernel<kDown, false, true>(ctx, redo, maps, "int4_block_down", stream, error)
+                        : down ? launch_kernel<kDown, false>(ctx, redo, maps, "int4_block_down", stream, error)
+                             : launch_kernel<kGateUp, false>(ctx, redo, maps, "int4_block_gate_up_act", stream, error);
         if (!ok) return false;
     }
     return true;
@@ -704,7 +855,8 @@ bool launch_block_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
     const FFConfig &c = ctx->cfg;
     LayerStore &Lm = const_cast<LayerStore &>(L);  // (its maps are encoded once per load)
     for (int mode = 0; mode < 2; ++mode) {
-        BlockArgs a{};
+        RedoArgs redo{};
+        BlockArgs &a = redo.a;
         a.T = (int)tokens;
         a.K = 1;
         a.perExpert = (int)tokens;
@@ -712,7 +864,7 @@ bool launch_block_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
         a.errorFlag = ctx->errorFlag;
         const bool down = mode == kDown;
         BlockKind &k = a.kind[0];
-        if (!setup_kind(mode, true, Lm.blockMapsReady, 1u << (2 * mode + 0), k, Lm.blockMap[mode][0], L.shared8W[down ? 2 : 0], L.shared8W[1], down ? c.d : c.sharedF,
+        if (!setup_kind(mode, true, 0, redo, Lm, L.shared8W[down ? 2 : 0], L.shared8W[1], down ? c.d : c.sharedF,
                         down ? c.sharedF : c.d, 1, (uint64_t)c.d * c.sharedF,
                         L.sharedScales + (down ? (uint64_t)(c.sharedF / 8) * 16 * padded_groups(c.d / 64) : 0), 0, error))
             return false;
@@ -722,8 +874,8 @@ bool launch_block_int8(FFContext *ctx, const LayerStore &L, const uint16_t *x, u
         k.outStride = down ? c.d : c.sharedF;
         BlockMaps maps;
         memcpy(&maps, Lm.blockMap[mode], sizeof(maps));
-        const bool ok = down ? launch_kernel<kDown, true>(ctx, a, maps, "shared_int8_down", stream, error)
-                             : launch_kernel<kGateUp, true>(ctx, a, maps, "shared_int8_gate_up_act", stream, error);
+        const bool ok = down ? launch_kernel<kDown, true>(ctx, redo, maps, "shared_int8_down", stream, error)
+                             : launch_kernel<kGateUp, true>(ctx, redo, maps, "shared_int8_gate_up_act", stream, error);
         if (!ok) return false;
     }
     return true;
