@@ -77,14 +77,6 @@ struct alignas(64) BlockMaps {
 };
 static_assert(sizeof(BlockMaps) == sizeof(LayerStore::blockMap[0]), "copied as one");
 
-__device__ __forceinline__ void box3(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar)
-        : "memory");
-}
-
 // ---- INT8: four groups of a tile against NT pairs of input rows ------------------------------------
 //
 // lo / hi: this lane's 16 codes of tile rows g and g + 8 per group, dig[j] its digits of pair j (columns 0..3 one row, 4..7
@@ -476,9 +468,9 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps, const __g
             const uint32_t slot = slots + (asked & 1u) * a.slotBytes, bar = bars + 8u * (asked & 1u);
             const int row = (int)askAt.tile * (MODE == kGateUp ? 8 : 16), x = (int)(askX * (kGroupBytes / 8u));
             bar_expect(bar, askBytes);
-            box3(slot, askMap, x, row, askZ, bar);
-            if (MODE == kGateUp) box3(slot + askHalf, askMap + 1, x, row, askZ, bar);
-            box3(slot + a.sbOffset, askMap + 2, (int)askX, (int)askAt.tile * 16, askZ, bar);
+            tma_load_3d(slot, askMap, x, row, askZ, bar);
+            if (MODE == kGateUp) tma_load_3d(slot + askHalf, askMap + 1, x, row, askZ, bar);
+            tma_load_3d(slot + a.sbOffset, askMap + 2, (int)askX, (int)askAt.tile * 16, askZ, bar);
         }
         ++asked;
         askX += askPart;
@@ -704,14 +696,9 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps, const __g
 
 bool encode3(CUtensorMap *map, CUtensorMapDataType type, const void *base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1,
              uint64_t s2, uint32_t b0, uint32_t b1, const char **error) {
-    EncodeTiledFn fn = encode_tiled(error);
-    if (!fn) return false;
     const cuuint64_t dims[3] = {d0, d1, d2}, strides[2] = {s1, s2};
-    const cuuint32_t box[3] = {b0, b1, 1}, elem[3] = {1, 1, 1};
-    const CUresult rc = fn(map, type, 3, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rc != CUDA_SUCCESS) return fail(error, "cuTensorMapEncodeTiled(block) failed: " + std::to_string((int)rc));
-    return true;
+    const cuuint32_t box[3] = {b0, b1, 1};
+    return encode_map(map, type, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE, "block", error);
 }
 
 // Slot row pitch of a kind: a part's bytes, padded so that a half-warp's reads fall on different banks

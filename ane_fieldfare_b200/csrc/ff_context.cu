@@ -86,7 +86,7 @@ void ff_destroy(FFContext *ctx) {
     void *ptrs[] = {ctx->logits, ctx->ids, ctx->weights, ctx->plan, ctx->routerCounts, ctx->acts, ctx->sharedActs, ctx->h1,
                     ctx->partials, ctx->xDev, ctx->yDev, ctx->xSorted, ctx->xShared, ctx->rowOfRoute, ctx->sortedPairs,
                     ctx->expertOffsets, ctx->blockCounts, ctx->units, ctx->unitCount,
-                    ctx->errorFlag, ctx->gridBarrier, ctx->phaseStamps, ctx->mapScratch, ctx->taggedLogits, ctx->taggedActs,
+                    ctx->errorFlag, ctx->gridBarrier, ctx->phaseStamps, ctx->taggedLogits, ctx->taggedActs,
                     ctx->logitsRows, ctx->xSums, ctx->actSums, ctx->routerParts, ctx->decodeValues};
     for (void *p : ptrs) cudaFree(p);
     if (ctx->hostStream) cudaStreamDestroy(ctx->hostStream);

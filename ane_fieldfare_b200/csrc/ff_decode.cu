@@ -160,16 +160,6 @@ __device__ __forceinline__ void warp_stamp(const DecodeArgs &a, int phase, int w
     }
 }
 
-// Box of a row-box map at (64-bit word x, row y, expert z) into shared memory (128-byte aligned).
-// x * 8 bytes must be a multiple of 16.
-__device__ __forceinline__ void box_copy(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar)
-        : "memory");
-}
-
 // Rows of bf16 values as digits (flat run index over all rows) by `threads` threads, this one number
 // `tid`; fetch(i, j, v, w) reads runs i and j (negative: none).  Rows of `groups` groups have their aux
 // entries `auxGroups` apart (0: one row).  No barrier at the end.
@@ -387,8 +377,8 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
         if (lane == 0) {
             bar_expect(myBar, (ge > gb ? 16u * pitch : 0u) + (part == 0 ? 4u * wordsGU : 0u));
             if (ge > gb) {
-                box_copy(slot, gateMap, gb * 4, tile * 8, expert, myBar);
-                box_copy(slot + 8u * pitch, upMap, gb * 4, tile * 8, expert, myBar);
+                tma_load_3d(slot, gateMap, gb * 4, tile * 8, expert, myBar);
+                tma_load_3d(slot + 8u * pitch, upMap, gb * 4, tile * 8, expert, myBar);
             }
             if (part == 0) bulk_copy(sb, words + (size_t)tile * wordsGU, 4u * wordsGU, myBar);
         }
@@ -408,7 +398,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
         even_range(groupsFs, 3, part, gb, ge);
         if (lane == 0) {
             bar_expect(myBar, (ge > gb ? 16u * a.strideSD : 0u) + (part == 0 ? 4u * wordsSD : 0u));
-            if (ge > gb) box_copy(slot, &maps.m[kMapSharedDown], gb * 4, tile * 16, 0, myBar);
+            if (ge > gb) tma_load_3d(slot, &maps.m[kMapSharedDown], gb * 4, tile * 16, 0, myBar);
             if (part == 0) bulk_copy(tripleBase + 48u * a.strideSD, a.sharedScales + (Fs >> 3) * wordsGU + (size_t)tile * wordsSD, 4u * wordsSD, myBar);
         }
         __syncwarp();
@@ -609,7 +599,7 @@ __device__ __forceinline__ void decode_body(const DecodeArgs &a, const DecodeMap
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const uint32_t id = sIds[i ? eHi : eLo];
-                box_copy(downSlot + (uint32_t)i * 8u * a.strideRD, &maps.m[kMapRoutedDown], 0, tile * 8, (int)id, myBar);
+                tma_load_3d(downSlot + (uint32_t)i * 8u * a.strideRD, &maps.m[kMapRoutedDown], 0, tile * 8, (int)id, myBar);
                 bulk_copy(downSlot + 16u * a.strideRD + (uint32_t)i * 4u * wordsRD,
                           a.scales + (size_t)id * a.scaleStride + (F >> 3) * wordsGU + (size_t)tile * wordsRD, 4u * wordsRD, myBar);
             }

@@ -8,7 +8,6 @@ namespace ff {
 
 constexpr int kGemvThreads = 256;
 constexpr int kRowsPerItem = (kGemvThreads / 32) * 4;
-constexpr int kDecodeDownRows = 8;  // output rows per CTA of the decode combine kernel
 
 __device__ __forceinline__ float bf2f(uint16_t b) { return __uint_as_float((uint32_t)b << 16); }
 
@@ -211,10 +210,8 @@ __device__ __forceinline__ void chunk_accumulate(const uint4 &v0, const uint4 &v
 }
 
 // One weight row (or a gate/up row pair) against NT staged input rows; returns the full sums in
-// every lane of the row's eight-lane group.  SMEM: the weight pointers address a copy of the rows
-// in shared memory (plain loads) instead of global memory (streaming loads).  `live` false skips the loads but keeps the
-// shuffles convergent.
-template <int NT, bool DUAL, bool SMEM = false>
+// every lane of the row's eight-lane group.  `live` false skips the loads but keeps the shuffles convergent.
+template <int NT, bool DUAL>
 __device__ __forceinline__ void row_dot(const uint8_t *w0, const uint16_t *s0, const uint16_t *b0,
                                         const uint8_t *w1, const uint16_t *s1, const uint16_t *b1,
                                         int row, int cols, bool live, const float *xs,
@@ -244,10 +241,10 @@ __device__ __forceinline__ void row_dot(const uint8_t *w0, const uint16_t *s0, c
         uint4 v0b[kDepth], v1b[kDepth];
         uint32_t sb0[kDepth], sb1[kDepth];  // scale | bias << 16
         auto fetch = [&](int c, int slot) {
-            v0b[slot] = SMEM ? p0[c] : load_stream(p0 + c);
+            v0b[slot] = load_stream(p0 + c);
             sb0[slot] = (uint32_t)sr0[c >> 1] | ((uint32_t)br0[c >> 1] << 16);
             if (DUAL) {
-                v1b[slot] = SMEM ? p1[c] : load_stream(p1 + c);
+                v1b[slot] = load_stream(p1 + c);
                 sb1[slot] = (uint32_t)sr1[c >> 1] | ((uint32_t)br1[c >> 1] << 16);
             }
         };

@@ -468,26 +468,16 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
     }
 }
 
-bool make_map(CUtensorMap *map, CUtensorMapDataType type, uint32_t rank, const void *base, const cuuint64_t *dims,
-              const cuuint64_t *strides, const cuuint32_t *box, CUtensorMapSwizzle swizzle, const char **error) {
-    EncodeTiledFn fn = encode_tiled(error);
-    if (!fn) return false;
-    const cuuint32_t elem[3] = {1, 1, 1};
-    const CUresult rc = fn(map, type, rank, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rc != CUDA_SUCCESS) return fail(error, "cuTensorMapEncodeTiled(INT8 GEMM) failed: " + std::to_string((int)rc));
-    return true;
-}
 // bf16 rows [rows][k], box of a CTA's half tile x 64 values; rows past the end read as zero
 bool make_token_map(CUtensorMap *map, const uint16_t *base, uint64_t rows, uint64_t k, uint64_t stride, const char **error) {
     const cuuint64_t dims[2] = {k, rows}, strides[1] = {stride * 2};
     const cuuint32_t box[2] = {kStepK, kMaxRows / 2};
-    return make_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, error);
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, "INT8 GEMM", error);
 }
 bool make_code_map(CUtensorMap *map, const uint8_t *base, uint64_t rows, uint64_t k, const char **error) {
     const cuuint64_t dims[3] = {k, rows, 1}, strides[2] = {k, k * rows};
     const cuuint32_t box[3] = {kStepK, 64, 1};
-    return make_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B, error);
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B, "INT8 GEMM", error);
 }
 
 // Tokens per tile: the size whose waves of units take the least time, at about 130 cycles a step plus
@@ -527,7 +517,6 @@ bool launch_one(FFContext *ctx, const CUtensorMap &tok, const CUtensorMap &sums,
                               tok, sums, w0, w1, args),
                    error);
     }
-    FF_CUDA_OK(cudaGetLastError(), error);
     return true;
 }
 
@@ -550,7 +539,6 @@ bool launch_shared_int8_gemm(FFContext *ctx, const LayerStore &L, const uint16_t
                               x, xStride, tokens, c.d, ctx->xSums),
                    error);
     }
-    FF_CUDA_OK(cudaGetLastError(), error);
     CUtensorMap tok, sums, w[2];
     Int8GemmArgs a{};
     for (int m = 0; m < 2; ++m) {

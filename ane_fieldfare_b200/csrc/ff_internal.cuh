@@ -198,7 +198,6 @@ struct FFContext {
     uint32_t *gridBarrier = nullptr;        // device: counters of the fused decode kernel (eight 64-bit, then eight 32-bit)
     volatile unsigned long long *mailbox = nullptr;  // pinned host word the decode kernel reports to
     uint32_t hostEpoch = 0;
-    CUtensorMap *mapScratch = nullptr;
 
     // tracing: CUDA events around every kernel launch, aggregated per kernel name
     bool tracing = false;

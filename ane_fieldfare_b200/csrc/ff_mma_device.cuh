@@ -5,6 +5,7 @@
 
 #include "ff_gemv_device.cuh"
 #include "ff_internal.cuh"
+#include "ff_tc_device.cuh"
 
 namespace ff {
 
@@ -19,19 +20,6 @@ __device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
 }
 __device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool bar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
 }
 // 16-byte aligned source and destination, size a multiple of 16.
 __device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
@@ -50,13 +38,13 @@ __device__ __forceinline__ void slot_release() { __syncwarp(); }
 // and the warp carries on (its rows are then wrong, the launch still ends).
 static __device__ __noinline__ bool slot_wait_slow(uint32_t bar, uint32_t parity) {
     bool done = false;
-    for (uint32_t i = 0; i < kCopySpinLimit && !done; ++i) done = bar_try_wait(bar, parity);
+    for (uint32_t i = 0; i < kCopySpinLimit && !done; ++i) done = mbar_try_wait(bar, parity);
     return done;
 }
 // (The first poll stands alone: a poll inside the bounded loop measured about 200 cycles on a
 // barrier that was already complete, a stand-alone one 7.)
 __device__ __forceinline__ void slot_wait(uint32_t bar, uint32_t &parity, uint32_t *errorFlag) {
-    bool done = bar_try_wait(bar, parity);
+    bool done = mbar_try_wait(bar, parity);
     if (!done) done = slot_wait_slow(bar, parity);
     if (!done && (threadIdx.x & 31) == 0) atomicExch(errorFlag, 10u);
     parity ^= 1u;

@@ -62,28 +62,15 @@ constexpr int kRouterBlockK = 256;  // inputs per streamed block: one step of ev
 constexpr int kRouterRing = 8;      // blocks in flight
 constexpr uint32_t kRouterBlockBytes = kRouterExperts * kRouterBlockK * 2;
 
-__device__ __forceinline__ bool rt_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 static __device__ __noinline__ bool rt_wait_slow(uint32_t bar, uint32_t parity) {
     bool done = false;
-    for (uint32_t spin = 0; spin < (1u << 22) && !done; ++spin) done = rt_try_wait(bar, parity);
+    for (uint32_t spin = 0; spin < (1u << 22) && !done; ++spin) done = mbar_try_wait(bar, parity);
     return done;
 }
 // bounded; the first poll stands alone (inside the bounded loop it costs about 200 cycles even
 // when the barrier is complete)
 __device__ __forceinline__ bool rt_wait(uint32_t bar, uint32_t parity) {
-    return rt_try_wait(bar, parity) || rt_wait_slow(bar, parity);
+    return mbar_try_wait(bar, parity) || rt_wait_slow(bar, parity);
 }
 
 template <int kTok>
@@ -410,7 +397,7 @@ constexpr uint32_t kNoRow = 0xFFFFFFFFu;  // of a route to no expert
 // this block + earlier in this warp's segment (earlier 32-route batches, then lower lanes).
 // `base`: of expert threadIdx.x, the first two terms.
 __device__ __forceinline__ void place_routes(const uint32_t *sRoutes, uint32_t *segCount, int n, int seg, uint32_t base,
-                                             const uint16_t *weights, int t0, int K, int E, FFTokenExpertPair *sorted,
+                                             int t0, int K, int E, FFTokenExpertPair *sorted,
                                              uint32_t *rowOfRoute) {
     const int e = threadIdx.x;
     if (e < E) {
@@ -438,8 +425,7 @@ __device__ __forceinline__ void place_routes(const uint32_t *sRoutes, uint32_t *
         __syncwarp();
         if (live) {
             const uint32_t token = (uint32_t)(t0 + i / K), rank = (uint32_t)(i % K);
-            const uint32_t wbits = weights ? (uint32_t)weights[(size_t)token * K + rank] : 0u;
-            sorted[pos] = FFTokenExpertPair{token, ex, rank, wbits};
+            sorted[pos] = FFTokenExpertPair{token, ex, rank, 0u};
         }
         if (rowOfRoute && valid) rowOfRoute[(size_t)t0 * K + i] = live ? pos : kNoRow;
     }
@@ -447,7 +433,7 @@ __device__ __forceinline__ void place_routes(const uint32_t *sRoutes, uint32_t *
 
 // Pass 3.
 __global__ void __launch_bounds__(256)
-k_route_scatter(const uint32_t *ids, const uint16_t *weights, int T, int K, int E,
+k_route_scatter(const uint32_t *ids, int T, int K, int E,
                 const uint32_t *blockCounts, const uint32_t *expertOffsets,
                 FFTokenExpertPair *sorted, uint32_t *rowOfRoute) {
     pdl_enter();
@@ -462,7 +448,7 @@ k_route_scatter(const uint32_t *ids, const uint16_t *weights, int T, int K, int 
     segment_histogram(sRoutes, n, seg, E, segCount);
     __syncthreads();
     const int e = threadIdx.x;
-    place_routes(sRoutes, segCount, n, seg, e < E ? expertOffsets[e] + blockCounts[(size_t)blockIdx.x * E + e] : 0u, weights, t0, K, E,
+    place_routes(sRoutes, segCount, n, seg, e < E ? expertOffsets[e] + blockCounts[(size_t)blockIdx.x * E + e] : 0u, t0, K, E,
                  sorted, rowOfRoute);
 }
 
@@ -485,7 +471,7 @@ k_route_sort(const uint32_t *ids, int T, int K, int E, uint32_t *expertOffsets, 
     if (e < E)
         for (int w = 0; w < 8; ++w) total += segCount[w * E + e];
     const uint32_t start = plan_row_tiles(total, E, expertOffsets, tiles, maxTiles, counts);
-    place_routes(sRoutes, segCount, n, seg, start, nullptr, 0, K, E, sorted, rowOfRoute);
+    place_routes(sRoutes, segCount, n, seg, start, 0, K, E, sorted, rowOfRoute);
 }
 
 // Row tiles of a dense problem: T rows of one "expert" (the shared FFN).
@@ -1109,34 +1095,20 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
 // tile that one CTA of a pair holds), 128-byte swizzle.
 static bool make_activation_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t k,
                                 uint64_t strideElems, uint32_t boxRows, const char **error) {
-    EncodeTiledFn fn = encode_tiled(error);
-    if (!fn) return false;
     cuuint64_t dims[2] = {k, rows};
     cuuint64_t strides[1] = {strideElems * 2};
     cuuint32_t box[2] = {(cuuint32_t)kTileK, boxRows};
-    cuuint32_t elem[2] = {1, 1};
-    CUresult rc = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides,
-                     box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rc != CUDA_SUCCESS) return fail(error, "cuTensorMapEncodeTiled(activations) failed: " + std::to_string((int)rc));
-    return true;
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, "activations", error);
 }
 
 // router matrix bf16 [experts][d]: boxes of 256 inputs x 8 experts, no swizzle; parts of a box past
 // the matrix read as zero.
 static bool make_router_map(CUtensorMap *map, const void *base, uint64_t experts, uint64_t d, const char **error) {
-    EncodeTiledFn fn = encode_tiled(error);
-    if (!fn) return false;
     if ((reinterpret_cast<uintptr_t>(base) & 15u) || (d * 2) % 16) return fail(error, "router rows must be 16-byte aligned");
     cuuint64_t dims[2] = {d, experts};
     cuuint64_t strides[1] = {d * 2};
     cuuint32_t box[2] = {(cuuint32_t)kRouterBlockK, (cuuint32_t)kRouterExperts};
-    cuuint32_t elem[2] = {1, 1};
-    CUresult rc = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, elem,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rc != CUDA_SUCCESS) return fail(error, "cuTensorMapEncodeTiled(router) failed: " + std::to_string((int)rc));
-    return true;
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE, "router", error);
 }
 
 // Packed codes of one matrix across all experts seen as 64-bit words [experts][rows][rowBytes/8],
@@ -1144,19 +1116,12 @@ static bool make_router_map(CUtensorMap *map, const void *base, uint64_t experts
 // `boxBytes` apart in shared memory.  Out-of-range parts of a box read as zero.
 bool make_row_box_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t rowBytes, uint64_t experts,
                       uint64_t expertStride, uint32_t boxBytes, uint32_t boxRows, const char **error) {
-    EncodeTiledFn fn = encode_tiled(error);
-    if (!fn) return false;
     if (rowBytes % 16 || boxBytes % 16 || boxBytes / 8 > 256 || boxRows > 256 || expertStride % 16)
         return fail(error, "row box does not fit a tensor map");
     cuuint64_t dims[3] = {rowBytes / 8, rows, experts};
     cuuint64_t strides[2] = {rowBytes, expertStride ? expertStride : rows * rowBytes};
     cuuint32_t box[3] = {boxBytes / 8, boxRows, 1};
-    cuuint32_t elem[3] = {1, 1, 1};
-    CUresult rc = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<void *>(base), dims, strides, box, elem,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rc != CUDA_SUCCESS) return fail(error, "cuTensorMapEncodeTiled(row boxes) failed: " + std::to_string((int)rc));
-    return true;
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE, "row boxes", error);
 }
 
 // Packed codes of one matrix across all experts: bytes [experts][rows][cols/2], box 64 rows x 128 bytes (four
@@ -1164,17 +1129,10 @@ bool make_row_box_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_
 // bank twice.  (Boxes of one step's 32 bytes kept the copying thread busy for 600 cycles a step.)
 static bool make_weight_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols,
                             uint64_t experts, uint64_t expertStride, const char **error) {
-    EncodeTiledFn fn = encode_tiled(error);
-    if (!fn) return false;
     cuuint64_t dims[3] = {cols / 2, rows, experts};
     cuuint64_t strides[2] = {cols / 2, expertStride};
     cuuint32_t box[3] = {(cuuint32_t)(kQuad * kTileK / 2), 64, 1};
-    cuuint32_t elem[3] = {1, 1, 1};
-    CUresult rc = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void *>(base), dims, strides,
-                     box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rc != CUDA_SUCCESS) return fail(error, "cuTensorMapEncodeTiled(weights) failed: " + std::to_string((int)rc));
-    return true;
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, "weights", error);
 }
 
 bool prefill_prepare_layer(FFContext *ctx, LayerStore &L, const char **error) {
@@ -1236,7 +1194,6 @@ static bool launch_gemm(FFContext *ctx, const uint16_t *x, uint64_t rows, const 
                               mapA, mapASmall, mapW0, mapW1, args),
                    error);
     }
-    FF_CUDA_OK(cudaGetLastError(), error);
     return true;
 }
 
@@ -1269,7 +1226,7 @@ static bool sort_routes(FFContext *ctx, const uint32_t *ids, uint32_t tokens, in
                    error);
     }
     LaunchScope scope(ctx, stream, "route_scatter");
-    FF_CUDA_OK(launch_pdl(k_route_scatter, blocks, 256, sortSmem, stream, ids, nullptr, T, K, E, ctx->blockCounts, offsets, sorted,
+    FF_CUDA_OK(launch_pdl(k_route_scatter, blocks, 256, sortSmem, stream, ids, T, K, E, ctx->blockCounts, offsets, sorted,
                           rowOfRoute),
                error);
     return true;
@@ -1293,7 +1250,6 @@ bool launch_prefill_routed(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
                               x, xStride, tokens, ctx->rowOfRoute, K, (int)c.d, ctx->xSorted),
                    error);
     }
-    FF_CUDA_OK(cudaGetLastError(), error);
 
     const uint32_t tileBound = pairs / kRowTile + (uint32_t)E;
     const uint64_t rows = (uint64_t)pairs + 256;
@@ -1362,7 +1318,6 @@ bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
                               x, xStride, tokens, nullptr, 0, (int)c.d, ctx->xShared),
                    error);
     }
-    FF_CUDA_OK(cudaGetLastError(), error);
     const uint32_t rowTiles = (tokens + kRowTile - 1) / kRowTile;
     const uint64_t rows = (uint64_t)tokens + 256;
     GemmArgs a{};

@@ -602,15 +602,9 @@ k_router_int8_lanes(const uint8_t *Q, const uint16_t *qScale, const uint16_t *qB
 
 bool router_map(CUtensorMap *map, const uint16_t *base, uint64_t rows, uint64_t d, uint64_t stride, uint32_t boxRows,
                 const char **error) {
-    EncodeTiledFn fn = encode_tiled(error);
-    if (!fn) return false;
     const cuuint64_t dims[2] = {d, rows}, strides[1] = {stride * 2};
-    const cuuint32_t box[2] = {kApproxK, boxRows}, elem[2] = {1, 1};
-    const CUresult rc = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t *>(base), dims, strides, box, elem,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rc != CUDA_SUCCESS) return fail(error, "cuTensorMapEncodeTiled(router) failed: " + std::to_string((int)rc));
-    return true;
+    const cuuint32_t box[2] = {kApproxK, boxRows};
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, "router", error);
 }
 
 }  // namespace
@@ -664,7 +658,6 @@ bool launch_router_select(FFContext *ctx, const LayerStore &L, const uint16_t *x
                                                                                          splits, ctx->routerParts, ctx->errorFlag),
                    error);
     }
-    FF_CUDA_OK(cudaGetLastError(), error);
     SelectArgs a{};
     a.W = L.routerW;
     a.Q = reinterpret_cast<const uint4 *>(L.routerLanes);
@@ -696,7 +689,6 @@ bool launch_router_select(FFContext *ctx, const LayerStore &L, const uint16_t *x
                               a),
                    error);
     }
-    FF_CUDA_OK(cudaGetLastError(), error);
     return true;
 }
 
@@ -717,7 +709,6 @@ bool launch_router_logits_int8(FFContext *ctx, const LayerStore &L, const uint16
                               lanes, L.routerAux, L.routerScale, L.logitBias, x, xStride, (int)tokens, E, D, logits, tail),
                    error);
     }
-    FF_CUDA_OK(cudaGetLastError(), error);
     return true;
 }
 

@@ -80,6 +80,7 @@ __device__ __forceinline__ bool mbar_wait_idle(uint32_t bar, uint32_t parity, vo
     return mbar_try_wait<kOrder>(bar, parity) || mbar_wait_slow<true, kOrder>(bar, parity, abortFlag);
 }
 
+// Box of a map at (x, y[, z]) into shared memory (128-byte aligned); x times the element's size a multiple of 16.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y,
                                             uint32_t bar) {
     asm volatile(
@@ -254,6 +255,18 @@ inline EncodeTiledFn encode_tiled(const char **error) {
     }();
     if (!fn) fail(error, "cuTensorMapEncodeTiled is not available from the driver");
     return fn;
+}
+
+// A map of `rank` dimensions without element strides; parts of a box past the tensor read as zero.
+inline bool encode_map(CUtensorMap *map, CUtensorMapDataType type, uint32_t rank, const void *base, const cuuint64_t *dims,
+                       const cuuint64_t *strides, const cuuint32_t *box, CUtensorMapSwizzle swizzle, const char *what, const char **error) {
+    const EncodeTiledFn fn = encode_tiled(error);
+    if (!fn) return false;
+    const cuuint32_t elem[3] = {1, 1, 1};
+    const CUresult rc = fn(map, type, rank, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (rc != CUDA_SUCCESS) return fail(error, std::string("cuTensorMapEncodeTiled(") + what + ") failed: " + std::to_string((int)rc));
+    return true;
 }
 
 }  // namespace ff
