@@ -200,7 +200,7 @@ FFContext *ff_create(int32_t deviceOrdinal, const FFConfig *config, const char *
         ok = ok && dev_alloc(ctx, &ctx->expertOffsets, c.experts + 1, error);
         ok = ok && dev_alloc(ctx, &ctx->blockCounts, (permuteBlocks + 1) * c.experts, error);
         ok = ok && dev_alloc(ctx, &ctx->units, (size_t)ctx->maxUnits * 4, error);
-        ok = ok && dev_alloc(ctx, &ctx->routerParts, router_parts_rows(T) * c.experts, error);
+        ok = ok && dev_alloc(ctx, &ctx->routerParts, router_parts_rows(T, ctx->smCount) * c.experts, error);
         ok = ok && dev_alloc(ctx, &ctx->unitCount, 8, error);
         if (ok) ok = cudaMemset(ctx->unitCount, 0, 32) == cudaSuccess;
     }

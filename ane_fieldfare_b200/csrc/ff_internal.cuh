@@ -344,7 +344,7 @@ bool launch_router_prefill(FFContext *ctx, const LayerStore &L, const uint16_t *
                            float *logits, cudaStream_t stream, const char **error);
 
 // ff_router.cu
-size_t router_parts_rows(size_t maxTokens);
+size_t router_parts_rows(size_t maxTokens, int smCount);
 bool router_prepare(FFContext *ctx, LayerStore &L, const char **error);
 bool launch_router_select(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens,
                           uint32_t *ids, uint16_t *weights, cudaStream_t stream, const char **error);

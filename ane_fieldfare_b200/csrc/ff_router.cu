@@ -35,7 +35,6 @@ constexpr int kApproxStages = 3;
 constexpr uint32_t kExpertTile = 128, kApproxK = 64;
 constexpr uint32_t kExpertBytes = kExpertTile * kApproxK * 2;
 constexpr uint32_t kMaxSplits = 8;   // parts of the contraction, summed by the selecting kernel
-constexpr uint32_t kSplitTiles = 148;  // tiles x splits aim at one CTA per SM
 constexpr int kApproxThreads = 192;  // warp 0 copies, warp 1 MMAs, warps 2-5 write out
 
 __device__ __forceinline__ void mma_bf16_ss(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t idesc, uint32_t accumulate) {
@@ -611,8 +610,8 @@ bool router_map(CUtensorMap *map, const uint16_t *base, uint64_t rows, uint64_t 
 
 // Rows of partial logits a context of `maxTokens` can need: splits are used only while the token
 // tiles leave SMs idle.
-size_t router_parts_rows(size_t maxTokens) {
-    return std::min<size_t>(maxTokens * kMaxSplits, std::max<size_t>(maxTokens, (size_t)kSplitTiles * 128));
+size_t router_parts_rows(size_t maxTokens, int smCount) {
+    return std::min<size_t>(maxTokens * kMaxSplits, std::max<size_t>(maxTokens, (size_t)smCount * 128));
 }
 
 bool router_prepare(FFContext *ctx, LayerStore &L, const char **error) {
@@ -641,7 +640,7 @@ bool launch_router_select(FFContext *ctx, const LayerStore &L, const uint16_t *x
     const uint32_t tileTokens = std::min(128u, (tokens + 31u) & ~31u);
     const uint32_t tiles = (tokens + tileTokens - 1) / tileTokens, expertTiles = (E + kExpertTile - 1) / kExpertTile;
     const uint32_t steps = D / kApproxK;
-    uint32_t splits = std::max(1u, std::min({kMaxSplits, kSplitTiles / std::max(1u, tiles * expertTiles), steps}));
+    uint32_t splits = std::max(1u, std::min({kMaxSplits, (uint32_t)ctx->smCount / std::max(1u, tiles * expertTiles), steps}));
     splits = (steps + (steps + splits - 1) / splits - 1) / ((steps + splits - 1) / splits);  // no empty split
     CUtensorMap mapW, mapX;
     if (!router_map(&mapW, L.routerFolded ? L.routerFolded : L.routerW, E, D, D, kExpertTile, error) ||
@@ -676,8 +675,13 @@ bool launch_router_select(FFContext *ctx, const LayerStore &L, const uint16_t *x
     a.parts = ctx->routerParts;
     a.ids = ids;
     a.weights = weights;
-    // One warp a row (INT8: two) once that fills the GPU (32 warps an SM), more where rows are few.
-    a.warpsPerRow = tokens >= 8192 && !L.routerQ ? 1 : tokens >= 2048 ? 2 : tokens >= 1024 ? 4 : 8;
+    // As many warps a row as keep the rows in one wave (the launch bounds give 24 warps an SM, 32 for INT8), INT8 two
+    // at least.  bf16, us of this kernel with 8 / 4 / 2 / 1 warps: 77 rows 14.8 / 18.9 / 20.9 / 21.0, 512 rows 23.0 / 18.9 /
+    // 19.0 / 23.0, 1500 rows 39.4 / 31.1 / 23.1 / 25.1, 2048 rows 49.5 / 39.3 / 33.2 / 27.1; INT8 with 8 / 4 / 2: 512 rows
+    // 25.0 / 26.0 / 35.4, 1024 rows 37.3 / 33.2 / 39.4, 2048 rows 57.9 / 51.8 / 49.7.
+    const uint32_t resident = (uint32_t)ctx->smCount * (L.routerQ ? 32u : 24u);
+    a.warpsPerRow = kSelectWarps;
+    while (a.warpsPerRow > (L.routerQ ? 2u : 1u) && (uint64_t)tokens * a.warpsPerRow > resident) a.warpsPerRow /= 2;
     const uint32_t perCta = kSelectWarps / a.warpsPerRow;
     const size_t rowBytes = (size_t)D * (L.routerQ ? 4 : 2);
     auto kernel = L.routerQ ? k_router_select<true> : k_router_select<false>;
