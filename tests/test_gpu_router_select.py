@@ -98,3 +98,30 @@ def test_selected_routes_of_tiny_and_huge_rows(form, weights_times):
         assert torch.equal(weights[0].view(torch.int16), weights[1].view(torch.int16))
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("form", ["bf16", "int8"])
+@pytest.mark.parametrize("rows", [443, 445, 1184, 1777, 4000])
+def test_selected_routes_at_every_number_of_warps(form, rows):
+    """Rows on either side of where a row gets fewer warps (148 SMs: 444, 888, 1776 rows; INT8 592, 1184)."""
+    from ane_fieldfare_b200 import hotpath as hp
+    experts, d, k = 64, 192, 6
+    ctx = hp.HotpathContext(layers=1, experts=experts, d=d, f=64, sharedF=0, topK=k, maxTokens=rows)
+    try:
+        if form == "int8":
+            ctx.loadRouterInt8(0, *int8_router(0x3A, experts, d))
+        else:
+            ctx.loadRouter(0, synth.normal_bf16(0x3B, "warps.router", (experts, d), 0.02))
+        x = hp.bf16_tensor(workload.make_tokens(0x3C, f"warps{rows}", rows, d), ctx.device)
+        got = [torch.full((rows, k), -1, dtype=torch.int32, device=ctx.device) for _ in range(2)]
+        weights = [torch.zeros((rows, k), dtype=torch.bfloat16, device=ctx.device) for _ in range(2)]
+        logits = torch.zeros((rows, experts), dtype=torch.float32, device=ctx.device)
+        router = hp.PrefillRouter(ctx)
+        router.encodeGemma4Block(None, 0, x, got[0], weights[0], rows, outLogits=logits)
+        router.encodeGemma4Block(None, 0, x, got[1], weights[1], rows)
+        torch.cuda.synchronize()
+        assert ctx.info().deviceErrorFlag == 0
+        assert torch.equal(got[0], got[1])
+        assert torch.equal(weights[0].view(torch.int16), weights[1].view(torch.int16))
+    finally:
+        ctx.close()
