@@ -182,7 +182,7 @@ FFContext *ff_create(int32_t deviceOrdinal, const FFConfig *config, const char *
     if (ok && T > (size_t)kMaxGemvRows) {
         const size_t pairs = T * K;
         const size_t permuteBlocks = (T + 255) / 256;
-        // one work unit per (expert, 128-row tile, column tile); tiles <= pairs/128 + experts
+        // row tiles hold up to 192 rows of one expert (at most pairs / 192 + experts of them; room for pairs / 128)
         ctx->maxUnits = (uint32_t)(2 * (pairs / 128 + c.experts + 2));  // row tiles: routed half, dense half
         ok = ok && dev_alloc(ctx, &ctx->xSorted, (pairs + 256) * c.d, error);
         if (ok) ok = cudaMemset(ctx->xSorted, 0, (pairs + 256) * c.d * 2) == cudaSuccess;

@@ -10,14 +10,13 @@
 //      rows and the shared down rows; the routed down rows are requested as the warps finish;
 //   C  routed down rows and the fixed-order combine onto the shared output (or the caller's
 //      residual).
-// Values cross from CTA to CTA as tagged 64-bit words that the readers poll (logits, routed
-// activations, shared output rows: value and validity in one L2 round trip), and through one
-// arrival counter (the shared activations between A and B).
+// Values cross from CTA to CTA as tagged 64-bit words that the readers poll (logits, shared activations,
+// routed activations, shared output rows): value and validity in one L2 round trip, nothing is cleared.
+// Tile counters beside them are hints when it is worth polling a long row; they order nothing.
 //
-// Weight rows reach the SM as asynchronous copies (completion counted on a per-warp mbarrier)
-// into a per-warp shared-memory slot: cp.async.bulk.tensor over row-box maps of the layer where a
-// tile's rows lie at one stride (one request brings 8 or 16 row pieces), cp.async.bulk for scale
-// runs and for the routed down rows of the eight scattered experts.
+// Weight rows reach the SM as asynchronous copies (completion counted on a per-warp mbarrier) into a
+// per-warp shared-memory slot: cp.async.bulk.tensor over row-box maps of the layer (one request brings 8
+// or 16 row pieces of one matrix), cp.async.bulk for a tile's scale | bias words.
 //
 // Row arithmetic runs on the integer tensor cores straight on the codes (ff_int_device.cuh): a warp task
 // is a tile of 16 weight rows, two runs of eight — gate and up rows of the same features, sixteen rows
@@ -27,12 +26,11 @@
 // order, so results do not depend on scheduling.
 //
 // What bounds a step: the chain router row -> logits through L2 -> routes -> routed rows from HBM (3.8
-// us for 19.5 MB) -> activations through L2 -> down rows.  Turning nibbles into bf16 pairs used to add
-// 4.6 us behind the routed rows' arrival and 1.0 us of ranking stood in front of them (23.7 us a step).
+// us for 19.5 MB) -> activations through L2 -> down rows: 15.7 us a step in a graph (2396 GB/s).
 //
-// Grid-wide waits poll arrival counters in global memory; cooperative launch guarantees that all
-// CTAs are resident.  Every spin (grid barrier, copy completion) is bounded: on running
-// out it raises the context's error flag and carries on, so the launch always ends.
+// Cooperative launch guarantees that all CTAs are resident.  Every spin (tagged words, hints, copy
+// completion) is bounded: on running out it raises the context's error flag and carries on, so the
+// launch always ends.  Shapes past one CTA's shared memory take launch_decode_general.
 //
 // Reference kernels replaced (paths inside the reference project):
 //   Sources/ANEFieldfareHotpath/Metal/MoE/moe.metal:65-120,242-319,500-517,548-570,597-638

@@ -1,22 +1,21 @@
 // Prefill path of the INT4 MoE block: router for many rows, device-side permute (counting sort by
 // expert), and the grouped INT4 -> bf16 GEMMs on the 5th-generation tensor cores.
 //
-// GEMM scheme.  A work unit is (row tile of up to 128 expert-sorted rows, column tile of 256
-// outputs: 128 gate + 128 up rows, or 256 down rows).  The wide column tile halves the re-reads of
-// the activation tile from L2, which bound the narrower tilings.  Per 64-wide step along the contraction (= one quantization group):
-//   * one thread issues TMA loads: the activations' [128 x 64] bf16 tile (128-byte swizzle) and
-//     four [64 rows x 32 bytes] tiles of packed 4-bit codes, completing on an mbarrier;
-//   * sixteen warps turn the packed tile into the bf16 operand tile in shared memory, half a
-//     weight row per thread: codes -> bf16 pairs by a mask trick, then one bf16x2 fused multiply-add
-//     with the group's scale and bias (a single rounding of q*scale+bias), stored in the
-//     128-byte-swizzled K-major layout the MMA descriptor expects;
-//   * one thread issues four tcgen05.mma (M=128, N=256, K=16) accumulating in TMEM, then
-//     tcgen05.commit to free the stage;
-//   * four warps drain the finished accumulator from TMEM (tcgen05.ld), apply the epilogue
-//     (GeGLU to bf16 activations, or bf16 partial rows scattered to (token, rank)), while the
-//     next unit's MMAs fill the other accumulator buffer.
+// GEMM scheme.  Two CTAs of a cluster work as one tensor-core unit (cta_group::2, M = 256).  A unit of work
+// is (row tile of up to 192 expert-sorted rows, two neighbouring tiles of 128 weight rows, one in either CTA:
+// 64 gate + 64 up rows of the same features, or 128 down rows).  The dequantized weights are the MMA's A
+// operand in tensor memory, the rows (tokens) its B operand in shared memory, half of the tile in either CTA.
+// Per CTA and 64-wide step along the contraction (= one quantization group):
+//   * warp 0 copies the token half tile (128-byte swizzle), completing on the leader's step barrier; warp 26
+//     copies packed codes, four steps of 128 weight rows at a time;
+//   * sixteen warps in four groups, a group every fourth step, turn codes into bf16 pairs (one fused multiply-add
+//     with the group's scale and bias, a single rounding of q*scale+bias) and store them to tensor memory;
+//   * warp 1 of the leader issues four tcgen05.mma (K=16 each) into one of two accumulators of 192 columns,
+//     and one tcgen05.commit that frees the step's stages in both CTAs;
+//   * eight warps in two sets drain the finished accumulator (GeGLU to bf16 activations, or bf16 partial rows
+//     scattered to (token, rank)) while the next unit's MMAs fill the other one.
 // Within every aligned run of eight contraction elements the order is 0,4,1,5,2,6,3,7 in BOTH
-// operands (the mask trick yields codes j and j+4 side by side), which leaves every dot product
+// operands (a masked word yields codes j and j+4 side by side), which leaves every dot product
 // unchanged; the activation buffers this file writes use that order.
 //
 // Every wait on an mbarrier is bounded; a wait that runs out sets the context's error flag and
