@@ -136,3 +136,37 @@ def test_int8_rows(zeros, powers, rows):
         assert ctx.info().deviceErrorFlag == 0
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("where", ["input", "activation"])
+@pytest.mark.parametrize("rows", [1, 2, 7, 16])
+def test_layer_with_shared_ffn(oracle, rows, where):
+    """Routed experts and shared FFN of a layer call: the outlier's weights are zero everywhere, the oracle adds in fp32.
+    activation: a feature whose up row is 2^20 times the others, its group's down weights zero."""
+    from ane_fieldfare_b200 import hotpath as hp
+    from conftest import assert_layer_close, oracle_layer
+    d, f, fs, column = 1088, 192, 320, 70
+    L = workload.make_layer(0x94, 0, experts=8, d=d, f=f, sharedF=fs, topK=3)
+    L.blobs, L.sharedBlob = L.blobs.copy(), L.sharedBlob.copy()
+    for blob, layout, width in [(b, L.layout, f) for b in L.blobs] + [(L.sharedBlob, L.sharedLayout, fs)]:
+        for name in ("down",) if where == "activation" else ("gate", "up"):
+            for part in gturbo.sub_tensor(blob, layout, name)[1:]:
+                part.reshape(d if name == "down" else width, -1)[:, column // 64] = 0
+        if where == "activation":
+            for part in gturbo.sub_tensor(blob, layout, "up")[1:]:
+                part.reshape(width, -1)[column] += np.uint16(20 << 7)
+    x = workload.make_tokens(0x95, f"outlier.layer{rows}", rows, d).reshape(rows, d)
+    if where == "input":
+        L.routerW[:, column] = 0
+        x[0::2, column] = synth.bf16_bits(np.float32([2.0 ** 24]))
+    ctx = hp.HotpathContext(layers=1, experts=8, d=d, f=f, sharedF=fs, topK=3, maxTokens=16)
+    try:
+        workload.load_layer(ctx, 0, L)
+        y = ctx.moeLayer(0, hp.bf16_tensor(x, ctx.device))
+        torch.cuda.synchronize()
+        assert ctx.info().deviceErrorFlag == 0
+        want, *_ = oracle.moe_layer(oracle_layer(oracle, L), x, oracle.MODE_DECODE if rows == 1 else oracle.MODE_PARTIALS)
+        rel_l2, _, _ = assert_layer_close(hp.bf16_numpy(y), want, oracle, f"outlier in the {where}, layer rows={rows}")
+        assert rel_l2 < 2.0 ** -9  # both sides round the same sums to bf16: a share of neighbours, no more than the rounding itself
+    finally:
+        ctx.close()
