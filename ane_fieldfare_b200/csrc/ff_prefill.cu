@@ -2,21 +2,27 @@
 // expert), and the grouped INT4 -> bf16 GEMMs on the 5th-generation tensor cores.
 //
 // GEMM scheme.  Two CTAs of a cluster work as one tensor-core unit (cta_group::2, M = 256).  A unit of work
-// is (row tile of up to 192 expert-sorted rows, two neighbouring tiles of 128 weight rows, one in either CTA:
-// 64 gate + 64 up rows of the same features, or 128 down rows).  The dequantized weights are the MMA's A
+// is (row tile of up to 128 or 192 expert-sorted rows, two neighbouring tiles of 128 weight rows, one in either
+// CTA: 64 gate + 64 up rows of the same features, or 128 down rows).  The dequantized weights are the MMA's A
 // operand in tensor memory, the rows (tokens) its B operand in shared memory, half of the tile in either CTA.
-// Per CTA and 64-wide step along the contraction (= one quantization group):
-//   * warp 0 copies the token half tile (128-byte swizzle), completing on the leader's step barrier; warp 26
-//     copies packed codes, four steps of 128 weight rows at a time;
-//   * sixteen warps in four groups, a group every fourth step, turn codes into bf16 pairs (one fused multiply-add
+// The contraction goes in steps of 64 (one quantization group), handed over two at a time.  Per CTA:
+//   * warp 0 copies the token half tiles of a pair of steps (128-byte swizzle), completing on the leader's step
+//     barrier; warp 26 copies packed codes, four steps of 128 weight rows at a time;
+//   * sixteen warps in four groups, a group every fourth pair, turn codes into bf16 pairs (one fused multiply-add
 //     with the group's scale and bias, a single rounding of q*scale+bias) and store them to tensor memory;
-//   * warp 1 of the leader issues four tcgen05.mma (K=16 each) into one of two accumulators of 192 columns,
-//     and one tcgen05.commit that frees the step's stages in both CTAs;
+//   * warp 1 of the leader issues a pair's eight tcgen05.mma (K=16 each) into one of two accumulators of 128 or 192
+//     columns, and one tcgen05.commit that frees the pair's stages in both CTAs;
 //   * eight warps in two sets drain the finished accumulator (GeGLU to bf16 activations, or bf16 partial rows
 //     scattered to (token, rank)) while the next unit's MMAs fill the other one.
 // Within every aligned run of eight contraction elements the order is 0,4,1,5,2,6,3,7 in BOTH
 // operands (a masked word yields codes j and j+4 side by side), which leaves every dot product
 // unchanged; the activation buffers this file writes use that order.
+//
+// What bounds it: few rows an expert, the instructions of the dequantizing warps (a step is 160 instructions of each
+// of its four warps, 72 of them the conversion itself) and the issuing warp's 430 cycles beside the MMAs of a
+// hand-over; many, the tensor core, then the power limit.  With a hand-over every step, a group every fourth one: 77
+// rows 252 us for two layers, 4096 rows 678 us; in pairs with a group's addresses running along 218 and 653; a group
+// per pair, its slots fixed 203 and 634; tiles of 128 rows with eight weight stages 193 at 77 rows.
 //
 // Every wait on an mbarrier is bounded; a wait that runs out sets the context's error flag and
 // the whole CTA leaves its loops, frees its TMEM and returns.
@@ -266,7 +272,8 @@ bool launch_router_prefill(FFContext *ctx, const LayerStore &L, const uint16_t *
 
 constexpr int kSortTokens = 256;  // tokens per permute block
 
-constexpr uint32_t kRowTile = 192;  // rows of one expert per GEMM unit (accumulator columns)
+// rows of one expert per GEMM unit (accumulator columns): see routed_tile_rows and dense_tile_rows
+constexpr uint32_t kRowTile = 192, kRowTileSmall = 128;
 
 struct RowTile {
     uint32_t rowStart;  // first row in expert-sorted order
@@ -296,11 +303,11 @@ __device__ __forceinline__ void segment_histogram(const uint32_t *routes, int n,
 // The experts' offsets and row tiles (up to kRowTile rows of one expert each, experts ascending) from thread
 // e's number of routes to expert e (0 from E on); a CTA of 256 threads.  Returns the expert's offset.
 // counts[0] = row tiles, counts[1] = pairs, counts[2] = experts with at least one pair.
-__device__ __forceinline__ uint32_t plan_row_tiles(uint32_t total, int E, uint32_t *expertOffsets, RowTile *tiles, uint32_t maxTiles,
-                                                   uint32_t *counts) {
+__device__ __forceinline__ uint32_t plan_row_tiles(uint32_t total, int E, uint32_t tileRows, uint32_t *expertOffsets, RowTile *tiles,
+                                                   uint32_t maxTiles, uint32_t *counts) {
     __shared__ uint32_t warpSums[3][8];
     const int e = threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t myTiles = (total + kRowTile - 1u) / kRowTile;
+    const uint32_t myTiles = (total + tileRows - 1u) / tileRows;
     uint32_t rows = total, tileEnd = myTiles;  // inclusive sums
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -329,8 +336,8 @@ __device__ __forceinline__ uint32_t plan_row_tiles(uint32_t total, int E, uint32
     const uint32_t start = rows - total;
     if (e < E) {
         expertOffsets[e] = start;
-        for (uint32_t i = 0, tix = tileEnd - myTiles; i < total; i += kRowTile, ++tix)
-            if (tix < maxTiles) tiles[tix] = RowTile{start + i, min(kRowTile, total - i), (uint32_t)e, 0u};
+        for (uint32_t i = 0, tix = tileEnd - myTiles; i < total; i += tileRows, ++tix)
+            if (tix < maxTiles) tiles[tix] = RowTile{start + i, min(tileRows, total - i), (uint32_t)e, 0u};
     }
     if (e == 255) {
         expertOffsets[E] = rows;
@@ -365,7 +372,7 @@ k_route_count(const uint32_t *ids, int T, int K, int E, uint32_t *blockCounts) {
 
 // Pass 2 (one block): exclusive prefix of every expert's counts over the blocks, then the plan.
 __global__ void __launch_bounds__(256)
-k_route_scan(uint32_t *blockCounts, int blocks, int E, uint32_t *expertOffsets, RowTile *tiles,
+k_route_scan(uint32_t *blockCounts, int blocks, int E, uint32_t tileRows, uint32_t *expertOffsets, RowTile *tiles,
              uint32_t maxTiles, uint32_t *counts) {
     pdl_enter();
     uint32_t total = 0;
@@ -386,7 +393,7 @@ k_route_scan(uint32_t *blockCounts, int blocks, int E, uint32_t *expertOffsets, 
         }
         total = run;
     }
-    plan_row_tiles(total, E, expertOffsets, tiles, maxTiles, counts);
+    plan_row_tiles(total, E, tileRows, expertOffsets, tiles, maxTiles, counts);
 }
 
 constexpr uint32_t kNoRow = 0xFFFFFFFFu;  // of a route to no expert
@@ -454,7 +461,7 @@ k_route_scatter(const uint32_t *ids, int T, int K, int E,
 // All three passes for one block's worth of tokens: a chunk of up to 256 has one launch in front of its
 // gather instead of three (77 tokens: 14 us of a layer's 130 between the routes and the sorted list).
 __global__ void __launch_bounds__(256)
-k_route_sort(const uint32_t *ids, int T, int K, int E, uint32_t *expertOffsets, RowTile *tiles, uint32_t maxTiles, uint32_t *counts,
+k_route_sort(const uint32_t *ids, int T, int K, int E, uint32_t tileRows, uint32_t *expertOffsets, RowTile *tiles, uint32_t maxTiles, uint32_t *counts,
              FFTokenExpertPair *sorted, uint32_t *rowOfRoute) {
     pdl_enter();
     extern __shared__ uint32_t sRoutes[];
@@ -469,16 +476,16 @@ k_route_sort(const uint32_t *ids, int T, int K, int E, uint32_t *expertOffsets, 
     uint32_t total = 0;
     if (e < E)
         for (int w = 0; w < 8; ++w) total += segCount[w * E + e];
-    const uint32_t start = plan_row_tiles(total, E, expertOffsets, tiles, maxTiles, counts);
+    const uint32_t start = plan_row_tiles(total, E, tileRows, expertOffsets, tiles, maxTiles, counts);
     place_routes(sRoutes, segCount, n, seg, start, 0, K, E, sorted, rowOfRoute);
 }
 
 // Row tiles of a dense problem: T rows of one "expert" (the shared FFN).
-__global__ void k_dense_tiles(int T, RowTile *tiles, uint32_t *counts) {
+__global__ void k_dense_tiles(int T, int tileRows, RowTile *tiles, uint32_t *counts) {
     pdl_enter();
-    const int n = (T + (int)kRowTile - 1) / (int)kRowTile;
+    const int n = (T + tileRows - 1) / tileRows;
     for (int i = threadIdx.x; i < n; i += blockDim.x)
-        tiles[i] = RowTile{(uint32_t)i * kRowTile, (uint32_t)min((int)kRowTile, T - i * (int)kRowTile), 0u, 0u};
+        tiles[i] = RowTile{(uint32_t)(i * tileRows), (uint32_t)min(tileRows, T - i * tileRows), 0u, 0u};
     if (threadIdx.x == 0) {
         counts[0] = (uint32_t)n;
         counts[1] = (uint32_t)T;
@@ -530,11 +537,10 @@ k_gather_rows(const uint16_t *x, uint32_t xStride, uint32_t rows, const uint32_t
 
 constexpr int kWeightRows = 128;  // weight rows of a unit = TMEM lanes of its accumulator
 constexpr int kTileK = 64;        // one quantization group per step
-constexpr int kTokStages = 8;     // token half tiles (TMA destinations)
+constexpr int kTokStages = 4;     // token half tiles of two steps (TMA destinations)
 constexpr int kQuad = 4;          // steps whose packed codes come as one copy (128 bytes of a weight row)
-constexpr int kPackStages = 3;    // quads of packed codes in flight
-constexpr int kGroups = 4;        // dequantizing groups: one for each step of a quad
-constexpr int kWStages = kGroups; // dequantized weight tiles in TMEM, one per dequantizing group
+constexpr int kMaxPackStages = 6; // quads of packed codes in flight: as many as shared memory holds
+constexpr int kGroups = 4;        // dequantizing groups: one for each slot of the step ring
 constexpr int kDequantWarps = 16; // four groups of four warps; a group covers the 128 TMEM lanes
 constexpr int kEpilogueSets = 2;  // of four warps each, taking turns at 32-token chunks
 // warp 0 token copies, warp 1 MMA, warps 2-17 dequantize, warps 18-25 epilogue (TMEM lane quarter =
@@ -543,13 +549,9 @@ constexpr int kFirstEpilogueWarp = 2 + kDequantWarps;
 constexpr int kCodeWarp = kFirstEpilogueWarp + 4 * kEpilogueSets;
 constexpr int kGemmThreads = (kCodeWarp + 1) * 32;
 constexpr int kEpilogueThreads = 128 * kEpilogueSets;
-constexpr uint32_t kTokHalfRows = kRowTile / 2;                   // rows of a token tile held by either CTA of a pair
 constexpr uint32_t kTokSmallRows = 32;                            // of those, copied for a small tile
-constexpr uint32_t kTokTileBytes = kTokHalfRows * kTileK * 2;     // 12288 (a multiple of the 1024-byte swizzle atom)
 constexpr uint32_t kPackTileBytes = kWeightRows * kTileK / 2 * kQuad;  // 16384: two [64 rows x 128 bytes] boxes
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kAccCols = kRowTile;                           // accumulators at columns 0 and 192
-constexpr uint32_t kWCol0 = 2 * kAccCols;                         // weight stages: 32 columns each from 384
 constexpr uint32_t kStagePitchGateUp = 64 * 2 + 16;               // bytes per token row of the output tile
 constexpr uint32_t kStagePitchDown = 128 * 2 + 16;
 constexpr uint32_t kStageBytesGateUp = 32u * kStagePitchGateUp;   // one 32-token output tile
@@ -557,16 +559,23 @@ constexpr uint32_t kStageBytesDown = 32u * kStagePitchDown;
 // per set two output tiles; down: two row tables, too
 constexpr uint32_t kEpilogueBytesGateUp = kEpilogueSets * 2u * kStageBytesGateUp;
 constexpr uint32_t kEpilogueBytesDown = kEpilogueSets * 2u * kStageBytesDown + 2u * kRowTile * 4u;
-constexpr uint32_t kScaleSlotBytes = kDequantWarps * 32 * 4;      // a scale word of every dequantizing thread
-static_assert(kWCol0 + kWStages * 32 <= kTmemCols, "tensor memory layout");
-static_assert(kRowTile % 32 == 0 && kRowTile <= 256 && (int)kRowTile <= kEpilogueThreads, "row tile");
-static_assert(kQuad == kGroups, "a group takes one step of every quad");
+constexpr uint32_t kScaleSlotBytes = kDequantWarps * 32 * 8;      // two scale words of every dequantizing thread
+__host__ __device__ constexpr uint32_t scale_buffer_bytes(uint32_t quads) { return (quads + 1u) / 2u * kScaleSlotBytes; }
+// Dequantized weight tiles in tensor memory, 32 columns each behind two accumulators of `tileRows` columns.
+__host__ __device__ constexpr uint32_t weight_stages(uint32_t tileRows) { return tileRows <= kRowTileSmall ? 8u : 4u; }
+// A CTA's half of a step's token tile (a multiple of the 1024-byte swizzle atom).
+__host__ __device__ constexpr uint32_t tok_tile_bytes(uint32_t tileRows) { return tileRows / 2u * kTileK * 2u; }
+static_assert(2 * kRowTile + weight_stages(kRowTile) * 32 <= kTmemCols && 2 * kRowTileSmall + weight_stages(kRowTileSmall) * 32 <= kTmemCols, "tensor memory layout");
+static_assert(kRowTile % 32 == 0 && (int)kRowTile <= kEpilogueThreads && kRowTileSmall % 32 == 0, "row tile");
+static_assert((int)weight_stages(kRowTileSmall) <= 2 * kTokStages && 2 * kTokStages % weight_stages(kRowTile) == 0, "rings");
+static_assert(kTokStages == kGroups && kQuad == 4, "a group owns a slot; two pairs a quad");
 
 enum GemmMode : int { kModeGateUp = 0, kModeDown = 1 };
 
 struct GemmArgs {
     const uint32_t *scaleWords;  // scale | bias words of expert 0 (see pack_scales), of its down rows for the down GEMM
     uint64_t scaleStride;        // words between experts
+    uint32_t tileRows, packStages;
     uint32_t scaleBuffers;       // units whose scale words are held in shared memory: 2, 1 or 0 (read per step)
     uint32_t K;                // contraction length (multiple of 64)
     uint32_t N;                // outputs per row: F (gate/up) or D (down)
@@ -637,7 +646,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ CUtensorMap mapTokSmall, const __grid_constant__ CUtensorMap mapW0,
                     const __grid_constant__ CUtensorMap mapW1, const GemmArgs args) {
     extern __shared__ uint8_t gemmSmemRaw[];
-    __shared__ uint64_t barriers[2 * kTokStages + 2 * kPackStages + 4 + 2 * kEpilogueSets + 1];
+    __shared__ __align__(64) uint64_t barriers[2 * kTokStages + 2 * kMaxPackStages + 4 + 2 * kEpilogueSets + 1];
     __shared__ uint32_t tmemBaseSlot;
     __shared__ volatile uint32_t abortFlag;
 
@@ -649,10 +658,10 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
     // carve-up: token stages (1024-aligned), packed stages, the epilogue's buffers, scale words
     // (stage addresses are computed, not tabulated: an array indexed by the running stage would
     // live in local memory)
-    const uint32_t tokBase = base, packBase = tokBase + kTokStages * kTokTileBytes;
-    auto tokAddrOf = [&](uint32_t s) { return tokBase + s * kTokTileBytes; };
+    const uint32_t tokBytes = tok_tile_bytes(args.tileRows), packBase = base + kTokStages * 2u * tokBytes;
+    auto tokAddrOf = [&](uint32_t s) { return base + s * 2u * tokBytes; };
     auto packAddrOf = [&](uint32_t s) { return packBase + s * kPackTileBytes; };
-    const uint32_t epilogueOffset = packBase + kPackStages * kPackTileBytes - rawBase;
+    const uint32_t epilogueOffset = packBase + args.packStages * kPackTileBytes - rawBase;
     uint8_t *epilogueSmem = gemmSmemRaw + epilogueOffset;
     const uint32_t scaleBase = rawBase + epilogueOffset + (MODE == kModeGateUp ? kEpilogueBytesGateUp : kEpilogueBytesDown);
 
@@ -661,8 +670,8 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
     auto barStep = [&](int s) { return barAt(s); };
     auto barTokEmpty = [&](int s) { return barAt(kTokStages + s); };
     auto barPackFull = [&](int s) { return barAt(2 * kTokStages + s); };
-    auto barPackEmpty = [&](int s) { return barAt(2 * kTokStages + kPackStages + s); };
-    constexpr int kBarAcc = 2 * kTokStages + 2 * kPackStages;
+    auto barPackEmpty = [&](int s) { return barAt(2 * kTokStages + kMaxPackStages + s); };
+    constexpr int kBarAcc = 2 * kTokStages + 2 * kMaxPackStages;
     auto barAccFull = [&](int s) { return barAt(kBarAcc + s); };
     auto barAccEmpty = [&](int s) { return barAt(kBarAcc + 2 + s); };
     auto barStage = [&](int set, int buffer) { return barAt(kBarAcc + 4 + 2 * set + buffer); };
@@ -680,9 +689,9 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
             mbar_init(barStep(s), 9);      // (leader's is used) a group's four warps in either CTA, the expected bytes
             mbar_init(barTokEmpty(s), 1);  // one tcgen05.commit
         }
-        for (int s = 0; s < kPackStages; ++s) {
+        for (int s = 0; s < kMaxPackStages; ++s) {
             mbar_init(barPackFull(s), 1);
-            mbar_init(barPackEmpty(s), kDequantWarps);  // every dequantizing warp
+            mbar_init(barPackEmpty(s), kDequantWarps / 2);  // the warps of two groups
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(barAccFull(s), 1);                     // one tcgen05.commit
@@ -722,6 +731,8 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
     auto ntOf = [&](uint32_t u) { return 2u * (u % nPairs) + ctaRank; };
     // accumulator columns of a tile: its rows to the next multiple of 32, half of them in either CTA
     auto columnsOf = [&](const RowTile &tile) { return max(32u, (tile.rows + 31u) & ~31u); };
+    // Tensor memory behind the two accumulators: a step's weight stage is its token stage, modulo the stages there are.
+    const uint32_t wCol0 = 2u * args.tileRows, wStages = weight_stages(args.tileRows), wMask = wStages - 1u;
     // weight rows of a unit: gate rows [64 nt, +64) | up rows [64 nt, +64) for the gate/up
     // GEMM, matrix rows [128 nt, +128) for the down GEMM; loaded as two boxes of 64 rows.  In tensor
     // memory gate and up stand in turn, eight lanes each, so that the epilogue's threads find both
@@ -744,15 +755,17 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
                 const uint32_t half = columnsOf(tile) >> 1;  // this CTA's half of the tile's rows
                 const int row0 = (int)(tile.rowStart + ctaRank * half);
                 const CUtensorMap *map = half <= kTokSmallRows ? &mapTokSmall : &mapTok;
-                const uint32_t bytes = (half <= kTokSmallRows ? kTokSmallRows : kTokHalfRows) * kTileK * 2;
-                for (uint32_t g = 0; g < groupsK; ++g) {
+                const uint32_t bytes = half <= kTokSmallRows ? tok_tile_bytes(2u * kTokSmallRows) : tokBytes;
+                for (uint32_t g = 0; g < kQuad * quadsK; g += 2) {
                     if (!mbar_wait_warp<true, Order::kPair>(barTokEmpty(ts), phase ^ 1u, &abortFlag)) {
                         ok = false;
                         break;
                     }
                     if (elect_one()) {
-                        if (leader) mbar_expect_tx(barStep(ts), 2u * bytes);
-                        tma_load_2d_pair(tokAddrOf(ts), map, (int)(g * kTileK), row0, leaderStep + 8u * ts);
+                        const uint32_t steps = g + 1u < groupsK ? 2u : g < groupsK ? 1u : 0u;  // fewer at a row's end
+                        if (leader) mbar_expect_tx(barStep(ts), 2u * steps * bytes);
+                        if (steps > 0u) tma_load_2d_pair(tokAddrOf(ts), map, (int)(g * kTileK), row0, leaderStep + 8u * ts);
+                        if (steps > 1u) tma_load_2d_pair(tokAddrOf(ts) + tokBytes, map, (int)((g + 1u) * kTileK), row0, leaderStep + 8u * ts);
                     }
                     ts = (ts + 1u) % kTokStages;
                     if (ts == 0) phase ^= 1u;
@@ -782,7 +795,7 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
                         tma_load_3d(packAddrOf(ps) + (uint32_t)h * (kPackTileBytes / 2), map,
                                     (int)(q * (kQuad * kTileK / 2)), wRow, (int)tile.expert, barPackFull(ps));
                     }
-                    if (++ps == kPackStages) {
+                    if (++ps == args.packStages) {
                         ps = 0;
                         phase ^= 1u;
                     }
@@ -796,7 +809,7 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
         // cost this thread 820 cycles for 384 of the tensor core.
         if (leader && firstUnit < units) {
             uint32_t ts = 0, phase = 0, acc = 0, accPhase = 0;
-            bool ok = true, ready = false;  // ready: seen that the next step's weights and tokens are there
+            bool ok = true, ready = false;  // ready: seen that the next pair's weights and tokens are there
             RowTile next = tileOf(firstUnit);
             for (uint32_t u = firstUnit; u < units && ok; u += unitStride) {
                 const RowTile tile = next;
@@ -804,41 +817,41 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
                 const uint32_t idesc = umma_idesc_bf16_m256(columnsOf(tile));
                 if (!mbar_wait_warp<true, Order::kPair>(barAccEmpty(acc), accPhase ^ 1u, &abortFlag)) break;
                 tc_fence_after();
-                const uint32_t tmemD = tmemBase + acc * kAccCols;
-                for (uint32_t g0 = 0; g0 < groupsK && ok; g0 += kWStages) {
-#pragma unroll
-                    for (uint32_t ws = 0; ws < kWStages; ++ws) {
-                        const uint32_t g = g0 + ws;
-                        if (g >= groupsK) break;
-                        if (!__all_sync(0xFFFFFFFFu, ready) &&
-                            !mbar_wait_warp<false, Order::kPair>(barStep(ts), phase, &abortFlag)) {
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after();
-                        // the next step's barrier is looked at now and the answer used after this step's MMAs
-                        const uint32_t tn = (ts + 1u) % kTokStages;
-                        if (tn == 0u) phase ^= 1u;
-                        ready = mbar_test_wait<Order::kPair>(barStep(tn), phase);
-                        const uint64_t descTok = umma_desc_sw128(tokAddrOf(ts));
-                        const uint32_t tmemW = tmemBase + kWCol0 + ws * 32u;
-                        if (elect_one()) {
-                            // (the wait was for both CTAs' operands; this look acquires the token halves, whose copies
-                            // complete on this CTA's barrier)
-                            (void)mbar_test_wait(barStep(ts), tn == 0u ? phase ^ 1u : phase);
-#pragma unroll
-                            for (uint32_t kk = 0; kk < kTileK / 16; ++kk) {
-                                // per 16-element slice: eight columns further in TMEM, 32 bytes (>> 4 = 2)
-                                // further in the token tile
-                                tc_mma_bf16_a_tmem(tmemD, tmemW + 8u * kk, descTok + 2u * kk, idesc,
-                                                   (g | kk) != 0u ? 1u : 0u);
-                            }
-                            // one signal per step: the token stage is free, and so is the weight stage that
-                            // the same step used (the dequantizers wait on the token ring's barrier, too)
-                            tc_commit_pair(barTokEmpty(ts));
-                        }
-                        ts = tn;
+                const uint32_t tmemD = tmemBase + acc * args.tileRows;
+                for (uint32_t g = 0; g < kQuad * quadsK; g += 2) {
+                    if (!__all_sync(0xFFFFFFFFu, ready) &&
+                        !mbar_wait_warp<false, Order::kPair>(barStep(ts), phase, &abortFlag)) {
+                        ok = false;
+                        break;
                     }
+                    tc_fence_after();
+                    // the next pair's barrier is looked at now and the answer used after this pair's MMAs
+                    const uint32_t tn = (ts + 1u) % kTokStages;
+                    if (tn == 0u) phase ^= 1u;
+                    ready = mbar_test_wait<Order::kPair>(barStep(tn), phase);
+                    const uint64_t descTok = umma_desc_sw128(tokAddrOf(ts));
+                    const uint32_t tmemW = tmemBase + wCol0 + (2u * ts & wMask) * 32u;
+                    if (elect_one()) {
+                        // (the wait was for both CTAs' operands; this look acquires the token halves, whose copies
+                        // complete on this CTA's barrier)
+                        (void)mbar_test_wait(barStep(ts), tn == 0u ? phase ^ 1u : phase);
+                        // per 16-element slice: eight columns further in TMEM, 32 bytes (>> 4 = 2) further in
+                        // the token tile
+                        if (g < groupsK) {
+#pragma unroll
+                            for (uint32_t kk = 0; kk < kTileK / 16; ++kk)
+                                tc_mma_bf16_a_tmem(tmemD, tmemW + 8u * kk, descTok + 2u * kk, idesc, (g | kk) != 0u ? 1u : 0u);
+                        }
+                        if (g + 1u < groupsK) {
+#pragma unroll
+                            for (uint32_t kk = 0; kk < kTileK / 16; ++kk)
+                                tc_mma_bf16_a_tmem(tmemD, tmemW + 32u + 8u * kk, descTok + (tokBytes >> 4) + 2u * kk, idesc, 1u);
+                        }
+                        // one signal per pair of steps: the token stage is free, and so are the weight stages that
+                        // they used (the dequantizers wait on the token ring's barrier, too)
+                        tc_commit_pair(barTokEmpty(ts));
+                    }
+                    ts = tn;
                 }
                 if (!ok) break;
                 if (elect_one()) tc_commit_pair(barAccFull(acc));
@@ -848,110 +861,116 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
         }
     } else if (warp < kFirstEpilogueWarp) {
         // ---------------- dequantizers ----------------
-        // Group `grp` (four warps, one per TMEM lane quarter) takes step `grp` of every quad and owns
-        // weight stage `grp`; a thread turns one weight row's 64 codes of the step into 32 bf16 pairs
-        // and stores them to its TMEM lane.  Four steps are in work at once, which hides a step's
-        // latencies behind the other groups' arithmetic.
-        const uint32_t grp = (uint32_t)(warp - 2) >> 2;
+        // Group `grp` (four warps, one per TMEM lane quarter) takes every fourth pair of steps, counted over all of
+        // the CTA's units: pair `grp & 1` of every second quad, and slot `grp` of the step ring.  A thread turns one
+        // weight row's 64 codes of a step into 32 bf16 pairs and stores them to its TMEM lane.  Four pairs are in work
+        // at once, which hides a pair's latencies behind the other groups' arithmetic.
+        const uint32_t grp = (uint32_t)(warp - 2) >> 2, half = grp & 1u, quadParity = grp >> 1;
         const uint32_t m = (uint32_t)(warp & 3) * 32u + (uint32_t)lane;  // TMEM lane
         // its feature within the unit (gate/up), its row in the loaded boxes
         const uint32_t feature = (m >> 4) * 8u + interleaved_element(m & 7u);
         const uint32_t boxRow = MODE == kModeGateUp ? ((m >> 3) & 1u) * 64u + feature : m;
-        const uint32_t tmemW = tmemBase + kWCol0 + grp * 32u + (((uint32_t)(warp & 3) * 32u) << 16);
         const uint32_t paddedK = (groupsK + 3u) & ~3u;
 
-        // The thread's scale words of a unit (one per quad) come as asynchronous copies into a private
-        // column of shared memory, one unit ahead: no global load is in flight in the steady loop (one
-        // in flight would hold up the releasing arrive below for its whole latency), and none is
-        // waited for at a unit's start.
-        const uint32_t myScales = scaleBase + 4u * (uint32_t)(threadIdx.x - 64);  // [buffer][quad][512 threads]
+        // The thread's scale words of a unit (two per pair) come as asynchronous copies into a private column of
+        // shared memory, one unit ahead: no global load is in flight in the steady loop (one in flight would hold up
+        // the releasing arrive below for its whole latency), and none is waited for at a unit's start.
+        const uint32_t myScales = scaleBase + 8u * (uint32_t)(threadIdx.x - 64);  // [buffer][every second quad][512 threads]
         auto scale_row = [&](uint32_t u, const RowTile &tile, bool &live) {
             const uint32_t nt = ntOf(u);
             const uint32_t wRow = MODE == kModeGateUp ? nt * 64u + feature : nt * 128u + m;
             live = wRow < args.N;
             const uint32_t row = MODE == kModeGateUp ? (wRow >> 3) * 16u + (wRow & 7u) + (m & 8u) : wRow;
-            return args.scaleWords + (size_t)tile.expert * args.scaleStride + (size_t)(live ? row : 0u) * paddedK + grp;
+            return args.scaleWords + (size_t)tile.expert * args.scaleStride + (size_t)(live ? row : 0u) * paddedK + 2u * half;
         };
-        auto fetch_scales = [&](uint32_t u, const RowTile &tile, uint32_t buffer) {
+        // quads first, first + 2, ...
+        auto fetch_scales = [&](uint32_t u, const RowTile &tile, uint32_t first, uint32_t buffer) {
             bool live;
-            const uint32_t *src = scale_row(u, tile, live);
-            uint32_t dst = myScales + buffer * quadsK * kScaleSlotBytes;
-            for (uint32_t q = 0; q < quadsK; ++q, dst += kScaleSlotBytes, src += kQuad)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(live ? 4u : 0u) : "memory");
+            const uint32_t *src = scale_row(u, tile, live) + first * kQuad;
+            uint32_t dst = myScales + buffer * scale_buffer_bytes(quadsK);
+            for (uint32_t q = first; q < quadsK; q += 2, dst += kScaleSlotBytes, src += 2 * kQuad)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(live ? 8u : 0u) : "memory");
         };
         auto scales_arrived = [] { asm volatile("cp.async.wait_all;" ::: "memory"); };
-        const uint32_t leaderStep = map_to_cta(barStep(0), 0u);
-        uint32_t ps = 0, pPhase = 0;
-        uint32_t step0 = 0;                 // steps of the CTA's earlier units
-        uint32_t lastStep = 0xFFFFFFFFu;    // this group's previous step
+        // What the loop needs stands in registers; the slots of the group are always the same.
+        const uint32_t rowOffset = boxRow * 128u, flip = boxRow & 7u;
+        uint32_t codes[4];  // its 64 bytes of a quad's row: 16-byte chunks with the 128-byte swizzle
+#pragma unroll
+        for (uint32_t c = 0; c < 4; ++c) codes[c] = packBase + rowOffset + (((4u * half + c) ^ flip) << 4);
+        const uint32_t stepBar = map_to_cta(barStep((int)grp), 0u);
+        const uint32_t tmemW = tmemBase + wCol0 + (2u * grp & wMask) * 32u + (((uint32_t)(warp & 3) * 32u) << 16);
+        // The weight stages were last read by the MMAs `wStages` steps back: their completion is that pair's signal
+        // on the token ring.  (A first pair waits for the parity of a phase before the barrier's first: not at all.)
+        const uint32_t freeBar = barTokEmpty((int)(wStages == 8u ? grp : grp ^ 2u));
+        uint32_t freePhase = wStages == 8u || grp < 2u ? 1u : 0u;
+        uint32_t ps = quadParity, pPhase = 0;
+        uint32_t quad0 = 0;  // quads of the CTA's earlier units
         bool ok = firstUnit < units;
         RowTile tile{}, next{};
         if (ok) {
             next = tileOf(firstUnit);
-            if (args.scaleBuffers) fetch_scales(firstUnit, next, 0);
+            if (args.scaleBuffers) fetch_scales(firstUnit, next, quadParity, 0);
         }
         uint32_t unitNo = 0;
-        for (uint32_t u = firstUnit; u < units && ok; u += unitStride, ++unitNo, step0 += groupsK) {
+        for (uint32_t u = firstUnit; u < units && ok; u += unitStride, ++unitNo, quad0 += quadsK) {
             tile = next;
             next = tileOf(u + unitStride);
+            const uint32_t first = (quad0 ^ quadParity) & 1u;
             const uint32_t buffer = args.scaleBuffers == 2 ? unitNo & 1u : 0u;
             if (args.scaleBuffers == 2) {
                 scales_arrived();
-                if (u + unitStride < units) fetch_scales(u + unitStride, next, buffer ^ 1u);
+                if (u + unitStride < units) fetch_scales(u + unitStride, next, (quad0 + quadsK ^ quadParity) & 1u, buffer ^ 1u);
             } else if (args.scaleBuffers == 1) {
-                if (unitNo) fetch_scales(u, tile, 0);
+                if (unitNo) fetch_scales(u, tile, first, 0);
                 scales_arrived();
             }
-            for (uint32_t q = 0; q < quadsK; ++q) {
-                if (!mbar_wait(barPackFull(ps), pPhase, &abortFlag)) {
+            uint32_t scaleAddr = myScales + buffer * scale_buffer_bytes(quadsK);
+            // (A row's last quad may have fewer than four steps: the rest is converted like any other, from codes
+            // that read as zero, and no MMA uses it.)
+            for (uint32_t q = first; q < quadsK; q += 2, scaleAddr += kScaleSlotBytes) {
+                if (!mbar_wait_warp<false, Order::kLocal>(barPackFull((int)ps), pPhase, &abortFlag)) {
                     ok = false;
                     break;
                 }
-                const uint32_t g = q * kQuad + grp;
-                uint32_t o[32];
-                if (g < groupsK) {
-                    uint32_t sb;
-                    if (args.scaleBuffers) {
-                        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sb) : "r"(myScales + (buffer * quadsK + q) * kScaleSlotBytes));
-                    } else {
-                        bool live;
-                        const uint32_t *src = scale_row(u, tile, live);
-                        sb = live ? __ldg(src + q * kQuad) : 0u;
-                    }
-                    // the row's 128 bytes lie as eight 16-byte chunks with the 128-byte swizzle
-                    const uint32_t src = packAddrOf(ps) + boxRow * 128u, flip = boxRow & 7u;
-                    uint32_t w[8];
-#pragma unroll
-                    for (uint32_t c = 0; c < 2; ++c)
-                        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                                     : "=r"(w[4 * c]), "=r"(w[4 * c + 1]), "=r"(w[4 * c + 2]), "=r"(w[4 * c + 3])
-                                     : "r"(src + (((2u * grp + c) ^ flip) << 4)));
-                    dequantize_words(w, sb, o);
+                uint32_t sb[2];
+                if (args.scaleBuffers) {
+                    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(sb[0]), "=r"(sb[1]) : "r"(scaleAddr));
+                } else {
+                    bool live;
+                    const uint32_t *src = scale_row(u, tile, live) + q * kQuad;
+                    sb[0] = live ? __ldg(src) : 0u;
+                    sb[1] = live ? __ldg(src + 1) : 0u;
                 }
+                uint32_t w[2][8], o[32];
+#pragma unroll
+                for (uint32_t c = 0; c < 4; ++c)
+                    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(w[c >> 1][4 * (c & 1)]), "=r"(w[c >> 1][4 * (c & 1) + 1]), "=r"(w[c >> 1][4 * (c & 1) + 2]),
+                                   "=r"(w[c >> 1][4 * (c & 1) + 3])
+                                 : "r"(codes[c] + ps * kPackTileBytes));
+                dequantize_words(w[0], sb[0], o);
                 // the codes are in registers: their tile may be copied over
                 __syncwarp();
-                if (lane == 0) mbar_arrive(barPackEmpty(ps));
-                if (++ps == kPackStages) {
-                    ps = 0;
+                if (lane == 0) mbar_arrive(barPackEmpty((int)ps));
+                ps += 2u;
+                if (ps >= args.packStages) {
+                    ps -= args.packStages;
                     pPhase ^= 1u;
                 }
-                if (g >= groupsK) continue;
-                // The weight stage was last read by the MMAs of this group's previous step: their completion
-                // is that step's signal on the token ring.  Waited for only here: the conversion above runs
-                // under those MMAs.
-                const uint32_t step = step0 + g;
-                if (lastStep != 0xFFFFFFFFu &&
-                    !mbar_wait<Order::kPair>(barTokEmpty(lastStep % kTokStages), (lastStep / kTokStages) & 1u, &abortFlag)) {
+                // (waited for only here: the conversion above runs under the MMAs that read the stages before)
+                if (!mbar_wait_warp<false, Order::kPair>(freeBar, freePhase, &abortFlag)) {
                     ok = false;
                     break;
                 }
-                lastStep = step;
+                freePhase ^= 1u;
                 tc_fence_after();
                 tc_store_32cols(tmemW, o);
+                dequantize_words(w[1], sb[1], o);
+                tc_store_32cols(tmemW + 32u, o);
                 tc_wait_st();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_pair(leaderStep + 8u * (step % kTokStages));
+                if (lane == 0) mbar_arrive_pair(stepBar);
             }
         }
         scales_arrived();  // nothing of this thread's is in flight when shared memory is released
@@ -1001,7 +1020,7 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
             if (!mbar_wait_idle<Order::kPair>(barAccFull(acc), accPhase, &abortFlag)) break;
             if (MODE == kModeDown && !mbar_wait(barRows, unitNo & 1u, &abortFlag)) break;
             tc_fence_after();
-            const uint32_t taddr = tmemBase + acc * kAccCols + ((quarter * 32u) << 16);
+            const uint32_t taddr = tmemBase + acc * args.tileRows + ((quarter * 32u) << 16);
 #pragma unroll 1
             for (uint32_t c0 = 32u * set; c0 < tile.rows; c0 += 32u * kEpilogueSets, ++chunk) {
                 const uint32_t buffer = chunk & 1u;
@@ -1090,8 +1109,8 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
 
 // ---- host side -----------------------------------------------------------------------------
 
-// bf16 activations [rows][k] (row pitch `strideElems`), box 64 x kTokHalfRows (the half of a row
-// tile that one CTA of a pair holds), 128-byte swizzle.
+// bf16 activations [rows][k] (row pitch `strideElems`), box 64 x `boxRows` (the half of a row tile that
+// one CTA of a pair holds), 128-byte swizzle.
 static bool make_activation_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t k,
                                 uint64_t strideElems, uint32_t boxRows, const char **error) {
     cuuint64_t dims[2] = {k, rows};
@@ -1162,10 +1181,30 @@ bool prefill_prepare_layer(FFContext *ctx, LayerStore &L, const char **error) {
 }
 
 // Shared memory of a GEMM over K with `buffers` units' scale words.
-static size_t gemm_smem_bytes(int mode, uint32_t K, uint32_t buffers) {
+static size_t gemm_smem_bytes(int mode, uint32_t K, uint32_t tileRows, uint32_t packStages, uint32_t buffers) {
     const size_t quads = (K / kTileK + kQuad - 1) / kQuad;
-    return 1024 + (size_t)kTokStages * kTokTileBytes + (size_t)kPackStages * kPackTileBytes +
-           (mode == kModeGateUp ? kEpilogueBytesGateUp : kEpilogueBytesDown) + buffers * quads * kScaleSlotBytes;
+    return 1024 + (size_t)kTokStages * 2 * tok_tile_bytes(tileRows) + (size_t)packStages * kPackTileBytes +
+           (mode == kModeGateUp ? kEpilogueBytesGateUp : kEpilogueBytesDown) + buffers * scale_buffer_bytes((uint32_t)quads);
+}
+
+// Rows of a routed GEMM's tiles.  Tiles of 128 rows leave tensor memory for eight weight stages instead of four, and a
+// step of few columns then costs what its conversion does; tiles of 192 convert an expert's weights fewer times.
+// Whole layer of d 2816, f 704, shared 2112, us with 128 / 192: 77 rows (5 an expert) 146 / 155, 613 (38) 203 / 209,
+// 1400 (87) 291 / 298, 1500 (94) 313 / 313, 2000 (125) 373 / 357, 4096 648 / 634.
+static uint32_t routed_tile_rows(uint32_t pairs, uint32_t experts) { return pairs <= 96u * experts ? kRowTileSmall : kRowTile; }
+
+// Of the shared FFN's two GEMMs: where whole waves of a step take less time (by their columns, 3 : 4).  us with 128 /
+// 192: 77 rows 23.7 / 25.8, 300 26.9 / 32.7, 613 35.2 / 39.3, 1000 42.8 / 46.3, 1500 50.6 / 55.3, 3000 97.9 / 89.9, 4096
+// 124.5 / 130.2.  (Up to 1000 rows, one or two waves, the smaller tile won whatever their number.)
+static uint32_t dense_tile_rows(const FFContext *ctx, uint32_t tokens) {
+    if (tokens <= 1024u) return kRowTileSmall;
+    const uint32_t d = ctx->cfg.d, f = ctx->cfg.sharedF, clusters = std::max(1u, (uint32_t)ctx->smCount / 2u);
+    const auto cost = [&](uint32_t rows) {
+        const uint64_t tiles = (tokens + rows - 1u) / rows;
+        const auto waves = [&](uint32_t nTiles) { return (tiles * ((nTiles + 1u) / 2u) + clusters - 1u) / clusters; };
+        return (waves((f + 63u) / 64u) * d + waves((d + 127u) / 128u) * f) * rows;
+    };
+    return cost(kRowTileSmall) * 9u <= cost(kRowTile) * 8u ? kRowTileSmall : kRowTile;
 }
 
 // `rows` activation rows of args.K elements at `x`
@@ -1174,14 +1213,17 @@ static bool launch_gemm(FFContext *ctx, const uint16_t *x, uint64_t rows, const 
                         const CUtensorMap &mapW1, GemmArgs args, uint32_t maxUnits,
                         cudaStream_t stream, const char **error) {
     CUtensorMap mapA, mapASmall;
-    if (!make_activation_map(&mapA, x, rows, args.K, args.K, kTokHalfRows, error) ||
+    if (!make_activation_map(&mapA, x, rows, args.K, args.K, args.tileRows / 2, error) ||
         !make_activation_map(&mapASmall, x, rows, args.K, args.K, kTokSmallRows, error))
         return false;
     auto kernel = k_grouped_int4_gemm<MODE>;
     // scale words one unit ahead where they fit, else the unit's own, else none (read step by step)
+    const auto smemOf = [&] { return gemm_smem_bytes(MODE, args.K, args.tileRows, args.packStages, args.scaleBuffers); };
     args.scaleBuffers = 2;
-    while (args.scaleBuffers && gemm_smem_bytes(MODE, args.K, args.scaleBuffers) > 226 * 1024) --args.scaleBuffers;
-    const size_t smem = gemm_smem_bytes(MODE, args.K, args.scaleBuffers);
+    args.packStages = 3;
+    while (args.scaleBuffers && smemOf() > 226 * 1024) --args.scaleBuffers;
+    while (args.packStages < (uint32_t)kMaxPackStages && smemOf() + kPackTileBytes <= 226 * 1024) ++args.packStages;
+    const size_t smem = smemOf();
     static KernelSmemMemo memo;
     if (!memo.prepare(kernel, ctx->device, smem, kGemmThreads, nullptr, error)) return false;
     // clusters of two CTAs; a cluster takes (row tile, pair of weight-row tiles) units
@@ -1202,7 +1244,7 @@ static bool check_gemm_shapes(const FFConfig &c, uint32_t f, const char **error)
 }
 
 // Sorts the routes (stable, by expert) and plans the row tiles.
-static bool sort_routes(FFContext *ctx, const uint32_t *ids, uint32_t tokens, int E, uint32_t *offsets, RowTile *tiles,
+static bool sort_routes(FFContext *ctx, const uint32_t *ids, uint32_t tokens, int E, uint32_t tileRows, uint32_t *offsets, RowTile *tiles,
                               FFTokenExpertPair *sorted, uint32_t *rowOfRoute, cudaStream_t stream, const char **error) {
     const int T = (int)tokens, K = (int)ctx->cfg.topK;
     const uint32_t blocks = (tokens + kSortTokens - 1) / kSortTokens;
@@ -1210,7 +1252,7 @@ static bool sort_routes(FFContext *ctx, const uint32_t *ids, uint32_t tokens, in
     const uint32_t maxTiles = ctx->maxUnits / 2;  // first half of the tile buffer
     if (blocks == 1) {
         LaunchScope scope(ctx, stream, "route_sort");
-        FF_CUDA_OK(launch_pdl(k_route_sort, 1, 256, sortSmem, stream, ids, T, K, E, offsets, tiles, maxTiles, ctx->unitCount, sorted,
+        FF_CUDA_OK(launch_pdl(k_route_sort, 1, 256, sortSmem, stream, ids, T, K, E, tileRows, offsets, tiles, maxTiles, ctx->unitCount, sorted,
                               rowOfRoute),
                    error);
         return true;
@@ -1221,7 +1263,7 @@ static bool sort_routes(FFContext *ctx, const uint32_t *ids, uint32_t tokens, in
     }
     {
         LaunchScope scope(ctx, stream, "route_scan");
-        FF_CUDA_OK(launch_pdl(k_route_scan, 1, 256, 0, stream, ctx->blockCounts, (int)blocks, E, offsets, tiles, maxTiles, ctx->unitCount),
+        FF_CUDA_OK(launch_pdl(k_route_scan, 1, 256, 0, stream, ctx->blockCounts, (int)blocks, E, tileRows, offsets, tiles, maxTiles, ctx->unitCount),
                    error);
     }
     LaunchScope scope(ctx, stream, "route_scatter");
@@ -1241,7 +1283,8 @@ bool launch_prefill_routed(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     if (!check_gemm_shapes(c, c.f, error) || !prefill_prepare_layer(ctx, L, error)) return false;
     const int K = (int)c.topK, E = (int)L.expertCount;
     RowTile *tiles = reinterpret_cast<RowTile *>(ctx->units);
-    if (!sort_routes(ctx, ids, tokens, E, ctx->expertOffsets, tiles, ctx->sortedPairs, ctx->rowOfRoute, stream, error)) return false;
+    const uint32_t tileRows = routed_tile_rows(tokens * c.topK, (uint32_t)E);
+    if (!sort_routes(ctx, ids, tokens, E, tileRows, ctx->expertOffsets, tiles, ctx->sortedPairs, ctx->rowOfRoute, stream, error)) return false;
     const uint32_t pairs = tokens * c.topK;
     {
         LaunchScope scope(ctx, stream, "gather_rows");
@@ -1250,9 +1293,10 @@ bool launch_prefill_routed(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
                    error);
     }
 
-    const uint32_t tileBound = pairs / kRowTile + (uint32_t)E;
+    const uint32_t tileBound = pairs / tileRows + (uint32_t)E;
     const uint64_t rows = (uint64_t)pairs + 256;
     GemmArgs a{};
+    a.tileRows = tileRows;
     a.scaleWords = L.routedScales;
     a.scaleStride = scale_words(c.d, c.f);
     a.K = c.d;
@@ -1291,7 +1335,7 @@ bool launch_route_sort(FFContext *ctx, const uint32_t *groupIds, uint32_t tokens
     if (!ctx->xSorted) return fail(error, "context was created with maxTokens <= 16: no prefill scratch");
     if (groups == 0 || groups > c.experts) return fail(error, "group count must be 1..experts of the context");
     if (tokens > c.maxTokens) return fail(error, "rows exceed the context's maxTokens");
-    return sort_routes(ctx, groupIds, tokens, (int)groups, offsets, reinterpret_cast<RowTile *>(ctx->units), sortedPairs, nullptr, stream,
+    return sort_routes(ctx, groupIds, tokens, (int)groups, kRowTile, offsets, reinterpret_cast<RowTile *>(ctx->units), sortedPairs, nullptr, stream,
                        error);
 }
 
@@ -1305,10 +1349,11 @@ bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     // dense problem: its row tiles live behind the routed ones in the units buffer
     RowTile *tiles = reinterpret_cast<RowTile *>(ctx->units) + ctx->maxUnits / 2;
     uint32_t *counts = ctx->unitCount + 4;
+    const uint32_t tileRows = dense_tile_rows(ctx, tokens);
     {
         LaunchScope scope(ctx, stream, "dense_tiles");
         FF_CUDA_OK(launch_pdl(k_dense_tiles, 1, 256, 0, stream,
-                              (int)tokens, tiles, counts),
+                              (int)tokens, (int)tileRows, tiles, counts),
                    error);
     }
     {
@@ -1317,9 +1362,10 @@ bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
                               x, xStride, tokens, nullptr, 0, (int)c.d, ctx->xShared),
                    error);
     }
-    const uint32_t rowTiles = (tokens + kRowTile - 1) / kRowTile;
+    const uint32_t rowTiles = (tokens + tileRows - 1) / tileRows;
     const uint64_t rows = (uint64_t)tokens + 256;
     GemmArgs a{};
+    a.tileRows = tileRows;
     a.scaleWords = L.sharedScales;
     a.K = c.d;
     a.N = c.sharedF;

@@ -138,3 +138,26 @@ def test_gemms_repeat_bit_for_bit(rows):
     finally:
         int8.close()
         ctx.close()
+
+
+@pytest.mark.parametrize("d,f,fs,rows", [(192, 320, 64, 384), (192, 320, 64, 385), (448, 128, 0, 769), (128, 64, 320, 8000),
+                                         (320, 64, 192, 8193)])
+def test_int4_gemm_tile_rows(oracle, d, f, fs, rows):
+    """Rows on either side of where the routed GEMMs (96 an expert) and the shared FFN's (whole waves) go over from tiles of
+    128 rows to 192, with contractions that end inside a quad of steps, in its first pair or its second."""
+    L = workload.make_layer(0x77, 0, experts=8, d=d, f=f, sharedF=fs, topK=2)
+    hp, ctx = context(L, rows)
+    try:
+        ld = oracle_layer(oracle, L)
+        x = workload.make_tokens(0x78, f"tiles{rows}", rows, d)
+        ids = torch.zeros((rows, 2), dtype=torch.int32, device=ctx.device)
+        y = ctx.moeLayer(0, hp.bf16_tensor(x, ctx.device), ids=ids)
+        torch.cuda.synchronize()
+        assert ctx.info().deviceErrorFlag == 0
+        want, _, ref_ids, _ = oracle.moe_layer(ld, x, oracle.MODE_PARTIALS | oracle.MODE_BF16_WEIGHTS)
+        assert np.array_equal(ids.cpu().numpy().astype(np.uint32), ref_ids)
+        # the kernels and the oracle round the same sums to bf16: 2^-9 at most where they fall on other sides
+        rel_l2, _, _ = assert_layer_close(hp.bf16_numpy(y), want, oracle, f"tile rows {d}x{f}+{fs} rows={rows}")
+        assert rel_l2 < 2.0 ** -9
+    finally:
+        ctx.close()
