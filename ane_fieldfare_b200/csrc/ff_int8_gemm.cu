@@ -4,7 +4,7 @@
 // would lose most of q's bits, and a tensor-core sum over the whole contraction is less exact than the
 // fp32 sums the operator promises (its 376 truncated additions moved 12 % of the outputs to the
 // neighbouring bf16 value), so the contraction stays in groups: q is exact in bf16 and is multiplied
-// as it is, a step of 64 inputs is one accumulation of four MMAs in tensor memory, and eight warps
+// as it is, a step of 64 inputs is one accumulation of four MMAs in tensor memory, and sixteen warps
 // fetch every step's sums and add them up in registers as acc = fma(s, sum, acc), rounded to nearest.
 // The bias part, sum_g b_g X_g with X_g the sum of the token over group g, is a few more steps of the
 // same kind: A = the row's biases, B = X_g as three bf16 pieces (their sum is X_g to fp32's 24 bits),
@@ -13,14 +13,15 @@
 // Two CTAs of a cluster work as one tensor-core unit (cta_group::2, M = 256: either CTA 128 weight
 // rows, half of the token tile).  Per CTA: warp 0 TMA producer, warp 1 MMA issuer (leader only),
 // warps 2-9 turn codes into bf16 pairs in tensor memory (two groups of four warps, alternate steps),
-// warps 10-17 drain: a thread owns one weight row and 64 tokens.  Tensor memory: three accumulators of
+// warps 10-25 drain: a thread owns one weight row and 32 tokens.  Tensor memory: three accumulators of
 // 128 columns, four operand stages of 32.
 //
-// What bounds it: the latency of a step's chain (codes -> operand -> MMA -> drain), with three
-// accumulators in flight: a wave of units takes 30 us for 47 steps whatever the tile, the tensor pipe is
-// 21 to 24 % active.  2000 rows of 2816 x 2112: gate/up 129 us and down 67 us; with one warp per
-// output row and four tokens on the FMA pipe, which re-read the codes from L2 for every four tokens,
-// 9.35 ms and 2.77 ms.
+// What bounds it: the draining warps.  A step is 2700 warp instructions of a CTA (128 tokens; 512 of them the
+// multiply-adds), and each warp goes through a step's wait, loads and arrival one after another, 800 to 900 cycles
+// for the tensor core's 256.  2000 rows of 2816 x 2112: gate/up and down 159 us; with eight draining warps of 64
+// tokens, which did not fit their registers, 196 us.  Measured and not kept: loads of 32 columns (181 us: nothing
+// overlaps them), eight warps with 152 registers by setmaxnreg and a load always in flight (199 us), packed
+// multiply-adds (the compiler moves as many registers as they save), one dequantizing group (171 us).
 //
 // Error against 64 bits: the tensor core truncates where it aligns a group's products, so a token with one
 // value of 2^16 times the rest whose weight q s + b is zero comes out 3.4e-3 off (fp32 FMAs 2.1e-3, the
@@ -47,11 +48,13 @@ constexpr uint32_t kStepK = 64;
 constexpr uint32_t kTokBytes = kMaxRows / 2 * kStepK * 2;  // a CTA's half of a token tile
 constexpr uint32_t kCodeBytes = 128 * kStepK;
 constexpr uint32_t kOperandCol = kAccs * kMaxRows;
-constexpr int kDrainThreads = 256;
+constexpr int kDrainSets = 4;       // of four warps each: a set drains kSetTokens of the tile's tokens
+constexpr int kDrainThreads = 128 * kDrainSets;
+constexpr uint32_t kSetTokens = kMaxRows / kDrainSets;
 constexpr int kThreads = (2 + 4 * kDequantGroups) * 32 + kDrainThreads;
-constexpr int kBarriers = 4 * kStages + 2 * kAccs + 3;
-constexpr uint32_t kXchgPitch = 17;                       // floats per exchanged row (16 + 1)
-constexpr uint32_t kXchgBytes = 128u * kXchgPitch * 4u;   // one half of the tokens
+constexpr int kBarriers = 4 * kStages + 2 * kAccs + kDrainSets + 1;
+constexpr uint32_t kPassTokens = 16;             // tokens of a set that become outputs at a time
+constexpr uint32_t kXchgBytes = 128u * 8u * 4u;  // half of them, of every row, from gate to up or back
 constexpr uint32_t kTilePitchGateUp = 64 * 2 + 16, kTilePitchDown = 128 * 2 + 16;
 static_assert(kOperandCol + kOperandStages * 32 <= 512, "tensor memory layout");
 static_assert(kStages % kOperandStages == 0 && kOperandStages % kDequantGroups == 0, "rings");
@@ -136,8 +139,8 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
     auto barCodeEmpty = [&](uint32_t s) { return barAt(3 * kStages + s); };
     auto barAccFull = [&](uint32_t s) { return barAt(4 * kStages + s); };
     auto barAccEmpty = [&](uint32_t s) { return barAt(4 * kStages + kAccs + s); };
-    auto barHalf = [&](uint32_t h) { return barAt(4 * kStages + 2 * kAccs + h); };
-    const uint32_t barScales = barAt(4 * kStages + 2 * kAccs + 2);
+    auto barSet = [&](uint32_t h) { return barAt(4 * kStages + 2 * kAccs + h); };
+    const uint32_t barScales = barAt(4 * kStages + 2 * kAccs + kDrainSets);
 
     // What the MMA issuer waits for lives in the leader: a step's barrier counts the arrivals of both CTAs'
     // dequantizers and the bytes of both CTAs' token copies.  Barriers that the MMAs' completion frees exist
@@ -156,8 +159,7 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
             mbar_init(barAccFull(s), 1);
             mbar_init(barAccEmpty(s), 2 * kDrainThreads / 32);
         }
-        mbar_init(barHalf(0), kDrainThreads / 2);
-        mbar_init(barHalf(1), kDrainThreads / 2);
+        for (uint32_t s = 0; s < kDrainSets; ++s) mbar_init(barSet(s), 128);
         mbar_init(barScales, kDrainThreads);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -225,13 +227,14 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
         // (the whole warp runs the loop and one elected lane issues: inside a `lane == 0` branch every
         // operand would go to the uniform registers by a loop over the active lanes)
         if (leader) {
-            uint32_t st = 0, phase = 0, op = 0, acc = 0, accPhase = 0;
+            uint32_t st = 0, phase = 0, op = 0, accPhases = 0;  // a bit for each accumulator; a unit starts with the first
             bool ok = true;
             for (uint32_t u = firstUnit; u < units && ok; u += unitStride) {
+                uint32_t acc = 0;
                 const uint32_t idesc = umma_idesc_bf16_m256(columnsOf(u));
                 for (uint32_t g = 0; g < steps; ++g) {
                     if (!mbar_wait_warp<false, Order::kPair>(barStep(st), phase, &abortFlag) ||
-                        !mbar_wait_warp<false, Order::kPair>(barAccEmpty(acc), accPhase ^ 1u, &abortFlag)) {
+                        !mbar_wait_warp<false, Order::kPair>(barAccEmpty(acc), (accPhases >> acc & 1u) ^ 1u, &abortFlag)) {
                         ok = false;
                         break;
                     }
@@ -253,10 +256,8 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
                         phase ^= 1u;
                     }
                     op = (op + 1u) % kOperandStages;
-                    if (++acc == kAccs) {
-                        acc = 0;
-                        accPhase ^= 1u;
-                    }
+                    accPhases ^= 1u << acc;
+                    if (++acc == kAccs) acc = 0;
                 }
             }
         }
@@ -333,24 +334,26 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
         }
     } else {
         // ---------------- drain: scaled sums in registers, then the outputs ----------------
-        const uint32_t t = (uint32_t)threadIdx.x - (2u + 4u * kDequantGroups) * 32u;  // 0..255
-        const uint32_t half = t >> 7, th = t & 127u;                                  // tokens [64 half, +64) of the tile
+        const uint32_t t = (uint32_t)threadIdx.x - (2u + 4u * kDequantGroups) * 32u;  // 0..511
+        const uint32_t set = t >> 7, th = t & 127u;                                   // its tokens of the tile start at kSetTokens set
         const uint32_t quarter = (uint32_t)(warp & 3), m = quarter * 32u + (uint32_t)lane;
-        const uint32_t tmemLane = tmemBase + ((quarter * 32u) << 16) + half * 64u;
-        float *xchg = reinterpret_cast<float *>(epilogue + half * kXchgBytes);  // gate/up only
+        const uint32_t tmemLane = tmemBase + ((quarter * 32u) << 16) + set * kSetTokens;
+        float *xchg = reinterpret_cast<float *>(epilogue + set * kXchgBytes);  // gate/up only
         constexpr uint32_t kTilePitch = MODE == kGateUp ? kTilePitchGateUp : kTilePitchDown;
-        uint8_t *tileBuf = epilogue + (MODE == kGateUp ? 2u * kXchgBytes : 0u) + half * 32u * kTilePitch;
-        uint32_t accNo = 0, accPhase = 0, halfPhase = 0, unitNo = 0;
-        // every thread of this half of the tokens
+        uint8_t *tileBuf = epilogue + (MODE == kGateUp ? kDrainSets * kXchgBytes : 0u) + set * kPassTokens * kTilePitch;
+        const uint32_t leaderAccEmpty = map_to_cta(barAccEmpty(0), 0u);
+        uint32_t accPhases = 0, setPhase = 0, unitNo = 0;  // a bit for each accumulator
+        // every thread of this set
         auto meet = [&]() {
-            mbar_arrive(barHalf(half));
-            const bool ok = mbar_wait(barHalf(half), halfPhase, &abortFlag);
-            halfPhase ^= 1u;
+            mbar_arrive(barSet(set));
+            const bool ok = mbar_wait_warp<false, Order::kLocal>(barSet(set), setPhase, &abortFlag);
+            setPhase ^= 1u;
             return ok;
         };
         bool ok = true;
         for (uint32_t u = firstUnit; u < units && ok; u += unitStride, ++unitNo) {
-            const uint32_t nt = ntOf(u), token0 = tokenOf(u), rows = rowsOf(u), cols = columnsOf(u);
+            const uint32_t nt = ntOf(u), token0 = tokenOf(u), rows = rowsOf(u);
+            const uint32_t setRows = min(rows, (set + 1u) * kSetTokens) - min(rows, set * kSetTokens);
             // the unit's scales: 128 rows (gate/up: 64 of either matrix), contiguous in memory
             uint16_t *scales = scaleBuf + (unitNo & 1u) * 128u * groupsK;
             for (uint32_t i = t; i < 16u * groupsK; i += kDrainThreads) {  // 16-byte pieces, 8 groupsK per 64 rows
@@ -363,65 +366,74 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
                 *reinterpret_cast<uint4 *>(scales + (size_t)i * 8) = v;
             }
             mbar_arrive(barScales);
-            if (!mbar_wait(barScales, unitNo & 1u, &abortFlag)) break;
+            if (!mbar_wait_warp<false, Order::kLocal>(barScales, unitNo & 1u, &abortFlag)) break;
             const uint16_t *myScale = scales + m * groupsK;
+            const auto scale_of = [&](uint32_t g) { return g < groupsK ? 128.0f * bf2f(myScale[g]) : 1.0f; };  // (the codes come as q / 128)
 
-            float sum[64];
+            float sums[kSetTokens];
 #pragma unroll
-            for (int j = 0; j < 64; ++j) sum[j] = 0.0f;
-            for (uint32_t g = 0; g < steps; ++g) {
-                const float s = g < groupsK ? 128.0f * bf2f(myScale[g]) : 1.0f;  // (the codes come as q / 128)
-                if (!mbar_wait<Order::kPair>(barAccFull(accNo), accPhase, &abortFlag)) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
+            for (int j = 0; j < (int)kSetTokens; ++j) sums[j] = 0.0f;
+            float s = scale_of(0);
+            for (uint32_t g0 = 0; g0 < steps && ok; g0 += kAccs) {
 #pragma unroll
-                for (uint32_t c = 0; c < 2; ++c) {
-                    if (half * 64u + c * 32u < cols) {
-                        uint32_t v[32];
-                        tc_load_32cols(tmemLane + accNo * kMaxRows + c * 32u, v);
-                        tc_wait_ld();
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) sum[c * 32 + j] = fmaf(s, __uint_as_float(v[j]), sum[c * 32 + j]);
+                for (uint32_t a = 0; a < kAccs; ++a) {  // unrolled: the accumulators' addresses are constants
+                    const uint32_t g = g0 + a;
+                    if (g >= steps) break;
+                    if (!mbar_wait_warp<false, Order::kPair>(barAccFull(a), accPhases >> a & 1u, &abortFlag)) {
+                        ok = false;
+                        break;
                     }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_pair(map_to_cta(barAccEmpty(accNo), 0u));
-                if (++accNo == kAccs) {
-                    accNo = 0;
-                    accPhase ^= 1u;
+                    accPhases ^= 1u << a;
+                    tc_fence_after();
+                    if (setRows) {
+#pragma unroll
+                        for (uint32_t h = 0; h < kSetTokens / 16u; ++h) {
+                            uint32_t v[16];
+                            tc_load_16cols(tmemLane + a * kMaxRows + 16u * h, v);
+                            tc_wait_ld();
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) sums[16 * h + j] = fmaf(s, __uint_as_float(v[j]), sums[16 * h + j]);
+                        }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_pair(leaderAccEmpty + 8u * a);
+                    s = scale_of(g + 1u);
                 }
             }
             if (!ok) break;
 #pragma unroll
-            for (uint32_t c = 0; c < 2; ++c) {
-                const uint32_t c0 = half * 64u + c * 32u;
-                if (!ok || c0 >= rows) break;  // the same for every thread of the half (ok apart, which ends the launch)
-                if (MODE == kGateUp) {
-                    // lanes 0..63 hold gate, 64..127 up of features [64 nt, +64): either side takes 16 of
-                    // the 32 tokens from the other and finishes them
-                    const bool isUp = m >= 64u;
-                    float *mine = xchg + m * kXchgPitch;
+            for (uint32_t c = 0; c < kSetTokens / kPassTokens; ++c) {
+                const uint32_t c0 = set * kSetTokens + c * kPassTokens;
+                if (!ok || c0 >= rows) break;  // the same for every thread of the set (ok apart, which ends the launch)
+                float sum[kPassTokens];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) mine[j] = isUp ? sum[c * 32 + j] : sum[c * 32 + 16 + j];
+                for (int j = 0; j < (int)kPassTokens; ++j)
+                    sum[j] = sums[c * kPassTokens + j];
+                if (MODE == kGateUp) {
+                    // lanes 0..63 hold gate, 64..127 up of features [64 nt, +64): either side takes 8 of the 16
+                    // tokens from the other and finishes them (a row's eight floats are turned by m / 4: no bank twice)
+                    const bool isUp = m >= 64u;
+                    float *mine = xchg + m * 8u;
+                    const uint32_t turn = (m >> 2) & 7u;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) mine[(uint32_t)j ^ turn] = isUp ? sum[j] : sum[8 + j];
                     if (!meet()) {
                         ok = false;
                         break;
                     }
-                    const float *theirs = xchg + (m ^ 64u) * kXchgPitch;
-                    uint16_t *col = reinterpret_cast<uint16_t *>(tileBuf + (isUp ? 16u : 0u) * kTilePitch) + (m & 63u);
+                    const float *theirs = xchg + (m ^ 64u) * 8u;
+                    uint16_t *col = reinterpret_cast<uint16_t *>(tileBuf + (isUp ? 8u : 0u) * kTilePitch) + (m & 63u);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const float own = isUp ? sum[c * 32 + 16 + j] : sum[c * 32 + j], other = theirs[j];
+                    for (int j = 0; j < 8; ++j) {
+                        const float own = isUp ? sum[8 + j] : sum[j], other = theirs[(uint32_t)j ^ turn];
                         const float gate = bf16_round(isUp ? other : own), up = bf16_round(isUp ? own : other);
                         col[(uint32_t)j * (kTilePitch / 2)] = f2bf(gelu_tanh(gate) * up);
                     }
                 } else {
                     uint16_t *col = reinterpret_cast<uint16_t *>(tileBuf) + m;
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) col[(uint32_t)j * (kTilePitch / 2)] = f2bf(sum[c * 32 + j]);
+                    for (int j = 0; j < (int)kPassTokens; ++j) col[(uint32_t)j * (kTilePitch / 2)] = f2bf(sum[j]);
                 }
                 if (!meet()) {
                     ok = false;
@@ -432,19 +444,19 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
                 const uint32_t piece = th % kPieces;
                 const uint32_t col0 = nt * (kPieces * 8u) + piece * 8u;
 #pragma unroll
-                for (uint32_t pass = 0; pass < 32u / kPerPass; ++pass) {
+                for (uint32_t pass = 0; pass < kPassTokens / kPerPass; ++pass) {
                     const uint32_t tok = pass * kPerPass + th / kPieces;
-                    const bool live = c0 + tok < rows && col0 < args.N;
+                    const bool store = c0 + tok < rows && col0 < args.N;
                     const size_t row = token0 + c0 + tok;
                     const uint4 val = *reinterpret_cast<const uint4 *>(tileBuf + tok * kTilePitch + piece * 16u);
-                    if (live) *reinterpret_cast<uint4 *>(args.out + row * args.N + col0) = val;
+                    if (store) *reinterpret_cast<uint4 *>(args.out + row * args.N + col0) = val;
                     if (MODE == kGateUp) {
                         // the tile's 64 features are one group of the down projection
-                        float s = sum8(val);
-                        s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);
-                        s += __shfl_xor_sync(0xFFFFFFFFu, s, 2);
-                        s += __shfl_xor_sync(0xFFFFFFFFu, s, 4);
-                        if (live && piece == 0) store_group_sum(args.sums + row * sums_pitch(args.N), nt, s);
+                        float sg = sum8(val);
+                        sg += __shfl_xor_sync(0xFFFFFFFFu, sg, 1);
+                        sg += __shfl_xor_sync(0xFFFFFFFFu, sg, 2);
+                        sg += __shfl_xor_sync(0xFFFFFFFFu, sg, 4);
+                        if (store && piece == 0) store_group_sum(args.sums + row * sums_pitch(args.N), nt, sg);
                     }
                 }
                 if (MODE == kDown && !meet()) {  // the tile is rewritten next (gate/up: behind the next exchange)
@@ -486,9 +498,9 @@ bool make_code_map(CUtensorMap *map, const uint8_t *base, uint64_t rows, uint64_
 }
 
 // Tokens per tile: the size whose waves of units take the least time.  A wave of gate/up units over 2816 inputs (47
-// steps) takes 21.8, 28.5, 30.1 and 31.3 us with tiles of 32, 64, 96 and 128 tokens (the slopes of 256 to 4096 rows).
+// steps) takes 21.6, 23.2, 24.9 and 26.8 us with tiles of 32, 64, 96 and 128 tokens (4096 rows, each size forced).
 uint32_t pick_tile_rows(uint32_t tokens, uint32_t nPairs, uint32_t clusters) {
-    constexpr uint32_t kWave[kMaxRows / 32] = {218, 285, 301, 313};
+    constexpr uint32_t kWave[kMaxRows / 32] = {216, 232, 249, 268};
     uint32_t best = kMaxRows;
     uint64_t bestCost = ~0ull;
     for (uint32_t r = 32; r <= kMaxRows; r += 32) {
@@ -504,7 +516,7 @@ uint32_t pick_tile_rows(uint32_t tokens, uint32_t nPairs, uint32_t clusters) {
 
 size_t smem_bytes(int mode, uint32_t K) {
     return 1024 + (size_t)kStages * (kTokBytes + kCodeBytes) + 2 * 128 * (size_t)(K / kStepK) * 2 +
-           (mode == kGateUp ? 2 * (kXchgBytes + 32 * kTilePitchGateUp) : 2 * 32 * kTilePitchDown);
+           (mode == kGateUp ? kDrainSets * (kXchgBytes + kPassTokens * kTilePitchGateUp) : kDrainSets * kPassTokens * kTilePitchDown);
 }
 
 template <int MODE>

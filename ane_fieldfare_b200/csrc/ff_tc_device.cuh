@@ -118,6 +118,15 @@ __device__ __forceinline__ void tc_load_32cols(uint32_t taddr, uint32_t (&r)[32]
         : "r"(taddr)
         : "memory");
 }
+// 16 consecutive fp32 columns of this thread's TMEM lane.
+__device__ __forceinline__ void tc_load_16cols(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
 // 16 lanes x 32 fp32 columns: r[4 j + i] is lane l / 4 (i < 2) or l / 4 + 8, column 8 j + 2 (l % 4) + i % 2,
 // for the warp's lane l.
 __device__ __forceinline__ void tc_load_16x32(uint32_t taddr, uint32_t (&r)[16]) {
