@@ -89,33 +89,55 @@ __global__ void __launch_bounds__(kGemvThreads) k_int4_gemv(const __grid_constan
 // compared for equality with the CPU oracle): lane l chains fmaf over elements
 // [256 i + 8 l, +8) for i = 0, 1, ... in increasing index, the lane sums are added by an xor
 // butterfly (16, 8, 4, 2, 1), then the per-expert logit bias is added.
+// The expert's row (and per-input scale) of the first kRowChunks * 256 inputs is requested in front of the wait for the
+// launch before, the token's row all together behind it.
+constexpr int kRowChunks = 11;
 __global__ void __launch_bounds__(256)
 k_router_logits(const uint16_t *W, const uint16_t *scale, const float *bias, const uint16_t *x,
                 uint32_t xStride, int E, int D, float *logits, RouterTail tail) {
-    pdl_enter();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e = min((int)blockIdx.x * 8 + warp, E - 1);  // (a warp past the experts repeats the last)
     const int t = blockIdx.y;
     const uint16_t *wr = W + (size_t)e * D;
     const uint16_t *xr = x + (size_t)t * xStride;
-    float acc = 0.0f;
-    for (int base = 8 * lane; base < D; base += 256) {
-        const uint4 wv = *reinterpret_cast<const uint4 *>(wr + base);
-        const uint4 xv = *reinterpret_cast<const uint4 *>(xr + base);
-        uint4 sv = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
-        if (scale) sv = *reinterpret_cast<const uint4 *>(scale + base);
-        const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
-        const uint32_t xx[4] = {xv.x, xv.y, xv.z, xv.w};
-        const uint32_t ss[4] = {sv.x, sv.y, sv.z, sv.w};
+    uint4 wv[kRowChunks];
+    auto fetch = [&](int first) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            float x0 = __uint_as_float(xx[k] << 16), x1 = __uint_as_float(xx[k] & 0xFFFF0000u);
-            if (scale) {
-                x0 = x0 * __uint_as_float(ss[k] << 16);
-                x1 = x1 * __uint_as_float(ss[k] & 0xFFFF0000u);
+        for (int i = 0; i < kRowChunks; ++i) {
+            const int base = first + 256 * i + 8 * lane;
+            if (base < D) wv[i] = __ldg(reinterpret_cast<const uint4 *>(wr + base));
+        }
+    };
+    fetch(0);
+    pdl_enter();
+    float acc = 0.0f;
+    for (int first = 0; first < D; first += 256 * kRowChunks) {
+        if (first) fetch(first);
+        uint4 xv[kRowChunks];
+#pragma unroll
+        for (int i = 0; i < kRowChunks; ++i) {
+            const int base = first + 256 * i + 8 * lane;
+            if (base < D) xv[i] = *reinterpret_cast<const uint4 *>(xr + base);
+        }
+#pragma unroll
+        for (int i = 0; i < kRowChunks; ++i) {
+            const int base = first + 256 * i + 8 * lane;
+            if (base >= D) break;
+            uint4 sv = make_uint4(0, 0, 0, 0);
+            if (scale) sv = __ldg(reinterpret_cast<const uint4 *>(scale + base));
+            const uint32_t ww[4] = {wv[i].x, wv[i].y, wv[i].z, wv[i].w};
+            const uint32_t xx[4] = {xv[i].x, xv[i].y, xv[i].z, xv[i].w};
+            const uint32_t ss[4] = {sv.x, sv.y, sv.z, sv.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                float x0 = __uint_as_float(xx[k] << 16), x1 = __uint_as_float(xx[k] & 0xFFFF0000u);
+                if (scale) {
+                    x0 = x0 * __uint_as_float(ss[k] << 16);
+                    x1 = x1 * __uint_as_float(ss[k] & 0xFFFF0000u);
+                }
+                acc = fmaf(__uint_as_float(ww[k] << 16), x0, acc);
+                acc = fmaf(__uint_as_float(ww[k] & 0xFFFF0000u), x1, acc);
             }
-            acc = fmaf(__uint_as_float(ww[k] << 16), x0, acc);
-            acc = fmaf(__uint_as_float(ww[k] & 0xFFFF0000u), x1, acc);
         }
     }
 #pragma unroll

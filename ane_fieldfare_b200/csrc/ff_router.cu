@@ -458,50 +458,70 @@ k_router_select(const SelectArgs a) {
 
 // ---- INT8 logits of every expert (decode and verify rows, or when the logits are asked for) --------
 
-// One warp per expert and NT rows, the codes in lane order: a lane's codes of eight groups are one
-// 128-bit load, so the row's 2816 codes are six loads in flight instead of 44 in turn (one row and 128
-// experts: 26 -> 12.7 us with the launch; bound by 88 dependent multiply-adds and one memory latency).
-template <int NT>
+// One warp per expert and NT rows, the codes in lane order: a lane's codes of eight groups are one 128-bit load.
+// What does not depend on the launch before (codes, scales | biases, per-input scale: the first 3072 inputs' at once) is
+// requested in front of the wait for it, the rows all together behind it, so that a warp waits for memory once: one row of
+// 2816 inputs and 128 experts 12.7 -> 7.2 us.  Bound by that latency, the 88 dependent multiply-adds and the ranking by the
+// last CTA.
+// (kLaneRuns: runs of eight groups whose operands a warp holds at a time.)
+template <int NT, int kLaneRuns>
 __global__ void __launch_bounds__(128)
 k_router_logits_int8(const uint4 *Q, const uint32_t *aux, const uint16_t *effScale, const float *bias, const uint16_t *x,
                      uint32_t xStride, int T, int E, int D, float *logits, RouterTail tail) {
-    pdl_enter();
+    __shared__ __align__(16) uint4 sAux[4][kLaneRuns * 2];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e = min((int)blockIdx.x * 4 + warp, E - 1), t0 = blockIdx.y * NT;  // (a warp past the experts repeats the last)
     const int groups = D >> 6, runs = (groups + 7) >> 3;
     const uint4 *q = Q + (size_t)e * runs * 32 + lane;
     const uint4 *sb = reinterpret_cast<const uint4 *>(aux + (size_t)e * runs * 8);
-    const uint16_t *xr[NT];
+    const uint32_t *eff = reinterpret_cast<const uint32_t *>(effScale) + lane;
+    uint4 qv[kLaneRuns];
+    uint32_t ev[8 * kLaneRuns];
+    auto fetch = [&](int r0) {
+        if (lane < 2 * kLaneRuns) sAux[warp][lane] = 2 * r0 + lane < 2 * runs ? __ldg(sb + 2 * r0 + lane) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int r = 0; r < kLaneRuns; ++r) qv[r] = r0 + r < runs ? __ldg(q + (r0 + r) * 32) : make_uint4(0, 0, 0, 0);
+        if (effScale) {
+#pragma unroll
+            for (int i = 0; i < 8 * kLaneRuns; ++i) ev[i] = __ldg(eff + min(8 * r0 + i, groups - 1) * 32);
+        }
+    };
+    fetch(0);
+    pdl_enter();
+    const uint32_t *xr[NT];
     float acc[NT];
 #pragma unroll
-    for (int i = 0; i < NT; ++i) {
-        xr[i] = x + (size_t)min(t0 + i, T - 1) * xStride + 2 * lane;
-        acc[i] = 0.0f;
+    for (int k = 0; k < NT; ++k) {
+        xr[k] = reinterpret_cast<const uint32_t *>(x + (size_t)min(t0 + k, T - 1) * xStride) + lane;
+        acc[k] = 0.0f;
     }
-#pragma unroll 2
-    for (int r = 0; r < runs; ++r) {
-        const uint4 qa = __ldg(q + r * 32);
-        const uint4 sa[2] = {__ldg(sb + 2 * r), __ldg(sb + 2 * r + 1)};
-        const int n = min(8, groups - 8 * r);
-        uint32_t xv[NT][8], ev[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int g = 8 * r + min(i, n - 1);
-            ev[i] = effScale ? __ldg(reinterpret_cast<const uint32_t *>(effScale + g * 64 + 2 * lane)) : 0u;
-#pragma unroll
-            for (int k = 0; k < NT; ++k) xv[k][i] = *reinterpret_cast<const uint32_t *>(xr[k] + g * 64);
+    for (int r0 = 0; r0 < runs; r0 += kLaneRuns) {
+        if (r0) {
+            __syncwarp();
+            fetch(r0);
         }
+        uint32_t xv[NT][8 * kLaneRuns];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            if (i < n) {
+        for (int i = 0; i < 8 * kLaneRuns; ++i)
 #pragma unroll
-                for (int k = 0; k < NT; ++k) {
-                    float x0 = __uint_as_float(xv[k][i] << 16), x1 = __uint_as_float(xv[k][i] & 0xFFFF0000u);
-                    if (effScale) {
-                        x0 = x0 * __uint_as_float(ev[i] << 16);
-                        x1 = x1 * __uint_as_float(ev[i] & 0xFFFF0000u);
+            for (int k = 0; k < NT; ++k) xv[k][i] = xr[k][min(8 * r0 + i, groups - 1) * 32];
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < kLaneRuns; ++r) {
+            const uint4 sa[2] = {sAux[warp][2 * r], sAux[warp][2 * r + 1]};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (8 * (r0 + r) + i < groups) {
+#pragma unroll
+                    for (int k = 0; k < NT; ++k) {
+                        const uint32_t w = xv[k][8 * r + i];
+                        float x0 = __uint_as_float(w << 16), x1 = __uint_as_float(w & 0xFFFF0000u);
+                        if (effScale) {
+                            x0 = x0 * __uint_as_float(ev[8 * r + i] << 16);
+                            x1 = x1 * __uint_as_float(ev[8 * r + i] & 0xFFFF0000u);
+                        }
+                        acc[k] = int8_group(qv[r], sa, i, x0, x1, x0 + x1, acc[k]);
                     }
-                    acc[k] = int8_group(qa, sa, i, x0, x1, x0 + x1, acc[k]);
                 }
             }
         }
@@ -703,13 +723,13 @@ bool launch_router_logits_int8(FFContext *ctx, const LayerStore &L, const uint16
     const uint4 *lanes = reinterpret_cast<const uint4 *>(L.routerLanes);
     {
         LaunchScope scope(ctx, stream, "router_logits_int8");
-        if (tokens == 1)
-            FF_CUDA_OK(launch_pdl(k_router_logits_int8<1>, dim3((E + 3) / 4, 1), 128, 0, stream,
-                              lanes, L.routerAux, L.routerScale, L.logitBias, x, xStride,
-                                                                           1, E, D, logits, tail),
+        // (a block: a warp per expert and row, for the latency; more rows: two rows and few registers a warp)
+        if (tokens <= (uint32_t)kMaxGemvRows)
+            FF_CUDA_OK(launch_pdl(k_router_logits_int8<1, 6>, dim3((E + 3) / 4, tokens), 128, 0, stream,
+                              lanes, L.routerAux, L.routerScale, L.logitBias, x, xStride, (int)tokens, E, D, logits, tail),
                    error);
         else
-            FF_CUDA_OK(launch_pdl(k_router_logits_int8<2>, dim3((E + 3) / 4, (tokens + 1) / 2), 128, 0, stream,
+            FF_CUDA_OK(launch_pdl(k_router_logits_int8<2, 2>, dim3((E + 3) / 4, (tokens + 1) / 2), 128, 0, stream,
                               lanes, L.routerAux, L.routerScale, L.logitBias, x, xStride, (int)tokens, E, D, logits, tail),
                    error);
     }
