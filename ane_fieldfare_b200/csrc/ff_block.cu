@@ -299,8 +299,13 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps, const __g
     const int g = lane >> 2, t = lane & 3;
     const uint32_t smem = sm_addr(smemRaw);
     constexpr uint32_t kGroupBytes = INT8 ? 64 : 32;
-    if (!(MODE == kDown)) pdl_wait();  // (the down kernel's plan and first weights need only what was there before its predecessor)
-    if (MODE == kGateUp) pdl_trigger();
+    // Plan and first weights of the down kernel need only what was there before its predecessor, those of the INT8 FFN
+    // nothing that a launch writes (a decode forward of four INT8 layers 193 -> 187.5 us with them in front of the wait).
+    constexpr bool kLateWait = MODE == kDown || INT8;
+    if (!kLateWait) {
+        pdl_wait();
+        pdl_trigger();
+    }
     if (threadIdx.x == 0) {
         sUneven = 0u;
         for (int i = 0; i < 2 * kMaxWarps; ++i) bar_init(sm_addr(&sBar[i]), 1);
@@ -571,8 +576,8 @@ k_block_int(const BlockArgs a, const __grid_constant__ BlockMaps maps, const __g
         }
     };
 
-    if (MODE == kDown) {
-        pdl_wait();  // from here on: the activations
+    if (kLateWait) {
+        pdl_wait();  // from here on: the input rows
         pdl_trigger();
     }
     uint32_t used = 0, done = 0;  // done: tiles of this CTA's earlier segments, modulo the warps
