@@ -300,11 +300,14 @@ __device__ __forceinline__ void segment_histogram(const uint32_t *routes, int n,
     }
 }
 
-// The experts' offsets and row tiles (up to kRowTile rows of one expert each, experts ascending) from thread
-// e's number of routes to expert e (0 from E on); a CTA of 256 threads.  Returns the expert's offset.
+constexpr uint32_t kNoRow = 0xFFFFFFFFu;  // of a route to no expert
+
+// The experts' offsets and row tiles (up to `tileRows` rows of one expert each, experts ascending) from thread
+// e's number of routes to expert e (0 from E on); a CTA of at least 256 threads, of which one in a cluster writes.
+// Returns the expert's offset.
 // counts[0] = row tiles, counts[1] = pairs, counts[2] = experts with at least one pair.
 __device__ __forceinline__ uint32_t plan_row_tiles(uint32_t total, int E, uint32_t tileRows, uint32_t *expertOffsets, RowTile *tiles,
-                                                   uint32_t maxTiles, uint32_t *counts) {
+                                                   uint32_t maxTiles, uint32_t *counts, bool writes = true) {
     __shared__ uint32_t warpSums[3][8];
     const int e = threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t myTiles = (total + tileRows - 1u) / tileRows;
@@ -318,7 +321,7 @@ __device__ __forceinline__ uint32_t plan_row_tiles(uint32_t total, int E, uint32
         }
     }
     const uint32_t active = __popc(__ballot_sync(0xFFFFFFFFu, total != 0u));
-    if (lane == 31) {
+    if (lane == 31 && warp < 8) {
         warpSums[0][warp] = rows;
         warpSums[1][warp] = tileEnd;
         warpSums[2][warp] = active;
@@ -334,6 +337,7 @@ __device__ __forceinline__ uint32_t plan_row_tiles(uint32_t total, int E, uint32
         activeAll += warpSums[2][w];
     }
     const uint32_t start = rows - total;
+    if (!writes) return start;
     if (e < E) {
         expertOffsets[e] = start;
         for (uint32_t i = 0, tix = tileEnd - myTiles; i < total; i += tileRows, ++tix)
@@ -396,8 +400,6 @@ k_route_scan(uint32_t *blockCounts, int blocks, int E, uint32_t tileRows, uint32
     plan_row_tiles(total, E, tileRows, expertOffsets, tiles, maxTiles, counts);
 }
 
-constexpr uint32_t kNoRow = 0xFFFFFFFFu;  // of a route to no expert
-
 // Every route's position in (expert, token, rank) order; writes the sorted pair list.
 // Position = expert offset + routes to the expert in earlier blocks + in earlier warp segments of
 // this block + earlier in this warp's segment (earlier 32-route batches, then lower lanes).
@@ -458,26 +460,83 @@ k_route_scatter(const uint32_t *ids, int T, int K, int E,
                  sorted, rowOfRoute);
 }
 
-// All three passes for one block's worth of tokens: a chunk of up to 256 has one launch in front of its
-// gather instead of three (77 tokens: 14 us of a layer's 130 between the routes and the sorted list).
-__global__ void __launch_bounds__(256)
-k_route_sort(const uint32_t *ids, int T, int K, int E, uint32_t tileRows, uint32_t *expertOffsets, RowTile *tiles, uint32_t maxTiles, uint32_t *counts,
-             FFTokenExpertPair *sorted, uint32_t *rowOfRoute) {
+// All three passes in one launch of a cluster of eight CTAs for up to kClusterRoutes routes: every CTA counts its
+// share, a warp its part of that with the routes and their matches in registers, the CTAs read one another's counts
+// from shared memory, plan alike, and place.  Bound by its latencies, then by eight SMs' matches and scattered stores.
+// us in a graph, Zipf routes, 128 experts, one launch / three: 77 rows 3.7 / -, 257 4.3 / 15.1, 613 5.1 / 15.3, 1500
+// 7.9 / 15.5, 4096 15.4 / 16.9, 6000 21.2 / 17.4 (hence the limit).  (CTAs of 1024 threads, or sixteen of them, are
+// faster by themselves, 10.9 us at 4096 rows, but wait longer for SMs beside the shared FFN: a layer of 300 rows 308 us
+// for 298.)
+constexpr int kSortCtas = 8, kSortThreads = 512, kSortRounds = 8;  // rounds of 32 routes of a warp
+constexpr int kClusterRoutes = kSortCtas * kSortThreads * kSortRounds;
+__global__ void __cluster_dims__(kSortCtas, 1, 1) __launch_bounds__(kSortThreads, 1)
+k_route_sort(const uint32_t *ids, int T, int K, int E, uint32_t tileRows, uint32_t *expertOffsets, RowTile *tiles, uint32_t maxTiles,
+             uint32_t *counts, FFTokenExpertPair *sorted, uint32_t *rowOfRoute) {
     pdl_enter();
-    extern __shared__ uint32_t sRoutes[];
-    __shared__ uint32_t segCount[8 * kMaxExperts];
-    const int n = T * K, seg = (n + 7) / 8;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) sRoutes[i] = ids[i];
-    for (int i = threadIdx.x; i < 8 * E; i += blockDim.x) segCount[i] = 0;
+    __shared__ uint32_t segCount[(kSortThreads / 32) * kMaxExperts];  // a warp's routes to every expert, then its next place
+    __shared__ uint32_t ctaCount[kMaxExperts], sBase[kMaxExperts];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, e = threadIdx.x;
+    const uint32_t cta = cluster_cta_rank();
+    const int perCta = (T + kSortCtas - 1) / kSortCtas * K, first = min((int)cta * perCta, T * K), n = min(perCta, T * K - first);
+    const int seg = (n + kSortThreads / 32 - 1) / (kSortThreads / 32), begin = warp * seg, end = min(n, begin + seg);
+    uint32_t *mine = segCount + warp * E;
+    uint32_t id[kSortRounds], peers[kSortRounds];
+#pragma unroll
+    for (int r = 0; r < kSortRounds; ++r) {
+        const int i = begin + 32 * r + lane;
+        id[r] = i < end ? ids[first + i] : 0xFFFFFFFFu;
+    }
+    for (int x = lane; x < E; x += 32) mine[x] = 0;
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < kSortRounds; ++r) {
+        if (begin + 32 * r >= end) break;
+        peers[r] = __match_any_sync(0xFFFFFFFFu, id[r]);
+        if (id[r] < (uint32_t)E && (peers[r] & ((1u << lane) - 1u)) == 0u) mine[id[r]] += (uint32_t)__popc(peers[r]);
+        __syncwarp();
+    }
     __syncthreads();
-    segment_histogram(sRoutes, n, seg, E, segCount);
+    if (e < E) {
+        uint32_t run = 0;
+#pragma unroll 8
+        for (int w = 0; w < kSortThreads / 32; ++w) {
+            const uint32_t c = segCount[w * E + e];
+            segCount[w * E + e] = run;
+            run += c;
+        }
+        ctaCount[e] = run;
+    }
+    cluster_sync_all();
+    uint32_t total = 0, earlier = 0;
+    if (e < E) {
+        uint32_t c[kSortCtas];
+        const uint32_t addr = smem_u32(ctaCount + e);
+#pragma unroll
+        for (uint32_t i = 0; i < kSortCtas; ++i) asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(c[i]) : "r"(map_to_cta(addr, i)));
+#pragma unroll
+        for (uint32_t i = 0; i < kSortCtas; ++i) {
+            total += c[i];
+            if (i < cta) earlier += c[i];
+        }
+    }
+    const uint32_t start = plan_row_tiles(total, E, tileRows, expertOffsets, tiles, maxTiles, counts, cta == 0u);
+    if (e < E) sBase[e] = start + earlier;
     __syncthreads();
-    const int e = threadIdx.x;
-    uint32_t total = 0;
-    if (e < E)
-        for (int w = 0; w < 8; ++w) total += segCount[w * E + e];
-    const uint32_t start = plan_row_tiles(total, E, tileRows, expertOffsets, tiles, maxTiles, counts);
-    place_routes(sRoutes, segCount, n, seg, start, 0, K, E, sorted, rowOfRoute);
+#pragma unroll
+    for (int r = 0; r < kSortRounds; ++r) {
+        if (begin + 32 * r >= end) break;
+        const int i = first + begin + 32 * r + lane;
+        const bool valid = begin + 32 * r + lane < end, live = valid && id[r] < (uint32_t)E;
+        const uint32_t lower = peers[r] & ((1u << lane) - 1u);
+        uint32_t pos = 0;
+        if (live) pos = sBase[id[r]] + mine[id[r]] + (uint32_t)__popc(lower);
+        __syncwarp();
+        if (live && lower == 0u) mine[id[r]] += (uint32_t)__popc(peers[r]);
+        __syncwarp();
+        if (live) sorted[pos] = FFTokenExpertPair{(uint32_t)(i / K), id[r], (uint32_t)(i % K), 0u};
+        if (rowOfRoute && valid) rowOfRoute[i] = live ? pos : kNoRow;
+    }
+    cluster_sync_all();  // no CTA leaves while another may read its counts
 }
 
 // Row tiles of a dense problem: T rows of one "expert" (the shared FFN).
@@ -1250,9 +1309,9 @@ static bool sort_routes(FFContext *ctx, const uint32_t *ids, uint32_t tokens, in
     const uint32_t blocks = (tokens + kSortTokens - 1) / kSortTokens;
     const size_t sortSmem = (size_t)kSortTokens * K * sizeof(uint32_t);
     const uint32_t maxTiles = ctx->maxUnits / 2;  // first half of the tile buffer
-    if (blocks == 1) {
+    if ((T + kSortCtas - 1) / kSortCtas * K <= kClusterRoutes / kSortCtas) {
         LaunchScope scope(ctx, stream, "route_sort");
-        FF_CUDA_OK(launch_pdl(k_route_sort, 1, 256, sortSmem, stream, ids, T, K, E, tileRows, offsets, tiles, maxTiles, ctx->unitCount, sorted,
+        FF_CUDA_OK(launch_pdl(k_route_sort, kSortCtas, kSortThreads, 0, stream, ids, T, K, E, tileRows, offsets, tiles, maxTiles, ctx->unitCount, sorted,
                               rowOfRoute),
                    error);
         return true;

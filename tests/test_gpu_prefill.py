@@ -236,3 +236,26 @@ def test_guest_plugin_contract(tiny, oracle):
     assert guest.profile == {"layers": 1, "pairs": tokens * L.topK}
     assert (partials[tokens * L.topK:] == -99.0).all()
     assert not (partials[:tokens * L.topK] == -99.0).all(dim=1).any()
+
+
+@pytest.mark.parametrize("tokens,groups,top", [(17, 1, 8), (255, 256, 8), (256, 128, 8), (257, 128, 8), (4096, 256, 8), (4097, 128, 8),
+                                               (4104, 3, 8), (5000, 16, 1), (40000, 128, 1)])
+def test_sort_routes_at_the_launch_edges(tokens, groups, top):
+    """One launch of a cluster up to 4096 eight-route rows, three launches beyond; uneven shares of its CTAs and warps, empty ones,
+    one group holding nearly all routes.  Exact against a stable sort on the host."""
+    hp = _hp()
+    ctx = hp.HotpathContext(layers=1, experts=max(8, groups), d=64, f=64, sharedF=0, topK=top, maxTokens=tokens)
+    try:
+        rng = np.random.default_rng(tokens)
+        ids = rng.integers(0, groups + 1, size=(tokens, top)).astype(np.int32)  # `groups` itself: dropped
+        ids[rng.random((tokens, top)) < 0.5] = groups // 2
+        pairs, offsets = hp.PrefillGroupedRoutedMoE(ctx).sortRoutesOnDevice(None, torch.from_numpy(ids).to(ctx.device), groups)
+        torch.cuda.synchronize()
+        flat = ids.reshape(-1)
+        keep = np.flatnonzero(flat < groups)
+        order = keep[np.argsort(flat[keep], kind="stable")]
+        assert np.array_equal(offsets.cpu().numpy(), np.concatenate([[0], np.cumsum(np.bincount(flat[keep], minlength=groups))]))
+        got = pairs.cpu().numpy()[:order.size]
+        assert np.array_equal(got[:, 0], order // top) and np.array_equal(got[:, 1], flat[order]) and np.array_equal(got[:, 2], order % top)
+    finally:
+        ctx.close()
