@@ -78,6 +78,11 @@ __device__ __forceinline__ bool rt_wait(uint32_t bar, uint32_t parity) {
     return mbar_try_wait(bar, parity) || rt_wait_slow(bar, parity);
 }
 
+// (a multiple of 16, so that the next warp's rows are aligned with an odd number of experts, too)
+__host__ __device__ inline size_t router_warp_bytes(int tokens, int D, int E) {
+    return ((size_t)tokens * D * 2 + (size_t)tokens * E * 4 + 15) & ~(size_t)15;
+}
+
 template <int kTok>
 __global__ void __launch_bounds__((kRouterTokensPerCta / kTok + 1) * 32)
 k_router_rows(const __grid_constant__ CUtensorMap mapW, const uint16_t *scale, const float *bias,
@@ -88,7 +93,7 @@ k_router_rows(const __grid_constant__ CUtensorMap mapW, const uint16_t *scale, c
     __shared__ __align__(8) uint64_t ringBar[2 * kRouterRing];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // ring of router blocks, then per computing warp: kTok input rows as bf16 and kTok x E logits
-    const size_t perWarp = (size_t)kTok * D * 2 + (size_t)kTok * E * 4;
+    const size_t perWarp = router_warp_bytes(kTok, D, E);
     const uint32_t ringAddr = (uint32_t)__cvta_generic_to_shared(rsmRaw);
     const uint32_t barBase = (uint32_t)__cvta_generic_to_shared(&ringBar[0]);
     auto barFull = [&](int s) { return barBase + 8u * (uint32_t)s; };
@@ -261,11 +266,10 @@ bool launch_router_prefill(FFContext *ctx, const LayerStore &L, const uint16_t *
     // encoding is host arithmetic only)
     CUtensorMap mapW;
     if (!make_router_map(&mapW, L.routerW, (uint64_t)E, (uint64_t)D, error)) return false;
-    // shared memory: the ring, and per CTA 32 tokens' inputs and logits whatever the split into warps
-    const size_t smem = (size_t)kRouterRing * kRouterBlockBytes +
-                        (size_t)kRouterTokensPerCta * ((size_t)D * 2 + (size_t)E * 4);
+    constexpr int kTok = 2;
+    const size_t smem = (size_t)kRouterRing * kRouterBlockBytes + (size_t)(kRouterTokensPerCta / kTok) * router_warp_bytes(kTok, D, E);
     if (smem > 226 * 1024) return fail(error, "model width too large for the router's shared memory");
-    return launch_router_rows<2>(ctx, L, mapW, smem, x, xStride, tokens, ids, weights, logits, stream, error);
+    return launch_router_rows<kTok>(ctx, L, mapW, smem, x, xStride, tokens, ids, weights, logits, stream, error);
 }
 
 // ---- device-side permute -------------------------------------------------------------------

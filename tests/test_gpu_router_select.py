@@ -125,3 +125,26 @@ def test_selected_routes_at_every_number_of_warps(form, rows):
         assert torch.equal(weights[0].view(torch.int16), weights[1].view(torch.int16))
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("experts", [9, 131])
+def test_logits_of_an_odd_number_of_experts(experts):
+    """The kernel that forms every logit of many rows keeps each warp's rows aligned: ids as a block's kernel gives them."""
+    from ane_fieldfare_b200 import hotpath as hp
+    rows, d, k = 40, 192, 5
+    ctx = hp.HotpathContext(layers=1, experts=experts, d=d, f=64, sharedF=0, topK=k, maxTokens=rows)
+    try:
+        ctx.loadRouter(0, synth.normal_bf16(0x40, "odd.router", (experts, d), 0.02))
+        x = hp.bf16_tensor(workload.make_tokens(0x41, "odd", rows, d), ctx.device)
+        got = [torch.full((rows, k), -1, dtype=torch.int32, device=ctx.device) for _ in range(2)]
+        weights = torch.zeros((rows, k), dtype=torch.bfloat16, device=ctx.device)
+        logits = torch.zeros((rows, experts), dtype=torch.float32, device=ctx.device)
+        router = hp.PrefillRouter(ctx)
+        router.encodeGemma4Block(None, 0, x, got[0], weights, rows, outLogits=logits)
+        for r in range(0, rows, 16):
+            router.encodeGemma4Block(None, 0, x[r:], got[1][r:], weights[r:], min(16, rows - r))
+        torch.cuda.synchronize()
+        assert ctx.info().deviceErrorFlag == 0
+        assert torch.equal(got[0], got[1])
+    finally:
+        ctx.close()
