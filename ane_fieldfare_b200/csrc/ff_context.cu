@@ -149,8 +149,8 @@ FFContext *ff_create(int32_t deviceOrdinal, const FFConfig *config, const char *
     ok = ok && dev_alloc(ctx, &ctx->weights, T * K, error);
     ok = ok && dev_alloc(ctx, &ctx->plan, 1, error);
     if (ok) ok = cudaMemset(ctx->plan, 0, sizeof(RoutePlan)) == cudaSuccess;
-    ok = ok && dev_alloc(ctx, &ctx->routerCounts, kMaxGemvRows, error);
-    if (ok) ok = cudaMemset(ctx->routerCounts, 0, kMaxGemvRows * 4) == cudaSuccess;
+    ok = ok && dev_alloc(ctx, &ctx->routerCounts, kRouterCounts, error);
+    if (ok) ok = cudaMemset(ctx->routerCounts, 0, kRouterCounts * 4) == cudaSuccess;
     ok = ok && dev_alloc(ctx, &ctx->acts, (T * K + 256) * c.f, error);  // +256: a GEMM row tile may overhang
     ok = ok && dev_alloc(ctx, &ctx->sharedActs, (T + 256) * c.sharedF, error);
     ok = ok && dev_alloc(ctx, &ctx->h1, T * c.d, error);

@@ -15,6 +15,7 @@ namespace ff {
 
 constexpr int kGroup = 64;        // codes per scale/bias pair
 constexpr int kMaxGemvRows = 16;  // input rows one GEMV job can carry (a verify block)
+constexpr int kRouterCounts = 64;
 constexpr int kDecodeMaps = 6;
 constexpr int kMaxExperts = 256;  // router width limit, as in the reference's prefill router
 
@@ -166,7 +167,7 @@ struct FFContext {
     uint32_t *ids = nullptr;        // [maxTokens][topK]
     uint16_t *weights = nullptr;    // [maxTokens][topK]
     ff::RoutePlan *plan = nullptr;
-    uint32_t *routerCounts = nullptr;  // [kMaxGemvRows] CTAs that have formed a row's logits
+    uint32_t *routerCounts = nullptr;  // [kRouterCounts] CTAs that have formed the logits of a row (a block) or of a tile of rows
     uint16_t *acts = nullptr;       // [maxTokens*topK][f]
     uint16_t *sharedActs = nullptr; // [maxTokens][sharedF]
     uint16_t *h1 = nullptr;         // [maxTokens][d]

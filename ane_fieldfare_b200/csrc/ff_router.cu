@@ -1,4 +1,5 @@
-// Router of a prefill chunk (more rows than a decode/verify block) when only the routes are asked for.
+// Router of a prefill chunk (more rows than a decode/verify block) when only the routes are asked for: up to kTileMaxRows
+// rows every logit in one launch (k_router_tile), more rows as follows.
 //
 // The contract is bitwise: logits are sums in a fixed fp32 order (bf16 router: lane l chains fmaf over
 // [256 i + 8 l, +8); INT8 router: over elements 64 g + 2 l, + 1; xor butterfly; then the logit bias),
@@ -539,6 +540,168 @@ k_router_logits_int8(const uint4 *Q, const uint32_t *aux, const uint16_t *effSca
                              tail.weights + (t0 + k) * tail.K, tail.counts + t0 + k, gridDim.x);
 }
 
+// ---- a short chunk: every logit in its order, and the top K, in one launch --------------------------
+
+// CTA (expert tile, token tile): a warp per expert, its row in registers (requested in front of the wait for the launch
+// before), kTileTokens rows in shared memory: bf16, or (WIDE) fp32 times the per-input scale.  The last CTA of a token
+// tile ranks its rows, a warp each.  A pair of expert and row is about 280 warp instructions, which bounds it; the
+// approximate logits and the selection behind them are two launches and cost less for more rows.  us in a graph for 128
+// experts and 2816 inputs, this / those: 17 rows 9.3 / 13.9, 77 11.3 / 16.4, 128 11.7 / 18.0, 160 15.1 / 18.0, 256 18.0 /
+// 18.0, 320 22.4 / 18.5; INT8 11.8 / 17.5, 14.9 / 21.0, 15.4 / 22.6, 21.9 / 23.1, 26.1 / 23.6.
+constexpr int kTileTokens = 8, kTileExperts = 8, kTileChunks = 11;
+constexpr uint32_t kTileMaxRows = 160;
+static_assert((kTileMaxRows + kTileTokens - 1) / kTileTokens <= (uint32_t)kRouterCounts, "a counter for every tile of rows");
+struct TileArgs {
+    const uint16_t *W;           // bf16 router [E][D], or
+    const uint4 *Q;              // INT8 router in lane order
+    const uint32_t *qAux;
+    const uint16_t *scale, *gain;
+    const float *bias;
+    const uint16_t *x;
+    uint32_t xStride;
+    int T, E, D, K;
+    float *logits;               // [T][E]
+    uint32_t *counts;            // CTAs of a token tile that are done, zero between launches
+    uint32_t *ids;
+    uint16_t *weights;
+};
+template <bool INT8, bool WIDE>
+__global__ void __launch_bounds__(kTileExperts * 32)
+k_router_tile(const TileArgs a) {
+    extern __shared__ __align__(16) uint8_t selectSmem[];
+    __shared__ uint32_t sLast;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int e = min((int)blockIdx.x * kTileExperts + warp, a.E - 1);  // (a warp past the experts repeats the last)
+    const int t0 = (int)blockIdx.y * kTileTokens, tokens = min(kTileTokens, a.T - t0);
+    constexpr int kRuns = 6;  // INT8: of eight groups
+    const int groups = a.D >> 6, runs = (groups + 7) >> 3;
+    uint4 wv[INT8 ? kRuns : kTileChunks], sb[INT8 ? 2 * kRuns : 1];
+    auto fetch = [&](int first) {  // INT8: run, else chunk of 256 inputs
+        if constexpr (INT8) {
+#pragma unroll
+            for (int r = 0; r < kRuns; ++r) {
+                const bool there = first + r < runs;
+                wv[r] = there ? __ldg(a.Q + ((size_t)e * runs + first + r) * 32 + lane) : make_uint4(0, 0, 0, 0);
+                const uint4 *aux = reinterpret_cast<const uint4 *>(a.qAux + (size_t)e * runs * 8) + 2 * (first + r);
+                sb[2 * r] = there ? __ldg(aux) : make_uint4(0, 0, 0, 0);
+                sb[2 * r + 1] = there ? __ldg(aux + 1) : make_uint4(0, 0, 0, 0);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < kTileChunks; ++i) {
+                const int base = (first + i) * 256 + 8 * lane;
+                wv[i] = base < a.D ? __ldg(reinterpret_cast<const uint4 *>(a.W + (size_t)e * a.D + base)) : make_uint4(0, 0, 0, 0);
+            }
+        }
+    };
+    fetch(0);
+    pdl_enter();
+    const uint32_t rowBytes = (uint32_t)a.D * (WIDE ? 4u : 2u);
+    {
+        const int chunks = a.D >> 3;
+        // a warp a row (past the rows: the last again, so that every row of the tile is defined)
+        const uint4 *src = reinterpret_cast<const uint4 *>(a.x + (size_t)(t0 + min(warp, tokens - 1)) * a.xStride);
+        uint8_t *dst = selectSmem + (uint32_t)warp * rowBytes;
+#pragma unroll 4
+        for (int c = lane; c < chunks; c += 32) {
+            const uint4 v = src[c];
+            if (!WIDE) {
+                reinterpret_cast<uint4 *>(dst)[c] = v;
+                continue;
+            }
+            uint4 sv = make_uint4(0, 0, 0, 0);
+            if (a.scale) sv = __ldg(reinterpret_cast<const uint4 *>(a.scale) + c);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w}, f[4] = {sv.x, sv.y, sv.z, sv.w};
+            float xe[8];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                xe[2 * k] = __uint_as_float(w[k] << 16);
+                xe[2 * k + 1] = __uint_as_float(w[k] & 0xFFFF0000u);
+                if (a.scale) {
+                    xe[2 * k] = xe[2 * k] * __uint_as_float(f[k] << 16);
+                    xe[2 * k + 1] = xe[2 * k + 1] * __uint_as_float(f[k] & 0xFFFF0000u);
+                }
+            }
+            reinterpret_cast<float4 *>(dst)[2 * c] = make_float4(xe[0], xe[1], xe[2], xe[3]);
+            reinterpret_cast<float4 *>(dst)[2 * c + 1] = make_float4(xe[4], xe[5], xe[6], xe[7]);
+        }
+    }
+    __syncthreads();
+    static_assert(kTileTokens == kTileExperts, "a warp stages a row");
+    float acc[kTileTokens];
+#pragma unroll
+    for (int t = 0; t < kTileTokens; ++t) acc[t] = 0.0f;
+    if constexpr (INT8) {
+        for (int first = 0; first < runs; first += kRuns) {
+            if (first) fetch(first);
+#pragma unroll
+            for (int r = 0; r < kRuns; ++r) {
+                const uint4 aux[2] = {sb[2 * r], sb[2 * r + 1]};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int g = 8 * (first + r) + i;
+                    if (g >= groups) break;
+#pragma unroll
+                    for (int t = 0; t < kTileTokens; ++t) {
+                        const float2 x = *reinterpret_cast<const float2 *>(selectSmem + (uint32_t)t * rowBytes + (uint32_t)(g * 32 + lane) * 8u);
+                        acc[t] = int8_group(wv[r], aux, i, x.x, x.y, x.x + x.y, acc[t]);
+                    }
+                }
+            }
+        }
+    } else {
+        const int chunks = (a.D + 255) >> 8;
+        for (int first = 0; first < chunks; first += kTileChunks) {
+            if (first) fetch(first);
+#pragma unroll
+            for (int i = 0; i < kTileChunks; ++i) {
+                const int base = (first + i) * 256 + 8 * lane;
+                if (base >= a.D) break;
+                const uint32_t ww[4] = {wv[i].x, wv[i].y, wv[i].z, wv[i].w};
+                float w[8];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    w[2 * k] = __uint_as_float(ww[k] << 16);
+                    w[2 * k + 1] = __uint_as_float(ww[k] & 0xFFFF0000u);
+                }
+#pragma unroll
+                for (int t = 0; t < kTileTokens; ++t) {
+                    const uint8_t *row = selectSmem + (uint32_t)t * rowBytes;
+                    float x[8];
+                    if (WIDE) {
+                        const float4 lo = *reinterpret_cast<const float4 *>(row + (uint32_t)base * 4u), hi = *reinterpret_cast<const float4 *>(row + (uint32_t)base * 4u + 16u);
+                        x[0] = lo.x, x[1] = lo.y, x[2] = lo.z, x[3] = lo.w, x[4] = hi.x, x[5] = hi.y, x[6] = hi.z, x[7] = hi.w;
+                    } else {
+                        const uint4 v = *reinterpret_cast<const uint4 *>(row + (uint32_t)base * 2u);
+                        const uint32_t xx[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            x[2 * k] = __uint_as_float(xx[k] << 16);
+                            x[2 * k + 1] = __uint_as_float(xx[k] & 0xFFFF0000u);
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) acc[t] = fmaf(w[k], x[k], acc[t]);
+                }
+            }
+        }
+    }
+    int which;
+    const float v = butterfly<kTileTokens>(acc, lane, which);
+    if ((lane & (32 / kTileTokens - 1)) == 0 && which < tokens) a.logits[(size_t)(t0 + which) * a.E + e] = a.bias ? v + a.bias[e] : v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        sLast = atomicInc(a.counts + blockIdx.y, gridDim.x - 1u) == gridDim.x - 1u ? 1u : 0u;
+    }
+    __syncthreads();
+    if (sLast && warp < tokens) {
+        __threadfence();
+        const size_t t = (size_t)(t0 + warp);
+        warp_topk(a.logits + t * a.E, a.E, a.K, a.gain, a.ids + t * a.K, a.weights + t * a.K);
+    }
+}
+
 // ---- at load: folded bf16 weights and the bound's coefficients --------------------------------------
 
 // One CTA per expert.  folded = bf16(w * scale) (null: the router's own bf16 rows are multiplied).  Norms in
@@ -652,9 +815,42 @@ bool router_prepare(FFContext *ctx, LayerStore &L, const char **error) {
     return true;
 }
 
+static bool launch_router_tile(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens, uint32_t *ids,
+                               uint16_t *weights, cudaStream_t stream, const char **error) {
+    TileArgs a{};
+    a.W = L.routerW;
+    a.Q = reinterpret_cast<const uint4 *>(L.routerLanes);
+    a.qAux = L.routerAux;
+    a.scale = L.routerScale;
+    a.gain = L.gain;
+    a.bias = L.logitBias;
+    a.x = x;
+    a.xStride = xStride;
+    a.T = (int)tokens;
+    a.E = (int)L.routerExperts;
+    a.D = (int)ctx->cfg.d;
+    a.K = (int)ctx->cfg.topK;
+    a.logits = ctx->routerParts;
+    a.counts = ctx->routerCounts;
+    a.ids = ids;
+    a.weights = weights;
+    const int form = L.routerQ ? 2 : L.routerScale ? 1 : 0;
+    auto kernel = form == 2 ? k_router_tile<true, true> : form == 1 ? k_router_tile<false, true> : k_router_tile<false, false>;
+    const size_t smem = (size_t)kTileTokens * a.D * (form ? 4 : 2);
+    static KernelSmemMemo memo[3];
+    if (!memo[form].prepare(kernel, ctx->device, smem, kTileExperts * 32, nullptr, error)) return false;
+    LaunchScope scope(ctx, stream, "router_tile");
+    FF_CUDA_OK(launch_pdl(kernel, dim3((a.E + kTileExperts - 1) / kTileExperts, (tokens + kTileTokens - 1) / kTileTokens), kTileExperts * 32, smem,
+                          stream, a),
+               error);
+    return true;
+}
+
 bool launch_router_select(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens,
                           uint32_t *ids, uint16_t *weights, cudaStream_t stream, const char **error) {
     const uint32_t E = L.routerExperts, D = ctx->cfg.d, K = ctx->cfg.topK;
+    if (tokens <= kTileMaxRows && (size_t)kTileTokens * D * (L.routerQ || L.routerScale ? 4 : 2) <= 200 * 1024)
+        return launch_router_tile(ctx, L, x, xStride, tokens, ids, weights, stream, error);
     // Token tile: as large as the rows allow (the router's 720 KB are read once per tile and split);
     // the contraction is split while tiles x splits stay within one CTA per SM.
     const uint32_t tileTokens = std::min(128u, (tokens + 31u) & ~31u);

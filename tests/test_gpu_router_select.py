@@ -127,6 +127,38 @@ def test_selected_routes_at_every_number_of_warps(form, rows):
         ctx.close()
 
 
+@pytest.mark.parametrize("form", ["bf16", "bf16_scaled", "int8"])
+@pytest.mark.parametrize("experts,d,rows", [(9, 64, 17), (12, 4160, 24), (130, 3072, 25), (128, 6400, 160), (128, 6464, 160), (128, 2816, 161)])
+def test_routes_of_a_short_chunk(form, experts, d, rows):
+    """Edges of the one-launch kernel: tiles of eight rows and experts, contractions of more than one set of a warp's registers,
+    and where the rows (160) or their width (fp32 rows of 6400) go over to the two launches.  Against blocks of 16 rows, twice
+    in a row (its counters)."""
+    from ane_fieldfare_b200 import hotpath as hp
+    k = 5
+    ctx = hp.HotpathContext(layers=1, experts=experts, d=d, f=64, sharedF=0, topK=k, maxTokens=rows)
+    try:
+        eff = None if form == "bf16" else synth.bf16_bits(synth.uniform(7, d, 0.5, 1.5))
+        if form == "int8":
+            ctx.loadRouterInt8(0, *int8_router(0x3D, experts, d), effectiveScale=eff)
+        else:
+            ctx.loadRouter(0, synth.normal_bf16(0x3E, "short.router", (experts, d), 0.02), effectiveScale=eff)
+        x = hp.bf16_tensor(workload.make_tokens(0x3F, f"short{rows}", rows, d), ctx.device)
+        got = [torch.full((rows, k), -1, dtype=torch.int32, device=ctx.device) for _ in range(3)]
+        weights = [torch.zeros((rows, k), dtype=torch.bfloat16, device=ctx.device) for _ in range(3)]
+        router = hp.PrefillRouter(ctx)
+        for r in range(0, rows, 16):  # a block's kernel
+            router.encodeGemma4Block(None, 0, x[r:], got[0][r:], weights[0][r:], min(16, rows - r))
+        for i in (1, 2):
+            router.encodeGemma4Block(None, 0, x, got[i], weights[i], rows)
+        torch.cuda.synchronize()
+        assert ctx.info().deviceErrorFlag == 0
+        for i in (1, 2):
+            assert torch.equal(got[0], got[i])
+            assert torch.equal(weights[0].view(torch.int16), weights[i].view(torch.int16))
+    finally:
+        ctx.close()
+
+
 @pytest.mark.parametrize("experts", [9, 131])
 def test_logits_of_an_odd_number_of_experts(experts):
     """The kernel that forms every logit of many rows keeps each warp's rows aligned: ids as a block's kernel gives them."""
