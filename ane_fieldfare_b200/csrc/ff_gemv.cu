@@ -179,7 +179,7 @@ k_reduce_token_major(const uint16_t *partials, const uint32_t *rowIndex, const u
 // above: rank ascending, then the residual); for rows that are 16-byte aligned.  B = 8: the loads
 // of eight ranks are issued together, for blocks of at most a wave, where their latencies one after another
 // are the time (77 rows 4.4 -> 3.5 us); B = 1 beyond, where more warps in flight beat more loads of each (32768
-// rows 363 us, with B = 8 450 us).
+// rows 363 us, with B = 8 450 us).  The partial rows are streamed: a layer of 4096 rows 614 -> 607 us, of 3000 485 -> 479.
 template <int B>
 __global__ void __launch_bounds__(256)
 k_reduce_token_major_x8(const uint16_t *partials, const uint32_t *rowIndex, const uint16_t *weights,
@@ -202,7 +202,7 @@ k_reduce_token_major_x8(const uint16_t *partials, const uint32_t *rowIndex, cons
             if (r0 + r < K) {
                 const size_t route = (size_t)t * K + r0 + r, row = rowIndex ? (size_t)rowIndex[route] : route;
                 w[r] = bf2f(weights[route]);
-                v[r] = *reinterpret_cast<const uint4 *>(partials + row * D + d);
+                v[r] = __ldcs(reinterpret_cast<const uint4 *>(partials + row * D + d));  // read once
             }
         }
 #pragma unroll
