@@ -239,12 +239,9 @@ bool ff_moe_layer(FFContext *ctx, uint32_t layer, const uint16_t *x, uint32_t to
         // Shared FFN and routed part do not need each other before the reduction: the shared FFN goes to
         // the side stream, so that it fills the SMs while router and sort run (short kernels, one CTA
         // to a few dozen).  The side stream has the lowest priority: the routed part is the longer chain.
-        // Only while the shared FFN's first GEMM is at most two waves of the chip: longer ones hold the SMs
-        // that the router and the sort wait for (77 rows 353 -> 282 us a layer pair; 2000 rows 607 -> 618).
-        // (INT8: counted in tiles of 128 rows; smaller ones are more units that take less time each.)
-        const uint32_t tileRows = shared8 ? 128u : 192u;
-        const uint32_t sharedUnits = (tokens + tileRows - 1u) / tileRows * ((cfg.sharedF + 127u) / 128u);  // CTA pairs
-        const bool side = sharedRows != nullptr && sharedUnits <= (uint32_t)ctx->smCount;
+        // us of a layer beside / behind the router: 800 rows 213 / 227, 2000 INT8 437 / 472, 3000 462 / 485, 4096 596 / 614,
+        // 6000 838 / 836, three layers of 32768 13 600 / 13 720.
+        const bool side = sharedRows != nullptr;
         if (side) {
             FF_CUDA_OK(cudaEventRecord(ctx->forked, c.stream), error);
             FF_CUDA_OK(cudaStreamWaitEvent(ctx->sideStream, ctx->forked, 0), error);
