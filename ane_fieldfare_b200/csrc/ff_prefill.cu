@@ -639,7 +639,7 @@ struct GemmArgs {
     const uint32_t *scaleWords;  // scale | bias words of expert 0 (see pack_scales), of its down rows for the down GEMM
     uint64_t scaleStride;        // words between experts
     uint32_t tileRows, packStages;
-    uint32_t scaleBuffers;       // units whose scale words are held in shared memory: 2, 1 or 0 (read per step)
+    uint32_t scaleBuffers;     // see GemmRings
     uint32_t K;                // contraction length (multiple of 64)
     uint32_t N;                // outputs per row: F (gate/up) or D (down)
     uint32_t nTiles;           // weight-row tiles: ceil(N/64) for gate/up, ceil(N/128) for down
@@ -1243,11 +1243,29 @@ bool prefill_prepare_layer(FFContext *ctx, LayerStore &L, const char **error) {
     return true;
 }
 
-// Shared memory of a GEMM over K with `buffers` units' scale words.
-static size_t gemm_smem_bytes(int mode, uint32_t K, uint32_t tileRows, uint32_t packStages, uint32_t buffers) {
-    const size_t quads = (K / kTileK + kQuad - 1) / kQuad;
-    return 1024 + (size_t)kTokStages * 2 * tok_tile_bytes(tileRows) + (size_t)packStages * kPackTileBytes +
-           (mode == kModeGateUp ? kEpilogueBytesGateUp : kEpilogueBytesDown) + buffers * scale_buffer_bytes((uint32_t)quads);
+// Slots that the code ring needs at least.  A group takes every second quad, so in a ring of odd length it skips every second
+// phase of a slot, and its parity says nothing about the phase it skips.  What orders that phase is the pair that the group
+// stored last: it waited for the MMAs `weightStages / 2` pairs further back, so quads up to 2 + weightStages / 4 back have
+// landed.  (Three slots with eight weight stages were one short: a conversion could start on the slot's former codes.)
+__host__ __device__ constexpr uint32_t min_pack_stages(uint32_t weightStages) { return 2u + weightStages / 4u; }
+
+// Sizes of a GEMM's rings for a contraction of K.
+struct GemmRings {
+    uint32_t packStages;    // quads of packed codes
+    uint32_t scaleBuffers;  // units whose scale words are held: 2 (one ahead), 1 (the unit's own) or 0 (read step by step)
+    size_t smem;
+};
+static GemmRings gemm_rings(int mode, uint32_t K, uint32_t tileRows) {
+    const uint32_t quads = (K / kTileK + kQuad - 1) / kQuad;
+    GemmRings r{min_pack_stages(weight_stages(tileRows)), 2, 0};
+    const auto bytes = [&] {
+        return 1024 + (size_t)kTokStages * 2 * tok_tile_bytes(tileRows) + (size_t)r.packStages * kPackTileBytes +
+               (mode == kModeGateUp ? kEpilogueBytesGateUp : kEpilogueBytesDown) + (size_t)r.scaleBuffers * scale_buffer_bytes(quads);
+    };
+    while (r.scaleBuffers && bytes() > 226 * 1024) --r.scaleBuffers;
+    while (r.packStages < (uint32_t)kMaxPackStages && bytes() + kPackTileBytes <= 226 * 1024) ++r.packStages;
+    r.smem = bytes();
+    return r;
 }
 
 // Rows of a routed GEMM's tiles.  Tiles of 128 rows leave tensor memory for eight weight stages instead of four, and a
@@ -1280,13 +1298,10 @@ static bool launch_gemm(FFContext *ctx, const uint16_t *x, uint64_t rows, const 
         !make_activation_map(&mapASmall, x, rows, args.K, args.K, kTokSmallRows, error))
         return false;
     auto kernel = k_grouped_int4_gemm<MODE>;
-    // scale words one unit ahead where they fit, else the unit's own, else none (read step by step)
-    const auto smemOf = [&] { return gemm_smem_bytes(MODE, args.K, args.tileRows, args.packStages, args.scaleBuffers); };
-    args.scaleBuffers = 2;
-    args.packStages = 3;
-    while (args.scaleBuffers && smemOf() > 226 * 1024) --args.scaleBuffers;
-    while (args.packStages < (uint32_t)kMaxPackStages && smemOf() + kPackTileBytes <= 226 * 1024) ++args.packStages;
-    const size_t smem = smemOf();
+    const GemmRings rings = gemm_rings(MODE, args.K, args.tileRows);
+    args.packStages = rings.packStages;
+    args.scaleBuffers = rings.scaleBuffers;
+    const size_t smem = rings.smem;
     static KernelSmemMemo memo;
     if (!memo.prepare(kernel, ctx->device, smem, kGemmThreads, nullptr, error)) return false;
     // clusters of two CTAs; a cluster takes (row tile, pair of weight-row tiles) units
@@ -1454,6 +1469,16 @@ bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
 }
 
 }  // namespace ff
+
+// For the host-side tests, not part of the interface: packed-code stages, weight stages, scale buffers and shared memory
+// of the GEMM over K (mode 0 gate/up, 1 down) with tiles of `tileRows` rows.
+extern "C" void ff_prefill_gemm_rings(uint32_t mode, uint32_t K, uint32_t tileRows, uint32_t *sizes) {
+    const ff::GemmRings r = ff::gemm_rings((int)mode, K, tileRows);
+    sizes[0] = r.packStages;
+    sizes[1] = ff::weight_stages(tileRows);
+    sizes[2] = r.scaleBuffers;
+    sizes[3] = (uint32_t)r.smem;
+}
 
 extern "C" bool ff_last_prefill_routes(FFContext *ctx, FFTokenExpertPair *sortedPairs,
                                        uint32_t *offsets, const char **error) {

@@ -161,3 +161,33 @@ def test_int4_gemm_tile_rows(oracle, d, f, fs, rows):
         assert rel_l2 < 2.0 ** -9
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("d,f,fs", [(3712, 64, 64), (5120, 64, 64), (9856, 64, 0), (128, 2688, 64), (128, 4096, 4096), (64, 7808, 64)])
+@pytest.mark.parametrize("rows", [384, 385])
+def test_int4_gemm_ring_sizes(oracle, d, f, fs, rows):
+    """Contractions that give the GEMMs each number of code slots and scale buffers, with tiles of 128 rows (up to 384 rows of two
+    routes to eight experts) and of 192: the oracle's rows, and the same bits beside other traffic on the chip."""
+    L = workload.make_layer(0x79, 0, experts=8, d=d, f=f, sharedF=fs, topK=2)
+    hp, ctx = context(L, rows)
+    try:
+        x = workload.make_tokens(0x7A, f"rings{rows}", rows, d)
+        xd, src = hp.bf16_tensor(x, ctx.device), torch.ones(1 << 26, dtype=torch.uint8, device=ctx.device)
+        ids = torch.zeros((rows, 2), dtype=torch.int32, device=ctx.device)
+        other, dst, first = torch.cuda.Stream(), torch.empty_like(src), None
+        for i in range(6):
+            with torch.cuda.stream(other):
+                for _ in range(i % 3):
+                    dst.copy_(src)
+            y = ctx.moeLayer(0, xd, ids=ids)
+            torch.cuda.synchronize()
+            first = y.clone() if first is None else first
+            assert torch.equal(y, first)
+        assert ctx.info().deviceErrorFlag == 0
+        want, _, ref_ids, _ = oracle.moe_layer(oracle_layer(oracle, L), x, oracle.MODE_PARTIALS | oracle.MODE_BF16_WEIGHTS)
+        assert np.array_equal(ids.cpu().numpy().astype(np.uint32), ref_ids)
+        # the kernels and the oracle round the same sums to bf16: 2^-9 at most where they fall on other sides
+        rel_l2, _, _ = assert_layer_close(hp.bf16_numpy(y), want, oracle, f"rings {d}x{f}+{fs} rows={rows}")
+        assert rel_l2 < 2.0 ** -9
+    finally:
+        ctx.close()

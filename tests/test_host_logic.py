@@ -157,3 +157,70 @@ def test_product_code_never_touches_the_oracle():
                 text = open(os.path.join(dirpath, name)).read()
                 assert "liboracle" not in text and "from oracle" not in text and \
                     "import oracle" not in text and "ffo_" not in text, name
+
+
+# ---- rings of the prefill GEMM ------------------------------------------------------------------
+
+
+def _stale_read(packStages, weightStages, quads=40):
+    """A step model of the prefill GEMM's code ring: copies of a quad of steps into `packStages` slots, each slot's barrier
+    seen only by its parity; group g converts pairs g, g + 4, ... (two pairs a quad) and stores a pair behind the MMAs of the
+    pair that used the same tensor memory, weightStages / 2 back; MMAs in order.  Copies may land in any order: one at a
+    time is withheld while all else goes as far as it can.  Returns (quad, withheld) of a conversion that started before its
+    codes were there, or None."""
+    back, pairs = weightStages // 2, 2 * quads
+    for withheld in range(quads // 2):
+        for late in (True, False):  # then it lands, and all must finish
+            if late:
+                landed, taken, stored = set(), [0] * quads, set()
+                issued = mmas = 0
+                at = [[g, 0] for g in range(4)]  # next pair; 0 wait for codes, 1 wait for tensor memory
+            else:
+                landed.add(withheld)
+            moved = True
+            while moved:
+                moved = False
+                while issued < quads and (issued < packStages or taken[issued - packStages] == 2):
+                    if issued != withheld or not late:
+                        landed.add(issued)
+                    issued += 1
+                    moved = True
+                for g in range(4):
+                    while at[g][0] < pairs:
+                        p, q = at[g][0], at[g][0] // 2
+                        if at[g][1] == 0:
+                            phases = sum(1 for c in landed if c % packStages == q % packStages)  # completed
+                            if phases % 2 == (q // packStages) % 2:
+                                break
+                            if q not in landed:
+                                return q, withheld
+                            taken[q] += 1
+                            at[g][1] = 1
+                        elif p - back >= mmas:
+                            break
+                        else:
+                            stored.add(p)
+                            at[g] = [p + 4, 0]
+                        moved = True
+                while mmas in stored:
+                    mmas += 1
+                    moved = True
+        assert mmas == pairs, f"{packStages} slots, {weightStages} stages: no progress behind copy {withheld}"
+    return None
+
+
+@pytest.mark.parametrize("tileRows", [128, 192])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_prefill_gemm_rings_never_alias_a_phase(mode, tileRows):
+    """Every ring that the plan picks: a group that skips a slot's phases (odd rings: the other groups' quads) is ordered behind
+    them by something else."""
+    assert _stale_read(3, 8) is not None and _stale_read(1, 4) is not None  # the model sees it
+    assert all(_stale_read(p, w) is None for p, w in [(3, 4), (4, 8), (5, 8), (6, 8)])
+    lib, sizes, seen = binding.load(), (ctypes.c_uint32 * 4)(), {}
+    for K in range(64, 16385, 64):
+        lib.ff_prefill_gemm_rings(mode, K, tileRows, sizes)
+        packStages, weightStages, scaleBuffers, smem = sizes
+        assert 2 * tileRows + 32 * weightStages <= 512 and 3 <= packStages <= 6 and scaleBuffers <= 2 and smem <= 227 * 1024, K
+        seen.setdefault((packStages, weightStages), K)
+    for (packStages, weightStages), K in seen.items():
+        assert _stale_read(packStages, weightStages) is None, (K, packStages, weightStages)
