@@ -1274,17 +1274,18 @@ static GemmRings gemm_rings(int mode, uint32_t K, uint32_t tileRows) {
 // 1400 (87) 291 / 298, 1500 (94) 313 / 313, 2000 (125) 373 / 357, 4096 648 / 634.
 static uint32_t routed_tile_rows(uint32_t pairs, uint32_t experts) { return pairs <= 96u * experts ? kRowTileSmall : kRowTile; }
 
-// Of the shared FFN's two GEMMs: where whole waves of a step take less time (by their columns, 3 : 4).  us with 128 /
-// 192: 77 rows 23.7 / 25.8, 300 26.9 / 32.7, 613 35.2 / 39.3, 1000 42.8 / 46.3, 1500 50.6 / 55.3, 3000 97.9 / 89.9, 4096
-// 124.5 / 130.2.  (Up to 1000 rows, one or two waves, the smaller tile won whatever their number.)
-static uint32_t dense_tile_rows(const FFContext *ctx, uint32_t tokens) {
-    if (tokens <= 1024u) return kRowTileSmall;
-    const uint32_t d = ctx->cfg.d, f = ctx->cfg.sharedF, clusters = std::max(1u, (uint32_t)ctx->smCount / 2u);
-    const auto cost = [&](uint32_t rows) {
-        const uint64_t tiles = (tokens + rows - 1u) / rows;
-        const auto waves = [&](uint32_t nTiles) { return (tiles * ((nTiles + 1u) / 2u) + clusters - 1u) / clusters; };
-        return (waves((f + 63u) / 64u) * d + waves((d + 127u) / 128u) * f) * rows;
+// Of the shared FFN's two GEMMs: where whole waves of a step take less time (by their columns, 3 : 4), and tiles of 128
+// rows while those of gate/up are at most two: then a wave's fill and drain count for more than its columns.  us with 128 /
+// 192 (d x f): 2816 x 2112, 77 rows 23.7 / 25.8, 613 34.1 / 38.4, 1000 (two waves) 40.6 / 44.6, 1500 50.6 / 55.3, 3000 97.9 /
+// 89.9, 4096 124.5 / 130.2; 2816 x 6144, 300 rows 46.5 / 53.9, 1000 (six waves) 101.0 / 85.8; 5120 x 8192, 513 rows 140.1 / 109.6.
+static uint32_t dense_tile_rows(uint32_t smCount, uint32_t d, uint32_t f, uint32_t tokens) {
+    const uint32_t clusters = std::max(1u, smCount / 2u);
+    const auto waves = [&](uint32_t rows, uint32_t nTiles) {
+        return ((uint64_t)((tokens + rows - 1u) / rows) * ((nTiles + 1u) / 2u) + clusters - 1u) / clusters;
     };
+    const uint32_t gateUp = (f + 63u) / 64u, down = (d + 127u) / 128u;
+    const auto cost = [&](uint32_t rows) { return (waves(rows, gateUp) * d + waves(rows, down) * f) * rows; };
+    if (waves(kRowTileSmall, gateUp) <= 2u) return kRowTileSmall;
     return cost(kRowTileSmall) * 9u <= cost(kRowTile) * 8u ? kRowTileSmall : kRowTile;
 }
 
@@ -1427,7 +1428,7 @@ bool launch_prefill_shared(FFContext *ctx, LayerStore &L, const uint16_t *x, uin
     // dense problem: its row tiles live behind the routed ones in the units buffer
     RowTile *tiles = reinterpret_cast<RowTile *>(ctx->units) + ctx->maxUnits / 2;
     uint32_t *counts = ctx->unitCount + 4;
-    const uint32_t tileRows = dense_tile_rows(ctx, tokens);
+    const uint32_t tileRows = dense_tile_rows((uint32_t)ctx->smCount, c.d, c.sharedF, tokens);
     {
         LaunchScope scope(ctx, stream, "dense_tiles");
         FF_CUDA_OK(launch_pdl(k_dense_tiles, 1, 256, 0, stream,
@@ -1478,6 +1479,10 @@ extern "C" void ff_prefill_gemm_rings(uint32_t mode, uint32_t K, uint32_t tileRo
     sizes[1] = ff::weight_stages(tileRows);
     sizes[2] = r.scaleBuffers;
     sizes[3] = (uint32_t)r.smem;
+}
+// ... and the rows of the shared FFN's tiles.
+extern "C" uint32_t ff_prefill_dense_tile_rows(uint32_t smCount, uint32_t d, uint32_t f, uint32_t tokens) {
+    return ff::dense_tile_rows(smCount, d, f, tokens);
 }
 
 extern "C" bool ff_last_prefill_routes(FFContext *ctx, FFTokenExpertPair *sortedPairs,
