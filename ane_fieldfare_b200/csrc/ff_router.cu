@@ -1,5 +1,5 @@
-// Router of a prefill chunk (more rows than a decode/verify block) when only the routes are asked for: up to kTileMaxRows
-// rows every logit in one launch (k_router_tile), more rows as follows.
+// Router of a prefill chunk (more rows than a decode/verify block) when only the routes are asked for: few pairs of row and
+// expert have every logit formed in one launch (k_router_tile), more as follows.
 //
 // The contract is bitwise: logits are sums in a fixed fp32 order (bf16 router: lane l chains fmaf over
 // [256 i + 8 l, +8); INT8 router: over elements 64 g + 2 l, + 1; xor butterfly; then the logit bias),
@@ -544,12 +544,11 @@ k_router_logits_int8(const uint4 *Q, const uint32_t *aux, const uint16_t *effSca
 
 // CTA (expert tile, token tile): a warp per expert, its row in registers (requested in front of the wait for the launch
 // before), kTileTokens rows in shared memory: bf16, or (WIDE) fp32 times the per-input scale.  The last CTA of a token
-// tile ranks its rows, a warp each.  A pair of expert and row is about 280 warp instructions, which bounds it; the
-// approximate logits and the selection behind them are two launches and cost less for more rows.  us in a graph for 128
-// experts and 2816 inputs, this / those: 17 rows 9.3 / 13.9, 77 11.3 / 16.4, 128 11.7 / 18.0, 160 15.1 / 18.0, 256 18.0 /
-// 18.0, 320 22.4 / 18.5; INT8 11.8 / 17.5, 14.9 / 21.0, 15.4 / 22.6, 21.9 / 23.1, 26.1 / 23.6.
+// tile ranks its rows, a warp each.  A pair of expert and row is about 280 warp instructions at 2816 inputs, which bounds
+// it; the approximate logits and the selection behind them are two launches and cost less for more pairs: see
+// router_tile_pays.
 constexpr int kTileTokens = 8, kTileExperts = 8, kTileChunks = 11;
-constexpr uint32_t kTileMaxRows = 160;
+constexpr uint32_t kTileMaxRows = 160;  // (measured up to here)
 static_assert((kTileMaxRows + kTileTokens - 1) / kTileTokens <= (uint32_t)kRouterCounts, "a counter for every tile of rows");
 struct TileArgs {
     const uint16_t *W;           // bf16 router [E][D], or
@@ -846,10 +845,31 @@ static bool launch_router_tile(FFContext *ctx, const LayerStore &L, const uint16
     return true;
 }
 
+// Whether k_router_tile takes less time than the two launches: these hardly grow with the rows, it by its CTAs an SM and
+// their inputs.  us in a graph on 148 SMs, this / those:
+//   bf16, 2816 inputs, CTAs an SM 1 (17 rows, 128 experts) 9.3 / 13.9, 2 (77 rows) 11.3 / 16.4, 3 (160 rows) 15.1 / 18.0, 4
+//     (128 rows, 256 experts) 19.0 / 20.3, 5 (160 rows) 24.5 / 20.4; 4096 inputs 3 18.3 / 18.9, 4 23.4 / 21.5; 6144 inputs 2 17.4 /
+//     19.9, 3 24.8 / 22.1;
+//   INT8, 2816 inputs, 2 15.1 / 22.6, 3 21.5 / 23.2, 4 26.8 / 25.0; one CTA's fp32 rows an SM, so that the second runs behind the
+//     first: 4096 inputs 1 14.1 / 21.7, 2 24.7 / 25.6 (codes from memory 38.9 / 35.8);
+//   bf16 with a per-input scale, whose rows are widened for every expert tile: 1024 inputs 2 11.0 / 14.6, 3 16.8 / 14.8; 2816
+//     inputs 1 13.7 / 16.4 (fewer than 64 experts, where the two launches are shorter, 12.4 / 11.9), 2 20.3 / 19.3, 3 35.5 / 19.5;
+//     4096 inputs 1 17.6 / 17.1.
+static bool router_tile_pays(const FFContext *ctx, const LayerStore &L, uint32_t tokens) {
+    const uint32_t D = ctx->cfg.d, E = L.routerExperts, sms = (uint32_t)ctx->smCount;
+    const size_t smem = (size_t)kTileTokens * D * (L.routerQ || L.routerScale ? 4 : 2), smBytes = 220 * 1024;
+    if (tokens > kTileMaxRows || smem > 200 * 1024) return false;
+    const uint32_t ctas = (E + kTileExperts - 1) / kTileExperts * ((tokens + kTileTokens - 1) / kTileTokens);
+    const uint32_t perSm = (ctas + sms - 1) / sms;
+    if (L.routerQ) return perSm * D <= 9216u && (perSm == 1u || 2 * smem <= smBytes);
+    if (L.routerScale) return perSm * D <= (E < 64u ? 2048u : 3000u);
+    return perSm * D <= 12288u;
+}
+
 bool launch_router_select(FFContext *ctx, const LayerStore &L, const uint16_t *x, uint32_t xStride, uint32_t tokens,
                           uint32_t *ids, uint16_t *weights, cudaStream_t stream, const char **error) {
     const uint32_t E = L.routerExperts, D = ctx->cfg.d, K = ctx->cfg.topK;
-    if (tokens <= kTileMaxRows && (size_t)kTileTokens * D * (L.routerQ || L.routerScale ? 4 : 2) <= 200 * 1024)
+    if (router_tile_pays(ctx, L, tokens))
         return launch_router_tile(ctx, L, x, xStride, tokens, ids, weights, stream, error);
     // Token tile: as large as the rows allow (the router's 720 KB are read once per tile and split);
     // the contraction is split while tiles x splits stay within one CTA per SM.

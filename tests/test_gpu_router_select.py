@@ -128,10 +128,11 @@ def test_selected_routes_at_every_number_of_warps(form, rows):
 
 
 @pytest.mark.parametrize("form", ["bf16", "bf16_scaled", "int8"])
-@pytest.mark.parametrize("experts,d,rows", [(9, 64, 17), (12, 4160, 24), (130, 3072, 25), (128, 6400, 160), (128, 6464, 160), (128, 2816, 161)])
+@pytest.mark.parametrize("experts,d,rows", [(9, 64, 17), (12, 4160, 24), (130, 3072, 25), (128, 6400, 160), (128, 6464, 160), (128, 2816, 161),
+                                               (16, 6400, 160), (16, 6464, 160), (16, 12288, 40)])
 def test_routes_of_a_short_chunk(form, experts, d, rows):
     """Edges of the one-launch kernel: tiles of eight rows and experts, contractions of more than one set of a warp's registers,
-    and where the rows (160) or their width (fp32 rows of 6400) go over to the two launches.  Against blocks of 16 rows, twice
+    and where the rows (160), their width (fp32 rows of 6400) or the pairs of row and expert go over to the two launches.  Against blocks of 16 rows, twice
     in a row (its counters)."""
     from ane_fieldfare_b200 import hotpath as hp
     k = 5
@@ -155,6 +156,35 @@ def test_routes_of_a_short_chunk(form, experts, d, rows):
         for i in (1, 2):
             assert torch.equal(got[0], got[i])
             assert torch.equal(weights[0].view(torch.int16), weights[i].view(torch.int16))
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("form,experts,d,rows,one", [
+    ("bf16", 128, 2816, 160, True), ("bf16", 256, 2816, 100, True), ("bf16", 256, 2816, 160, False), ("bf16", 256, 4096, 128, False),
+    ("bf16", 128, 6144, 160, False), ("bf16", 256, 1024, 160, True), ("bf16_scaled", 128, 2816, 64, True),
+    ("bf16_scaled", 128, 2816, 77, False), ("bf16_scaled", 128, 2816, 160, False), ("bf16_scaled", 128, 4096, 40, False),
+    ("bf16_scaled", 128, 1024, 128, True), ("bf16_scaled", 16, 2816, 17, False), ("int8", 128, 2816, 77, True),
+    ("int8", 128, 2816, 160, True), ("int8", 256, 2816, 160, False), ("int8", 128, 4096, 64, True), ("int8", 128, 4096, 128, False),
+    ("int8", 128, 6144, 160, False)])
+def test_short_chunks_take_the_shorter_way(form, experts, d, rows, one):
+    """One launch or two, on 148 SMs, where the other was measurably slower (or no faster with weights from memory)."""
+    from ane_fieldfare_b200 import hotpath as hp
+    ctx = hp.HotpathContext(layers=1, experts=experts, d=d, f=64, sharedF=0, topK=8, maxTokens=rows)
+    try:
+        if ctx.info().smCount != 148:
+            pytest.skip("measured on 148 SMs")
+        eff = None if form == "bf16" else synth.bf16_bits(synth.uniform(7, d, 0.5, 1.5))
+        if form == "int8":
+            ctx.loadRouterInt8(0, *int8_router(0x3D, experts, d), effectiveScale=eff)
+        else:
+            ctx.loadRouter(0, synth.normal_bf16(0x3E, "way.router", (experts, d), 0.02), effectiveScale=eff)
+        x = hp.bf16_tensor(workload.make_tokens(0x3F, f"way{rows}", rows, d), ctx.device)
+        ids = torch.zeros((rows, 8), dtype=torch.int32, device=ctx.device)
+        weights = torch.zeros((rows, 8), dtype=torch.bfloat16, device=ctx.device)
+        ctx.setTracing(True)
+        hp.PrefillRouter(ctx).encodeGemma4Block(None, 0, x, ids, weights, rows)
+        assert set(ctx.trace()) == ({"router_tile"} if one else {"router_approx", "router_select"})
     finally:
         ctx.close()
 
