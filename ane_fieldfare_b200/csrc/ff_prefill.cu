@@ -468,9 +468,9 @@ k_route_scatter(const uint32_t *ids, int T, int K, int E,
 // share, a warp its part of that with the routes and their matches in registers, the CTAs read one another's counts
 // from shared memory, plan alike, and place.  Bound by its latencies, then by eight SMs' matches and scattered stores.
 // us in a graph, Zipf routes, 128 experts, one launch / three: 77 rows 3.7 / -, 257 4.3 / 15.1, 613 5.1 / 15.3, 1500
-// 7.9 / 15.5, 4096 15.4 / 16.9, 6000 21.2 / 17.4 (hence the limit).  (CTAs of 1024 threads, or sixteen of them, are
-// faster by themselves, 10.9 us at 4096 rows, but wait longer for SMs beside the shared FFN: a layer of 300 rows 308 us
-// for 298.)
+// 7.9 / 15.5, 4096 15.4 / 16.9, 6000 21.2 / 17.4 (for fewer routes a row see sort_in_one_launch).  (CTAs of 1024 threads, or
+// sixteen of them, are faster by themselves, 10.9 us at 4096 rows, but wait longer for SMs beside the shared FFN: a layer of
+// 300 rows 308 us for 298.)
 constexpr int kSortCtas = 8, kSortThreads = 512, kSortRounds = 8;  // rounds of 32 routes of a warp
 constexpr int kClusterRoutes = kSortCtas * kSortThreads * kSortRounds;
 __global__ void __cluster_dims__(kSortCtas, 1, 1) __launch_bounds__(kSortThreads, 1)
@@ -1322,6 +1322,14 @@ static bool check_gemm_shapes(const FFConfig &c, uint32_t f, const char **error)
     return true;
 }
 
+// Whether k_route_sort takes less time than the three launches: it grows with the routes (3.1 us and 0.4 for every 1024),
+// they with the routes of a block of 256 rows.  us in a graph, 128 experts, one launch / three: one route a row 8192 routes 6.5 /
+// 7.3, 16384 9.6 / 8.8, 32768 16.0 / 12.2; two a row 8192 6.4 / 8.4, 16384 9.6 / 9.0, 32768 16.1 / 10.9; four a row 16384 9.6 /
+// 11.2, 24576 12.9 / 11.7; eight a row 32768 16.3 / 18.0.
+static bool sort_in_one_launch(uint32_t tokens, uint32_t topK) {
+    return tokens * topK <= 8192u + 3072u * topK && (tokens + kSortCtas - 1) / kSortCtas * topK <= (uint32_t)(kClusterRoutes / kSortCtas);
+}
+
 // Sorts the routes (stable, by expert) and plans the row tiles.
 static bool sort_routes(FFContext *ctx, const uint32_t *ids, uint32_t tokens, int E, uint32_t tileRows, uint32_t *offsets, RowTile *tiles,
                               FFTokenExpertPair *sorted, uint32_t *rowOfRoute, cudaStream_t stream, const char **error) {
@@ -1329,7 +1337,7 @@ static bool sort_routes(FFContext *ctx, const uint32_t *ids, uint32_t tokens, in
     const uint32_t blocks = (tokens + kSortTokens - 1) / kSortTokens;
     const size_t sortSmem = (size_t)kSortTokens * K * sizeof(uint32_t);
     const uint32_t maxTiles = ctx->maxUnits / 2;  // first half of the tile buffer
-    if ((T + kSortCtas - 1) / kSortCtas * K <= kClusterRoutes / kSortCtas) {
+    if (sort_in_one_launch(tokens, ctx->cfg.topK)) {
         LaunchScope scope(ctx, stream, "route_sort");
         FF_CUDA_OK(launch_pdl(k_route_sort, kSortCtas, kSortThreads, 0, stream, ids, T, K, E, tileRows, offsets, tiles, maxTiles, ctx->unitCount, sorted,
                               rowOfRoute),
