@@ -89,12 +89,17 @@ __global__ void __launch_bounds__(kGemvThreads) k_int4_gemv(const __grid_constan
 // compared for equality with the CPU oracle): lane l chains fmaf over elements
 // [256 i + 8 l, +8) for i = 0, 1, ... in increasing index, the lane sums are added by an xor
 // butterfly (16, 8, 4, 2, 1), then the per-expert logit bias is added.
-// The expert's row (and per-input scale) of the first kRowChunks * 256 inputs is requested in front of the wait for the
-// launch before, the token's row all together behind it.
-constexpr int kRowChunks = 11;
+// The expert's row of the first kRowChunks * 256 inputs, and the per-input scale (by way of shared memory: the CTA's eight
+// warps need the same), are requested in front of the wait for the launch before, the token's row all together behind it.
+// Bound by its latencies.  us in a graph, 128 experts, in loads of a few chunks / eleven chunks with the scale fetched where
+// it is used / now: 2816 inputs, one row 5.3 / 5.5 / 5.0, 16 rows 6.6 / 6.8 / 6.3; scaled 6.3 / 6.8 / 5.2, 7.5 / 7.9 / 6.7; 4096
+// inputs, scaled, one row 7.4 / 8.2 / 5.7.  Eleven chunks, all of 2816 inputs, are no faster there than twelve and take a second
+// turn for 2880 to 3072 (scaled, 16 rows 7.3 / 6.9).
+template <int kRowChunks>
 __global__ void __launch_bounds__(256)
 k_router_logits(const uint16_t *W, const uint16_t *scale, const float *bias, const uint16_t *x,
                 uint32_t xStride, int E, int D, float *logits, RouterTail tail) {
+    __shared__ __align__(16) uint4 sScale[kRowChunks * 32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e = min((int)blockIdx.x * 8 + warp, E - 1);  // (a warp past the experts repeats the last)
     const int t = blockIdx.y;
@@ -107,24 +112,31 @@ k_router_logits(const uint16_t *W, const uint16_t *scale, const float *bias, con
             const int base = first + 256 * i + 8 * lane;
             if (base < D) wv[i] = __ldg(reinterpret_cast<const uint4 *>(wr + base));
         }
+        if (scale)
+            for (int i = threadIdx.x; i < kRowChunks * 32 && first + 8 * i < D; i += 256)
+                sScale[i] = __ldg(reinterpret_cast<const uint4 *>(scale + first) + i);
     };
     fetch(0);
     pdl_enter();
     float acc = 0.0f;
     for (int first = 0; first < D; first += 256 * kRowChunks) {
-        if (first) fetch(first);
+        if (first) {
+            if (scale) __syncthreads();  // every warp is done with the scales before
+            fetch(first);
+        }
         uint4 xv[kRowChunks];
 #pragma unroll
         for (int i = 0; i < kRowChunks; ++i) {
             const int base = first + 256 * i + 8 * lane;
             if (base < D) xv[i] = *reinterpret_cast<const uint4 *>(xr + base);
         }
+        if (scale) __syncthreads();
 #pragma unroll
         for (int i = 0; i < kRowChunks; ++i) {
             const int base = first + 256 * i + 8 * lane;
             if (base >= D) break;
             uint4 sv = make_uint4(0, 0, 0, 0);
-            if (scale) sv = __ldg(reinterpret_cast<const uint4 *>(scale + base));
+            if (scale) sv = sScale[32 * i + lane];
             const uint32_t ww[4] = {wv[i].x, wv[i].y, wv[i].z, wv[i].w};
             const uint32_t xx[4] = {xv[i].x, xv[i].y, xv[i].z, xv[i].w};
             const uint32_t ss[4] = {sv.x, sv.y, sv.z, sv.w};
@@ -737,9 +749,10 @@ bool launch_router_topk(FFContext *ctx, const LayerStore &L, const uint16_t *x, 
     if (L.routerQ) return launch_router_logits_int8(ctx, L, x, xStride, tokens, lg, tail, stream, error);
     {
         LaunchScope scope(ctx, stream, "router_logits");
-        FF_CUDA_OK(launch_pdl(k_router_logits, dim3((E + 7) / 8, tokens), 256, 0, stream, L.routerW, L.routerScale, L.logitBias, x, xStride,
-                              E, D, lg, tail),
-                   error);
+        // twelve chunks in flight (two CTAs an SM) while the CTAs are at most one wave; more CTAs: four, and four an SM
+        const dim3 grid((E + 7) / 8, tokens);
+        auto kernel = grid.x * grid.y <= 2u * (uint32_t)ctx->smCount ? k_router_logits<12> : k_router_logits<4>;
+        FF_CUDA_OK(launch_pdl(kernel, grid, 256, 0, stream, L.routerW, L.routerScale, L.logitBias, x, xStride, E, D, lg, tail), error);
     }
     return true;
 }
