@@ -78,9 +78,10 @@ __device__ __forceinline__ bool rt_wait(uint32_t bar, uint32_t parity) {
     return mbar_try_wait(bar, parity) || rt_wait_slow(bar, parity);
 }
 
-// (a multiple of 16, so that the next warp's rows are aligned with an odd number of experts, too)
+// A multiple of 16, so that the next warp's rows are aligned: the logits of an even number of rows take an even number of
+// experts' room.  (The sum rounded up instead: 17 rows of 2816 inputs and 128 experts 143.5 us, so 140.0.)
 __host__ __device__ inline size_t router_warp_bytes(int tokens, int D, int E) {
-    return ((size_t)tokens * D * 2 + (size_t)tokens * E * 4 + 15) & ~(size_t)15;
+    return (size_t)tokens * D * 2 + (size_t)tokens * (E + (E & 1)) * 4;
 }
 
 template <int kTok>
@@ -89,6 +90,7 @@ k_router_rows(const __grid_constant__ CUtensorMap mapW, const uint16_t *scale, c
               const uint16_t *gain, const uint16_t *x, uint32_t xStride, int T, int E, int D, int K,
               uint32_t *ids, uint16_t *weights, float *logitsOut, uint32_t *errorFlag) {
     constexpr int kRouterWarps = kRouterTokensPerCta / kTok;
+    static_assert(kTok % 2 == 0, "see router_warp_bytes");
     extern __shared__ __align__(128) uint8_t rsmRaw[];
     __shared__ __align__(8) uint64_t ringBar[2 * kRouterRing];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
