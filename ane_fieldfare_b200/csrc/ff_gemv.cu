@@ -191,8 +191,10 @@ k_reduce_token_major(const uint16_t *partials, const uint32_t *rowIndex, const u
 // above: rank ascending, then the residual); for rows that are 16-byte aligned.  B = 8: the loads
 // of eight ranks are issued together, for blocks of at most a wave, where their latencies one after another
 // are the time (77 rows 4.4 -> 3.5 us); B = 1 beyond, where more warps in flight beat more loads of each (32768
-// rows 363 us, with B = 8 450 us).  The partial rows are streamed: a layer of 4096 rows 614 -> 607 us, of 3000 485 -> 479.
-template <int B>
+// rows 363 us, with B = 8 450 us).  STREAM: the partial rows are streamed, which pays from four of them a row on: eight a row,
+// written and reduced, 1500 rows of 2816 36.2 -> 33.7 us, 4096 102.0 -> 91.0 (a layer of 4096 rows 614 -> 607); four, 4096 rows
+// 54.9 -> 48.8; three 39.5 -> 41.5, two 26.9 -> 28.6.
+template <int B, bool STREAM>
 __global__ void __launch_bounds__(256)
 k_reduce_token_major_x8(const uint16_t *partials, const uint32_t *rowIndex, const uint16_t *weights,
                         const uint16_t *residual, uint16_t *y, int T, int K, int D) {
@@ -214,7 +216,8 @@ k_reduce_token_major_x8(const uint16_t *partials, const uint32_t *rowIndex, cons
             if (r0 + r < K) {
                 const size_t route = (size_t)t * K + r0 + r, row = rowIndex ? (size_t)rowIndex[route] : route;
                 w[r] = bf2f(weights[route]);
-                v[r] = __ldcs(reinterpret_cast<const uint4 *>(partials + row * D + d));  // read once
+                const uint4 *src = reinterpret_cast<const uint4 *>(partials + row * D + d);
+                v[r] = STREAM ? __ldcs(src) : *src;  // read once
             }
         }
 #pragma unroll
@@ -793,7 +796,9 @@ bool launch_reduce(FFContext *ctx, const uint16_t *partials, const uint16_t *wei
         if (wide) {
             const size_t items = (size_t)tokens * (D / 8);
             const unsigned blocks = (unsigned)((items + 255) / 256);
-            auto kernel = blocks <= (unsigned)ctx->smCount * 4 ? k_reduce_token_major_x8<8> : k_reduce_token_major_x8<1>;
+            auto kernel = blocks <= (unsigned)ctx->smCount * 4 ? k_reduce_token_major_x8<8, true>
+                          : ctx->cfg.topK > 3                  ? k_reduce_token_major_x8<1, true>
+                                                               : k_reduce_token_major_x8<1, false>;
             FF_CUDA_OK(launch_pdl(kernel, blocks, 256, 0, stream,
                               partials, rowIndex, weights, residual, y, (int)tokens, (int)ctx->cfg.topK, D),
                    error);

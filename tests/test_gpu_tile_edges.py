@@ -191,3 +191,24 @@ def test_int4_gemm_ring_sizes(oracle, d, f, fs, rows):
         assert rel_l2 < 2.0 ** -9
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("top", [1, 2, 3, 8])
+@pytest.mark.parametrize("rows", [70, 2368, 2369])
+def test_reduce_at_every_form(oracle, top, rows):
+    """Up to four CTAs an SM (2368 rows of 512 on 148) and beyond, with the partial rows streamed and not: the oracle's bits."""
+    from ane_fieldfare_b200 import hotpath as hp
+    d = 512
+    ctx = hp.HotpathContext(layers=1, experts=8, d=d, f=64, sharedF=0, topK=top, maxTokens=rows)
+    try:
+        p = synth.bf16_bits(synth.uniform(1, rows * top * d, -2, 2)).reshape(rows * top, d)
+        w = synth.bf16_bits(synth.uniform(2, rows * top, 0, 1)).reshape(rows, top)
+        r = synth.bf16_bits(synth.uniform(3, rows * d, -1, 1)).reshape(rows, d)
+        for residual in (None, r):
+            y = torch.zeros((rows, d), dtype=torch.bfloat16, device=ctx.device)
+            hp.PrefillMoE(ctx).encodeReduceTokenMajor(None, hp.bf16_tensor(p, ctx.device), hp.bf16_tensor(w, ctx.device), y, rows,
+                                                      residual=None if residual is None else hp.bf16_tensor(residual, ctx.device))
+            torch.cuda.synchronize()
+            assert np.array_equal(hp.bf16_numpy(y), oracle.reduce_token_major(p, w, residual, rows, top, d))
+    finally:
+        ctx.close()
