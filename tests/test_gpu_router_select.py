@@ -1,7 +1,8 @@
-"""A prefill chunk's routes (approximate logits on the tensor cores, exact logits of the experts that
-can matter) against the kernels that form every logit in the defined order (the same call with the
-logits asked for, which other tests pin against the oracle): ids and weights bit for bit, at the edges
-of the token tiles, with tied experts, all-zero, non-finite and huge rows and a bias of -inf."""
+"""A prefill chunk's routes against the kernels that form every logit in the defined order (the same call with the
+logits asked for, or blocks of 16 rows, which other tests pin against the oracle): ids and weights bit for bit, with
+tied experts, all-zero, non-finite and huge rows and a bias of -inf.  A short chunk has every logit formed in one launch;
+the rest goes through approximate logits on the tensor cores and exact ones of the experts that can matter, at the
+edges of its token tiles (32, 64, 96 and 128 rows) and with every number of warps a row."""
 import numpy as np
 import pytest
 
@@ -12,38 +13,48 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
+def load_router(ctx, form, experts, d):
+    """A router with tied experts (8 to 11) and one of bias -inf."""
+    bias = synth.normal(3, experts).astype(np.float32)
+    bias[1] = -np.inf
+    bias[8:12] = bias[8]  # (with equal weights below: exact ties)
+    eff = gain = None
+    if form != "bf16":
+        eff = synth.bf16_bits(synth.uniform(7, d, 0.5, 1.5))
+        gain = synth.bf16_bits(synth.uniform(8, experts, 0.5, 1.5))
+    if form == "int8":
+        codes, scales, biases = int8_router(0x31, experts, d)
+        for m in (codes, scales, biases):
+            m[8:12] = m[8]
+        ctx.loadRouterInt8(0, codes, scales, biases, effectiveScale=eff, perExpertScale=gain, logitBias=bias)
+    else:
+        w = synth.normal_bf16(0x32, "select.router", (experts, d), 0.02)
+        w[8:12] = w[8]
+        ctx.loadRouter(0, w, effectiveScale=eff, perExpertScale=gain, logitBias=bias)
+
+
+def special_rows(hp, ctx, rows, d):
+    """Rows d + 8 apart, zero, non-finite, huge and tiny ones among them."""
+    wide = torch.zeros((rows, d + 8), dtype=torch.bfloat16, device=ctx.device)
+    wide[:, :d] = hp.bf16_tensor(workload.make_tokens(0x33, f"select{rows}", rows, d), ctx.device)
+    wide[1, :d] = 0
+    wide[2, 5] = float("nan")
+    wide[3, 6] = float("inf")
+    wide[4, :d] *= 1e30
+    wide[5, :d] *= 1e-30
+    wide[6, 7] = 3e4
+    return wide
+
+
 @pytest.mark.parametrize("form", ["bf16", "bf16_scaled", "int8"])
 @pytest.mark.parametrize("experts,d,k", [(16, 128, 8), (128, 2816, 8), (256, 448, 3), (130, 2496, 8)])
-@pytest.mark.parametrize("rows", [17, 32, 129, 700])
+@pytest.mark.parametrize("rows", [17, 32, 129, 161, 300, 700])
 def test_selected_routes_equal_the_exact_ones(form, experts, d, k, rows):
     from ane_fieldfare_b200 import hotpath as hp
     ctx = hp.HotpathContext(layers=1, experts=experts, d=d, f=64, sharedF=0, topK=k, maxTokens=700)
     try:
-        bias = synth.normal(3, experts).astype(np.float32)
-        bias[1] = -np.inf
-        bias[8:12] = bias[8]  # (with equal weights below: exact ties)
-        eff = gain = None
-        if form != "bf16":
-            eff = synth.bf16_bits(synth.uniform(7, d, 0.5, 1.5))
-            gain = synth.bf16_bits(synth.uniform(8, experts, 0.5, 1.5))
-        if form == "int8":
-            codes, scales, biases = int8_router(0x31, experts, d)
-            for m in (codes, scales, biases):
-                m[8:12] = m[8]
-            ctx.loadRouterInt8(0, codes, scales, biases, effectiveScale=eff, perExpertScale=gain, logitBias=bias)
-        else:
-            w = synth.normal_bf16(0x32, "select.router", (experts, d), 0.02)
-            w[8:12] = w[8]
-            ctx.loadRouter(0, w, effectiveScale=eff, perExpertScale=gain, logitBias=bias)
-        x = hp.bf16_tensor(workload.make_tokens(0x33, f"select{rows}", rows, d), ctx.device)
-        wide = torch.zeros((rows, d + 8), dtype=torch.bfloat16, device=ctx.device)
-        wide[:, :d] = x
-        wide[1, :d] = 0
-        wide[2, 5] = float("nan")
-        wide[3, 6] = float("inf")
-        wide[4, :d] *= 1e30
-        wide[5, :d] *= 1e-30
-        wide[6, 7] = 3e4
+        load_router(ctx, form, experts, d)
+        wide = special_rows(hp, ctx, rows, d)
         got = [torch.full((rows, k), -1, dtype=torch.int32, device=ctx.device) for _ in range(2)]
         weights = [torch.zeros((rows, k), dtype=torch.bfloat16, device=ctx.device) for _ in range(2)]
         logits = torch.zeros((rows, experts), dtype=torch.float32, device=ctx.device)
@@ -185,6 +196,34 @@ def test_short_chunks_take_the_shorter_way(form, experts, d, rows, one):
         ctx.setTracing(True)
         hp.PrefillRouter(ctx).encodeGemma4Block(None, 0, x, ids, weights, rows)
         assert set(ctx.trace()) == ({"router_tile"} if one else {"router_approx", "router_select"})
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("form,experts,d,rows", [
+    *[("bf16_scaled", 128, 4096, r) for r in (17, 33, 65, 97)], *[("int8", 256, 6464, r) for r in (17, 33, 65, 97)],
+    *[("bf16", 256, 6464, r) for r in (33, 65, 97)]])
+def test_selected_routes_of_small_token_tiles(form, experts, d, rows):
+    """The two launches with token tiles of 32, 64, 96 and 128 rows."""
+    from ane_fieldfare_b200 import hotpath as hp
+    k = 8
+    ctx = hp.HotpathContext(layers=1, experts=experts, d=d, f=64, sharedF=0, topK=k, maxTokens=rows)
+    try:
+        load_router(ctx, form, experts, d)
+        x = special_rows(hp, ctx, rows, d)
+        got = [torch.full((rows, k), -1, dtype=torch.int32, device=ctx.device) for _ in range(2)]
+        weights = [torch.zeros((rows, k), dtype=torch.bfloat16, device=ctx.device) for _ in range(2)]
+        router = hp.PrefillRouter(ctx)
+        for r in range(0, rows, 16):
+            router.encodeGemma4Block(None, 0, x[r:], got[0][r:], weights[0][r:], min(16, rows - r), d + 8)
+        ctx.setTracing(True)
+        router.encodeGemma4Block(None, 0, x, got[1], weights[1], rows, d + 8)
+        if ctx.info().smCount == 148:
+            assert set(ctx.trace()) == {"router_approx", "router_select"}
+        torch.cuda.synchronize()
+        assert ctx.info().deviceErrorFlag == 0
+        assert torch.equal(got[0], got[1])
+        assert torch.equal(weights[0].view(torch.int16), weights[1].view(torch.int16))
     finally:
         ctx.close()
 
