@@ -182,8 +182,9 @@ FFContext *ff_create(int32_t deviceOrdinal, const FFConfig *config, const char *
     if (ok && T > (size_t)kMaxGemvRows) {
         const size_t pairs = T * K;
         const size_t permuteBlocks = (T + 255) / 256;
-        // row tiles hold up to 192 rows of one expert (at most pairs / 192 + experts of them; room for pairs / 128)
-        ctx->maxUnits = (uint32_t)(2 * (pairs / 128 + c.experts + 2));  // row tiles: routed half, dense half
+        // row tiles, a half for the routed and one for the dense ones: at most rows / tile rows and one more an expert, all
+        // of which tiles of kRowTileSmall rows need (k_route_sort and k_route_scan leave out what does not fit)
+        ctx->maxUnits = (uint32_t)(2 * (pairs / kRowTileSmall + c.experts + 2));
         ok = ok && dev_alloc(ctx, &ctx->xSorted, (pairs + 256) * c.d, error);
         if (ok) ok = cudaMemset(ctx->xSorted, 0, (pairs + 256) * c.d * 2) == cudaSuccess;
         if (c.sharedF) {
@@ -448,7 +449,7 @@ bool ff_load_shared_int8(FFContext *ctx, uint32_t layer, const FFProjection *gat
         L.shared = nullptr;
         L.mapsReady = false;
         L.decodeMapsReady = false;
-    L.blockMapsReady = 0;
+        L.blockMapsReady = 0;
     }
     free_shared8(L);
     for (int m = 0; m < 3; ++m) {

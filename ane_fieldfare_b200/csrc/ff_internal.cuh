@@ -16,6 +16,8 @@ namespace ff {
 constexpr int kGroup = 64;        // codes per scale/bias pair
 constexpr int kMaxGemvRows = 16;  // input rows one GEMV job can carry (a verify block)
 constexpr int kRouterCounts = 64;
+// rows of one expert per unit of the prefill GEMM (accumulator columns): see routed_tile_rows and dense_tile_rows
+constexpr uint32_t kRowTile = 192, kRowTileSmall = 128;
 constexpr int kDecodeMaps = 6;
 constexpr int kMaxExperts = 256;  // router width limit, as in the reference's prefill router
 

@@ -278,9 +278,6 @@ bool launch_router_prefill(FFContext *ctx, const LayerStore &L, const uint16_t *
 
 constexpr int kSortTokens = 256;  // tokens per permute block
 
-// rows of one expert per GEMM unit (accumulator columns): see routed_tile_rows and dense_tile_rows
-constexpr uint32_t kRowTile = 192, kRowTileSmall = 128;
-
 struct RowTile {
     uint32_t rowStart;  // first row in expert-sorted order
     uint32_t rows;      // 1..kRowTile
@@ -806,9 +803,9 @@ k_grouped_int4_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_con
 
     if (warp == 0) {
         // ---------------- token copies ----------------
-        // A step is one copy, of 32 rows where the tile's half needs no more and of 96 otherwise.  (16 rows
-        // at a time, as many as needed, were slower than 96 always: 353 us against 339 with 77 tokens.
-        // It is the copies, not their bytes, that cost.)
+        // A pair of steps is two copies, of 32 rows where the tile's half needs no more and of the whole half (64 or
+        // 96) otherwise.  (16 rows at a time, as many as needed, were slower than 96 always: 353 us against 339 with 77
+        // tokens.  It is the copies, not their bytes, that cost.)
         if (firstUnit < units) {
             uint32_t ts = 0, phase = 0;
             bool ok = true;
