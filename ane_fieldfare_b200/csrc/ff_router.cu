@@ -939,14 +939,16 @@ bool launch_router_logits_int8(FFContext *ctx, const LayerStore &L, const uint16
     const uint4 *lanes = reinterpret_cast<const uint4 *>(L.routerLanes);
     {
         LaunchScope scope(ctx, stream, "router_logits_int8");
-        // (a block: a warp per expert and row, for the latency; more rows: two rows and few registers a warp)
-        if (tokens <= (uint32_t)kMaxGemvRows)
-            FF_CUDA_OK(launch_pdl(k_router_logits_int8<1, 6>, dim3((E + 3) / 4, tokens), 128, 0, stream,
-                              lanes, L.routerAux, L.routerScale, L.logitBias, x, xStride, (int)tokens, E, D, logits, tail),
-                   error);
-        else
-            FF_CUDA_OK(launch_pdl(k_router_logits_int8<2, 2>, dim3((E + 3) / 4, (tokens + 1) / 2), 128, 0, stream,
-                              lanes, L.routerAux, L.routerScale, L.logitBias, x, xStride, (int)tokens, E, D, logits, tail),
+        // A block: a warp per expert and row, for the latency, with the operands of six runs of eight groups in flight (three
+        // CTAs an SM); two runs where the row has no more, or where the CTAs would be more than two waves.  us in a graph, six / two:
+        // 512 inputs, one row and 128 experts 5.5 / 4.8, 16 rows 8.6 / 6.1; 2816 inputs, 16 rows and 128 experts 9.4 / 11.5; 4096 inputs,
+        // 16 rows and 256 experts 23.9 / 18.2.  More rows: two rows and few registers a warp.
+        const dim3 grid((E + 3) / 4, tokens <= (uint32_t)kMaxGemvRows ? tokens : (tokens + 1) / 2);
+        const bool few = D <= 1024 || grid.x * grid.y > 6u * (uint32_t)ctx->smCount;
+        auto kernel = tokens <= (uint32_t)kMaxGemvRows ? (few ? k_router_logits_int8<1, 2> : k_router_logits_int8<1, 6>)
+                                                       : (D <= 512 ? k_router_logits_int8<2, 1> : k_router_logits_int8<2, 2>);
+        FF_CUDA_OK(launch_pdl(kernel, grid, 128, 0, stream, lanes, L.routerAux, L.routerScale, L.logitBias, x, xStride, (int)tokens, E, D,
+                              logits, tail),
                    error);
     }
     return true;

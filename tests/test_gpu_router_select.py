@@ -251,28 +251,35 @@ def test_logits_of_an_odd_number_of_experts(experts):
         ctx.close()
 
 
-@pytest.mark.parametrize("scaled", [False, True])
+@pytest.mark.parametrize("form", ["bf16", "bf16_scaled", "int8"])
 @pytest.mark.parametrize("experts,d,rows", [(9, 64, 1), (16, 3072, 16), (16, 3136, 5), (128, 2816, 16), (256, 2880, 9), (256, 2880, 16),
-                                            (160, 6208, 16)])
-def test_block_router_at_its_edges(oracle, experts, d, rows, scaled):
+                                            (160, 6208, 16), (130, 512, 13), (130, 576, 14)])
+def test_block_router_at_its_edges(oracle, experts, d, rows, form):
     """A block's logits with one turn of a warp's chunks and more, one wave of CTAs and more: the oracle's, bit for bit."""
     from ane_fieldfare_b200 import hotpath as hp
     k = 5
     ctx = hp.HotpathContext(layers=1, experts=experts, d=d, f=64, sharedF=0, topK=k, maxTokens=16)
     try:
-        w = synth.normal_bf16(0x41, "block.router", (experts, d), 0.02)
         x = workload.make_tokens(0x42, f"block{rows}", rows, d)
-        eff = synth.bf16_bits(synth.uniform(7, d, 0.5, 1.5)) if scaled else None
-        ctx.loadRouter(0, w, effectiveScale=eff)
+        eff = None if form == "bf16" else synth.bf16_bits(synth.uniform(7, d, 0.5, 1.5))
+        if form == "int8":
+            router = int8_router(0x43, experts, d)
+            ctx.loadRouterInt8(0, *router, effectiveScale=eff)
+        else:
+            router = synth.normal_bf16(0x41, "block.router", (experts, d), 0.02)
+            ctx.loadRouter(0, router, effectiveScale=eff)
         ids = torch.full((rows, k), -1, dtype=torch.int32, device=ctx.device)
         weights = torch.zeros((rows, k), dtype=torch.bfloat16, device=ctx.device)
         logits = torch.zeros((rows, experts), dtype=torch.float32, device=ctx.device)
         hp.PrefillRouter(ctx).encodeGemma4Block(None, 0, hp.bf16_tensor(x, ctx.device), ids, weights, rows, outLogits=logits)
         torch.cuda.synchronize()
         assert ctx.info().deviceErrorFlag == 0
-        layer = oracle.LayerData(experts=np.zeros(16, dtype=np.uint8), stride=0, off=(0,) * 9, E=experts, D=d, F=64, K=k, router_w=w,
-                                 router_scale=eff)
-        ref_ids, ref_w, ref_logits = oracle.router_topk(layer, x)
+        if form == "int8":
+            ref_ids, ref_w, ref_logits = oracle.router_topk_int8(*router, x, k, effective_scale=eff)
+        else:
+            ref_ids, ref_w, ref_logits = oracle.router_topk(
+                oracle.LayerData(experts=np.zeros(16, dtype=np.uint8), stride=0, off=(0,) * 9, E=experts, D=d, F=64, K=k, router_w=router,
+                                 router_scale=eff), x)
         assert np.array_equal(logits.cpu().numpy(), ref_logits)
         assert np.array_equal(ids.cpu().numpy().astype(np.uint32), ref_ids)
         assert np.array_equal(hp.bf16_numpy(weights), ref_w)
