@@ -48,13 +48,36 @@ def special_rows(hp, ctx, rows, d):
 
 @pytest.mark.parametrize("form", ["bf16", "bf16_scaled", "int8"])
 @pytest.mark.parametrize("experts,d,k", [(16, 128, 8), (128, 2816, 8), (256, 448, 3), (130, 2496, 8)])
-@pytest.mark.parametrize("rows", [17, 32, 129, 161, 300, 700])
+@pytest.mark.parametrize("rows", [17, 32, 129, 700])
 def test_selected_routes_equal_the_exact_ones(form, experts, d, k, rows):
     from ane_fieldfare_b200 import hotpath as hp
     ctx = hp.HotpathContext(layers=1, experts=experts, d=d, f=64, sharedF=0, topK=k, maxTokens=700)
     try:
-        load_router(ctx, form, experts, d)
-        wide = special_rows(hp, ctx, rows, d)
+        bias = synth.normal(3, experts).astype(np.float32)
+        bias[1] = -np.inf
+        bias[8:12] = bias[8]  # (with equal weights below: exact ties)
+        eff = gain = None
+        if form != "bf16":
+            eff = synth.bf16_bits(synth.uniform(7, d, 0.5, 1.5))
+            gain = synth.bf16_bits(synth.uniform(8, experts, 0.5, 1.5))
+        if form == "int8":
+            codes, scales, biases = int8_router(0x31, experts, d)
+            for m in (codes, scales, biases):
+                m[8:12] = m[8]
+            ctx.loadRouterInt8(0, codes, scales, biases, effectiveScale=eff, perExpertScale=gain, logitBias=bias)
+        else:
+            w = synth.normal_bf16(0x32, "select.router", (experts, d), 0.02)
+            w[8:12] = w[8]
+            ctx.loadRouter(0, w, effectiveScale=eff, perExpertScale=gain, logitBias=bias)
+        x = hp.bf16_tensor(workload.make_tokens(0x33, f"select{rows}", rows, d), ctx.device)
+        wide = torch.zeros((rows, d + 8), dtype=torch.bfloat16, device=ctx.device)
+        wide[:, :d] = x
+        wide[1, :d] = 0
+        wide[2, 5] = float("nan")
+        wide[3, 6] = float("inf")
+        wide[4, :d] *= 1e30
+        wide[5, :d] *= 1e-30
+        wide[6, 7] = 3e4
         got = [torch.full((rows, k), -1, dtype=torch.int32, device=ctx.device) for _ in range(2)]
         weights = [torch.zeros((rows, k), dtype=torch.bfloat16, device=ctx.device) for _ in range(2)]
         logits = torch.zeros((rows, experts), dtype=torch.float32, device=ctx.device)
@@ -67,6 +90,13 @@ def test_selected_routes_equal_the_exact_ones(form, experts, d, k, rows):
         assert torch.equal(weights[0].view(torch.int16), weights[1].view(torch.int16))
     finally:
         ctx.close()
+
+@pytest.mark.parametrize("form", ["bf16", "bf16_scaled", "int8"])
+@pytest.mark.parametrize("experts,d,k", [(16, 128, 8), (128, 2816, 8), (256, 448, 3), (130, 2496, 8)])
+@pytest.mark.parametrize("rows", [161, 192, 300])
+def test_selected_routes_behind_approximate_logits(form, experts, d, k, rows):
+    """The same where the two launches run with eight warps a row."""
+    test_selected_routes_equal_the_exact_ones(form, experts, d, k, rows)
 
 
 @pytest.mark.parametrize("form", ["bf16", "bf16_scaled", "int8"])
@@ -139,11 +169,10 @@ def test_selected_routes_at_every_number_of_warps(form, rows):
 
 
 @pytest.mark.parametrize("form", ["bf16", "bf16_scaled", "int8"])
-@pytest.mark.parametrize("experts,d,rows", [(9, 64, 17), (12, 4160, 24), (130, 3072, 25), (128, 6400, 160), (128, 6464, 160), (128, 2816, 161),
-                                               (16, 6400, 160), (16, 6464, 160), (16, 12288, 40)])
+@pytest.mark.parametrize("experts,d,rows", [(9, 64, 17), (12, 4160, 24), (130, 3072, 25), (128, 6400, 160), (128, 6464, 160), (128, 2816, 161)])
 def test_routes_of_a_short_chunk(form, experts, d, rows):
     """Edges of the one-launch kernel: tiles of eight rows and experts, contractions of more than one set of a warp's registers,
-    and where the rows (160), their width (fp32 rows of 6400) or the pairs of row and expert go over to the two launches.  Against blocks of 16 rows, twice
+    and where the rows (160) or their width (fp32 rows of 6400) go over to the two launches.  Against blocks of 16 rows, twice
     in a row (its counters)."""
     from ane_fieldfare_b200 import hotpath as hp
     k = 5
@@ -169,6 +198,12 @@ def test_routes_of_a_short_chunk(form, experts, d, rows):
             assert torch.equal(weights[0].view(torch.int16), weights[i].view(torch.int16))
     finally:
         ctx.close()
+
+@pytest.mark.parametrize("form", ["bf16", "bf16_scaled", "int8"])
+@pytest.mark.parametrize("experts,d,rows", [(16, 6400, 160), (16, 6464, 160), (16, 12288, 40)])
+def test_routes_of_a_short_chunk_of_few_experts(form, experts, d, rows):
+    """The same at the widths' edge (fp32 rows of 6400) where the pairs of row and expert are few."""
+    test_routes_of_a_short_chunk(form, experts, d, rows)
 
 
 @pytest.mark.parametrize("form,experts,d,rows,one", [
