@@ -94,61 +94,74 @@ __global__ void __launch_bounds__(kGemvThreads) k_int4_gemv(const __grid_constan
 // Bound by its latencies.  us in a graph, 128 experts, in loads of a few chunks / eleven chunks with the scale fetched where
 // it is used / now: 2816 inputs, one row 5.3 / 5.5 / 5.0, 16 rows 6.6 / 6.8 / 6.3; scaled 6.3 / 6.8 / 5.2, 7.5 / 7.9 / 6.7; 4096
 // inputs, scaled, one row 7.4 / 8.2 / 5.7.  Eleven chunks, all of 2816 inputs, are no faster there than twelve and take a second
-// turn for 2880 to 3072 (scaled, 16 rows 7.3 / 6.9).
+// turn for 2880 to 3072 (scaled, 16 rows 7.3 / 6.9).  kRowChunks 0: loads where they are used, in few registers (39).
 template <int kRowChunks>
 __global__ void __launch_bounds__(256)
 k_router_logits(const uint16_t *W, const uint16_t *scale, const float *bias, const uint16_t *x,
                 uint32_t xStride, int E, int D, float *logits, RouterTail tail) {
-    __shared__ __align__(16) uint4 sScale[kRowChunks * 32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e = min((int)blockIdx.x * 8 + warp, E - 1);  // (a warp past the experts repeats the last)
     const int t = blockIdx.y;
     const uint16_t *wr = W + (size_t)e * D;
     const uint16_t *xr = x + (size_t)t * xStride;
-    uint4 wv[kRowChunks];
-    auto fetch = [&](int first) {
-#pragma unroll
-        for (int i = 0; i < kRowChunks; ++i) {
-            const int base = first + 256 * i + 8 * lane;
-            if (base < D) wv[i] = __ldg(reinterpret_cast<const uint4 *>(wr + base));
-        }
-        if (scale)
-            for (int i = threadIdx.x; i < kRowChunks * 32 && first + 8 * i < D; i += 256)
-                sScale[i] = __ldg(reinterpret_cast<const uint4 *>(scale + first) + i);
-    };
-    fetch(0);
-    pdl_enter();
     float acc = 0.0f;
-    for (int first = 0; first < D; first += 256 * kRowChunks) {
-        if (first) {
-            if (scale) __syncthreads();  // every warp is done with the scales before
-            fetch(first);
+    auto add_chunk = [&](const uint4 &w, const uint4 &v, const uint4 &s) {
+        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+        const uint32_t xx[4] = {v.x, v.y, v.z, v.w};
+        const uint32_t ss[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            float x0 = __uint_as_float(xx[k] << 16), x1 = __uint_as_float(xx[k] & 0xFFFF0000u);
+            if (scale) {
+                x0 = x0 * __uint_as_float(ss[k] << 16);
+                x1 = x1 * __uint_as_float(ss[k] & 0xFFFF0000u);
+            }
+            acc = fmaf(__uint_as_float(ww[k] << 16), x0, acc);
+            acc = fmaf(__uint_as_float(ww[k] & 0xFFFF0000u), x1, acc);
         }
-        uint4 xv[kRowChunks];
-#pragma unroll
-        for (int i = 0; i < kRowChunks; ++i) {
-            const int base = first + 256 * i + 8 * lane;
-            if (base < D) xv[i] = *reinterpret_cast<const uint4 *>(xr + base);
+    };
+    if constexpr (kRowChunks == 0) {
+        pdl_enter();
+        for (int base = 8 * lane; base < D; base += 256) {
+            const uint4 w = *reinterpret_cast<const uint4 *>(wr + base);
+            const uint4 v = *reinterpret_cast<const uint4 *>(xr + base);
+            uint4 s = make_uint4(0, 0, 0, 0);
+            if (scale) s = *reinterpret_cast<const uint4 *>(scale + base);
+            add_chunk(w, v, s);
         }
-        if (scale) __syncthreads();
+    } else {
+        __shared__ __align__(16) uint4 sScale[kRowChunks * 32];
+        uint4 wv[kRowChunks];
+        auto fetch = [&](int first) {
 #pragma unroll
-        for (int i = 0; i < kRowChunks; ++i) {
-            const int base = first + 256 * i + 8 * lane;
-            if (base >= D) break;
-            uint4 sv = make_uint4(0, 0, 0, 0);
-            if (scale) sv = sScale[32 * i + lane];
-            const uint32_t ww[4] = {wv[i].x, wv[i].y, wv[i].z, wv[i].w};
-            const uint32_t xx[4] = {xv[i].x, xv[i].y, xv[i].z, xv[i].w};
-            const uint32_t ss[4] = {sv.x, sv.y, sv.z, sv.w};
+            for (int i = 0; i < kRowChunks; ++i) {
+                const int base = first + 256 * i + 8 * lane;
+                if (base < D) wv[i] = __ldg(reinterpret_cast<const uint4 *>(wr + base));
+            }
+            if (scale)
+                for (int i = threadIdx.x; i < kRowChunks * 32 && first + 8 * i < D; i += 256)
+                    sScale[i] = __ldg(reinterpret_cast<const uint4 *>(scale + first) + i);
+        };
+        fetch(0);
+        pdl_enter();
+        for (int first = 0; first < D; first += 256 * kRowChunks) {
+            if (first) {
+                if (scale) __syncthreads();  // every warp is done with the scales before
+                fetch(first);
+            }
+            uint4 xv[kRowChunks];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                float x0 = __uint_as_float(xx[k] << 16), x1 = __uint_as_float(xx[k] & 0xFFFF0000u);
-                if (scale) {
-                    x0 = x0 * __uint_as_float(ss[k] << 16);
-                    x1 = x1 * __uint_as_float(ss[k] & 0xFFFF0000u);
-                }
-                acc = fmaf(__uint_as_float(ww[k] << 16), x0, acc);
-                acc = fmaf(__uint_as_float(ww[k] & 0xFFFF0000u), x1, acc);
+            for (int i = 0; i < kRowChunks; ++i) {
+                const int base = first + 256 * i + 8 * lane;
+                if (base < D) xv[i] = *reinterpret_cast<const uint4 *>(xr + base);
+            }
+            if (scale) __syncthreads();
+#pragma unroll
+            for (int i = 0; i < kRowChunks; ++i) {
+                if (first + 256 * i + 8 * lane >= D) break;
+                uint4 s = make_uint4(0, 0, 0, 0);
+                if (scale) s = sScale[32 * i + lane];
+                add_chunk(wv[i], xv[i], s);
             }
         }
     }
@@ -752,9 +765,13 @@ bool launch_router_topk(FFContext *ctx, const LayerStore &L, const uint16_t *x, 
     if (L.routerQ) return launch_router_logits_int8(ctx, L, x, xStride, tokens, lg, tail, stream, error);
     {
         LaunchScope scope(ctx, stream, "router_logits");
-        // twelve chunks in flight (two CTAs an SM) while the CTAs are at most one wave; more CTAs: four, and four an SM
+        // Twelve chunks in flight (two CTAs an SM) while the CTAs are at most one wave of them, four (and four an SM) where they
+        // are more than three an SM, loads where they are used in between.  us in a graph, 12 / 0 / 4: 160 experts, 16 rows, 4096
+        // inputs 8.3 / 7.4 / 8.6, 6144 9.8 / 8.4 / 10.3, scaled 12.6 / 10.7 / 12.5; 256 experts, 9 rows, 6144 inputs 9.4 / 9.6 / 9.5, 13
+        // rows 12.8 / 10.0 / 11.1, 16 rows 13.2 / 12.3 / 11.7, scaled 16.1 / 15.5 / 14.1.
         const dim3 grid((E + 7) / 8, tokens);
-        auto kernel = grid.x * grid.y <= 2u * (uint32_t)ctx->smCount ? k_router_logits<12> : k_router_logits<4>;
+        const uint32_t perSm = (grid.x * grid.y + (uint32_t)ctx->smCount - 1u) / (uint32_t)ctx->smCount;
+        auto kernel = perSm <= 2u ? k_router_logits<12> : perSm == 3u ? k_router_logits<0> : k_router_logits<4>;
         FF_CUDA_OK(launch_pdl(kernel, grid, 256, 0, stream, L.routerW, L.routerScale, L.logitBias, x, xStride, E, D, lg, tail), error);
     }
     return true;
