@@ -939,14 +939,27 @@ bool launch_router_logits_int8(FFContext *ctx, const LayerStore &L, const uint16
     const uint4 *lanes = reinterpret_cast<const uint4 *>(L.routerLanes);
     {
         LaunchScope scope(ctx, stream, "router_logits_int8");
-        // A block: a warp per expert and row, for the latency, with the operands of six runs of eight groups in flight (three
-        // CTAs an SM); two runs where the row has no more, or where the CTAs would be more than two waves.  us in a graph, six / two:
-        // 512 inputs, one row and 128 experts 5.5 / 4.8, 16 rows 8.6 / 6.1; 2816 inputs, 16 rows and 128 experts 9.4 / 11.5; 4096 inputs,
-        // 16 rows and 256 experts 23.9 / 18.2.  More rows: two rows and few registers a warp.
+        // A turn of a warp's loop loads all its places, so what it holds follows the row's runs of eight groups.
+        // A block: a warp per expert and row, for the latency, with up to six runs in flight (three CTAs an SM): four where that
+        // makes the row's turns even (1088 to 2048 and 3136 to 4096 inputs), two where the row has no more or where the CTAs would
+        // be more than six an SM.  us in a graph, six / four / two: 512 inputs, 128 experts, one row 6.0 / 5.6 / 5.3, 16 rows 9.6 / 6.9 /
+        // 6.4; 2816 inputs, 128 experts, one row 5.8 / 6.6 / 6.7, 16 rows 9.5 / 10.0 / 11.5; 4096 inputs, 128 experts, one row 7.8 / 6.8 /
+        // 7.7, 16 rows 15.1 / 10.6 / 13.6, 256 experts, 13 rows 20.2 / 16.0 / 15.5, 16 rows 24.5 / 17.7 / 17.9.
+        // More rows: two rows and few registers a warp, and two runs where their number is even; else three where it divides
+        // or the CTAs are few, else one.  three / two / one, 128 experts: 1536 inputs, 17 rows 6.6 / 7.3 / -, 160 rows 18.9 / 21.5 / -;
+        // 2304 inputs, 160 rows - / 29.5 / 27.5; 2816 inputs, 160 rows 31.1 / 31.4 / 32.0; 4096 inputs, 160 rows 43.5 / 41.4 / 41.9.
         const dim3 grid((E + 3) / 4, tokens <= (uint32_t)kMaxGemvRows ? tokens : (tokens + 1) / 2);
-        const bool few = D <= 1024 || grid.x * grid.y > 6u * (uint32_t)ctx->smCount;
-        auto kernel = tokens <= (uint32_t)kMaxGemvRows ? (few ? k_router_logits_int8<1, 2> : k_router_logits_int8<1, 6>)
-                                                       : (D <= 512 ? k_router_logits_int8<2, 1> : k_router_logits_int8<2, 2>);
+        const uint32_t ctas = grid.x * grid.y, sms = (uint32_t)ctx->smCount;
+        const uint32_t runs = ((uint32_t)D / 64u + 7u) / 8u, turns = (runs + 5u) / 6u, inTurn = (runs + turns - 1u) / turns;
+        auto kernel = k_router_logits_int8<1, 6>;
+        if (tokens <= (uint32_t)kMaxGemvRows) {
+            if (inTurn <= 2u || ctas > 6u * sms) kernel = k_router_logits_int8<1, 2>;
+            else if (inTurn <= 4u) kernel = k_router_logits_int8<1, 4>;
+        } else if (runs % 2u == 0u) {
+            kernel = k_router_logits_int8<2, 2>;
+        } else {
+            kernel = runs % 3u == 0u || (runs > 3u && ctas <= 3u * sms) ? k_router_logits_int8<2, 3> : k_router_logits_int8<2, 1>;
+        }
         FF_CUDA_OK(launch_pdl(kernel, grid, 128, 0, stream, lanes, L.routerAux, L.routerScale, L.logitBias, x, xStride, (int)tokens, E, D,
                               logits, tail),
                    error);

@@ -320,3 +320,27 @@ def test_block_router_at_its_edges(oracle, experts, d, rows, form):
         assert np.array_equal(hp.bf16_numpy(weights), ref_w)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("d", [64, 512, 1088, 1536, 2304, 2816, 3584, 4672])
+@pytest.mark.parametrize("experts,rows", [(10, 17), (256, 33)])
+def test_int8_logits_of_many_rows(d, experts, rows):
+    """Logits asked for, with one, two and three runs of a row held at a time and odd last runs: as blocks of 16 rows give them."""
+    from ane_fieldfare_b200 import hotpath as hp
+    k = 5
+    ctx = hp.HotpathContext(layers=1, experts=experts, d=d, f=64, sharedF=0, topK=k, maxTokens=rows)
+    try:
+        ctx.loadRouterInt8(0, *int8_router(0x44, experts, d), effectiveScale=synth.bf16_bits(synth.uniform(7, d, 0.5, 1.5)))
+        x = hp.bf16_tensor(workload.make_tokens(0x45, f"many{rows}", rows, d), ctx.device)
+        got = [(torch.full((rows, k), -1, dtype=torch.int32, device=ctx.device), torch.zeros((rows, k), dtype=torch.bfloat16, device=ctx.device),
+                torch.zeros((rows, experts), dtype=torch.float32, device=ctx.device)) for _ in range(2)]
+        router = hp.PrefillRouter(ctx)
+        for r in range(0, rows, 16):
+            router.encodeGemma4Block(None, 0, x[r:], got[0][0][r:], got[0][1][r:], min(16, rows - r), outLogits=got[0][2][r:])
+        router.encodeGemma4Block(None, 0, x, got[1][0], got[1][1], rows, outLogits=got[1][2])
+        torch.cuda.synchronize()
+        assert ctx.info().deviceErrorFlag == 0
+        assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1].view(torch.int16), got[1][1].view(torch.int16))
+        assert torch.equal(got[0][2], got[1][2])
+    finally:
+        ctx.close()
