@@ -206,7 +206,8 @@ k_reduce_token_major(const uint16_t *partials, const uint32_t *rowIndex, const u
 // are the time (77 rows 4.4 -> 3.5 us); B = 1 beyond, where more warps in flight beat more loads of each (32768
 // rows 363 us, with B = 8 450 us).  STREAM: the partial rows are streamed, which pays from four of them a row on: eight a row,
 // written and reduced, 1500 rows of 2816 36.2 -> 33.7 us, 4096 102.0 -> 91.0 (a layer of 4096 rows 614 -> 607); four, 4096 rows
-// 54.9 -> 48.8; three 39.5 -> 41.5, two 26.9 -> 28.6.
+// 54.9 -> 48.8; three 39.5 -> 41.5, two 26.9 -> 28.6.  With B = 8 from eight on: 200 rows of 2816 2.7 -> 2.4; six, 40 rows of 6144
+// 2.1 -> 2.5, five, 128 rows of 1024 1.9 -> 2.3.
 template <int B, bool STREAM>
 __global__ void __launch_bounds__(256)
 k_reduce_token_major_x8(const uint16_t *partials, const uint32_t *rowIndex, const uint16_t *weights,
@@ -813,9 +814,9 @@ bool launch_reduce(FFContext *ctx, const uint16_t *partials, const uint16_t *wei
         if (wide) {
             const size_t items = (size_t)tokens * (D / 8);
             const unsigned blocks = (unsigned)((items + 255) / 256);
-            auto kernel = blocks <= (unsigned)ctx->smCount * 4 ? k_reduce_token_major_x8<8, true>
-                          : ctx->cfg.topK > 3                  ? k_reduce_token_major_x8<1, true>
-                                                               : k_reduce_token_major_x8<1, false>;
+            const uint32_t K = ctx->cfg.topK;
+            auto kernel = blocks <= (unsigned)ctx->smCount * 4 ? (K == 8 ? k_reduce_token_major_x8<8, true> : k_reduce_token_major_x8<8, false>)
+                                                               : (K > 3 ? k_reduce_token_major_x8<1, true> : k_reduce_token_major_x8<1, false>);
             FF_CUDA_OK(launch_pdl(kernel, blocks, 256, 0, stream,
                               partials, rowIndex, weights, residual, y, (int)tokens, (int)ctx->cfg.topK, D),
                    error);
