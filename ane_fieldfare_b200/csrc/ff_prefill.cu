@@ -1273,19 +1273,22 @@ static GemmRings gemm_rings(int mode, uint32_t K, uint32_t tileRows) {
 // 1400 (87) 291 / 298, 1500 (94) 313 / 313, 2000 (125) 373 / 357, 4096 648 / 634.
 static uint32_t routed_tile_rows(uint32_t pairs, uint32_t experts) { return pairs <= 96u * experts ? kRowTileSmall : kRowTile; }
 
-// Of the shared FFN's two GEMMs: where whole waves of a step take less time (by their columns, 3 : 4), and tiles of 128
-// rows while those of gate/up are at most two: then a wave's fill and drain count for more than its columns.  us with 128 /
-// 192 (d x f): 2816 x 2112, 77 rows 23.7 / 25.8, 613 34.1 / 38.4, 1000 (two waves) 40.6 / 44.6, 1500 50.6 / 55.3, 3000 97.9 /
-// 89.9, 4096 124.5 / 130.2; 2816 x 6144, 300 rows 46.5 / 53.9, 1000 (six waves) 101.0 / 85.8; 5120 x 8192, 513 rows 140.1 / 109.6.
+// Of the shared FFN's two GEMMs: where whole waves of a step take less time; a step of 192 rows takes 1.36 times one of 128
+// (their columns 1.5).  And tiles of 128 rows while gate/up has at most two waves of them, unless those of 192 save both
+// GEMMs a wave: the second is mostly the last row tile's units, which have few columns.  us with 128 / 192 (d x f, waves of
+// gate/up and down): 2816 x 2112, 77 rows (1, 1 / 1, 1) 23.7 / 25.8, 613 (2, 1 / 1, 1) 34.1 / 38.4, 1500 50.6 / 55.3, 3000 97.9 / 89.9,
+// 4096 124.5 / 130.2; 4096 x 2048, 613 rows (2, 2 / 1, 1) 50.9 / 42.1; 6144 x 1024, 1500 rows (2, 4 / 1, 3) 64.8 / 54.8; 5120 x 1536, 3000
+// rows (4, 7 / 3, 5) 118.4 / 125.3; 2816 x 6144, 300 rows 46.5 / 53.9, 1000 101.0 / 85.8, 4096 (21, 5 / 15, 4) 326.9 / 342.6.
 static uint32_t dense_tile_rows(uint32_t smCount, uint32_t d, uint32_t f, uint32_t tokens) {
     const uint32_t clusters = std::max(1u, smCount / 2u);
     const auto waves = [&](uint32_t rows, uint32_t nTiles) {
         return ((uint64_t)((tokens + rows - 1u) / rows) * ((nTiles + 1u) / 2u) + clusters - 1u) / clusters;
     };
     const uint32_t gateUp = (f + 63u) / 64u, down = (d + 127u) / 128u;
-    const auto cost = [&](uint32_t rows) { return (waves(rows, gateUp) * d + waves(rows, down) * f) * rows; };
-    if (waves(kRowTileSmall, gateUp) <= 2u) return kRowTileSmall;
-    return cost(kRowTileSmall) * 9u <= cost(kRowTile) * 8u ? kRowTileSmall : kRowTile;
+    const uint64_t gSmall = waves(kRowTileSmall, gateUp), dSmall = waves(kRowTileSmall, down);
+    const uint64_t gLarge = waves(kRowTile, gateUp), dLarge = waves(kRowTile, down);
+    if (gSmall <= 2u && (gLarge == gSmall || dLarge == dSmall)) return kRowTileSmall;
+    return (gSmall * d + dSmall * f) * 100u <= (gLarge * d + dLarge * f) * 136u ? kRowTileSmall : kRowTile;
 }
 
 // `rows` activation rows of args.K elements at `x`

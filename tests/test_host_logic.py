@@ -230,7 +230,8 @@ def test_prefill_gemm_rings_never_alias_a_phase(mode, tileRows):
     (2816, 2112, 77, 128), (2816, 2112, 613, 128), (2816, 2112, 1024, 128), (2816, 2112, 1500, 128), (2816, 2112, 3000, 192),
     (2816, 2112, 4096, 128), (2816, 4096, 300, 128), (2816, 4096, 700, 128), (2816, 4096, 900, 192), (2816, 6144, 300, 128),
     (2816, 6144, 1000, 192), (4096, 4096, 613, 192), (4096, 4096, 1000, 128), (5120, 8192, 513, 192), (5120, 8192, 900, 192),
-    (4096, 1024, 1000, 128)])
+    (4096, 1024, 1000, 128), (4096, 2048, 613, 192), (4096, 2048, 1000, 128), (5120, 1536, 1000, 192), (5120, 1536, 3000, 128),
+    (6144, 1024, 1000, 128), (6144, 1024, 1500, 192), (2048, 768, 1700, 192), (2816, 6144, 4096, 128), (1024, 2816, 1700, 128)])
 def test_dense_tile_rows_follow_the_waves(d, f, rows, want):
     """The shared FFN's row tile on 148 SMs where one of the two was 4 % faster at least, whatever the number of rows."""
     assert binding.load().ff_prefill_dense_tile_rows(148, d, f, rows) == want
