@@ -57,6 +57,7 @@ constexpr uint32_t kPassTokens = 16;             // tokens of a set that become 
 constexpr uint32_t kXchgBytes = 128u * 8u * 4u;  // half of them, of every row, from gate to up or back
 constexpr uint32_t kTilePitchGateUp = 64 * 2 + 16, kTilePitchDown = 128 * 2 + 16;
 static_assert(kOperandCol + kOperandStages * 32 <= 512, "tensor memory layout");
+static_assert(kSetTokens == 32, "tiles are multiples of a set's tokens");
 static_assert(kStages % kOperandStages == 0 && kOperandStages % kDequantGroups == 0, "rings");
 
 enum Mode : int { kGateUp = 0, kDown = 1 };
@@ -123,6 +124,9 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rawBase = smem_u32(smemRaw), base = (rawBase + 1023u) & ~1023u;
     const uint32_t groupsK = args.K / kStepK, steps = groupsK + 3u * sum_blocks(args.K);
+    // Draining sets whose tokens a tile has; the rest of the sixteen warps would only wait and arrive, which small tiles paid
+    // for at every step.
+    const uint32_t drainSets = args.tileRows / kSetTokens, drainThreads = 128u * drainSets;
 
     // carve-up: token tiles, code tiles, two buffers of scales, exchange rows (gate/up), output tiles
     auto tokAddr = [&](uint32_t s) { return base + s * kTokBytes; };
@@ -157,10 +161,10 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
         }
         for (uint32_t s = 0; s < kAccs; ++s) {
             mbar_init(barAccFull(s), 1);
-            mbar_init(barAccEmpty(s), 2 * kDrainThreads / 32);
+            mbar_init(barAccEmpty(s), 2 * drainThreads / 32);
         }
         for (uint32_t s = 0; s < kDrainSets; ++s) mbar_init(barSet(s), 128);
-        mbar_init(barScales, kDrainThreads);
+        mbar_init(barScales, drainThreads);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -332,9 +336,9 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
             stepNo += kDequantGroups;
             g += kDequantGroups;
         }
-    } else {
+    } else if (warp < (int)(2u + 4u * kDequantGroups + 4u * drainSets)) {
         // ---------------- drain: scaled sums in registers, then the outputs ----------------
-        const uint32_t t = (uint32_t)threadIdx.x - (2u + 4u * kDequantGroups) * 32u;  // 0..511
+        const uint32_t t = (uint32_t)threadIdx.x - (2u + 4u * kDequantGroups) * 32u;  // 0..drainThreads - 1
         const uint32_t set = t >> 7, th = t & 127u;                                   // its tokens of the tile start at kSetTokens set
         const uint32_t quarter = (uint32_t)(warp & 3), m = quarter * 32u + (uint32_t)lane;
         const uint32_t tmemLane = tmemBase + ((quarter * 32u) << 16) + set * kSetTokens;
@@ -356,7 +360,7 @@ k_int8_gemm(const __grid_constant__ CUtensorMap mapTok, const __grid_constant__ 
             const uint32_t setRows = min(rows, (set + 1u) * kSetTokens) - min(rows, set * kSetTokens);
             // the unit's scales: 128 rows (gate/up: 64 of either matrix), contiguous in memory
             uint16_t *scales = scaleBuf + (unitNo & 1u) * 128u * groupsK;
-            for (uint32_t i = t; i < 16u * groupsK; i += kDrainThreads) {  // 16-byte pieces, 8 groupsK per 64 rows
+            for (uint32_t i = t; i < 16u * groupsK; i += drainThreads) {  // 16-byte pieces, 8 groupsK per 64 rows
                 const uint32_t part = i / (8u * groupsK), piece = i - part * 8u * groupsK;
                 const uint32_t row0 = MODE == kGateUp ? nt * 64u : nt * 128u + part * 64u;
                 uint4 v = make_uint4(0, 0, 0, 0);
