@@ -13,13 +13,14 @@
 // Two CTAs of a cluster work as one tensor-core unit (cta_group::2, M = 256: either CTA 128 weight
 // rows, half of the token tile).  Per CTA: warp 0 TMA producer, warp 1 MMA issuer (leader only),
 // warps 2-9 turn codes into bf16 pairs in tensor memory (two groups of four warps, alternate steps),
-// warps 10-25 drain: a thread owns one weight row and 32 tokens.  Tensor memory: three accumulators of
+// warps 10-25 drain, four for every 32 tokens of the tile: a thread owns one weight row and 32 tokens.  Tensor memory: three accumulators of
 // 128 columns, four operand stages of 32.
 //
 // What bounds it: the draining warps.  A step is 2700 warp instructions of a CTA (128 tokens; 512 of them the
 // multiply-adds), and each warp goes through a step's wait, loads and arrival one after another, 800 to 900 cycles
-// for the tensor core's 256.  2000 rows of 2816 x 2112: gate/up and down 159 us; with eight draining warps of 64
-// tokens, which did not fit their registers, 196 us.  Measured and not kept: loads of 32 columns (181 us: nothing
+// for the tensor core's 256.  2000 rows of 2816 x 2112: gate/up and down 153 us; with eight draining warps of 64
+// tokens, which did not fit their registers, 191 us.  Small tiles leave draining warps without tokens: with these waiting and
+// arriving at every step, 17 rows 39.9 us, 300 rows 44.7, and 36.1 and 42.2 without them.  Measured and not kept: loads of 32 columns (181 us: nothing
 // overlaps them), eight warps with 152 registers by setmaxnreg and a load always in flight (199 us), packed
 // multiply-adds (the compiler moves as many registers as they save), one dequantizing group (171 us).
 //
@@ -502,9 +503,9 @@ bool make_code_map(CUtensorMap *map, const uint8_t *base, uint64_t rows, uint64_
 }
 
 // Tokens per tile: the size whose waves of units take the least time.  A wave of gate/up units over 2816 inputs (47
-// steps) takes 21.6, 23.2, 24.9 and 26.8 us with tiles of 32, 64, 96 and 128 tokens (4096 rows, each size forced).
+// steps) takes 18.7, 20.1, 22.3 and 24.8 us with tiles of 32, 64, 96 and 128 tokens (4096 rows, each size forced).
 uint32_t pick_tile_rows(uint32_t tokens, uint32_t nPairs, uint32_t clusters) {
-    constexpr uint32_t kWave[kMaxRows / 32] = {216, 232, 249, 268};
+    constexpr uint32_t kWave[kMaxRows / 32] = {187, 201, 223, 248};
     uint32_t best = kMaxRows;
     uint64_t bestCost = ~0ull;
     for (uint32_t r = 32; r <= kMaxRows; r += 32) {
